@@ -523,6 +523,11 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
                         int64_t workspace_bytes, void *d_stage, int64_t stage_bytes, float *d_prob, float *h_prob,
                         int32_t *d_status, void *stream);
 
+/* Average precision, ROC area and accuracy of every batch of a scored stream (evaluation/evaluation.py:30-44):
+ * batch i covers edges [i * bs, (i + 1) * bs), h_out[3 * i .. 3 * i + 2] = {AP, AUC, share of edges with
+ * pos >= neg}.  Host memory only; a score that is not finite is ORCA_E_BADARG. */
+int orca_link_metrics(const float *h_pos, const float *h_neg, int64_t n_edges, int32_t bs, double *h_out);
+
 /* Sharing the exchange buffer of the multi-GPU split between the processes of one node (no counterpart
  * in the reference).  orca_ipc_export: the 64-byte CUDA IPC handle of the allocation that holds d_ptr and
  * d_ptr's offset inside it; orca_ipc_open (in another process, on its own GPU): the address of the same

@@ -17,6 +17,7 @@ DIM = 172
 QT_DIM = 1032
 QT_LD = 1056
 MSG_DIM = 688
+E_BADARG = 1      # ORCA_E_BADARG
 CAND_CAP = 2048   # ORCA_CAND_CAP
 EXCHANGE_SLOTS = 4  # ORCA_EXCHANGE_SLOTS
 FLAG_WORDS = 48     # ORCA_FLAG_WORDS
@@ -124,6 +125,7 @@ SYMBOLS = {
     "orca_tgn_eval_batch_sharded": (C.c_int, [C.POINTER(TgnT), _I32, _V, _V, _I32, _V, _I32, _I32, _V, _I64, _V, _V,
                                               _V, _V, _V, _V]),
     "orca_tgn_eval_epoch": (C.c_int, [C.POINTER(TgnT), C.POINTER(EpochT), _I32, _V, _I64, _V, _I64, _V, _V, _V, _V]),
+    "orca_link_metrics": (C.c_int, [_V, _V, _I64, _I32, _V]),
     "orca_stage_h2d": (C.c_int, [_V, _V, C.c_int64, _V]),
     "orca_ipc_export": (C.c_int, [_V, _V, C.POINTER(C.c_int64)]),
     "orca_ipc_open": (C.c_int, [_V, C.c_int64, C.POINTER(C.c_void_p)]),

