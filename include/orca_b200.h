@@ -149,6 +149,13 @@ int orca_sample_topk_mark(const int64_t *d_indptr, const int32_t *d_adj_nbr, con
                           int32_t *d_nbr, int32_t *d_eid, float *d_edge_times, float *d_delta,
                           int32_t *d_status, const uint8_t *d_cache_flag, uint32_t *d_cand_bitmap,
                           void *stream);
+/* The same from host arrays to host tables, synchronously.  h_pinned (page-locked) and d_buffer have the same
+ * layout: times 8 * n_query | ids 4 * n_query, padded to 16 | status 16 | neighbours | edge ids | edge times, each
+ * table 4 * n_query * k bytes; the tables are read from h_pinned when the call returns. */
+int orca_sample_topk_host(const int64_t *d_indptr, const int32_t *d_adj_nbr, const int32_t *d_adj_eid,
+                          const double *d_adj_ts, int64_t n_nodes, const int64_t *h_nodes, const double *h_ts,
+                          int32_t n_query, int32_t k, void *h_pinned, void *d_buffer, int64_t buffer_bytes,
+                          void *stream);
 
 /* find_before (utils/util.py:129-131) on its own: the number of interactions of d_nodes[i]
  * strictly before d_ts[i]. */

@@ -94,6 +94,7 @@ SYMBOLS = {
     "orca_sample_topk": (C.c_int, [_V, _V, _V, _V, _I64, _V, _V, _I32, _V, _I32, _V, _V, _V, _V, _V, _V]),
     "orca_sample_topk_mark": (C.c_int, [_V, _V, _V, _V, _I64, _V, _V, _I32, _V, _I32, _V, _V, _V, _V, _V, _V, _V, _V]),
     "orca_find_uncached_marked": (C.c_int, [_V, _I32, _I64, _V, _V, _I32, _V, _V, _V]),
+    "orca_sample_topk_host": (C.c_int, [_V, _V, _V, _V, _I64, _V, _V, _I32, _I32, _V, _V, _I64, _V]),
     "orca_find_before": (C.c_int, [_V, _V, _I64, _V, _V, _I32, _V, _V]),
     "orca_find_uncached_scratch_bytes": (_I64, [_I64]),
     "orca_find_uncached": (C.c_int, [_V, _I32, _I32, _V, _I64, _V, _V, _I32, _V, _V, _V, _V]),

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <numeric>
 #include <stdarg.h>
+#include <string.h>
 #include <vector>
 
 #include "common.cuh"
@@ -784,6 +785,38 @@ int orca_sample_topk_mark(const int64_t *d_indptr, const int32_t *d_adj_nbr, con
   return orca_sample_topk_impl(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, d_nodes, d_ts, n_query_cap,
                           d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status, d_cache_flag,
                           d_cand_bitmap, stream);
+}
+
+// A caller with host arrays: ids narrowed and times copied into page-locked memory, one copy in, the sampling launch,
+// one copy out (status word and the three tables lie together), one wait.  40 k queries of k = 10 move 4.8 MB out,
+// 0.1 ms of bus time, which is what bounds the call.
+int orca_sample_topk_host(const int64_t *d_indptr, const int32_t *d_adj_nbr, const int32_t *d_adj_eid,
+                          const double *d_adj_ts, int64_t n_nodes, const int64_t *h_nodes, const double *h_ts,
+                          int32_t n_query, int32_t k, void *h_pinned, void *d_buffer, int64_t buffer_bytes, void *stream) {
+  ORCA_CHECK_ARG(h_nodes && h_ts && h_pinned && d_buffer && n_query > 0 && k >= 1 && k <= ORCA_MAX_K);
+  const int64_t off_status = ((int64_t)n_query * 12 + 15) & ~15ll, off_out = off_status + 16;
+  const int64_t table = (int64_t)n_query * k * 4, total = off_out + 3 * table;
+  if (buffer_bytes < total)
+    return set_error(ORCA_E_CAPACITY, "orca_sample_topk_host: buffers of %lld bytes, %lld needed", (long long)buffer_bytes,
+                     (long long)total);
+  cudaStream_t s = (cudaStream_t)stream;
+  char *h = (char *)h_pinned, *d = (char *)d_buffer;
+  memcpy(h, h_ts, (size_t)n_query * 8);
+  int32_t *ids = (int32_t *)(h + (int64_t)n_query * 8);
+  for (int32_t i = 0; i < n_query; ++i) ids[i] = (int32_t)h_nodes[i];
+  memset(h + off_status, 0, 16);
+  ORCA_CUDA(cudaMemcpyAsync(d, h, (size_t)off_out, cudaMemcpyHostToDevice, s));
+  const int rc = orca_sample_topk(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, (int32_t *)(d + (int64_t)n_query * 8),
+                                  (double *)d, n_query, nullptr, k, (int32_t *)(d + off_out),
+                                  (int32_t *)(d + off_out + table), (float *)(d + off_out + 2 * table), nullptr,
+                                  (int32_t *)(d + off_status), stream);
+  if (rc == ORCA_OK)
+    ORCA_CUDA(cudaMemcpyAsync(h + off_status, d + off_status, (size_t)(total - off_status), cudaMemcpyDeviceToHost, s));
+  ORCA_CUDA(cudaStreamSynchronize(s));
+  if (rc) return rc;
+  const int32_t *status = (const int32_t *)(h + off_status);
+  if (status[0] != 0) return set_error(status[0], "device status %d (detail %d)", status[0], status[3]);
+  return ORCA_OK;
 }
 
 int orca_find_before(const int64_t *d_indptr, const double *d_adj_ts, int64_t n_nodes,

@@ -15,6 +15,8 @@ from . import _lib
 
 
 class NeighborFinder:
+    PINNED_TABLE = 64 << 20     # bytes of one returned table up to which it stays in page-locked memory
+
     def __init__(self, node_to_neighbors, node_to_edge_idxs, node_to_edge_timestamps, device="cuda"):
         """Same arguments as utils/util.py:123-126: per-node arrays, each already sorted by time."""
         lens = np.fromiter((len(a) for a in node_to_neighbors), dtype=np.int64, count=len(node_to_neighbors))
@@ -86,8 +88,29 @@ class NeighborFinder:
         """Returns (neighbors int32 [Q,K], edge_idxs int32 [Q,K], edge_times float32 [Q,K]) as NumPy
         arrays: the K most recent interactions strictly before each query time, right-aligned,
         zero-padded on the left."""
-        nbr, eid, et, _ = self.sample_device(source_nodes, timestamps, n_neighbors)
-        return nbr.cpu().numpy(), eid.cpu().numpy(), et.cpu().numpy()
+        q, k = len(source_nodes), int(n_neighbors)
+        table = 4 * q * k
+        # The tables are returned in the page-locked memory that they were copied to: a fresh pageable array of a few
+        # MB costs more in page faults than the whole call.  Tables too large to keep page-locked, inputs that are
+        # already on the GPU and empty queries take the general path.
+        if not 0 < table <= self.PINNED_TABLE or isinstance(source_nodes, torch.Tensor) or isinstance(timestamps, torch.Tensor):
+            nbr, eid, et, _ = self.sample_device(source_nodes, timestamps, n_neighbors)
+            return nbr.cpu().numpy(), eid.cpu().numpy(), et.cpu().numpy()
+        nodes = np.ascontiguousarray(source_nodes, dtype=np.int64)
+        ts = np.ascontiguousarray(timestamps, dtype=np.float64)
+        if nodes.shape != (q,) or ts.shape != (q,):
+            raise ValueError("source_nodes and timestamps must be one-dimensional and of one length")
+        out = (12 * q + 15) // 16 * 16 + 16
+        pin = torch.empty(out + 3 * table, dtype=torch.uint8, pin_memory=True)
+        dev = torch.empty(out + 3 * table, dtype=torch.uint8, device=self.device)
+        with torch.cuda.device(self.device):
+            _lib.check(_lib.lib().orca_sample_topk_host(
+                self.indptr.data_ptr(), self.adj_nbr.data_ptr(), self.adj_eid.data_ptr(), self.adj_ts.data_ptr(),
+                self.n_nodes, nodes.ctypes.data, ts.ctypes.data, q, k, pin.data_ptr(), dev.data_ptr(), dev.numel(),
+                _lib.stream_ptr(self.device)))
+        h = pin.numpy()
+        part = lambda i, dt: h[out + i * table:out + (i + 1) * table].view(dt).reshape(q, k)
+        return part(0, np.int32), part(1, np.int32), part(2, np.float32)
 
     def sample_device(self, source_nodes, timestamps, n_neighbors, want_delta=False):
         """Same as get_temporal_neighbor but the tables stay on the device (torch tensors);
