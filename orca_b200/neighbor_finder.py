@@ -50,23 +50,26 @@ class NeighborFinder:
         self.device = dev = _lib.require_cuda(device)
         self.n_nodes = int(n_nodes)
         E = len(sources)
-        up = lambda a, dt: torch.as_tensor(np.array(a, dtype=dt, order="C")).to(dev)     # (a copy: the input may be read-only)
-        src, dst, eidx = (up(a, np.int64) for a in (sources, destinations, edge_idxs))
-        ts = up(timestamps, np.float64)
+        src, dst, eidx = (np.ascontiguousarray(a, dtype=np.int64) for a in (sources, destinations, edge_idxs))
+        ts = np.ascontiguousarray(timestamps, dtype=np.float64)
+        if not len(src) == len(dst) == len(eidx) == len(ts):
+            raise ValueError("sources, destinations, edge_idxs and timestamps must have one length")
         L = _lib.lib()
         with torch.cuda.device(dev):
+            new = torch.empty if E else torch.zeros      # (one spare element keeps the pointers of an empty graph valid)
             self.indptr = torch.empty(self.n_nodes + 1, dtype=torch.int64, device=dev)
-            self.adj_nbr = torch.zeros(max(2 * E, 1), dtype=torch.int32, device=dev)
-            self.adj_eid = torch.zeros(max(2 * E, 1), dtype=torch.int32, device=dev)
-            self.adj_ts = torch.zeros(max(2 * E, 1), dtype=torch.float64, device=dev)
-            ws_bytes = L.orca_csr_build_workspace_bytes(E, self.n_nodes)
-            ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-            status = torch.zeros(4, dtype=torch.int32, device=dev)
-            _lib.check(L.orca_csr_build(src.data_ptr(), dst.data_ptr(), eidx.data_ptr(), ts.data_ptr(), E,
-                                        self.n_nodes, self.indptr.data_ptr(), self.adj_nbr.data_ptr(),
-                                        self.adj_eid.data_ptr(), self.adj_ts.data_ptr(), status.data_ptr(),
-                                        ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev)))
-            _lib.check(L.orca_read_status(None, status.data_ptr(), None, _lib.stream_ptr(dev)))
+            self.adj_nbr = new(max(2 * E, 1), dtype=torch.int32, device=dev)
+            self.adj_eid = new(max(2 * E, 1), dtype=torch.int32, device=dev)
+            self.adj_ts = new(max(2 * E, 1), dtype=torch.float64, device=dev)
+            ws = torch.empty(max(L.orca_csr_build_workspace_bytes(E, self.n_nodes), 256), dtype=torch.uint8, device=dev)
+            pin = torch.empty(max(L.orca_csr_build_pinned_bytes(E), 1), dtype=torch.uint8, pin_memory=True)
+            stream = torch.cuda.current_stream(dev)
+            rc = L.orca_csr_build_from_host(src.ctypes.data, dst.ctypes.data, eidx.ctypes.data, ts.ctypes.data, E,
+                                            self.n_nodes, pin.data_ptr(), pin.numel(), self.indptr.data_ptr(),
+                                            self.adj_nbr.data_ptr(), self.adj_eid.data_ptr(), self.adj_ts.data_ptr(),
+                                            ws.data_ptr(), ws.numel(), stream.cuda_stream)
+            stream.synchronize()                         # (the pinned chunks go back to their pool)
+            _lib.check(rc)
         return self
 
     # --- utils/util.py:129-131
