@@ -228,6 +228,7 @@ typedef struct {
   const float *ln_w; /* [172]        */
   const float *ln_b; /* [172]        */
   const float *Mq_tc, *G_tc, *W2t_tc;
+  const float *Mq_img, *G_img, *W2_img;   /* operands of the batch entry points' kernels (rows as images) */
 } orca_attn_weights_t;
 
 /* Step 1 of TemporalAttentionLayer.forward (model/temporal_attention.py:41-48, the query side of
@@ -326,6 +327,7 @@ typedef struct {
   const float *Wg;
   const float *bg;     /* padded to 704 entries */
   const float *Wg_tc;
+  const float *Wg_chain; /* images of 32 gate columns for the memory chain of orca_tgn_eval_group */
 } orca_gru_weights_t;
 
 /* Replaces SequenceMemoryUpdater.update_memory / update_memory_in_test with nn.GRUCell
@@ -538,6 +540,32 @@ typedef struct {
 int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_cap, void *d_workspace,
                         int64_t workspace_bytes, void *d_stage, int64_t stage_bytes, float *d_prob, float *h_prob,
                         int32_t *d_status, void *stream);
+
+/* ------------------------------------------------------------------------------------------
+ * A group of consecutive batches of a stream as one unit of work (one GPU, tensor-core projections; with the
+ * budgeted recursion every batch needs a plan).  Results and state tables are those of the batches one by one, bit
+ * for bit.  Enqueues the copies of the group's inputs (pinned host memory, laid out as in orca_epoch_t), its kernels
+ * and the copy of its scores ([pos | neg] of batch after batch); nothing is synchronised, everything is complete in
+ * `stream` order.  A stream is given as group after group, `first` set for the first one of every uninterrupted run:
+ * nothing else may use the model's tables in between.  Groups of one run share bs, nb_max, u_cap, plan_cap and the
+ * workspace; only the last batch of the last group may be short (b_last < bs).
+ */
+#define ORCA_GROUP_MAX 32
+typedef struct {
+  const int32_t *h_i32;
+  const double *h_ts;         /* of the group's first edge */
+  const int64_t *off_i32;     /* nb offsets into h_i32, batch after batch without gaps */
+  const int32_t *n_plan;      /* nb plan lengths */
+  int32_t nb, bs, b_last;     /* batches of this group; edges of a batch and of the group's last one */
+  int32_t nb_max, u_cap, plan_cap; /* most batches of a group, most uncached neighbours and plan entries of a batch */
+  int32_t first;
+} orca_group_t;
+/* batches worth putting into one group */
+int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode);
+int64_t orca_group_workspace_bytes(int32_t bs, int32_t nb_max, int32_t k, int32_t u_cap, int32_t plan_cap,
+                                   int64_t n_nodes, int32_t n_layers, int32_t mode);
+int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_workspace, int64_t workspace_bytes,
+                        float *d_prob, float *h_prob, int32_t *d_status, void *stream);
 
 /* Average precision, ROC area and accuracy of every batch of a scored stream (evaluation/evaluation.py:30-44):
  * batch i covers edges [i * bs, (i + 1) * bs), h_out[3 * i .. 3 * i + 2] = {AP, AUC, share of edges with

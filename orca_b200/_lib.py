@@ -30,7 +30,7 @@ c_i32p = C.c_void_p
 
 class AttnWeights(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b",
-                                          "Mq_tc", "G_tc", "W2t_tc")]
+                                          "Mq_tc", "G_tc", "W2t_tc", "Mq_img", "G_img", "W2_img")]
 
 
 class ScoreWeights(C.Structure):
@@ -39,7 +39,7 @@ class ScoreWeights(C.Structure):
 
 
 class GruWeights(C.Structure):
-    _fields_ = [("Wg", C.c_void_p), ("bg", C.c_void_p), ("Wg_tc", C.c_void_p)]
+    _fields_ = [("Wg", C.c_void_p), ("bg", C.c_void_p), ("Wg_tc", C.c_void_p), ("Wg_chain", C.c_void_p)]
 
 
 class MemoryT(C.Structure):
@@ -78,6 +78,11 @@ class TgnT(C.Structure):
 class EpochT(C.Structure):
     _fields_ = [("h_i32", C.c_void_p), ("h_ts", C.c_void_p), ("off_i32", C.c_void_p), ("off_ts", C.c_void_p),
                 ("off_prob", C.c_void_p), ("b", C.c_void_p), ("n_plan", C.c_void_p), ("n_batches", C.c_int64)]
+
+
+class GroupT(C.Structure):
+    _fields_ = [("h_i32", C.c_void_p), ("h_ts", C.c_void_p), ("off_i32", C.c_void_p), ("n_plan", C.c_void_p)] + \
+        [(n, C.c_int32) for n in ("nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap", "first")]
 
 
 # every symbol the header declares: name -> (restype, argtypes)
@@ -128,6 +133,9 @@ SYMBOLS = {
     "orca_tgn_eval_batch_sharded": (C.c_int, [C.POINTER(TgnT), _I32, _V, _V, _I32, _V, _I32, _I32, _V, _I64, _V, _V,
                                               _V, _V, _V, _V]),
     "orca_tgn_eval_epoch": (C.c_int, [C.POINTER(TgnT), C.POINTER(EpochT), _I32, _V, _I64, _V, _I64, _V, _V, _V, _V]),
+    "orca_group_size": (_I32, [_I32, _I32, _I32, _I32]),
+    "orca_group_workspace_bytes": (_I64, [_I32, _I32, _I32, _I32, _I32, _I64, _I32, _I32]),
+    "orca_tgn_eval_group": (C.c_int, [C.POINTER(TgnT), C.POINTER(GroupT), _V, _I64, _V, _V, _V, _V]),
     "orca_link_metrics": (C.c_int, [_V, _V, _I64, _I32, _V]),
     "orca_stage_h2d": (C.c_int, [_V, _V, C.c_int64, _V]),
     "orca_ipc_export": (C.c_int, [_V, _V, C.POINTER(C.c_int64)]),
@@ -180,7 +188,8 @@ def ptr(t):
     raise TypeError(type(t))
 
 
-ATTN_FIELDS = ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b", "Mq_tc", "G_tc", "W2t_tc")
+ATTN_FIELDS = ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b", "Mq_tc", "G_tc", "W2t_tc", "Mq_img",
+               "G_img", "W2_img")
 
 
 def attn_struct(w):

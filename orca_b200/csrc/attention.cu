@@ -4,59 +4,43 @@
 // and V projections are folded into the query (qt) and into the output GEMM, so the memory side of
 // this kernel is pure HBM traffic:
 //   in : qt row (2 x 2064 B) + valid slots x (688 + 688) B of gathered rows + K * 12 B of indices
-//   out: ctx row (4128 B) + 1 flag
+//   out: ctx row (4128 B, fp32 or as bf16 head / tail operand image) + 1 flag
 #include <algorithm>
 #include <vector>
 
 #include "common.cuh"
+#include "attn_out.cuh"
 #include "context.cuh"
+#include "index_ops.cuh"
+#include "tc_ptx.cuh"
 
 namespace orca {
 
-#ifndef ORCA_GA_THREADS
-#define ORCA_GA_THREADS 256
-#endif
-constexpr int GA_THREADS = ORCA_GA_THREADS;
-constexpr int GA_SMEM_LIMIT = 226 * 1024;   // dynamic shared memory one block may ask for
-constexpr int GA_WARPS = GA_THREADS / 32;
-
-// One warp per query row, two passes over its valid neighbour slots:
-//   pass 1  every lane owns a fixed set of key columns -- 16-byte pieces l, l+32, l+64 of the
-//           gathered [neighbour | edge feature] part, loaded straight from the tables into registers
-//           with 128-bit loads (the next slot's pieces are requested before the current slot is
-//           processed), and column PAIRS l, l+32, l+64 of the time-encoding part, which is computed
-//           (cos of delta * w) two columns at a time with the packed two-wide fp32 instructions of this
-//           architecture (fma.rn.f32x2: half the issue slots for the range reduction, the dot products
-//           and the weighted sums) and parked in shared memory.  The lane's partial dot products with
-//           the two query heads are parked too; no cross-lane work happens inside the slot loop.
-//   softmax the 2 * slots partial-sum rows are reduced by 2 * slots lanes at once, the two heads'
-//           softmax runs across lanes;
-//   pass 2  the gathered pieces are loaded again (they sit in L1/L2 now), the time encodings come back
-//           from shared memory, and the weighted key sum is accumulated in registers.
-// Keeping the reductions and the exponentials out of the slot loops matters: with one row per warp
-// the kernel is bound by the length of each warp's dependent instruction chain, not by bandwidth (a
-// single pass with a running softmax needs a warp-wide reduction per slot and measured 15 % slower).
-// (The 688-byte rows are not moved by cp.async.bulk: an SM retires only about one small bulk copy
-// per ~130 cycles, which capped an earlier version at 1.5 TB/s whatever else it did.)
+// One warp per query row.  A row's slots are taken two at a time: their pieces are loaded into registers -- every lane
+// owns 16-byte pieces l, l + 32, l + 64 of the gathered [neighbour | edge feature] part and column PAIRS l, l + 32,
+// l + 64 of the time-encoding part, which is computed (cos of delta * w) two columns at a time with the packed
+// two-wide fp32 instructions of this architecture while the loads are in flight -- then come the partial dot products
+// with the two query heads, one cross-lane sum of all four logits at once, a running softmax and the weighted sums, all
+// from the same registers.
+// What bounds it (51 k rows of ten slots, 163 us): the instructions of a row (1500 a warp, 600 of them the time
+// encodings) against 16 resident warps per SM; issue slots 45 % busy, DRAM 30 %, L2 20 %.  Measured against it: two
+// passes over the rows with parked logits and time encodings (the form before) 178 us; four slots a step at 12 warps
+// 186; slots copied ahead with cp.async, two or four at a time, 167 to 201; the long cosine inlined with a variant of
+// the loop per range, 360 (instruction cache).  The 688-byte rows are not moved by cp.async.bulk: an SM retires only
+// about one small bulk copy per ~130 cycles.
 //
-// Work distribution.  Rows differ tenfold in cost (0 to k valid slots, 1 to 14 us) and a launch holds
-// only two to three rows per resident warp, so WHO gets WHICH row decides the length of the launch:
+// Work distribution.  Rows differ tenfold in cost (0 to k valid slots) and a launch of a single batch holds only two
+// to three rows per resident warp, so WHO gets WHICH row decides the length of the launch:
 //   - rows are handed out by ticket (one atomic per row on a counter the launch leaves at zero again);
-//   - a warp draws its next ticket only when it enters pass 2 of the current row: drawing it a whole
-//     row ahead commits slow warps to one more row while fast warps run dry (measured: 38 -> 33 us);
 //   - tickets walk the rows in the order of `order` (rows sorted by falling number of valid slots,
 //     made by row_order_kernel beside the sampling), so that the launch ends on its lightest rows.
-// The slot indices of the next row are loaded during pass 2; its projected query (4.2 KB) is read straight
-// from global memory when the row starts (staging it in shared memory with cp.async during pass 2 was
-// measured 6 % slower: the 4.2 KB per warp are better left free).
-// No block-level synchronisation; a block is eight independent warps.
+// A warp draws its next ticket when it starts a row and reads it after the row's first slots; the indices of the next
+// row are loaded while the rest of the row is worked on.  No block-level synchronisation, no shared memory.
+constexpr int GA_THREADS = 64, GA_BLOCKS = 8;    // 16 warps per SM at 128 registers
+constexpr int GS = 2;                           // slots per step
 constexpr int GA_MEM_F4 = 2 * D / 4;            // 86 sixteen-byte pieces of [neighbour | edge feature]
 constexpr int GA_ROW_F4 = D / 4;                // 43 pieces per table row
 constexpr int GA_P_ITERS = 3;                   // pieces / time-column pairs per lane (the third for lanes 0..21)
-constexpr int GA_TE_LD = 172;                   // floats per parked time encoding
-constexpr int GA_PART_LD = 33;                  // 32 partial sums + 1 pad (conflict-free column reads)
-// (a multiple of four floats: every warp's area starts on a 16-byte boundary)
-__host__ __device__ constexpr int ga_warp_floats(int k) { return (k * GA_TE_LD + 2 * k * GA_PART_LD + 3) & ~3; }
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
@@ -76,15 +60,20 @@ __device__ __forceinline__ float2 cos_small2(float2 x) {
   return make_float2(__cosf(r.x), __cosf(r.y));
 }
 
-// Time encodings of one slot for this lane's column pairs: the first NL pair groups (64 columns each) hold
-// large arguments (fixed-point reduction), the others small ones (packed fp32 reduction).  w decreases with
-// the column, so "large" groups are always a prefix; NL is uniform over the warp and the body is branch free.
-template <int NL>
-__device__ __forceinline__ void time_terms(float dt, const float2 (&wt)[GA_P_ITERS], float2 (&te)[GA_P_ITERS]) {
+// Arguments beyond the fixed-point range (or not finite) are rare: their cosine is a call, so that its long code does
+// not stand in the loops six times over (the kernel has to stay within the instruction cache).
+__device__ __noinline__ float cos_far(float x) { return cos_any(x); }
+
+// Time encodings of one slot for this lane's column pairs: the first nl pair groups (64 columns each) hold large
+// arguments (fixed-point reduction), the others small ones (packed fp32 reduction); nl < 0: beyond both.  w decreases
+// with the column, so "large" groups are always a prefix; nl is uniform over the warp.
+__device__ __forceinline__ void time_terms(float dt, int nl, const float2 (&wt)[GA_P_ITERS], float2 (&te)[GA_P_ITERS]) {
 #pragma unroll
   for (int i = 0; i < GA_P_ITERS; ++i) {
     const float2 x = mul2(dup2(dt), wt[i]);
-    te[i] = i < NL ? make_float2(cos_fixed(x.x), cos_fixed(x.y)) : cos_small2(x);
+    if (nl < 0) te[i] = make_float2(cos_far(x.x), cos_far(x.y));
+    else if (i < nl) te[i] = make_float2(cos_fixed(x.x), cos_fixed(x.y));
+    else te[i] = cos_small2(x);
   }
 }
 
@@ -124,21 +113,56 @@ row_order_kernel(const int32_t *__restrict__ nbr_a, int n_cap_a, const int32_t *
   for (int r = tid; r < n; r += 1024) order[atomicAdd(&s_bin[count(r)], 1)] = r;
 }
 
-__global__ void __launch_bounds__(GA_THREADS, 2)
+// Loads one slot's pieces of this lane: piece l of the neighbour row; piece l + 32 of the concatenation (neighbour row
+// for l < 11, else edge row piece l - 11); piece l + 64 (edge row piece l + 21, l < 22; the other lanes re-read piece 0
+// of the edge row, which is never used).
+struct SlotRows {
+  const float4 *n0, *n1;
+  int at1, at2, split;
+  bool from_edge;
+  const float4 *e_tab;
+  __device__ __forceinline__ void load(int nb, int ei, int lane, float4 (&x)[3]) const {
+    const float4 *nrow = (nb >= split ? n1 : n0) + (size_t)nb * GA_ROW_F4;
+    const float4 *erow = e_tab + (size_t)ei * GA_ROW_F4;
+    x[0] = __ldg(nrow + lane);
+    x[1] = __ldg((from_edge ? erow : nrow) + at1);
+    x[2] = __ldg(erow + at2);
+  }
+};
+
+// Sums V values (V a power of two up to 32) over the warp: lane l returns the total of value l / (32 / V).
+template <int V>
+__device__ __forceinline__ float warp_sum_many(float (&v)[V], int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  int o = 16;
+#pragma unroll
+  for (int n = V / 2; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {   // a lane keeps the half of the values that its bit names and hands over the other
+      const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(FULL, give, o);
+    }
+  }
+  float s = v[0];
+  for (; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+  return s;
+}
+
+template <bool IMAGE>
+__global__ void __launch_bounds__(GA_THREADS, GA_BLOCKS)
 attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_table,
+                   const float *__restrict__ nbr_table2, int nbr_split,
                    const float *__restrict__ edge_table, const float *__restrict__ time_w,
                    const int32_t *__restrict__ nbr, const int32_t *__restrict__ eid,
                    const float *__restrict__ delta, int k, int n_cap, const int32_t *__restrict__ d_n,
-                   const int32_t *__restrict__ order, float *__restrict__ ctx, uint8_t *__restrict__ valid_out,
+                   const int32_t *__restrict__ order, void *__restrict__ ctx, uint8_t *__restrict__ valid_out,
                    int32_t *__restrict__ ticket, unsigned long long *__restrict__ prof) {
-  extern __shared__ __align__(128) float smem[];
   constexpr unsigned FULL = 0xffffffffu;
   dep_trigger();
   dep_wait();
   const int n = rows_of(n_cap, d_n);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float *s_te = smem + warp * ga_warp_floats(k);  // [k][172]
-  float *s_part = s_te + k * GA_TE_LD;            // [2k][33]
+  const int lane = threadIdx.x & 31;
   const bool third = lane + 64 < GA_MEM_F4;       // lanes 0..21 own a third piece / pair
   // this lane's time-encoding frequencies, as column pairs, and the largest frequency of each pair group
   float2 wt[GA_P_ITERS];
@@ -147,6 +171,13 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     wt[i] = (i < 2 || third) ? __ldg(reinterpret_cast<const float2 *>(time_w) + lane + 32 * i) : make_float2(0.f, 0.f);
   const float wg0 = __ldg(time_w), wg1 = __ldg(time_w + 64), wg2 = __ldg(time_w + 128);
   unsigned long long prof_rows = 0, prof_slots = 0;
+  SlotRows rows;
+  rows.n0 = reinterpret_cast<const float4 *>(nbr_table), rows.n1 = reinterpret_cast<const float4 *>(nbr_table2);
+  rows.e_tab = reinterpret_cast<const float4 *>(edge_table);
+  rows.from_edge = lane >= GA_ROW_F4 - 32;
+  rows.at1 = rows.from_edge ? lane - (GA_ROW_F4 - 32) : lane + 32;
+  rows.at2 = third ? lane + 64 - GA_ROW_F4 : 0;
+  rows.split = nbr_split;
 
   auto row_of_ticket = [&](int t) -> int { return order != nullptr ? order[t] : t; };
   auto load_indices = [&](int r, int &o_nbr, int &o_eid, float &o_dt) {
@@ -166,41 +197,28 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   float my_dt = 0.f;
   if (row >= 0) load_indices(row, my_nbr, my_eid, my_dt);
   while (row >= 0) {
+    // the next ticket is drawn now and its row's indices are requested after the first slots (see above)
+    if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
     int next = -1, nx_nbr = 0, nx_eid = 0;
     float nx_dt = 0.f;
-    const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
-    if (vmask == 0) {
-      // every slot is padding: the layer ignores the attention term for this row
-      if (lane == 0) valid_out[row] = 0;
-      if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
-      tkt = __shfl_sync(FULL, tkt, 0);
-      if (tkt < n) {
-        next = row_of_ticket(tkt);
+    bool drawn = false;
+    auto draw_next = [&]() {
+      const int t = __shfl_sync(FULL, tkt, 0);
+      if (t < n) {
+        next = row_of_ticket(t);
         load_indices(next, nx_nbr, nx_eid, nx_dt);
       }
-    } else {
-      const int n_valid = __popc(vmask);
-      // this lane's pieces of a slot: piece l of the neighbour row; piece l+32 of the concatenation
-      // (neighbour row for l < 11, else edge row piece l-11); piece l+64 (edge row piece l+21, l < 22).
-      // Addresses are selected, loads are unconditional (lanes without a third piece re-read piece 0
-      // of the edge row; their third accumulator is never written out).
-      auto load_slot = [&](int j, float4(&x)[3]) {
-        const int nb = __shfl_sync(FULL, my_nbr, j), ei = __shfl_sync(FULL, my_eid, j);
-        const float4 *nrow = reinterpret_cast<const float4 *>(nbr_table + (size_t)nb * D);
-        const float4 *erow = reinterpret_cast<const float4 *>(edge_table + (size_t)ei * D);
-        const float4 *p1 = lane < GA_ROW_F4 - 32 ? nrow + lane + 32 : erow + lane - (GA_ROW_F4 - 32);
-        const float4 *p2 = third ? erow + lane + 64 - GA_ROW_F4 : erow;
-        x[0] = __ldg(nrow + lane);
-        x[1] = __ldg(p1);
-        x[2] = __ldg(p2);
-      };
-      // two slot buffers used alternately (no register copies): while one slot is processed the next one
-      // is in flight
-      float4 xa[3], xb[3];
-      unsigned todo = vmask;
-      int j0 = __ffs(todo) - 1;
-      todo &= todo - 1;
-      load_slot(j0, xa);
+    };
+    const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
+    const int n_valid = __popc(vmask);
+    float4 am0[3], am1[3];                         // weighted sums of the gathered part, heads 0 / 1
+    float2 at0[GA_P_ITERS], at1[GA_P_ITERS];       // and of the time part
+#pragma unroll
+    for (int i = 0; i < 3; ++i) am0[i] = am1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
+    float inv0 = 0.f, inv1 = 0.f;
+    if (n_valid > 0) {
       // which pair groups of this lane's slot need the fixed-point cosine (see time_terms)
       int my_nl;
       {
@@ -208,173 +226,139 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         my_nl = (adt * wg0 >= 32768.f ? 1 : 0) + (adt * wg1 >= 32768.f ? 1 : 0) + (adt * wg2 >= 32768.f ? 1 : 0);
         if (!(adt * wg0 < 1073741824.f)) my_nl = -1;   // beyond the fixed-point range (or not finite)
       }
-      // the lane's pieces of the two query heads
-      float4 qa[3], qb[3];
-      float2 qta[GA_P_ITERS], qtb[GA_P_ITERS];
       const float *q_src = qt + (size_t)row * QT_LD;
+      float m = -INFINITY, sum = 0.f;     // running maximum / sum of this lane's head
+      unsigned todo = vmask;
+      // GS slots at a time, each row of them in registers from its dot products to its weighted sum: nothing is
+      // loaded twice, and the cross-lane sums of 2 * GS logits cost little more than those of one
+      constexpr int V = 2 * GS, LPV = 32 / V;
+      for (int left = n_valid; left > 0; left -= GS) {
+        float4 x[GS][3];
+        float2 te[GS][GA_P_ITERS];
+        int js[GS];
 #pragma unroll
-      for (int i = 0; i < GA_P_ITERS; ++i) {
-        const int f = (i < 2 || third) ? lane + 32 * i : 0;
-        qa[i] = __ldg(reinterpret_cast<const float4 *>(q_src) + f);
-        qb[i] = __ldg(reinterpret_cast<const float4 *>(q_src + QT_HEAD) + f);
-        qta[i] = __ldg(reinterpret_cast<const float2 *>(q_src + 2 * D) + f);
-        qtb[i] = __ldg(reinterpret_cast<const float2 *>(q_src + QT_HEAD + 2 * D) + f);
-      }
-
-      // ---- pass 1: time encodings and partial logits, slot by slot
-      auto pass1_slot = [&](int it, int j, const float4(&x)[3]) {
-        const float dt = __shfl_sync(FULL, my_dt, j);
-        const int nl = __shfl_sync(FULL, my_nl, j);
-        float2 te[GA_P_ITERS];
-        switch (nl) {
-          case 0: time_terms<0>(dt, wt, te); break;
-          case 1: time_terms<1>(dt, wt, te); break;
-          case 2: time_terms<2>(dt, wt, te); break;
-          case 3: time_terms<3>(dt, wt, te); break;
-          default:
-#pragma unroll
-            for (int i = 0; i < GA_P_ITERS; ++i) te[i] = make_float2(cos_any(dt * wt[i].x), cos_any(dt * wt[i].y));
+        for (int s = 0; s < GS; ++s) {
+          const int j = todo ? __ffs(todo) - 1 : -1;
+          js[s] = j;
+          todo &= todo - 1;
+          const int jj = j >= 0 ? j : js[0];      // (an empty place repeats the first slot with weight zero)
+          rows.load(__shfl_sync(FULL, my_nbr, jj), __shfl_sync(FULL, my_eid, jj), lane, x[s]);
         }
-        float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);   // head 0 / head 1, two partial sums each
+#pragma unroll
+        for (int s = 0; s < GS; ++s) {
+          const int jj = js[s] >= 0 ? js[s] : js[0];
+          const float dt = __shfl_sync(FULL, my_dt, jj);
+          const int nl = __shfl_sync(FULL, my_nl, jj);
+          time_terms(dt, nl, wt, te[s]);
+        }
+        // partial logits: value 2 * s + head
+        float2 a0[GS], a1[GS];
+#pragma unroll
+        for (int s = 0; s < GS; ++s) a0[s] = a1[s] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < GA_P_ITERS; ++i) {
           if (i < 2 || third) {
-            reinterpret_cast<float2 *>(s_te + it * GA_TE_LD)[lane + 32 * i] = te[i];
-            a0 = fma2(te[i], qta[i], a0);
-            a1 = fma2(te[i], qtb[i], a1);
-            a0 = fma2(lo2(x[i]), lo2(qa[i]), a0);
-            a0 = fma2(hi2(x[i]), hi2(qa[i]), a0);
-            a1 = fma2(lo2(x[i]), lo2(qb[i]), a1);
-            a1 = fma2(hi2(x[i]), hi2(qb[i]), a1);
+            const float4 qa = __ldg(reinterpret_cast<const float4 *>(q_src) + lane + 32 * i);
+            const float4 qb = __ldg(reinterpret_cast<const float4 *>(q_src + QT_HEAD) + lane + 32 * i);
+            const float2 qta = __ldg(reinterpret_cast<const float2 *>(q_src + 2 * D) + lane + 32 * i);
+            const float2 qtb = __ldg(reinterpret_cast<const float2 *>(q_src + QT_HEAD + 2 * D) + lane + 32 * i);
+#pragma unroll
+            for (int s = 0; s < GS; ++s) {
+              a0[s] = fma2(te[s][i], qta, a0[s]);
+              a1[s] = fma2(te[s][i], qtb, a1[s]);
+              a0[s] = fma2(lo2(x[s][i]), lo2(qa), a0[s]);
+              a0[s] = fma2(hi2(x[s][i]), hi2(qa), a0[s]);
+              a1[s] = fma2(lo2(x[s][i]), lo2(qb), a1[s]);
+              a1[s] = fma2(hi2(x[s][i]), hi2(qb), a1[s]);
+            }
           }
         }
-        s_part[(2 * it) * GA_PART_LD + lane] = a0.x + a0.y;
-        s_part[(2 * it + 1) * GA_PART_LD + lane] = a1.x + a1.y;
-      };
-      for (int it = 0; it < n_valid; it += 2) {
-        int j1 = -1;
-        if (todo) {
-          j1 = __ffs(todo) - 1;
-          todo &= todo - 1;
-          load_slot(j1, xb);
-        }
-        pass1_slot(it, j0, xa);
-        if (j1 < 0) break;
-        if (todo) {
-          j0 = __ffs(todo) - 1;
-          todo &= todo - 1;
-          load_slot(j0, xa);
-        }
-        pass1_slot(it + 1, j1, xb);
-      }
-      __syncwarp();
-      // the next ticket is drawn now, not a row ahead; pass 2's first slot goes out before the softmax
-      if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
-      todo = vmask;
-      load_slot(__ffs(todo) - 1, xa);
-      todo &= todo - 1;
-
-      // ---- softmax: lane p reduces partial row p = 2 * slot + head; heads live on even / odd lanes
-      // (k <= 16 keeps all 2k rows on the 32 lanes; for larger k a lane takes rows p and p + 32)
-      float prob_lo = 0.f, prob_hi = 0.f;
-      {
-        float lg_lo = -INFINITY, lg_hi = -INFINITY;
-        if (lane < 2 * n_valid) {
-          float a = 0.f, b = 0.f;
-#pragma unroll 8
-          for (int t = 0; t < 32; t += 2) {
-            a += s_part[lane * GA_PART_LD + t];
-            b += s_part[lane * GA_PART_LD + t + 1];
-          }
-          lg_lo = a + b;
-        }
-        if (lane + 32 < 2 * n_valid) {
-          float a = 0.f, b = 0.f;
-#pragma unroll 8
-          for (int t = 0; t < 32; t += 2) {
-            a += s_part[(lane + 32) * GA_PART_LD + t];
-            b += s_part[(lane + 32) * GA_PART_LD + t + 1];
-          }
-          lg_hi = a + b;
-        }
-        float m = fmaxf(lg_lo, lg_hi);               // lanes of equal parity hold the same head
+        float v[V];
 #pragma unroll
-        for (int o = 2; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-        const float e_lo = lane < 2 * n_valid ? expf(lg_lo - m) : 0.f;
-        const float e_hi = lane + 32 < 2 * n_valid ? expf(lg_hi - m) : 0.f;
-        float sum = e_lo + e_hi;
+        for (int s = 0; s < GS; ++s) v[2 * s] = a0[s].x + a0[s].y, v[2 * s + 1] = a1[s].x + a1[s].y;
+        // lane l holds value l / LPV = 2 * slot + head; head = one lane bit
+        float lg = warp_sum_many<V>(v, lane);
+        const int slot = lane / (2 * LPV);
 #pragma unroll
-        for (int o = 2; o < 32; o <<= 1) sum += __shfl_xor_sync(FULL, sum, o);
-        const float inv = 1.f / sum;
-        prob_lo = e_lo * inv;
-        prob_hi = e_hi * inv;
-      }
-      // the next row of this warp: its indices are requested now and land during pass 2
-      tkt = __shfl_sync(FULL, tkt, 0);
-      if (tkt < n) {
-        next = row_of_ticket(tkt);
-        load_indices(next, nx_nbr, nx_eid, nx_dt);
-      }
-
-      // ---- pass 2: weighted key sum
-      float4 am0[3], am1[3];                         // gathered part, heads 0 / 1
-      float2 at0[GA_P_ITERS], at1[GA_P_ITERS];       // time part
+        for (int s = 1; s < GS; ++s)
+          if (slot == s && js[s] < 0) lg = -INFINITY;
+        float top = lg;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) am0[i] = am1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int o = 2 * LPV; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
+        const float m_new = fmaxf(m, top);
+        const float scale = expf(m - m_new);       // (0 the first time)
+        const float p = expf(lg - m_new);
+        float ps = p;
 #pragma unroll
-      for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
-      auto pass2_slot = [&](int it, const float4(&x)[3]) {
-        const int p = 2 * it;
-        const float p0 = p < 32 ? __shfl_sync(FULL, prob_lo, p) : __shfl_sync(FULL, prob_hi, p - 32);
-        const float p1 = p < 32 ? __shfl_sync(FULL, prob_lo, p + 1) : __shfl_sync(FULL, prob_hi, p - 31);
-        const float2 P0 = dup2(p0), P1 = dup2(p1);
+        for (int o = 2 * LPV; o < 32; o <<= 1) ps += __shfl_xor_sync(FULL, ps, o);
+        sum = sum * scale + ps;
+        m = m_new;
+        const float2 S0 = dup2(__shfl_sync(FULL, scale, 0)), S1 = dup2(__shfl_sync(FULL, scale, LPV));
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           float2 r;
-          r = fma2(P0, lo2(x[i]), lo2(am0[i])); am0[i].x = r.x; am0[i].y = r.y;
-          r = fma2(P0, hi2(x[i]), hi2(am0[i])); am0[i].z = r.x; am0[i].w = r.y;
-          r = fma2(P1, lo2(x[i]), lo2(am1[i])); am1[i].x = r.x; am1[i].y = r.y;
-          r = fma2(P1, hi2(x[i]), hi2(am1[i])); am1[i].z = r.x; am1[i].w = r.y;
+          r = mul2(S0, lo2(am0[i])); am0[i].x = r.x; am0[i].y = r.y;
+          r = mul2(S0, hi2(am0[i])); am0[i].z = r.x; am0[i].w = r.y;
+          r = mul2(S1, lo2(am1[i])); am1[i].x = r.x; am1[i].y = r.y;
+          r = mul2(S1, hi2(am1[i])); am1[i].z = r.x; am1[i].w = r.y;
+          at0[i] = mul2(S0, at0[i]);
+          at1[i] = mul2(S1, at1[i]);
         }
 #pragma unroll
-        for (int i = 0; i < GA_P_ITERS; ++i) {
-          if (i < 2 || third) {
-            const float2 te = reinterpret_cast<const float2 *>(s_te + it * GA_TE_LD)[lane + 32 * i];
-            at0[i] = fma2(P0, te, at0[i]);
-            at1[i] = fma2(P1, te, at1[i]);
+        for (int s = 0; s < GS; ++s) {
+          const float2 P0 = dup2(__shfl_sync(FULL, p, 2 * s * LPV)), P1 = dup2(__shfl_sync(FULL, p, (2 * s + 1) * LPV));
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            float2 r;
+            r = fma2(P0, lo2(x[s][i]), lo2(am0[i])); am0[i].x = r.x; am0[i].y = r.y;
+            r = fma2(P0, hi2(x[s][i]), hi2(am0[i])); am0[i].z = r.x; am0[i].w = r.y;
+            r = fma2(P1, lo2(x[s][i]), lo2(am1[i])); am1[i].x = r.x; am1[i].y = r.y;
+            r = fma2(P1, hi2(x[s][i]), hi2(am1[i])); am1[i].z = r.x; am1[i].w = r.y;
+            at0[i] = fma2(P0, te[s][i], at0[i]);
+            at1[i] = fma2(P1, te[s][i], at1[i]);
           }
         }
-      };
-      for (int it = 0; it < n_valid; it += 2) {
-        const bool more = todo != 0;
-        if (more) {
-          load_slot(__ffs(todo) - 1, xb);
-          todo &= todo - 1;
-        }
-        pass2_slot(it, xa);
-        if (!more) break;
-        if (todo) {
-          load_slot(__ffs(todo) - 1, xa);
-          todo &= todo - 1;
-        }
-        pass2_slot(it + 1, xb);
-      }
-      // write the row: [head 0: gathered 344 | time 172][head 1: ...]
-      float *out = ctx + (size_t)row * QT;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        if (i < 2 || third) {
-          reinterpret_cast<float4 *>(out)[lane + 32 * i] = am0[i];
-          reinterpret_cast<float4 *>(out + KEY)[lane + 32 * i] = am1[i];
-          reinterpret_cast<float2 *>(out + 2 * D)[lane + 32 * i] = at0[i];
-          reinterpret_cast<float2 *>(out + KEY + 2 * D)[lane + 32 * i] = at1[i];
+        if (!drawn) {
+          // the next row of this warp: its indices land while this one is finished
+          drawn = true;
+          draw_next();
         }
       }
-      if (lane == 0) valid_out[row] = 1;
+      inv0 = 1.f / __shfl_sync(FULL, sum, 0), inv1 = 1.f / __shfl_sync(FULL, sum, LPV);
       prof_rows += 1;
       prof_slots += (unsigned long long)n_valid;
-      __syncwarp();   // the parked values of this row are dead before the next row overwrites them
     }
+    if (!drawn) draw_next();
+    // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
+    // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
+    if (IMAGE || n_valid > 0) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const int f = lane + 32 * i;
+        if (i < 2 || third) {
+          const float4 m0 = make_float4(am0[i].x * inv0, am0[i].y * inv0, am0[i].z * inv0, am0[i].w * inv0);
+          const float4 m1 = make_float4(am1[i].x * inv1, am1[i].y * inv1, am1[i].z * inv1, am1[i].w * inv1);
+          const float2 t0 = make_float2(at0[i].x * inv0, at0[i].y * inv0);
+          const float2 t1 = make_float2(at1[i].x * inv1, at1[i].y * inv1);
+          if (IMAGE) {
+            char *im = (char *)ctx;
+            img::put4<img::CTX_STAGES>(im, row, 4 * f, m0);
+            img::put4<img::CTX_STAGES>(im, row, KEY + 4 * f, m1);
+            img::put2<img::CTX_STAGES>(im, row, 2 * D + 2 * f, t0);
+            img::put2<img::CTX_STAGES>(im, row, KEY + 2 * D + 2 * f, t1);
+          } else {
+            float *out = (float *)ctx + (size_t)row * QT;
+            reinterpret_cast<float4 *>(out)[f] = m0;
+            reinterpret_cast<float4 *>(out + KEY)[f] = m1;
+            reinterpret_cast<float2 *>(out + 2 * D)[f] = t0;
+            reinterpret_cast<float2 *>(out + KEY + 2 * D)[f] = t1;
+          }
+        }
+      }
+    }
+    if (IMAGE && lane < (img::CTX_STAGES * img::STAGE_K - QT) / 4)    // padding
+      img::put4<img::CTX_STAGES>((char *)ctx, row, QT + 4 * lane, make_float4(0.f, 0.f, 0.f, 0.f));
+    if (lane == 0) valid_out[row] = n_valid > 0 ? 1 : 0;
     row = next;
     my_nbr = nx_nbr;
     my_eid = nx_eid;
@@ -394,12 +378,16 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   }
 }
 
+// d_nbr_table2 (optional): neighbour rows >= nbr_split are read from it; its address is already moved back by
+// nbr_split rows
 // `ticket`: two zeroed device words that the launch leaves at zero; launches that may overlap on the GPU
 // need words of their own
 int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float *d_edge_table,
                        const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid, const float *d_delta,
                        int k, int n_rows_cap, const int32_t *d_n_rows, int rows_hint, const int32_t *d_order,
-                       float *d_ctx, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream) {
+                       void *d_ctx, bool image, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream,
+                       const float *d_nbr_table2, int nbr_split) {
+  if (d_nbr_table2 == nullptr) nbr_split = 0x7fffffff;
   ORCA_CHECK_ARG(d_qt && d_nbr_table && d_edge_table && d_time_w && d_nbr && d_eid && d_delta && d_ctx &&
                  d_valid && d_ticket);
   ORCA_CHECK_ARG(k >= 1 && k <= ORCA_MAX_K && n_rows_cap >= 0);
@@ -408,16 +396,6 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
   if (n_rows_cap == 0) return ORCA_OK;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_attn_gather: no context for the current device");
-  // two blocks per SM share its shared memory (1 KB per block is the system's): as many warps per block as
-  // fit into half of it
-  const int warps = std::max(1, std::min(GA_WARPS, (GA_SMEM_LIMIT / 2 - 1024) / (ga_warp_floats(k) * (int)sizeof(float))));
-  const size_t smem = (size_t)warps * ga_warp_floats(k) * sizeof(float);
-  static thread_local int configured_device = -1;
-  if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(attn_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   GA_SMEM_LIMIT / 2));
-    configured_device = c->device;
-  }
   GatherProfile &pf = c->prof;
   if (pf.on) {
     if (pf.used + 2 > pf.ev.size()) {
@@ -431,16 +409,17 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
   }
   // one resident wave at most; fewer blocks when the caller expects fewer rows than the capacity
   const int rows = rows_hint > 0 ? std::min(rows_hint, n_rows_cap) : n_rows_cap;
-  const int grid = std::min(ceil_div(rows, warps), c->sm_count * 2);
+  const int grid = std::min(ceil_div(rows, GA_THREADS / 32), c->sm_count * GA_BLOCKS);
+  auto kernel = image ? attn_gather_kernel<true> : attn_gather_kernel<false>;
   // (the profiling events would sit between this kernel and its neighbours: plain launch then)
   if (pf.on)
-    attn_gather_kernel<<<grid, warps * 32, smem, stream>>>(d_qt, d_nbr_table, d_edge_table, d_time_w, d_nbr, d_eid,
-                                                           d_delta, k, n_rows_cap, d_n_rows, d_order, d_ctx, d_valid,
-                                                           d_ticket, pf.d_counters);
+    kernel<<<grid, GA_THREADS, 0, stream>>>(d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table, d_time_w, d_nbr, d_eid,
+                                            d_delta, k, n_rows_cap, d_n_rows, d_order, d_ctx, d_valid, d_ticket,
+                                            pf.d_counters);
   else
-    ORCA_CUDA(launch_dep(attn_gather_kernel, grid, warps * 32, smem, stream, d_qt, d_nbr_table, d_edge_table,
-                         d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_ctx, d_valid, d_ticket,
-                         (unsigned long long *)nullptr));
+    ORCA_CUDA(launch_dep(kernel, grid, GA_THREADS, 0, stream, d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table,
+                         d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_ctx, d_valid,
+                         d_ticket, (unsigned long long *)nullptr));
   if (pf.on) {
     ORCA_CUDA(cudaEventRecord(pf.ev[pf.used + 1], stream));
     pf.used += 2;
@@ -477,5 +456,5 @@ extern "C" int orca_attn_gather(const float *d_qt, const float *d_nbr_table, con
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_attn_gather: no context for the current device");
   return launch_attn_gather(d_qt, d_nbr_table, d_edge_table, d_time_w, d_nbr, d_eid, d_delta, k, n_rows_cap,
-                            d_n_rows, 0, nullptr, d_ctx, d_valid, c->d_words + CTX_TICKET_MAIN, (cudaStream_t)stream);
+                            d_n_rows, 0, nullptr, d_ctx, false, d_valid, c->d_words + CTX_TICKET_MAIN, (cudaStream_t)stream);
 }

@@ -1,0 +1,318 @@
+// Output side of an attention layer on the tensor cores:
+//   out[r] = LayerNorm(relu([ctx | feat] . G + b1 + valid * g) . W2t + b2), optional history push and peer delivery
+//
+// The rows come as an operand image (attn_out.cuh): bf16 heads and tails, split once by the kernels that computed them,
+// in the form the tensor core reads.  So the main loop is nothing but bulk copies and MMAs: one thread streams stages
+// of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three, one thread multiplies, eight warps do the
+// two epilogues -- of one row block while the stages of the next are already landing.  A block of 128 rows takes 39
+// stages of 6 MMAs (10.5 us of tensor time) and 1.5 MB from L2.  The general projection kernel, whose producer warps
+// load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; here
+// TODO.
+// Between the two products the hidden tile stays on the SM (bias + ReLU, split, A image of the second product), and
+// the second product's accumulators reuse the first one's columns.
+// Warp 0: copies.  Warp 1: tensor memory, MMA issue.  Warps 2-9: epilogues (thread = row, then warp = row).
+#include <algorithm>
+
+#include "attn_out.cuh"
+#include "context.cuh"
+#include "tc_ptx.cuh"
+
+namespace orca {
+namespace ao {
+
+constexpr int BM = img::ROWS, BN = 176;
+constexpr int STAGES = 3;
+constexpr int A_STAGE = img::STAGE_BYTES, W_LBO = BN * 16, W_STAGE = 2 * 4 * W_LBO, STAGE = A_STAGE + W_STAGE;
+constexpr int K_STAGES = img::CTX_STAGES + img::FEAT_STAGES;                     // 39
+constexpr int K2_CHUNKS = BN / 8, K2_STAGES = (K2_CHUNKS + 3) / 4;               // 22, 6
+constexpr int A2_LBO = BM * 16 + 16, A2_BYTES = K2_CHUNKS * A2_LBO;
+constexpr int TILE_LD = 180;                       // floats per row of the output tile (conflict-free 16-byte stores)
+constexpr int FRONT = 90 * 1024;                   // hidden image, then output tile
+static_assert(2 * A2_BYTES <= FRONT && BM * TILE_LD * 4 <= FRONT && STAGE % 1024 == 0, "");
+constexpr int SMEM = FRONT + STAGES * STAGE + 1024;
+constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
+constexpr int TMEM_COLS = 512, SMALL = 256;
+
+using img::desc_sw64;
+
+__global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __grid_constant__ OutArgs g) {
+  using namespace tc;
+  extern __shared__ unsigned char raw[];
+  __shared__ __align__(16) float s_b1[BN], s_g[BN], s_b2[BN], s_lw[BN], s_lb[BN];
+  __shared__ __align__(8) unsigned long long s_bar[2 * STAGES + 4];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u, ring = base + FRONT;
+  auto full = [&](int s) { return smem_addr(&s_bar[s]); };
+  auto empty = [&](int s) { return smem_addr(&s_bar[STAGES + s]); };
+  const uint32_t acc1 = smem_addr(&s_bar[2 * STAGES]), a2bar = smem_addr(&s_bar[2 * STAGES + 1]),
+                 acc2 = smem_addr(&s_bar[2 * STAGES + 2]), tfree = smem_addr(&s_bar[2 * STAGES + 3]);
+  dep_trigger();
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    mbar_init(acc1, 1);
+    mbar_init(a2bar, EPI_WARPS);
+    mbar_init(acc2, 1);
+    mbar_init(tfree, EPI_WARPS);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  for (int i = tid; i < BN; i += THREADS) {
+    const bool in = i < D;
+    s_b1[i] = in ? g.w.b1[i] : 0.f;
+    s_g[i] = in ? g.w.g[i] : 0.f;
+    s_b2[i] = in ? g.w.b2[i] : 0.f;
+    s_lw[i] = in ? g.w.ln_w[i] : 0.f;
+    s_lb[i] = in ? g.w.ln_b[i] : 0.f;
+  }
+  dep_wait();
+  const int M = rows_of(g.n_cap, g.d_n);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
+  bool alive = true;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ stages
+    if (lane == 0) {
+      const char *w1 = reinterpret_cast<const char *>(g.w.G_img), *w2 = reinterpret_cast<const char *>(g.w.W2_img);
+      int it = 0;
+      for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x) {
+        const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
+        const char *feat = g.feat + (size_t)blk * img::FEAT_STAGES * A_STAGE;
+        for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
+          const int s = it % STAGES;
+          const uint32_t at = ring + s * STAGE;
+          mbar_wait(empty(s), ((it / STAGES) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
+          if (st < K_STAGES) {
+            mbar_expect_tx(full(s), STAGE);
+            bulk_g2s(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
+                     A_STAGE, full(s));
+            bulk_g2s(at + A_STAGE, w1 + (size_t)st * W_STAGE, W_STAGE, full(s));
+          } else {
+            mbar_expect_tx(full(s), W_STAGE);
+            bulk_g2s(at + A_STAGE, w2 + (size_t)(st - K_STAGES) * W_STAGE, W_STAGE, full(s));
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issue
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    int it = 0, t = 0;
+    for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x, ++t) {
+      if (t > 0) mbar_wait(tfree, (t - 1) & 1, g.status, 710, alive, g.wait_limit);
+      tc_fence_after();
+      for (int st = 0; st < K_STAGES; ++st, ++it) {
+        const int s = it % STAGES;
+        const uint32_t a = ring + s * STAGE, w = a + A_STAGE;
+        const bool half = st == img::CTX_STAGES - 1 || st == K_STAGES - 1;     // (the second step is nothing but padding)
+        mbar_wait(full(s), (it / STAGES) & 1, g.status, 711, alive, g.wait_limit);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks) {
+            if (ks == 1 && half) break;
+            const uint64_t ah = desc_sw64(a + ks * 32), al = desc_sw64(a + A_STAGE / 2 + ks * 32);
+            const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
+            const uint32_t more = (st > 0 || ks > 0) ? 1u : 0u;
+            mma_bf16(tmem, ah, bh, idesc, more);
+            mma_bf16(tmem + SMALL, al, bh, idesc, more);
+            mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
+          }
+          mma_commit(empty(s));
+          if (st == K_STAGES - 1) mma_commit(acc1);
+        }
+        __syncwarp();
+      }
+      mbar_wait(a2bar, t & 1, g.status, 712, alive, g.wait_limit);
+      tc_fence_after();
+      for (int st = 0; st < K2_STAGES; ++st, ++it) {
+        const int s = it % STAGES;
+        const uint32_t w = ring + s * STAGE + A_STAGE, a = base + st * 4 * A2_LBO;
+        mbar_wait(full(s), (it / STAGES) & 1, g.status, 713, alive, g.wait_limit);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks) {
+            if (2 * st + ks >= K2_CHUNKS / 2) break;
+            const uint64_t ah = make_desc(a + ks * 2 * A2_LBO, A2_LBO, 128);
+            const uint64_t al = make_desc(a + A2_BYTES + ks * 2 * A2_LBO, A2_LBO, 128);
+            const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
+            const uint32_t more = (st > 0 || ks > 0) ? 1u : 0u;
+            mma_bf16(tmem, ah, bh, idesc, more);
+            mma_bf16(tmem + SMALL, al, bh, idesc, more);
+            mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
+          }
+          mma_commit(empty(s));
+          if (st == K2_STAGES - 1) mma_commit(acc2);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogues
+    const int ew = warp - 2, quarter = warp & 3, half = ew >> 2;
+    const int row = quarter * 32 + lane;
+    const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
+    const int ch0 = half ? 6 : 0, ch1 = half ? BN / 16 : 6;     // accumulator chunks of 16 columns of this warp
+    const bool has1 = lane + 32 < D / 4;
+    const float4 f4z = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto vec = [&](const float *s, int j, bool on) { return on ? *reinterpret_cast<const float4 *>(s + 4 * j) : f4z; };
+    int t = 0;
+    for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x, ++t) {
+      const int m0 = blk * BM, m_rows = min(BM, M - m0);
+      const float on = (row < m_rows && (g.valid == nullptr || g.valid[m0 + row] != 0)) ? 1.f : 0.f;
+      // history push: lane i holds what row ew + 8 * i of the output pass needs
+      int push_id = 0, push = 0;
+      if (g.push_table != nullptr && lane < BM / EPI_WARPS && ew + EPI_WARPS * lane < m_rows) {
+        const int m = m0 + ew + EPI_WARPS * lane;
+        push_id = g.push_ids[m];
+        push = g.push_win != nullptr ? g.push_win[m]
+               : (m >= g.push_all_from || g.push_last_pos[push_id] == (unsigned long long)(g.push_base + m)) ? 1 : 0;
+      }
+      // first: hidden = relu(acc + b1 + valid * g), split, A image of the second product
+      mbar_wait(acc1, t & 1, g.status, 720, alive, g.wait_limit);
+      tc_fence_after();
+      for (int ch = ch0; ch < ch1; ++ch) {
+        float v[16];
+        tmem_ld16_sum(trow + ch * 16, SMALL, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + s_b1[ch * 16 + i] + on * s_g[ch * 16 + i], 0.f);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint4 hi, lo;
+          split_chunk(make_float4(v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3]),
+                      make_float4(v[8 * h + 4], v[8 * h + 5], v[8 * h + 6], v[8 * h + 7]), hi, lo);
+          st_shared_v4(base + (uint32_t)(2 * ch + h) * A2_LBO + row * 16, hi);
+          st_shared_v4(base + A2_BYTES + (uint32_t)(2 * ch + h) * A2_LBO + row * 16, lo);
+        }
+      }
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a2bar);
+      // second: accumulators -> row-major tile (over the hidden image, which has been read), then whole rows
+      mbar_wait(acc2, t & 1, g.status, 721, alive, g.wait_limit);
+      tc_fence_after();
+      for (int ch = ch0; ch < ch1; ++ch) {
+        float v[16];
+        tmem_ld16_sum(trow + ch * 16, SMALL, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          st_shared_f4(base + (uint32_t)(row * TILE_LD + ch * 16 + q * 4) * 4u,
+                       make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tfree);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      constexpr int RB = 4;     // rows in flight per warp
+      for (int i0 = 0; i0 < BM / EPI_WARPS; i0 += RB) {
+        if (ew + EPI_WARPS * i0 >= m_rows) break;
+        float4 a[RB], b[RB];
+        float sum[RB], sq[RB];
+        const float4 bA = vec(s_b2, lane, true), bB = vec(s_b2, lane + 32, has1);
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const uint32_t ra = base + (uint32_t)((ew + EPI_WARPS * (i0 + k)) * TILE_LD + 4 * lane) * 4u;
+          const float4 x = ld_shared_f4(ra), y = has1 ? ld_shared_f4(ra + 512u) : f4z;
+          a[k] = make_float4(x.x + bA.x, x.y + bA.y, x.z + bA.z, x.w + bA.w);
+          b[k] = make_float4(y.x + bB.x, y.y + bB.y, y.z + bB.z, y.w + bB.w);
+          // both moments in one sweep (the row is O(1) after the merger, so E[y^2] - mean^2 loses nothing that matters
+          // at the 1e-5 epsilon)
+          sum[k] = (a[k].x + a[k].y) + (a[k].z + a[k].w) + (b[k].x + b[k].y) + (b[k].z + b[k].w);
+          sq[k] = a[k].x * a[k].x + a[k].y * a[k].y + a[k].z * a[k].z + a[k].w * a[k].w + b[k].x * b[k].x + b[k].y * b[k].y +
+                  b[k].z * b[k].z + b[k].w * b[k].w;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int k = 0; k < RB; ++k) {
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+            sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], o);
+          }
+        const float4 wA = vec(s_lw, lane, true), wB = vec(s_lw, lane + 32, has1);
+        const float4 lA = vec(s_lb, lane, true), lB = vec(s_lb, lane + 32, has1);
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const int r = ew + EPI_WARPS * (i0 + k);
+          const int to = __shfl_sync(0xffffffffu, push_id, i0 + k), win = __shfl_sync(0xffffffffu, push, i0 + k);
+          if (r >= m_rows) continue;
+          const float mean = sum[k] * (1.f / D);
+          const float inv = 1.f / sqrtf(fmaxf(sq[k] - sum[k] * mean, 0.f) * (1.f / D) + 1e-5f);
+          const float4 ya = make_float4((a[k].x - mean) * inv * wA.x + lA.x, (a[k].y - mean) * inv * wA.y + lA.y,
+                                        (a[k].z - mean) * inv * wA.z + lA.z, (a[k].w - mean) * inv * wA.w + lA.w);
+          const float4 yb = make_float4((b[k].x - mean) * inv * wB.x + lB.x, (b[k].y - mean) * inv * wB.y + lB.y,
+                                        (b[k].z - mean) * inv * wB.z + lB.z, (b[k].w - mean) * inv * wB.w + lB.w);
+          auto store = [&](float *o) {
+            *reinterpret_cast<float4 *>(o + 4 * lane) = ya;
+            if (has1) *reinterpret_cast<float4 *>(o + 4 * lane + 128) = yb;
+          };
+          store(g.out + (size_t)(m0 + r) * D);
+          if (g.push_table != nullptr && win != 0) store(g.push_table + (size_t)to * D);
+          if (m0 + r < g.out_image_rows) {     // (columns 172 .. 191 are padding)
+            img::put4<img::FEAT_STAGES>(g.out_image, m0 + r, 4 * lane, ya);
+            if (lane < 16) img::put4<img::FEAT_STAGES>(g.out_image, m0 + r, 128 + 4 * lane, has1 ? yb : f4z);
+          }
+          // multi-GPU exchange: the row also goes to every rank's exchange buffer (peer stores)
+          for (int q = 0; q < g.peer.world; ++q) store(g.peer.rows[q] + g.peer.off + (size_t)(m0 + r) * D);
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");     // the tile has been read: the next hidden image may land
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  }
+  if (g.peer.world > 0) {
+    // every CTA (with or without rows) checks out; the last one posts the batch's sequence number to all ranks, after
+    // every CTA's peer stores have been fenced system-wide
+    __threadfence_system();
+    __syncthreads();
+    if (tid == 0 && atomicAdd(g.peer.counter, 1) == (int)gridDim.x - 1) {
+      *g.peer.counter = 0;
+      __threadfence_system();
+      for (int q = 0; q < g.peer.world; ++q)
+        asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(g.peer.flags[q] + g.peer.rank), "r"(g.peer.seq)
+                     : "memory");
+    }
+  }
+}
+
+}  // namespace ao
+
+int attn_output_rows(const OutArgs &args, cudaStream_t s) {
+  if (args.n_cap <= 0) return ORCA_OK;
+  Ctx *c = cur();
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_output_rows: no context for the current device");
+  ORCA_CHECK_ARG(args.w.G_img && args.w.W2_img && args.ctx && args.feat && args.out);
+  static thread_local int configured_device = -1;
+  if (configured_device != c->device) {
+    ORCA_CUDA(cudaFuncSetAttribute(ao::attn_output_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ao::SMEM));
+    configured_device = c->device;
+  }
+  OutArgs g = args;
+  g.status = c->status_word;
+  g.wait_limit = c->wait_limit;
+  const int grid = std::min(ceil_div(g.n_cap, ao::BM), c->sm_count);
+  ORCA_CUDA(launch_dep(ao::attn_output_image_kernel, grid, ao::THREADS, ao::SMEM, s, g));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+}  // namespace orca

@@ -1,0 +1,430 @@
+// Query side of an attention layer on the tensor cores: qt[r] = feat[row of r] . Mq + cq, [rows, 1056] floats.
+//
+// A launch writes 4.2 KB per row and reads 0.7: at many rows it is bound by those writes.  A CTA keeps its weight
+// tile (heads and tails of 96 or 176 columns) for the whole launch and walks row blocks of 128.
+// attn_query_image_kernel takes the rows as an operand image (attn_out.cuh): one thread streams 16 KB stages through a
+// ring, one multiplies, eight warps carry the other accumulator buffer from tensor memory to qt, a thread per row and
+// 32 bytes a store (whole sectors, no staging).  51 k rows: 155 us for the general projection kernel (six column
+// tiles, weights streamed again for every row block, load, product and store one after the other), TODO us here.
+// attn_query_kernel takes the rows as floats and splits them itself, eleven times over (170 us): it serves the callers
+// that have no buffer for an image.
+#include <algorithm>
+
+#include "attn_out.cuh"
+#include "context.cuh"
+#include "tc_gemm.cuh"
+#include "tc_ptx.cuh"
+
+namespace orca {
+namespace aq {
+
+constexpr int BM = 128, BN = 96, TILES = QT_LD / BN;     // 11
+constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;           // K = 172, padded to 176
+constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
+constexpr int A_LBO = BM * 16 + 16, A_BYTES = CHUNKS * A_LBO;   // (+16: conflict-free 16-byte stores)
+constexpr int TILE_LD = BN + 4;                          // floats per row of the output tile: likewise
+constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + BM * TILE_LD * 4 + 1024;
+constexpr int PRODUCERS = 256, THREADS = PRODUCERS + 128 + 32;
+constexpr int TMEM_COLS = 512, BUF_COLS = 2 * BN;        // two buffers of main + cross-term accumulators
+
+struct Args {
+  tc::RowSrc feat;
+  int n_cap;
+  const int32_t *d_n;
+  const void *w;          // weights.pack_query
+  const float *bias;
+  float *qt;
+  int32_t *status;
+  long long wait_limit;
+};
+
+__global__ void __launch_bounds__(THREADS, 1) attn_query_kernel(const __grid_constant__ Args g) {
+  using namespace tc;
+  extern __shared__ unsigned char raw[];
+  __shared__ int s_row[2][BM];
+  __shared__ __align__(16) float s_bias[BN];
+  __shared__ __align__(8) unsigned long long s_bar[8];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int nt = blockIdx.x;
+  const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u;
+  const uint32_t w_hi = base, w_lo = base + W_BYTES, a_hi = base + 2 * W_BYTES, a_lo = a_hi + A_BYTES,
+                 tile = a_lo + A_BYTES;
+  const uint32_t wbar = smem_addr(&s_bar[0]), afull = smem_addr(&s_bar[1]), aempty = smem_addr(&s_bar[2]);
+  auto accfull = [&](int b) { return smem_addr(&s_bar[3 + b]); };
+  auto accfree = [&](int b) { return smem_addr(&s_bar[5 + b]); };
+  dep_trigger();
+  if (tid == 0) {
+    mbar_init(wbar, 1);
+    mbar_init(afull, PRODUCERS / 32);
+    mbar_init(aempty, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accfull(b), 1);
+      mbar_init(accfree(b), 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(wbar, 2 * W_BYTES);       // (weights: written by nobody but the host, long ago)
+    bulk_g2s(w_hi, reinterpret_cast<const char *>(g.w) + (size_t)nt * 2 * W_BYTES, 2 * W_BYTES, wbar);
+  }
+  if (warp == 12) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid < BN) s_bias[tid] = g.bias[nt * BN + tid];
+  dep_wait();
+  const int M = rows_of(g.n_cap, g.d_n);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
+  bool alive = true;
+
+  if (warp < 8) {
+    // ------------------------------------------------------------------ rows -> images
+    constexpr int PER = BM * CHUNKS / PRODUCERS;     // 11 chunks of 8 columns per thread and block
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x[PER][2];
+    auto find_rows = [&](int blk, int buf) {
+      if (tid < BM) {
+        const int m = blk * BM + tid;
+        s_row[buf][tid] = m < M ? (g.feat.idx ? g.feat.idx[m] : m + g.feat.add) : -1;
+      }
+    };
+    auto load = [&](int buf) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int u = tid + i * PRODUCERS, row = u / CHUNKS, c = u - row * CHUNKS;
+        const int r = s_row[buf][row];
+        x[i][0] = x[i][1] = zero;
+        if (r >= 0) {
+          const float4 *p = reinterpret_cast<const float4 *>(g.feat.base(r) + (size_t)r * D) + 2 * c;
+          x[i][0] = *p;
+          if (c < CHUNKS - 1) x[i][1] = p[1];
+        }
+      }
+    };
+    int blk = blockIdx.y, t = 0;
+    if (blk * BM < M) find_rows(blk, 0);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (blk * BM < M) load(0);
+    for (; blk * BM < M; blk += gridDim.y, ++t) {
+      const int next = blk + gridDim.y;
+      if (next * BM < M) find_rows(next, (t + 1) & 1);
+      if (t > 0) mbar_wait(aempty, (t - 1) & 1, g.status, 510, alive, g.wait_limit);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int u = tid + i * PRODUCERS, row = u / CHUNKS, c = u - row * CHUNKS;
+        uint4 hi, lo;
+        split_chunk(x[i][0], x[i][1], hi, lo);
+        st_shared_v4(a_hi + c * A_LBO + row * 16, hi);
+        st_shared_v4(a_lo + c * A_LBO + row * 16, lo);
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(afull);
+      asm volatile("bar.sync 1, 256;" ::: "memory");     // the next block's rows are known
+      if (next * BM < M) load((t + 1) & 1);
+    }
+  } else if (warp < 12) {
+    // ------------------------------------------------------------------ accumulators -> qt
+    const int quarter = warp & 3;
+    const uint32_t rows_at = tile + (uint32_t)(quarter * 32) * (TILE_LD * 4);
+    int t = 0;
+    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
+      const int b = t & 1;
+      mbar_wait(accfull(b), (t >> 1) & 1, g.status, 520, alive, g.wait_limit);
+      tc_fence_after();
+      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * BUF_COLS;
+#pragma unroll
+      for (int ch = 0; ch < BN / 16; ++ch) {
+        float v[16];
+        tmem_ld16_sum(acc + ch * 16, BN, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 bias = *reinterpret_cast<const float4 *>(&s_bias[ch * 16 + q * 4]);
+          st_shared_f4(rows_at + (uint32_t)(lane * TILE_LD + ch * 16 + q * 4) * 4u,
+                       make_float4(v[q * 4] + bias.x, v[q * 4 + 1] + bias.y, v[q * 4 + 2] + bias.z, v[q * 4 + 3] + bias.w));
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(accfree(b));
+      const int m0 = blk * BM + quarter * 32;
+#pragma unroll 8
+      for (int i = 0; i < BN / 4; ++i) {      // the warp's 32 rows, 24 pieces each
+        const int u = lane + 32 * i, r = u / (BN / 4), c = u - r * (BN / 4);
+        const float4 v = ld_shared_f4(rows_at + (uint32_t)(r * TILE_LD + c * 4) * 4u);
+        if (m0 + r < M) *reinterpret_cast<float4 *>(g.qt + (size_t)(m0 + r) * QT_LD + nt * BN + c * 4) = v;
+      }
+      __syncwarp();
+    }
+  } else {
+    // ------------------------------------------------------------------ MMA issue
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    mbar_wait(wbar, 0, g.status, 530, alive, g.wait_limit);
+    int t = 0;
+    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
+      const int b = t & 1;
+      const uint32_t d = tmem + b * BUF_COLS;
+      if (t >= 2) mbar_wait(accfree(b), ((t >> 1) & 1) ^ 1, g.status, 531, alive, g.wait_limit);
+      mbar_wait(afull, t & 1, g.status, 532, alive, g.wait_limit);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+      for (int ks = 0; ks < STEPS; ++ks) {
+        const uint64_t ah = make_desc(a_hi + ks * 2 * A_LBO, A_LBO, 128), al = make_desc(a_lo + ks * 2 * A_LBO, A_LBO, 128);
+        const uint64_t bh = make_desc(w_hi + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w_lo + ks * 2 * W_LBO, W_LBO, 128);
+        const uint32_t more = ks > 0 ? 1u : 0u;
+        mma_bf16(d, ah, bh, idesc, more);
+        mma_bf16(d + BN, al, bh, idesc, more);
+        mma_bf16(d + BN, ah, bl, idesc, 1u);
+      }
+      mma_commit(aempty);
+      mma_commit(accfull(b));
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 12) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+}  // namespace aq
+
+// ---------------------------------------------------------------------------------------------------------------------
+namespace aqi {
+
+using aq::BM;
+using aq::CHUNKS;
+using aq::STEPS;
+constexpr int BN = 176, TILES = QT_LD / BN;                   // 6
+constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
+constexpr int STAGES = 5, STAGE = img::STAGE_BYTES;
+constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
+constexpr int RING = (2 * W_BYTES + 1023) / 1024 * 1024;      // (the swizzle wants aligned stages)
+constexpr int SMEM = RING + STAGES * STAGE + 1024;
+constexpr int TMEM_COLS = 512, SMALL = 256;                   // one buffer of main + cross-term accumulators
+
+struct Args {
+  const char *image;
+  int n_cap;
+  const int32_t *d_n;
+  const void *w;
+  const float *bias;
+  float *qt;
+  int32_t *status;
+  long long wait_limit;
+};
+
+__device__ __forceinline__ void st_global_v8(float *p, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+__global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __grid_constant__ Args g) {
+  using namespace tc;
+  extern __shared__ unsigned char raw[];
+  __shared__ __align__(16) float s_bias[BN];
+  __shared__ __align__(8) unsigned long long s_bar[2 * STAGES + 3];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int nt = blockIdx.x;
+  const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u, ring = base + RING;
+  auto full = [&](int s) { return smem_addr(&s_bar[s]); };
+  auto empty = [&](int s) { return smem_addr(&s_bar[STAGES + s]); };
+  const uint32_t wbar = smem_addr(&s_bar[2 * STAGES]);
+  const uint32_t accfull = smem_addr(&s_bar[2 * STAGES + 1]), accfree = smem_addr(&s_bar[2 * STAGES + 2]);
+  dep_trigger();
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    mbar_init(wbar, 1);
+    mbar_init(accfull, 1);
+    mbar_init(accfree, EPI_WARPS);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(wbar, 2 * W_BYTES);       // (weights: written by nobody but the host, long ago)
+    bulk_g2s(base, reinterpret_cast<const char *>(g.w) + (size_t)nt * 2 * W_BYTES, 2 * W_BYTES, wbar);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid >= 64 && tid < 64 + BN) s_bias[tid - 64] = g.bias[nt * BN + tid - 64];
+  dep_wait();
+  const int M = rows_of(g.n_cap, g.d_n);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
+  bool alive = true;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y) {
+        const char *rows = g.image + (size_t)blk * img::FEAT_STAGES * STAGE;
+        for (int st = 0; st < img::FEAT_STAGES; ++st, ++it) {
+          const int s = it % STAGES;
+          mbar_wait(empty(s), ((it / STAGES) & 1) ^ 1, g.status, 540, alive, g.wait_limit);
+          mbar_expect_tx(full(s), STAGE);
+          bulk_g2s(ring + s * STAGE, rows + (size_t)st * STAGE, STAGE, full(s));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    mbar_wait(wbar, 0, g.status, 550, alive, g.wait_limit);
+    int it = 0, t = 0;
+    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
+      if (t > 0) mbar_wait(accfree, (t - 1) & 1, g.status, 551, alive, g.wait_limit);
+#pragma unroll
+      for (int st = 0; st < img::FEAT_STAGES; ++st, ++it) {
+        const int s = it % STAGES;
+        const uint32_t a = ring + s * STAGE;
+        mbar_wait(full(s), (it / STAGES) & 1, g.status, 552, alive, g.wait_limit);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks) {
+            if (2 * st + ks >= STEPS) continue;
+            const uint32_t w = base + (2 * st + ks) * 2 * W_LBO;
+            const uint64_t ah = img::desc_sw64(a + ks * 32), al = img::desc_sw64(a + STAGE / 2 + ks * 32);
+            const uint64_t bh = make_desc(w, W_LBO, 128), bl = make_desc(w + W_BYTES, W_LBO, 128);
+            const uint32_t more = st > 0 || ks > 0 ? 1u : 0u;
+            mma_bf16(tmem, ah, bh, idesc, more);
+            mma_bf16(tmem + SMALL, al, bh, idesc, more);
+            mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
+          }
+          mma_commit(empty(s));
+          if (st == img::FEAT_STAGES - 1) mma_commit(accfull);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // (six chunks of 16 columns for the first four warps, five for the others)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const int c0 = half * 6, nc = half ? 5 : 6;
+    int t = 0;
+    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
+      const int m = blk * BM + quarter * 32 + lane;
+      mbar_wait(accfull, t & 1, g.status, 560, alive, g.wait_limit);
+      tc_fence_after();
+      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + c0 * 16;
+      float *out = g.qt + (size_t)m * QT_LD + nt * BN + c0 * 16;
+      float v[6][16];
+#pragma unroll
+      for (int ch = 0; ch < 6; ++ch)
+        if (ch < nc) tmem_ld16_sum(acc + ch * 16, SMALL, v[ch]);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(accfree);      // (the next block's products may start before this one is stored)
+      if (m < M) {
+#pragma unroll
+        for (int ch = 0; ch < 6; ++ch)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (ch >= nc) continue;
+            float y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = v[ch][8 * q + i] + s_bias[(c0 + ch) * 16 + 8 * q + i];
+            st_global_v8(out + ch * 16 + 8 * q, y);
+          }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// rows -> operand image: a thread per 16-byte chunk (eight columns)
+__global__ void __launch_bounds__(256) feat_image_kernel(tc::RowSrc feat, int n_cap, const int32_t *d_n, char *image) {
+  dep_trigger();
+  dep_wait();
+  constexpr int CH = img::FEAT_STAGES * img::STAGE_K / 8;
+  const int n = rows_of(n_cap, d_n);
+  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < (long long)n * CH; u += (long long)gridDim.x * blockDim.x) {
+    const int m = (int)(u / CH), c = (int)(u - (long long)m * CH);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    if (c < CHUNKS) {
+      const int r = feat.idx ? feat.idx[m] : m + feat.add;
+      const float4 *p = reinterpret_cast<const float4 *>(feat.base(r) + (size_t)r * D) + 2 * c;
+      x = *p;
+      if (c < CHUNKS - 1) y = p[1];
+    }
+    uint4 hi, lo;
+    tc::split_chunk(x, y, hi, lo);
+    char *o = img::at<img::FEAT_STAGES>(image, m, 8 * c);
+    *reinterpret_cast<uint4 *>(o) = hi;
+    *reinterpret_cast<uint4 *>(o + img::STAGE_BYTES / 2) = lo;
+  }
+}
+
+}  // namespace aqi
+
+int feat_image(const tc::RowSrc &feat, int n_cap, const int32_t *d_n, char *d_image, cudaStream_t s) {
+  if (n_cap <= 0) return ORCA_OK;
+  Ctx *c = cur();
+  const int sms = c != nullptr ? c->sm_count : 148;
+  const long long units = (long long)n_cap * (img::FEAT_STAGES * 4);
+  const int grid = (int)std::min<long long>((units + 255) / 256, sms * 8);
+  ORCA_CUDA(launch_dep(aqi::feat_image_kernel, grid, 256, 0, s, feat, n_cap, d_n, d_image));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_cap, const int32_t *d_n, float *d_qt,
+                     cudaStream_t s) {
+  if (n_cap <= 0) return ORCA_OK;
+  Ctx *c = cur();
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_query_image: no context for the current device");
+  ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && ((uintptr_t)d_qt & 31) == 0);
+  static thread_local int configured_device = -1;
+  if (configured_device != c->device) {
+    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
+    configured_device = c->device;
+  }
+  const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, c->status_word, c->wait_limit};
+  const dim3 grid(aqi::TILES, std::min(ceil_div(n_cap, aqi::BM), std::max(1, c->sm_count / aqi::TILES)));
+  ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+int attn_query_rows(const orca_attn_weights_t *w, const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_qt,
+                    cudaStream_t s) {
+  if (n_cap <= 0) return ORCA_OK;
+  Ctx *c = cur();
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_query_rows: no context for the current device");
+  static thread_local int configured_device = -1;
+  if (configured_device != c->device) {
+    ORCA_CUDA(cudaFuncSetAttribute(aq::attn_query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aq::SMEM));
+    configured_device = c->device;
+  }
+  const aq::Args g{feat, n_cap, d_n, w->Mq_tc, w->cq, d_qt, c->status_word, c->wait_limit};
+  const dim3 grid(aq::TILES, std::min(ceil_div(n_cap, aq::BM), std::max(1, c->sm_count / aq::TILES)));
+  ORCA_CUDA(launch_dep(aq::attn_query_kernel, grid, aq::THREADS, aq::SMEM, s, g));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+}  // namespace orca

@@ -19,7 +19,8 @@ static int create_ctx(Ctx **out) {
   ORCA_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
   for (int q = 0; q < Ctx::kStageSlots; ++q) ORCA_CUDA(cudaEventCreateWithFlags(&c->ev_slot[q], cudaEventDisableTiming));
   cudaEvent_t *evs[] = {&c->fork, &c->join, &c->ev_in, &c->ev_flags, &c->ev_o1, &c->ev_g2, &c->ev_state,
-                        &c->ev_idx[0], &c->ev_idx[1], &c->ev_done[0], &c->ev_done[1]};
+                        &c->ev_idx[0], &c->ev_idx[1], &c->ev_done[0], &c->ev_done[1], &c->ev_gin, &c->ev_gidx[0],
+                        &c->ev_gidx[1], &c->ev_gchain[0], &c->ev_gchain[1], &c->ev_gdone[0], &c->ev_gdone[1]};
   for (cudaEvent_t *e : evs) ORCA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   ORCA_CUDA(cudaMalloc(&c->d_words, CTX_WORDS * sizeof(int32_t)));
   ORCA_CUDA(cudaMemset(c->d_words, 0, CTX_WORDS * sizeof(int32_t)));
@@ -39,7 +40,8 @@ static void destroy_ctx(Ctx *c) {
   for (cudaEvent_t e : c->ev_slot)
     if (e) cudaEventDestroy(e);
   cudaEvent_t evs[] = {c->fork, c->join, c->ev_in, c->ev_flags, c->ev_o1, c->ev_g2, c->ev_state, c->ev_idx[0],
-                       c->ev_idx[1], c->ev_done[0], c->ev_done[1]};
+                       c->ev_idx[1], c->ev_done[0], c->ev_done[1], c->ev_gin, c->ev_gidx[0], c->ev_gidx[1],
+                       c->ev_gchain[0], c->ev_gchain[1], c->ev_gdone[0], c->ev_gdone[1]};
   for (cudaEvent_t e : evs)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->trace.ev) cudaEventDestroy(e);

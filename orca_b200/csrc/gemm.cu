@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "attn_out.cuh"
 #include "context.cuh"
 #include "index_ops.cuh"
 #include "tc_gemm.cuh"
@@ -205,7 +206,7 @@ __device__ __forceinline__ float half_warp_sum(float v) {
   return v;
 }
 
-struct OutArgs {
+struct SimtOutArgs {
   orca_attn_weights_t w;
   const float *ctx;
   const uint8_t *valid;
@@ -218,7 +219,7 @@ struct OutArgs {
   const uint8_t *push_win;
 };
 
-__global__ void __launch_bounds__(F2_THREADS) attn_output_kernel(OutArgs g) {
+__global__ void __launch_bounds__(F2_THREADS) attn_output_kernel(SimtOutArgs g) {
   extern __shared__ __align__(16) unsigned char raw[];
   F2Smem &s = *reinterpret_cast<F2Smem *>(raw);
   const int M = rows_of(g.m_cap, g.d_m);
@@ -415,6 +416,79 @@ static int ensure_f2_smem() {
 
 static inline int kblocks(int k) { return (k + tc::BK - 1) / tc::BK; }
 
+namespace orca {
+
+// Arguments of the tensor-core projections.  The functions that end in _rows serve a group of batches (group.cu): rows
+// of a two-part table, tensor cores only.
+static tc::Args output_args(const orca_attn_weights_t *w, const float *d_ctx, const uint8_t *d_valid,
+                            const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_out) {
+  tc::Args a{};
+  a.a0 = tc::RowSrc{d_ctx, nullptr, QT, 0, 0};
+  a.a1 = feat;
+  a.Kd = QT + D;
+  a.row_valid = d_valid;
+  a.zero_cols = QT;
+  a.w_packed = w->G_tc;
+  a.n_kblocks = kblocks(QT + D);
+  a.m_cap = n_cap;
+  a.d_m = d_n;
+  a.bias = w->b1;
+  a.bias2 = w->g;
+  a.w2_packed = w->W2t_tc;
+  a.bias_out = w->b2;
+  a.ln_w = w->ln_w;
+  a.ln_b = w->ln_b;
+  a.out = d_out;
+  return a;
+}
+static tc::Args score_args(const orca_score_weights_t *w, const float *d_emb, int rows, float *d_prob) {
+  tc::Args a{};
+  a.a0 = tc::RowSrc{d_emb, nullptr, D, 0, 0};
+  a.a1 = tc::RowSrc{d_emb, nullptr, D, 0, 0};
+  a.Kd = 2 * D;
+  a.w_packed = w->W1t_tc;
+  a.n_kblocks = kblocks(2 * D);
+  a.m_cap = rows;
+  a.bias = w->b1;
+  a.w2 = w->w2;
+  a.b2 = w->b2;
+  a.out = d_prob;
+  return a;
+}
+int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
+               float *d_prob, cudaStream_t s) {
+  tc::Args a = score_args(w, d_emb, rows, d_prob);
+  a.a0.idx = d_a;
+  a.a1.idx = d_b;
+  return tc::launch(tc::EPI_SCORE, a, 1, s);
+}
+static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
+                         const int32_t *d_mem_rows, int n_cap, const int32_t *d_n, float *d_out) {
+  tc::Args a{};
+  a.a0 = tc::RowSrc{mem->messages, d_nodes, MSG, 0, 0};
+  a.a1 = tc::RowSrc{mem->memory, d_mem_rows, D, 0, 0};
+  a.Kd = MSG + D;
+  a.w_packed = w->Wg_tc;
+  a.n_kblocks = kblocks(tc::GRU_K);
+  a.m_cap = n_cap;
+  a.d_m = d_n;
+  a.bias = w->bg;
+  a.out = d_out;
+  a.memory = mem->memory;
+  a.nodes = d_mem_rows;
+  return a;
+}
+int gru_project_rows(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
+                     const int32_t *d_mem_rows, const float *mem2, int mem_split, int n_cap, const int32_t *d_n,
+                     float *d_out, cudaStream_t s) {
+  tc::Args a = gru_args(w, mem, d_nodes, d_mem_rows, n_cap, d_n, d_out);
+  a.a1.p2 = a.memory2 = mem2;
+  a.a1.split = a.memory_split = mem_split;
+  return tc::launch(tc::EPI_GRU, a, 4, s);
+}
+
+}  // namespace orca
+
 extern "C" {
 
 int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int32_t *d_idx,
@@ -423,17 +497,7 @@ int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int
   if (n_rows_cap == 0) return ORCA_OK;
   if (projection_mode() == 0) {
     ORCA_CHECK_ARG(w->Mq_tc != nullptr);
-    tc::Args a{};
-    a.a0 = tc::RowSrc{d_feat, d_idx, D, 0, 0};
-    a.Kd = D;
-    a.w_packed = w->Mq_tc;
-    a.n_kblocks = kblocks(D);
-    a.m_cap = n_rows_cap;
-    a.d_m = d_n_rows;
-    a.bias = w->cq;
-    a.out = d_qt;
-    a.out_ld = QT_LD;
-    return tc::launch(tc::EPI_BIAS, a, QT_LD / tc::BN, (cudaStream_t)stream);
+    return attn_query_rows(w, tc::RowSrc{d_feat, d_idx, D, 0, 0}, n_rows_cap, d_n_rows, d_qt, (cudaStream_t)stream);
   }
   F1Args g{};
   g.a0 = RowSrc{d_feat, d_idx, D, 0, 0};
@@ -459,7 +523,7 @@ int orca_attn_output(const orca_attn_weights_t *w, const float *d_ctx, const uin
                      void *stream) {
   ORCA_CHECK_ARG(d_push_table == nullptr || (d_push_ids && d_push_win));
   return orca::attn_output_impl(w, d_ctx, d_valid, d_feat, d_idx, n_rows_cap, d_n_rows, d_out, d_push_table,
-                                d_push_ids, d_push_win, nullptr, 0, 0, d_scratch_hidden, 0, (cudaStream_t)stream);
+                                d_push_ids, d_push_win, nullptr, 0, 0, d_scratch_hidden, (cudaStream_t)stream);
 }
 
 }  // extern "C"
@@ -478,15 +542,13 @@ __global__ void win_from_last_pos_kernel(const int32_t *__restrict__ ids, int ca
 
 bool projections_on_tensor_cores() { return projection_mode() == 0; }
 
-// d_push_win given: rows with a non-zero byte are pushed.  Otherwise (d_last_pos given) row i is
-// pushed when i >= all_from or when last_pos[push_ids[i]] == base + i; `d_push_win` is then only
-// scratch for the fp32 debug path and may be NULL in tensor-core mode.  rows_hint (> 0): the live row
-// count the caller expects (n_rows_cap is a capacity); it only steers how the work is spread.
+// d_push_win given: rows with a non-zero byte are pushed.  Otherwise (d_last_pos given, fp32 projections only) row i is
+// pushed when i >= all_from or when last_pos[push_ids[i]] == base + i, and `d_push_win` is scratch.
 int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uint8_t *d_valid, const float *d_feat,
                      const int32_t *d_idx, int32_t n_rows_cap, const int32_t *d_n_rows, float *d_out,
                      float *d_push_table, const int32_t *d_push_ids, const uint8_t *d_push_win,
                      const int64_t *d_last_pos, long long base, int all_from, float *d_scratch_hidden,
-                     int rows_hint, cudaStream_t stream, const tc::PeerOut *peer) {
+                     cudaStream_t stream) {
   ORCA_CHECK_ARG(w && w->G && w->b1 && w->g && w->W2t && w->b2 && w->ln_w && w->ln_b);
   ORCA_CHECK_ARG(d_ctx && d_valid && d_feat && d_out && n_rows_cap >= 0);
   if (n_rows_cap == 0) return ORCA_OK;
@@ -504,37 +566,16 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
     // One kernel: relu([ctx | feat] . G + b1 + valid * g) stays on the SM as the A operand of the second
     // product (. W2t + b2), whose epilogue is the LayerNorm with the history push.  (The hidden tile never
     // goes to HBM; d_scratch_hidden is not used in this mode.)
-    (void)rows_hint;
     (void)d_scratch_hidden;
-    tc::Args a{};
-    a.a0 = tc::RowSrc{d_ctx, nullptr, QT, 0, 0};
-    a.a1 = tc::RowSrc{d_feat, d_idx, D, 0, 0};
-    a.Kd = QT + D;
-    a.row_valid = d_valid;
-    a.zero_cols = QT;
-    a.w_packed = w->G_tc;
-    a.n_kblocks = kblocks(QT + D);
-    a.m_cap = n_rows_cap;
-    a.d_m = d_n_rows;
-    a.bias = w->b1;
-    a.bias2 = w->g;
-    a.w2_packed = w->W2t_tc;
-    a.bias_out = w->b2;
-    a.ln_w = w->ln_w;
-    a.ln_b = w->ln_b;
-    a.out = d_out;
+    tc::Args a = output_args(w, d_ctx, d_valid, tc::RowSrc{d_feat, d_idx, D, 0, 0}, n_rows_cap, d_n_rows, d_out);
     a.push_table = d_push_table;
     a.push_ids = d_push_ids;
-    a.push_win = d_last_pos ? nullptr : d_push_win;
-    a.push_last_pos = reinterpret_cast<const unsigned long long *>(d_last_pos);
-    a.push_base = base;
-    a.push_all_from = all_from;
-    if (peer != nullptr) a.peer = *peer;
+    a.push_win = d_push_win;
     return tc::launch(tc::EPI_MERGER, a, 1, (cudaStream_t)stream);
   }
   int rc = ensure_f2_smem();
   if (rc) return rc;
-  OutArgs g{};
+  SimtOutArgs g{};
   g.w = *w;
   g.ctx = d_ctx;
   g.valid = d_valid;
@@ -562,18 +603,7 @@ int gru_project(const orca_gru_weights_t *w, const orca_memory_t *mem, const int
   if (n_cap == 0) return ORCA_OK;
   if (projection_mode() == 0) {
     ORCA_CHECK_ARG(w->Wg_tc != nullptr);
-    tc::Args a{};
-    a.a0 = tc::RowSrc{mem->messages, d_nodes, MSG, 0, 0};
-    a.a1 = tc::RowSrc{mem->memory, d_nodes, D, 0, 0};
-    a.Kd = MSG + D;
-    a.w_packed = w->Wg_tc;
-    a.n_kblocks = kblocks(MSG + D);
-    a.m_cap = n_cap;
-    a.d_m = d_n;
-    a.bias = w->bg;
-    a.out = d_scratch_h;
-    a.memory = mem->memory;
-    a.nodes = d_nodes;
+    tc::Args a = gru_args(w, mem, d_nodes, d_nodes, n_cap, d_n, d_scratch_h);
     if (peer != nullptr) {
       // one rank of the multi-GPU split: every world-th listed node from `rank`, rows delivered to all ranks
       a.peer = *peer;
@@ -624,18 +654,10 @@ int orca_score(const orca_score_weights_t *w, const float *d_emb, int32_t b, flo
   if (b == 0) return ORCA_OK;
   if (projection_mode() == 0) {
     ORCA_CHECK_ARG(w->W1t_tc != nullptr);
-    tc::Args a{};
+    tc::Args a = score_args(w, d_emb, 2 * b, d_prob);
     // row m < b pairs (src m, dst m); row m >= b pairs (src m-b, neg m-b): table rows m % b and b + m
-    a.a0 = tc::RowSrc{d_emb, nullptr, D, b, 0};
-    a.a1 = tc::RowSrc{d_emb, nullptr, D, 0, b};
-    a.Kd = 2 * D;
-    a.w_packed = w->W1t_tc;
-    a.n_kblocks = kblocks(2 * D);
-    a.m_cap = 2 * b;
-    a.bias = w->b1;
-    a.w2 = w->w2;
-    a.b2 = w->b2;
-    a.out = d_prob;
+    a.a0.mod = b;
+    a.a1.add = b;
     return tc::launch(tc::EPI_SCORE, a, 1, (cudaStream_t)stream);
   }
   int rc = ensure_f2_smem();

@@ -23,14 +23,20 @@ int launch_uncached_finish(const orca_tgn_t *m, int n_query, int32_t *nodes_io, 
 int launch_last_occ_compact(const int32_t *d_ids, int n, int64_t n_nodes, int64_t *d_last_pos, long long base,
                             int32_t *d_compact, int32_t *d_n_compact, int32_t *d_status, cudaStream_t s);
 
+// cache flags after a batch with a plan (History.update_flag): those of m->prev_plan cleared, those of d_plan set
+int launch_plan_flags(const orca_tgn_t *m, const int32_t *d_plan, int n_plan, cudaStream_t s);
+
 // the fused gather-attention kernel (attention.cu); d_ticket: two zeroed device words that the launch
 // leaves at zero (launches that may overlap on the GPU need words of their own); rows_hint > 0: the live
 // row count the caller expects (n_rows_cap is a capacity); d_order (optional): the row ids in the order the
-// warps should take them (launch_row_order)
+// warps should take them (launch_row_order); image: d_ctx is the output kernel's operand image (attn_out.cuh) instead of
+// [rows, 1032] floats; d_nbr_table2 (optional): neighbour rows >= nbr_split are read from it, its
+// address already moved back by nbr_split rows
 int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float *d_edge_table,
                        const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid, const float *d_delta,
                        int k, int n_rows_cap, const int32_t *d_n_rows, int rows_hint, const int32_t *d_order,
-                       float *d_ctx, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream);
+                       void *d_ctx, bool image, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream,
+                       const float *d_nbr_table2 = nullptr, int nbr_split = 0);
 // rows of two neighbour tables sorted by falling number of valid slots (one launch, one block per table)
 int launch_row_order(const int32_t *d_nbr_a, int n_cap_a, const int32_t *d_n_a, int32_t *d_order_a,
                      const int32_t *d_nbr_b, int n_cap_b, const int32_t *d_n_b, int32_t *d_order_b, int k,

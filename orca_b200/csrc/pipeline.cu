@@ -27,6 +27,7 @@
 #include <cstring>
 #include <vector>
 
+#include "attn_out.cuh"
 #include "common.cuh"
 #include "context.cuh"
 #include "index_ops.cuh"
@@ -48,12 +49,15 @@ struct IdxBuf {
 };
 // projection / gather buffers of one attention layer in flight (one set per compute lane)
 struct LaneBuf {
-  float *qt, *ctx, *hidden; uint8_t *valid;
+  float *qt, *hidden;
+  char *ctx, *feat;    // operand images of the attention sums and of the rows' own features (attn_out.cuh)
+  uint8_t *valid;
 };
 struct Workspace {
   IdxBuf idx[2];
   LaneBuf lane[2];
   float *emb1[2];
+  char *feat2[2];            // operand image of layer 2's own features, written by layer 1 (one GPU)
   float *emb2;
   uint8_t *win1;
   float *gru_h;
@@ -96,11 +100,13 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
   for (int q = 0; q < 2; ++q) {
     const size_t rows = q == 0 ? R1 : N;   // lane 0: layer 1 (and the one-lane modes), lane 1: layer 2
     w.lane[q].qt = (float *)take(rows * QT_LD * 4);
-    w.lane[q].ctx = (float *)take(rows * QT * 4);
+    w.lane[q].ctx = (char *)take(img::bytes(rows, img::CTX_STAGES));   // (no smaller than [rows, 1032] floats)
+    w.lane[q].feat = (char *)take(img::bytes(rows, img::FEAT_STAGES));
     w.lane[q].hidden = (float *)take(rows * D * 4);
     w.lane[q].valid = (uint8_t *)take(rows);
   }
   for (int q = 0; q < 2; ++q) w.emb1[q] = (float *)take(R1 * D * 4);
+  for (int q = 0; q < 2; ++q) w.feat2[q] = (char *)take(img::bytes(N, img::FEAT_STAGES));
   w.emb2 = (float *)take(N * D * 4);
   w.win1 = (uint8_t *)take(R1);
   w.gru_h = (float *)take(2 * (size_t)b_cap * D * 4);
@@ -159,6 +165,16 @@ plan_flags_kernel(uint8_t *__restrict__ flag, int64_t n_nodes, int32_t *__restri
       if (i0 + u * 1024 < n_plan) prev_plan[i0 + u * 1024] = v[u];
     }
   }
+}
+
+int launch_plan_flags(const orca_tgn_t *m, const int32_t *d_plan, int n_plan, cudaStream_t s) {
+  const int n_prev = *m->n_prev_plan >= 0 ? *m->n_prev_plan : 0;
+  if (*m->n_prev_plan < 0) ORCA_CUDA(cudaMemsetAsync(m->cache_flag, 0, (size_t)m->n_nodes, s));
+  plan_flags_kernel<<<1, 1024, 0, s>>>(m->cache_flag, m->n_nodes, m->prev_plan, n_prev, d_plan, n_plan);
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  *m->n_prev_plan = n_plan;
+  return ORCA_OK;
 }
 
 // ---- row sharding over `world` ranks: layer-1 row i -> rank i % world, slot i / world
@@ -329,6 +345,50 @@ using namespace orca;
 
 namespace orca {
 
+// The three steps of an attention layer.  On the tensor cores the attention sums travel as the output kernel's operand
+// image (attn_out.cuh), with the fp32 projections as [rows, 1032] floats, in the same buffer.
+// (have_image: the layer below has left the image of this layer's rows in l.feat)
+static int layer_query(const orca_attn_weights_t *w, const float *d_feat, const int32_t *d_idx, int cap,
+                       const int32_t *d_n, LaneBuf &l, cudaStream_t s, bool have_image = false) {
+  if (projections_on_tensor_cores()) {
+    if (!have_image) {
+      const int rc = feat_image(tc::RowSrc{d_feat, d_idx, D, 0, 0}, cap, d_n, l.feat, s);
+      if (rc) return rc;
+    }
+    return attn_query_image(w, l.feat, cap, d_n, l.qt, s);
+  }
+  return orca_attn_query(w, d_feat, d_idx, cap, d_n, l.qt, s);
+}
+static int layer_gather(const orca_tgn_t *m, const float *d_nbr_table, const int32_t *d_nbr, const int32_t *d_eid,
+                        const float *d_dt, int cap, const int32_t *d_n, int rows_hint, const int32_t *d_order, LaneBuf &l,
+                        int32_t *d_ticket, cudaStream_t s) {
+  return launch_attn_gather(l.qt, d_nbr_table, m->edge_table, m->time_w, d_nbr, d_eid, d_dt, m->k, cap, d_n, rows_hint,
+                            d_order, l.ctx, projections_on_tensor_cores(), l.valid, d_ticket, s);
+}
+struct Push {      // optional history push (OutArgs); win: flags, or scratch of the fp32 path when there are records
+  float *table = nullptr;
+  const int32_t *ids = nullptr;
+  const uint8_t *win = nullptr;
+  const int64_t *last_pos = nullptr;
+  long long base = 0;
+  int all_from = 0;
+};
+static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d_feat, const int32_t *d_idx, int cap,
+                        const int32_t *d_n, float *d_out, const Push &push, cudaStream_t s,
+                        const tc::PeerOut *peer = nullptr, char *d_image = nullptr, int image_rows = 0) {
+  if (!projections_on_tensor_cores())
+    return attn_output_impl(w, (const float *)l.ctx, l.valid, d_feat, d_idx, cap, d_n, d_out, push.table, push.ids,
+                            push.win, push.last_pos, push.base, push.all_from, l.hidden, s);
+  OutArgs a{};
+  a.w = *w, a.ctx = l.ctx, a.feat = l.feat, a.valid = l.valid, a.n_cap = cap, a.d_n = d_n, a.out = d_out;
+  a.push_table = push.table, a.push_ids = push.ids, a.push_win = push.last_pos != nullptr ? nullptr : push.win;
+  a.push_last_pos = reinterpret_cast<const unsigned long long *>(push.last_pos);
+  a.push_base = push.base, a.push_all_from = push.all_from;
+  if (peer != nullptr) a.peer = *peer;
+  a.out_image = d_image, a.out_image_rows = d_image != nullptr ? image_rows : 0;
+  return attn_output_rows(a, s);
+}
+
 static Ctx *ctx_of(const orca_tgn_t *m) {
   return m->ctx != nullptr ? reinterpret_cast<Ctx *>(m->ctx) : default_ctx();
 }
@@ -361,13 +421,11 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1, x.ts1, N,
                               nullptr, k, x.nbr1, x.eid1, nullptr, x.dt1, d_status, s));
     ORCA_TRY(tr.mark(PH_SAMPLE_TOP, s));
-    ORCA_TRY(orca_attn_query(&m->attn[0], m->mem.memory, x.nodes1, N, nullptr, l.qt, s));
+    ORCA_TRY(layer_query(&m->attn[0], m->mem.memory, x.nodes1, N, nullptr, l, s));
     ORCA_TRY(tr.mark(PH_QUERY_L2, s));
-    ORCA_TRY(launch_attn_gather(l.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1, x.eid1, x.dt1, k, N, nullptr,
-                                0, nullptr, l.ctx, l.valid, tk, s));
+    ORCA_TRY(layer_gather(m, m->mem.memory, x.nbr1, x.eid1, x.dt1, N, nullptr, 0, nullptr, l, tk, s));
     ORCA_TRY(tr.mark(PH_GATHER_L2, s));
-    ORCA_TRY(orca_attn_output(&m->attn[0], l.ctx, l.valid, m->mem.memory, x.nodes1, N, nullptr, emb_top,
-                              nullptr, nullptr, nullptr, l.hidden, s));
+    ORCA_TRY(layer_output(&m->attn[0], l, m->mem.memory, x.nodes1, N, nullptr, emb_top, Push{}, s));
     ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
   } else {
     // top-level neighbour table; then the row list of layer 1 by recursion mode
@@ -403,28 +461,27 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     }
     ORCA_TRY(tr.mark(PH_LAST_OCC_L1, s));
     // layer 1 over memory rows; with unlimited reuse its output rows are pushed into the history table
-    ORCA_TRY(orca_attn_query(&m->attn[0], m->mem.memory, x.nodes1, R1, d_n1, l.qt, s));
+    ORCA_TRY(layer_query(&m->attn[0], m->mem.memory, x.nodes1, R1, d_n1, l, s));
     ORCA_TRY(tr.mark(PH_QUERY_L1, s));
-    ORCA_TRY(launch_attn_gather(l.qt, m->mem.memory, m->edge_table, m->time_w, nbr1, eid1, dt1, k, R1, d_n1,
-                                mode == ORCA_MODE_NO_REUSE ? R1 : N, nullptr, l.ctx, l.valid, tk, s));
+    ORCA_TRY(layer_gather(m, m->mem.memory, nbr1, eid1, dt1, R1, d_n1, mode == ORCA_MODE_NO_REUSE ? R1 : N, nullptr, l, tk,
+                          s));
     ORCA_TRY(tr.mark(PH_GATHER_L1, s));
-    ORCA_TRY(attn_output_impl(&m->attn[0], l.ctx, l.valid, m->mem.memory, x.nodes1, R1, d_n1, w.emb1[0],
-                              push1 ? m->hist_emb : nullptr, push1 ? x.nodes1 : nullptr, push1 ? w.win1 : nullptr,
-                              nullptr, 0, N, l.hidden, mode == ORCA_MODE_NO_REUSE ? R1 : N, s));
+    ORCA_TRY(layer_output(&m->attn[0], l, m->mem.memory, x.nodes1, R1, d_n1, w.emb1[0],
+                          push1 ? Push{m->hist_emb, x.nodes1, w.win1} : Push{}, s, nullptr, w.feat2[0], N));
     ORCA_TRY(tr.mark(PH_OUTPUT_L1, s));
     if (c->overlap && !tr.on) {
       ORCA_TRY(link(s, c->aux, c->fork));
       forked = true;
     }
     ORCA_TRY(tr.mark(PH_FLAGS, s));
+    LaneBuf l2 = l;
+    l2.feat = w.feat2[0];
     // layer 2 over the history rows (or, without reuse, the fresh layer-1 rows) of the top-level neighbours
-    ORCA_TRY(orca_attn_query(&m->attn[1], w.emb1[0], nullptr, N, nullptr, l.qt, s));
+    ORCA_TRY(layer_query(&m->attn[1], w.emb1[0], nullptr, N, nullptr, l2, s, true));
     ORCA_TRY(tr.mark(PH_QUERY_L2, s));
-    ORCA_TRY(launch_attn_gather(l.qt, table2, m->edge_table, m->time_w, gather2, x.eid2, x.dt2, k, N, nullptr, 0,
-                                nullptr, l.ctx, l.valid, tk, s));
+    ORCA_TRY(layer_gather(m, table2, gather2, x.eid2, x.dt2, N, nullptr, 0, nullptr, l2, tk, s));
     ORCA_TRY(tr.mark(PH_GATHER_L2, s));
-    ORCA_TRY(orca_attn_output(&m->attn[1], l.ctx, l.valid, w.emb1[0], nullptr, N, nullptr, emb_top, nullptr,
-                              nullptr, nullptr, l.hidden, s));
+    ORCA_TRY(layer_output(&m->attn[1], l2, w.emb1[0], nullptr, N, nullptr, emb_top, Push{}, s));
     ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
   }
   ORCA_TRY(orca_score(&m->score, emb_top, b, d_prob, s));
@@ -494,7 +551,8 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
   const int p = c->parity;
   c->last_parity = p;
   IdxBuf &x = w.idx[p];
-  LaneBuf &l1 = w.lane[0], &l2 = w.lane[lanes ? 1 : 0];
+  LaneBuf &l1 = w.lane[0], l2 = w.lane[lanes ? 1 : 0];
+  if (!sharded) l2.feat = w.feat2[p];
   int64_t *lp_push = m->last_pos + (size_t)p * m->n_nodes, *lp_msg = m->last_pos + 2 * (size_t)m->n_nodes;
   const long long base1 = c->base1;
   float *emb1 = d_emb1_local != nullptr ? d_emb1_local : w.emb1[p];
@@ -559,12 +617,7 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_idx[p], si));
     // cache flags of this batch (History.update_flag): read next by the next batch's head kernel
     if (d_plan != nullptr) {
-      const int n_prev = *m->n_prev_plan >= 0 ? *m->n_prev_plan : 0;
-      if (*m->n_prev_plan < 0) ORCA_CUDA(cudaMemsetAsync(m->cache_flag, 0, (size_t)m->n_nodes, si));
-      plan_flags_kernel<<<1, 1024, 0, si>>>(m->cache_flag, m->n_nodes, m->prev_plan, n_prev, d_plan, n_plan);
-      ORCA_COUNT_LAUNCH();
-      ORCA_LAUNCH_CHECK();
-      *m->n_prev_plan = n_plan;
+      ORCA_TRY(launch_plan_flags(m, d_plan, n_plan, si));
     } else {
       // plan-less rule: the flags of the pushed ids are set and never cleared
       set_flags_counted_kernel<<<std::min(ceil_div(R1, 256), 1024), 256, 0, si>>>(m->cache_flag, m->n_nodes,
@@ -620,18 +673,18 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     const int32_t *rows1 = sharded ? x.loc_nodes : x.nodes1;
     const int32_t *d_n1 = sharded ? x.n1_loc : x.n1;
     const int cap1 = sharded ? rpr : R1;
-    ORCA_TRY(orca_attn_query(&m->attn[0], m->mem.memory, rows1, cap1, d_n1, l1.qt, sa));
+    ORCA_TRY(layer_query(&m->attn[0], m->mem.memory, rows1, cap1, d_n1, l1, sa));
     ORCA_TRY(tr.mark(PH_QUERY_L1, s));
-    ORCA_TRY(launch_attn_gather(l1.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1, x.eid1, x.dt1, k, cap1, d_n1,
-                                sharded ? rpr : N, x.order1, l1.ctx, l1.valid, c->d_words + CTX_TICKET_MAIN, sa));
+    ORCA_TRY(layer_gather(m, m->mem.memory, x.nbr1, x.eid1, x.dt1, cap1, d_n1, sharded ? rpr : N, x.order1, l1,
+                          c->d_words + CTX_TICKET_MAIN, sa));
     ORCA_TRY(tr.mark(PH_GATHER_L1, s));
     if (!sharded) {
       // the push into the history table waits for the previous batch's top layer to have read it
       if (sa != s && c->g2_recorded) ORCA_CUDA(cudaStreamWaitEvent(sa, c->ev_g2, 0));
       // (winners of the push come from the records of the head kernel; the appended rows are distinct
       // out-of-batch nodes, so each of them wins)
-      ORCA_TRY(attn_output_impl(&m->attn[0], l1.ctx, l1.valid, m->mem.memory, x.nodes1, R1, x.n1, emb1, m->hist_emb,
-                                x.nodes1, w.win1, lp_push, base1, N, l1.hidden, N, sa));
+      ORCA_TRY(layer_output(&m->attn[0], l1, m->mem.memory, x.nodes1, R1, x.n1, emb1,
+                            Push{m->hist_emb, x.nodes1, w.win1, lp_push, base1, N}, sa, nullptr, l2.feat, N));
     } else if (direct && projections_on_tensor_cores()) {
       // the LayerNorm epilogue of layer 1 delivers the rows itself: one kernel computes and exchanges
       const long long seq = c->xseq;
@@ -650,11 +703,9 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
                              d_status, c->wait_limit));
         ORCA_COUNT_LAUNCH();
       }
-      ORCA_TRY(attn_output_impl(&m->attn[0], l1.ctx, l1.valid, m->mem.memory, x.loc_nodes, rpr, x.n1_loc, emb1,
-                                nullptr, nullptr, nullptr, nullptr, 0, 0, l1.hidden, 0, sa, &po));
+      ORCA_TRY(layer_output(&m->attn[0], l1, m->mem.memory, x.loc_nodes, rpr, x.n1_loc, emb1, Push{}, sa, &po));
     } else {
-      ORCA_TRY(orca_attn_output(&m->attn[0], l1.ctx, l1.valid, m->mem.memory, x.loc_nodes, rpr, x.n1_loc, emb1,
-                                nullptr, nullptr, nullptr, l1.hidden, sa));
+      ORCA_TRY(layer_output(&m->attn[0], l1, m->mem.memory, x.loc_nodes, rpr, x.n1_loc, emb1, Push{}, sa));
       if (direct) {
         // (fp32 debug projections: a separate kernel fans the rows out)
         const long long seq = c->xseq;
@@ -731,17 +782,16 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     if (rows2 > 0) {
       ORCA_CHECK_ARG(d_prob != nullptr);
       float *emb_top = d_emb_out ? d_emb_out : w.emb2;
-      ORCA_TRY(orca_attn_query(&m->attn[1], feat2, feat2_idx, rows2, nullptr, l2.qt, s));
+      ORCA_TRY(layer_query(&m->attn[1], feat2, feat2_idx, rows2, nullptr, l2, s, !sharded));
       ORCA_TRY(tr.mark(PH_QUERY_L2, s));
-      ORCA_TRY(launch_attn_gather(l2.qt, m->hist_emb, m->edge_table, m->time_w, nbr2, eid2, dt2, k, rows2, nullptr, 0,
-                                  x.order2, l2.ctx, l2.valid, c->d_words + CTX_TICKET_SIDE, s));
+      ORCA_TRY(layer_gather(m, m->hist_emb, nbr2, eid2, dt2, rows2, nullptr, 0, x.order2, l2,
+                            c->d_words + CTX_TICKET_SIDE, s));
       ORCA_TRY(tr.mark(PH_GATHER_L2, s));
       if (!sharded && sa != s) {
         ORCA_CUDA(cudaEventRecord(c->ev_g2, s));
         c->g2_recorded = true;
       }
-      ORCA_TRY(orca_attn_output(&m->attn[1], l2.ctx, l2.valid, feat2, feat2_idx, rows2, nullptr, emb_top, nullptr,
-                                nullptr, nullptr, l2.hidden, s));
+      ORCA_TRY(layer_output(&m->attn[1], l2, feat2, feat2_idx, rows2, nullptr, emb_top, Push{}, s));
       ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
       ORCA_TRY(orca_score(&m->score, emb_top, b2, d_prob, s));
       ORCA_TRY(tr.mark(PH_SCORE, s));

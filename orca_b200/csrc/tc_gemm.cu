@@ -42,142 +42,14 @@
 // Every wait on an mbarrier is bounded; a wait that gives up records ORCA_E_TIMEOUT and the kernel
 // runs to its end (tensor memory is always released).
 #include <algorithm>
-#include <cuda_bf16.h>
 
 #include "common.cuh"
 #include "context.cuh"
 #include "tc_gemm.cuh"
+#include "tc_ptx.cuh"
 
 namespace orca {
 namespace tc {
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait (`limit` SM clocks, about a second by default); records the failure if the barrier never
-// flipped.  `alive` makes the failure sticky: a thread that gave up once does not wait again, so a
-// broken pipeline drains in one limit instead of one time-out per stage.
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int32_t *status, int where, bool &alive,
-                                          long long limit) {
-  if (!alive) return;
-  if (mbar_try(bar, parity)) return;
-  const long long t0 = clock64();
-  while (!mbar_try(bar, parity)) {
-    if (clock64() - t0 > limit) {
-      report(status, ORCA_E_TIMEOUT, where);
-      alive = false;
-      return;
-    }
-  }
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// shared-memory matrix descriptor, no swizzle, K-major: 8 rows x 16 bytes form one contiguous
-// 128-byte core matrix; `lbo` = bytes between the two 16-byte K chunks of one MMA, `sbo` = bytes
-// between consecutive 8-row groups
-__device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3fff);
-  d |= (uint64_t)((lbo >> 4) & 0x3fff) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3fff) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version of this architecture
-  return d;
-}
-
-// D[tmem] (+)= A[smem] . B[smem]^T, 128 x 176 x 16, bf16 inputs, fp32 accumulate
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// 16 consecutive accumulator columns of this thread's lane (= tile row)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-// main accumulator + cross-term accumulator: both loads in flight, one wait
-__device__ __forceinline__ void tmem_ld16_sum(uint32_t taddr, float (&v)[16]) {
-  uint32_t a[16], b[16];
-  tmem_ld16_nowait(taddr, a);
-  tmem_ld16_nowait(taddr + TMEM_SMALL, b);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
-}
-
-__device__ __forceinline__ float4 ld_shared_f4(uint32_t saddr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(saddr));
-  return v;
-}
-__device__ __forceinline__ void st_shared_f4(uint32_t saddr, float4 v) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-               : "memory");
-}
-
-// x ~ head + tail, both bf16 (round to nearest even), for 8 consecutive K elements: one 16-byte chunk
-// of the head image and one of the tail image.  Packed conversions (two floats per instruction).
-__device__ __forceinline__ uint32_t pack_split(float x0, float x1, uint32_t &lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-  const uint32_t hb = *reinterpret_cast<const uint32_t *>(&h);
-  const float r0 = x0 - __uint_as_float(hb << 16);
-  const float r1 = x1 - __uint_as_float(hb & 0xffff0000u);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(r0, r1);
-  lo = *reinterpret_cast<const uint32_t *>(&l);
-  return hb;
-}
-__device__ __forceinline__ void split_chunk(const float4 a, const float4 b, uint4 &hi, uint4 &lo) {
-  hi.x = pack_split(a.x, a.y, lo.x);
-  hi.y = pack_split(a.z, a.w, lo.y);
-  hi.z = pack_split(b.x, b.y, lo.z);
-  hi.w = pack_split(b.z, b.w, lo.w);
-}
 
 struct Smem {
   uint32_t base;  // shared-window address of the (1024-byte aligned) stage ring
@@ -186,16 +58,6 @@ struct Smem {
   __device__ uint32_t b_hi(int s) const { return base + s * STAGE_BYTES + 2 * A_BYTES; }
   __device__ uint32_t b_lo(int s) const { return base + s * STAGE_BYTES + 2 * A_BYTES + B_BYTES; }
 };
-
-__device__ __forceinline__ const float *src_row(const RowSrc &s, int m) {
-  const int r = s.idx ? s.idx[m] : (s.mod > 0 ? m % s.mod : m) + s.add;
-  return s.p + (size_t)r * s.width;
-}
-
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-               : "memory");
-}
 
 __device__ __align__(16) float g_zero16[4] = {0.f, 0.f, 0.f, 0.f};
 
@@ -219,7 +81,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
   constexpr int BNv = tile_bn<EPI>();
   const int c0 = nt * BNv;
   const int j0 = lane, j1 = lane + 32;
-  const int nj = (EPI == EPI_BIAS || EPI == EPI_GRU) ? BNv / 4 : D / 4;
+  const int nj = EPI == EPI_GRU ? BNv / 4 : D / 4;
   const bool has0 = j0 < nj;      // (only a 96-column tile leaves lanes without a first piece)
   const bool has1 = j1 < nj;
   const float4 f4z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -250,20 +112,12 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       b[k] = has1 ? add4(ld_shared_f4(ra + 512u), bB) : f4z;
       hA[k] = hB[k] = 0.f;
       if (EPI == EPI_GRU && ok[k]) {
-        const float *hrow = g.memory + (size_t)mb[k] * D;
+        const float *hrow = (g.memory2 != nullptr && mb[k] >= g.memory_split ? g.memory2 : g.memory) + (size_t)mb[k] * D;
         if (uA < D) hA[k] = hrow[uA];
         if (has1 && uB < D) hB[k] = hrow[uB];
       }
     }
-    if (EPI == EPI_BIAS) {
-#pragma unroll
-      for (int k = 0; k < RB; ++k)
-        if (ok[k]) {
-          float *o = g.out + (size_t)m[k] * g.out_ld + c0;
-          *reinterpret_cast<float4 *>(o + 4 * j0) = a[k];
-          if (has1) *reinterpret_cast<float4 *>(o + 4 * j1) = b[k];
-        }
-    } else if (EPI == EPI_LAYERNORM) {
+    if (EPI == EPI_LAYERNORM) {
       // both moments in one sweep (the row is O(1) after the merger, so E[y^2] - mean^2 loses nothing
       // that matters at the 1e-5 epsilon)
       float sum[RB], sumsq[RB];
@@ -299,12 +153,6 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
             *reinterpret_cast<float4 *>(prow + 4 * j0) = ya;
             if (has1) *reinterpret_cast<float4 *>(prow + 4 * j1) = yb;
           }
-          // multi-GPU exchange: the row also goes to every rank's exchange buffer (peer stores)
-          for (int q = 0; q < g.peer.world; ++q) {
-            float *prow = g.peer.rows[q] + g.peer.off + (size_t)m[k] * D;
-            *reinterpret_cast<float4 *>(prow + 4 * j0) = ya;
-            if (has1) *reinterpret_cast<float4 *>(prow + 4 * j1) = yb;
-          }
         }
     } else {  // EPI_GRU: four gate columns per unit, unit = nt * 44 + j
 #pragma unroll
@@ -313,14 +161,12 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
           // (row of the whole list; with the multi-GPU split the row also goes to every rank's buffer)
           const size_t orow = (size_t)(g.row_stride > 1 ? m[k] * g.row_stride + g.row_off : m[k]) * D;
           if (uA < D) {
-            const float rg = 1.f / (1.f + expf(-a[k].x)), z = 1.f / (1.f + expf(-a[k].y));
-            const float h = (1.f - z) * tanhf(a[k].z + rg * a[k].w) + z * hA[k];
+            const float h = gru_gates(a[k], hA[k]);
             if (g.peer.world == 0) g.out[orow + uA] = h;
             for (int q = 0; q < g.peer.world; ++q) g.peer.rows[q][g.peer.off + orow + uA] = h;
           }
           if (has1 && uB < D) {
-            const float rg = 1.f / (1.f + expf(-b[k].x)), z = 1.f / (1.f + expf(-b[k].y));
-            const float h = (1.f - z) * tanhf(b[k].z + rg * b[k].w) + z * hB[k];
+            const float h = gru_gates(b[k], hB[k]);
             if (g.peer.world == 0) g.out[orow + uB] = h;
             for (int q = 0; q < g.peer.world; ++q) g.peer.rows[q][g.peer.off + orow + uB] = h;
           }
@@ -333,7 +179,7 @@ template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
   extern __shared__ unsigned char raw[];
   const int nt = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const bool producer = warp < 4 || warp >= 6;
   const int grp = warp >= 6 ? 1 : 0;
   const int pw = grp ? warp - 6 : warp;   // producer warp within its group: tile rows pw*32 .. pw*32+31
@@ -378,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
     if (r < BM && m < limit) {
       if (kMerger && g.push_table != nullptr) {
         meta_b = g.push_ids[m];
-        if (g.push_win != nullptr) meta_a = g.push_win[m];
+        meta_a = g.push_win[m];
       }
       if (EPI == EPI_GRU) meta_b = g.nodes[rstride > 1 ? min(m * rstride + g.row_off, g.idx_limit - 1) : m];
     }
@@ -410,27 +256,22 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
       const int r1 = __shfl_sync(0xffffffffu, ri1, 4 * i + rsub);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int c = col + 4 * h;
+        int c = col + 4 * h;
+        if (EPI == EPI_GRU) {
+          // five parts of 172 columns, each padded to 176: [edge features | time encoding | own memory | other
+          // memory] of the message (stored as own, other, edge, time), then the memory row
+          const int part = c / GRU_PART, o = c - part * GRU_PART;
+          c = o >= D || part > 4 ? Kd : part == 4 ? MSG + o : (part ^ 2) * D + o;
+        }
         const bool in0 = c < w0;
         const int r = in0 ? r0 : r1;
-        const float *bp = in0 ? g.a0.p + (size_t)r * w0 + c : g.a1.p + (size_t)r * w1 + (c - w0);
+        const float *bp = in0 ? g.a0.base(r) + (size_t)r * w0 + c : g.a1.base(r) + (size_t)r * w1 + (c - w0);
         x[2 * i + h] = *((c >= Kd || r < 0) ? zero : reinterpret_cast<const float4 *>(bp));
       }
     }
   };
   auto fix_rows = [&](int m0) {   // after the live count is known
     if (producer && m0 + pw * 32 + lane >= M) ri0 = ri1 = -1;
-  };
-  // (called after the tile's first stage has been requested: the lookup is two dependent loads and its
-  // result is only needed by the output pass)
-  auto push_winners = [&](int m0) {
-    if (kMerger && g.push_table != nullptr && g.push_win == nullptr) {
-      // winners by record; only for live rows: the id of a row past the live count is not a valid index
-      const int r = warp + (THREADS / 32) * lane;
-      const int m = m0 + r;
-      if (r < BM && m < M)
-        meta_a = (m >= g.push_all_from || g.push_last_pos[meta_b] == (unsigned long long)(g.push_base + m)) ? 1 : 0;
-    }
   };
   // ---- set-up that reads nothing an earlier kernel wrote: barriers, tensor memory, epilogue vectors
   if (tid == 0) {
@@ -456,7 +297,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
   __shared__ __align__(16) float s_bias[BN], s_v1[BN], s_v2[BN];
   __shared__ __align__(16) float s_out[kMerger ? 3 : 1][kMerger ? BN : 4];   // merger: bias, weight, shift of the LayerNorm
   if (warp == 4 || warp == 5) {
-    const int lim = (EPI == EPI_BIAS || EPI == EPI_GRU) ? BNv : D - nt * BNv;   // columns of this tile that exist
+    const int lim = EPI == EPI_GRU ? BNv : D - nt * BNv;   // columns of this tile that exist
     for (int i = tid - 128; i < BN; i += 64) {
       const bool in = i < lim && i < BNv;
       s_bias[i] = in ? g.bias[nt * BNv + i] : 0.f;
@@ -480,11 +321,10 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
   }
   fix_rows(blockIdx.y * BM);
   if ((int)blockIdx.y * BM < M && producer && grp < nkb) load_stage(grp);   // in flight across the barrier
-  push_winners(blockIdx.y * BM);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *slot_ptr;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *slot_ptr, 0);
   bool alive = true;
   float *tile = reinterpret_cast<float *>(raw + (base - raw_addr));
   __shared__ float s_dot[2][BM];   // scorer: partial dot products of the two column halves
@@ -499,7 +339,6 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
       prefetch_rows(m0, M);
       fix_rows(m0);
       if (producer && grp < nkb) load_stage(grp);
-      push_winners(m0);
     }
     if (producer) {
       // ---------------------------------------------------------------- producer groups
@@ -553,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
       __syncwarp();
     } else {
       // ---------------------------------------------------------------- MMA issue
-      if (lane == 0) {
+      {
         // fp32 accumulate, bf16 x bf16, both K-major, N = 176 (96), M = 128
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BNv >> 3) << 17) |
                                    ((uint32_t)(BM >> 4) << 24);
@@ -562,6 +401,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
           const int u = t * (s ? uses1 : uses0) + (kb >> 1);
           mbar_wait(full(s), u & 1, g.status, 300 + s, alive, g.wait_limit);
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ++ks) {
             const uint64_t ah = make_desc(sm.a_hi(s) + ks * 2 * A_LBO, A_LBO, A_SBO);
@@ -575,8 +415,10 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
             mma_bf16(tmem + TMEM_SMALL, ah, bl, idesc, 1u);
           }
           mma_commit(empty(s));  // the stage may be refilled once these MMAs have read it
+          if (kb == nkb - 1) mma_commit(accbar);
+          }
+          __syncwarp();
         }
-        mma_commit(accbar);
         if (kMerger) {
           // second product: hidden tile (A image written by the first epilogue) x second weights, into the
           // same accumulator columns (the first epilogue has read them when a2bar completes)
@@ -596,11 +438,14 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
             const uint64_t bh = make_desc(wb, B_LBO, B_SBO);
             const uint64_t bl = make_desc(wb + wtail, B_LBO, B_SBO);
             const uint32_t first = ks > 0 ? 1u : 0u;
-            mma_bf16(tmem, ah, bh, idesc, first);
-            mma_bf16(tmem + TMEM_SMALL, al, bh, idesc, first);
-            mma_bf16(tmem + TMEM_SMALL, ah, bl, idesc, 1u);
+            if (elect_one()) {
+              mma_bf16(tmem, ah, bh, idesc, first);
+              mma_bf16(tmem + TMEM_SMALL, al, bh, idesc, first);
+              mma_bf16(tmem + TMEM_SMALL, ah, bl, idesc, 1u);
+              if (ks == A2_CHUNKS / 2 - 1) mma_commit(accbar);
+            }
+            __syncwarp();
           }
-          mma_commit(accbar);
         }
       }
       __syncwarp();
@@ -625,7 +470,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
         const uint32_t arow = base + (uint32_t)row * 16u;
         for (int ch = grp ? kHalf : 0; ch < (grp ? BN / 16 : kHalf); ++ch) {
           float v[16];
-          tmem_ld16_sum(trow + ch * 16, v);
+          tmem_ld16_sum(trow + ch * 16, TMEM_SMALL, v);
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + s_bias[ch * 16 + i] + row_on * s_v1[ch * 16 + i], 0.f);
 #pragma unroll
@@ -650,7 +495,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
       const int ch0 = grp ? kSplit : 0, ch1 = grp ? BNv / 16 : kSplit;
       for (int ch = ch0; ch < ch1; ++ch) {
         float v[16];
-        tmem_ld16_sum(trow + ch * 16, v);
+        tmem_ld16_sum(trow + ch * 16, TMEM_SMALL, v);
         if (EPI == EPI_SCORE) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -683,7 +528,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
-  if ((EPI == EPI_GRU || kMerger) && g.peer.world > 0) {
+  if (EPI == EPI_GRU && g.peer.world > 0) {
     // every CTA (with or without rows) checks out; the last one posts the batch's sequence number to all
     // ranks, after every CTA's peer stores have been fenced system-wide
     __threadfence_system();
@@ -707,7 +552,6 @@ int launch(int epilogue, const Args &a, int n_tiles, cudaStream_t stream) {
   if (c == nullptr) return set_error(ORCA_E_CUDA, "tc::launch: no context for the current device");
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<EPI_BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     ORCA_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<EPI_GRU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     ORCA_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<EPI_SCORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     ORCA_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<EPI_MERGER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -721,7 +565,6 @@ int launch(int epilogue, const Args &a, int n_tiles, cudaStream_t stream) {
   // count (m_cap is a capacity) leave at once
   dim3 grid(n_tiles, std::min(ceil_div(a.m_cap, BM), std::max(1, c->sm_count / n_tiles)), 1);
   switch (epilogue) {
-    case EPI_BIAS: ORCA_CUDA(launch_dep(tc_gemm_kernel<EPI_BIAS>, grid, THREADS, SMEM_BYTES, stream, b)); break;
     case EPI_GRU: ORCA_CUDA(launch_dep(tc_gemm_kernel<EPI_GRU>, grid, THREADS, SMEM_BYTES, stream, b)); break;
     case EPI_SCORE: ORCA_CUDA(launch_dep(tc_gemm_kernel<EPI_SCORE>, grid, THREADS, SMEM_BYTES, stream, b)); break;
     case EPI_MERGER:

@@ -38,6 +38,9 @@ constexpr int TMEM_SMALL = 256;
 constexpr int TILE_LD = 180;     // floats per row of the epilogue's output tile: 16-byte row-wise stores of a
                                  // warp (one row per lane) then spread over all banks
 
+constexpr int GRU_PART = 176;    // the memory update's K is laid out in five parts of 172 columns padded to 176 (11 MMA steps)
+constexpr int GRU_K = 5 * GRU_PART;
+
 // A logical A row is the concatenation of up to two gathered table rows
 struct RowSrc {
   const float *p;      // table base, row stride = width floats
@@ -45,9 +48,13 @@ struct RowSrc {
   int width;
   int mod;
   int add;
+  // optional second table: rows >= split are read from p2, whose address is already moved back by split rows
+  const float *p2 = nullptr;
+  int split = 0;
+  __device__ const float *base(int r) const { return p2 != nullptr && r >= split ? p2 : p; }
 };
 
-// LAYERNORM / GRU epilogue that also delivers the rows to the other GPUs of the node (the exchange of the
+// LayerNorm / GRU epilogue that also delivers the rows to the other GPUs of the node (the exchange of the
 // multi-GPU split): row m goes to rows[q] + off + m * 172 floats for every rank q (peer stores over
 // NVLink; the own buffer is one of them), and the last CTA to finish posts `seq` in word `rank` of every
 // rank's flag array.  counter: a zeroed word of the own flag array.
@@ -60,9 +67,10 @@ struct PeerOut {
 };
 
 // EPI_MERGER: hidden = relu(A . W + bias + valid * bias2) kept on the SM, then LayerNorm(hidden . W2 + bias_out)
-// with the LayerNorm epilogue (push, peer fan-out).  EPI_LAYERNORM names that epilogue inside the kernel; it
-// is not a kernel of its own (values 1 and 2 were the two separate kernels the merger replaced).
-enum Epilogue { EPI_BIAS = 0, EPI_LAYERNORM = 2, EPI_GRU = 3, EPI_SCORE = 4, EPI_MERGER = 5 };
+// with the LayerNorm epilogue (push); serves orca_attn_output, whose rows come as floats (the batch entry points use
+// attn_out.cu).  EPI_LAYERNORM names that epilogue inside the kernel; it
+// is not a kernel of its own.
+enum Epilogue { EPI_LAYERNORM = 2, EPI_GRU = 3, EPI_SCORE = 4, EPI_MERGER = 5 };
 
 struct Args {
   RowSrc a0, a1;             // a1.width == 0 when unused
@@ -77,8 +85,7 @@ struct Args {
   // a1.idx, nodes; idx_limit entries) and d_m counts the entries of the whole lists; row_stride <= 1: off
   int row_stride, row_off, idx_limit;
   const float *bias;         // [n_tiles * BN]
-  float *out;                // BIAS: [m, out_ld]; HIDDEN / LAYERNORM: [m, 172]; GRU: [m, 172]; SCORE: [m]
-  int out_ld;
+  float *out;                // MERGER, GRU: [m, 172]; SCORE: [m]
   // MERGER, first product: + valid * bias2; second product: packed weights (3 k-blocks) and bias
   const float *bias2;
   const void *w2_packed;
@@ -87,13 +94,12 @@ struct Args {
   const float *ln_w, *ln_b;
   float *push_table;
   const int32_t *push_ids;
-  const uint8_t *push_win;                  // winners by flag, or (push_win == nullptr) by record:
-  const unsigned long long *push_last_pos;  // row m wins if m >= push_all_from or
-  long long push_base;                      // push_last_pos[push_ids[m]] == push_base + m
-  int push_all_from;
+  const uint8_t *push_win;
   // GRU
   const float *memory;
   const int32_t *nodes;
+  const float *memory2;      // optional: rows >= memory_split (as in RowSrc)
+  int memory_split;
   // SCORE
   const float *w2;
   float b2;
@@ -112,7 +118,13 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
                      const int32_t *d_idx, int32_t n_rows_cap, const int32_t *d_n_rows, float *d_out,
                      float *d_push_table, const int32_t *d_push_ids, const uint8_t *d_push_win,
                      const int64_t *d_last_pos, long long base, int all_from, float *d_scratch_hidden,
-                     int rows_hint, cudaStream_t stream, const tc::PeerOut *peer = nullptr);
+                     cudaStream_t stream);
+// scorer and GRU over the rows of a group of batches (gemm.cu); tensor cores only
+int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
+               float *d_prob, cudaStream_t s);
+int gru_project_rows(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
+                     const int32_t *d_mem_rows, const float *mem2, int mem_split, int n_cap, const int32_t *d_n,
+                     float *d_out, cudaStream_t s);
 // whether the projections run on the tensor cores (orca_set_projection_mode(0)); the fp32 debug path has
 // no peer fan-out
 bool projections_on_tensor_cores();

@@ -107,14 +107,17 @@ class GRUMemoryUpdater(nn.Module):
         if self._prepared is None:
             sd = {"memory_updater.memory_updater." + k: v.detach().cpu().numpy()
                   for k, v in self.memory_updater.state_dict().items()}
-            w = weights.prepare_gru(sd)
+            w = weights.prepare_gru(sd, pack=False)
             dev = self.memory_updater.weight_ih.device
-            self._prepared = {k: torch.from_numpy(v).to(dev) for k, v in w.items()}
+            w = {k: torch.from_numpy(v).to(dev) for k, v in w.items()}
+            w["Wg_tc"], w["Wg_chain"] = weights.pack_gru(w["Wg"])
+            self._prepared = w
         return self._prepared
 
     def c_struct(self):
         p = self.prepared()
-        return _lib.GruWeights(p["Wg"].data_ptr(), p["bg"].data_ptr(), p["Wg_tc"].data_ptr())
+        return _lib.GruWeights(p["Wg"].data_ptr(), p["bg"].data_ptr(), p["Wg_tc"].data_ptr(),
+                               p["Wg_chain"].data_ptr())
 
     def _run(self, memory: Memory, ids: torch.Tensor, clear: bool):
         n = ids.numel()

@@ -205,6 +205,7 @@ class TGN(nn.Module):
             ctx = C.c_void_p(0)
             _lib.check(_lib.lib().orca_ctx_create(C.byref(ctx)))
         self._ctx = ctx
+        self._options = {}             # what set_option has set
         self._input_stream = None      # stream the batch inputs are made ready on (None: the current stream)
         # candidate bitmap of the uncached set, followed by the candidate list (length word + entries)
         self._cand_bitmap = torch.zeros((self.n_nodes + 31) // 32 + 1 + _lib.CAND_CAP, dtype=torch.int32,
@@ -233,6 +234,7 @@ class TGN(nn.Module):
         """Switch of this model's context (_lib.OPT_*: projection mode, overlap, dependent launch,
         look-ahead, wait limit, trace)."""
         _lib.check(_lib.lib().orca_ctx_set(self._ctx, int(option), int(value)))
+        self._options[int(option)] = int(value)
 
     def last_layer1_nodes(self, n_rows):
         """Node ids of the last batch's layer-1 row list [src | dst | neg | uncached] (its first n_rows
@@ -368,9 +370,11 @@ class TGN(nn.Module):
             up = lambda d: {k: (torch.from_numpy(v).to(dev) if isinstance(v, np.ndarray) else v) for k, v in d.items()}
             self._prepared = {
                 "time_w": torch.from_numpy(weights.prepare_time(sd)).to(dev),
-                "attn": [up(weights.prepare_attention(sd, l)) for l in range(self.n_layers)],
+                "attn": [up(weights.prepare_attention(sd, l, pack=False)) for l in range(self.n_layers)],
                 "score": up(weights.prepare_score(sd)),
             }
+            for a in self._prepared["attn"]:
+                a.update(weights.packed_attention(a))
         return self._prepared
 
     def attn_struct(self, layer):
@@ -667,6 +671,12 @@ class TGN(nn.Module):
         if self._mode != MODE_BUDGET:
             cache_plan = None
         world, rank = self._world, self._rank
+        # Groups of batches on one GPU; one batch after the other where a batch's work depends on the one before in
+        # full (flags without a plan accumulate), in the debug modes and when the batch is split over GPUs
+        if world == 1 and (cache_plan is not None or self._mode != MODE_BUDGET or self.n_layers == 1) and \
+                not any(self._options.get(o) for o in (_lib.OPT_PROJECTION_MODE, _lib.OPT_TRACE)):
+            return self._eval_groups(sources, destinations, negatives, timestamps, edge_idxs, k, bs,
+                                     cache_plan if self.n_layers == 2 else None)
         if world > 1 and getattr(self, "_exchange", None) is None:
             raise NotImplementedError("eval_epoch on several GPUs needs the direct exchange (set_distributed)")
         b = np.full(nb, bs, dtype=np.int32)
@@ -781,6 +791,77 @@ class TGN(nn.Module):
                 neg[lo + r:lo + int(b[i]):wb] = every[wa + r, o + n:o + 2 * n]
                 o += 2 * n
         return pos, neg
+
+    def _eval_groups(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan):
+        """eval_epoch in groups of consecutive batches (orca_tgn_eval_group)."""
+        L = _lib.lib()
+        E = len(sources)
+        nb = (E + bs - 1) // bs
+        mode = self._mode if self.n_layers == 2 else MODE_BUDGET
+        budget = self.n_layers == 2 and mode == MODE_BUDGET
+        n_plan = np.zeros(nb, dtype=np.int32)
+        if cache_plan is not None:
+            n_plan[:] = [len(cache_plan[i]) for i in range(nb)]
+        most = int(n_plan.max())
+        if budget:
+            h = self.embedding_module.histories[0]
+            if most > h.prev_plan.numel():
+                h.prev_plan = torch.zeros(most, dtype=torch.int32, device=self.device)
+                h.n_prev[0] = -1
+        keep = self.__dict__.setdefault("_group_buffers", {})
+        u_cap = min(3 * bs * k, self.n_nodes) if budget else 0
+        nb_max = min(L.orca_group_size(bs, k, self.n_layers, mode), nb)
+        shape = (bs, k, u_cap, self.n_layers, mode, self.n_nodes)
+        if keep.get("shape") != shape or keep["nb_max"] < nb_max or keep["plan_cap"] < most:
+            if keep.get("shape") == shape:
+                nb_max, most = max(nb_max, keep["nb_max"]), max(most, keep["plan_cap"])
+            nbytes = L.orca_group_workspace_bytes(bs, nb_max, k, u_cap, most, self.n_nodes, self.n_layers, mode)
+            if keep.get("ws") is None or keep["ws"].numel() < nbytes:
+                keep["ws"] = None         # (an epoch ends with a synchronisation: nothing is using the old one)
+                keep["ws"] = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            keep.update(shape=shape, nb_max=nb_max, plan_cap=most)
+        nb_max, plan_cap, ws = keep["nb_max"], keep["plan_cap"], keep["ws"]
+
+        def pinned(name, n, dtype):
+            t = keep.get(name)
+            if t is None or t.numel() < n:
+                t = keep[name] = torch.empty(max(n, 1), dtype=dtype, pin_memory=True)
+            return t
+
+        off = np.zeros(nb + 1, dtype=np.int64)
+        off[1:] = np.cumsum(4 * np.minimum(bs, E - bs * np.arange(nb)) + n_plan)
+        h_i32, h_ts, h_prob = (pinned("i32", int(off[-1]), torch.int32), pinned("ts", E, torch.float64),
+                               pinned("prob", 2 * E, torch.float32))
+        if keep.get("d_prob") is None or keep["d_prob"].numel() < 2 * E:
+            keep["d_prob"] = torch.empty(2 * E, dtype=torch.float32, device=self.device)
+        hi, hts, d_prob = h_i32.numpy(), h_ts.numpy(), keep["d_prob"]
+        desc = self._descriptor(k)
+        stream = torch.cuda.current_stream(self.device)
+        # the library never waits for the host: while the GPU works on a group the next one is packed
+        for i0 in range(0, nb, nb_max):
+            i1 = min(nb, i0 + nb_max)
+            lo, up = i0 * bs, min(E, i1 * bs)
+            hts[lo:up] = timestamps[lo:up]
+            for i in range(i0, i1):
+                a, b = i * bs, min(E, (i + 1) * bs)
+                n, o = b - a, int(off[i])
+                hi[o:o + n] = sources[a:b]
+                hi[o + n:o + 2 * n] = destinations[a:b]
+                hi[o + 2 * n:o + 3 * n] = negatives[a:b]
+                hi[o + 3 * n:o + 4 * n] = edge_idxs[a:b]
+                if n_plan[i]:
+                    hi[o + 4 * n:off[i + 1]] = cache_plan[i]
+            g = _lib.GroupT(h_i32.data_ptr(), h_ts.data_ptr() + 8 * lo, off.ctypes.data + 8 * i0, n_plan.ctypes.data + 4 * i0,
+                            i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap, i0 == 0)
+            _lib.check(L.orca_tgn_eval_group(desc, C.byref(g), ws.data_ptr(), ws.numel(), d_prob.data_ptr() + 8 * lo,
+                                             h_prob.data_ptr() + 8 * lo, self._status.data_ptr(), stream.cuda_stream))
+        stream.synchronize()
+        # per batch [pos | neg]; the last batch may be short
+        scores, full = h_prob.numpy()[:2 * E], E // bs
+        out = np.empty((2, E), dtype=np.float32)
+        out[:, :full * bs].reshape(2, full, bs)[:] = scores[:2 * full * bs].reshape(full, 2, bs).transpose(1, 0, 2)
+        out[:, full * bs:] = scores[2 * full * bs:].reshape(2, -1)
+        return out[0], out[1]
 
     def update_memory(self, memory, positives):
         self.memory_updater.update_memory(memory, positives)

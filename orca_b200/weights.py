@@ -18,17 +18,30 @@ from __future__ import annotations
 import math
 
 import numpy as np
+import torch
 
 D = 172
 HEADS = 2
 QT_HEAD = 528     # column stride of one head of the projected query (516 used)
 TC_BN, TC_BK = 176, 64
+GRU_PART, CHAIN_N = 176, 32
 
 
-def _bf16_round(x):
-    """float32 -> nearest bfloat16 (ties to even), returned as float32 with the low 16 bits zero."""
-    u = np.ascontiguousarray(x, dtype=np.float32).view(np.uint32).astype(np.uint64)
-    return ((u + 0x7FFF + ((u >> 16) & 1)) & 0xFFFF0000).astype(np.uint32).view(np.float32)
+def _packed(W, shape, image):
+    """Operand images of a matrix (or of matrices one below the other): heads and tails of the float32 values, each
+    zero padded into `shape` and rearranged by `image`, stacked behind image dimension 0 or where `image` says.  head =
+    the value rounded to bf16, tail = the remainder rounded to bf16 (16 significant bits together).  Runs where W lives:
+    a torch tensor on the GPU is packed there (the host's rearranging takes 10 ms a model)."""
+    parts = W if isinstance(W, (list, tuple)) else [(W, 0)]
+    host = not isinstance(parts[0][0], torch.Tensor)
+    parts = [(torch.as_tensor(np.ascontiguousarray(p, dtype=np.float32)) if host else p.float(), at) for p, at in parts]
+    P = torch.zeros(shape, dtype=torch.float32, device=parts[0][0].device)
+    for p, at in parts:
+        P[at:at + p.shape[0], :p.shape[1]] = p
+    head = P.to(torch.bfloat16)
+    tail = (P - head.float()).to(torch.bfloat16)
+    out = image(torch.stack([head, tail]).view(torch.int16)).contiguous()
+    return out.numpy().view(np.uint16) if host else out
 
 
 def pack_tc(W, bn=None):
@@ -38,29 +51,55 @@ def pack_tc(W, bn=None):
     One (tile, block) stage image is [head | tail], each [8 chunks][bn columns][8 bf16]: element
     (k, n) of the block sits at chunk k // 8, column n, position k % 8 -- the K-major, no-swizzle
     core-matrix layout the MMA reads from shared memory -- so that a stage is one contiguous bulk
-    copy.  head = the value rounded to bf16, tail = the remainder rounded to bf16 (16 significant
-    bits together).  Returned as uint16 [n_tiles, n_kblocks, 2, 8, bn, 8]."""
-    W = np.asarray(W, dtype=np.float32)
+    copy.  Returned as uint16 [n_tiles, n_kblocks, 2, 8, bn, 8]."""
     K, N = W.shape
     bn = bn or TC_BN
     nkb, nt = -(-K // TC_BK), -(-N // bn)
-    P = np.zeros((nkb * TC_BK, nt * bn), dtype=np.float32)
-    P[:K, :N] = W
-    head = _bf16_round(P)
-    tail = _bf16_round(P - head)
+    return _packed(W, (nkb * TC_BK, nt * bn),
+                   lambda X: X.reshape(2, nkb, TC_BK // 8, 8, nt, bn).permute(4, 1, 0, 2, 5, 3))
 
-    def image(X):  # [nkb*64, nt*176] -> [nt, nkb, 8, 176, 8] of bf16 bit patterns
-        bits = (X.view(np.uint32) >> 16).astype(np.uint16)
-        return bits.reshape(nkb, TC_BK // 8, 8, nt, bn).transpose(3, 0, 1, 4, 2)
 
-    return np.ascontiguousarray(np.stack([image(head), image(tail)], axis=2))
+def pack_query(W, bn):
+    """Query weights [172, 1056] for csrc/attn_query.cu: K padded to 176, one image per bn columns, each
+    [head | tail][K / 8][bn columns][8]: uint16 [1056 / bn, 2, 22, bn, 8]."""
+    return _packed(W, (GRU_PART, W.shape[1]),
+                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, bn).permute(3, 0, 1, 4, 2))
+
+
+def pack_stages(*parts):
+    """Weights with 172 columns for csrc/attn_out.cu: the parts one below the other, each padded to a multiple of 32
+    rows; one stage per 32 rows, each [head | tail][4 chunks][176 columns][8]."""
+    at = np.cumsum([0] + [-(-len(p) // 32) * 32 for p in parts])
+    return _packed(list(zip(parts, at[:-1])), (int(at[-1]), TC_BN),
+                   lambda X: X.reshape(2, -1, 4, 8, TC_BN).permute(1, 0, 2, 4, 3))
+
+
+def pack_gru(Wg, dim=D):
+    """Memory-update weights [860, 688] for the tensor-core kernels, which read K in five parts of 172 rows, each padded
+    to 176: what does not depend on the batch before comes first (csrc/chain.cu) -- edge features, time encoding, own
+    memory, other memory, memory.  Returned for csrc/tc_gemm.cu (pack_tc) and as one image per 32 gate columns (eight
+    units) for csrc/chain.cu, each [head | tail][K / 8][32 columns][8]."""
+    part = [(Wg[at * dim:(at + 1) * dim], to * GRU_PART) for to, at in enumerate((2, 3, 0, 1, 4))]
+    K, N = 5 * GRU_PART, Wg.shape[1]
+    nkb, nt, nc = -(-K // TC_BK), -(-N // TC_BN), -(-N // CHAIN_N)
+    return (_packed(part, (nkb * TC_BK, nt * TC_BN),
+                    lambda X: X.reshape(2, nkb, TC_BK // 8, 8, nt, TC_BN).permute(4, 1, 0, 2, 5, 3)),
+            _packed(part, (K, nc * CHAIN_N), lambda X: X.reshape(2, -1, 8, nc, CHAIN_N).permute(3, 0, 1, 4, 2)))
+
+
+def packed_attention(w):
+    """The operand images that go with prepare_attention's matrices (numpy arrays or tensors)."""
+    kd2 = w["G"].shape[0] - w["Mq"].shape[0]
+    return {"G_tc": pack_tc(w["G"]), "W2t_tc": pack_tc(w["W2t"]), "Mq_tc": pack_query(w["Mq"], 96),
+            "Mq_img": pack_query(w["Mq"], TC_BN), "G_img": pack_stages(w["G"][:kd2], w["G"][kd2:]),
+            "W2_img": pack_stages(w["W2t"])}
 
 
 def _f64(x):
     return np.asarray(x, dtype=np.float64)
 
 
-def prepare_attention(sd, layer: int, dim: int = D, heads: int = HEADS):
+def prepare_attention(sd, layer: int, dim: int = D, heads: int = HEADS, pack: bool = True):
     p = f"embedding_module.attention_models.{layer}."
     Wq = _f64(sd[p + "multi_head_target.q_proj_weight"])
     Wk = _f64(sd[p + "multi_head_target.k_proj_weight"])
@@ -97,12 +136,12 @@ def prepare_attention(sd, layer: int, dim: int = D, heads: int = HEADS):
         "ln_w": _f64(sd[p + "norm.weight"]), "ln_b": _f64(sd[p + "norm.bias"]),
     }
     out = {k: np.ascontiguousarray(v, dtype=np.float32) for k, v in out.items()}
-    for k in ("Mq", "G", "W2t"):
-        out[k + "_tc"] = pack_tc(out[k])
+    if pack:
+        out.update(packed_attention(out))
     return out
 
 
-def prepare_gru(sd, dim: int = D):
+def prepare_gru(sd, dim: int = D, pack: bool = True):
     p = "memory_updater.memory_updater."
     Wih, Whh = _f64(sd[p + "weight_ih"]), _f64(sd[p + "weight_hh"])
     bih, bhh = _f64(sd[p + "bias_ih"]), _f64(sd[p + "bias_hh"])
@@ -124,7 +163,10 @@ def prepare_gru(sd, dim: int = D):
     Wg = np.ascontiguousarray(Wg, dtype=np.float32)
     bg_pad = np.zeros(4 * TC_BN, dtype=np.float32)
     bg_pad[:4 * dim] = bg
-    return {"Wg": Wg, "bg": bg_pad, "Wg_tc": pack_tc(Wg)}
+    out = {"Wg": Wg, "bg": bg_pad}
+    if pack:
+        out["Wg_tc"], out["Wg_chain"] = pack_gru(Wg)
+    return out
 
 
 def prepare_score(sd):

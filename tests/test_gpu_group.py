@@ -1,0 +1,66 @@
+"""Groups of batches (TGN.eval_epoch on one GPU) against one call per batch: the same bits in the scores and in every
+state table, for each recursion, for batch sizes from one edge to more than a tile, for streams that end inside a
+group, at a group's last batch and with a short batch, and for a second epoch on the same buffers."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import graph
+from orca_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(g, bs, k, budget, strategy, E):
+    import argparse
+    import types
+    from orca_b200.cache import get_cache_plan
+    from orca_b200.neighbor_finder import get_neighbor_finder
+    nf = get_neighbor_finder(g)
+    data = types.SimpleNamespace(sources=g.sources[:E], destinations=g.destinations[:E], timestamps=g.timestamps[:E])
+    return get_cache_plan(argparse.Namespace(bs=bs, n_degree=k, budget=budget), data, nf, g.n_nodes, strategy)
+
+
+# (graph, batch size, k, edges, recursion, layers)
+CASES = [("t_nb2", 37, 10, 5011, "budget", 2),       # 136 batches: five groups, the last one short
+         ("t_bip2", 64, 5, 64 * 64, "budget", 2),    # two full groups
+         ("t_2q", 1, 10, 70, "budget", 2),           # one edge a batch
+         ("t_lru", 300, 20, 5999, "budget", 2),      # k above 16; more rows than a tile of either kernel
+         ("t_nb2", 1500, 3, 5000, "budget", 2),      # three batches and a bit
+         ("t_nb2", 50, 10, 2030, "all", 2),          # unlimited reuse
+         ("t_nb2", 50, 10, 2030, "none", 2),         # no reuse: a layer-1 row per sampled neighbour
+         ("t_lru", 33, 20, 700, "none", 2),
+         ("c1", 129, 10, 6000, "budget", 1)]
+
+
+@pytest.mark.parametrize("name,bs,k,E,recursion,layers", CASES)
+def test_group_equals_batches(name, bs, k, E, recursion, layers):
+    import dataclasses
+    from test_gpu_model import make_model
+    g = graph(name)
+    budget = 0 if recursion == "all" else g.spec.budget
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs, n_degree=k, n_layers=layers, budget=budget))
+    neg = synthetic.negative_destinations(g, seed=1)
+    plan = _plan(g, bs, k, g.spec.budget, g.spec.strategy, E) if recursion == "budget" else None
+    a, b = make_model(g), make_model(g)
+    reuse = recursion != "none"
+    nb = -(-E // bs)
+    for epoch in range(2):
+        pos, ngs = [], []
+        for i in range(nb):
+            sl = slice(i * bs, min(E, (i + 1) * bs))
+            p, q = a.compute_edge_probabilities(g.sources[sl], g.destinations[sl], neg[sl], g.timestamps[sl],
+                                                g.edge_idxs[sl], k, reuse, False, plan[i] if plan else None)
+            pos.append(p.cpu().numpy().ravel()), ngs.append(q.cpu().numpy().ravel())
+        ca = a.check_status()
+        p2, q2 = b.eval_epoch(g.sources[:E], g.destinations[:E], neg[:E], g.timestamps[:E], g.edge_idxs[:E], k, bs, plan,
+                              reuse=reuse)
+        cb = b.check_status()
+        assert np.array_equal(np.concatenate(pos), p2) and np.array_equal(np.concatenate(ngs), q2), epoch
+        if recursion == "budget" and layers == 2:
+            assert ca[:2] == cb[:2]
+        for t in ("memory", "last_update", "messages", "timestamps", "nodes_dev"):
+            assert torch.equal(getattr(a.memory, t), getattr(b.memory, t)), (epoch, t)
+        if layers == 2:
+            ha, hb = a.embedding_module.histories[0], b.embedding_module.histories[0]
+            assert torch.equal(ha.emb, hb.emb) and torch.equal(ha.cache_flag_dev, hb.cache_flag_dev)
