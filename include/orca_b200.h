@@ -542,6 +542,22 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
                         int32_t *d_status, void *stream);
 
 /* ------------------------------------------------------------------------------------------
+ * One batch from host arrays (one GPU): orca_tgn_eval_batch with its inputs narrowed into a ring of ORCA_CALL_SLOTS
+ * page-locked slots and copied from there on the context's copy stream.  Waits only when the ring is full.  The status
+ * word follows the batch to h_status (page-locked) in `stream` order.
+ */
+#define ORCA_CALL_SLOTS 8
+typedef struct {
+  const int64_t *src, *dst, *neg, *eidx, *plan;
+  const double *ts;
+  int32_t b, n_plan;          /* n_plan < 0: no plan */
+  void *h_ring, *d_ring;      /* ORCA_CALL_SLOTS slots each, page-locked host memory / device memory */
+  int64_t slot_bytes;         /* a slot holds 16 * b + 4 * n_plan (rounded up to 16) + 8 * b bytes; multiple of 256 */
+} orca_call_t;
+int orca_tgn_call(const orca_tgn_t *m, const orca_call_t *a, int32_t u_cap, void *d_workspace, int64_t workspace_bytes,
+                  float *d_prob, float *d_emb_out, int32_t *d_status, int32_t *h_status, void *stream);
+
+/* ------------------------------------------------------------------------------------------
  * A group of consecutive batches of a stream as one unit of work (one GPU, tensor-core projections; with the
  * budgeted recursion every batch needs a plan).  Results and state tables are those of the batches one by one, bit
  * for bit.  Enqueues the copies of the group's inputs (pinned host memory, laid out as in orca_epoch_t), its kernels

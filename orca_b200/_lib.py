@@ -80,6 +80,14 @@ class EpochT(C.Structure):
                 ("off_prob", C.c_void_p), ("b", C.c_void_p), ("n_plan", C.c_void_p), ("n_batches", C.c_int64)]
 
 
+CALL_SLOTS = 8      # ORCA_CALL_SLOTS
+
+
+class CallT(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("src", "dst", "neg", "eidx", "plan", "ts")] + \
+        [("b", C.c_int32), ("n_plan", C.c_int32), ("h_ring", C.c_void_p), ("d_ring", C.c_void_p), ("slot_bytes", C.c_int64)]
+
+
 class GroupT(C.Structure):
     _fields_ = [("h_i32", C.c_void_p), ("h_ts", C.c_void_p), ("off_i32", C.c_void_p), ("n_plan", C.c_void_p)] + \
         [(n, C.c_int32) for n in ("nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap", "first")]
@@ -133,6 +141,7 @@ SYMBOLS = {
     "orca_tgn_eval_batch_sharded": (C.c_int, [C.POINTER(TgnT), _I32, _V, _V, _I32, _V, _I32, _I32, _V, _I64, _V, _V,
                                               _V, _V, _V, _V]),
     "orca_tgn_eval_epoch": (C.c_int, [C.POINTER(TgnT), C.POINTER(EpochT), _I32, _V, _I64, _V, _I64, _V, _V, _V, _V]),
+    "orca_tgn_call": (C.c_int, [C.POINTER(TgnT), C.POINTER(CallT), _I32, _V, _I64, _V, _V, _V, _V, _V]),
     "orca_group_size": (_I32, [_I32, _I32, _I32, _I32]),
     "orca_group_workspace_bytes": (_I64, [_I32, _I32, _I32, _I32, _I32, _I64, _I32, _I32]),
     "orca_tgn_eval_group": (C.c_int, [C.POINTER(TgnT), C.POINTER(GroupT), _V, _I64, _V, _V, _V, _V]),

@@ -18,6 +18,7 @@ static int create_ctx(Ctx **out) {
   ORCA_CUDA(cudaStreamCreateWithFlags(&c->lane1, cudaStreamNonBlocking));
   ORCA_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
   for (int q = 0; q < Ctx::kStageSlots; ++q) ORCA_CUDA(cudaEventCreateWithFlags(&c->ev_slot[q], cudaEventDisableTiming));
+  for (cudaEvent_t &e : c->ev_call) ORCA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   cudaEvent_t *evs[] = {&c->fork, &c->join, &c->ev_in, &c->ev_flags, &c->ev_o1, &c->ev_g2, &c->ev_state,
                         &c->ev_idx[0], &c->ev_idx[1], &c->ev_done[0], &c->ev_done[1], &c->ev_gin, &c->ev_gidx[0],
                         &c->ev_gidx[1], &c->ev_gchain[0], &c->ev_gchain[1], &c->ev_gdone[0], &c->ev_gdone[1]};
@@ -38,6 +39,8 @@ static void destroy_ctx(Ctx *c) {
   if (c->lane1) cudaStreamSynchronize(c->lane1);
   if (c->copy) cudaStreamSynchronize(c->copy);
   for (cudaEvent_t e : c->ev_slot)
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : c->ev_call)
     if (e) cudaEventDestroy(e);
   cudaEvent_t evs[] = {c->fork, c->join, c->ev_in, c->ev_flags, c->ev_o1, c->ev_g2, c->ev_state, c->ev_idx[0],
                        c->ev_idx[1], c->ev_done[0], c->ev_done[1], c->ev_gin, c->ev_gidx[0], c->ev_gidx[1],

@@ -50,6 +50,11 @@ struct Ctx {
   cudaEvent_t ev_slot[kStageSlots] = {nullptr, nullptr, nullptr, nullptr};
   bool slot_used[kStageSlots] = {false, false, false, false};
   long long stage_seq = 0;
+  // calls with host arrays (orca_tgn_call): one pinned and one device slot per call in flight
+  static constexpr int kCallSlots = 8;
+  cudaEvent_t ev_call[kCallSlots] = {};
+  bool call_used[kCallSlots] = {};
+  long long call_seq = 0;
   cudaEvent_t fork = nullptr, join = nullptr, ev_in = nullptr, ev_flags = nullptr;
   cudaEvent_t ev_o1 = nullptr, ev_g2 = nullptr, ev_state = nullptr;
   cudaEvent_t ev_idx[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr};

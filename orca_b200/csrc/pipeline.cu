@@ -960,6 +960,43 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
   return ORCA_OK;
 }
 
+// The whole of one call with host arrays: narrowed into the call's pinned slot, copied on the copy stream, computed, the
+// status word on its way back.  (As a dozen of torch calls this took 50 us of host time, half of a small call.)
+int orca_tgn_call(const orca_tgn_t *m, const orca_call_t *a, int32_t u_cap, void *d_workspace, int64_t workspace_bytes,
+                  float *d_prob, float *d_emb_out, int32_t *d_status, int32_t *h_status, void *stream) {
+  ORCA_CHECK_ARG(m && a && d_prob && d_status && h_status && a->src && a->dst && a->neg && a->eidx && a->ts && a->b > 0 &&
+                 a->h_ring && a->d_ring && m->world <= 1);
+  Ctx *c = ctx_of(m);
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_tgn_call: no context for the current device");
+  cudaStream_t s = (cudaStream_t)stream;
+  const int b = a->b, n_plan = a->n_plan > 0 ? a->n_plan : 0;
+  const int64_t n_i32 = 4ll * b + n_plan, off_ts = (n_i32 * 4 + 15) & ~15ll, bytes = off_ts + 8ll * b;
+  if (bytes > a->slot_bytes)
+    return set_error(ORCA_E_CAPACITY, "orca_tgn_call: slots of %lld bytes, %lld needed", (long long)a->slot_bytes,
+                     (long long)bytes);
+  const int slot = (int)(c->call_seq++ % Ctx::kCallSlots);
+  if (c->call_used[slot]) ORCA_CUDA(cudaEventSynchronize(c->ev_call[slot]));   // (eight calls ahead of the GPU: wait)
+  char *h = (char *)a->h_ring + slot * a->slot_bytes, *d = (char *)a->d_ring + slot * a->slot_bytes;
+  int32_t *o = (int32_t *)h;
+  auto narrow = [&](const int64_t *x, int n) {
+    for (int i = 0; i < n; ++i) o[i] = (int32_t)x[i];
+    o += n;
+  };
+  narrow(a->src, b), narrow(a->dst, b), narrow(a->neg, b), narrow(a->eidx, b);
+  if (n_plan > 0) narrow(a->plan, n_plan);
+  memcpy(h + off_ts, a->ts, (size_t)b * 8);
+  ORCA_CUDA(cudaMemcpyAsync(d, h, (size_t)bytes, cudaMemcpyHostToDevice, c->copy));
+  orca_tgn_t mm = *m;
+  mm.input_stream = c->copy;
+  ORCA_TRY(orca_tgn_eval_batch(&mm, (const int32_t *)d, (const double *)(d + off_ts), b,
+                               a->n_plan >= 0 ? (const int32_t *)d + 4 * (size_t)b : nullptr, n_plan, u_cap, d_workspace,
+                               workspace_bytes, d_prob, d_emb_out, d_status, stream));
+  ORCA_CUDA(cudaMemcpyAsync(h_status, d_status, 16, cudaMemcpyDeviceToHost, s));
+  ORCA_CUDA(cudaEventRecord(c->ev_call[slot], s));
+  c->call_used[slot] = true;
+  return ORCA_OK;
+}
+
 int orca_ipc_export(const void *d_ptr, void *h_handle, int64_t *h_offset) {
   ORCA_CHECK_ARG(d_ptr && h_handle && h_offset);
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "handle size");

@@ -21,6 +21,7 @@ from .memory import Memory, get_memory_updater
 
 # recursion modes of the fused batch entry point (ORCA_MODE_* of the C header)
 MODE_BUDGET, MODE_REUSE_ALL, MODE_NO_REUSE = 0, 1, 2
+_I64 = np.dtype(np.int64)
 
 
 class MergeLayer(nn.Module):
@@ -206,6 +207,7 @@ class TGN(nn.Module):
             _lib.check(_lib.lib().orca_ctx_create(C.byref(ctx)))
         self._ctx = ctx
         self._options = {}             # what set_option has set
+        self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self._input_stream = None      # stream the batch inputs are made ready on (None: the current stream)
         # candidate bitmap of the uncached set, followed by the candidate list (length word + entries)
         self._cand_bitmap = torch.zeros((self.n_nodes + 31) // 32 + 1 + _lib.CAND_CAP, dtype=torch.int32,
@@ -395,24 +397,31 @@ class TGN(nn.Module):
         """The model descriptor of the fused batch entry.  Graph, weights and scratch pointers are filled
         once per (neighbour finder, prepared weights, k); the state tables can be replaced between calls
         (restore_memory, restore_history) and are refreshed every time."""
-        nf = self.embedding_module.neighbor_finder
+        d, mods = self.__dict__, self._modules        # (plain look-ups: this runs once per batch)
+        em = mods["embedding_module"].__dict__
+        nf = em["neighbor_finder"]
         w = self._weights()
-        gw = self.memory_updater.prepared()
-        ref = getattr(self, "_desc_ref", None)   # the objects themselves are kept: identities cannot be reused
+        gw = mods["memory_updater"].prepared()
+        ref = d.get("_desc_ref")                      # the objects themselves are kept: identities cannot be reused
         if ref is not None and ref[0] is nf and ref[1] is w and ref[2] is gw and ref[3] == k:
-            t = self._desc
-            t.mem = self.memory.c_struct()
-            if self.n_layers == 2 and hasattr(self.embedding_module, "histories"):
-                h = self.embedding_module.histories[0]
-                t.hist_emb = h.emb.data_ptr()
-                t.cache_flag = h.cache_flag_dev.data_ptr()
-                t.prev_plan = h.prev_plan.data_ptr()
-                t.n_prev_plan = h.n_prev.ctypes.data_as(C.POINTER(C.c_int32))
-                t.plan_cap = h.prev_plan.numel()
-            t.rank, t.world = self._rank, self._world
-            t.layer1_ranks = self._layer1_ranks
-            t.mode = self._mode
-            t.input_stream = self._input_stream
+            t, m, tm = d["_desc"], mods["memory"].__dict__, d["_desc_mem"]
+            tm.memory, tm.last_update, tm.messages = (m["memory"].data_ptr(), m["last_update"].data_ptr(),
+                                                      m["messages"].data_ptr())
+            tm.msg_ts, tm.msg_flag = m["timestamps"].data_ptr(), m["nodes_dev"].data_ptr()
+            hist = mods["embedding_module"]._modules.get("histories") if self.n_layers == 2 else None
+            if hist is not None:
+                h = hist[0].__dict__
+                t.hist_emb = h["emb"].data_ptr()
+                t.cache_flag = h["cache_flag_dev"].data_ptr()
+                t.prev_plan = h["prev_plan"].data_ptr()
+                if d.get("_desc_n_prev") is not h["n_prev"]:
+                    d["_desc_n_prev"] = h["n_prev"]
+                    t.n_prev_plan = h["n_prev"].ctypes.data_as(C.POINTER(C.c_int32))
+                t.plan_cap = h["prev_plan"].numel()
+            t.rank, t.world = d["_rank"], d["_world"]
+            t.layer1_ranks = d["_layer1_ranks"]
+            t.mode = d["_mode"]
+            t.input_stream = d["_input_stream"]
             return t
         t = _lib.TgnT()
         if getattr(self, "_exchange", None) is not None:
@@ -425,7 +434,7 @@ class TGN(nn.Module):
             t.exchange_cap = cap
             t.gru_cap = gcap if grus else 0
             t.exchange_seq = self._exchange_seq.ctypes.data_as(C.POINTER(C.c_int64))
-        self._desc_ref, self._desc = (nf, w, gw, k), t
+        d["_desc_ref"], d["_desc"], d["_desc_mem"], d["_desc_n_prev"] = (nf, w, gw, k), t, t.mem, None
         t.indptr, t.adj_nbr, t.adj_eid, t.adj_ts = (nf.indptr.data_ptr(), nf.adj_nbr.data_ptr(),
                                                     nf.adj_eid.data_ptr(), nf.adj_ts.data_ptr())
         t.edge_table = self.edge_raw_features.data_ptr()
@@ -463,7 +472,7 @@ class TGN(nn.Module):
         if self.n_layers == 2 and self._mode == MODE_NO_REUSE:
             u_cap = 3 * b * k          # one layer-1 row per neighbour slot
         key = (b, u_cap, k)
-        if self._ws_key != key:
+        if self.__dict__["_ws_key"] != key:
             # the workspace layout follows (b, u_cap, k): batches of another size get a workspace of their own
             # (kept, so that a stream whose last batch is short does not reallocate twice); the library's
             # side streams may still be reading the old one, hence the synchronisation
@@ -492,6 +501,61 @@ class TGN(nn.Module):
                 h.prev_plan = torch.zeros(len(cache_plan), dtype=torch.int32, device=self.device)
                 h.n_prev[0] = -1
         n_plan = len(cache_plan) if cache_plan is not None else 0
+        if self._world > 1:
+            return self._eval_batch_staged(source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs, k,
+                                           cache_plan, n_plan, want_emb)
+        # One library call: the host arrays are narrowed into a ring of pinned slots, copied and worked on there.
+        # (Host time per call is what bounds a small batch: plain attribute access and no torch call that can be
+        # left out.)
+        d = self.__dict__
+        host = [a if type(a) is np.ndarray and a.dtype == _I64 and a.flags.c_contiguous else np.ascontiguousarray(a, dtype=_I64)
+                for a in (source_nodes, destination_nodes, negative_nodes, edge_idxs)]
+        ts = np.ascontiguousarray(edge_times, dtype=np.float64)
+        if not b == len(host[1]) == len(host[2]) == len(host[3]) == len(ts):
+            raise ValueError("the arrays of a batch must have one length")
+        pl = np.ascontiguousarray(cache_plan, dtype=_I64) if n_plan else None
+        need = 24 * b + 4 * n_plan + 16
+        ring = d.get("_call_ring")
+        if ring is None or ring[2] < need:
+            ring = self._make_call_ring(need)
+        ws, u_cap = self._workspace(b, k)
+        prob = torch.empty(2 * b, device=self.device)
+        emb = torch.empty(3 * b, _lib.DIM, device=self.device) if want_emb else None
+        c = ring[3]
+        c.src, c.dst, c.neg, c.eidx = (a.__array_interface__["data"][0] for a in host)
+        c.ts = ts.__array_interface__["data"][0]
+        c.plan = pl.__array_interface__["data"][0] if n_plan else None
+        c.b, c.n_plan = b, n_plan if cache_plan is not None else -1
+        rc = L.orca_tgn_call(self._descriptor(k), c, u_cap, ws.data_ptr(), ws.numel(), prob.data_ptr(),
+                             emb.data_ptr() if want_emb else None, self._status.data_ptr(), ring[4],
+                             torch._C._cuda_getCurrentRawStream(d["_device_index"]))
+        if rc:
+            _lib.check(rc)
+        d["last_scores"] = prob     # [2b] = [pos | neg]: one contiguous tensor for callers that copy both
+        return prob, emb
+
+    def _make_call_ring(self, need):
+        """Pinned and device slots for the calls in flight, the call descriptor that names them and the pinned copy of
+        the status word."""
+        if self.__dict__.get("_call_ring") is not None:
+            torch.cuda.synchronize(self.device)       # calls may still be reading the smaller one
+        slot = 1 << max(17, (need - 1).bit_length())
+        h = torch.empty(_lib.CALL_SLOTS * slot, dtype=torch.uint8, pin_memory=True)
+        dev = torch.empty(_lib.CALL_SLOTS * slot, dtype=torch.uint8, device=self.device)
+        torch.cuda.current_stream(self.device).synchronize()   # (the copies run on a stream of their own)
+        if self._status_host is None:
+            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
+        c = _lib.CallT()
+        c.h_ring, c.d_ring, c.slot_bytes = h.data_ptr(), dev.data_ptr(), slot
+        ring = self.__dict__["_call_ring"] = (h, dev, slot, c, self._status_host.data_ptr())
+        self.__dict__["_status_view"] = self._status_host.numpy()
+        return ring
+
+    def _eval_batch_staged(self, source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs, k, cache_plan,
+                           n_plan, want_emb):
+        """One batch of the multi-GPU split."""
+        L = _lib.lib()
+        b = len(source_nodes)
         n_i32 = 4 * b + n_plan
         off_ts = (n_i32 * 4 + 15) // 16 * 16
         total = off_ts + 8 * b
@@ -531,20 +595,11 @@ class TGN(nn.Module):
         self._input_stream = self._copy_stream.cuda_stream     # the library orders its side streams after the copy
         stream = cur.cuda_stream
         ws, u_cap = self._workspace(b, k)
-        prob = torch.empty(2 * b, device=self.device)
-        emb = torch.empty(3 * b, _lib.DIM, device=self.device) if want_emb else None
         desc = self._descriptor(k)
         base = dev.data_ptr()
         d_plan = base + 16 * b if cache_plan is not None else None
-        if self._world > 1:
-            prob, emb = self._eval_batch_sharded(desc, base, base + off_ts, b, d_plan, n_plan, u_cap, ws, want_emb)
-            self.last_scores = prob
-            self._release_dev(ds, cur)
-            return prob, emb
-        _lib.check(L.orca_tgn_eval_batch(desc, base, base + off_ts, b, d_plan, n_plan, u_cap, ws.data_ptr(),
-                                         ws.numel(), prob.data_ptr(), _lib.ptr(emb), self._status.data_ptr(),
-                                         stream))
-        self.last_scores = prob     # [2b] = [pos | neg]: one contiguous tensor for callers that copy both
+        prob, emb = self._eval_batch_sharded(desc, base, base + off_ts, b, d_plan, n_plan, u_cap, ws, want_emb)
+        self.last_scores = prob
         self._release_dev(ds, cur)
         return prob, emb
 
@@ -566,12 +621,17 @@ class TGN(nn.Module):
         """Raises the device-side error of an earlier batch once its status copy has landed (capacity of the
         uncached set, ids outside a table, a bounded wait that gave up): the reference API has no status
         call, so the error surfaces at the start of a later call instead of being dropped."""
-        if self._status_pending and self._status_event.query():
+        v = self.__dict__.get("_status_view")
+        if v is None:
+            if not (self._status_pending and self._status_event.query()):
+                return
             self._status_pending = False
-            code = int(self._status_host[0])
-            if code != 0:
-                raise _lib.OrcaError(code, f"a kernel of an earlier batch reported error {code} "
-                                           f"(detail {int(self._status_host[3])}); results since then are invalid")
+            v = self._status_host.numpy()
+        code = int(v[0])
+        if code != 0:
+            v[0] = 0
+            raise _lib.OrcaError(code, f"a kernel of an earlier batch reported error {code} "
+                                       f"(detail {int(v[3])}); results since then are invalid")
 
     def _eval_batch_sharded(self, desc, d_i32, d_ts, b, d_plan, n_plan, u_cap, ws, want_emb):
         if self.n_layers != 2:
@@ -608,8 +668,10 @@ class TGN(nn.Module):
         (rows at layer 1, unique positives, kernel launches) of the last batch."""
         h = np.zeros(4, dtype=np.int32)
         self._status_pending = False       # (this call reads, reports and clears the word itself)
-        _lib.check(_lib.lib().orca_read_status(self._ctx, self._status.data_ptr(), h.ctypes.data,
-                                               _lib.stream_ptr(self.device)))
+        rc = _lib.lib().orca_read_status(self._ctx, self._status.data_ptr(), h.ctypes.data, _lib.stream_ptr(self.device))
+        if self.__dict__.get("_status_view") is not None:
+            self._status_view[0] = 0       # (the copies behind the batches have landed)
+        _lib.check(rc)
         self.last_counts = (int(h[1]), int(h[2]), int(h[3]))
         return self.last_counts
 
@@ -623,15 +685,14 @@ class TGN(nn.Module):
             raise AttributeError("reuse=True needs a model built with args.reuse (no history tables)")
         if mode != MODE_BUDGET and self._world > 1:
             raise NotImplementedError("the multi-GPU split is built for the budgeted recursion only")
-        self._mode = mode
-        self.batch_counter += 1
+        self.__dict__["_mode"] = mode
+        self.__dict__["batch_counter"] += 1      # (nn.Module's own attribute assignment costs a microsecond and more)
         if self.test_mode is False:
             # model/tgn_model.py:109-111: pending messages are flushed when eval starts
             self.update_memory_in_test(self.memory)
             self.test_mode = True
 
     # ---- model/tgn_model.py:95-147
-    @torch.no_grad()
     def compute_temporal_embeddings(self, source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs,
                                     n_neighbors, reuse, train, cache_plan):
         self._enter(reuse, train)
@@ -641,14 +702,13 @@ class TGN(nn.Module):
         return emb[:b], emb[b:2 * b], emb[2 * b:]
 
     # ---- model/tgn_model.py:150-157
-    @torch.no_grad()
     def compute_edge_probabilities(self, source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs,
                                    n_neighbors, reuse, train, cache_plan):
         self._enter(reuse, train)
         b = len(source_nodes)
         prob, _ = self._eval_batch(source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs,
                                    n_neighbors, cache_plan, want_emb=False)
-        return prob[:b].unsqueeze(1), prob[b:].unsqueeze(1)
+        return prob.view(2, b, 1).unbind(0)
 
     # ---- a whole stream of batches in one library call (the loop of evaluation/evaluation.py:18-37)
     @torch.no_grad()
