@@ -560,11 +560,13 @@ int orca_tgn_call(const orca_tgn_t *m, const orca_call_t *a, int32_t u_cap, void
 /* ------------------------------------------------------------------------------------------
  * A group of consecutive batches of a stream as one unit of work (one GPU, tensor-core projections; with the
  * budgeted recursion every batch needs a plan).  Results and state tables are those of the batches one by one, bit
- * for bit.  Enqueues the copies of the group's inputs (pinned host memory, laid out as in orca_epoch_t), its kernels
- * and the copy of its scores ([pos | neg] of batch after batch); nothing is synchronised, everything is complete in
- * `stream` order.  A stream is given as group after group, `first` set for the first one of every uninterrupted run:
- * nothing else may use the model's tables in between.  Groups of one run share bs, nb_max, u_cap, plan_cap and the
- * workspace; only the last batch of the last group may be short (b_last < bs).
+ * for bit.  Phase 1 enqueues the copies of the group's inputs (pinned host memory, laid out as in orca_epoch_t), its
+ * index kernels and its memory updates; phase 2 waits for the index kernels' row count, then enqueues the layers, the
+ * scores and their copy ([pos | neg] of batch after batch).  Everything is complete in `stream` order behind phase 2.
+ * A stream is given as group 0, 1, ...: phase 1 of a group may precede phase 2 of the one before it (and should: it
+ * runs beside it), not of an earlier one; nothing else may use the model's tables from phase 1 of group 0 to phase 2 of
+ * the last.  The groups share bs, nb_max, u_cap, plan_cap, the workspace and h_rows; only the last batch of the last
+ * group may be short (b_last < bs).
  */
 #define ORCA_GROUP_MAX 32
 typedef struct {
@@ -572,9 +574,11 @@ typedef struct {
   const double *h_ts;         /* of the group's first edge */
   const int64_t *off_i32;     /* nb offsets into h_i32, batch after batch without gaps */
   const int32_t *n_plan;      /* nb plan lengths */
+  int32_t *h_rows;            /* two page-locked words: row counts of the groups in flight */
+  int64_t seq;                /* number of the group in its stream */
+  int32_t phase;              /* 1, 2 or 3 (both) */
   int32_t nb, bs, b_last;     /* batches of this group; edges of a batch and of the group's last one */
   int32_t nb_max, u_cap, plan_cap; /* most batches of a group, most uncached neighbours and plan entries of a batch */
-  int32_t first;
 } orca_group_t;
 /* batches worth putting into one group */
 int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode);

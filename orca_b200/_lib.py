@@ -89,8 +89,8 @@ class CallT(C.Structure):
 
 
 class GroupT(C.Structure):
-    _fields_ = [("h_i32", C.c_void_p), ("h_ts", C.c_void_p), ("off_i32", C.c_void_p), ("n_plan", C.c_void_p)] + \
-        [(n, C.c_int32) for n in ("nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap", "first")]
+    _fields_ = [(n, C.c_void_p) for n in ("h_i32", "h_ts", "off_i32", "n_plan", "h_rows")] + [("seq", C.c_int64)] + \
+        [(n, C.c_int32) for n in ("phase", "nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap")]
 
 
 # every symbol the header declares: name -> (restype, argtypes)

@@ -3,7 +3,8 @@
 //
 // The rows come as an operand image (attn_out.cuh): bf16 heads and tails, split once by the kernels that computed them,
 // in the form the tensor core reads.  So the main loop is nothing but bulk copies and MMAs: one thread streams stages
-// of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three, one thread multiplies, eight warps do the
+// of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three (of five for the first product of a CTA's
+// first block, while the room of the hidden tile is still unused: a launch of few blocks waits for these loads), one thread multiplies, eight warps do the
 // two epilogues -- of one row block while the stages of the next are already landing.  A block of 128 rows takes 39
 // stages of 6 MMAs (10.5 us of tensor time) and 1.5 MB from L2.  The general projection kernel, whose producer warps
 // load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; here
@@ -29,6 +30,9 @@ constexpr int A2_LBO = BM * 16 + 16, A2_BYTES = K2_CHUNKS * A2_LBO;
 constexpr int TILE_LD = 180;                       // floats per row of the output tile (conflict-free 16-byte stores)
 constexpr int FRONT = 90 * 1024;                   // hidden image, then output tile
 static_assert(2 * A2_BYTES <= FRONT && BM * TILE_LD * 4 <= FRONT && STAGE % 1024 == 0, "");
+constexpr int FIRST = 5;                           // stages of the first product of a CTA's first block
+static_assert((FIRST - STAGES) * STAGE <= FRONT && K_STAGES % FIRST == FIRST - 1, "");
+constexpr int FIRST_USES = K_STAGES / FIRST + 1;   // of each of the first STAGES slots
 constexpr int SMEM = FRONT + STAGES * STAGE + 1024;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
 constexpr int TMEM_COLS = 512, SMALL = 256;
@@ -39,17 +43,21 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
   using namespace tc;
   extern __shared__ unsigned char raw[];
   __shared__ __align__(16) float s_b1[BN], s_g[BN], s_b2[BN], s_lw[BN], s_lb[BN];
-  __shared__ __align__(8) unsigned long long s_bar[2 * STAGES + 4];
+  __shared__ __align__(8) unsigned long long s_bar[2 * FIRST + 4];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u, ring = base + FRONT;
   auto full = [&](int s) { return smem_addr(&s_bar[s]); };
-  auto empty = [&](int s) { return smem_addr(&s_bar[STAGES + s]); };
-  const uint32_t acc1 = smem_addr(&s_bar[2 * STAGES]), a2bar = smem_addr(&s_bar[2 * STAGES + 1]),
-                 acc2 = smem_addr(&s_bar[2 * STAGES + 2]), tfree = smem_addr(&s_bar[2 * STAGES + 3]);
+  auto empty = [&](int s) { return smem_addr(&s_bar[FIRST + s]); };
+  const uint32_t acc1 = smem_addr(&s_bar[2 * FIRST]), a2bar = smem_addr(&s_bar[2 * FIRST + 1]),
+                 acc2 = smem_addr(&s_bar[2 * FIRST + 2]), tfree = smem_addr(&s_bar[2 * FIRST + 3]);
+  // stage number `it` of this CTA: its slot, how often the slot was used before, and where it lies
+  auto slot_of = [&](int it) { return it < K_STAGES ? it % FIRST : (it - K_STAGES) % STAGES; };
+  auto use_of = [&](int it) { return it < K_STAGES ? it / FIRST : FIRST_USES + (it - K_STAGES) / STAGES; };
+  auto place = [&](int s) { return s < STAGES ? ring + s * STAGE : base + (s - STAGES) * STAGE; };
   dep_trigger();
   if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < FIRST; ++s) {
       mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
     }
@@ -90,9 +98,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
         const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
         const char *feat = g.feat + (size_t)blk * img::FEAT_STAGES * A_STAGE;
         for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
-          const int s = it % STAGES;
-          const uint32_t at = ring + s * STAGE;
-          mbar_wait(empty(s), ((it / STAGES) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
+          const int s = slot_of(it);
+          const uint32_t at = place(s);
+          mbar_wait(empty(s), (use_of(it) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
           if (st < K_STAGES) {
             mbar_expect_tx(full(s), STAGE);
             bulk_g2s(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
@@ -114,10 +122,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       if (t > 0) mbar_wait(tfree, (t - 1) & 1, g.status, 710, alive, g.wait_limit);
       tc_fence_after();
       for (int st = 0; st < K_STAGES; ++st, ++it) {
-        const int s = it % STAGES;
-        const uint32_t a = ring + s * STAGE, w = a + A_STAGE;
+        const int s = slot_of(it);
+        const uint32_t a = place(s), w = a + A_STAGE;
         const bool half = st == img::CTX_STAGES - 1 || st == K_STAGES - 1;     // (the second step is nothing but padding)
-        mbar_wait(full(s), (it / STAGES) & 1, g.status, 711, alive, g.wait_limit);
+        mbar_wait(full(s), use_of(it) & 1, g.status, 711, alive, g.wait_limit);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -138,9 +146,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       mbar_wait(a2bar, t & 1, g.status, 712, alive, g.wait_limit);
       tc_fence_after();
       for (int st = 0; st < K2_STAGES; ++st, ++it) {
-        const int s = it % STAGES;
-        const uint32_t w = ring + s * STAGE + A_STAGE, a = base + st * 4 * A2_LBO;
-        mbar_wait(full(s), (it / STAGES) & 1, g.status, 713, alive, g.wait_limit);
+        const int s = slot_of(it);
+        const uint32_t w = place(s) + A_STAGE, a = base + st * 4 * A2_LBO;
+        mbar_wait(full(s), use_of(it) & 1, g.status, 713, alive, g.wait_limit);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll

@@ -5,15 +5,19 @@
 // a pipeline filled and drained, two launches) whatever the batch size, and it is the only part of a group that is
 // serial: with small batches it is what a stream waits for.  What a batch really waits for is its memory rows.  So
 // one cooperative grid walks the batches:
-//   - 22 column tiles of 32 gate columns (eight units) times RB row blocks of 32 updates, one CTA each.  A CTA keeps
-//     its weight columns (880 x 32, bf16 head and tail, 113 KB) in shared memory for the whole launch.
+//   - 22 column tiles of 32 gate columns (eight units) times up to six row blocks of 64 updates, one CTA each.  A CTA
+//     keeps its weight columns (880 x 32, bf16 head and tail, 113 KB) in shared memory for the whole launch.
 //   - K is laid out so that what does not depend on the batch before comes first: edge features and time encoding
-//     (352 columns) are gathered, converted and multiplied for batch n + 1 while batch n is still being finished.
+//     (352 columns).  A launch of its own splits them for all updates of the group (computed in the chain, the cosines
+//     alone were half of a turn), and they are multiplied for batch n + 1 while batch n is still being finished.
 //   - Then the grid meets at a counter, and only the node's own and the other endpoint's memory rows (2 x 688 bytes
-//     an update) are gathered, converted and multiplied; the GRU's hidden operand is the own row's image again.
+//     an update) are gathered, split and multiplied; the GRU's hidden operand is the own row's image again.
 //   - The result goes to the log row of the update; message table, times and flags follow in one launch at the end.
+// MMAs of 64 rows: an MMA of 32 columns is bound by its reads of the row operand.  Row r of the tile sits in tensor
+// memory lane 32 * (r / 16) + r % 16.
 // A step's products are the ones of the projection kernel, k-step by k-step, so the results are the same bits.
-// Warp 0: epilogue (gates; thread = update).  Warps 1-8: gather and split.  Warp 9: MMA issue, tensor memory.
+// Warps 0-3: epilogue (16 rows each, a lane for four of a row's units).  Warps 4-11: gather and split.  Warp 12: MMA
+// issue, tensor memory.
 // Every wait is bounded; one that gives up reports ORCA_E_TIMEOUT and the kernel runs to its end.
 #include "chain.cuh"
 #include "context.cuh"
@@ -23,48 +27,91 @@
 namespace orca {
 namespace grp {
 
-constexpr int ROWS = 32;                       // updates per row block (the MMA's other 96 rows are never read back)
+constexpr int ROWS = 64;                       // updates per row block
 constexpr int COLS = 32, UNITS = COLS / 4;     // gate columns / units per CTA
 constexpr int COL_TILES = (4 * D + COLS - 1) / COLS;   // 22
 constexpr int PART_CHUNKS = tc::GRU_PART / 8;  // 22 chunks of 8 K elements per part
 constexpr int PART_STEPS = tc::GRU_PART / 16;  // 11 MMA steps per part
 constexpr int W_LBO = COLS * 16, W_BYTES = 5 * PART_CHUNKS * W_LBO;
-constexpr int A_LBO = ROWS * 16 + 16, A_BYTES = 4 * PART_CHUNKS * A_LBO;   // (+16: conflict-free 16-byte stores)
-// (an MMA reads 128 rows of a chunk, of which 32 are there: the last chunk's reads run 1520 bytes further)
-constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 2048 + 1024 + 256;
-constexpr int PRODUCERS = 256, THREADS = 64 + PRODUCERS;
+// two parts of K at a time: first edge features and time encoding, then, once those have been read, the memory rows
+constexpr int A_CHUNKS = 2 * PART_CHUNKS, A_LBO = ROWS * 16 + 16, A_BYTES = A_CHUNKS * A_LBO;   // (+16: conflict-free stores)
+constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 1024;
+constexpr int EPI_WARPS = 4, PRODUCERS = 256, THREADS = 32 * EPI_WARPS + PRODUCERS + 32;
 constexpr int TMEM_COLS = 128, BUF_COLS = 64, SMALL = 32;   // two accumulator buffers of main + cross terms
-constexpr int META = 4;                        // steps whose row indices are kept
+constexpr int META = 4;                        // steps whose memory rows are kept
+constexpr int PER = 6;                         // chunks a producer thread has in flight: 34 rows at a time
+
+// Edge features and time encoding of every update, split: 44 chunks of [heads 16 bytes | tails 16 bytes].  The memory
+// rows that the chain will read from the table start on their way into L2.
+__global__ void __launch_bounds__(256) update_image_kernel(const __grid_constant__ ChainArgs g) {
+  const Args &a = g.a;
+  dep_trigger();
+  dep_wait();
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.nb * 2 * a.bs; i += (gridDim.x * blockDim.x) >> 5) {
+    const int n = i / (2 * a.bs), w = i - n * 2 * a.bs;
+    if (w >= a.cnt->n_win[n]) continue;
+    const float gap = a.win_gap != nullptr ? a.win_gap[i] : a.win_t[i] - g.mem.last_update[a.win_node[i]];
+    if (lane < 12) {
+      const int r = lane < 6 ? a.win_mem[i] : a.win_other[i];
+      if (r < a.n_nodes)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)(g.mem.memory + (size_t)r * D) + min((lane % 6) * 128, ROW_BYTES - 4)));
+    }
+    const float4 *e = reinterpret_cast<const float4 *>(g.edge_table + (size_t)a.win_eid[i] * D);
+    for (int c = lane; c < A_CHUNKS; c += 32) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+      if (c < PART_CHUNKS) {
+        x = __ldg(e + 2 * c);
+        if (c < PART_CHUNKS - 1) y = __ldg(e + 2 * c + 1);
+      } else {
+        const int d = (c - PART_CHUNKS) * 8;
+        const float4 w0 = __ldg(reinterpret_cast<const float4 *>(g.time_w + d));
+        x = make_float4(cos_any(gap * w0.x), cos_any(gap * w0.y), cos_any(gap * w0.z), cos_any(gap * w0.w));
+        if (d + 4 < D) {
+          const float4 w1 = __ldg(reinterpret_cast<const float4 *>(g.time_w + d + 4));
+          y = make_float4(cos_any(gap * w1.x), cos_any(gap * w1.y), cos_any(gap * w1.z), cos_any(gap * w1.w));
+        }
+      }
+      uint4 hi, lo;
+      tc::split_chunk(x, y, hi, lo);
+      uint4 *o = reinterpret_cast<uint4 *>(g.image) + ((size_t)i * A_CHUNKS + c) * 2;
+      o[0] = hi;
+      o[1] = lo;
+    }
+  }
+}
 
 __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_constant__ ChainArgs g) {
   using namespace tc;
   extern __shared__ unsigned char raw[];
   __shared__ int s_win[MAX_BATCHES];
-  __shared__ int s_self[META][ROWS], s_other[META][ROWS], s_eid[META][ROWS];
-  __shared__ float s_gap[META][ROWS];
+  __shared__ int s_self[META][ROWS], s_other[META][ROWS];
   __shared__ __align__(16) float s_bias[COLS];
   __shared__ __align__(8) unsigned long long s_bar[8];
   __shared__ uint32_t s_tmem;
   const Args &a = g.a;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int ct = blockIdx.x, rb = blockIdx.y, n_cta = gridDim.x * gridDim.y, stride = gridDim.y * ROWS;
+  const int ct = blockIdx.x, rb = blockIdx.y, n_rb = gridDim.y, n_cta = gridDim.x * gridDim.y;
   const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u;
   const uint32_t w_hi = base, w_lo = base + W_BYTES, a_hi = base + 2 * W_BYTES, a_lo = a_hi + A_BYTES;
   const uint32_t wbar = smem_addr(&s_bar[0]), ebar = smem_addr(&s_bar[1]), mbar = smem_addr(&s_bar[2]),
-                 accbar = smem_addr(&s_bar[3]);
-  auto tfree = [&](int b) { return smem_addr(&s_bar[4 + b]); };
+                 edone = smem_addr(&s_bar[3]), accbar = smem_addr(&s_bar[4]);
+  auto tfree = [&](int b) { return smem_addr(&s_bar[5 + b]); };
+  // rows of a row block in a batch: the updates spread over the blocks, in steps of eight, at most a tile's
+  auto rows_per = [&](int win) { return min(ROWS, ((win + n_rb - 1) / n_rb + 7) & ~7); };
   if (tid == 0) {
     mbar_init(wbar, 1);
     mbar_init(ebar, PRODUCERS / 32);
     mbar_init(mbar, PRODUCERS / 32);
+    mbar_init(edone, 1);
     mbar_init(accbar, 1);
-    mbar_init(tfree(0), 1);
-    mbar_init(tfree(1), 1);
+    mbar_init(tfree(0), EPI_WARPS);
+    mbar_init(tfree(1), EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(wbar, 2 * W_BYTES);
     bulk_g2s(w_hi, reinterpret_cast<const char *>(g.w) + (size_t)ct * 2 * W_BYTES, 2 * W_BYTES, wbar);
   }
-  if (warp == 9) {
+  if (warp == 12) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
                  "r"(TMEM_COLS)
                  : "memory");
@@ -79,102 +126,78 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
   bool alive = true;
   auto mem_row = [&](int r) { return (r >= a.n_nodes ? g.log : g.mem.memory) + (size_t)r * D; };
 
-  int s = 0;    // steps of this CTA so far: 32 updates of one batch each
-  if (warp == 0) {
+  int s = 0;    // steps of this CTA so far: the rows of one turn of one batch each
+  if (warp < EPI_WARPS) {
     // ------------------------------------------------------------------ gates
+    const int row = warp * 16 + (lane & 15), hi = lane >> 4;     // this lane: units 4 * hi .. 4 * hi + 3 of the row
+    const int u0 = ct * UNITS + 4 * hi;
     for (int n = 0; n < a.nb; ++n) {
-      for (int r0 = rb * ROWS; r0 < s_win[n]; r0 += stride, ++s) {
-        const bool live = r0 + lane < s_win[n];
-        mbar_wait(mbar, s & 1, g.status, 610, alive, g.wait_limit);   // (the batches before are complete then)
-        float4 h0 = make_float4(0.f, 0.f, 0.f, 0.f), h1 = h0;
-        const bool two = ct * UNITS + 4 < D;      // the last tile has four units
-        if (live) {
-          const float4 *h = reinterpret_cast<const float4 *>(mem_row(s_self[s & (META - 1)][lane]) + ct * UNITS);
-          h0 = __ldcg(h);
-          if (two) h1 = __ldcg(h + 1);
-        }
+      const int rows = rows_per(s_win[n]);
+      for (int r0 = rb * rows; r0 < s_win[n]; r0 += n_rb * rows, ++s) {
+        const bool live = row < rows && r0 + row < s_win[n] && u0 < D;      // (the last tile has four units)
+        mbar_wait(mbar, s & 1, g.status, 610, alive, g.wait_limit);         // (the batches before are complete then)
+        float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live) h = __ldcg(reinterpret_cast<const float4 *>(mem_row(s_self[s & (META - 1)][row]) + u0));
         mbar_wait(accbar, s & 1, g.status, 611, alive, g.wait_limit);
         tc_fence_after();
-        float v[32];
-        {
-          float x[16];
-          const uint32_t t = tmem + (s & 1) * BUF_COLS;
-          tmem_ld16_sum(t, SMALL, x);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = x[i];
-          tmem_ld16_sum(t + 16, SMALL, x);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[16 + i] = x[i];
-        }
+        float x[16], y[16];
+        const uint32_t t = tmem + ((uint32_t)(warp * 32) << 16) + (s & 1) * BUF_COLS;
+        tmem_ld16_sum(t, SMALL, x);
+        tmem_ld16_sum(t + 16, SMALL, y);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(tfree(s & 1));
-        float y[8];
-        const float ho[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+        // (rows live in the lower 16 lanes: the upper ones take over the second half of their columns)
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          y[u] = gru_gates(make_float4(v[4 * u] + s_bias[4 * u], v[4 * u + 1] + s_bias[4 * u + 1],
-                                       v[4 * u + 2] + s_bias[4 * u + 2], v[4 * u + 3] + s_bias[4 * u + 3]), ho[u]);
-        if (live) {
-          float4 *o = reinterpret_cast<float4 *>(g.log_out + (size_t)(n * 2 * a.bs + r0 + lane) * D + ct * UNITS);
-          o[0] = make_float4(y[0], y[1], y[2], y[3]);
-          if (two) o[1] = make_float4(y[4], y[5], y[6], y[7]);
+        for (int i = 0; i < 16; ++i) {
+          const float z = __shfl_sync(0xffffffffu, y[i], lane & 15);
+          if (hi) x[i] = z;
         }
+        const float *b = s_bias + 16 * hi;
+        const float ho[4] = {h.x, h.y, h.z, h.w};
+        float o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          o[u] = gru_gates(make_float4(x[4 * u] + b[4 * u], x[4 * u + 1] + b[4 * u + 1], x[4 * u + 2] + b[4 * u + 2],
+                                       x[4 * u + 3] + b[4 * u + 3]), ho[u]);
+        if (live)
+          *reinterpret_cast<float4 *>(g.log_out + (size_t)(n * 2 * a.bs + r0 + row) * D + u0) = make_float4(o[0], o[1], o[2], o[3]);
       }
-      __threadfence();
-      __syncwarp();
+      __syncwarp();      // (the release below covers the warp's stores)
       if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&a.cnt->arrived[n]) : "memory");
     }
-  } else if (warp < 9) {
+  } else if (warp < 12) {
     // ------------------------------------------------------------------ gather and split
-    const int pt = tid - 32;
-    auto put = [&](int chunk, int row, const float4 x, const float4 y) {
-      uint4 hi, lo;
-      split_chunk(x, y, hi, lo);
+    const int pt = tid - 32 * EPI_WARPS;
+    auto put = [&](int chunk, int row, uint4 hi, uint4 lo) {
       st_shared_v4(a_hi + chunk * A_LBO + row * 16, hi);
       st_shared_v4(a_lo + chunk * A_LBO + row * 16, lo);
     };
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int N_UNITS = ROWS * 2 * PART_CHUNKS;     // 16-byte image chunks of two parts
-    constexpr int PER = (N_UNITS + PRODUCERS - 1) / PRODUCERS;
     for (int n = 0; n < a.nb; ++n) {
       bool met = n == 0;
-      for (int r0 = rb * ROWS; r0 < s_win[n]; r0 += stride, ++s) {
-        const int q = s & (META - 1), rows = min(ROWS, s_win[n] - r0);
+      const int full_rows = rows_per(s_win[n]);
+      for (int r0 = rb * full_rows; r0 < s_win[n]; r0 += n_rb * full_rows, ++s) {
+        const int q = s & (META - 1), rows = min(full_rows, s_win[n] - r0), n_units = rows * A_CHUNKS;
+        const int at = n * 2 * a.bs + r0;
         if (pt < rows) {
-          const int at = n * 2 * a.bs + r0 + pt;
-          s_self[q][pt] = a.win_mem[at];
-          s_other[q][pt] = a.win_other[at];
-          s_eid[q][pt] = a.win_eid[at];
-          s_gap[q][pt] = a.win_gap[at];
+          s_self[q][pt] = a.win_mem[at + pt];
+          s_other[q][pt] = a.win_other[at + pt];
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        // edge features and time encoding: chunks 0 .. 43
-        float4 x[PER][2];
+        // edge features and time encoding
+        const uint4 *im = reinterpret_cast<const uint4 *>(g.image) + (size_t)at * A_CHUNKS * 2;
+        for (int u0 = pt; u0 - pt < n_units; u0 += PER * PRODUCERS) {
+          uint4 e[PER][2];
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int u = pt + i * PRODUCERS, row = u / (2 * PART_CHUNKS), c = u - row * (2 * PART_CHUNKS);
-          x[i][0] = x[i][1] = zero;
-          if (row < rows && c < PART_CHUNKS) {
-            const float4 *e = reinterpret_cast<const float4 *>(g.edge_table + (size_t)s_eid[q][row] * D) + 2 * c;
-            x[i][0] = __ldg(e);
-            if (c < PART_CHUNKS - 1) x[i][1] = __ldg(e + 1);
-          } else if (row < rows) {
-            const float gap = s_gap[q][row];
-            const int d = (c - PART_CHUNKS) * 8;
-            const float4 w0 = __ldg(reinterpret_cast<const float4 *>(g.time_w + d));
-            x[i][0] = make_float4(cos_any(gap * w0.x), cos_any(gap * w0.y), cos_any(gap * w0.z), cos_any(gap * w0.w));
-            if (d + 4 < D) {
-              const float4 w1 = __ldg(reinterpret_cast<const float4 *>(g.time_w + d + 4));
-              x[i][1] = make_float4(cos_any(gap * w1.x), cos_any(gap * w1.y), cos_any(gap * w1.z), cos_any(gap * w1.w));
-            }
+          for (int i = 0; i < PER; ++i) {
+            const int u = u0 + i * PRODUCERS;
+            if (u < n_units) e[i][0] = __ldg(im + 2 * u), e[i][1] = __ldg(im + 2 * u + 1);
           }
-        }
-        if (s > 0) mbar_wait(accbar, (s - 1) & 1, g.status, 620, alive, g.wait_limit);   // the image is free again
+          if (s > 0) mbar_wait(accbar, (s - 1) & 1, g.status, 620, alive, g.wait_limit);   // the image is free again
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int u = pt + i * PRODUCERS, row = u / (2 * PART_CHUNKS), c = u - row * (2 * PART_CHUNKS);
-          if (row < rows) put(c, row, x[i][0], x[i][1]);
+          for (int i = 0; i < PER; ++i) {
+            const int u = u0 + i * PRODUCERS;
+            if (u < n_units) put(u % A_CHUNKS, u / A_CHUNKS, e[i][0], e[i][1]);
+          }
         }
         fence_async_smem();
         __syncwarp();
@@ -188,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
             for (;;) {
               int v;
               asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&a.cnt->arrived[n - 1]) : "memory");
-              if (v >= n_cta) break;
+              if (v >= n_cta * EPI_WARPS) break;
               if (clock64() - t0 > g.wait_limit) {
                 report(g.status, ORCA_E_TIMEOUT, 621);
                 alive = false;
@@ -196,24 +219,32 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
               }
             }
           }
-          asm volatile("bar.sync 1, 256;" ::: "memory");
         }
-        // own and other memory: chunks 44 .. 87
+        asm volatile("bar.sync 1, 256;" ::: "memory");     // (and the memory rows' numbers are known)
+        // own and other memory
+        for (int u0 = pt; u0 - pt < n_units; u0 += PER * PRODUCERS) {
+          float4 x[PER][2];
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int u = pt + i * PRODUCERS, row = u / (2 * PART_CHUNKS), c = u - row * (2 * PART_CHUNKS);
-          x[i][0] = x[i][1] = zero;
-          if (row < rows) {
-            const int cc = c < PART_CHUNKS ? c : c - PART_CHUNKS;
-            const float4 *m = reinterpret_cast<const float4 *>(mem_row(c < PART_CHUNKS ? s_self[q][row] : s_other[q][row])) + 2 * cc;
-            x[i][0] = __ldcg(m);
-            if (cc < PART_CHUNKS - 1) x[i][1] = __ldcg(m + 1);
+          for (int i = 0; i < PER; ++i) {
+            const int u = u0 + i * PRODUCERS, row = u / A_CHUNKS, c = u - row * A_CHUNKS;
+            x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (u < n_units) {
+              const int cc = c < PART_CHUNKS ? c : c - PART_CHUNKS;
+              const float4 *m = reinterpret_cast<const float4 *>(mem_row(c < PART_CHUNKS ? s_self[q][row] : s_other[q][row])) + 2 * cc;
+              x[i][0] = __ldcg(m);
+              if (cc < PART_CHUNKS - 1) x[i][1] = __ldcg(m + 1);
+            }
           }
-        }
+          mbar_wait(edone, s & 1, g.status, 622, alive, g.wait_limit);     // the first two parts have been read
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int u = pt + i * PRODUCERS, row = u / (2 * PART_CHUNKS), c = u - row * (2 * PART_CHUNKS);
-          if (row < rows) put(2 * PART_CHUNKS + c, row, x[i][0], x[i][1]);
+          for (int i = 0; i < PER; ++i) {
+            const int u = u0 + i * PRODUCERS, row = u / A_CHUNKS, c = u - row * A_CHUNKS;
+            if (u < n_units) {
+              uint4 hi, lo;
+              split_chunk(x[i][0], x[i][1], hi, lo);
+              put(c, row, hi, lo);
+            }
+          }
         }
         fence_async_smem();
         __syncwarp();
@@ -222,10 +253,11 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
     }
   } else {
     // ------------------------------------------------------------------ MMA issue
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COLS >> 3) << 17) | (8u << 24);   // M = 128
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COLS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
     mbar_wait(wbar, 0, g.status, 630, alive, g.wait_limit);
-    for (int n = 0; n < a.nb; ++n)
-      for (int r0 = rb * ROWS; r0 < s_win[n]; r0 += stride, ++s) {
+    for (int n = 0; n < a.nb; ++n) {
+      const int rows = rows_per(s_win[n]);
+      for (int r0 = rb * rows; r0 < s_win[n]; r0 += n_rb * rows, ++s) {
         const uint32_t d = tmem + (s & 1) * BUF_COLS;
         if (s >= 2) mbar_wait(tfree(s & 1), ((s >> 1) & 1) ^ 1, g.status, 631, alive, g.wait_limit);
         // parts of K: edge features, time encoding | own memory, other memory, own memory again
@@ -235,7 +267,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
           if (part == 2) mbar_wait(mbar, s & 1, g.status, 633, alive, g.wait_limit);
           if (part == 0 || part == 2) tc_fence_after();
           if (elect_one()) {
-            const int ap = part < 4 ? part : 2;
+            const int ap = part == 4 ? 0 : part & 1;      // place of the part's rows in the image
 #pragma unroll
             for (int ks = 0; ks < PART_STEPS; ++ks) {
               const uint32_t ao = (ap * PART_STEPS + ks) * 2 * A_LBO, wo = (part * PART_STEPS + ks) * 2 * W_LBO;
@@ -246,15 +278,17 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
               mma_bf16(d + SMALL, al, bh, idesc, more);
               mma_bf16(d + SMALL, ah, bl, idesc, 1u);
             }
+            if (part == 1) mma_commit(edone);
             if (part == 4) mma_commit(accbar);
           }
           __syncwarp();
         }
       }
+    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 12) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
@@ -271,7 +305,8 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
     const int n = i / (2 * a.bs), w = i - n * 2 * a.bs;
     if (w >= a.cnt->n_win[n]) continue;
     const int node = a.win_node[i];
-    if ((unsigned long long)a.bits[node].positive >> (n + 1)) continue;
+    if (a.nb > 1 && (unsigned long long)a.bits[node].positive >> (n + 1)) continue;
+    const float gap = a.win_gap != nullptr ? a.win_gap[i] : a.win_t[i] - g.mem.last_update[node];
     float *dst = g.mem.messages + (size_t)node * MSG + part * D;
     auto row = [&](int r) { return (r >= a.n_nodes ? g.log : g.mem.memory) + (size_t)r * D; };
     if (part < 3) {
@@ -279,9 +314,9 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
                                                                   : g.edge_table + (size_t)a.win_eid[i] * D;
       if (lane < D / 4) reinterpret_cast<float4 *>(dst)[lane] = reinterpret_cast<const float4 *>(src)[lane];
     } else {
-      const float gap = a.win_gap[i];
       for (int d = lane; d < D; d += 64) dst[d] = cos_any(gap * __ldg(g.time_w + d));
     }
+    __syncthreads();     // (the last update has been read)
     if (threadIdx.x == 0) {
       const float t = a.win_t[i];
       g.mem.msg_ts[node] = t;
@@ -291,7 +326,7 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
   }
 }
 
-int launch_gru_chain(const ChainArgs &args, cudaStream_t s) {
+static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "launch_gru_chain: no context for the current device");
   static thread_local int configured_device = -1;
@@ -302,10 +337,11 @@ int launch_gru_chain(const ChainArgs &args, cudaStream_t s) {
   ChainArgs g = args;
   g.status = c->status_word;
   g.wait_limit = c->wait_limit;
-  // all row blocks that fit at one CTA per SM: a batch with more updates than rows takes another turn per batch
-  const int blocks = std::max(1, std::min(ceil_div(2 * g.a.bs, ROWS), c->sm_count / COL_TILES));
+  const int most = g.a.nb * 2 * g.a.bs;
+  ORCA_CUDA(launch_dep(update_image_kernel, std::min(ceil_div(most, 8), c->sm_count * 8), 256, 0, s, g));
+  ORCA_COUNT_LAUNCH();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(COL_TILES, blocks);
+  cfg.gridDim = dim3(COL_TILES, std::max(1, std::min(blocks, c->sm_count / COL_TILES)));
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = s;
@@ -313,10 +349,52 @@ int launch_gru_chain(const ChainArgs &args, cudaStream_t s) {
   attr[0].id = cudaLaunchAttributeCooperative;     // the CTAs wait for one another
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g.a.nb > 1 ? 1 : 0;
   ORCA_CUDA(cudaLaunchKernelEx(&cfg, gru_chain_kernel, g));
   ORCA_COUNT_LAUNCH();
-  ORCA_CUDA(launch_dep(last_messages_kernel, c->sm_count * 4, 256, 0, s, g));
+  ORCA_CUDA(launch_dep(last_messages_kernel, std::min(most, c->sm_count * 4), 256, 0, s, g));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+int launch_gru_chain(const ChainArgs &g, cudaStream_t s) {
+  // all row blocks that fit at one CTA per SM: a batch with more updates than rows takes another turn
+  return launch(g, ceil_div(2 * g.a.bs, 8), s);
+}
+
+__global__ void __launch_bounds__(256) scatter_updates_kernel(float *__restrict__ memory, const int32_t *__restrict__ node,
+                                                              const Counters *__restrict__ cnt, int cap,
+                                                              const float *__restrict__ rows) {
+  dep_trigger();
+  dep_wait();
+  const int t = threadIdx.x & 63, n = min(cap, cnt->n_win[0]);
+  for (int w = blockIdx.x * 4 + threadIdx.x / 64; w < n; w += gridDim.x * 4)
+    if (t < D / 4)
+      reinterpret_cast<float4 *>(memory + (size_t)node[w] * D)[t] = reinterpret_cast<const float4 *>(rows + (size_t)w * D)[t];
+}
+
+int launch_gru_single(const orca_memory_t &mem, const orca_gru_weights_t &w, const float *edge_table, const float *time_w,
+                      int b, const int32_t *d_node, const int32_t *d_other, const int32_t *d_eid, const float *d_t,
+                      Counters *d_cnt, void *d_image, float *d_rows, cudaStream_t s) {
+  ORCA_CHECK_ARG(w.Wg_chain != nullptr && w.bg != nullptr);
+  ChainArgs g{};
+  g.a.nb = 1, g.a.bs = g.a.b_last = b, g.a.n_nodes = mem.n_nodes, g.a.cnt = d_cnt;
+  // (every row is read from the memory table: its ids are its rows)
+  g.a.win_node = const_cast<int32_t *>(d_node), g.a.win_mem = const_cast<int32_t *>(d_node);
+  g.a.win_other = const_cast<int32_t *>(d_other), g.a.win_eid = const_cast<int32_t *>(d_eid);
+  g.a.win_t = const_cast<float *>(d_t);
+  g.mem = mem, g.log = mem.memory, g.log_out = d_rows, g.edge_table = edge_table, g.time_w = time_w;
+  g.w = w.Wg_chain, g.bias = w.bg, g.image = d_image;
+  // two fifths of the positions of a batch are winners, or fewer: as few row blocks as take those in one turn, since the
+  // launch runs beside the layers
+  return launch(g, ceil_div(2 * b * 2 / 5, ROWS), s);
+}
+
+int scatter_updates(const orca_memory_t &mem, const int32_t *d_node, const Counters *d_cnt, int cap, const float *d_rows,
+                    cudaStream_t s) {
+  ORCA_CUDA(launch_dep(scatter_updates_kernel, std::min(ceil_div(cap, 4), 592), 256, 0, s, mem.memory, d_node, d_cnt, cap,
+                       d_rows));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

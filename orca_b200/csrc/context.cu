@@ -21,7 +21,8 @@ static int create_ctx(Ctx **out) {
   for (cudaEvent_t &e : c->ev_call) ORCA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   cudaEvent_t *evs[] = {&c->fork, &c->join, &c->ev_in, &c->ev_flags, &c->ev_o1, &c->ev_g2, &c->ev_state,
                         &c->ev_idx[0], &c->ev_idx[1], &c->ev_done[0], &c->ev_done[1], &c->ev_gin, &c->ev_gidx[0],
-                        &c->ev_gidx[1], &c->ev_gchain[0], &c->ev_gchain[1], &c->ev_gdone[0], &c->ev_gdone[1]};
+                        &c->ev_gidx[1], &c->ev_gchain[0], &c->ev_gchain[1], &c->ev_gdone[0], &c->ev_gdone[1], &c->ev_gcount[0],
+                        &c->ev_gcount[1]};
   for (cudaEvent_t *e : evs) ORCA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   ORCA_CUDA(cudaMalloc(&c->d_words, CTX_WORDS * sizeof(int32_t)));
   ORCA_CUDA(cudaMemset(c->d_words, 0, CTX_WORDS * sizeof(int32_t)));
@@ -44,7 +45,7 @@ static void destroy_ctx(Ctx *c) {
     if (e) cudaEventDestroy(e);
   cudaEvent_t evs[] = {c->fork, c->join, c->ev_in, c->ev_flags, c->ev_o1, c->ev_g2, c->ev_state, c->ev_idx[0],
                        c->ev_idx[1], c->ev_done[0], c->ev_done[1], c->ev_gin, c->ev_gidx[0], c->ev_gidx[1],
-                       c->ev_gchain[0], c->ev_gchain[1], c->ev_gdone[0], c->ev_gdone[1]};
+                       c->ev_gchain[0], c->ev_gchain[1], c->ev_gdone[0], c->ev_gdone[1], c->ev_gcount[0], c->ev_gcount[1]};
   for (cudaEvent_t e : evs)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->trace.ev) cudaEventDestroy(e);

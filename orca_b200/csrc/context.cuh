@@ -69,8 +69,8 @@ struct Ctx {
   int last_batch_launches = 0;
   // groups of batches (group.cu): per parity, what the next user of its buffers waits for
   cudaEvent_t ev_gin = nullptr, ev_gidx[2] = {nullptr, nullptr}, ev_gchain[2] = {nullptr, nullptr}, ev_gdone[2] = {nullptr, nullptr};
+  cudaEvent_t ev_gcount[2] = {nullptr, nullptr};
   bool gdone_recorded[2] = {false, false};
-  long long gseq = 0;
   int32_t *d_words = nullptr;             // CTX_WORDS zeroed int32
   Tracer trace;
   GatherProfile prof;

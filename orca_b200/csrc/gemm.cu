@@ -418,8 +418,7 @@ static inline int kblocks(int k) { return (k + tc::BK - 1) / tc::BK; }
 
 namespace orca {
 
-// Arguments of the tensor-core projections.  The functions that end in _rows serve a group of batches (group.cu): rows
-// of a two-part table, tensor cores only.
+// Arguments of the tensor-core projections (score_rows serves a group of batches, group.cu).
 static tc::Args output_args(const orca_attn_weights_t *w, const float *d_ctx, const uint8_t *d_valid,
                             const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_out) {
   tc::Args a{};
@@ -462,11 +461,11 @@ int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t 
   a.a1.idx = d_b;
   return tc::launch(tc::EPI_SCORE, a, 1, s);
 }
-static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
-                         const int32_t *d_mem_rows, int n_cap, const int32_t *d_n, float *d_out) {
+static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes, int n_cap,
+                         const int32_t *d_n, float *d_out) {
   tc::Args a{};
   a.a0 = tc::RowSrc{mem->messages, d_nodes, MSG, 0, 0};
-  a.a1 = tc::RowSrc{mem->memory, d_mem_rows, D, 0, 0};
+  a.a1 = tc::RowSrc{mem->memory, d_nodes, D, 0, 0};
   a.Kd = MSG + D;
   a.w_packed = w->Wg_tc;
   a.n_kblocks = kblocks(tc::GRU_K);
@@ -475,16 +474,8 @@ static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, 
   a.bias = w->bg;
   a.out = d_out;
   a.memory = mem->memory;
-  a.nodes = d_mem_rows;
+  a.nodes = d_nodes;
   return a;
-}
-int gru_project_rows(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
-                     const int32_t *d_mem_rows, const float *mem2, int mem_split, int n_cap, const int32_t *d_n,
-                     float *d_out, cudaStream_t s) {
-  tc::Args a = gru_args(w, mem, d_nodes, d_mem_rows, n_cap, d_n, d_out);
-  a.a1.p2 = a.memory2 = mem2;
-  a.a1.split = a.memory_split = mem_split;
-  return tc::launch(tc::EPI_GRU, a, 4, s);
 }
 
 }  // namespace orca
@@ -603,7 +594,7 @@ int gru_project(const orca_gru_weights_t *w, const orca_memory_t *mem, const int
   if (n_cap == 0) return ORCA_OK;
   if (projection_mode() == 0) {
     ORCA_CHECK_ARG(w->Wg_tc != nullptr);
-    tc::Args a = gru_args(w, mem, d_nodes, d_nodes, n_cap, d_n, d_scratch_h);
+    tc::Args a = gru_args(w, mem, d_nodes, n_cap, d_n, d_scratch_h);
     if (peer != nullptr) {
       // one rank of the multi-GPU split: every world-th listed node from `rank`, rows delivered to all ranks
       a.peer = *peer;

@@ -184,7 +184,6 @@ __global__ void __launch_bounds__(1024) count_kernel(const __grid_constant__ Arg
     if (a.layers == 2 && a.mode == ORCA_MODE_NO_REUSE) sum = batch_rows * a.k;
     const int rows = batch_rows + sum;
     a.cnt->n_rows = rows;
-    for (int c = 0; c < a.n_chunks; ++c) a.cnt->n_chunk[c] = max(0, min(a.chunk, rows - c * a.chunk));
     if (a.status != nullptr) {     // counts of the last batch (status word layout, common.cuh)
       const int last = 3 * a.b_last;
       a.status[1] = a.budget() ? last + max(0, s_cand[a.nb - 1] - 1)
@@ -273,37 +272,6 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
   }
 }
 
-// ------------------------------------------------------------------------------------------------ memory chain
-// raw messages of one batch (state.cu: message_store_kernel), one block per memory update
-__global__ void __launch_bounds__(256)
-message_kernel(orca_memory_t mem, const float *log, const float *__restrict__ edge_table,
-               const float *__restrict__ time_w, const __grid_constant__ Args a, int n) {
-  dep_trigger();
-  dep_wait();
-  const int w = blockIdx.x;
-  if (w >= a.cnt->n_win[n]) return;
-  const int at = n * 2 * a.bs + w;
-  const int node = a.win_node[at];
-  const float t = a.win_t[at];
-  const int part = threadIdx.x / 64, lane = threadIdx.x % 64;
-  float *dst = mem.messages + (size_t)node * MSG + part * D;
-  auto row = [&](int r) { return (r >= a.n_nodes ? log : mem.memory) + (size_t)r * D; };
-  if (part < 3) {
-    const float *src = part == 0 ? row(a.win_mem[at]) : part == 1 ? row(a.win_other[at])
-                                                                 : edge_table + (size_t)a.win_eid[at] * D;
-    if (lane < D / 4) reinterpret_cast<float4 *>(dst)[lane] = reinterpret_cast<const float4 *>(src)[lane];
-  } else {
-    const float gap = a.win_gap[at];
-    for (int d = lane; d < D; d += 64) dst[d] = cos_any(gap * __ldg(time_w + d));
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {     // the update follows in this stream: times and flag as it leaves them
-    mem.msg_ts[node] = t;
-    mem.last_update[node] = t;
-    mem.msg_flag[node] = 0;
-  }
-}
-
 // ------------------------------------------------------------------------------------------------ last versions
 __device__ __forceinline__ void copy_row(float *dst, const float *src, int t) {
   if (t < D / 4) reinterpret_cast<float4 *>(dst)[t] = reinterpret_cast<const float4 *>(src)[t];
@@ -356,14 +324,10 @@ static int group_size(int bs, int k, int layers, int mode) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, 49152 / rows));
 }
 
-// Batches up to this size take the one-launch memory chain (chain.cu): its turns of 192 updates are cheaper than a pair
-// of launches per batch as long as a batch needs few of them, and it occupies the whole chip meanwhile.
-constexpr int CHAIN_MAX_BS = 1024;
-
 // Index buffers (two of each) and main-stream buffers.  The layer-1 rows that exist at all are few more than the
 // batches' own, but a batch with a cold cache can recompute every sampled neighbour: the projected queries and
-// attention sums (8.4 KB a row) are sized for `chunk` rows, and layer 1 runs over as many chunks as the worst case
-// has (the kernels of a chunk without rows return at once).
+// attention sums (9 KB a row) are sized for `chunk` rows, and layer 1 runs over as many chunks as there are: the
+// index kernels' row count comes back to the host while the group before is still being worked on.
 struct Parity {
   NodeBits *bits;
   Entry *table;
@@ -375,6 +339,7 @@ struct Parity {
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;
   char *stage;
+  void *upd_image;         // split inputs of the memory updates (chain.cu)
 };
 struct Buffers {
   Parity par[2];
@@ -384,7 +349,7 @@ struct Buffers {
   uint8_t *valid;
   uint32_t table_size, app_size;
   int64_t rows_max;        // layer-1 rows a group can have
-  int chunk, n_chunks;
+  int chunk;
   size_t stage_bytes, total;
 };
 
@@ -398,7 +363,6 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
   const int64_t apps = budget ? (int64_t)nb * (u_cap + 1) : no_reuse ? batch_rows * k : 0;
   w.rows_max = batch_rows + apps;
   w.chunk = (int)(no_reuse ? w.rows_max : std::min<int64_t>(w.rows_max, batch_rows + std::max<int64_t>(u_cap + 1, batch_rows / 4)));
-  w.n_chunks = (int)((w.rows_max + w.chunk - 1) / w.chunk);
   w.table_size = pow2_at_least(2 * batch_rows);
   w.app_size = pow2_at_least(budget ? 2 * apps : 1);
   w.stage_bytes = align_up((size_t)(4 * E + (int64_t)nb * plan_cap) * 4) + align_up((size_t)E * 8);
@@ -425,6 +389,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.win_t = (float *)take((size_t)2 * E * 4);
     x.win_gap = (float *)take((size_t)2 * E * 4);
     x.stage = (char *)take(w.stage_bytes);
+    x.upd_image = take(update_image_bytes(2 * E));
   }
   w.log = (float *)take((size_t)2 * 2 * E * D * 4);
   w.qt = (float *)take((size_t)w.chunk * QT_LD * 4);
@@ -438,7 +403,8 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
   return w;
 }
 
-static int launch_index(const Args &a, const float *last_update, size_t zero_bytes, cudaStream_t s, int sms) {
+static int launch_index(const Args &a, const float *last_update, size_t zero_bytes, int32_t *h_rows, cudaEvent_t counted,
+                        cudaStream_t s, int sms) {
   ORCA_CUDA(cudaMemsetAsync(a.bits, 0, zero_bytes, s));
   const int E = a.edges(), rows = 3 * E;
   const bool wide = a.k > 16;
@@ -448,6 +414,8 @@ static int launch_index(const Args &a, const float *last_update, size_t zero_byt
   else ORCA_CUDA(launch_dep(head_kernel<16>, grid_rows, 256, 0, s, a));
   ORCA_CUDA(launch_dep(mark_kernel, grid_slots, 256, 0, s, a));
   ORCA_CUDA(launch_dep(count_kernel, 1, 1024, 0, s, a));
+  ORCA_CUDA(cudaMemcpyAsync(h_rows, &a.cnt->n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  ORCA_CUDA(cudaEventRecord(counted, s));
   if (a.layers == 2 && a.mode != ORCA_MODE_REUSE_ALL) {
     const int grid = a.mode == ORCA_MODE_NO_REUSE ? sms * 16 : sms * 2;
     if (wide) ORCA_CUDA(launch_dep(append_kernel<32>, grid, 256, 0, s, a));
@@ -488,7 +456,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
                         float *d_prob, float *h_prob, int32_t *d_status, void *stream) {
   ORCA_CHECK_ARG(m && g && d_workspace && d_prob && d_status && g->h_i32 && g->h_ts && g->off_i32 && g->n_plan);
   ORCA_CHECK_ARG(g->nb > 0 && g->nb <= g->nb_max && g->nb_max <= grp::MAX_BATCHES && g->bs > 0 && g->b_last > 0 &&
-                 g->b_last <= g->bs && g->u_cap >= 0);
+                 g->b_last <= g->bs && g->u_cap >= 0 && g->h_rows && g->seq >= 0);
   ORCA_CHECK_ARG((m->n_layers == 1 || m->n_layers == 2) && m->k >= 1 && m->k <= ORCA_MAX_K && m->world <= 1);
   const int layers = m->n_layers, k = m->k, mode = layers == 2 ? m->mode : ORCA_MODE_BUDGET;
   ORCA_CHECK_ARG(mode == ORCA_MODE_BUDGET || mode == ORCA_MODE_REUSE_ALL || mode == ORCA_MODE_NO_REUSE);
@@ -504,15 +472,15 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   if ((int64_t)w.total > workspace_bytes)
     return set_error(ORCA_E_CAPACITY, "orca_tgn_eval_group: workspace of %lld bytes, %lld needed", (long long)workspace_bytes,
                      (long long)w.total);
-  ORCA_CHECK_ARG(w.n_chunks <= grp::MAX_CHUNKS && w.rows_max < (1 << grp::APP_ROW_BITS) &&
+  ORCA_CHECK_ARG(w.rows_max < (1 << grp::APP_ROW_BITS) &&
                  m->n_nodes + w.rows_max < INT_MAX);
-  const int p = (int)(c->gseq++ & 1);
+  const int p = (int)(g->seq & 1);
   const grp::Parity &x = w.par[p], &prev = w.par[p ^ 1];
   const int E_max = g->nb_max * g->bs;
   grp::Args a{};
   a.indptr = m->indptr, a.adj_nbr = m->adj_nbr, a.adj_eid = m->adj_eid, a.adj_ts = m->adj_ts, a.n_nodes = m->n_nodes;
   a.nb = g->nb, a.bs = g->bs, a.b_last = g->b_last, a.k = k, a.mode = mode, a.layers = layers;
-  a.u_cap1 = g->u_cap + 1, a.chunk = w.chunk, a.n_chunks = w.n_chunks;
+  a.u_cap1 = g->u_cap + 1;
   const int64_t base_i32 = g->off_i32[0];
   int64_t n_i32 = 0;
   for (int n = 0; n < g->nb; ++n) {
@@ -529,7 +497,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   a.cache_flag = m->cache_flag, a.status = d_status;
   a.bits = x.bits, a.table = x.table, a.app_table = x.app_table, a.cnt = x.cnt;
   a.table_mask = w.table_size - 1, a.app_mask = w.app_size - 1;
-  if (!g->first) a.prev_bits = prev.bits, a.prev_table = prev.table, a.prev_mask = w.table_size - 1;
+  if (g->seq > 0) a.prev_bits = prev.bits, a.prev_table = prev.table, a.prev_mask = w.table_size - 1;
   a.cand = x.cand, a.app_node = x.app_node, a.nbr1 = x.nbr1, a.eid1 = x.eid1, a.dt1 = x.dt1, a.nbr2 = x.nbr2;
   a.own1 = x.own1, a.score0 = x.score0, a.score1 = x.score1;
   a.win_node = x.win_node, a.win_eid = x.win_eid, a.win_mem = x.win_mem, a.win_other = x.win_other, a.win_t = x.win_t, a.win_gap = x.win_gap;
@@ -541,12 +509,12 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
 
   int32_t *saved_status = c->status_word;
   c->status_word = d_status;
-  launch_counter() = 0;
+  if (g->phase & 1) launch_counter() = 0;
   cudaStream_t s = (cudaStream_t)stream, si = c->overlap ? c->idx : s, sx = c->overlap ? c->aux : s;
-  auto body = [&]() -> int {
+  auto prepare = [&]() -> int {
     // ---- inputs and index stream
     cudaStream_t sc = c->overlap ? c->copy : s;
-    if (g->first) {
+    if (g->seq == 0) {
       ORCA_CUDA(cudaEventRecord(c->ev_gin, s));
       if (sc != s) ORCA_CUDA(cudaStreamWaitEvent(sc, c->ev_gin, 0));
       c->gdone_recorded[0] = c->gdone_recorded[1] = false;
@@ -558,50 +526,49 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
       ORCA_CUDA(cudaEventRecord(c->ev_gin, sc));
       ORCA_CUDA(cudaStreamWaitEvent(si, c->ev_gin, 0));
     }
-    ORCA_TRY(grp::launch_index(a, m->mem.last_update, x.zero_bytes, si, c->sm_count));
-    if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_gidx[p], si));
+    ORCA_TRY(grp::launch_index(a, m->mem.last_update, x.zero_bytes, g->h_rows + p, c->ev_gcount[p], si, c->sm_count));
+    if (si != sx) {
+      ORCA_CUDA(cudaEventRecord(c->ev_gidx[p], si));
+      ORCA_CUDA(cudaStreamWaitEvent(sx, c->ev_gidx[p], 0));
+    }
     if (budget) {
       const int last = g->nb - 1;
       ORCA_TRY(launch_plan_flags(m, a.img + a.off[last] + 4 * g->b_last, a.n_plan[last], si));
     }
+    if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_gidx[p], si));     // (from here on: index work and flags)
     // ---- memory chain
-    if (sx != s) ORCA_CUDA(cudaStreamWaitEvent(sx, c->ev_gidx[p], 0));
-    if (g->bs <= grp::CHAIN_MAX_BS) {
-      grp::ChainArgs ch{a, m->mem, log, w.log + (size_t)p * 2 * E_max * D, m->edge_table, m->time_w, m->gru.Wg_chain, m->gru.bg,
-                        nullptr, 0};
-      ORCA_TRY(grp::launch_gru_chain(ch, sx));
-    } else {
-      for (int n = 0; n < g->nb; ++n) {
-        const int b = a.b_of(n), at = n * 2 * g->bs;
-        ORCA_CUDA(launch_dep(grp::message_kernel, 2 * b, 256, 0, sx, m->mem, log, m->edge_table, m->time_w, a, n));
-        ORCA_COUNT_LAUNCH();
-        ORCA_TRY(gru_project_rows(&m->gru, &m->mem, x.win_node + at, x.win_mem + at, log, (int)m->n_nodes, 2 * b,
-                                  &x.cnt->n_win[n], w.log + (size_t)(p * 2 * E_max + at) * D, sx));
-      }
-    }
+    grp::ChainArgs ch{a, m->mem, log, w.log + (size_t)p * 2 * E_max * D, m->edge_table, m->time_w, m->gru.Wg_chain, m->gru.bg,
+                      x.upd_image, nullptr, 0};
+    ORCA_TRY(grp::launch_gru_chain(ch, sx));
+    if (sx != s) ORCA_CUDA(cudaEventRecord(c->ev_gchain[p], sx));
+    return ORCA_OK;
+  };
+  auto finish = [&]() -> int {
+    ORCA_CUDA(cudaEventSynchronize(c->ev_gcount[p]));
+    const int n_rows = g->h_rows[p];
+    ORCA_CHECK_ARG(n_rows >= 3 * E && n_rows <= w.rows_max);
     if (sx != s) {
-      ORCA_CUDA(cudaEventRecord(c->ev_gchain[p], sx));
       ORCA_CUDA(cudaStreamWaitEvent(s, c->ev_gchain[p], 0));
+      ORCA_CUDA(cudaStreamWaitEvent(s, c->ev_gidx[p], 0));
     }
-    // ---- main stream
     int32_t *tk = c->d_words + CTX_TICKET_MAIN;
-    auto output = [&](int layer, int cap, const int32_t *d_n, float *out) {
+    auto output = [&](int layer, int rows, float *out) {
       OutArgs o{};
-      o.w = m->attn[layer], o.ctx = w.ctx, o.feat = layer == 0 ? w.feat : w.feat2, o.valid = w.valid, o.n_cap = cap, o.d_n = d_n, o.out = out;
+      o.w = m->attn[layer], o.ctx = w.ctx, o.feat = layer == 0 ? w.feat : w.feat2, o.valid = w.valid, o.n_cap = rows;
+      o.out = out;
       return o;
     };
-    for (int ch = 0; ch < w.n_chunks; ++ch) {
-      const int64_t r0 = (int64_t)ch * w.chunk;
-      const int cap = (int)std::min<int64_t>(w.chunk, w.rows_max - r0);
-      const int32_t *d_n = &x.cnt->n_chunk[ch];
+    for (int r0 = 0; r0 < n_rows; r0 += w.chunk) {
+      const int rows = std::min(w.chunk, n_rows - r0);
+      const size_t slot = (size_t)r0 * k;
       const tc::RowSrc own{m->mem.memory, x.own1 + r0, D, 0, 0, log, (int)m->n_nodes};
-      ORCA_TRY(feat_image(own, cap, d_n, w.feat, s));
-      ORCA_TRY(attn_query_image(&m->attn[0], w.feat, cap, d_n, w.qt, s));
-      ORCA_TRY(launch_attn_gather(w.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1 + r0 * k, x.eid1 + r0 * k,
-                                  x.dt1 + r0 * k, k, cap, d_n, 0, nullptr, w.ctx, true, w.valid, tk, s, log, (int)m->n_nodes));
-      OutArgs o = output(0, cap, d_n, w.emb1 + r0 * D);
+      ORCA_TRY(feat_image(own, rows, nullptr, w.feat, s));
+      ORCA_TRY(attn_query_image(&m->attn[0], w.feat, rows, nullptr, w.qt, s));
+      ORCA_TRY(launch_attn_gather(w.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1 + slot, x.eid1 + slot, x.dt1 + slot, k,
+                                  rows, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, log, (int)m->n_nodes));
+      OutArgs o = output(0, rows, w.emb1 + (size_t)r0 * D);
       // (the batch rows are layer 2's rows; they all lie in the first chunk)
-      if (layers == 2 && ch == 0) o.out_image = w.feat2, o.out_image_rows = 3 * E;
+      if (layers == 2 && r0 == 0) o.out_image = w.feat2, o.out_image_rows = 3 * E;
       ORCA_TRY(attn_output_rows(o, s));
     }
     const float *top = w.emb1;
@@ -610,7 +577,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
       // (without reuse every row lies in the layer-1 output: the first part is never read)
       ORCA_TRY(launch_attn_gather(w.qt, history ? m->hist_emb : m->mem.memory, m->edge_table, m->time_w, x.nbr2, x.eid1,
                                   x.dt1, k, 3 * E, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, emb, (int)m->n_nodes));
-      ORCA_TRY(attn_output_rows(output(1, 3 * E, nullptr, w.emb2), s));
+      ORCA_TRY(attn_output_rows(output(1, 3 * E, w.emb2), s));
       top = w.emb2;
     }
     // (positions of a short last batch's scores: the arrays are indexed by 2 * bs per batch, only the last is short)
@@ -619,13 +586,13 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
                          m->hist_emb));
     ORCA_COUNT_LAUNCH();
     if (h_prob != nullptr) ORCA_CUDA(cudaMemcpyAsync(h_prob, d_prob, (size_t)2 * E * 4, cudaMemcpyDeviceToHost, s));
-    if (si != s) {      // the caller's stream is behind everything the group enqueued
-      ORCA_CUDA(cudaEventRecord(c->ev_gidx[p], si));
-      ORCA_CUDA(cudaStreamWaitEvent(s, c->ev_gidx[p], 0));
-    }
     ORCA_CUDA(cudaEventRecord(c->ev_gdone[p], s));
     c->gdone_recorded[p] = true;
     return ORCA_OK;
+  };
+  auto body = [&]() -> int {
+    if (g->phase & 1) ORCA_TRY(prepare());
+    return g->phase & 2 ? finish() : ORCA_OK;
   };
   const int rc = body();
   c->status_word = saved_status;

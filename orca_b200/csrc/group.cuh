@@ -8,7 +8,6 @@ namespace grp {
 
 constexpr int MAX_BATCHES = ORCA_GROUP_MAX;   // (a batch is a bit of a 32-bit word)
 static_assert(MAX_BATCHES <= 32, "a batch of the group is a bit of a 32-bit word");
-constexpr int MAX_CHUNKS = 32;                // row chunks of layer 1 (see Layout::chunk)
 
 // What the batches of the group do with a node: bit n belongs to batch n.
 struct NodeBits {
@@ -30,7 +29,6 @@ struct Counters {
   int32_t dropped[MAX_BATCHES];            // smallest candidate of the batch (-1: none): it is not recomputed
   int32_t app_off[MAX_BATCHES + 1];        // first recomputed row of the batch, counted from the group's first
   int32_t n_rows;                          // layer-1 rows of the group
-  int32_t n_chunk[MAX_CHUNKS];             // of them in every chunk
   double t_max[MAX_BATCHES];               // latest query time of the batch
   int32_t arrived[MAX_BATCHES];            // CTAs of the memory chain that have finished the batch
 };
@@ -45,7 +43,6 @@ struct Args {
   const double *ts;                 // times of batch n at n * bs
   int nb, bs, b_last, k, mode, layers;
   int u_cap1;                       // candidates a batch can have (list capacity)
-  int chunk, n_chunks;              // layer-1 rows per chunk
   int off[MAX_BATCHES], n_plan[MAX_BATCHES];
   const uint8_t *cache_flag;        // flags before the group's first batch
   int32_t *status;

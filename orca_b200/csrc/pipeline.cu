@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "attn_out.cuh"
+#include "chain.cuh"
 #include "common.cuh"
 #include "context.cuh"
 #include "index_ops.cuh"
@@ -45,6 +46,8 @@ struct IdxBuf {
   int32_t *cat_dst; int32_t *win_pos; int32_t *n_win; int32_t *win_nodes;
   int32_t *loc_nodes; double *loc_ts; int32_t *n1_loc;               // sharded layer 1
   int32_t *feat_idx; int32_t *nbr2_loc, *eid2_loc; float *dt2_loc;  // sharded layer 2 / no-reuse index
+  int32_t *upd_node, *upd_other, *upd_eid; float *upd_t;   // memory updates of the batch (chain.cu)
+  grp::Counters *cnt;                                       // of which n_win[0] is their number
   int32_t *order1, *order2;                    // rows of the two gather launches, heaviest first
 };
 // projection / gather buffers of one attention layer in flight (one set per compute lane)
@@ -61,6 +64,7 @@ struct Workspace {
   float *emb2;
   uint8_t *win1;
   float *gru_h;
+  void *upd_image;           // split inputs of the memory updates (chain.cu)
   void *bitmap;
   size_t bytes;
 };
@@ -85,7 +89,12 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
     x.dt2 = (float *)take(N * k * 4);
     x.cat_dst = (int32_t *)take(2 * (size_t)b_cap * 4);
     x.win_pos = (int32_t *)take(2 * (size_t)b_cap * 4);
-    x.n_win = (int32_t *)take(4);
+    x.cnt = (grp::Counters *)take(sizeof(grp::Counters));
+    x.n_win = x.cnt != nullptr ? &x.cnt->n_win[0] : nullptr;
+    x.upd_node = (int32_t *)take(2 * (size_t)b_cap * 4);
+    x.upd_other = (int32_t *)take(2 * (size_t)b_cap * 4);
+    x.upd_eid = (int32_t *)take(2 * (size_t)b_cap * 4);
+    x.upd_t = (float *)take(2 * (size_t)b_cap * 4);
     x.win_nodes = (int32_t *)take(2 * (size_t)b_cap * 4);
     x.loc_nodes = (int32_t *)take(R1 * 4);
     x.loc_ts = (double *)take(R1 * 8);
@@ -110,6 +119,7 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
   w.emb2 = (float *)take(N * D * 4);
   w.win1 = (uint8_t *)take(R1);
   w.gru_h = (float *)take(2 * (size_t)b_cap * D * 4);
+  w.upd_image = take(grp::update_image_bytes(2 * (int64_t)b_cap));
   w.bitmap = take((size_t)orca_find_uncached_scratch_bytes(n_nodes));
   w.bytes = off;
   return w;
@@ -389,6 +399,16 @@ static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d
   return attn_output_rows(a, s);
 }
 
+// Raw messages and GRU of a batch by the memory chain's kernel (chain.cu), or as a pair of launches (fp32 projections,
+// multi-GPU, and batches of more than 1024 edges: there the chain's kernel takes several turns on most of the chip while
+// the layers beside it want it; 2000 edges: 131 us a call with the pair, 141 with the chain)
+static bool one_launch_updates(int b) { return projections_on_tensor_cores() && b <= 1024; }
+static UpdateList updates_of(const IdxBuf &x, const double *d_ts) {
+  UpdateList u;
+  u.ts = d_ts, u.node = x.upd_node, u.other = x.upd_other, u.eid = x.upd_eid, u.t = x.upd_t;
+  return u;
+}
+
 static Ctx *ctx_of(const orca_tgn_t *m) {
   return m->ctx != nullptr ? reinterpret_cast<Ctx *>(m->ctx) : default_ctx();
 }
@@ -489,14 +509,22 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
 
   // raw messages of the batch (last occurrence per node in [src|dst]) and the memory update
   cudaStream_t ms = forked ? c->aux : s;
+  const bool single = one_launch_updates(b);
   ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, *m->epoch_base, x.win_pos, x.n_win,
-                                   d_status, ms));
+                                   d_status, ms, updates_of(x, d_batch_ts)));
   *m->epoch_base += 2 * b;
   ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
+  if (single) {
+    ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid, x.upd_t,
+                                    x.cnt, w.upd_image, w.gru_h, ms));
+    ORCA_TRY(tr.mark(PH_MESSAGE, s));
+    ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, ms));
+  } else {
   ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
                               d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, ms));
   ORCA_TRY(tr.mark(PH_MESSAGE, s));
   ORCA_TRY(orca_gru_update(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, ms));
+  }
   ORCA_TRY(tr.mark(PH_GRU, s));
   if (forked) ORCA_TRY(link(c->aux, s, c->join));
   publish_counts_kernel<<<1, 1, 0, s>>>(x.n1, x.n_win, d_status);
@@ -611,8 +639,9 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
       ORCA_TRY(launch_row_order(x.nbr1, R1, x.n1, x.order1, x.nbr1, N, nullptr, x.order2, k, si));
     ORCA_TRY(tr.mark(PH_SAMPLE_L1, s));
     // winners of the raw messages: last occurrence per node in [src|dst] (model/tgn_model.py:172-176)
+    const bool single = !sharded && one_launch_updates(b);
     ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, c->base_msg, x.win_pos, x.n_win,
-                                     d_status, si));
+                                     d_status, si, updates_of(x, d_batch_ts)));
     ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
     if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_idx[p], si));
     // cache flags of this batch (History.update_flag): read next by the next batch's head kernel
@@ -636,10 +665,14 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
       if (si != s) ORCA_CUDA(cudaStreamWaitEvent(sx, c->ev_idx[p], 0));
       else ORCA_TRY(link(s, sx, c->fork));
     }
-    ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
-                                d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, sx));
+    if (!single)
+      ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
+                                  d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, sx));
     ORCA_TRY(tr.mark(PH_MESSAGE, s));
-    if (gru_split && !in_a) {
+    if (single) {
+      ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid,
+                                      x.upd_t, x.cnt, w.upd_image, w.gru_h, sx));
+    } else if (gru_split && !in_a) {
       // (split by layer: the layer-1 ranks compute the memory update; this rank only receives the rows)
     } else if (gru_split) {
       // the memory update is split by node: this rank computes every wa-th unique positive and stores the
@@ -728,7 +761,8 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     // ------------------------------------------------------------------ side lane: the memory table is written
     if (!gru_split) {
       ORCA_TRY(wait_on(sx, sa, c->ev_o1));
-      ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, sx));
+      if (!sharded && one_launch_updates(b)) ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, sx));
+      else ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, sx));
       if (sx != s) {
         ORCA_CUDA(cudaEventRecord(c->ev_state, sx));
         c->state_recorded = true;

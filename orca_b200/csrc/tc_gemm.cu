@@ -112,7 +112,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       b[k] = has1 ? add4(ld_shared_f4(ra + 512u), bB) : f4z;
       hA[k] = hB[k] = 0.f;
       if (EPI == EPI_GRU && ok[k]) {
-        const float *hrow = (g.memory2 != nullptr && mb[k] >= g.memory_split ? g.memory2 : g.memory) + (size_t)mb[k] * D;
+        const float *hrow = g.memory + (size_t)mb[k] * D;
         if (uA < D) hA[k] = hrow[uA];
         if (has1 && uB < D) hB[k] = hrow[uB];
       }
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
         }
         const bool in0 = c < w0;
         const int r = in0 ? r0 : r1;
-        const float *bp = in0 ? g.a0.base(r) + (size_t)r * w0 + c : g.a1.base(r) + (size_t)r * w1 + (c - w0);
+        const float *bp = in0 ? g.a0.p + (size_t)r * w0 + c : g.a1.p + (size_t)r * w1 + (c - w0);
         x[2 * i + h] = *((c >= Kd || r < 0) ? zero : reinterpret_cast<const float4 *>(bp));
       }
     }

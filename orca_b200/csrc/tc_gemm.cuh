@@ -98,8 +98,6 @@ struct Args {
   // GRU
   const float *memory;
   const int32_t *nodes;
-  const float *memory2;      // optional: rows >= memory_split (as in RowSrc)
-  int memory_split;
   // SCORE
   const float *w2;
   float b2;
@@ -119,12 +117,9 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
                      float *d_push_table, const int32_t *d_push_ids, const uint8_t *d_push_win,
                      const int64_t *d_last_pos, long long base, int all_from, float *d_scratch_hidden,
                      cudaStream_t stream);
-// scorer and GRU over the rows of a group of batches (gemm.cu); tensor cores only
+// scorer over the rows of a group of batches (gemm.cu); tensor cores only
 int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
                float *d_prob, cudaStream_t s);
-int gru_project_rows(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes,
-                     const int32_t *d_mem_rows, const float *mem2, int mem_split, int n_cap, const int32_t *d_n,
-                     float *d_out, cudaStream_t s);
 // whether the projections run on the tensor cores (orca_set_projection_mode(0)); the fp32 debug path has
 // no peer fan-out
 bool projections_on_tensor_cores();

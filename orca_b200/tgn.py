@@ -897,8 +897,10 @@ class TGN(nn.Module):
         hi, hts, d_prob = h_i32.numpy(), h_ts.numpy(), keep["d_prob"]
         desc = self._descriptor(k)
         stream = torch.cuda.current_stream(self.device)
-        # the library never waits for the host: while the GPU works on a group the next one is packed
-        for i0 in range(0, nb, nb_max):
+        h_rows = pinned("rows", 2, torch.int32)
+        groups = []
+
+        def prepare(i0):
             i1 = min(nb, i0 + nb_max)
             lo, up = i0 * bs, min(E, i1 * bs)
             hts[lo:up] = timestamps[lo:up]
@@ -912,9 +914,23 @@ class TGN(nn.Module):
                 if n_plan[i]:
                     hi[o + 4 * n:off[i + 1]] = cache_plan[i]
             g = _lib.GroupT(h_i32.data_ptr(), h_ts.data_ptr() + 8 * lo, off.ctypes.data + 8 * i0, n_plan.ctypes.data + 4 * i0,
-                            i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap, i0 == 0)
+                            h_rows.data_ptr(), len(groups), 1, i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap)
+            groups.append((g, lo))
+            enqueue(g, lo)
+
+        def enqueue(g, lo):
             _lib.check(L.orca_tgn_eval_group(desc, C.byref(g), ws.data_ptr(), ws.numel(), d_prob.data_ptr() + 8 * lo,
                                              h_prob.data_ptr() + 8 * lo, self._status.data_ptr(), stream.cuda_stream))
+
+        # a group's index work and memory updates are enqueued ahead of the layers of the group before it
+        starts = range(0, nb, nb_max)
+        prepare(0)
+        for j in range(len(starts)):
+            if j + 1 < len(starts):
+                prepare(starts[j + 1])
+            g, lo = groups[j]
+            g.phase = 2
+            enqueue(g, lo)
         stream.synchronize()
         # per batch [pos | neg]; the last batch may be short
         scores, full = h_prob.numpy()[:2 * E], E // bs
