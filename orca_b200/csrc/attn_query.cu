@@ -5,7 +5,7 @@
 // attn_query_image_kernel takes the rows as an operand image (attn_out.cuh): one thread streams 16 KB stages through a
 // ring, one multiplies, eight warps carry the other accumulator buffer from tensor memory to qt, a thread per row and
 // 32 bytes a store (whole sectors, no staging).  51 k rows: 155 us for the general projection kernel (six column
-// tiles, weights streamed again for every row block, load, product and store one after the other), TODO us here.
+// tiles, weights streamed again for every row block, load, product and store one after the other), 75 here.
 // attn_query_kernel takes the rows as floats and splits them itself, eleven times over (170 us): it serves the callers
 // that have no buffer for an image.
 #include <algorithm>
