@@ -373,8 +373,9 @@ class TGN(nn.Module):
             self._prepared = {
                 "time_w": torch.from_numpy(weights.prepare_time(sd)).to(dev),
                 "attn": [up(weights.prepare_attention(sd, l, pack=False)) for l in range(self.n_layers)],
-                "score": up(weights.prepare_score(sd)),
+                "score": up(weights.prepare_score(sd, pack=False)),
             }
+            self._prepared["score"]["W1t_tc"] = weights.pack_tc(self._prepared["score"]["W1t"])
             for a in self._prepared["attn"]:
                 a.update(weights.packed_attention(a))
         return self._prepared

@@ -169,10 +169,10 @@ def prepare_gru(sd, dim: int = D, pack: bool = True):
     return out
 
 
-def prepare_score(sd):
+def prepare_score(sd, pack: bool = True):
     W1t = np.ascontiguousarray(_f64(sd["affinity_score.fc1.weight"]).T, dtype=np.float32)
     return {
-        "W1t": W1t, "W1t_tc": pack_tc(W1t),
+        "W1t": W1t, **({"W1t_tc": pack_tc(W1t)} if pack else {}),
         "b1": np.asarray(sd["affinity_score.fc1.bias"], dtype=np.float32),
         "w2": np.ascontiguousarray(np.asarray(sd["affinity_score.fc2.weight"], dtype=np.float32).reshape(-1)),
         "b2": float(np.asarray(sd["affinity_score.fc2.bias"]).reshape(-1)[0]),
