@@ -1,18 +1,22 @@
 // LRU and 2Q cache planning on the device (utils/cache.py:338-403 and 175-333, with read_batches :19-89).
 //
 // Both policies walk the batches in order and evict at random: numba's np.random.choice(..., replace=False)
-// is a Fisher-Yates shuffle driven by its private Mersenne Twister, first entries kept.  One draw decides
-// the next swap and how many draws a swap consumes depends on the draws themselves (rejection sampling), so
-// the shuffle is one serial chain per batch: thread 0 of the block walks it, generator state in shared
-// memory.  Everything around it is data parallel over the block: the split of the batch's neighbour table
-// into targets / out-of-batch neighbours (stamps), the reuse statistics, sets as bitmaps that list their
-// members in ascending order by a popcount scan (np.unique / np.where of the reference), and the LRU
-// evictions, which are the first entries of numba's argsort of the last-use times (tie_order.cuh).
-// One CTA of 1024 threads per plan.
+// is a Fisher-Yates shuffle driven by its private Mersenne Twister, first entries kept.  How many numbers a swap
+// consumes depends on the numbers (rejection sampling), but not on what is shuffled: one warp takes the generator's
+// numbers 32 at a time and finds by votes which of them are accepted and for which swap.  The swaps themselves are one
+// serial chain, in shared memory, and are left out where the whole list is taken whatever its order.
+// The rest is data parallel over the block: the split of the batch's neighbour table into targets / out-of-batch
+// neighbours (stamps; eight entries a thread at a time, so that their loads overlap), the reuse statistics, sets as
+// bitmaps that list their members in ascending order by a popcount scan (np.unique / np.where of the reference), and
+// the LRU evictions, which are the first entries of numba's argsort of the last-use times (tie_shared.cuh, or
+// tie_order.cuh for lists that do not fit shared memory).
+// One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
+// 250 batches of 600 edges with 20 neighbours, LRU: 19.2 ms a plan with draws, swaps, bitmaps and sort
+// in global memory, 11.4 here.
 #include <algorithm>
 
 #include "common.cuh"
-#include "tie_order.cuh"
+#include "tie_shared.cuh"
 
 namespace orca {
 namespace rnd {
@@ -30,37 +34,54 @@ struct Twister {
     for (int i = 1; i < N; ++i) s[i] = 1812433253u * (s[i - 1] ^ (s[i - 1] >> 30)) + (uint32_t)i;
     pos = N;
   }
+  // The rest by one warp.  A chunk of 32 words needs words of later chunks (still old) and words 227 places back.
   __device__ void refill() {
-    for (int i = 0; i < N; ++i) {
-      const uint32_t y = (s[i] & 0x80000000u) | (s[(i + 1) % N] & 0x7fffffffu);
-      s[i] = s[(i + M) % N] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-    }
-    pos = 0;
-  }
-  __device__ uint32_t next() {
-    if (pos >= N) refill();
-    uint32_t y = s[pos++];
-    y ^= y >> 11;
-    y ^= (y << 7) & 0x9d2c5680u;
-    y ^= (y << 15) & 0xefc60000u;
-    return y ^ (y >> 18);
-  }
-  __device__ int below(int n) {   // n <= 2^31 here
-    if (n <= 1) return 0;
-    const uint32_t mask = 0xffffffffu >> __clz((unsigned)(n - 1));
-    while (true) {
-      const uint32_t r = next() & mask;
-      if (r < (uint32_t)n) return (int)r;
+    const int lane = threadIdx.x & 31;
+    for (int i0 = 0; i0 < N; i0 += 32) {
+      const int i = i0 + lane;
+      uint32_t v = 0;
+      if (i < N) {
+        const uint32_t y = (s[i] & 0x80000000u) | (s[(i + 1) % N] & 0x7fffffffu);
+        v = s[(i + M) % N] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+      }
+      __syncwarp();
+      if (i < N) s[i] = v;
+      __syncwarp();
     }
   }
-  // Fisher-Yates from the back, as numba shuffles; the caller keeps the first entries
-  __device__ void shuffle(int32_t *x, int n) {
-    for (int i = n - 1; i > 0; --i) {
-      const int j = below(i + 1);
-      const int32_t a = x[i];
-      x[i] = x[j];
-      x[j] = a;
+  // The draws of a shuffle of n entries, from the back: entry i swaps with draw[i] (draw may be null: the generator
+  // moves on all the same).  Number l of a group of 32 is accepted iff it lies below its bound, which falls by one for
+  // every number accepted before it: the votes settle from the left, in two or three rounds as a rule, 33 at most.
+  __device__ void draws(int n, int32_t *draw) {
+    const int lane = threadIdx.x & 31;
+    int at = pos;
+    while (n > 1) {
+      if (at >= N) {
+        refill();
+        at = 0;
+      }
+      const bool have = lane < N - at;
+      uint32_t y = have ? s[at + lane] : 0;
+      y ^= y >> 11;
+      y ^= (y << 7) & 0x9d2c5680u;
+      y ^= (y << 15) & 0xefc60000u;
+      y ^= y >> 18;
+      uint32_t accepted = 0, r = 0;
+      int bound = 0;
+      for (int round = 0; round <= 33; ++round) {
+        bound = n - __popc(accepted & ((1u << lane) - 1u));
+        r = bound > 1 ? y & (0xffffffffu >> __clz(bound - 1)) : 0;
+        const uint32_t a = __ballot_sync(0xffffffffu, have && bound > 1 && r < (uint32_t)bound);
+        if (a == accepted) break;
+        accepted = a;
+      }
+      if (draw != nullptr && ((accepted >> lane) & 1u)) draw[bound - 1] = (int32_t)r;
+      at += __popc(__ballot_sync(0xffffffffu, have && bound > 1));
+      n -= __popc(accepted);
     }
+    __syncwarp();
+    if (lane == 0) pos = at;
+    __syncwarp();
   }
 };
 
@@ -71,23 +92,27 @@ struct Work {
   int32_t *list[4];               // [cap] member lists
   tie::Buf sort;
   int64_t cap;
+  int cap_shared;                 // entries of a list in shared memory
+  bool bm_shared;                 // the bitmaps, and one of the targets in place of the stamps, lie behind them
 };
 
-// (bitmap words are changed by atomics, which act in L2: they are read from there, not through L1)
-__device__ __forceinline__ bool bit(const uint32_t *bm, int32_t v) { return (__ldcg(&bm[v >> 5]) >> (v & 31)) & 1u; }
+// (bitmaps lie in shared memory where they fit, else in global memory, where their words are changed by atomics, which
+// act in L2: they are read from there, not through L1)
+__device__ __forceinline__ uint32_t word(const uint32_t *bm, int64_t i) { return *(const volatile uint32_t *)&bm[i]; }
+__device__ __forceinline__ bool bit(const uint32_t *bm, int32_t v) { return (word(bm, v >> 5) >> (v & 31)) & 1u; }
 __device__ __forceinline__ void set_bit(uint32_t *bm, int32_t v) { atomicOr(&bm[v >> 5], 1u << (v & 31)); }
 __device__ __forceinline__ void clear_bit(uint32_t *bm, int32_t v) { atomicAnd(&bm[v >> 5], ~(1u << (v & 31))); }
 
 // Members of a bitmap in ascending order -> out; returns their number (the same in every thread).  All T
 // threads call it; `clear` empties the bitmap on the way.  s_cnt: NW ints of shared memory.
-__device__ int list_members(uint32_t *bm, int64_t words, int32_t *out, bool clear, int *s_cnt) {
+__device__ __forceinline__ int list_members(uint32_t *bm, int64_t words, int32_t *out, bool clear, int *s_cnt) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wchunk = (int)(((words + NW - 1) / NW + 31) & ~31ll);
   __syncthreads();   // (earlier writes to the bitmap; earlier readers of s_cnt)
   int cnt = 0;
   for (int j = lane; j < wchunk; j += 32) {
     const int64_t wi = (int64_t)warp * wchunk + j;
-    if (wi < words) cnt += __popc(__ldcg(&bm[wi]));
+    if (wi < words) cnt += __popc(word(bm, wi));
   }
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   if (lane == 0) s_cnt[warp] = cnt;
@@ -102,7 +127,7 @@ __device__ int list_members(uint32_t *bm, int64_t words, int32_t *out, bool clea
     const int64_t wi = (int64_t)warp * wchunk + j + lane;
     uint32_t bits = 0;
     if (wi < words) {
-      bits = __ldcg(&bm[wi]);
+      bits = word(bm, wi);
       if (clear && bits) bm[wi] = 0;
     }
     const int c = __popc(bits);
@@ -122,10 +147,49 @@ __device__ int list_members(uint32_t *bm, int64_t words, int32_t *out, bool clea
   return n;
 }
 
+// Fisher-Yates of x[0 .. n) from the back, as numba shuffles; the caller keeps the first entries.  `any_order`: the
+// caller keeps all of them, so that only the generator has to move.  All T threads call it.
+__device__ void shuffle(const Work &w, Twister &rng, int32_t *x, int n, bool any_order) {
+  __syncthreads();
+  if (any_order) {
+    if (threadIdx.x < 32) rng.draws(n, nullptr);
+    __syncthreads();
+    return;
+  }
+  const bool fits = n <= w.cap_shared;
+  int32_t *at = fits ? (int32_t *)tie::smem : x, *draw = fits ? at + w.cap_shared : w.sort.lpos;
+  if (threadIdx.x < 32) rng.draws(n, draw);
+  if (fits)
+    for (int i = threadIdx.x; i < n; i += T) at[i] = x[i];
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int i = n - 1; i > 0; --i) {
+      const int j = draw[i];
+      const int32_t a = at[i];
+      at[i] = at[j];
+      at[j] = a;
+    }
+  __syncthreads();
+  if (fits)
+    for (int i = threadIdx.x; i < n; i += T) x[i] = at[i];
+  __syncthreads();
+}
+
 // the first `count` entries of numba's argsort of key[ids[i]] (i < n): calls f(id) for each of them
 template <class F>
 __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int count, const int32_t *key, int *s_a,
                                  int *s_b, F f) {
+  if (n <= w.cap_shared) {
+    const tie::Shared sh{w.cap_shared};
+    for (int i = threadIdx.x; i < n; i += T) {
+      sh.key(i) = key[ids[i]];
+      sh.idx(i) = (uint16_t)i;
+    }
+    const auto use = [&](int, int i) { f(ids[i]); };
+    if (n <= 4 * T) tie::sort_first_shared<4>(sh, (uint32_t *)s_a, n, count, use);
+    else tie::sort_first_shared<20>(sh, (uint32_t *)s_a, n, count, use);
+    return true;
+  }
   for (int i = threadIdx.x; i < n; i += T) w.sort.e[i] = ((uint64_t)(uint32_t)key[ids[i]] << 32) | (uint32_t)i;
   __syncthreads();
   if (!tie::sort_first(w.sort, n, count, s_a, s_b)) return false;
@@ -133,6 +197,51 @@ __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int c
     if (tie::place_of(w.sort, pos, count) >= 0) f(ids[(uint32_t)w.sort.e[pos]]);
   __syncthreads();
   return true;
+}
+
+// The bitmaps of a plan (SH: in shared memory, behind the lists); one more for the targets of a batch if so.
+constexpr int N_BM = 5;
+template <bool SH>
+__device__ __forceinline__ uint32_t *bitmap(const Work &w, int i, int64_t words) {
+  return SH ? (uint32_t *)(tie::smem + tie::Shared::BYTES * w.cap_shared) + i * words : w.bm[i];
+}
+template <bool SH>
+__device__ void clear_bitmaps(const Work &w, int64_t words) {
+  for (int64_t i = threadIdx.x; i < (SH ? N_BM + 1 : N_BM) * words; i += T)
+    bitmap<SH>(w, SH ? 0 : (int)(i / words), words)[SH ? i : i % words] = 0;
+}
+
+// Calls use(v, load(v)) for the out-of-batch entries of a batch's neighbour table, eight entries a thread at a time.
+// Most entries are targets or padding: `load` is left to the others, since one block's scattered loads are what this
+// phase waits for.
+constexpr int STEP = 8;
+template <bool SH, class Load, class Use>
+__device__ __forceinline__ void for_neighbors(const Work &w, uint32_t *target, const int32_t *q, int m2, const int32_t *tab, int n,
+                              int32_t now, Load load, Use use) {
+  for (int i = threadIdx.x; i < m2; i += T) {
+    if (SH) set_bit(target, q[i]);
+    else w.stamp[q[i]] = now;
+  }
+  __syncthreads();
+  for (int i0 = threadIdx.x; i0 < n; i0 += STEP * T) {
+    int32_t v[STEP];
+    bool out[STEP];
+    decltype(load(0)) x[STEP];
+#pragma unroll
+    for (int u = 0; u < STEP; ++u) v[u] = i0 + u * T < n ? tab[i0 + u * T] : 0;
+#pragma unroll
+    for (int u = 0; u < STEP; ++u) out[u] = v[u] != 0 && !(SH ? bit(target, v[u]) : w.stamp[v[u]] == now);
+#pragma unroll
+    for (int u = 0; u < STEP; ++u)
+      if (out[u]) x[u] = load(v[u]);
+#pragma unroll
+    for (int u = 0; u < STEP; ++u)
+      if (out[u]) use(v[u], x[u]);
+  }
+  if (SH) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < m2; i += T) target[q[i] >> 5] = 0;
+  }
 }
 
 struct Totals {
@@ -153,7 +262,8 @@ __device__ void write_totals(const Totals &t, int64_t *stats) {
 }
 
 // ------------------------------------------------------------------------------ LRU (utils/cache.py:338-403)
-__global__ void __launch_bounds__(T) lru_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
+template <bool SH>
+__global__ void __launch_bounds__(T, 1) lru_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
                                                 int32_t k, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
                                                 int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
                                                 int32_t *status) {
@@ -161,7 +271,9 @@ __global__ void __launch_bounds__(T) lru_kernel(const int32_t *nodes, const int3
   __shared__ int s_a[NW], s_b[NW];
   const int tid = threadIdx.x;
   const int64_t nb = (n_edges + bs - 1) / bs, words = (n_nodes + 31) / 32;
-  uint32_t *cached = w.bm[0], *candbm = w.bm[1];
+  clear_bitmaps<SH>(w, words);
+  uint32_t *cached = bitmap<SH>(w, 0, words), *candbm = bitmap<SH>(w, 1, words);
+  uint32_t *target = SH ? bitmap<SH>(w, N_BM, words) : nullptr;
   int32_t *used_at = w.t0, *arrived = w.t1;
   int32_t *cand = w.list[0], *held = w.list[1];
   for (int64_t v = tid; v < n_nodes; v += T) {
@@ -169,7 +281,6 @@ __global__ void __launch_bounds__(T) lru_kernel(const int32_t *nodes, const int3
     used_at[v] = 0;
     arrived[v] = 0;
   }
-  for (int64_t i = tid; i < words; i += T) cached[i] = candbm[i] = 0;
   if (tid == 0) rng.seed(seed);
   __syncthreads();
   Totals tot;
@@ -178,33 +289,31 @@ __global__ void __launch_bounds__(T) lru_kernel(const int32_t *nodes, const int3
     const int64_t s = b * bs;
     const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
     const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
-    for (int i = tid; i < m2; i += T) w.stamp[q[i]] = (int32_t)b;
-    __syncthreads();
-    for (int i = tid; i < m2 * k; i += T) {
-      const int32_t v = tab[i];
-      if (v == 0 || w.stamp[v] == (int32_t)b) continue;
-      if (bit(cached, v)) {
-        ++tot.reuse;
-        tot.dist += b - arrived[v];
-        used_at[v] = (int32_t)b;
-      } else {
-        ++tot.recompute;
-        set_bit(candbm, v);
-      }
-    }
+    for_neighbors<SH>(w, target, q, m2, tab, m2 * k, (int32_t)b,
+                  [&](int32_t v) { return make_int2((int)bit(cached, v), arrived[v]); },
+                  [&](int32_t v, int2 x) {
+                    if (x.x) {
+                      ++tot.reuse;
+                      tot.dist += b - x.y;
+                      used_at[v] = (int32_t)b;
+                    } else {
+                      ++tot.recompute;
+                      set_bit(candbm, v);
+                    }
+                  });
     const int n_cand = list_members(candbm, words, cand, true, s_a);
     const int n_held = list_members(cached, words, held, false, s_a);
     const int room = budget - n_held;
     const int evict = room >= n_cand ? 0 : min(n_cand - room, n_held);
     const int take = (evict + room >= n_cand) ? n_cand : budget;
     if (evict != 0) {
-      if (!for_first_by_key(w, held, n_held, evict, used_at, s_a, s_b, [&](int32_t v) { clear_bit(cached, v); })) {
+      if (!for_first_by_key(w, held, n_held, evict, used_at, s_a, s_b,
+                            [&](int32_t v) { clear_bit(cached, v); })) {
         if (tid == 0) report(status, ORCA_E_TIMEOUT, (int)b);
         break;
       }
     }
-    if (tid == 0) rng.shuffle(cand, n_cand);
-    __syncthreads();
+    shuffle(w, rng, cand, n_cand, take == n_cand);
     for (int i = tid; i < take; i += T) {
       const int32_t v = cand[i];
       set_bit(cached, v);
@@ -226,7 +335,8 @@ __global__ void __launch_bounds__(T) lru_kernel(const int32_t *nodes, const int3
 
 // ------------------------------------------------------------------------------ 2Q (utils/cache.py:175-333)
 // a FIFO half and an LRU half of budget / 2 entries each
-__global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
+template <bool SH>
+__global__ void __launch_bounds__(T, 1) twoq_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
                                                  int32_t k, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
                                                  int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
                                                  int32_t *status) {
@@ -235,14 +345,16 @@ __global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int
   const int tid = threadIdx.x;
   const int64_t nb = (n_edges + bs - 1) / bs, words = (n_nodes + 31) / 32;
   const int half = budget / 2;
-  uint32_t *fifo = w.bm[0], *lru = w.bm[1], *promote_bm = w.bm[2], *fresh_bm = w.bm[3], *touched_bm = w.bm[4];
+  clear_bitmaps<SH>(w, words);
+  uint32_t *fifo = bitmap<SH>(w, 0, words), *lru = bitmap<SH>(w, 1, words), *promote_bm = bitmap<SH>(w, 2, words);
+  uint32_t *fresh_bm = bitmap<SH>(w, 3, words), *touched_bm = bitmap<SH>(w, 4, words);
+  uint32_t *target = SH ? bitmap<SH>(w, N_BM, words) : nullptr;
   int32_t *lru_used = w.t0, *lru_arr = w.t1, *fifo_arr = w.t2;
   int32_t *promote = w.list[0], *fresh = w.list[1], *touched = w.list[2], *ids = w.list[3];
   for (int64_t v = tid; v < n_nodes; v += T) {
     w.stamp[v] = -1;
     lru_used[v] = lru_arr[v] = fifo_arr[v] = 0;
   }
-  for (int64_t i = tid; i < words; i += T) fifo[i] = lru[i] = promote_bm[i] = fresh_bm[i] = touched_bm[i] = 0;
   if (tid == 0) rng.seed(seed);
   __syncthreads();
   Totals tot;
@@ -254,24 +366,22 @@ __global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int
     const int64_t s = b * bs;
     const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
     const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
-    for (int i = tid; i < m2; i += T) w.stamp[q[i]] = now;
-    __syncthreads();
-    for (int i = tid; i < m2 * k; i += T) {
-      const int32_t v = tab[i];
-      if (v == 0 || w.stamp[v] == now) continue;
-      if (bit(fifo, v)) {
-        ++tot.reuse;
-        tot.dist += now - fifo_arr[v];
-        set_bit(promote_bm, v);
-      } else if (bit(lru, v)) {
-        ++tot.reuse;
-        tot.dist += now - lru_arr[v];
-        set_bit(touched_bm, v);
-      } else {
-        ++tot.recompute;
-        set_bit(fresh_bm, v);
-      }
-    }
+    for_neighbors<SH>(w, target, q, m2, tab, m2 * k, now,
+                  [&](int32_t v) { return make_int4((int)bit(fifo, v), (int)bit(lru, v), fifo_arr[v], lru_arr[v]); },
+                  [&](int32_t v, int4 x) {
+                    if (x.x) {
+                      ++tot.reuse;
+                      tot.dist += now - x.z;
+                      set_bit(promote_bm, v);
+                    } else if (x.y) {
+                      ++tot.reuse;
+                      tot.dist += now - x.w;
+                      set_bit(touched_bm, v);
+                    } else {
+                      ++tot.recompute;
+                      set_bit(fresh_bm, v);
+                    }
+                  });
     const int n_promote = list_members(promote_bm, words, promote, true, s_a);
     const int n_fresh = list_members(fresh_bm, words, fresh, true, s_a);
     const int n_touched = list_members(touched_bm, words, touched, true, s_a);
@@ -290,8 +400,7 @@ __global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int
       for (int64_t i = tid; i < words; i += T) fifo[i] = 0;
       for (int64_t v = tid; v < n_nodes; v += T) fifo_arr[v] = 0;
       __syncthreads();
-      if (tid == 0) rng.shuffle(ids, n_fresh);
-      __syncthreads();
+      shuffle(w, rng, ids, n_fresh, n_fresh == half);
       for (int i = tid; i < half; i += T) {
         set_bit(fifo, ids[i]);
         fifo_arr[ids[i]] = now;
@@ -299,8 +408,7 @@ __global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int
       n_fifo = half;
     } else {
       const int n_ids = list_members(fifo, words, ids, false, s_a);
-      if (tid == 0) rng.shuffle(ids, n_ids);
-      __syncthreads();
+      shuffle(w, rng, ids, n_ids, false);
       for (int i = tid; i < n_fresh - fifo_room; i += T) clear_bit(fifo, ids[i]);
       __syncthreads();
       for (int i = tid; i < n_fresh; i += T) {
@@ -339,8 +447,7 @@ __global__ void __launch_bounds__(T) twoq_kernel(const int32_t *nodes, const int
       __syncthreads();
       for (int i = tid; i < n_promote; i += T) ids[i] = promote[i];
       __syncthreads();
-      if (tid == 0) rng.shuffle(ids, n_promote);
-      __syncthreads();
+      shuffle(w, rng, ids, n_promote, false);
       for (int i = tid; i < half - n_touched; i += T) admit(ids[i]);
       n_lru = half;
     }
@@ -446,18 +553,26 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
     w.sort.swaps = (int32_t *)take(2 * L.cap * 4);
     w.sort.cap = L.cap;
   }
+  // Shared memory: lists first (no list is longer than the graph has nodes), then six bitmaps where they fit (up to
+  // some 200,000 nodes): each of their scattered reads costs a trip to L2 otherwise.
+  constexpr int64_t per = tie::Shared::BYTES, most = per * tie::SHARED_MAX;
+  const int64_t bitmaps = (rnd::N_BM + 1) * ((n_nodes + 31) / 32) * 4;
+  w.cap_shared = (int)((std::min({L.cap, n_nodes, (int64_t)tie::SHARED_MAX}) + 15) & ~15ll);
+  if (per * w.cap_shared + bitmaps > most && per * (budget + 16ll) + bitmaps <= most)
+    w.cap_shared = (int)(((most - bitmaps) / per) & ~15ll);
+  w.bm_shared = per * w.cap_shared + bitmaps <= most;
+  const int smem = (int)(per * w.cap_shared + (w.bm_shared ? bitmaps : 0));
   cudaStream_t s = (cudaStream_t)stream;
   ORCA_CUDA(cudaMemsetAsync(d_stats, 0, 3 * sizeof(int64_t), s));
   if (n_edges == 0) {
     ORCA_CUDA(cudaMemsetAsync(d_plan_off, 0, sizeof(int64_t), s));
     return ORCA_OK;
   }
-  if (strategy == 1)
-    rnd::lru_kernel<<<1, rnd::T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, seed, w, d_plan_flat,
-                                        plan_cap, d_plan_off, d_stats, d_status);
-  else
-    rnd::twoq_kernel<<<1, rnd::T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, seed, w, d_plan_flat,
-                                         plan_cap, d_plan_off, d_stats, d_status);
+  auto kernel = strategy == 1 ? (w.bm_shared ? rnd::lru_kernel<true> : rnd::lru_kernel<false>)
+                              : (w.bm_shared ? rnd::twoq_kernel<true> : rnd::twoq_kernel<false>);
+  ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kernel<<<1, rnd::T, smem, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, seed, w, d_plan_flat, plan_cap,
+                                 d_plan_off, d_stats, d_status);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;
