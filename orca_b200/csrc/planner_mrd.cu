@@ -17,9 +17,14 @@
 //                     new cache.
 //
 // The first `budget` places of numba's argsort, with its order among equal keys, come from the steps described
-// in tie_order.cuh: block-wide in the one-CTA kernel, spread over the cluster in the cluster kernel.
+// in tie_order.cuh: block-wide in the one-CTA kernel.  In the cluster kernel the CTAs take
+// whole ranges each, in shared memory (tie_shared.cuh); for lists that do not fit, every step is spread over the
+// cluster.  200 batches of 2000 edges with 10,500 candidates: 43.5 ms a plan with all steps spread (a level then costs
+// five cluster barriers with trips to L2 between them, 10 us), 24 here.
+#include <algorithm>
+
 #include "common.cuh"
-#include "tie_order.cuh"
+#include "tie_shared.cuh"
 
 namespace orca {
 namespace mrd {
@@ -255,6 +260,7 @@ struct ClusterWork {
   int32_t *place;   // [cap] per range, at index lo: where its pivot ends up
   int32_t *live;    // [1] id of the last partition depth that left a live range
   uint32_t *fresh2; // [2][words] fresh bitmaps of even / odd batches
+  int cap_shared;   // longest list that is sorted in shared memory
 };
 
 __global__ void __launch_bounds__(T, 1) next_use_cluster_kernel(const int32_t *nodes, const int32_t *nbr,
@@ -309,10 +315,87 @@ __device__ __forceinline__ void park_pivot_cg(const Work &w, int lo, int hi) {
   w.pivot[lo] = key_of(c);
 }
 
+// ---- the argsort of a list that fits shared memory
+// Ranges are independent of each other: a CTA takes those that start in its slice of the list, in its shared memory.
+// At first that is one CTA with the whole list, then two with half of it each, and so on: entries and ranges go through
+// global memory after each turn, until no range is longer than SPLIT and every CTA finishes what it has.
+constexpr int SPLIT = 1024, LEVELS = 2;   // (levels a turn; 1: 28 ms a plan, 3 as 2; SPLIT 512 and 2048 as 1024)
+
+// One CTA's part of a turn: positions [base, base + m), whole ranges.  FINISH: all levels, then f(place, entry) for the
+// places below `keep`; otherwise LEVELS at most, until no range is longer than SPLIT; returns whether one still is.
+template <bool FINISH, class F>
+__device__ __forceinline__ bool sort_part(tie::Shared w, uint32_t *tot, uint64_t *e, uint32_t *ranges, int base, int m,
+                                          int keep, bool whole, F f) {
+#pragma unroll 4
+  for (int pos = threadIdx.x; pos < m; pos += T) {
+    const uint64_t x = ldcg64(&e[base + pos]);
+    const uint32_t g = whole ? tie::range(0, m - 1) : __ldcg(&ranges[base + pos]);
+    const int lo = tie::lo_of(g) - base, hi = tie::hi_of(g) - base;
+    w.key(pos) = key_of(x);
+    w.idx(pos) = (uint16_t)x;
+    w.ranges(pos) = tie::range(lo, hi);
+    if (!whole && pos == hi && live(lo, hi, keep - base)) w.pivot(lo) = key_of(x);   // (parked there)
+  }
+  __syncthreads();
+  if (whole) {
+    if (threadIdx.x == 0 && live(0, m - 1, keep)) tie::park_pivot(w, 0, m - 1);
+    __syncthreads();
+  }
+  const bool more = tie::partition(w, tot, m, keep - base, FINISH ? 15 : SPLIT, FINISH ? m : LEVELS);
+#pragma unroll 4
+  for (int pos = threadIdx.x; pos < m; pos += T) {
+    const uint32_t r = w.ranges(pos);
+    const int lo = tie::lo_of(r), hi = tie::hi_of(r);
+    if (FINISH) {
+      if (lo < keep - base) {
+        const int place = base + tie::place_of(w, pos, lo, hi);
+        if (place < keep) f(place, (int)w.idx(pos));
+      }
+    } else {
+      e[base + pos] = (uint64_t)(uint32_t)w.key(pos) << 32 | w.idx(pos);
+      ranges[base + pos] = tie::range(base + lo, base + hi);
+    }
+  }
+  return more;
+}
+
+// All CTAs, behind a cluster barrier: calls f(place, entry) for the first `keep` places of the argsort of e[0 .. n).
+template <class F>
+__device__ __forceinline__ void sort_first_cluster(tie::Shared w, uint32_t *tot, uint64_t *e, uint32_t *ranges,
+                                                   int32_t *live_word, int &epoch, int n, int keep, F f) {
+  const int all = min(n, keep), per = (all + (int)cluster_size() - 1) / (int)cluster_size();
+  const int from = (int)cluster_rank() * per;
+  bool more = n > SPLIT, whole = true;
+  while (true) {   // (ends: every turn takes the pivot out of each range longer than SPLIT)
+    int base = 0, m = cluster_rank() == 0 ? n : 0;
+    if (!whole) {
+      m = 0;
+      if (from < all) {
+        const uint32_t a = __ldcg(&ranges[from]), z = __ldcg(&ranges[min(from + per, all) - 1]);
+        base = tie::lo_of(a) == from ? from : tie::hi_of(a) + 1;
+        m = tie::hi_of(z) + 1 - base;   // (none or less: one range from before the slice to behind it)
+      }
+    }
+    if (!more) {
+      if (m > 0) sort_part<true>(w, tot, e, ranges, base, m, keep, whole, f);
+      return;
+    }
+    ++epoch;
+    if (m > 0) {
+      const bool mine = sort_part<false>(w, tot, e, ranges, base, m, keep, whole, [](int, int) {});
+      if (mine && threadIdx.x == 0) *live_word = epoch;
+    }
+    cluster_sync();
+    more = __ldcg(live_word) >= epoch;   // (a CTA ahead of this one may have counted on)
+    whole = false;
+  }
+}
+
 __global__ void __launch_bounds__(T, 1) mrd_cluster_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges,
                                                            int32_t bs, int32_t k, int64_t n_nodes, int32_t budget,
                                                            ClusterWork cw, int32_t *plan, int64_t plan_cap,
                                                            int64_t *plan_off, int64_t *stats, int32_t *status) {
+  __shared__ uint32_t s_tot[NW];
   const Work &w = cw.w;
   const int GT = T * (int)cluster_size();
   const int gt = (int)cluster_rank() * T + threadIdx.x;
@@ -463,6 +546,18 @@ __global__ void __launch_bounds__(T, 1) mrd_cluster_kernel(const int32_t *nodes,
       }
     }
     cluster_sync();
+    const auto admit = [&](int place, int entry) {
+      const int32_t v = __ldcg(&w.cand[entry]);
+      plan[used + place] = v;
+      atomicOr(&w.cached[v >> 5], 1u << (v & 31));
+      if ((__ldcg(&fresh[v >> 5]) >> (v & 31)) & 1u) w.since[v] = (int32_t)b;
+    };
+    if (gt == 0) plan_off[b] = used;
+    if (n <= cw.cap_shared) {   // uniform over the cluster
+      sort_first_cluster(tie::Shared{cw.cap_shared}, s_tot, w.e, (uint32_t *)w.seg, cw.live, epoch, n, keep, admit);
+      used += keep;
+      continue;
+    }
     if (any && gt == 0) park_pivot_cg(w, 0, n - 1);
     cluster_sync();
     int depth = 0;
@@ -569,7 +664,6 @@ __global__ void __launch_bounds__(T, 1) mrd_cluster_kernel(const int32_t *nodes,
       break;
     }
     // ranges shorter than 16: stable order by key; the first `keep` places are the new cache
-    if (gt == 0) plan_off[b] = used;
 #pragma unroll
     for (int i = 0; i < MAX_ITEMS; ++i) {
       if (i < items && hi[i] >= 0 && lo[i] < keep) {
@@ -581,12 +675,7 @@ __global__ void __launch_bounds__(T, 1) mrd_cluster_kernel(const int32_t *nodes,
           const int32_t ko = key_of(ldcg64(&w.e[qpos]));
           place += (ko < kv || (ko == kv && qpos < pos)) ? 1 : 0;
         }
-        if (place < keep) {
-          const int32_t v = __ldcg(&w.cand[(uint32_t)me]);
-          plan[used + place] = v;
-          atomicOr(&w.cached[v >> 5], 1u << (v & 31));
-          if ((__ldcg(&fresh[v >> 5]) >> (v & 31)) & 1u) w.since[v] = (int32_t)b;
-        }
+        if (place < keep) admit(place, (int)(uint32_t)me);
       }
     }
     used += keep;
@@ -674,16 +763,20 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
     return ORCA_OK;
   }
   // A cluster of 16 (else 8) CTAs shares every phase when the device can place such a cluster and the
-  // candidate list fits its threads' registers (measured at c5: 0.81 s with 16 CTAs, 0.91 s with 8, 2.3 s
-  // with one CTA; a phase costs a cluster barrier of ~600 cycles, an L2 round trip of ~300 per dependent
-  // load and the release of its stores); one CTA does the same work otherwise.
+  // candidate list fits its threads' registers (a phase costs a cluster barrier of ~600 cycles, an L2 round
+  // trip of ~300 per dependent load and the release of its stores; one CTA needs 2.8 times as long where all
+  // steps are spread); one CTA does the same work otherwise.
   const int64_t cap = mrd::cand_cap(bs, k, budget);
+  const int cap_shared = (int)((std::min<int64_t>(cap, tie::SHARED_MAX) + 15) & ~15ll);
+  const int smem = tie::Shared::BYTES * cap_shared;
+  ORCA_CUDA(cudaFuncSetAttribute(mrd::mrd_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int cluster = 0;
   for (int c : {16, 8}) {
     if (cluster != 0 || cap > (int64_t)mrd::MAX_ITEMS * mrd::T * c) continue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c);
     cfg.blockDim = dim3(mrd::T);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -712,6 +805,7 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
     cw.fresh2 = w.fresh;
     cw.tot = (int2 *)(base + L.off[15]);
     cw.place = (int32_t *)(base + L.off[16]);
+    cw.cap_shared = cap_shared;
     cw.live = (int32_t *)(base + L.off[17]);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster);
@@ -726,6 +820,7 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
     cfg.numAttrs = 1;
     ORCA_CUDA(cudaLaunchKernelEx(&cfg, mrd::next_use_cluster_kernel, d_nodes, d_nbr, n_edges, bs, k, n_nodes, w));
     ORCA_COUNT_LAUNCH();
+    cfg.dynamicSmemBytes = smem;
     ORCA_CUDA(cudaLaunchKernelEx(&cfg, mrd::mrd_cluster_kernel, d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, cw,
                                  d_plan_flat, plan_cap, d_plan_off, d_stats, d_status));
     ORCA_COUNT_LAUNCH();

@@ -12,7 +12,7 @@
 // tie_order.cuh for lists that do not fit shared memory).
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
 // 250 batches of 600 edges with 20 neighbours, LRU: 19.2 ms a plan with draws, swaps, bitmaps and sort
-// in global memory, 11.4 here.
+// in global memory, 12.1 here.
 #include <algorithm>
 
 #include "common.cuh"
@@ -156,8 +156,8 @@ __device__ void shuffle(const Work &w, Twister &rng, int32_t *x, int n, bool any
     __syncthreads();
     return;
   }
-  const bool fits = n <= w.cap_shared;
-  int32_t *at = fits ? (int32_t *)tie::smem : x, *draw = fits ? at + w.cap_shared : w.sort.lpos;
+  const bool fits = 8ll * n <= (int64_t)tie::Shared::BYTES * w.cap_shared;
+  int32_t *at = fits ? (int32_t *)tie::smem : x, *draw = fits ? at + n : w.sort.lpos;
   if (threadIdx.x < 32) rng.draws(n, draw);
   if (fits)
     for (int i = threadIdx.x; i < n; i += T) at[i] = x[i];
@@ -186,8 +186,7 @@ __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int c
       sh.idx(i) = (uint16_t)i;
     }
     const auto use = [&](int, int i) { f(ids[i]); };
-    if (n <= 4 * T) tie::sort_first_shared<4>(sh, (uint32_t *)s_a, n, count, use);
-    else tie::sort_first_shared<20>(sh, (uint32_t *)s_a, n, count, use);
+    tie::sort_first_shared(sh, (uint32_t *)s_a, n, count, use);
     return true;
   }
   for (int i = threadIdx.x; i < n; i += T) w.sort.e[i] = ((uint64_t)(uint32_t)key[ids[i]] << 32) | (uint32_t)i;
@@ -553,11 +552,13 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
     w.sort.swaps = (int32_t *)take(2 * L.cap * 4);
     w.sort.cap = L.cap;
   }
-  // Shared memory: lists first (no list is longer than the graph has nodes), then six bitmaps where they fit (up to
-  // some 200,000 nodes): each of their scattered reads costs a trip to L2 otherwise.
+  // Shared memory: lists first, then six bitmaps where they fit (up to some 200,000 nodes: each of their scattered reads
+  // costs a trip to L2 otherwise).  The lists that are sorted are no longer than the budget; more room than for those,
+  // or for the shuffles of 7000 entries, only takes L1 from the table entries' loads (the same time with room for
+  // every node here).
   constexpr int64_t per = tie::Shared::BYTES, most = per * tie::SHARED_MAX;
   const int64_t bitmaps = (rnd::N_BM + 1) * ((n_nodes + 31) / 32) * 4;
-  w.cap_shared = (int)((std::min({L.cap, n_nodes, (int64_t)tie::SHARED_MAX}) + 15) & ~15ll);
+  w.cap_shared = (int)((std::min({L.cap, n_nodes, std::max<int64_t>(budget, 4096), (int64_t)tie::SHARED_MAX}) + 15) & ~15ll);
   if (per * w.cap_shared + bitmaps > most && per * (budget + 16ll) + bitmaps <= most)
     w.cap_shared = (int)(((most - bitmaps) / per) & ~15ll);
   w.bm_shared = per * w.cap_shared + bitmaps <= most;

@@ -82,12 +82,13 @@ def test_mrd_long_ranges_of_equal_keys():
     assert (int(stats[0]), int(stats[1])) == wstats[:2]
 
 
-@pytest.mark.parametrize("strategy", ["LRU", "2Q"])
+@pytest.mark.parametrize("strategy", ["MRD", "LRU", "2Q"])
 @pytest.mark.parametrize("n_src,n_edges,bs,budget", [(3000, 30000, 600, 1200),     # lists of one entry a thread
+                                                     (60000, 60000, 2000, 24000),  # MRD: some fit shared memory
                                                      (60000, 40000, 2000, 9000),   # of up to twenty
                                                      (60000, 60000, 4000, 44000),  # longer than shared memory takes
                                                      (400000, 20000, 1000, 2000)])  # bitmaps in global memory
-def test_random_policies_at_the_limits_of_shared_memory(strategy, n_src, n_edges, bs, budget):
+def test_plans_at_the_limits_of_shared_memory(strategy, n_src, n_edges, bs, budget):
     from oracle import planner
     from orca_b200 import synthetic
     spec = dataclasses.replace(synthetic.SPECS["t_nb2"], n_src=n_src, n_edges=n_edges, bs=bs, budget=budget)
