@@ -113,28 +113,44 @@ __global__ void __launch_bounds__(256) mark_kernel(const __grid_constant__ Args 
   dep_wait();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   if (a.budget()) {
+    // Node 0 pads the tables: it is in thousands of slots and a candidate of nearly every batch.  One thread a block
+    // and batch asks for it (all of them queued at its word: 62 us for eight batches of 2000 edges, 11 so).
+    __shared__ uint32_t padded;
+    if (threadIdx.x == 0) padded = 0;
+    __syncthreads();
     const int n_slots = 3 * a.edges() * a.k, per = 3 * a.bs * a.k;
     for (int i = tid; i < n_slots; i += step) {
       const int n = i / per, v = a.nbr1[i];
       const uint32_t bit = 1u << n;
+      if (v == 0 && ((*(volatile uint32_t *)&padded & bit) || (atomicOr(&padded, bit) & bit))) continue;
       // (through L1: hub nodes are sampled thousands of times, and a stale word only costs the atomic below)
       const uint4 b = *reinterpret_cast<const uint4 *>(&a.bits[v]);
       if ((b.y & bit) || (b.w & bit) || (n > 0 ? (b.x & bit) != 0 : a.cache_flag[v] != 0)) continue;
+      if (__ldcg(&a.bits[v].fetched) & bit) continue;
       if (atomicOr(&a.bits[v].fetched, bit) & bit) continue;
       const int p = place(&a.cnt->n_cand[n], n);
       if (p < a.u_cap1) a.cand[(size_t)n * a.u_cap1 + p] = v;
       atomicMax(&a.cnt->low_cand[n], INT_MAX - v);
     }
   }
+  // (a warp stays together here, for one atomic a warp and batch)
   const int n_pos = 2 * a.edges(), per = 2 * a.bs;
-  for (int i = tid; i < n_pos; i += step) {
-    const int n = i / per, r = i - n * per, b = a.b_of(n);
+  for (int i0 = tid & ~31; i0 < n_pos; i0 += step) {
+    const int i = i0 + (threadIdx.x & 31), n = min(i, n_pos - 1) / per, r = i - n * per, b = a.b_of(n);
     const int32_t *batch = a.img + a.off[n];
-    const int v = batch[r];
-    if (v < 0 || v >= a.n_nodes) continue;
-    Entry *e = a.table + find_entry(a.table, a.table_mask, v, n);
-    if (e->pos != r + 1) continue;
-    const int w = place(&a.cnt->n_win[n], n);
+    const int v = i < n_pos ? batch[r] : -1;
+    Entry *e = nullptr;
+    if (v >= 0 && v < a.n_nodes) {
+      e = a.table + find_entry(a.table, a.table_mask, v, n);
+      if (e->pos != r + 1) e = nullptr;
+    }
+    __syncwarp();
+    const unsigned group = __match_any_sync(0xffffffffu, e != nullptr ? n : -1);
+    const int leader = __ffs(group) - 1, lane = threadIdx.x & 31;
+    int w = 0;
+    if (e != nullptr && lane == leader) w = atomicAdd(&a.cnt->n_win[n], __popc(group));
+    w = __shfl_sync(0xffffffffu, w, leader) + __popc(group & ((1u << lane) - 1u));
+    if (e == nullptr) continue;
     e->pos = IN_LOG | w;     // (no other position of the node equals it)
     const int at = n * per + w, other = r < b ? batch[b + r] : batch[r - b];
     a.win_node[at] = v;
