@@ -634,6 +634,24 @@ class TGN(nn.Module):
             raise _lib.OrcaError(code, f"a kernel of an earlier batch reported error {code} "
                                        f"(detail {int(v[3])}); results since then are invalid")
 
+    def _finish_epoch(self, stream):
+        """Waits for a stream of batches whose scores are on their way to the host and brings the status word along.
+        Returns the error to raise, or None: a whole-stream call has no later call to report through."""
+        if self._status_host is None:
+            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
+            self._status_event = torch.cuda.Event()
+        with torch.cuda.stream(stream):
+            self._status_host.copy_(self._status, non_blocking=True)
+        stream.synchronize()
+        v = self._status_host.numpy()
+        code, detail = int(v[0]), int(v[3])
+        if code == 0:
+            return None
+        self._status.zero_()
+        v[0] = 0
+        return _lib.OrcaError(code, f"a kernel reported error {code} (detail {detail}); the scores and the state tables "
+                                    "are invalid")
+
     def _eval_batch_sharded(self, desc, d_i32, d_ts, b, d_plan, n_plan, u_cap, ws, want_emb):
         if self.n_layers != 2:
             raise NotImplementedError("the multi-GPU split is built for the two-layer model")
@@ -720,7 +738,8 @@ class TGN(nn.Module):
         batch: the batches are packed into pinned host memory, and the library copies each batch to the
         device, runs it and copies its scores back, batch after batch, asynchronously.
         cache_plan: list with one id array per batch (or None: the plan-less flag rule).
-        Returns (pos, neg): float32 numpy arrays with one score per edge."""
+        Returns (pos, neg): float32 numpy arrays with one score per edge.  Raises what the kernels of these or of
+        earlier batches reported (ids outside a table, a bounded wait that gave up)."""
         L = _lib.lib()
         E = len(sources)
         bs, k = int(batch_size), int(n_neighbors)
@@ -823,7 +842,9 @@ class TGN(nn.Module):
             _lib.check(L.orca_tgn_eval_epoch(desc, C.byref(ep), u_cap, ws.data_ptr(), ws.numel(),
                                              dev["stage"].data_ptr(), dev["stage"].numel(), dev["prob"].data_ptr(),
                                              h_prob.data_ptr(), self._status.data_ptr(), stream.cuda_stream))
-        stream.synchronize()
+        failed = self._finish_epoch(stream)
+        if failed is not None and world == 1:
+            raise failed
         local = h_prob.numpy()[:n_scores]
         pos = np.empty(E, dtype=np.float32)
         neg = np.empty(E, dtype=np.float32)
@@ -851,6 +872,8 @@ class TGN(nn.Module):
                 pos[lo + r:lo + int(b[i]):wb] = every[wa + r, o:o + n]
                 neg[lo + r:lo + int(b[i]):wb] = every[wa + r, o + n:o + 2 * n]
                 o += 2 * n
+        if failed is not None:      # (behind the exchange, which every rank takes part in)
+            raise failed
         return pos, neg
 
     def _eval_groups(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan):
@@ -932,7 +955,9 @@ class TGN(nn.Module):
             g, lo = groups[j]
             g.phase = 2
             enqueue(g, lo)
-        stream.synchronize()
+        failed = self._finish_epoch(stream)
+        if failed is not None:
+            raise failed
         # per batch [pos | neg]; the last batch may be short
         scores, full = h_prob.numpy()[:2 * E], E // bs
         out = np.empty((2, E), dtype=np.float32)

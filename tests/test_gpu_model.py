@@ -495,3 +495,45 @@ def test_device_side_errors_surface_through_the_reference_api():
     with pytest.raises(_lib.OrcaError) as err:
         m.compute_edge_probabilities(src, dst, np.roll(dst, 3), ts, eidx, spec.n_degree, True, False, plan[2])
     assert err.value.code == 4
+
+
+@pytest.mark.parametrize("planned", [True, False])      # groups of batches / batch by batch
+def test_device_side_errors_of_a_stream_are_raised_by_its_own_call(planned):
+    """A user who scores a stream in one call has no later call to hear of an error through: eval_epoch raises what
+    its kernels left in the status word (here put there by the host), once, and the next stream runs."""
+    from orca_b200 import _lib
+    g = graph("t_nb2")
+    spec = g.spec
+    gold = golden("t_nb2")
+    plan = unpack(gold[f"plan_{spec.strategy}_flat"], gold[f"plan_{spec.strategy}_off"]) if planned else None
+    m = make_model(g)
+    E = 3 * spec.bs
+    run = lambda: m.eval_epoch(g.sources[:E], g.destinations[:E], np.roll(g.destinations[:E], 3), g.timestamps[:E],
+                               g.edge_idxs[:E], spec.n_degree, spec.bs, plan)
+    run()
+    m._status[0] = 6                     # ORCA_E_TIMEOUT, as report() would leave it
+    with pytest.raises(_lib.OrcaError) as err:
+        run()
+    assert err.value.code == 6
+    pos, neg = run()
+    assert np.isfinite(pos).all() and np.isfinite(neg).all()
+
+
+@pytest.mark.parametrize("layers", [1, 2])
+def test_a_stream_with_an_id_outside_the_table_is_refused(layers):
+    """(The kernels of a group read such an id as node 0: sampling reports it, its rows and the tables it would index
+    are guarded.)"""
+    import dataclasses
+    from orca_b200 import _lib
+    g = graph("t_nb2")
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, n_layers=layers))
+    spec = g.spec
+    gold = golden("t_nb2")
+    plan = unpack(gold[f"plan_{spec.strategy}_flat"], gold[f"plan_{spec.strategy}_off"])
+    E = 2 * spec.bs + 5
+    for where in range(3):
+        ids = [np.array(a) for a in (g.sources[:E], g.destinations[:E], np.roll(g.destinations[:E], 3))]
+        ids[where][spec.bs + 7] = g.n_nodes
+        with pytest.raises(_lib.OrcaError) as err:
+            make_model(g).eval_epoch(*ids, g.timestamps[:E], g.edge_idxs[:E], spec.n_degree, spec.bs, plan)
+        assert err.value.code == 5       # ORCA_E_BOUNDS
