@@ -740,7 +740,6 @@ class TGN(nn.Module):
         cache_plan: list with one id array per batch (or None: the plan-less flag rule).
         Returns (pos, neg): float32 numpy arrays with one score per edge.  Raises what the kernels of these or of
         earlier batches reported (ids outside a table, a bounded wait that gave up)."""
-        L = _lib.lib()
         E = len(sources)
         bs, k = int(batch_size), int(n_neighbors)
         nb = (E + bs - 1) // bs
@@ -750,15 +749,29 @@ class TGN(nn.Module):
         self.batch_counter += nb - 1
         if self._mode != MODE_BUDGET:
             cache_plan = None
-        world, rank = self._world, self._rank
+        world = self._world
         # Groups of batches on one GPU; one batch after the other where a batch's work depends on the one before in
         # full (flags without a plan accumulate), in the debug modes and when the batch is split over GPUs
-        if world == 1 and (cache_plan is not None or self._mode != MODE_BUDGET or self.n_layers == 1) and \
-                not any(self._options.get(o) for o in (_lib.OPT_PROJECTION_MODE, _lib.OPT_TRACE)):
-            return self._eval_groups(sources, destinations, negatives, timestamps, edge_idxs, k, bs,
-                                     cache_plan if self.n_layers == 2 else None)
         if world > 1 and getattr(self, "_exchange", None) is None:
             raise NotImplementedError("eval_epoch on several GPUs needs the direct exchange (set_distributed)")
+        try:
+            if world == 1 and (cache_plan is not None or self._mode != MODE_BUDGET or self.n_layers == 1) and \
+                    not any(self._options.get(o) for o in (_lib.OPT_PROJECTION_MODE, _lib.OPT_TRACE)):
+                return self._eval_groups(sources, destinations, negatives, timestamps, edge_idxs, k, bs,
+                                         cache_plan if self.n_layers == 2 else None)
+            return self._eval_chunks(sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan)
+        except BaseException:
+            # (an array that cannot be packed, an allocation that fails: batches before it may be in flight, on the
+            # library's streams too, and the next call writes into the same buffers)
+            torch.cuda.synchronize(self.device)
+            raise
+
+    def _eval_chunks(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan):
+        """eval_epoch batch after batch (orca_tgn_eval_epoch)."""
+        L = _lib.lib()
+        E = len(sources)
+        nb = (E + bs - 1) // bs
+        world, rank = self._world, self._rank
         b = np.full(nb, bs, dtype=np.int32)
         b[-1] = E - (nb - 1) * bs
         n_plan = np.full(nb, -1, dtype=np.int32)
@@ -901,7 +914,8 @@ class TGN(nn.Module):
                 nb_max, most = max(nb_max, keep["nb_max"]), max(most, keep["plan_cap"])
             nbytes = L.orca_group_workspace_bytes(bs, nb_max, k, u_cap, most, self.n_nodes, self.n_layers, mode)
             if keep.get("ws") is None or keep["ws"].numel() < nbytes:
-                keep["ws"] = None         # (an epoch ends with a synchronisation: nothing is using the old one)
+                # (an epoch ends with a synchronisation: nothing is using the old one.  The allocation may fail.)
+                keep["shape"] = keep["ws"] = None
                 keep["ws"] = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             keep.update(shape=shape, nb_max=nb_max, plan_cap=most)
         nb_max, plan_cap, ws = keep["nb_max"], keep["plan_cap"], keep["ws"]

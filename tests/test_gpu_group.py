@@ -64,3 +64,36 @@ def test_group_equals_batches(name, bs, k, E, recursion, layers):
         if layers == 2:
             ha, hb = a.embedding_module.histories[0], b.embedding_module.histories[0]
             assert torch.equal(ha.emb, hb.emb) and torch.equal(ha.cache_flag_dev, hb.cache_flag_dev)
+
+
+def test_a_stream_that_fails_leaves_a_model_that_works(monkeypatch):
+    """A stream can fail in the middle -- here an id that cannot be packed, in the third group, and a workspace that
+    cannot be allocated.  What was enqueued has finished when the error is raised, and the next stream runs as on a
+    fresh model."""
+    from test_gpu_model import make_model
+    g = graph("t_nb2")
+    bs, k, E = 20, 10, 2000
+    neg = synthetic.negative_destinations(g, seed=1)
+    plan = _plan(g, bs, k, g.spec.budget, g.spec.strategy, E)
+    m, fresh = make_model(g), make_model(g)
+    run = lambda model, plan, n, k=k: model.eval_epoch(g.sources[:n], g.destinations[:n], neg[:n], g.timestamps[:n],
+                                                       g.edge_idxs[:n], k, bs, plan)
+    state = [t.clone() for t in m.memory.backup_memory()]
+    waits = []
+    synchronize = torch.cuda.synchronize
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: (waits.append(a), synchronize(*a))[1])
+    bad = list(plan)
+    bad[70] = ["not an id"] * len(plan[70])
+    with pytest.raises(ValueError):
+        run(m, bad, E)
+    assert waits
+    del waits[:]
+    with pytest.raises(Exception):
+        run(m, plan, E, k=33)              # (no workspace for more than 32 neighbours)
+    assert waits
+    m.memory.restore_memory(state)
+    m.embedding_module.reset_history()
+    m.embedding_module.histories[0].cache_flag = np.zeros(g.n_nodes)
+    for a, b in zip(run(m, plan, E), run(fresh, plan, E)):
+        assert np.array_equal(a, b)
+    assert torch.equal(m.memory.memory, fresh.memory.memory)
