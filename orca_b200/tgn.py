@@ -544,12 +544,11 @@ class TGN(nn.Module):
         h = torch.empty(_lib.CALL_SLOTS * slot, dtype=torch.uint8, pin_memory=True)
         dev = torch.empty(_lib.CALL_SLOTS * slot, dtype=torch.uint8, device=self.device)
         torch.cuda.current_stream(self.device).synchronize()   # (the copies run on a stream of their own)
-        if self._status_host is None:
-            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
+        status = self._status_buffer()
         c = _lib.CallT()
         c.h_ring, c.d_ring, c.slot_bytes = h.data_ptr(), dev.data_ptr(), slot
-        ring = self.__dict__["_call_ring"] = (h, dev, slot, c, self._status_host.data_ptr())
-        self.__dict__["_status_view"] = self._status_host.numpy()
+        ring = self.__dict__["_call_ring"] = (h, dev, slot, c, status.data_ptr())
+        self.__dict__["_status_view"] = status.numpy()
         return ring
 
     def _eval_batch_staged(self, source_nodes, destination_nodes, negative_nodes, edge_times, edge_idxs, k, cache_plan,
@@ -611,10 +610,7 @@ class TGN(nn.Module):
         ev.record(stream)
         # The status word follows the batch to pinned host memory without a synchronisation; the next call
         # that finds the copy complete raises what the kernels reported (_raise_reported).
-        if self._status_host is None:
-            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
-            self._status_event = torch.cuda.Event()
-        self._status_host.copy_(self._status, non_blocking=True)
+        self._status_buffer().copy_(self._status, non_blocking=True)
         self._status_event.record(stream)
         self._status_pending = True
 
@@ -634,14 +630,18 @@ class TGN(nn.Module):
             raise _lib.OrcaError(code, f"a kernel of an earlier batch reported error {code} "
                                        f"(detail {int(v[3])}); results since then are invalid")
 
+    def _status_buffer(self):
+        """The pinned copy of the status word; made, with the event behind its copies, by whichever path runs first."""
+        if self._status_host is None:
+            self._status_event = torch.cuda.Event()
+            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
+        return self._status_host
+
     def _finish_epoch(self, stream):
         """Waits for a stream of batches whose scores are on their way to the host and brings the status word along.
         Returns the error to raise, or None: a whole-stream call has no later call to report through."""
-        if self._status_host is None:
-            self._status_host = torch.zeros(4, dtype=torch.int32).pin_memory()
-            self._status_event = torch.cuda.Event()
         with torch.cuda.stream(stream):
-            self._status_host.copy_(self._status, non_blocking=True)
+            self._status_buffer().copy_(self._status, non_blocking=True)
         stream.synchronize()
         v = self._status_host.numpy()
         code, detail = int(v[0]), int(v[3])

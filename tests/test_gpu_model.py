@@ -537,3 +537,27 @@ def test_a_stream_with_an_id_outside_the_table_is_refused(layers):
         with pytest.raises(_lib.OrcaError) as err:
             make_model(g).eval_epoch(*ids, g.timestamps[:E], g.edge_idxs[:E], spec.n_degree, spec.bs, plan)
         assert err.value.code == 5       # ORCA_E_BOUNDS
+
+
+def test_the_status_copy_serves_every_path_whichever_ran_first():
+    """The calls of one GPU, whole streams and the batches of the multi-GPU split share the pinned status word: a model
+    that has scored on its own can be split afterwards (the end of a split batch is called by hand here)."""
+    from orca_b200 import _lib
+    g = graph("t_nb2")
+    spec = g.spec
+    for first in ("call", "stream"):
+        m = make_model(g)
+        _, src, dst, ts, eidx = next(iter(batches(g, 1)))
+        batch = (src, dst, np.roll(dst, 3), ts, eidx)
+        if first == "call":
+            m.compute_edge_probabilities(*batch, spec.n_degree, True, False, None)
+        else:
+            m.eval_epoch(*batch, spec.n_degree, spec.bs, None)
+        m.check_status()
+        m._status[0] = 4                 # ORCA_E_CAPACITY, as report() would leave it
+        m._ev_free = [None]
+        m._release_dev(0, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        with pytest.raises(_lib.OrcaError) as err:
+            m.compute_edge_probabilities(*batch, spec.n_degree, True, False, None)
+        assert err.value.code == 4
