@@ -640,8 +640,7 @@ class TGN(nn.Module):
     def _finish_epoch(self, stream):
         """Waits for a stream of batches whose scores are on their way to the host and brings the status word along.
         Returns the error to raise, or None: a whole-stream call has no later call to report through."""
-        with torch.cuda.stream(stream):
-            self._status_buffer().copy_(self._status, non_blocking=True)
+        self._status_buffer().copy_(self._status, non_blocking=True)      # (`stream` is the current stream)
         stream.synchronize()
         v = self._status_host.numpy()
         code, detail = int(v[0]), int(v[3])
