@@ -503,6 +503,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     const int plan = std::max(g->n_plan[n], 0);
     ORCA_CHECK_ARG(g->off_i32[n] == base_i32 + n_i32 && plan <= g->plan_cap && (!budget || g->n_plan[n] >= 0));
     a.off[n] = (int)n_i32, a.n_plan[n] = plan;
+    if (g->phase & 1) ORCA_TRY(check_batch_ids(m, g->h_i32 + base_i32 + n_i32, a.b_of(n), n, "orca_tgn_eval_group"));
     n_i32 += 4ll * a.b_of(n) + plan;
   }
   if (budget) ORCA_CHECK_ARG(a.n_plan[g->nb - 1] <= m->plan_cap);

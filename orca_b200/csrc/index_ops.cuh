@@ -5,6 +5,11 @@
 
 namespace orca {
 
+// Host: ORCA_E_BOUNDS if a node or edge id of the batch [src | dst | neg | edge ids] (4 * b int32) lies outside its table
+// (n_edge_rows <= 0: the descriptor does not say how many edges there are).  The kernels of a single batch read the
+// rows of these ids as they come.
+int check_batch_ids(const orca_tgn_t *m, const int32_t *h_batch, int b, int64_t batch, const char *who);
+
 // rows [src | dst | neg] of the batch with their query times, the [dst | src] partner list, the
 // neighbour table of those rows, candidate marking (bitmap + list) and the last-occurrence record of
 // every row's node in d_last_pos (record = base + row)

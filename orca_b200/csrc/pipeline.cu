@@ -847,6 +847,22 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
   return ORCA_OK;
 }
 
+// (two passes over a few thousand ids that are in the cache: 1 us for 2000 edges)
+int check_batch_ids(const orca_tgn_t *m, const int32_t *h_batch, int b, int64_t batch, const char *who) {
+  auto outside = [&](const int32_t *x, int n, int64_t lim, const char *what) -> int {
+    int32_t sign = 0, top = 0;
+    for (int i = 0; i < n; ++i) sign |= x[i], top = std::max(top, x[i]);
+    if (sign >= 0 && top < lim) return ORCA_OK;
+    int i = 0;
+    while (x[i] >= 0 && x[i] < lim) ++i;
+    return set_error(ORCA_E_BOUNDS, "%s: %s %d of batch %lld is outside [0,%lld)", who, what, (int)x[i], (long long)batch,
+                     (long long)lim);
+  };
+  const int rc = outside(h_batch, 3 * b, m->n_nodes, "node");
+  if (rc || m->n_edge_rows <= 0) return rc;
+  return outside(h_batch + 3 * (size_t)b, b, m->n_edge_rows, "edge");
+}
+
 }  // namespace orca
 
 extern "C" {
@@ -962,6 +978,7 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
     if (off_ts + 8ll * b > slot_bytes)
       return set_error(ORCA_E_CAPACITY, "orca_tgn_eval_epoch: staging slot of %lld bytes, batch %lld needs %lld",
                        (long long)slot_bytes, (long long)i, (long long)(off_ts + 8ll * b));
+    ORCA_TRY(check_batch_ids(m, e->h_i32 + e->off_i32[i], b, i, "orca_tgn_eval_epoch"));
     const int slot = (int)(c->stage_seq++ % kSlots);   // (the ring carries over from call to call)
     char *d_slot = (char *)d_stage + slot * slot_bytes;
     // the copy of batch i runs on the copy stream, ahead of the kernels of the batches before it; a slot is
@@ -1012,11 +1029,14 @@ int orca_tgn_call(const orca_tgn_t *m, const orca_call_t *a, int32_t u_cap, void
   if (c->call_used[slot]) ORCA_CUDA(cudaEventSynchronize(c->ev_call[slot]));   // (eight calls ahead of the GPU: wait)
   char *h = (char *)a->h_ring + slot * a->slot_bytes, *d = (char *)a->d_ring + slot * a->slot_bytes;
   int32_t *o = (int32_t *)h;
+  uint64_t wide = 0;      // set where an id is negative or does not fit 31 bits
   auto narrow = [&](const int64_t *x, int n) {
-    for (int i = 0; i < n; ++i) o[i] = (int32_t)x[i];
+    for (int i = 0; i < n; ++i) o[i] = (int32_t)x[i], wide |= (uint64_t)x[i] >> 31;
     o += n;
   };
   narrow(a->src, b), narrow(a->dst, b), narrow(a->neg, b), narrow(a->eidx, b);
+  if (wide != 0) return set_error(ORCA_E_BOUNDS, "orca_tgn_call: an id of the batch is negative or has more than 31 bits");
+  ORCA_TRY(check_batch_ids(m, (const int32_t *)h, b, 0, "orca_tgn_call"));
   if (n_plan > 0) narrow(a->plan, n_plan);
   memcpy(h + off_ts, a->ts, (size_t)b * 8);
   ORCA_CUDA(cudaMemcpyAsync(d, h, (size_t)bytes, cudaMemcpyHostToDevice, c->copy));

@@ -520,9 +520,10 @@ def test_device_side_errors_of_a_stream_are_raised_by_its_own_call(planned):
 
 
 @pytest.mark.parametrize("layers", [1, 2])
-def test_a_stream_with_an_id_outside_the_table_is_refused(layers):
-    """(The kernels of a group read such an id as node 0: sampling reports it, its rows and the tables it would index
-    are guarded.)"""
+def test_an_id_outside_its_table_is_refused(layers):
+    """A node or edge id that the tables have no row for, in each array of a batch, first and last entry, is an error of
+    the call (the kernels read the rows of a batch's ids unchecked), and the model goes on as if the batch had never
+    been there."""
     import dataclasses
     from orca_b200 import _lib
     g = graph("t_nb2")
@@ -530,13 +531,27 @@ def test_a_stream_with_an_id_outside_the_table_is_refused(layers):
     spec = g.spec
     gold = golden("t_nb2")
     plan = unpack(gold[f"plan_{spec.strategy}_flat"], gold[f"plan_{spec.strategy}_off"])
-    E = 2 * spec.bs + 5
-    for where in range(3):
-        ids = [np.array(a) for a in (g.sources[:E], g.destinations[:E], np.roll(g.destinations[:E], 3))]
-        ids[where][spec.bs + 7] = g.n_nodes
-        with pytest.raises(_lib.OrcaError) as err:
-            make_model(g).eval_epoch(*ids, g.timestamps[:E], g.edge_idxs[:E], spec.n_degree, spec.bs, plan)
-        assert err.value.code == 5       # ORCA_E_BOUNDS
+    E, k, bs = 2 * spec.bs + 5, spec.n_degree, spec.bs
+    good = [g.sources[:E], g.destinations[:E], np.roll(g.destinations[:E], 3), g.timestamps[:E], g.edge_idxs[:E]]
+    m, other = make_model(g), make_model(g)
+    call = lambda m, x, i: m.compute_edge_probabilities(*[a[i * bs:(i + 1) * bs] for a in x], k, True, False, plan[i])
+    call(m, good, 0), call(other, good, 0)
+    for which, lim in ((0, g.n_nodes), (1, g.n_nodes), (2, g.n_nodes), (4, g.n_edges + 1)):
+        for at, bad in ((bs, -1), (2 * bs - 1, lim), (bs + 3, 1 << 32)):
+            x = [np.array(a) for a in good]
+            x[which][at] = bad
+            with pytest.raises(_lib.OrcaError) as err:
+                call(m, x, 1)
+            assert err.value.code == 5           # ORCA_E_BOUNDS
+            if bad == 1 << 32:                   # (a stream's arrays are narrowed by numpy)
+                continue
+            for p in (plan, None):
+                with pytest.raises(_lib.OrcaError) as err:
+                    make_model(g).eval_epoch(*x, k, bs, p)
+                assert err.value.code == 5
+    for a, b in zip(call(m, good, 1), call(other, good, 1)):
+        assert torch.equal(a, b)
+    assert torch.equal(m.memory.memory, other.memory.memory)
 
 
 def test_the_status_copy_serves_every_path_whichever_ran_first():
