@@ -396,8 +396,8 @@ class TGN(nn.Module):
     # ---- model descriptor for the fused batch entry point ----------------------------------------
     def _descriptor(self, k):
         """The model descriptor of the fused batch entry.  Graph, weights and scratch pointers are filled
-        once per (neighbour finder, prepared weights, k); the state tables can be replaced between calls
-        (restore_memory, restore_history) and are refreshed every time."""
+        once per (neighbour finder, prepared weights, k); the state tables and the edge features can be replaced
+        between calls (restore_memory, restore_history, edge_raw_features) and are refreshed every time."""
         d, mods = self.__dict__, self._modules        # (plain look-ups: this runs once per batch)
         em = mods["embedding_module"].__dict__
         nf = em["neighbor_finder"]
@@ -423,6 +423,8 @@ class TGN(nn.Module):
             t.layer1_ranks = d["_layer1_ranks"]
             t.mode = d["_mode"]
             t.input_stream = d["_input_stream"]
+            edges = d["edge_raw_features"]
+            t.edge_table, t.n_edge_rows = edges.data_ptr(), edges.shape[0]
             return t
         t = _lib.TgnT()
         if getattr(self, "_exchange", None) is not None:

@@ -576,3 +576,22 @@ def test_the_status_copy_serves_every_path_whichever_ran_first():
         with pytest.raises(_lib.OrcaError) as err:
             m.compute_edge_probabilities(*batch, spec.n_degree, True, False, None)
         assert err.value.code == 4
+
+
+def test_edge_features_can_be_replaced_between_calls():
+    """``edge_raw_features`` is an attribute of the model, as in the reference: a table put in its place is the one
+    that the next call reads (the old one is kept alive here)."""
+    g = graph("t_nb2")
+    spec = g.spec
+    m, fresh = make_model(g), make_model(g)
+    old = m.edge_raw_features
+    table = torch.cat([old * -0.5 + 0.25, old])
+    it = iter(batches(g, 2))
+    for _, src, dst, ts, eidx in it:
+        batch = (src, dst, np.roll(dst, 3), ts, eidx, spec.n_degree, True, False, None)
+        a, b = m.compute_edge_probabilities(*batch), fresh.compute_edge_probabilities(*batch)
+        if m.edge_raw_features is old:
+            assert all(torch.equal(x, y) for x, y in zip(a, b))
+            m.edge_raw_features = table
+            fresh.edge_raw_features.copy_(table[:len(old)])
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
