@@ -210,6 +210,12 @@ def stream_ptr(device=None):
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def settle(device):
+    """Waits for what the caller's stream has been given.  The library's own streams start a batch without waiting for
+    that stream, so whoever reads or writes state tables there, outside a batch, ends with this."""
+    torch.cuda.current_stream(device).synchronize()
+
+
 def require_cuda(device):
     device = torch.device(device)
     if device.type != "cuda":

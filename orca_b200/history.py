@@ -76,6 +76,7 @@ class History(torch.nn.Module):
             _lib.check(L.orca_history_set_flags(self.cache_flag_dev.data_ptr(), self.num_embeddings,
                                                 self.prev_plan.data_ptr(), 0, ids.data_ptr(), ids.numel(), s))
             self.n_prev[0] = -1
+        _lib.settle(self._device)
 
     # ---- modules/history.py:32-36
     @torch.no_grad()
@@ -84,6 +85,7 @@ class History(torch.nn.Module):
         out = torch.empty(ids.numel(), self.embedding_dim, device=self._device)
         _lib.check(_lib.lib().orca_history_pull(self.emb.data_ptr(), ids.data_ptr(), ids.numel(),
                                                 out.data_ptr(), _lib.stream_ptr(self._device)))
+        _lib.settle(self._device)
         return out
 
     # ---- modules/history.py:38-40; among duplicate ids the last occurrence provides the row
@@ -103,6 +105,7 @@ class History(torch.nn.Module):
         self.epoch[0] += n
         _lib.check(L.orca_history_push(self.emb.data_ptr(), x.data_ptr(), ids.data_ptr(), win.data_ptr(),
                                        n, None, s))
+        _lib.settle(self._device)
 
     # ---- modules/history.py:42-46
     def push_and_pull(self, x, push_inds, pull_inds):

@@ -55,18 +55,25 @@ class Memory(nn.Module):
         self.messages[ix] = messages
         self.timestamps[ix] = timestamps
 
+    # (what is read here is read before the next batch rewrites it)
     def get_memory(self, node_idxs):
-        return self.memory[self._ix(node_idxs), :]
+        rows = self.memory[self._ix(node_idxs), :]
+        _lib.settle(self.device)
+        return rows
 
     def set_memory(self, node_idxs, values):
         self.memory[self._ix(node_idxs), :] = values
 
     def get_last_update(self, node_idxs):
-        return self.last_update[self._ix(node_idxs)]
+        times = self.last_update[self._ix(node_idxs)]
+        _lib.settle(self.device)
+        return times
 
     def backup_memory(self):
-        return (self.memory.clone(), self.last_update.clone(), self.messages.clone(), self.nodes_dev.clone(),
-                self.timestamps.clone())
+        copies = (self.memory.clone(), self.last_update.clone(), self.messages.clone(), self.nodes_dev.clone(),
+                  self.timestamps.clone())
+        _lib.settle(self.device)
+        return copies
 
     def restore_memory(self, memory_backup):
         self.memory, self.last_update, self.messages = (memory_backup[0].clone(), memory_backup[1].clone(),
@@ -128,6 +135,7 @@ class GRUMemoryUpdater(nn.Module):
         gw, ms = self.c_struct(), memory.c_struct()
         _lib.check(L.orca_gru_update(gw, ms, ids.data_ptr(), n, None, 1 if clear else 0, scratch.data_ptr(),
                                      _lib.stream_ptr(memory.device)))
+        _lib.settle(memory.device)
 
     @torch.no_grad()
     def update_memory(self, memory: Memory, positives):

@@ -88,7 +88,9 @@ class GraphAttentionEmbedding(nn.Module):
             for _ in range(n_layers)])
 
     def backup_history(self):
-        return [self.histories[i].emb.clone() for i in range(self.n_layers - 1)]
+        copies = [self.histories[i].emb.clone() for i in range(self.n_layers - 1)]
+        _lib.settle(self.device)
+        return copies
 
     def restore_history(self, backup):
         for i in range(self.n_layers - 1):
@@ -131,6 +133,14 @@ class _Staging:
             ev = torch.cuda.Event()
             self.events[i] = ev
         ev.record(stream)
+
+
+def _versions(tables):
+    """The tensors' counters of in-place writes; None where they are not kept (tensors made in inference mode)."""
+    try:
+        return [x._version for x in tables]
+    except RuntimeError:
+        return None
 
 
 class TGN(nn.Module):
@@ -397,7 +407,10 @@ class TGN(nn.Module):
     def _descriptor(self, k):
         """The model descriptor of the fused batch entry.  Graph, weights and scratch pointers are filled
         once per (neighbour finder, prepared weights, k); the state tables and the edge features can be replaced
-        between calls (restore_memory, restore_history, edge_raw_features) and are refreshed every time."""
+        between calls (restore_memory, restore_history, edge_raw_features) and are refreshed every time.
+        A batch starts on the library's streams, which do not wait for the caller's.  So weights that have just been
+        packed and tables that were replaced or written in place since the last call (their version counters say so) are
+        waited for here."""
         d, mods = self.__dict__, self._modules        # (plain look-ups: this runs once per batch)
         em = mods["embedding_module"].__dict__
         nf = em["neighbor_finder"]
@@ -405,28 +418,30 @@ class TGN(nn.Module):
         gw = mods["memory_updater"].prepared()
         ref = d.get("_desc_ref")                      # the objects themselves are kept: identities cannot be reused
         if ref is not None and ref[0] is nf and ref[1] is w and ref[2] is gw and ref[3] == k:
-            t, m, tm = d["_desc"], mods["memory"].__dict__, d["_desc_mem"]
-            tm.memory, tm.last_update, tm.messages = (m["memory"].data_ptr(), m["last_update"].data_ptr(),
-                                                      m["messages"].data_ptr())
-            tm.msg_ts, tm.msg_flag = m["timestamps"].data_ptr(), m["nodes_dev"].data_ptr()
+            t, m, edges = d["_desc"], mods["memory"].__dict__, d["edge_raw_features"]
+            tables = [m["memory"], m["last_update"], m["messages"], m["timestamps"], m["nodes_dev"], edges]
             hist = mods["embedding_module"]._modules.get("histories") if self.n_layers == 2 else None
-            if hist is not None:
-                h = hist[0].__dict__
-                t.hist_emb = h["emb"].data_ptr()
-                t.cache_flag = h["cache_flag_dev"].data_ptr()
-                t.prev_plan = h["prev_plan"].data_ptr()
-                if d.get("_desc_n_prev") is not h["n_prev"]:
+            h = hist._modules["0"].__dict__ if hist is not None else None
+            if h is not None:
+                tables += (h["emb"], h["cache_flag_dev"], h["prev_plan"])
+                if d["_desc_n_prev"] is not h["n_prev"]:
                     d["_desc_n_prev"] = h["n_prev"]
                     t.n_prev_plan = h["n_prev"].ctypes.data_as(C.POINTER(C.c_int32))
-                t.plan_cap = h["prev_plan"].numel()
-            t.rank, t.world = d["_rank"], d["_world"]
-            t.layer1_ranks = d["_layer1_ranks"]
-            t.mode = d["_mode"]
-            t.input_stream = d["_input_stream"]
-            edges = d["edge_raw_features"]
-            t.edge_table, t.n_edge_rows = edges.data_ptr(), edges.shape[0]
+            seen = ([x.data_ptr() for x in tables], _versions(tables), d["_mode"], d["_rank"], d["_world"],
+                    d["_layer1_ranks"], d["_input_stream"])
+            if seen != d["_desc_seen"] or edges is not d["_desc_edges"] or seen[1] is None:
+                d["_desc_seen"], d["_desc_edges"] = seen, edges
+                tm = d["_desc_mem"]
+                tm.memory, tm.last_update, tm.messages, tm.msg_ts, tm.msg_flag, t.edge_table = seen[0][:6]
+                t.n_edge_rows = edges.shape[0]
+                if h is not None:
+                    t.hist_emb, t.cache_flag, t.prev_plan = seen[0][6:]
+                    t.plan_cap = h["prev_plan"].numel()
+                t.mode, t.rank, t.world, t.layer1_ranks, t.input_stream = seen[2:]
+                _lib.settle(self.device)
             return t
         t = _lib.TgnT()
+        d["_desc_seen"] = d["_desc_edges"] = None
         if getattr(self, "_exchange", None) is not None:
             rows, flags, cap, _, grus, gcap = self._exchange
             for r in range(len(rows)):
@@ -468,6 +483,7 @@ class TGN(nn.Module):
         t.mode = self._mode
         t.ctx = self._ctx
         t.input_stream = self._input_stream
+        _lib.settle(self.device)
         return t
 
     def _workspace(self, b, k):

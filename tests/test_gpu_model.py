@@ -595,3 +595,87 @@ def test_edge_features_can_be_replaced_between_calls():
             m.edge_raw_features = table
             fresh.edge_raw_features.copy_(table[:len(old)])
     assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def _after_a_long_kernel(f):
+    """f() behind some milliseconds of work on the caller's stream: what it enqueues there runs late."""
+    torch.cuda._sleep(20_000_000)
+    return f()
+
+
+def test_a_batch_sees_what_was_written_on_the_callers_stream():
+    """Tables replaced, written in place or written by the library's own calls between two batches, and weights that
+    are packed at the first one, are complete when a batch starts on the library's streams; copies taken between two
+    batches hold what the first one left."""
+    g = graph("t_nb2")
+    spec = g.spec
+    k = spec.n_degree
+    gold = golden("t_nb2")
+    plan = unpack(gold[f"plan_{spec.strategy}_flat"], gold[f"plan_{spec.strategy}_off"])
+    bat = [(s, d, np.roll(d, 3), t, e, k, True, False, plan[b]) for b, s, d, t, e in batches(g, 4)]
+
+    def want(change):     # the same with everything waited for
+        m = make_model(g)
+        for i, x in enumerate(bat[:3]):
+            if i == 2:
+                change(m)
+                torch.cuda.synchronize()
+            r = m.compute_edge_probabilities(*x)
+            torch.cuda.synchronize()
+        return [t.cpu() for t in r] + [m.memory.memory.cpu()]
+
+    rows = torch.randn(g.n_nodes, 172, device="cuda")
+    ids = np.arange(1, g.n_nodes)
+    shift = (torch.randn(g.n_nodes, device="cuda") * 5).cpu()
+    state = make_model(g).memory.backup_memory()
+    changes = [lambda m: m.memory.memory.copy_(rows),
+               lambda m: m.memory.set_memory(ids, rows[1:]),
+               lambda m: m.memory.restore_memory((rows,) + state[1:]),
+               lambda m: m.embedding_module.histories[0].emb.copy_(rows),
+               lambda m: m.embedding_module.histories[0].push(rows[1:], ids),
+               lambda m: m.embedding_module.histories[0].update_flag(ids[::3], None),
+               lambda m: m.embedding_module.reset_history(),
+               lambda m: m.memory.last_update.copy_(shift.cuda()),
+               lambda m: m.edge_raw_features.mul_(0.5)]
+    for n, change in enumerate(changes):
+        w = want(change)
+        m = make_model(g)
+        for x in bat[:2]:
+            m.compute_edge_probabilities(*x)
+        _after_a_long_kernel(lambda: change(m))
+        r = [t.cpu() for t in m.compute_edge_probabilities(*bat[2])] + [m.memory.memory.cpu()]
+        assert all(torch.equal(a, b) for a, b in zip(r, w)), n
+    # weights packed late, at the first call
+    w = want(lambda m: m.refresh_weights())
+    m = make_model(g)
+    for x in bat[:2]:
+        m.compute_edge_probabilities(*x)
+    m.refresh_weights()
+    torch.cuda._sleep(20_000_000)
+    r = [t.cpu() for t in m.compute_edge_probabilities(*bat[2])] + [m.memory.memory.cpu()]
+    assert all(torch.equal(a, b) for a, b in zip(r, w))
+    # copies taken between two batches
+    m, o = make_model(g), make_model(g)
+    for x in bat[:2]:
+        m.compute_edge_probabilities(*x), o.compute_edge_probabilities(*x)
+    torch.cuda.synchronize()
+    late = _after_a_long_kernel(lambda: (*m.memory.backup_memory(), *m.embedding_module.backup_history(),
+                                         m.memory.get_memory(ids), m.memory.get_last_update(ids),
+                                         m.embedding_module.histories[0].pull(ids)))
+    m.compute_edge_probabilities(*bat[2])
+    now = (*o.memory.backup_memory(), *o.embedding_module.backup_history(), o.memory.get_memory(ids),
+           o.memory.get_last_update(ids), o.embedding_module.histories[0].pull(ids))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(late, now))
+
+
+def test_a_model_made_in_inference_mode_scores():
+    g = graph("t_nb2")
+    with torch.inference_mode():
+        m = make_model(g)
+        _, s, d, t, e = next(iter(batches(g, 1)))
+        out = [m.compute_edge_probabilities(s, d, np.roll(d, 3), t, e, g.spec.n_degree, True, False, None) for _ in range(2)]
+    o = make_model(g)
+    for r in out:
+        for a, b in zip(r, o.compute_edge_probabilities(s, d, np.roll(d, 3), t, e, g.spec.n_degree, True, False, None)):
+            assert torch.equal(a, b)
