@@ -17,11 +17,10 @@
 // time (eight loads in flight); lanes with the same digit find one another with match.any, so a record's rank among
 // its digit is the warp's running count plus the number of lower lanes in its group.
 #include <algorithm>
-#include <thread>
-#include <vector>
 
 #include "common.cuh"
 #include "context.cuh"
+#include "host_threads.cuh"
 
 namespace orca {
 namespace csr {
@@ -401,9 +400,10 @@ extern "C" int64_t orca_csr_build_workspace_bytes(int64_t n_edges, int64_t n_nod
 
 // slots of the packing threads: 16 threads keep ahead of the bus on this pool's hosts (16 cores), and a thread is
 // worth starting for a chunk or more
+constexpr int MOST_THREADS = 16;
 static int pack_threads(int64_t n_edges) {
   const int64_t chunks = (n_edges + csr::CHUNK - 1) >> csr::CHUNK_LOG;
-  return (int)std::max<int64_t>(1, std::min<int64_t>({16, chunks, (int64_t)std::thread::hardware_concurrency()}));
+  return (int)std::max<int64_t>(1, std::min<int64_t>({MOST_THREADS, chunks, (int64_t)std::thread::hardware_concurrency()}));
 }
 
 extern "C" int64_t orca_csr_build_pinned_bytes(int64_t n_edges) {
@@ -465,24 +465,23 @@ extern "C" int orca_csr_build_from_host(const int64_t *h_src, const int64_t *h_d
                      (long long)pinned_bytes, (long long)(2 * csr::CHUNK_BYTES));
   int device = 0;
   ORCA_CUDA(cudaGetDevice(&device));
-  std::vector<csr::Packed> seen((size_t)threads);
-  std::vector<std::thread> pool;
+  csr::Packed seen[MOST_THREADS];
   auto part = [&](int t) {
     csr::pack_chunks(h_src, h_dst, h_eidx, h_ts, n_edges, n_nodes, t, threads,
                      (char *)h_pinned + (size_t)t * 2 * csr::CHUNK_BYTES, csr::Edges{base + L.edges}, device, s, &seen[t]);
   };
-  for (int t = 1; t < threads; ++t) pool.emplace_back(part, t);
-  part(0);
-  for (std::thread &t : pool) t.join();
+  rc = on_threads(threads, part, "orca_csr_build_from_host");
   bool in_order = true;
   int64_t bad = -1;
-  for (const csr::Packed &p : seen) {
-    if (p.rc != ORCA_OK) return set_error(p.rc, "%s", p.err);
+  for (int t = 0; t < threads; ++t) {
+    const csr::Packed &p = seen[t];
+    if (p.rc != ORCA_OK) rc = set_error(p.rc, "%s", p.err);
     in_order = in_order && p.in_order;
     if (p.bad_edge >= 0 && (bad < 0 || p.bad_edge < bad)) bad = p.bad_edge;
   }
+  if (rc || bad >= 0) cudaStreamSynchronize(s);     // (copies from the pinned slots may be in flight)
+  if (rc) return rc;
   if (bad >= 0) {
-    ORCA_CUDA(cudaStreamSynchronize(s));     // (copies from the pinned slots may be in flight)
     return set_error(ORCA_E_BOUNDS, "orca_csr_build_from_host: edge %lld has an endpoint outside [0,%lld)", (long long)bad,
                      (long long)n_nodes);
   }

@@ -10,10 +10,10 @@
 #include <string.h>
 
 #include <algorithm>
-#include <thread>
 #include <vector>
 
 #include "common.cuh"
+#include "host_threads.cuh"
 
 namespace orca {
 namespace metrics {
@@ -97,20 +97,20 @@ extern "C" int orca_link_metrics(const float *h_pos, const float *h_neg, int64_t
   ORCA_CHECK_ARG(h_pos && h_neg && h_out && n_edges >= 0 && bs > 0);
   const int64_t nb = (n_edges + bs - 1) / bs;
   // a thread is worth starting for about 64 k scores (a millisecond); at most eight
-  const int64_t want = std::min<int64_t>({8, nb, 1 + n_edges / 65536, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
-  std::vector<int64_t> bad((size_t)std::max<int64_t>(want, 1), -1);
-  auto work = [&](int64_t t) {
+  constexpr int MOST = 8;
+  const int want = (int)std::min<int64_t>({MOST, nb, 1 + n_edges / 65536, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
+  int64_t bad[MOST];
+  auto work = [&](int t) {
+    bad[t] = -1;
     metrics::Scratch s;
     for (int64_t i = t; i < nb; i += want) {
       const int64_t lo = i * bs, n = std::min<int64_t>(bs, n_edges - lo);
       if (!metrics::one_batch(h_pos + lo, h_neg + lo, n, h_out + 3 * i, s) && bad[t] < 0) bad[t] = i;
     }
   };
-  std::vector<std::thread> threads;
-  for (int64_t t = 1; t < want; ++t) threads.emplace_back(work, t);
-  if (want > 0) work(0);
-  for (std::thread &t : threads) t.join();
-  for (int64_t b : bad)
-    if (b >= 0) return set_error(ORCA_E_BADARG, "orca_link_metrics: a score of batch %lld is not finite", (long long)b);
+  const int rc = on_threads(want, work, "orca_link_metrics");
+  if (rc) return rc;
+  for (int t = 0; t < want; ++t)
+    if (bad[t] >= 0) return set_error(ORCA_E_BADARG, "orca_link_metrics: a score of batch %lld is not finite", (long long)bad[t]);
   return ORCA_OK;
 }

@@ -439,7 +439,7 @@ using namespace orca;
 extern "C" int orca_plan_host(int32_t strategy, const int64_t *h_src, const int64_t *h_dst, int64_t n_edges,
                               int32_t bs, int32_t k, const int32_t *h_nbr, int64_t n_nodes, int32_t budget,
                               uint32_t seed, int32_t *h_plan_flat, int64_t plan_cap, int64_t *h_plan_off,
-                              double *h_stats) {
+                              double *h_stats) try {
   ORCA_CHECK_ARG(h_src && h_dst && h_nbr && h_plan_flat && h_plan_off && h_stats);
   ORCA_CHECK_ARG(n_edges >= 0 && bs > 0 && k >= 1 && k <= ORCA_MAX_K && n_nodes > 0 && budget > 0);
   ORCA_CHECK_ARG(strategy >= 0 && strategy <= 2);
@@ -460,4 +460,6 @@ extern "C" int orca_plan_host(int32_t strategy, const int64_t *h_src, const int6
   h_stats[1] = st.recompute;
   h_stats[2] = st.dist;
   return ORCA_OK;
+} catch (const std::bad_alloc &) {
+  return set_error(ORCA_E_CAPACITY, "orca_plan_host: out of host memory");
 }

@@ -625,7 +625,7 @@ int orca_version(void) { return 1; }
 
 int orca_csr_build_host(const int64_t *h_src, const int64_t *h_dst, const int64_t *h_eidx,
                         const double *h_ts, int64_t n_edges, int64_t n_nodes, int64_t *h_indptr,
-                        int32_t *h_nbr, int32_t *h_eid, double *h_adj_ts) {
+                        int32_t *h_nbr, int32_t *h_eid, double *h_adj_ts) try {
   ORCA_CHECK_ARG(h_src && h_dst && h_eidx && h_ts && h_indptr && h_nbr && h_eid && h_adj_ts);
   ORCA_CHECK_ARG(n_edges >= 0 && n_nodes > 0);
   std::fill(h_indptr, h_indptr + n_nodes + 1, (int64_t)0);
@@ -663,6 +663,8 @@ int orca_csr_build_host(const int64_t *h_src, const int64_t *h_dst, const int64_
     }
   }
   return ORCA_OK;
+} catch (const std::bad_alloc &) {
+  return orca::set_error(ORCA_E_CAPACITY, "orca_csr_build_host: out of host memory");
 }
 
 static int orca_sample_topk_impl(const int64_t *d_indptr, const int32_t *d_adj_nbr, const int32_t *d_adj_eid,

@@ -4,6 +4,8 @@ the oracle.  No GPU is needed (no kernel is launched)."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -95,3 +97,38 @@ def test_no_fallback_without_cuda():
         History(10, 172, device="cuda")
     with pytest.raises(RuntimeError):
         History(10, 172, device="cpu")
+
+
+LIMITED = """
+import ctypes, resource, sys
+import numpy as np
+from orca_b200 import _lib
+L = _lib.lib()
+n, nodes = 300000, 8 << 20
+pos, neg, out = np.linspace(0.1, 0.9, n).astype(np.float32), np.full(n, 0.5, np.float32), np.empty((74, 3))
+want = out.copy()
+ids, ts = np.zeros(1, np.int64), np.zeros(1)
+indptr, adj = np.zeros(nodes + 1, np.int64), [np.zeros(2, t) for t in (np.int32, np.int32, np.float64)]
+args = [a.ctypes.data for a in (ids, ids, ids, ts)] + [1, nodes] + [a.ctypes.data for a in (indptr, *adj)]
+for i in range(74):     # (one batch a call: no threads yet, whose stacks would be kept)
+    m = min(4096, n - 4096 * i)
+    assert L.orca_link_metrics(pos[4096 * i:].ctypes.data, neg[4096 * i:].ctypes.data, m, 4096, want[i:].ctypes.data) == 0
+# room for small allocations, not for another thread's stack or for 64 MB
+size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size + (6 << 20),) * 2)
+rc = {"metrics": lambda: L.orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, 4096, out.ctypes.data),
+      "csr": lambda: L.orca_csr_build_host(*args), "plan": lambda: L.orca_plan_host(
+          0, ids.ctypes.data, ids.ctypes.data, 1, 1, 1, adj[0].ctypes.data, nodes, 1, 0, adj[1].ctypes.data, 2,
+          indptr.ctypes.data, out.ctypes.data)}[sys.argv[1]]()
+print("rc", rc, bool((out == want).all()))
+"""
+
+
+@pytest.mark.parametrize("entry,said", [("metrics", "rc 0 True"), ("csr", "rc 4"), ("plan", "rc 4")])
+def test_no_exception_leaves_an_entry_point(entry, said):
+    """Threads that cannot be started and host memory that is not there end neither the process (the shares are done by
+    the calling thread) nor go unsaid (an error code)."""
+    build.build()
+    env = dict(os.environ, OMP_NUM_THREADS="1", OPENBLAS_NUM_THREADS="1", MALLOC_ARENA_MAX="1")
+    r = subprocess.run([sys.executable, "-c", LIMITED, entry], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and said in r.stdout, (r.returncode, r.stdout, r.stderr[-2000:])
