@@ -546,7 +546,7 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
  * page-locked slots and copied from there on the context's copy stream.  Waits only when the ring is full.  The status
  * word follows the batch to h_status (page-locked) in `stream` order.
  * The entry points that are given a batch in host memory (this one, orca_tgn_eval_epoch, orca_tgn_eval_group) return
- * ORCA_E_BOUNDS, with nothing of the batch enqueued, for a node or edge id outside its table.
+ * ORCA_E_BOUNDS, with no kernel of the batch enqueued, for a node or edge id outside its table.
  */
 #define ORCA_CALL_SLOTS 8
 typedef struct {

@@ -503,7 +503,6 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     const int plan = std::max(g->n_plan[n], 0);
     ORCA_CHECK_ARG(g->off_i32[n] == base_i32 + n_i32 && plan <= g->plan_cap && (!budget || g->n_plan[n] >= 0));
     a.off[n] = (int)n_i32, a.n_plan[n] = plan;
-    if (g->phase & 1) ORCA_TRY(check_batch_ids(m, g->h_i32 + base_i32 + n_i32, a.b_of(n), n, "orca_tgn_eval_group"));
     n_i32 += 4ll * a.b_of(n) + plan;
   }
   if (budget) ORCA_CHECK_ARG(a.n_plan[g->nb - 1] <= m->plan_cap);
@@ -539,6 +538,8 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     if (c->gdone_recorded[p] && sc != s) ORCA_CUDA(cudaStreamWaitEvent(sc, c->ev_gdone[p], 0));
     ORCA_CUDA(cudaMemcpyAsync(x.stage, g->h_i32 + base_i32, (size_t)n_i32 * 4, cudaMemcpyHostToDevice, sc));
     ORCA_CUDA(cudaMemcpyAsync(x.stage + ts_off, g->h_ts, (size_t)E * 8, cudaMemcpyHostToDevice, sc));
+    for (int n = 0; n < g->nb; ++n)     // (while the copies are on the bus)
+      ORCA_TRY(check_batch_ids(m, g->h_i32 + base_i32 + a.off[n], a.b_of(n), n, "orca_tgn_eval_group"));
     if (si != sc) {     // (in order behind the copies: the parity's buffers are free, too)
       ORCA_CUDA(cudaEventRecord(c->ev_gin, sc));
       ORCA_CUDA(cudaStreamWaitEvent(si, c->ev_gin, 0));
