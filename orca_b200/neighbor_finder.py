@@ -8,14 +8,53 @@ int32, edge id int32, timestamp float64) resident in HBM, built there by ``orca_
 """
 from __future__ import annotations
 
+import collections
+import threading
+
 import numpy as np
 import torch
 
 from . import _lib
 
 
+class _Lent:
+    """Bytes of page-locked memory that returned tables hold, over the process: at most `limit` of them."""
+
+    def __init__(self, limit):
+        self.limit, self.held = limit, 0
+        self.back = collections.deque()     # (what came back; filled by __del__, which must not wait for a lock)
+        self.lock = threading.Lock()
+
+    def take(self, n):
+        """A share of n bytes, which comes back when it and the arrays made from it are gone; None: there is no room."""
+        with self.lock:
+            while self.back:
+                self.held -= self.back.popleft()
+            if self.held + n > self.limit:
+                return None
+            self.held += n
+        return _Share(self.back, n)
+
+
+class _Share:
+    __slots__ = ("back", "n", "pin", "__array_interface__")
+
+    def __init__(self, back, n):
+        self.back, self.n = back, n
+
+    def array(self, pin):
+        """The page-locked tensor of bytes as an array that keeps this share."""
+        self.pin = pin
+        self.__array_interface__ = {"data": (pin.data_ptr(), False), "shape": (pin.numel(),), "typestr": "|u1", "version": 3}
+        return np.asarray(self)
+
+    def __del__(self):
+        self.back.append(self.n)
+
+
 class NeighborFinder:
     PINNED_TABLE = 64 << 20     # bytes of one returned table up to which it stays in page-locked memory
+    LENT = _Lent(256 << 20)     # and of all that callers hold: a few calls' tables of the largest size
 
     def __init__(self, node_to_neighbors, node_to_edge_idxs, node_to_edge_timestamps, device="cuda"):
         """Same arguments as utils/util.py:123-126: per-node arrays, each already sorted by time."""
@@ -94,16 +133,20 @@ class NeighborFinder:
         q, k = len(source_nodes), int(n_neighbors)
         table = 4 * q * k
         # The tables are returned in the page-locked memory that they were copied to: a fresh pageable array of a few
-        # MB costs more in page faults than the whole call.  Tables too large to keep page-locked, inputs that are
-        # already on the GPU and empty queries take the general path.
-        if not 0 < table <= self.PINNED_TABLE or isinstance(source_nodes, torch.Tensor) or isinstance(timestamps, torch.Tensor):
+        # MB costs more in page faults than the whole call (40 k queries of ten: 195 us so, 860 on the general path).
+        # Tables too large for that, more of them than callers may hold, inputs that are already on the GPU and empty
+        # queries take the general path.
+        out = (12 * q + 15) // 16 * 16 + 16
+        share = None
+        if 0 < table <= self.PINNED_TABLE and not isinstance(source_nodes, torch.Tensor) and not isinstance(timestamps, torch.Tensor):
+            share = self.LENT.take(1 << (out + 3 * table - 1).bit_length())      # (the pool's blocks are powers of two)
+        if share is None:
             nbr, eid, et, _ = self.sample_device(source_nodes, timestamps, n_neighbors)
             return nbr.cpu().numpy(), eid.cpu().numpy(), et.cpu().numpy()
         nodes = np.ascontiguousarray(source_nodes, dtype=np.int64)
         ts = np.ascontiguousarray(timestamps, dtype=np.float64)
         if nodes.shape != (q,) or ts.shape != (q,):
             raise ValueError("source_nodes and timestamps must be one-dimensional and of one length")
-        out = (12 * q + 15) // 16 * 16 + 16
         pin = torch.empty(out + 3 * table, dtype=torch.uint8, pin_memory=True)
         dev = torch.empty(out + 3 * table, dtype=torch.uint8, device=self.device)
         with torch.cuda.device(self.device):
@@ -111,7 +154,7 @@ class NeighborFinder:
                 self.indptr.data_ptr(), self.adj_nbr.data_ptr(), self.adj_eid.data_ptr(), self.adj_ts.data_ptr(),
                 self.n_nodes, nodes.ctypes.data, ts.ctypes.data, q, k, pin.data_ptr(), dev.data_ptr(), dev.numel(),
                 _lib.stream_ptr(self.device)))
-        h = pin.numpy()
+        h = share.array(pin)
         part = lambda i, dt: h[out + i * table:out + (i + 1) * table].view(dt).reshape(q, k)
         return part(0, np.int32), part(1, np.int32), part(2, np.float32)
 

@@ -67,3 +67,30 @@ def test_neighbor_tables_from_host_arrays(q, k):
         lo, hi = oracle.indptr[nodes[i]], oracle.indptr[nodes[i] + 1]
         row = oracle.nbr[lo:hi][oracle.ts[lo:hi] < times[i]][-k:]
         assert np.array_equal(got[0][i], np.r_[np.zeros(k - len(row), np.int32), row])
+
+
+def test_tables_that_callers_keep_hold_a_bounded_amount_of_page_locked_memory():
+    """Tables of many calls, or one table of each, stay with the caller: page-locked up to a limit, ordinary arrays
+    beyond it, with the same contents; what is dropped can be page-locked again."""
+    from orca_b200.neighbor_finder import NeighborFinder
+    src, dst, eidx, ts = _stream(5000, 300, True, 9)
+    nf = NeighborFinder.build_on_device(src, dst, eidx, ts, 300)
+    rs = np.random.RandomState(3)
+    nodes, times = rs.randint(0, 300, 60000), rs.rand(60000) * 2000
+    locked = lambda a: torch.from_numpy(a).is_pinned()
+    want = [t.cpu().numpy() for t in nf.sample_device(nodes, times, 20)[:3]]
+    for keep in (slice(0, 3), slice(1, 2)):      # all three tables, or the middle one, which holds its neighbours
+        held, n = [], 0
+        for _ in range(24):                      # 14.4 MB a call
+            tables = nf.get_temporal_neighbor(nodes, times, 20)
+            n += locked(tables[0])
+            held += tables[keep]
+            for t, w in zip(tables, want):
+                assert np.array_equal(t, w)
+        assert 2 <= n and n * 3 * 4 * nodes.size * 20 <= 256 << 20
+        del tables
+        held.clear()
+        assert all(locked(t) for t in nf.get_temporal_neighbor(nodes, times, 20))
+    with pytest.raises(Exception):
+        nf.get_temporal_neighbor(nodes, times, 33)      # (a call that fails holds nothing)
+    assert all(locked(t) for t in nf.get_temporal_neighbor(nodes, times, 20))
