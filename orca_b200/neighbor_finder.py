@@ -9,6 +9,7 @@ int32, edge id int32, timestamp float64) resident in HBM, built there by ``orca_
 from __future__ import annotations
 
 import collections
+import operator
 import threading
 
 import numpy as np
@@ -130,23 +131,25 @@ class NeighborFinder:
         """Returns (neighbors int32 [Q,K], edge_idxs int32 [Q,K], edge_times float32 [Q,K]) as NumPy
         arrays: the K most recent interactions strictly before each query time, right-aligned,
         zero-padded on the left."""
-        q, k = len(source_nodes), int(n_neighbors)
+        k = operator.index(n_neighbors)
+        host = not isinstance(source_nodes, torch.Tensor) and not isinstance(timestamps, torch.Tensor)
+        if host:
+            nodes, ts = np.asarray(source_nodes), np.asarray(timestamps)
+            host = nodes.ndim == 1 and ts.shape == nodes.shape
+        q = nodes.size if host else 0
         table = 4 * q * k
         # The tables are returned in the page-locked memory that they were copied to: a fresh pageable array of a few
         # MB costs more in page faults than the whole call (40 k queries of ten: 195 us so, 860 on the general path).
-        # Tables too large for that, more of them than callers may hold, inputs that are already on the GPU and empty
-        # queries take the general path.
+        # Tables too large for that, more of them than callers may hold, inputs that are already on the GPU, of other
+        # shapes than one list of nodes with a time each, and empty queries take the general path.
         out = (12 * q + 15) // 16 * 16 + 16
         share = None
-        if 0 < table <= self.PINNED_TABLE and not isinstance(source_nodes, torch.Tensor) and not isinstance(timestamps, torch.Tensor):
+        if 0 < table <= self.PINNED_TABLE:
             share = self.LENT.take(1 << (out + 3 * table - 1).bit_length())      # (the pool's blocks are powers of two)
         if share is None:
             nbr, eid, et, _ = self.sample_device(source_nodes, timestamps, n_neighbors)
             return nbr.cpu().numpy(), eid.cpu().numpy(), et.cpu().numpy()
-        nodes = np.ascontiguousarray(source_nodes, dtype=np.int64)
-        ts = np.ascontiguousarray(timestamps, dtype=np.float64)
-        if nodes.shape != (q,) or ts.shape != (q,):
-            raise ValueError("source_nodes and timestamps must be one-dimensional and of one length")
+        nodes, ts = np.ascontiguousarray(nodes, dtype=np.int64), np.ascontiguousarray(ts, dtype=np.float64)
         pin = torch.empty(out + 3 * table, dtype=torch.uint8, pin_memory=True)
         dev = torch.empty(out + 3 * table, dtype=torch.uint8, device=self.device)
         with torch.cuda.device(self.device):
@@ -166,7 +169,9 @@ class NeighborFinder:
             if not isinstance(source_nodes, torch.Tensor) else source_nodes.to(self.device, torch.int32)
         ts = torch.as_tensor(np.asarray(timestamps), dtype=torch.float64).to(self.device) \
             if not isinstance(timestamps, torch.Tensor) else timestamps.to(self.device, torch.float64)
-        q = nodes.numel()
+        nodes, ts, q = nodes.contiguous(), ts.contiguous(), nodes.numel()
+        if ts.numel() < q:
+            raise ValueError("every source node needs a timestamp")
         nbr = torch.zeros((q, k), dtype=torch.int32, device=self.device)
         eid = torch.zeros((q, k), dtype=torch.int32, device=self.device)
         et = torch.zeros((q, k), dtype=torch.float32, device=self.device)

@@ -94,3 +94,30 @@ def test_tables_that_callers_keep_hold_a_bounded_amount_of_page_locked_memory():
     with pytest.raises(Exception):
         nf.get_temporal_neighbor(nodes, times, 33)      # (a call that fails holds nothing)
     assert all(locked(t) for t in nf.get_temporal_neighbor(nodes, times, 20))
+
+
+def test_neighbor_tables_for_every_form_of_query():
+    """One node, a matrix of nodes, lists, strided and read-only arrays, ids and times of other types, more times than
+    nodes: what a list of nodes with a time each gives.  A node without a time is an error."""
+    from orca_b200.neighbor_finder import NeighborFinder
+    src, dst, eidx, ts = _stream(5000, 300, True, 9)
+    nf = NeighborFinder.build_on_device(src, dst, eidx, ts, 300)
+    rs = np.random.RandomState(5)
+    nodes, times = rs.randint(0, 300, 24), np.floor(rs.rand(24) * 1500)
+    want = nf.get_temporal_neighbor(nodes, times, 7)
+    frozen = nodes.copy()
+    frozen.flags.writeable = False
+    for n, t in ((nodes.reshape(4, 6), times.reshape(4, 6)), (list(nodes), list(times)), (frozen, times),
+                 (np.repeat(nodes, 2)[::2], np.repeat(times, 3)[::3]), (nodes.astype(np.float32), times.astype(np.int64)),
+                 (nodes, np.r_[times, 5.0]), (nodes.reshape(24, 1), times), (torch.from_numpy(nodes).cuda(), times),
+                 (torch.from_numpy(np.repeat(nodes, 2)).int().cuda()[::2], torch.from_numpy(np.repeat(times, 2)).cuda()[::2]),
+                 (np.asfortranarray(nodes.reshape(4, 6).astype(np.int32)), times.reshape(4, 6))):
+        for g, w in zip(nf.get_temporal_neighbor(n, t, np.int64(7)), want):
+            assert g.dtype == w.dtype and np.array_equal(g, w)
+    for g, w in zip(nf.get_temporal_neighbor(int(nodes[3]), float(times[3]), 7), want):
+        assert np.array_equal(g, w[3:4])
+    for n, t in ((nodes, times[:-1]), (nodes.reshape(4, 6), times[0])):
+        with pytest.raises(ValueError):
+            nf.get_temporal_neighbor(n, t, 7)
+    with pytest.raises(TypeError):
+        nf.get_temporal_neighbor(nodes, times, 7.5)
