@@ -21,7 +21,7 @@ from .memory import Memory, get_memory_updater
 
 # recursion modes of the fused batch entry point (ORCA_MODE_* of the C header)
 MODE_BUDGET, MODE_REUSE_ALL, MODE_NO_REUSE = 0, 1, 2
-_I64 = np.dtype(np.int64)
+_I64, _F64 = np.dtype(np.int64), np.dtype(np.float64)
 
 
 class MergeLayer(nn.Module):
@@ -133,6 +133,16 @@ class _Staging:
             ev = torch.cuda.Event()
             self.events[i] = ev
         ev.record(stream)
+
+
+def _column(a, n, dtype):
+    """One of a batch's arrays as n contiguous values: as it is, or as an assignment to n values takes it (one value
+    stands for all; another length is a ValueError)."""
+    if type(a) is np.ndarray and a.dtype == dtype and a.shape == (n,) and a.flags.c_contiguous:
+        return a
+    out = np.empty(n, dtype=dtype)
+    out[:] = a
+    return out
 
 
 def _versions(tables):
@@ -527,12 +537,9 @@ class TGN(nn.Module):
         # (Host time per call is what bounds a small batch: plain attribute access and no torch call that can be
         # left out.)
         d = self.__dict__
-        host = [a if type(a) is np.ndarray and a.dtype == _I64 and a.flags.c_contiguous else np.ascontiguousarray(a, dtype=_I64)
-                for a in (source_nodes, destination_nodes, negative_nodes, edge_idxs)]
-        ts = np.ascontiguousarray(edge_times, dtype=np.float64)
-        if not b == len(host[1]) == len(host[2]) == len(host[3]) == len(ts):
-            raise ValueError("the arrays of a batch must have one length")
-        pl = np.ascontiguousarray(cache_plan, dtype=_I64) if n_plan else None
+        host = [_column(a, b, _I64) for a in (source_nodes, destination_nodes, negative_nodes, edge_idxs)]
+        ts = _column(edge_times, b, _F64)
+        pl = _column(cache_plan, n_plan, _I64) if n_plan else None
         need = 24 * b + 4 * n_plan + 16
         ring = d.get("_call_ring")
         if ring is None or ring[2] < need:

@@ -679,3 +679,25 @@ def test_a_model_made_in_inference_mode_scores():
     for r in out:
         for a, b in zip(r, o.compute_edge_probabilities(s, d, np.roll(d, 3), t, e, g.spec.n_degree, True, False, None)):
             assert torch.equal(a, b)
+
+
+def test_a_call_takes_the_forms_of_arrays_it_took_before():
+    """Lists, other types, strided arrays, one value for all, a matrix of one row: what plain arrays give.  Another
+    length or a matrix with a row per edge is refused."""
+    g = graph("t_nb2")
+    k = g.spec.n_degree
+    _, src, dst, ts, eidx = next(iter(batches(g, 1)))
+    neg = np.full(len(src), dst[0])
+    plan = np.arange(5, 50)
+    run = lambda *a, plan=plan: [t.cpu() for t in make_model(g).compute_edge_probabilities(*a, k, True, False, plan)]
+    want = run(src, dst, neg, ts, eidx)
+    for a in ((list(src), list(dst), list(neg), list(ts), list(eidx)),
+              (src.astype(np.int32), dst.astype(np.float64), neg, ts, np.repeat(eidx, 2)[::2]),
+              (torch.from_numpy(np.array(src)), dst, dst[:1], ts, eidx),
+              (src, dst, dst[0], ts, eidx),
+              (src, dst[None, :], neg, ts[None, :], eidx)):
+        assert all(torch.equal(x, y) for x, y in zip(run(*a, plan=list(plan)), want))
+    for a in ((src, dst[:-1], neg, ts, eidx), (src, dst, np.r_[neg, 1], ts, eidx), (src, dst, neg, ts[:0], eidx),
+              (src, dst, np.stack([neg, neg], 1), ts, eidx), (src, dst, neg, ts[:, None], eidx)):
+        with pytest.raises(ValueError):
+            run(*a)
