@@ -213,9 +213,9 @@ int orca_last_occurrence(const int32_t *d_ids, int32_t n_cap, const int32_t *d_n
  *                                                            516 used per head, stride ORCA_QT_LD)
  *   hid  = relu([ctx | h_src] . G + b1 + valid * g)         [*, 172]
  *   out  = LayerNorm(hid . W2t + b2) * ln_w + ln_b          [*, 172]
- * All matrices are row-major [in, out] float32.  The *_tc members hold the same matrices split into
- * a bf16 head and a bf16 tail and packed into the stage images of the tensor-core kernel
- * (orca_b200/weights.py: pack_tc).
+ * All matrices are row-major [in, out] float32.  The *_tc and *_img members hold the same matrices split into
+ * a bf16 head and a bf16 tail and packed into the stage images of the tensor-core kernels
+ * (orca_b200/weights.py: pack_tc, pack_query, pack_stages).
  */
 typedef struct {
   const float *Mq;   /* [172, 1056]  */
@@ -227,12 +227,13 @@ typedef struct {
   const float *b2;   /* [172]        */
   const float *ln_w; /* [172]        */
   const float *ln_b; /* [172]        */
-  const float *Mq_tc, *G_tc, *W2t_tc;
-  const float *Mq_img, *G_img, *W2_img;   /* operands of the batch entry points' kernels (rows as images) */
+  const float *G_tc, *W2t_tc;
+  const float *Mq_img, *G_img, *W2_img;   /* operands of the kernels that take their rows as images */
 } orca_attn_weights_t;
 
 /* Step 1 of TemporalAttentionLayer.forward (model/temporal_attention.py:41-48, the query side of
- * nn.MultiheadAttention): qt[r] = feat[idx ? idx[r] : r] . Mq + cq. */
+ * nn.MultiheadAttention): qt[r] = feat[idx ? idx[r] : r] . Mq + cq.  Takes 768 bytes a row of scratch memory from the
+ * context's pool, in stream order. */
 int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int32_t *d_idx,
                     int32_t n_rows_cap, const int32_t *d_n_rows, float *d_qt, void *stream);
 

@@ -30,7 +30,7 @@ c_i32p = C.c_void_p
 
 class AttnWeights(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b",
-                                          "Mq_tc", "G_tc", "W2t_tc", "Mq_img", "G_img", "W2_img")]
+                                          "G_tc", "W2t_tc", "Mq_img", "G_img", "W2_img")]
 
 
 class ScoreWeights(C.Structure):
@@ -197,7 +197,7 @@ def ptr(t):
     raise TypeError(type(t))
 
 
-ATTN_FIELDS = ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b", "Mq_tc", "G_tc", "W2t_tc", "Mq_img",
+ATTN_FIELDS = ("Mq", "cq", "G", "b1", "g", "W2t", "b2", "ln_w", "ln_b", "G_tc", "W2t_tc", "Mq_img",
                "G_img", "W2_img")
 
 

@@ -73,11 +73,9 @@ struct OutArgs {
 };
 // operand image of rows of a (two-part) table
 int feat_image(const tc::RowSrc &feat, int n_cap, const int32_t *d_n, char *d_image, cudaStream_t s);
-// qt = feat . Mq + cq, from the rows' image, or from the rows themselves
+// qt = feat . Mq + cq, from the rows' image
 int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_cap, const int32_t *d_n, float *d_qt,
                      cudaStream_t s);
-int attn_query_rows(const orca_attn_weights_t *w, const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_qt,
-                    cudaStream_t s);
 int attn_output_rows(const OutArgs &g, cudaStream_t s);
 
 }  // namespace orca

@@ -1,13 +1,12 @@
 // Query side of an attention layer on the tensor cores: qt[r] = feat[row of r] . Mq + cq, [rows, 1056] floats.
 //
 // A launch writes 4.2 KB per row and reads 0.7: at many rows it is bound by those writes.  A CTA keeps its weight
-// tile (heads and tails of 96 or 176 columns) for the whole launch and walks row blocks of 128.
-// attn_query_image_kernel takes the rows as an operand image (attn_out.cuh): one thread streams 16 KB stages through a
-// ring, one multiplies, eight warps carry the other accumulator buffer from tensor memory to qt, a thread per row and
-// 32 bytes a store (whole sectors, no staging).  51 k rows: 155 us for the general projection kernel (six column
-// tiles, weights streamed again for every row block, load, product and store one after the other), 75 here.
-// attn_query_kernel takes the rows as floats and splits them itself, eleven times over (170 us): it serves the callers
-// that have no buffer for an image.
+// tile (heads and tails of 176 columns) for the whole launch and walks row blocks of 128, which come as an operand image
+// (attn_out.cuh): one thread streams 16 KB stages through a ring, one multiplies, eight warps carry the accumulators from
+// tensor memory to qt, a thread per row and 32 bytes a store (whole sectors, no staging).  51 k rows: 145 us for the
+// general projection kernel (weights streamed again for every row block, load, product and store one after the other),
+// 75 here.  orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
+// for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
 #include <algorithm>
 
 #include "attn_out.cuh"
@@ -16,193 +15,10 @@
 #include "tc_ptx.cuh"
 
 namespace orca {
-namespace aq {
-
-constexpr int BM = 128, BN = 96, TILES = QT_LD / BN;     // 11
-constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;           // K = 172, padded to 176
-constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
-constexpr int A_LBO = BM * 16 + 16, A_BYTES = CHUNKS * A_LBO;   // (+16: conflict-free 16-byte stores)
-constexpr int TILE_LD = BN + 4;                          // floats per row of the output tile: likewise
-constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + BM * TILE_LD * 4 + 1024;
-constexpr int PRODUCERS = 256, THREADS = PRODUCERS + 128 + 32;
-constexpr int TMEM_COLS = 512, BUF_COLS = 2 * BN;        // two buffers of main + cross-term accumulators
-
-struct Args {
-  tc::RowSrc feat;
-  int n_cap;
-  const int32_t *d_n;
-  const void *w;          // weights.pack_query
-  const float *bias;
-  float *qt;
-  int32_t *status;
-  long long wait_limit;
-};
-
-__global__ void __launch_bounds__(THREADS, 1) attn_query_kernel(const __grid_constant__ Args g) {
-  using namespace tc;
-  extern __shared__ unsigned char raw[];
-  __shared__ int s_row[2][BM];
-  __shared__ __align__(16) float s_bias[BN];
-  __shared__ __align__(8) unsigned long long s_bar[8];
-  __shared__ uint32_t s_tmem;
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int nt = blockIdx.x;
-  const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u;
-  const uint32_t w_hi = base, w_lo = base + W_BYTES, a_hi = base + 2 * W_BYTES, a_lo = a_hi + A_BYTES,
-                 tile = a_lo + A_BYTES;
-  const uint32_t wbar = smem_addr(&s_bar[0]), afull = smem_addr(&s_bar[1]), aempty = smem_addr(&s_bar[2]);
-  auto accfull = [&](int b) { return smem_addr(&s_bar[3 + b]); };
-  auto accfree = [&](int b) { return smem_addr(&s_bar[5 + b]); };
-  dep_trigger();
-  if (tid == 0) {
-    mbar_init(wbar, 1);
-    mbar_init(afull, PRODUCERS / 32);
-    mbar_init(aempty, 1);
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(accfull(b), 1);
-      mbar_init(accfree(b), 4);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(wbar, 2 * W_BYTES);       // (weights: written by nobody but the host, long ago)
-    bulk_g2s(w_hi, reinterpret_cast<const char *>(g.w) + (size_t)nt * 2 * W_BYTES, 2 * W_BYTES, wbar);
-  }
-  if (warp == 12) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid < BN) s_bias[tid] = g.bias[nt * BN + tid];
-  dep_wait();
-  const int M = rows_of(g.n_cap, g.d_n);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
-  bool alive = true;
-
-  if (warp < 8) {
-    // ------------------------------------------------------------------ rows -> images
-    constexpr int PER = BM * CHUNKS / PRODUCERS;     // 11 chunks of 8 columns per thread and block
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 x[PER][2];
-    auto find_rows = [&](int blk, int buf) {
-      if (tid < BM) {
-        const int m = blk * BM + tid;
-        s_row[buf][tid] = m < M ? (g.feat.idx ? g.feat.idx[m] : m + g.feat.add) : -1;
-      }
-    };
-    auto load = [&](int buf) {
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int u = tid + i * PRODUCERS, row = u / CHUNKS, c = u - row * CHUNKS;
-        const int r = s_row[buf][row];
-        x[i][0] = x[i][1] = zero;
-        if (r >= 0) {
-          const float4 *p = reinterpret_cast<const float4 *>(g.feat.base(r) + (size_t)r * D) + 2 * c;
-          x[i][0] = *p;
-          if (c < CHUNKS - 1) x[i][1] = p[1];
-        }
-      }
-    };
-    int blk = blockIdx.y, t = 0;
-    if (blk * BM < M) find_rows(blk, 0);
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (blk * BM < M) load(0);
-    for (; blk * BM < M; blk += gridDim.y, ++t) {
-      const int next = blk + gridDim.y;
-      if (next * BM < M) find_rows(next, (t + 1) & 1);
-      if (t > 0) mbar_wait(aempty, (t - 1) & 1, g.status, 510, alive, g.wait_limit);
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int u = tid + i * PRODUCERS, row = u / CHUNKS, c = u - row * CHUNKS;
-        uint4 hi, lo;
-        split_chunk(x[i][0], x[i][1], hi, lo);
-        st_shared_v4(a_hi + c * A_LBO + row * 16, hi);
-        st_shared_v4(a_lo + c * A_LBO + row * 16, lo);
-      }
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(afull);
-      asm volatile("bar.sync 1, 256;" ::: "memory");     // the next block's rows are known
-      if (next * BM < M) load((t + 1) & 1);
-    }
-  } else if (warp < 12) {
-    // ------------------------------------------------------------------ accumulators -> qt
-    const int quarter = warp & 3;
-    const uint32_t rows_at = tile + (uint32_t)(quarter * 32) * (TILE_LD * 4);
-    int t = 0;
-    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
-      const int b = t & 1;
-      mbar_wait(accfull(b), (t >> 1) & 1, g.status, 520, alive, g.wait_limit);
-      tc_fence_after();
-      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * BUF_COLS;
-#pragma unroll
-      for (int ch = 0; ch < BN / 16; ++ch) {
-        float v[16];
-        tmem_ld16_sum(acc + ch * 16, BN, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 bias = *reinterpret_cast<const float4 *>(&s_bias[ch * 16 + q * 4]);
-          st_shared_f4(rows_at + (uint32_t)(lane * TILE_LD + ch * 16 + q * 4) * 4u,
-                       make_float4(v[q * 4] + bias.x, v[q * 4 + 1] + bias.y, v[q * 4 + 2] + bias.z, v[q * 4 + 3] + bias.w));
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(accfree(b));
-      const int m0 = blk * BM + quarter * 32;
-#pragma unroll 8
-      for (int i = 0; i < BN / 4; ++i) {      // the warp's 32 rows, 24 pieces each
-        const int u = lane + 32 * i, r = u / (BN / 4), c = u - r * (BN / 4);
-        const float4 v = ld_shared_f4(rows_at + (uint32_t)(r * TILE_LD + c * 4) * 4u);
-        if (m0 + r < M) *reinterpret_cast<float4 *>(g.qt + (size_t)(m0 + r) * QT_LD + nt * BN + c * 4) = v;
-      }
-      __syncwarp();
-    }
-  } else {
-    // ------------------------------------------------------------------ MMA issue
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-    mbar_wait(wbar, 0, g.status, 530, alive, g.wait_limit);
-    int t = 0;
-    for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
-      const int b = t & 1;
-      const uint32_t d = tmem + b * BUF_COLS;
-      if (t >= 2) mbar_wait(accfree(b), ((t >> 1) & 1) ^ 1, g.status, 531, alive, g.wait_limit);
-      mbar_wait(afull, t & 1, g.status, 532, alive, g.wait_limit);
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-      for (int ks = 0; ks < STEPS; ++ks) {
-        const uint64_t ah = make_desc(a_hi + ks * 2 * A_LBO, A_LBO, 128), al = make_desc(a_lo + ks * 2 * A_LBO, A_LBO, 128);
-        const uint64_t bh = make_desc(w_hi + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w_lo + ks * 2 * W_LBO, W_LBO, 128);
-        const uint32_t more = ks > 0 ? 1u : 0u;
-        mma_bf16(d, ah, bh, idesc, more);
-        mma_bf16(d + BN, al, bh, idesc, more);
-        mma_bf16(d + BN, ah, bl, idesc, 1u);
-      }
-      mma_commit(aempty);
-      mma_commit(accfull(b));
-      }
-      __syncwarp();
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 12) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-  }
-}
-
-}  // namespace aq
-
-// ---------------------------------------------------------------------------------------------------------------------
 namespace aqi {
 
-using aq::BM;
-using aq::CHUNKS;
-using aq::STEPS;
+constexpr int BM = 128;
+constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;                // K = 172, padded to 176
 constexpr int BN = 176, TILES = QT_LD / BN;                   // 6
 constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
 constexpr int STAGES = 5, STAGE = img::STAGE_BYTES;
@@ -222,12 +38,19 @@ struct Args {
   long long wait_limit;
 };
 
-__device__ __forceinline__ void st_global_v8(float *p, const float (&v)[8]) {
+template <bool WIDE>
+__device__ __forceinline__ void st_global_8(float *p, const float (&v)[8]) {
+  if (!WIDE) {     // (a result that is aligned to 16 bytes only)
+    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    return;
+  }
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
                "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                : "memory");
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __grid_constant__ Args g) {
   using namespace tc;
   extern __shared__ unsigned char raw[];
@@ -340,7 +163,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
             float y[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) y[i] = v[ch][8 * q + i] + s_bias[(c0 + ch) * 16 + 8 * q + i];
-            st_global_v8(out + ch * 16 + 8 * q, y);
+            st_global_8<WIDE>(out + ch * 16 + 8 * q, y);
           }
       }
     }
@@ -395,33 +218,17 @@ int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_ca
   if (n_cap <= 0) return ORCA_OK;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_query_image: no context for the current device");
-  ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && ((uintptr_t)d_qt & 31) == 0);
+  ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && ((uintptr_t)d_qt & 15) == 0);
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
+    for (auto kernel : {aqi::attn_query_image_kernel<true>, aqi::attn_query_image_kernel<false>})
+      ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
     configured_device = c->device;
   }
   const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, c->status_word, c->wait_limit};
   const dim3 grid(aqi::TILES, std::min(ceil_div(n_cap, aqi::BM), std::max(1, c->sm_count / aqi::TILES)));
-  ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
-  ORCA_COUNT_LAUNCH();
-  ORCA_LAUNCH_CHECK();
-  return ORCA_OK;
-}
-
-int attn_query_rows(const orca_attn_weights_t *w, const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_qt,
-                    cudaStream_t s) {
-  if (n_cap <= 0) return ORCA_OK;
-  Ctx *c = cur();
-  if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_query_rows: no context for the current device");
-  static thread_local int configured_device = -1;
-  if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(aq::attn_query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aq::SMEM));
-    configured_device = c->device;
-  }
-  const aq::Args g{feat, n_cap, d_n, w->Mq_tc, w->cq, d_qt, c->status_word, c->wait_limit};
-  const dim3 grid(aq::TILES, std::min(ceil_div(n_cap, aq::BM), std::max(1, c->sm_count / aq::TILES)));
-  ORCA_CUDA(launch_dep(aq::attn_query_kernel, grid, aq::THREADS, aq::SMEM, s, g));
+  auto kernel = ((uintptr_t)d_qt & 31) == 0 ? aqi::attn_query_image_kernel<true> : aqi::attn_query_image_kernel<false>;
+  ORCA_CUDA(launch_dep(kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

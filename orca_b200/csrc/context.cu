@@ -30,6 +30,26 @@ static int create_ctx(Ctx **out) {
   return ORCA_OK;
 }
 
+void *scratch_alloc(Ctx *c, size_t bytes, cudaStream_t s) {
+  static std::mutex mu;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (c->scratch == nullptr) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = c->device;
+      unsigned long long kept = 64ull << 20;
+      if (cudaMemPoolCreate(&c->scratch, &props) != cudaSuccess) c->scratch = nullptr;
+      else cudaMemPoolSetAttribute(c->scratch, cudaMemPoolAttrReleaseThreshold, &kept);
+    }
+  }
+  void *p = nullptr;
+  if (c->scratch != nullptr && cudaMallocFromPoolAsync(&p, bytes, c->scratch, s) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
 static void destroy_ctx(Ctx *c) {
   if (c == nullptr) return;
   int prev = -1;
@@ -55,6 +75,7 @@ static void destroy_ctx(Ctx *c) {
   if (c->lane1) cudaStreamDestroy(c->lane1);
   if (c->copy) cudaStreamDestroy(c->copy);
   if (c->d_words) cudaFree(c->d_words);
+  if (c->scratch) cudaMemPoolDestroy(c->scratch);
   if (prev >= 0) cudaSetDevice(prev);
   delete c;
 }

@@ -72,6 +72,7 @@ struct Ctx {
   cudaEvent_t ev_gcount[2] = {nullptr, nullptr};
   bool gdone_recorded[2] = {false, false};
   int32_t *d_words = nullptr;             // CTX_WORDS zeroed int32
+  cudaMemPool_t scratch = nullptr;        // made on first use (scratch_alloc)
   Tracer trace;
   GatherProfile prof;
 };
@@ -80,6 +81,9 @@ struct Ctx {
 // default context of the current device (created on first use; nullptr if that fails)
 Ctx *cur();
 Ctx *default_ctx();
+// device memory in the order of stream s for entry points whose callers bring no scratch, given back with cudaFreeAsync;
+// the context keeps up to 64 MB of it between calls.  nullptr: there is none to be had.
+void *scratch_alloc(Ctx *c, size_t bytes, cudaStream_t s);
 struct CtxScope {
   Ctx *prev;
   explicit CtxScope(Ctx *c);

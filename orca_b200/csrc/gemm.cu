@@ -487,8 +487,19 @@ int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int
   ORCA_CHECK_ARG(w && w->Mq && w->cq && d_feat && d_qt && n_rows_cap >= 0);
   if (n_rows_cap == 0) return ORCA_OK;
   if (projection_mode() == 0) {
-    ORCA_CHECK_ARG(w->Mq_tc != nullptr);
-    return attn_query_rows(w, tc::RowSrc{d_feat, d_idx, D, 0, 0}, n_rows_cap, d_n_rows, d_qt, (cudaStream_t)stream);
+    // the rows' operand image lies in scratch memory, 768 bytes a row beside the 4224 of the result
+    Ctx *c = cur();
+    if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_attn_query: no context for the current device");
+    ORCA_CHECK_ARG(w->Mq_img != nullptr);
+    cudaStream_t s = (cudaStream_t)stream;
+    void *image = scratch_alloc(c, img::bytes(n_rows_cap, img::FEAT_STAGES), s);
+    if (image != nullptr) {
+      int rc = feat_image(tc::RowSrc{d_feat, d_idx, D, 0, 0}, n_rows_cap, d_n_rows, (char *)image, s);
+      if (rc == ORCA_OK) rc = attn_query_image(w, (const char *)image, n_rows_cap, d_n_rows, d_qt, s);
+      ORCA_CUDA(cudaFreeAsync(image, s));
+      return rc;
+    }
+    // (no room for it: the fp32 tiles need none)
   }
   F1Args g{};
   g.a0 = RowSrc{d_feat, d_idx, D, 0, 0};

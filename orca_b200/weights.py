@@ -59,11 +59,11 @@ def pack_tc(W, bn=None):
                    lambda X: X.reshape(2, nkb, TC_BK // 8, 8, nt, bn).permute(4, 1, 0, 2, 5, 3))
 
 
-def pack_query(W, bn):
-    """Query weights [172, 1056] for csrc/attn_query.cu: K padded to 176, one image per bn columns, each
-    [head | tail][K / 8][bn columns][8]: uint16 [1056 / bn, 2, 22, bn, 8]."""
+def pack_query(W):
+    """Query weights [172, 1056] for csrc/attn_query.cu: K padded to 176, one image per 176 columns, each
+    [head | tail][K / 8][176 columns][8]: uint16 [6, 2, 22, 176, 8]."""
     return _packed(W, (GRU_PART, W.shape[1]),
-                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, bn).permute(3, 0, 1, 4, 2))
+                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, TC_BN).permute(3, 0, 1, 4, 2))
 
 
 def pack_stages(*parts):
@@ -90,9 +90,8 @@ def pack_gru(Wg, dim=D):
 def packed_attention(w):
     """The operand images that go with prepare_attention's matrices (numpy arrays or tensors)."""
     kd2 = w["G"].shape[0] - w["Mq"].shape[0]
-    return {"G_tc": pack_tc(w["G"]), "W2t_tc": pack_tc(w["W2t"]), "Mq_tc": pack_query(w["Mq"], 96),
-            "Mq_img": pack_query(w["Mq"], TC_BN), "G_img": pack_stages(w["G"][:kd2], w["G"][kd2:]),
-            "W2_img": pack_stages(w["W2t"])}
+    return {"G_tc": pack_tc(w["G"]), "W2t_tc": pack_tc(w["W2t"]), "Mq_img": pack_query(w["Mq"]),
+            "G_img": pack_stages(w["G"][:kd2], w["G"][kd2:]), "W2_img": pack_stages(w["W2t"])}
 
 
 def _f64(x):

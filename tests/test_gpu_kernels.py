@@ -265,6 +265,26 @@ def test_attention_layer(dev, k, n, layer):
             assert np.array_equal(pt[src_ids[r]], got[r])
 
 
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 // 6 + 1, 9000])
+def test_attention_query(dev, n):
+    """The stand-alone query projection against 64 bits, rows past the device-side count untouched, an output that is
+    aligned to 16 bytes only.  Operands carry 16 significant bits: relative error of a sum of 172 products below 1e-4
+    of the largest result (TOL_TC's argument)."""
+    from orca_b200 import _lib, weights
+    L = _lib.lib()
+    w = {kk: torch.from_numpy(v).to(dev) for kk, v in weights.prepare_attention(state_dict(2), 0).items()}
+    gen = torch.Generator(device=dev).manual_seed(n)
+    table = torch.randn(500, D, device=dev, generator=gen)
+    idx = torch.randint(0, 500, (n + 7,), device=dev, generator=gen, dtype=torch.int32)
+    count = torch.tensor([n], dtype=torch.int32, device=dev)
+    out = torch.full(((n + 7) * 1056 + 4,), 3.0, device=dev)[4:].view(n + 7, 1056)
+    _lib.check(L.orca_attn_query(_lib.attn_struct(w), table.data_ptr(), idx.data_ptr(), n + 7, count.data_ptr(),
+                                 out.data_ptr(), _lib.stream_ptr(dev)))
+    want = table.double()[idx[:n].long()] @ w["Mq"].double() + w["cq"].double()
+    assert float((out[:n] - want).abs().max() / want.abs().max()) < 1e-4
+    assert bool((out[n:] == 3.0).all())
+
+
 # ------------------------------------------------------------------------------- history
 def test_history_push_pull_flags(dev):
     from orca_b200.history import History
