@@ -399,9 +399,11 @@ static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d
   return attn_output_rows(a, s);
 }
 
-// Raw messages and GRU of a batch by the memory chain's kernel (chain.cu), or as a pair of launches (fp32 projections,
-// multi-GPU, and batches of more than 1024 edges: there the chain's kernel takes several turns on most of the chip while
-// the layers beside it want it; 2000 edges: 131 us a call with the pair, 141 with the chain)
+// Raw messages and GRU of a batch by the memory chain's kernel (chain.cu), or as a pair of launches.  The chain's kernel
+// is the faster one where a batch's launches stand in one line (eval_serial; one layer, us a call, pair / chain: 37 edges
+// 100.5 / 97.5, 200 115 / 102.6, 500 128 / 117, 800 125 / 123, 1024 129 / 130), not in the lanes of a budgeted batch,
+// where it takes most of the chip while the layers beside it want it (200 edges 84.3 / 85.0, 500 84.7 / 86.5, 800 94.8 /
+// 100.5, 1024 104.7 / 111.2, 2000 147 / 154).  The fp32 projections take the pair.
 static bool one_launch_updates(int b) { return projections_on_tensor_cores() && b <= 1024; }
 static UpdateList updates_of(const IdxBuf &x, const double *d_ts) {
   UpdateList u;
@@ -639,9 +641,8 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
       ORCA_TRY(launch_row_order(x.nbr1, R1, x.n1, x.order1, x.nbr1, N, nullptr, x.order2, k, si));
     ORCA_TRY(tr.mark(PH_SAMPLE_L1, s));
     // winners of the raw messages: last occurrence per node in [src|dst] (model/tgn_model.py:172-176)
-    const bool single = !sharded && one_launch_updates(b);
     ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, c->base_msg, x.win_pos, x.n_win,
-                                     d_status, si, updates_of(x, d_batch_ts)));
+                                     d_status, si));
     ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
     if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_idx[p], si));
     // cache flags of this batch (History.update_flag): read next by the next batch's head kernel
@@ -665,14 +666,10 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
       if (si != s) ORCA_CUDA(cudaStreamWaitEvent(sx, c->ev_idx[p], 0));
       else ORCA_TRY(link(s, sx, c->fork));
     }
-    if (!single)
-      ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
-                                  d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, sx));
+    ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
+                                d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, sx));
     ORCA_TRY(tr.mark(PH_MESSAGE, s));
-    if (single) {
-      ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid,
-                                      x.upd_t, x.cnt, w.upd_image, w.gru_h, sx));
-    } else if (gru_split && !in_a) {
+    if (gru_split && !in_a) {
       // (split by layer: the layer-1 ranks compute the memory update; this rank only receives the rows)
     } else if (gru_split) {
       // the memory update is split by node: this rank computes every wa-th unique positive and stores the
@@ -761,8 +758,7 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     // ------------------------------------------------------------------ side lane: the memory table is written
     if (!gru_split) {
       ORCA_TRY(wait_on(sx, sa, c->ev_o1));
-      if (!sharded && one_launch_updates(b)) ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, sx));
-      else ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, sx));
+      ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, sx));
       if (sx != s) {
         ORCA_CUDA(cudaEventRecord(c->ev_state, sx));
         c->state_recorded = true;
