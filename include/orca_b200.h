@@ -546,8 +546,8 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
  * One batch from host arrays (one GPU): orca_tgn_eval_batch with its inputs narrowed into a ring of ORCA_CALL_SLOTS
  * page-locked slots and copied from there on the context's copy stream.  Waits only when the ring is full.  The status
  * word follows the batch to h_status (page-locked) in `stream` order.
- * The entry points that are given a batch in host memory (this one, orca_tgn_eval_epoch, orca_tgn_eval_group) return
- * ORCA_E_BOUNDS, with no kernel of the batch enqueued, for a node or edge id outside its table.
+ * An id outside its table: this entry and orca_tgn_eval_epoch return ORCA_E_BOUNDS with nothing of the batch enqueued;
+ * the kernels of orca_tgn_eval_group read it as node or edge 0 and leave ORCA_E_BOUNDS in the status word.
  */
 #define ORCA_CALL_SLOTS 8
 typedef struct {

@@ -139,6 +139,10 @@ __global__ void __launch_bounds__(256) mark_kernel(const __grid_constant__ Args 
     const int i = i0 + (threadIdx.x & 31), n = min(i, n_pos - 1) / per, r = i - n * per, b = a.b_of(n);
     const int32_t *batch = a.img + a.off[n];
     const int v = i < n_pos ? batch[r] : -1;
+    // (node ids outside the table are reported by the sampling and are no updates; edge ids here)
+    const int eid = i < n_pos ? batch[3 * b + r % b] : 0;
+    const bool known = eid >= 0 && eid < a.n_edge_rows;
+    if (!known) report(a.status, ORCA_E_BOUNDS, eid);
     Entry *e = nullptr;
     if (v >= 0 && v < a.n_nodes) {
       e = a.table + find_entry(a.table, a.table_mask, v, n);
@@ -155,7 +159,7 @@ __global__ void __launch_bounds__(256) mark_kernel(const __grid_constant__ Args 
     const int at = n * per + w, other = r < b ? batch[b + r] : batch[r - b];
     a.win_node[at] = v;
     a.win_other[at] = other >= 0 && other < a.n_nodes ? other : 0;
-    a.win_eid[at] = batch[3 * b + r % b];
+    a.win_eid[at] = known ? eid : 0;
     a.win_t[at] = (float)a.ts[n * a.bs + r % b];
   }
 }
@@ -497,6 +501,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   a.indptr = m->indptr, a.adj_nbr = m->adj_nbr, a.adj_eid = m->adj_eid, a.adj_ts = m->adj_ts, a.n_nodes = m->n_nodes;
   a.nb = g->nb, a.bs = g->bs, a.b_last = g->b_last, a.k = k, a.mode = mode, a.layers = layers;
   a.u_cap1 = g->u_cap + 1;
+  a.n_edge_rows = m->n_edge_rows > 0 ? (int)std::min<int64_t>(m->n_edge_rows, INT_MAX) : INT_MAX;
   const int64_t base_i32 = g->off_i32[0];
   int64_t n_i32 = 0;
   for (int n = 0; n < g->nb; ++n) {
@@ -538,8 +543,6 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     if (c->gdone_recorded[p] && sc != s) ORCA_CUDA(cudaStreamWaitEvent(sc, c->ev_gdone[p], 0));
     ORCA_CUDA(cudaMemcpyAsync(x.stage, g->h_i32 + base_i32, (size_t)n_i32 * 4, cudaMemcpyHostToDevice, sc));
     ORCA_CUDA(cudaMemcpyAsync(x.stage + ts_off, g->h_ts, (size_t)E * 8, cudaMemcpyHostToDevice, sc));
-    for (int n = 0; n < g->nb; ++n)     // (while the copies are on the bus)
-      ORCA_TRY(check_batch_ids(m, g->h_i32 + base_i32 + a.off[n], a.b_of(n), n, "orca_tgn_eval_group"));
     if (si != sc) {     // (in order behind the copies: the parity's buffers are free, too)
       ORCA_CUDA(cudaEventRecord(c->ev_gin, sc));
       ORCA_CUDA(cudaStreamWaitEvent(si, c->ev_gin, 0));

@@ -39,6 +39,7 @@ struct Args {
   const int32_t *adj_nbr, *adj_eid;
   const double *adj_ts;
   int64_t n_nodes;
+  int n_edge_rows;
   const int32_t *img;               // [src | dst | neg | eidx | plan] of batch n at off[n]
   const double *ts;                 // times of batch n at n * bs
   int nb, bs, b_last, k, mode, layers;

@@ -522,8 +522,8 @@ def test_device_side_errors_of_a_stream_are_raised_by_its_own_call(planned):
 @pytest.mark.parametrize("layers", [1, 2])
 def test_an_id_outside_its_table_is_refused(layers):
     """A node or edge id that the tables have no row for, in each array of a batch, first and last entry, is an error of
-    the call (the kernels read the rows of a batch's ids unchecked), and the model goes on as if the batch had never
-    been there."""
+    the call.  A batch of a single call has never been there (its kernels would read the rows of its ids unchecked); the
+    kernels of a group guard theirs."""
     import dataclasses
     from orca_b200 import _lib
     g = graph("t_nb2")
