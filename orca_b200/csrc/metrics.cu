@@ -26,14 +26,20 @@ static inline uint32_t falling_key(float x) {
   return (u >> 31) ? u : ~(u | 0x80000000u);
 }
 
-static void sort_keys(std::vector<uint32_t> &v, std::vector<uint32_t> &tmp) {
+struct Scratch {
+  std::vector<uint32_t> pos, neg, tmp;
+  uint32_t count[3][2048];
+};
+
+static void sort_keys(std::vector<uint32_t> &v, Scratch &s) {
+  std::vector<uint32_t> &tmp = s.tmp;
+  uint32_t (&count)[3][2048] = s.count;
   const size_t n = v.size();
   if (n < 128) {   // (three passes over 2048 counters cost more than the comparisons)
     std::sort(v.begin(), v.end());
     return;
   }
   tmp.resize(n);
-  static thread_local uint32_t count[3][2048];
   memset(count, 0, sizeof(count));
   for (uint32_t k : v) ++count[0][k & 2047], ++count[1][(k >> 11) & 2047], ++count[2][k >> 22];
   for (int p = 0; p < 3; ++p) {
@@ -49,10 +55,6 @@ static void sort_keys(std::vector<uint32_t> &v, std::vector<uint32_t> &tmp) {
   }
 }
 
-struct Scratch {
-  std::vector<uint32_t> pos, neg, tmp;
-};
-
 // false: a score is not finite
 static bool one_batch(const float *pos, const float *neg, int64_t n, double *out, Scratch &s) {
   s.pos.resize(n);
@@ -66,8 +68,8 @@ static bool one_batch(const float *pos, const float *neg, int64_t n, double *out
     s.neg[i] = falling_key(neg[i]);
   }
   if (!finite) return false;
-  sort_keys(s.pos, s.tmp);
-  sort_keys(s.neg, s.tmp);
+  sort_keys(s.pos, s);
+  sort_keys(s.neg, s);
   double ap = 0, twice_area = 0;   // (counts are whole numbers: the area is exact up to 2^53)
   int64_t tp = 0, fp = 0;
   while (tp < n || fp < n) {
