@@ -582,6 +582,7 @@ typedef struct {
   int32_t phase;              /* 1, 2 or 3 (both) */
   int32_t nb, bs, b_last;     /* batches of this group; edges of a batch and of the group's last one */
   int32_t nb_max, u_cap, plan_cap; /* most batches of a group, most uncached neighbours and plan entries of a batch */
+  int32_t *h_status;          /* page-locked, may be NULL: four words, the status word as phase 2 leaves it */
 } orca_group_t;
 /* batches worth putting into one group */
 int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode);

@@ -90,7 +90,8 @@ class CallT(C.Structure):
 
 class GroupT(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("h_i32", "h_ts", "off_i32", "n_plan", "h_rows")] + [("seq", C.c_int64)] + \
-        [(n, C.c_int32) for n in ("phase", "nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap")]
+        [(n, C.c_int32) for n in ("phase", "nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap")] + \
+        [("h_status", C.c_void_p)]
 
 
 # every symbol the header declares: name -> (restype, argtypes)

@@ -297,9 +297,12 @@ __device__ __forceinline__ void copy_row(float *dst, const float *src, int t) {
   if (t < D / 4) reinterpret_cast<float4 *>(dst)[t] = reinterpret_cast<const float4 *>(src)[t];
 }
 __global__ void __launch_bounds__(256)
-write_back_kernel(const __grid_constant__ Args a, const float *log, const float *emb1, float *memory, float *history) {
+write_back_kernel(const __grid_constant__ Args a, const float *log, const float *emb1, float *memory, float *history,
+                  int32_t *h_status) {
   dep_trigger();
   dep_wait();
+  // the last kernel of the group: what the others have reported goes straight to the host
+  if (h_status != nullptr && blockIdx.x == 0 && threadIdx.x < 4) h_status[threadIdx.x] = __ldcg(a.status + threadIdx.x);
   const int t = threadIdx.x & 63;
   const int n_upd = a.nb * 2 * a.bs, batch_rows = 3 * a.edges();
   const int n_items = n_upd + (a.keeps_history() ? a.cnt->n_rows : 0);
@@ -604,7 +607,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     // (positions of a short last batch's scores: the arrays are indexed by 2 * bs per batch, only the last is short)
     ORCA_TRY(score_rows(&m->score, top, x.score0, x.score1, 2 * E, d_prob, s));
     ORCA_CUDA(launch_dep(grp::write_back_kernel, c->sm_count * 8, 256, 0, s, a, log, (const float *)w.emb1, m->mem.memory,
-                         m->hist_emb));
+                         m->hist_emb, g->h_status));
     ORCA_COUNT_LAUNCH();
     if (h_prob != nullptr) ORCA_CUDA(cudaMemcpyAsync(h_prob, d_prob, (size_t)2 * E * 4, cudaMemcpyDeviceToHost, s));
     ORCA_CUDA(cudaEventRecord(c->ev_gdone[p], s));

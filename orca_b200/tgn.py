@@ -663,9 +663,8 @@ class TGN(nn.Module):
         return self._status_host
 
     def _finish_epoch(self, stream):
-        """Waits for a stream of batches whose scores are on their way to the host and brings the status word along.
+        """Waits for a stream of batches whose scores and status word (to _status_buffer) are on their way to the host.
         Returns the error to raise, or None: a whole-stream call has no later call to report through."""
-        self._status_buffer().copy_(self._status, non_blocking=True)      # (`stream` is the current stream)
         stream.synchronize()
         v = self._status_host.numpy()
         code, detail = int(v[0]), int(v[3])
@@ -879,6 +878,7 @@ class TGN(nn.Module):
             _lib.check(L.orca_tgn_eval_epoch(desc, C.byref(ep), u_cap, ws.data_ptr(), ws.numel(),
                                              dev["stage"].data_ptr(), dev["stage"].numel(), dev["prob"].data_ptr(),
                                              h_prob.data_ptr(), self._status.data_ptr(), stream.cuda_stream))
+        self._status_buffer().copy_(self._status, non_blocking=True)      # (`stream` is the current stream)
         failed = self._finish_epoch(stream)
         if failed is not None and world == 1:
             raise failed
@@ -959,7 +959,7 @@ class TGN(nn.Module):
         hi, hts, d_prob = h_i32.numpy(), h_ts.numpy(), keep["d_prob"]
         desc = self._descriptor(k)
         stream = torch.cuda.current_stream(self.device)
-        h_rows = pinned("rows", 2, torch.int32)
+        h_rows, h_status = pinned("rows", 2, torch.int32), self._status_buffer().data_ptr()
         groups = []
 
         def prepare(i0):
@@ -976,7 +976,7 @@ class TGN(nn.Module):
                 if n_plan[i]:
                     hi[o + 4 * n:off[i + 1]] = cache_plan[i]
             g = _lib.GroupT(h_i32.data_ptr(), h_ts.data_ptr() + 8 * lo, off.ctypes.data + 8 * i0, n_plan.ctypes.data + 4 * i0,
-                            h_rows.data_ptr(), len(groups), 1, i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap)
+                            h_rows.data_ptr(), len(groups), 1, i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap, h_status)
             groups.append((g, lo))
             enqueue(g, lo)
 
