@@ -22,11 +22,13 @@ namespace orca {
 // two-wide fp32 instructions of this architecture while the loads are in flight -- then come the partial dot products
 // with the two query heads, one cross-lane sum of all four logits at once, a running softmax and the weighted sums, all
 // from the same registers.
-// What bounds it (51 k rows of ten slots, 163 us): the instructions of a row (1500 a warp, 600 of them the time
-// encodings) against 16 resident warps per SM; issue slots 45 % busy, DRAM 30 %, L2 20 %.  Measured against it: two
-// passes over the rows with parked logits and time encodings (the form before) 178 us; four slots a step at 12 warps
-// 186; slots copied ahead with cp.async, two or four at a time, 167 to 201; the long cosine inlined with a variant of
-// the loop per range, 360 (instruction cache).  The 688-byte rows are not moved by cp.async.bulk: an SM retires only
+// What bounds it (48 k rows of ten slots, 165 us; under the profiler 169): the instructions of a row (1800 a warp, a
+// third of them the time encodings) against 16 resident warps per SM: issue slots 49 % busy, a warp issues every 8
+// cycles (3 of them for loads), DRAM 29 %, L2 25 %, L1 50 %.  Measured against it: two passes over the rows with parked
+// logits and time encodings (the form before) 178 us; four slots a step at 12 warps 186; slots copied ahead with
+// cp.async, two or four at a time, 167 to 201; the long cosine inlined with a variant of the loop per range, 360
+// (instruction cache).  A launch of a single batch is no faster than the two passes were (6000 rows 29.2 us, before
+// 28.9): there the two or three rows of each warp, one after the other, are what it takes.  The 688-byte rows are not moved by cp.async.bulk: an SM retires only
 // about one small bulk copy per ~130 cycles.
 //
 // Work distribution.  Rows differ tenfold in cost (0 to k valid slots) and a launch of a single batch holds only two

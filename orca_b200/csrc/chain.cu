@@ -5,7 +5,8 @@
 // a pipeline filled and drained, two launches) whatever the batch size, and it is the only part of a group that is
 // serial: with small batches it is what a stream waits for.  What a batch really waits for is its memory rows.  So
 // one cooperative grid walks the batches:
-//   - 22 column tiles of 32 gate columns (eight units) times up to six row blocks of 64 updates, one CTA each.  A CTA
+//   - 22 column tiles of 32 gate columns (eight units) times row blocks of 64 updates, one CTA each: up to six for a
+//     single batch, five for a group, whose layers run beside it (launch).  A CTA
 //     keeps its weight columns (880 x 32, bf16 head and tail, 113 KB) in shared memory for the whole launch.
 //   - K is laid out so that what does not depend on the batch before comes first: edge features and time encoding
 //     (352 columns).  A launch of its own splits them for all updates of the group (computed in the chain, the cosines

@@ -341,7 +341,10 @@ static inline uint32_t pow2_at_least(uint64_t x) {
 }
 
 // Batches per group: enough rows for several tiles of every projection kernel on every SM (48 k rows = 2.6 row
-// blocks of 128 per SM), at most a bit each.
+// blocks of 128 per SM), at most a bit each.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without reuse,
+// by rows of a group: 12 k 3.67 / 3.76 / 8.03 / 5.29, 24 k 3.19 / 3.34 / 7.00 / 3.07, 36 k 3.12 / 3.11 / 6.53 / 2.59, 48 k
+// 3.05 / 3.08 / 6.47 / 2.36, 64 k 3.11 / 3.13 / 6.43 / 2.25, 96 k 3.11 / 3.12 / 6.38 / 2.08: up to 48 k every stream
+// gains, beyond it some lose 2 % (a short stream has too few groups to overlap) and the workspace keeps growing.
 static int group_size(int bs, int k, int layers, int mode) {
   const int64_t rows = 3ll * bs * (layers == 2 && mode == ORCA_MODE_NO_REUSE ? 1 + k : 1);
   return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, 49152 / rows));

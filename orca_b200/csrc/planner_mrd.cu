@@ -20,7 +20,7 @@
 // in tie_order.cuh: block-wide in the one-CTA kernel.  In the cluster kernel the CTAs take
 // whole ranges each, in shared memory (tie_shared.cuh); for lists that do not fit, every step is spread over the
 // cluster.  200 batches of 2000 edges with 10,500 candidates: 43.5 ms a plan with all steps spread (a level then costs
-// five cluster barriers with trips to L2 between them, 10 us), 24 here.
+// five cluster barriers with trips to L2 between them, 10 us), 25.5 to 27 here.
 #include <algorithm>
 
 #include "common.cuh"

@@ -12,7 +12,7 @@
 // tie_order.cuh for lists that do not fit shared memory).
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
 // 250 batches of 600 edges with 20 neighbours, LRU: 19.2 ms a plan with draws, swaps, bitmaps and sort
-// in global memory, 12.1 here.
+// in global memory, 12.1 to 12.4 here.
 #include <algorithm>
 
 #include "common.cuh"
