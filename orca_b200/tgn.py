@@ -792,6 +792,7 @@ class TGN(nn.Module):
     def _eval_chunks(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan):
         """eval_epoch batch after batch (orca_tgn_eval_epoch)."""
         L = _lib.lib()
+        _lib.settle(self.device)      # (the first batch's lanes do not wait for the caller's stream)
         E = len(sources)
         nb = (E + bs - 1) // bs
         world, rank = self._world, self._rank

@@ -667,6 +667,18 @@ def test_a_batch_sees_what_was_written_on_the_callers_stream():
            o.memory.get_last_update(ids), o.embedding_module.histories[0].pull(ids))
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(late, now))
+    # a table that the caller reads itself, before a whole stream
+    E = spec.bs
+    for p in (plan[3:4], None):
+        m = make_model(g)
+        for x in bat[:2]:
+            m.compute_edge_probabilities(*x)
+        torch.cuda.synchronize()
+        before = m.memory.memory.cpu()
+        late = _after_a_long_kernel(lambda: m.memory.memory.clone())
+        m.eval_epoch(g.sources[3 * E:4 * E], g.destinations[3 * E:4 * E], bat[3][2], g.timestamps[3 * E:4 * E],
+                     g.edge_idxs[3 * E:4 * E], k, E, p)
+        assert torch.equal(late.cpu(), before)
 
 
 def test_a_model_made_in_inference_mode_scores():
