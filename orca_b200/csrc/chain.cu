@@ -39,6 +39,7 @@ constexpr int A_CHUNKS = 2 * PART_CHUNKS, A_LBO = ROWS * 16 + 16, A_BYTES = A_CH
 constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 1024;
 constexpr int EPI_WARPS = 4, PRODUCERS = 256, THREADS = 32 * EPI_WARPS + PRODUCERS + 32;
 constexpr int TMEM_COLS = 128, BUF_COLS = 64, SMALL = 32;   // two accumulator buffers of main + cross terms
+constexpr int GROUP_ROWS = 32;                 // updates a row block takes before there is another one (16 to 64: the same)
 constexpr int META = 4;                        // steps whose memory rows are kept
 constexpr int PER = 6;                         // chunks a producer thread has in flight: 34 rows at a time
 
@@ -92,14 +93,12 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
   __shared__ uint32_t s_tmem;
   const Args &a = g.a;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int ct = blockIdx.x, rb = blockIdx.y, n_rb = gridDim.y, n_cta = gridDim.x * gridDim.y;
+  const int ct = blockIdx.x, rb = blockIdx.y;
   const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u;
   const uint32_t w_hi = base, w_lo = base + W_BYTES, a_hi = base + 2 * W_BYTES, a_lo = a_hi + A_BYTES;
   const uint32_t wbar = smem_addr(&s_bar[0]), ebar = smem_addr(&s_bar[1]), mbar = smem_addr(&s_bar[2]),
                  edone = smem_addr(&s_bar[3]), accbar = smem_addr(&s_bar[4]);
   auto tfree = [&](int b) { return smem_addr(&s_bar[5 + b]); };
-  // rows of a row block in a batch: the updates spread over the blocks, in steps of eight, at most a tile's
-  auto rows_per = [&](int win) { return min(ROWS, ((win + n_rb - 1) / n_rb + 7) & ~7); };
   if (tid == 0) {
     mbar_init(wbar, 1);
     mbar_init(ebar, PRODUCERS / 32);
@@ -125,6 +124,14 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
   bool alive = true;
+  // row blocks of a group whose last updates are done elsewhere: as many as the batch with the most updates asks for; the
+  // others have nothing to do
+  int most = 0;
+  for (int n = 0; n < a.nb; ++n) most = max(most, s_win[n]);
+  const int n_rb = a.split ? max(1, min((int)gridDim.y, (most + GROUP_ROWS - 1) / GROUP_ROWS)) : (int)gridDim.y;
+  const int n_cta = gridDim.x * n_rb, nb = rb < n_rb ? a.nb : 0;
+  // rows of a row block in a batch: the updates spread over the blocks, in steps of eight, at most a tile's
+  auto rows_per = [&](int win) { return min(ROWS, ((win + n_rb - 1) / n_rb + 7) & ~7); };
   auto mem_row = [&](int r) { return (r >= a.n_nodes ? g.log : g.mem.memory) + (size_t)r * D; };
 
   int s = 0;    // steps of this CTA so far: the rows of one turn of one batch each
@@ -132,7 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
     // ------------------------------------------------------------------ gates
     const int row = warp * 16 + (lane & 15), hi = lane >> 4;     // this lane: units 4 * hi .. 4 * hi + 3 of the row
     const int u0 = ct * UNITS + 4 * hi;
-    for (int n = 0; n < a.nb; ++n) {
+    for (int n = 0; n < nb; ++n) {
       const int rows = rows_per(s_win[n]);
       for (int r0 = rb * rows; r0 < s_win[n]; r0 += n_rb * rows, ++s) {
         const bool live = row < rows && r0 + row < s_win[n] && u0 < D;      // (the last tile has four units)
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
       st_shared_v4(a_hi + chunk * A_LBO + row * 16, hi);
       st_shared_v4(a_lo + chunk * A_LBO + row * 16, lo);
     };
-    for (int n = 0; n < a.nb; ++n) {
+    for (int n = 0; n < nb; ++n) {
       bool met = n == 0;
       const int full_rows = rows_per(s_win[n]);
       for (int r0 = rb * full_rows; r0 < s_win[n]; r0 += n_rb * full_rows, ++s) {
@@ -256,7 +263,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
     // ------------------------------------------------------------------ MMA issue
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COLS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
     mbar_wait(wbar, 0, g.status, 630, alive, g.wait_limit);
-    for (int n = 0; n < a.nb; ++n) {
+    for (int n = 0; n < nb; ++n) {
       const int rows = rows_per(s_win[n]);
       for (int r0 = rb * rows; r0 < s_win[n]; r0 += n_rb * rows, ++s) {
         const uint32_t d = tmem + (s & 1) * BUF_COLS;
@@ -302,11 +309,10 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
   dep_trigger();
   dep_wait();
   const int part = threadIdx.x / 64, lane = threadIdx.x % 64;
-  for (int i = blockIdx.x; i < a.nb * 2 * a.bs; i += gridDim.x) {
-    const int n = i / (2 * a.bs), w = i - n * 2 * a.bs;
-    if (w >= a.cnt->n_win[n]) continue;
+  const int n = a.last_at != nullptr ? a.cnt->n_last : a.cnt->n_win[0];
+  for (int l = blockIdx.x; l < n; l += gridDim.x) {
+    const int i = a.last_at != nullptr ? a.last_at[l] : l;
     const int node = a.win_node[i];
-    if (a.nb > 1 && (unsigned long long)a.bits[node].positive >> (n + 1)) continue;
     const float gap = a.win_gap != nullptr ? a.win_gap[i] : a.win_t[i] - g.mem.last_update[node];
     float *dst = g.mem.messages + (size_t)node * MSG + part * D;
     auto row = [&](int r) { return (r >= a.n_nodes ? g.log : g.mem.memory) + (size_t)r * D; };

@@ -13,8 +13,9 @@
 //   index stream   neighbour tables of all batch rows; bit sets per node (cached / in batch / positive / recomputed,
 //                  one bit per batch) and a (node, batch) hash table; recomputed rows; resolution of the ids; the
 //                  cache flags of the group's last plan
-//   chain stream   raw messages and GRU of batch 0, 1, ... into the log.  Runs a group ahead of the main stream:
-//                  rows of the group before are read from that group's log
+//   chain stream   raw messages and GRU of batch 0, 1, ... into the log, of large groups only those that a later batch
+//                  reads; the others behind it, at once.  Runs a group ahead of the main stream: rows of the group
+//                  before are read from that group's log
 //   main stream    layer 1, layer 2, scores of all batches; then the last version of every rewritten row goes to
 //                  the memory and history tables
 // Buffers of the index and chain streams exist twice (group parity).
@@ -148,13 +149,15 @@ __global__ void __launch_bounds__(256) mark_kernel(const __grid_constant__ Args 
       e = a.table + find_entry(a.table, a.table_mask, v, n);
       if (e->pos != r + 1) e = nullptr;
     }
+    const bool back = e != nullptr && a.split && !a.again(v, n);
     __syncwarp();
-    const unsigned group = __match_any_sync(0xffffffffu, e != nullptr ? n : -1);
+    const unsigned group = __match_any_sync(0xffffffffu, e != nullptr ? 2 * n + (back ? 1 : 0) : -1);
     const int leader = __ffs(group) - 1, lane = threadIdx.x & 31;
     int w = 0;
-    if (e != nullptr && lane == leader) w = atomicAdd(&a.cnt->n_win[n], __popc(group));
+    if (e != nullptr && lane == leader) w = atomicAdd(back ? &a.cnt->n_back[n] : &a.cnt->n_win[n], __popc(group));
     w = __shfl_sync(0xffffffffu, w, leader) + __popc(group & ((1u << lane) - 1u));
     if (e == nullptr) continue;
+    if (back) w = per - 1 - w;
     e->pos = IN_LOG | w;     // (no other position of the node equals it)
     const int at = n * per + w, other = r < b ? batch[b + r] : batch[r - b];
     a.win_node[at] = v;
@@ -205,10 +208,10 @@ __global__ void __launch_bounds__(1024) count_kernel(const __grid_constant__ Arg
     const int rows = batch_rows + sum;
     a.cnt->n_rows = rows;
     if (a.status != nullptr) {     // counts of the last batch (status word layout, common.cuh)
-      const int last = 3 * a.b_last;
-      a.status[1] = a.budget() ? last + max(0, s_cand[a.nb - 1] - 1)
-                    : a.layers == 2 && a.mode == ORCA_MODE_NO_REUSE ? last * (1 + a.k) : last;
-      a.status[2] = a.cnt->n_win[a.nb - 1];
+      const int rows_last = 3 * a.b_last;
+      a.status[1] = a.budget() ? rows_last + max(0, s_cand[a.nb - 1] - 1)
+                    : a.layers == 2 && a.mode == ORCA_MODE_NO_REUSE ? rows_last * (1 + a.k) : rows_last;
+      a.status[2] = a.cnt->n_win[a.nb - 1] + a.cnt->n_back[a.nb - 1];
     }
   }
 }
@@ -279,8 +282,13 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
   const int per = 2 * a.bs;
   for (int i = tid; i < a.nb * per; i += step) {
     const int n = i / per, r = i - n * per, b = a.b_of(n);
-    if (r < a.cnt->n_win[n]) {
+    if (a.is_update(n, r)) {
       const int v = a.win_node[i], row = memory_row_early(a, v, n);
+      if (!a.again(v, n)) {
+        const int l = place(&a.cnt->n_last, 0);
+        a.last_at[l] = i;
+        a.last_node[l] = v;
+      }
       a.win_mem[i] = row;
       a.win_gap[i] = a.win_t[i] - last_update_of(a, last_update, v, row);
       a.win_other[i] = memory_row_early(a, a.win_other[i], n);
@@ -304,15 +312,11 @@ write_back_kernel(const __grid_constant__ Args a, const float *log, const float 
   // the last kernel of the group: what the others have reported goes straight to the host
   if (h_status != nullptr && blockIdx.x == 0 && threadIdx.x < 4) h_status[threadIdx.x] = __ldcg(a.status + threadIdx.x);
   const int t = threadIdx.x & 63;
-  const int n_upd = a.nb * 2 * a.bs, batch_rows = 3 * a.edges();
+  const int n_upd = a.cnt->n_last, batch_rows = 3 * a.edges();
   const int n_items = n_upd + (a.keeps_history() ? a.cnt->n_rows : 0);
   for (int i = blockIdx.x * 4 + threadIdx.x / 64; i < n_items; i += gridDim.x * 4) {
     if (i < n_upd) {
-      const int n = i / (2 * a.bs), w = i - n * 2 * a.bs;
-      if (w >= a.cnt->n_win[n]) continue;
-      const int v = a.win_node[i];
-      if ((unsigned long long)a.bits[v].positive >> (n + 1)) continue;      // a later batch rewrites it
-      copy_row(memory + (size_t)v * D, log + (size_t)(a.log_base + i) * D, t);
+      copy_row(memory + (size_t)a.last_node[i] * D, log + (size_t)(a.log_base + a.last_at[i]) * D, t);
       continue;
     }
     const int row = i - n_upd;
@@ -350,6 +354,14 @@ static int group_size(int bs, int k, int layers, int mode) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, 49152 / rows));
 }
 
+// The memory chain is serial, so only what a later batch of the group reads belongs there: in a group of 2000-edge
+// batches on the largest graph 125 of a batch's 890 updates.  The others, every node's last update in the group, wait for
+// nobody, and one launch of the general projection does them behind the chain (chain 208 -> 74 us a group on half of the
+// SMs).  That launch and the message rows it reads are 25 us of latency, which a group with few updates does not win
+// back: streams of 27 x 600 / 16 x 1000 / 8 x 2000 edges a group 3.08 / 3.08 / 6.46 ms without, 3.04 / 3.03 / 5.79 with;
+// 7 x 200 (no reuse) / 32 x 200 2.36 / 2.14 without, 2.38 / 2.13 with.
+constexpr int SPLIT_FROM = 16384;      // positions [src | dst] of a group
+
 // Index buffers (two of each) and main-stream buffers.  The layer-1 rows that exist at all are few more than the
 // batches' own, but a batch with a cold cache can recompute every sampled neighbour: the projected queries and
 // attention sums (9 KB a row) are sized for `chunk` rows, and layer 1 runs over as many chunks as there are: the
@@ -364,6 +376,7 @@ struct Parity {
   float *dt1;
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;
+  int32_t *last_at, *last_node;
   char *stage;
   void *upd_image;         // split inputs of the memory updates (chain.cu)
 };
@@ -414,6 +427,8 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.win_other = (int32_t *)take((size_t)2 * E * 4);
     x.win_t = (float *)take((size_t)2 * E * 4);
     x.win_gap = (float *)take((size_t)2 * E * 4);
+    x.last_at = (int32_t *)take((size_t)2 * E * 4);
+    x.last_node = (int32_t *)take((size_t)2 * E * 4);
     x.stage = (char *)take(w.stage_bytes);
     x.upd_image = take(update_image_bytes(2 * E));
   }
@@ -528,6 +543,8 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   a.cand = x.cand, a.app_node = x.app_node, a.nbr1 = x.nbr1, a.eid1 = x.eid1, a.dt1 = x.dt1, a.nbr2 = x.nbr2;
   a.own1 = x.own1, a.score0 = x.score0, a.score1 = x.score1;
   a.win_node = x.win_node, a.win_eid = x.win_eid, a.win_mem = x.win_mem, a.win_other = x.win_other, a.win_t = x.win_t, a.win_gap = x.win_gap;
+  a.last_at = x.last_at, a.last_node = x.last_node;
+  a.split = 2 * E > grp::SPLIT_FROM;
   a.prev_win_t = prev.win_t;
   a.log_base = (int)m->n_nodes + p * 2 * E_max, a.prev_log_base = (int)m->n_nodes + (p ^ 1) * 2 * E_max;
   // second parts of the two-part tables, moved back by the first part's rows
@@ -567,6 +584,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     grp::ChainArgs ch{a, m->mem, log, w.log + (size_t)p * 2 * E_max * D, m->edge_table, m->time_w, m->gru.Wg_chain, m->gru.bg,
                       x.upd_image, nullptr, 0};
     ORCA_TRY(grp::launch_gru_chain(ch, sx));
+    if (a.split) ORCA_TRY(gru_rows(&m->gru, m->mem, x.last_node, x.last_at, 2 * g->nb * g->bs, &x.cnt->n_last, ch.log_out, sx));
     if (sx != s) ORCA_CUDA(cudaEventRecord(c->ev_gchain[p], sx));
     return ORCA_OK;
   };

@@ -25,7 +25,11 @@ struct Entry {
 constexpr int32_t IN_LOG = 1 << 30;
 
 struct Counters {
-  int32_t n_cand[MAX_BATCHES], n_win[MAX_BATCHES], low_cand[MAX_BATCHES] /* INT_MAX - smallest candidate */;
+  int32_t n_cand[MAX_BATCHES], low_cand[MAX_BATCHES] /* INT_MAX - smallest candidate */;
+  // Memory updates of the batch: the memory chain's lie at the front of the batch's places, those that are left to one
+  // launch behind the chain (Args::split) at the back.
+  int32_t n_win[MAX_BATCHES], n_back[MAX_BATCHES];
+  int32_t n_last;                          // entries of last_at
   int32_t dropped[MAX_BATCHES];            // smallest candidate of the batch (-1: none): it is not recomputed
   int32_t app_off[MAX_BATCHES + 1];        // first recomputed row of the batch, counted from the group's first
   int32_t n_rows;                          // layer-1 rows of the group
@@ -64,15 +68,21 @@ struct Args {
   int32_t *nbr2;                    // batch rows: rows of (history table | layer-1 output)
   int32_t *own1;                    // row of (memory table | log) of the row's own node
   int32_t *score0, *score1;         // the two embeddings of every score
-  // memory updates: batch n's at n * 2 * bs
+  // memory updates: batch n's at n * 2 * bs (Counters says which of these places are taken)
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;           // time of the update, and since the node's update before it
+  int32_t *last_at, *last_node;     // the last update of every node that the group updates: place, node
+  int split;                        // whether last updates are left out of the memory chain (group.cu)
   const float *prev_win_t;
   int log_base, prev_log_base;      // row of (memory table | log) where this / the previous group's log starts
 
   __host__ __device__ int b_of(int n) const { return n == nb - 1 ? b_last : bs; }
   __host__ __device__ int edges() const { return (nb - 1) * bs + b_last; }
   __device__ bool budget() const { return layers == 2 && mode == ORCA_MODE_BUDGET; }
+  // whether place w of batch n holds an update
+  __device__ bool is_update(int n, int w) const { return w < cnt->n_win[n] || w >= 2 * bs - cnt->n_back[n]; }
+  // whether a later batch of the group updates node v (and reads what batch n's update leaves)
+  __device__ bool again(int v, int n) const { return (unsigned long long)__ldcg(&bits[v].positive) >> (n + 1) != 0; }
   __device__ bool keeps_history() const { return layers == 2 && mode != ORCA_MODE_NO_REUSE; }
 };
 

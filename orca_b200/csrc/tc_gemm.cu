@@ -112,7 +112,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       b[k] = has1 ? add4(ld_shared_f4(ra + 512u), bB) : f4z;
       hA[k] = hB[k] = 0.f;
       if (EPI == EPI_GRU && ok[k]) {
-        const float *hrow = g.memory + (size_t)mb[k] * D;
+        const float *hrow = g.memory + (size_t)mb[k] * g.memory_ld;
         if (uA < D) hA[k] = hrow[uA];
         if (has1 && uB < D) hB[k] = hrow[uB];
       }
@@ -159,7 +159,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       for (int k = 0; k < RB; ++k)
         if (ok[k]) {
           // (row of the whole list; with the multi-GPU split the row also goes to every rank's buffer)
-          const size_t orow = (size_t)(g.row_stride > 1 ? m[k] * g.row_stride + g.row_off : m[k]) * D;
+          const size_t orow = (size_t)(g.out_rows != nullptr ? ma[k] : g.row_stride > 1 ? m[k] * g.row_stride + g.row_off : m[k]) * D;
           if (uA < D) {
             const float h = gru_gates(a[k], hA[k]);
             if (g.peer.world == 0) g.out[orow + uA] = h;
@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
         meta_b = g.push_ids[m];
         meta_a = g.push_win[m];
       }
+      if (EPI == EPI_GRU && g.out_rows != nullptr) meta_a = g.out_rows[m];
       if (EPI == EPI_GRU) meta_b = g.nodes[rstride > 1 ? min(m * rstride + g.row_off, g.idx_limit - 1) : m];
     }
   };
@@ -259,9 +260,10 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
         int c = col + 4 * h;
         if (EPI == EPI_GRU) {
           // five parts of 172 columns, each padded to 176: [edge features | time encoding | own memory | other
-          // memory] of the message (stored as own, other, edge, time), then the memory row
+          // memory] of the message (stored as own, other, edge, time), then the memory row (no second source: the
+          // message's own part again)
           const int part = c / GRU_PART, o = c - part * GRU_PART;
-          c = o >= D || part > 4 ? Kd : part == 4 ? MSG + o : (part ^ 2) * D + o;
+          c = o >= D || part > 4 ? Kd : part == 4 ? (w1 != 0 ? MSG + o : o) : (part ^ 2) * D + o;
         }
         const bool in0 = c < w0;
         const int r = in0 ? r0 : r1;

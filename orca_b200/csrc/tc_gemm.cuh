@@ -96,8 +96,10 @@ struct Args {
   const int32_t *push_ids;
   const uint8_t *push_win;
   // GRU
-  const float *memory;
+  const float *memory;       // old memory values: row nodes[m], memory_ld floats each
+  int memory_ld;
   const int32_t *nodes;
+  const int32_t *out_rows;   // optional: result row of m (else m)
   // SCORE
   const float *w2;
   float b2;
@@ -120,6 +122,10 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
 // scorer over the rows of a group of batches (gemm.cu); tensor cores only
 int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
                float *d_prob, cudaStream_t s);
+// GRU of rows whose messages are in the message table and whose memory row is the own part of it: row m is the message
+// of node d_node[m], its new memory goes to row d_out_row[m] (gemm.cu); tensor cores only
+int gru_rows(const orca_gru_weights_t *w, const orca_memory_t &mem, const int32_t *d_node, const int32_t *d_out_row, int cap,
+             const int32_t *d_n, float *d_out, cudaStream_t s);
 // whether the projections run on the tensor cores (orca_set_projection_mode(0)); the fp32 debug path has
 // no peer fan-out
 bool projections_on_tensor_cores();

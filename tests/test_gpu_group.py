@@ -30,7 +30,8 @@ CASES = [("t_nb2", 37, 10, 5011, "budget", 2),       # 136 batches: five groups,
          ("t_nb2", 50, 10, 2030, "all", 2),          # unlimited reuse
          ("t_nb2", 50, 10, 2030, "none", 2),         # no reuse: a layer-1 row per sampled neighbour
          ("t_lru", 33, 20, 700, "none", 2),
-         ("c1", 129, 10, 6000, "budget", 1)]
+         ("c1", 129, 10, 6000, "budget", 1),
+         ("c1", 600, 10, 20000, "budget", 2)]        # a group whose last updates leave the memory chain, then one without
 
 
 @pytest.mark.parametrize("name,bs,k,E,recursion,layers", CASES)
