@@ -1,0 +1,678 @@
+// Cache plans from lists of distinct nodes (utils/cache.py:19-166, MRD).
+//
+// The policy is sequential over batches, so a plan takes as long as one batch's step times their number.  Most of what a
+// step used to do needs no earlier batch, and is done for all batches at once, a block per batch:
+//   batch_lists_kernel   the distinct nodes of a batch in ascending order, with their number of table entries: 40,000
+//                        table entries of a batch of 2000 edges are 900 endpoints and 550 out-of-batch neighbours
+//   sort_plan_kernel     the order of a plan: the first `budget` places of numba's argsort of a batch's candidates
+// What is left to one block, batch after batch (mrd_lists_kernel): candidates = cached | distinct nodes, and WHICH of
+// them the sort leaves in its first `budget` places.  For that, of numba's quicksort (tie_order.cuh) only the steps on
+// the range that the budget line falls into are needed, one or two as a rule: two candidates in three share the largest
+// key, which is the first pivot then, and where the equal keys of a range end up follows from its length alone.
+// 200 batches of 2000 edges, 10,700 candidates each, ms of kernels: 24.4 with the kernels of planner_mrd.cu, which walk
+// tables and sort whole lists batch after batch on a cluster of 16 SMs, 4.4 here: lists 0.13, next uses 0.39, the serial
+// step 3.5 (17.7 us a batch: the block's instructions and barriers), orders 0.29.
+#include <algorithm>
+
+#include "common.cuh"
+#include "context.cuh"
+#include "planner_lists.cuh"
+
+namespace orca {
+namespace lists {
+
+// ------------------------------------------------------------------------------ lists
+// One block a batch, blocks walk the batches.  Two bitmaps over the nodes (the batch's nodes, its endpoints) and the
+// prefix counts of the first, in global memory, left empty.  Bound by the latency of the table entries' lookups.
+__global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
+                                                        int32_t k, int64_t n_nodes, Lists l, uint32_t *bitmaps, int32_t *code,
+                                                        int32_t code_init) {
+  __shared__ int s_cnt[NW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t words = (n_nodes + 31) / 32, nb = (n_edges + bs - 1) / bs;
+  uint32_t *all = bitmaps + blockIdx.x * 3 * words, *target = all + words;
+  int32_t *before = (int32_t *)(target + words);
+  for (int64_t i = tid; i < 2 * words; i += T) all[i] = 0;
+  if (code != nullptr)
+    for (int64_t v = blockIdx.x * T + tid; v < n_nodes; v += (int64_t)gridDim.x * T) code[v] = code_init;
+  __syncthreads();
+  const int64_t chunk = ((words + NW - 1) / NW + 31) & ~31ll;     // words of a warp
+  constexpr int STEP = 8;
+  for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    const int64_t s = b * bs;
+    const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
+    const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
+    int32_t *id = l.id + b * l.stride, *mult = l.mult + b * l.stride;
+    for (int i = tid; i < m2; i += T) {
+      const int32_t v = q[i];
+      const uint32_t bit = 1u << (v & 31);
+      if (!(__ldcg(&target[v >> 5]) & bit)) {
+        atomicOr(&target[v >> 5], bit);
+        atomicOr(&all[v >> 5], bit);
+      }
+    }
+    __syncthreads();
+    // f(v) for the out-of-batch entries of the table, several at a time: their lookups overlap
+    const auto neighbors = [&](auto f) {
+      for (int64_t i0 = tid; i0 < (int64_t)m2 * k; i0 += STEP * T) {
+        int32_t v[STEP];
+        uint32_t w[STEP];
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) v[u] = i0 + u * T < (int64_t)m2 * k ? tab[i0 + u * T] : 0;
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) w[u] = v[u] != 0 ? __ldcg(&target[v[u] >> 5]) : 0;
+#pragma unroll
+        for (int u = 0; u < STEP; ++u)
+          if (v[u] != 0 && !((w[u] >> (v[u] & 31)) & 1u)) f(v[u]);
+      }
+    };
+    neighbors([&](int32_t v) {
+      const uint32_t bit = 1u << (v & 31);
+      if (!(__ldcg(&all[v >> 5]) & bit)) atomicOr(&all[v >> 5], bit);
+    });
+    __syncthreads();
+    int cnt = 0;
+    for (int64_t j = lane; j < chunk; j += 32) {
+      const int64_t wi = warp * chunk + j;
+      if (wi < words) cnt += __popc(__ldcg(&all[wi]));
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
+    const int c_lane = s_cnt[lane];
+    int base = __reduce_add_sync(0xffffffffu, lane < warp ? c_lane : 0);
+    const int n = __reduce_add_sync(0xffffffffu, c_lane);
+    for (int64_t j = 0; j < chunk; j += 32) {
+      const int64_t wi = warp * chunk + j + lane;
+      uint32_t bits = wi < words ? __ldcg(&all[wi]) : 0;
+      const int c = __popc(bits);
+      if (!__any_sync(0xffffffffu, c != 0)) continue;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      int pos = base + incl - c;
+      base += __shfl_sync(0xffffffffu, incl, 31);
+      if (bits != 0) {
+        before[wi] = pos;
+        const uint32_t t = __ldcg(&target[wi]);
+        for (; bits != 0; bits &= bits - 1, ++pos) {
+          const int bit = __ffs(bits) - 1;
+          id[pos] = (int32_t)(wi * 32 + bit) | ((t >> bit) & 1u ? TARGET : 0);
+          mult[pos] = 0;
+        }
+      }
+    }
+    if (tid == 0) l.count[b] = n;
+    __syncthreads();
+    neighbors([&](int32_t v) {
+      atomicAdd(&mult[__ldcg(&before[v >> 5]) + __popc(__ldcg(&all[v >> 5]) & ((1u << (v & 31)) - 1u))], 1);
+    });
+    __syncthreads();
+    for (int i = tid; i < n; i += T) {
+      const int32_t v = __ldcg(&id[i]) & ~TARGET;
+      all[v >> 5] = 0;
+      target[v >> 5] = 0;
+    }
+    __syncthreads();
+  }
+}
+
+int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
+                       const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init, cudaStream_t s) {
+  const Ctx *c = cur();
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "launch_batch_lists: no context for the current device");
+  const int grid = blocks_for((n_edges + bs - 1) / bs, n_nodes, std::min(c->sm_count, MOST_BLOCKS));
+  batch_lists_kernel<<<grid, T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, l, (uint32_t *)d_scratch, d_code, code_init);
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}
+
+// ------------------------------------------------------------------------------ MRD
+// A node's state is a word: key << 16 | the batch its embedding was computed in.  An entry of the selection: key and place
+// in the candidate list.
+constexpr int KEY_BITS = 16, IDX_BITS = 14;
+constexpr uint32_t FAR = (1u << KEY_BITS) - 1, IDX = (1u << IDX_BITS) - 1;    // FAR: no next use as a neighbour
+static_assert(CAP <= 1 << IDX_BITS && KEY_BITS + IDX_BITS <= 32, "an entry is a word");
+
+// The key of every listed node at its batch: the batch of its next use if that is as an out-of-batch neighbour, else
+// FAR.  (The reference sorts by the distance to it, or 1e8 + 1: the same order.)  One block, backwards: a batch waits for
+// one trip to L2, what the next one needs is under way before.
+__global__ void __launch_bounds__(T) next_use_lists_kernel(Lists l, int64_t nb, int32_t *next, int32_t *key) {
+  const int tid = threadIdx.x;
+  constexpr int AHEAD = 2;
+  const auto load = [&](int64_t b, int n, int i) { return i < n ? l.id[b * l.stride + i] : 0; };
+  int n = l.count[nb - 1], n_next = nb > 1 ? l.count[nb - 2] : 0;
+  int32_t x[AHEAD], y[AHEAD];
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u) x[u] = load(nb - 1, n, tid + u * T);
+  for (int64_t b = nb - 1; b >= 0; --b) {
+    const auto node = [&](int i, int32_t e) {
+      const int32_t v = e & ~TARGET;
+      key[b * l.stride + i] = __ldcg(&next[v]);
+      next[v] = e < 0 ? (int32_t)FAR : (int32_t)b;     // (distinct nodes: nobody else reads or writes it in this batch)
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+      if (tid + u * T < n) node(tid + u * T, x[u]);
+    for (int i = tid + AHEAD * T; i < n; i += T) node(i, l.id[b * l.stride + i]);
+    const int n_after = b > 1 ? l.count[b - 2] : 0;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) y[u] = b > 0 ? load(b - 1, n_next, tid + u * T) : 0;
+    __syncthreads();
+    n = n_next;
+    n_next = n_after;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) x[u] = y[u];
+  }
+}
+
+struct State {           // of a plan, between the launches for its chunks of batches
+  int32_t n_cached, failed;
+  int64_t used;
+  unsigned long long reuse, recompute, dist;
+};
+struct MrdArgs {
+  Lists l;
+  const int32_t *key;           // of the listed nodes
+  int64_t b0, b1, nb;           // batches of this launch, of the plan
+  int32_t budget, cap;
+  State *st;
+  int32_t *cached;              // [cap] cached ids, ascending (between launches)
+  uint32_t *cached_state;       // [cap] their states
+  int32_t *place;               // [cap] of the listed nodes: cached ids before it
+  int2 *cand;                   // [batches of a launch][cap] candidates and their states
+  int32_t *cand_n;              // [batches of a launch]
+  int64_t plan_cap;
+  int64_t *plan_off;
+  int32_t *status;
+};
+
+// Bitmaps over places of a list, with the number of bits before each word.
+struct Word {
+  uint32_t bits;
+  int32_t before;
+};
+// Fills `before` in; returns the number of bits.  All T threads, n <= T words, behind a barrier; ends with one.
+__device__ __forceinline__ int count_words(Word *w, int n, int32_t *s_w) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = tid < n ? __popc(w[tid].bits) : 0;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) s_w[warp] = incl;
+  __syncthreads();
+  const int x = s_w[lane];
+  const int before = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0), all = __reduce_add_sync(0xffffffffu, x);
+  if (tid < n) w[tid].before = before + incl - c;
+  __syncthreads();
+  return all;
+}
+__device__ __forceinline__ bool bit_of(Word w, int i) { return (w.bits >> (i & 31)) & 1u; }
+__device__ __forceinline__ int bits_before(Word w, int i) { return w.before + __popc(w.bits & ((1u << (i & 31)) - 1u)); }
+// the place of bit number m (there are more than m)
+__device__ __forceinline__ int bit_number(const Word *w, int n, int m) {
+  int lo = 0, hi = n;      // the last word with no more than m bits before it
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (w[mid].before <= m) lo = mid;
+    else hi = mid;
+  }
+  uint32_t bits = w[lo].bits;
+  m -= w[lo].before;
+  int at = 0;
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+    const int c = __popc(bits & ((1u << half) - 1u));
+    if (m >= c) m -= c, at += half, bits >>= half;
+  }
+  return 32 * lo + at;
+}
+
+// Numba's quicksort on a range [lo, hi] of equal keys: the place of the entry that ends up at place y.  A step parks the
+// middle entry at the end, turns the others round and puts it back in the middle; ranges of fewer than 16 stay as they
+// are.  So: down to the range in which y stays, and back through the steps.
+__device__ __forceinline__ int source_of_equal(int y, int lo, int hi) {
+  constexpr int DEPTH = 11;      // (the range is halved: no longer than 2^DEPTH * 15)
+  static_assert(CAP <= 15 << DEPTH, "");
+  int l[DEPTH], h[DEPTH], d = 0;
+  bool there = false;
+#pragma unroll
+  for (int i = 0; i < DEPTH; ++i) {
+    l[i] = lo, h[i] = hi;
+    const int mid = (lo + hi) >> 1;
+    there |= hi - lo < 15 || y == mid;
+    if (!there) {
+      d = i + 1;
+      if (y < mid) hi = mid - 1;
+      else lo = mid + 1;
+    }
+  }
+  int q = y;
+#pragma unroll
+  for (int i = DEPTH - 1; i >= 0; --i)
+    if (i < d) {
+      const int mid = (l[i] + h[i]) >> 1;
+      if (q == h[i]) q = mid;
+      q = l[i] + h[i] - 1 - q;
+      if (q == mid) q = h[i];
+    }
+  return q;
+}
+
+// Calls drop(entry's index) for the entries of e[0 .. n) (key << IDX_BITS | index, in candidate order) that numba's
+// argsort leaves at `keep` or behind, 0 < keep < n: its steps on the range that contains the line, until that range is
+// short or its keys are equal.  left, right: [n]; words: [(n + 31) / 32].  All T threads; no barrier at the end.
+//
+// A step whose pivot is the largest key there is, FAR, is the usual one, and needs no swap: its left list is the FAR
+// entries, its right list everything, so that the m-th FAR entry from the left goes to place hi - 1 - m for as long as it
+// lies left of that, and these places are the right part.
+template <class F>
+__device__ __forceinline__ void select_first(uint32_t *e, int n, int keep, uint16_t *left, uint16_t *right, Word *words,
+                                             uint32_t *s_tot, int32_t *s_place, F drop) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const auto key = [&](int i) { return e[i] >> IDX_BITS; };
+  const auto swap = [&](int i, int j) { const uint32_t x = e[i]; e[i] = e[j]; e[j] = x; };
+  const auto park = [&](int lo, int hi) {
+    const int mid = (lo + hi) >> 1;
+    uint32_t a = e[lo], c = e[mid], d = e[hi], t;
+    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
+    if (d >> IDX_BITS < c >> IDX_BITS) t = d, d = c, c = t;
+    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
+    e[lo] = a, e[mid] = d, e[hi] = c;
+  };
+  int lo = 0, hi = n - 1;
+  bool line = true, equal = false;      // the line falls into [lo, hi]; all its keys are equal
+  if (hi - lo >= 15) {
+    if (tid == 0) park(lo, hi);
+    __syncthreads();
+  }
+  while (line && !equal && hi - lo >= 15) {
+    const uint32_t p = key(hi);
+    if (p == FAR) {
+      // FAR entries of [lo, hi), a bit each; their number before every word
+      const int len = hi - lo, n_words = (len + 31) / 32;
+#pragma unroll 4
+      for (int i0 = warp * 32; i0 < len; i0 += T) {
+        const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < len && key(lo + i0 + lane) == FAR);
+        if (lane == 0) words[i0 >> 5].bits = w;
+      }
+      if (tid == 0) *s_place = 0;
+      __syncthreads();
+      count_words(words, n_words, (int32_t *)s_tot);
+      // swaps of the step: entry m at i swaps while i + m < len - 1, which grows from entry to entry
+      if (tid < n_words) {
+        uint32_t w = words[tid].bits;
+        const int first = 32 * tid + words[tid].before;
+        if (w != 0 && first + 31 - __clz(w) + __popc(w) - 1 >= len - 1) {     // (the word's last one does not)
+          int c = 0;
+          for (; w != 0 && first + __ffs(w) - 1 + c < len - 1; w &= w - 1) ++c;
+          w = (1u << c) - 1u;
+        }
+        if (w != 0) atomicAdd(s_place, __popc(w));
+      }
+      __syncthreads();
+      const int swaps = *s_place, mid = len - 1 - swaps;
+      // the pivot's place: the middle, if a FAR entry that need not swap lies there, else where the right part begins
+      bool stays = false;
+      if (mid >= 0 && mid < len) {
+        const Word w = words[mid >> 5];
+        stays = bit_of(w, mid) && bits_before(w, mid) == swaps;
+      }
+      const int m = lo + (stays ? mid : len - swaps);
+      if (keep > m + 1) {
+        // the right part: its places hi - 1, hi - 2, ... hold the first FAR entries, place hi the one after them
+        for (int y = keep + tid; y <= hi; y += T) {
+          const int q = source_of_equal(y, m + 1, hi);
+          drop((int)(e[lo + bit_number(words, n_words, q == hi ? hi - m - 1 : hi - 1 - q)] & IDX));
+        }
+        for (int pos = hi + 1 + tid; pos < n; pos += T) drop((int)(e[pos] & IDX));
+        return;      // (the parked entry is the pivot, at m: it stays)
+      }
+      __syncthreads();      // (s_place)
+    }
+    const int len = hi - lo, items = (len + T - 1) / T, first = lo + warp * 32 * items + lane;
+    uint32_t fl = 0, fr = 0, at = 0;
+    for (int i = 0; i < items; ++i) {
+      const int pos = first + 32 * i;
+      const uint32_t kv = pos < hi ? key(pos) : 0;
+      const bool l = pos < hi && kv >= p, r = pos < hi && kv <= p;
+      fl |= (l ? 1u : 0u) << i;
+      fr |= (r ? 1u : 0u) << i;
+      at += __popc(__ballot_sync(0xffffffffu, l)) | __popc(__ballot_sync(0xffffffffu, r)) << 16;
+    }
+    if (lane == 0) s_tot[warp] = at;
+    __syncthreads();
+    const uint32_t t = s_tot[lane], all = __reduce_add_sync(0xffffffffu, t);
+    at = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
+    const int nl = all & 0xffff, nr = all >> 16;
+    if (nl == len && nr == len) {       // (uniform over the block)
+      __syncthreads();
+      if (tid == 0) swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
+      equal = true;
+      break;
+    }
+    for (int i = 0; i < items; ++i) {
+      const int pos = first + 32 * i;
+      const bool l = (fl >> i) & 1u, r = (fr >> i) & 1u;
+      const uint32_t ml = __ballot_sync(0xffffffffu, l), mr = __ballot_sync(0xffffffffu, r);
+      if (l) left[(at & 0xffff) + __popc(ml & lt)] = (uint16_t)pos;
+      if (r) right[(at >> 16) + __popc(mr & lt)] = (uint16_t)pos;
+      at += __popc(ml) | __popc(mr) << 16;
+    }
+    __syncthreads();
+    // the m-th of the left list swaps with the m-th from the end of the right list while it lies left of it
+    const int pairs = min(nl, nr);
+    for (int m = tid; m < pairs; m += T) {
+      const int pl = left[m], pr = right[nr - 1 - m];
+      if (pl >= pr) {
+        if (m == 0) *s_place = pl;
+        break;                          // (behind a pair that does not swap, none does)
+      }
+      const int next_l = m + 1 < nl ? (int)left[m + 1] : hi;
+      if (m + 1 >= pairs || next_l >= (int)right[nr - 2 - m]) *s_place = min(next_l, pr);
+      swap(pl, pr);
+    }
+    if (tid == 0 && pairs == 0) *s_place = nl > 0 ? (int)left[0] : hi;
+    __syncthreads();
+    const int m = *s_place;             // the pivot's place
+    const int old_hi = hi;
+    if (keep <= m) {
+      line = keep > lo && keep < m;     // (keep == m: the left part stays, the rest goes)
+      hi = m - 1;
+      if (!line) lo = keep, hi = keep - 1;
+    } else {
+      line = keep > m + 1;
+      lo = m + 1;
+      if (!line) hi = lo - 1;
+    }
+    if (tid == 0) {
+      swap(m, old_hi);
+      if (line && !equal && hi - lo >= 15) park(lo, hi);
+    }
+    __syncthreads();
+  }
+  if (equal) __syncthreads();           // (the entries of the undone step)
+  if (equal) {
+    for (int y = keep + tid; y <= hi; y += T) drop((int)(e[source_of_equal(y, lo, hi)] & IDX));
+    lo = hi + 1;
+  }
+  for (int pos = lo + tid; pos < n; pos += T) {
+    if (pos <= hi) {
+      const uint32_t k = key(pos);
+      int place = lo;
+      for (int q = lo; q <= hi; ++q) place += key(q) < k || (key(q) == k && q < pos) ? 1 : 0;
+      if (place < keep) continue;
+    }
+    drop((int)(e[pos] & IDX));
+  }
+}
+
+// Forward sweep over batches b0 .. b1, one block.  Shared memory: [cached ids | later the lists of a step][entries of the
+// selection], `cap` words each, then bitmaps.  What a batch costs is the walk over all of its candidates, twice (into the
+// list and back into the cached ids): a warp takes a word of the bitmaps at a time.
+__global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__ MrdArgs g) {
+  extern __shared__ __align__(16) char raw[];
+  __shared__ uint32_t s_tot[NW];
+  __shared__ int32_t s_place;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cap = g.cap, n_words = cap / 32;
+  int32_t *s_cached = (int32_t *)raw;
+  uint32_t *s_ent = (uint32_t *)(s_cached + cap);
+  uint16_t *left = (uint16_t *)s_cached, *right = left + cap;
+  Word *s_list = (Word *)(s_ent + cap), *s_new = s_list + n_words, *s_kept = s_new + n_words;
+  uint32_t *s_known = (uint32_t *)(s_kept + n_words);
+  if (g.st->failed) return;
+  int n_cached = g.st->n_cached;
+  int64_t used = g.st->used;
+  unsigned long long reuse = 0, recompute = 0, dist = 0;
+  for (int i = tid; i < n_cached; i += T) s_cached[i] = g.cached[i];
+  bool failed = false;
+  // the first nodes of the next batch's list, loaded ahead
+  constexpr int AHEAD = 2;
+  int32_t x_next[AHEAD], mult_next[AHEAD];
+  int n_next = g.l.count[g.b0];
+  const auto load_ahead = [&](int64_t b) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int64_t i = tid + u * T;
+      x_next[u] = i < n_next ? g.l.id[b * g.l.stride + i] : 0;
+      mult_next[u] = i < n_next ? g.l.mult[b * g.l.stride + i] : 0;
+    }
+  };
+  load_ahead(g.b0);
+  for (int64_t b = g.b0; b < g.b1; ++b) {
+    const int64_t at = b * g.l.stride;
+    const int n_list = n_next;
+    int2 *cand = g.cand + (b - g.b0) * cap;
+    if (n_list > cap) {      // (uniform over the block)
+      failed = true;
+      break;
+    }
+    for (int i = tid; i < n_words; i += T) s_new[i].bits = s_known[i] = s_list[i].bits = 0;
+    __syncthreads();         // (and the cached ids are there)
+    // which of the batch's nodes are cached: a bit in s_list; statistics of the reuse
+    const auto look_up = [&](int i, int32_t x, int m) {
+      bool cached = false;
+      if (i < n_list) {
+        const int32_t v = x & ~TARGET;
+        int lo = 0, hi = n_cached;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (s_cached[mid] < v) lo = mid + 1;
+          else hi = mid;
+        }
+        cached = lo < n_cached && s_cached[lo] == v;
+        g.place[i] = lo;
+        if (x >= 0) {
+          if (cached) {
+            reuse += m;
+            dist += (unsigned long long)m * (unsigned long long)(b - (g.cached_state[lo] & 0xffffu));
+          } else {
+            recompute += m;
+          }
+        }
+      }
+      const uint32_t w = __ballot_sync(0xffffffffu, cached);
+      if (lane == 0) s_list[i >> 5].bits = w;
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+      if (u * T + warp * 32 < n_list) look_up(tid + u * T, x_next[u], mult_next[u]);
+    for (int i0 = AHEAD * T + warp * 32; i0 < n_list; i0 += T) {
+      const int i = i0 + lane;
+      look_up(i, i < n_list ? g.l.id[at + i] : 0, i < n_list ? g.l.mult[at + i] : 0);
+    }
+    __syncthreads();
+    const int n = n_cached + n_list - count_words(s_list, n_words, (int32_t *)s_tot);
+    if (n > cap) {
+      failed = true;
+      break;
+    }
+    // candidates in ascending order: first the batch's nodes, then the other cached ones around them
+    const auto place = [&](int i, int32_t x) {
+      if (i >= n_list) return;
+      const uint32_t key = (uint32_t)g.key[at + i];
+      const Word w = s_list[i >> 5];
+      const int c = g.place[i], pos = c + i - bits_before(w, i);
+      const bool cached = bit_of(w, i);
+      s_ent[pos] = key << IDX_BITS | (uint32_t)pos;
+      cand[pos] = make_int2(x & ~TARGET, (int)(key << 16 | (x < 0 || !cached ? (uint32_t)b : g.cached_state[c] & 0xffffu)));
+      atomicOr(cached ? &s_known[pos >> 5] : &s_new[pos >> 5].bits, 1u << (pos & 31));
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) place(tid + u * T, x_next[u]);
+    for (int i = tid + AHEAD * T; i < n_list; i += T) place(i, g.l.id[at + i]);
+    if (b + 1 < g.b1) {
+      n_next = g.l.count[b + 1];
+      load_ahead(b + 1);
+    }
+    __syncthreads();
+    count_words(s_new, n_words, (int32_t *)s_tot);
+#pragma unroll 4
+    for (int w = warp; w < n_words; w += NW) {
+      const Word add = s_new[w];
+      const int pos = 32 * w + lane;
+      if (pos < n && !(((add.bits | s_known[w]) >> lane) & 1u)) {
+        const int c = pos - bits_before(add, lane);
+        const uint32_t st = g.cached_state[c];
+        s_ent[pos] = st >> 16 << IDX_BITS | (uint32_t)pos;
+        cand[pos] = make_int2(s_cached[c], (int)st);
+      }
+      if (lane == 0) s_kept[w].bits = n >= 32 * w + 32 ? 0xffffffffu : n > 32 * w ? (1u << (n - 32 * w)) - 1u : 0u;
+    }
+    const int keep = min(n, g.budget);
+    if (used + keep > g.plan_cap) {      // (uniform over the block)
+      if (tid == 0) report(g.status, ORCA_E_CAPACITY, (int)b);
+      failed = true;
+      break;
+    }
+    __syncthreads();
+    if (keep < n)
+      select_first(s_ent, n, keep, left, right, s_list, s_tot, &s_place,
+                   [&](int i) { atomicAnd(&s_kept[i >> 5].bits, ~(1u << (i & 31))); });
+    __syncthreads();
+    count_words(s_kept, n_words, (int32_t *)s_tot);
+#pragma unroll 4
+    for (int w = warp; w < n_words; w += NW) {
+      const Word kept = s_kept[w];
+      if (!bit_of(kept, lane)) continue;
+      const int c = bits_before(kept, lane);
+      const int2 x = __ldcg(&cand[32 * w + lane]);
+      s_cached[c] = x.x;
+      g.cached_state[c] = (uint32_t)x.y;
+    }
+    if (tid == 0) {
+      g.plan_off[b] = used;
+      g.cand_n[b - g.b0] = n;
+    }
+    n_cached = keep;
+    used += keep;
+  }
+  __syncthreads();
+  for (int i = tid; i < n_cached && !failed; i += T) g.cached[i] = s_cached[i];
+  for (int o = 16; o > 0; o >>= 1) {
+    reuse += __shfl_xor_sync(0xffffffffu, reuse, o);
+    recompute += __shfl_xor_sync(0xffffffffu, recompute, o);
+    dist += __shfl_xor_sync(0xffffffffu, dist, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&g.st->reuse, reuse);
+    atomicAdd(&g.st->recompute, recompute);
+    atomicAdd(&g.st->dist, dist);
+  }
+  if (tid == 0) {
+    g.st->n_cached = n_cached;
+    g.st->used = used;
+    g.st->failed = failed;
+    if (g.b1 == g.nb) g.plan_off[g.nb] = used;
+  }
+}
+
+// The order of the plans of a launch's batches, a block each; the last one's totals.
+__global__ void __launch_bounds__(T, 1) sort_plan_kernel(const __grid_constant__ MrdArgs g, int32_t *plan, int64_t *stats) {
+  __shared__ uint32_t s_tot[NW];
+  if (g.st->failed) return;
+  if (g.b1 == g.nb && blockIdx.x == 0 && threadIdx.x == 0)
+    stats[0] = g.st->reuse, stats[1] = g.st->recompute, stats[2] = g.st->dist;
+  const tie::Shared w{g.cap};
+  for (int64_t b = g.b0 + blockIdx.x; b < g.b1; b += gridDim.x) {
+    const int n = g.cand_n[b - g.b0], keep = min(n, g.budget);
+    const int2 *cand = g.cand + (b - g.b0) * g.cap;
+    int32_t *out = plan + g.plan_off[b];
+    for (int i = threadIdx.x; i < n; i += T) {
+      w.key(i) = (int32_t)((uint32_t)cand[i].y >> 16);
+      w.idx(i) = (uint16_t)i;
+    }
+    tie::sort_first_shared(w, s_tot, n, keep, [&](int place, int i) { out[place] = cand[i].x; });
+  }
+}
+
+constexpr int64_t CHUNK = 512;      // batches of a launch: bounds the candidates that wait for their order (2 x 4 * CAP bytes each)
+
+struct MrdLayout {
+  int64_t state, id, mult, count, key, next, scratch, cached, cached_state, place, cand, cand_n, total;
+  int32_t cap;
+};
+static MrdLayout mrd_layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
+  MrdLayout L;
+  const int64_t nb = (n_edges + bs - 1) / bs, stride = stride_of(bs, k, n_nodes), chunk = std::min(nb, CHUNK);
+  L.cap = (int32_t)((std::min<int64_t>({(int64_t)budget + 2ll * bs * (k + 1), n_nodes, (int64_t)CAP}) + 31) & ~31ll);
+  int64_t at = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t o = at;
+    at += (bytes + 255) & ~255ll;
+    return o;
+  };
+  L.state = take(sizeof(State));
+  L.id = take(nb * stride * 4);
+  L.mult = take(nb * stride * 4);
+  L.count = take(nb * 4);
+  L.key = take(nb * stride * 4);
+  L.next = take(n_nodes * 4);
+  L.scratch = take(scratch_bytes(nb, n_nodes));
+  L.cached = take(L.cap * 4);
+  L.cached_state = take(L.cap * 4);
+  L.place = take(L.cap * 4);
+  L.cand = take(chunk * L.cap * 8);
+  L.cand_n = take(chunk * 4);
+  L.total = at;
+  return L;
+}
+
+// (a key has to name every batch)
+bool mrd_takes(int64_t n_edges, int32_t bs) { return (n_edges + bs - 1) / bs < (int64_t)FAR; }
+int64_t mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
+  return mrd_layout(n_edges, bs, k, n_nodes, budget).total;
+}
+
+int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
+               int32_t budget, int32_t *d_plan, int64_t plan_cap, int64_t *d_plan_off, int64_t *d_stats, int32_t *d_status,
+               void *d_workspace, const int32_t **d_failed, cudaStream_t s) {
+  const Ctx *c = cur();
+  if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_plan_mrd: no context for the current device");
+  const MrdLayout L = mrd_layout(n_edges, bs, k, n_nodes, budget);
+  char *base = (char *)d_workspace;
+  MrdArgs g{};
+  g.l.id = (int32_t *)(base + L.id), g.l.mult = (int32_t *)(base + L.mult), g.l.count = (int32_t *)(base + L.count);
+  g.l.stride = stride_of(bs, k, n_nodes);
+  g.key = (int32_t *)(base + L.key);
+  g.nb = (n_edges + bs - 1) / bs;
+  g.budget = budget, g.cap = L.cap;
+  g.st = (State *)(base + L.state);
+  g.cached = (int32_t *)(base + L.cached), g.cached_state = (uint32_t *)(base + L.cached_state);
+  g.place = (int32_t *)(base + L.place);
+  g.cand = (int2 *)(base + L.cand);
+  g.cand_n = (int32_t *)(base + L.cand_n);
+  g.plan_cap = plan_cap, g.plan_off = d_plan_off, g.status = d_status;
+  ORCA_CUDA(cudaMemsetAsync(g.st, 0, sizeof(State), s));
+  int rc = launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, g.l, base + L.scratch, (int32_t *)(base + L.next),
+                              (int32_t)FAR, s);
+  if (rc != ORCA_OK) return rc;
+  next_use_lists_kernel<<<1, T, 0, s>>>(g.l, g.nb, (int32_t *)(base + L.next), (int32_t *)(base + L.key));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  const int smem = 8 * L.cap + 7 * (L.cap / 32) * 4, smem_sort = tie::Shared::BYTES * L.cap;
+  ORCA_CUDA(cudaFuncSetAttribute(mrd_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  ORCA_CUDA(cudaFuncSetAttribute(sort_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_sort));
+  for (g.b0 = 0; g.b0 < g.nb; g.b0 = g.b1) {
+    g.b1 = std::min(g.nb, g.b0 + CHUNK);
+    mrd_lists_kernel<<<1, T, smem, s>>>(g);
+    ORCA_COUNT_LAUNCH();
+    ORCA_LAUNCH_CHECK();
+    sort_plan_kernel<<<(int)std::min<int64_t>(g.b1 - g.b0, c->sm_count), T, smem_sort, s>>>(g, d_plan, d_stats);
+    ORCA_COUNT_LAUNCH();
+    ORCA_LAUNCH_CHECK();
+  }
+  *d_failed = &g.st->failed;
+  return ORCA_OK;
+}
+
+}  // namespace lists
+}  // namespace orca

@@ -1,7 +1,8 @@
 // MRD cache planning on the device (utils/cache.py:19-89 read_batches + :92-166 MRD_numba).
 //
 // Input: the query list of all batches (batch b = its sources, then its destinations) and the neighbour
-// table the sampling kernel produced for it.  Two persistent kernels walk the batches (each exists for one
+// table the sampling kernel produced for it.  Plans whose candidate lists are all of at most lists::CAP entries are made
+// by planner_lists.cu; the kernels here serve the others.  Two persistent kernels walk the batches (each exists for one
 // CTA and for one thread-block cluster; the cluster form is the one normally launched):
 //
 //   next_use_kernel   backwards.  Keeps, per node, the code of its nearest LATER use
@@ -24,6 +25,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "planner_lists.cuh"
 #include "tie_shared.cuh"
 
 namespace orca {
@@ -60,8 +62,10 @@ using tie::key_of;
 using tie::live;
 
 // ------------------------------------------------------------------------------ backward pass
+// (only_if, in all of these kernels: a word that is zero when the plan has been made already)
 __global__ void __launch_bounds__(T) next_use_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges,
-                                                     int32_t bs, int32_t k, int64_t n_nodes, Work w) {
+                                                     int32_t bs, int32_t k, int64_t n_nodes, Work w, const int32_t *only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   const int tid = threadIdx.x;
   const int64_t nb = (n_edges + bs - 1) / bs;
   for (int64_t v = tid; v < n_nodes; v += T) {
@@ -100,8 +104,9 @@ __global__ void __launch_bounds__(T) next_use_kernel(const int32_t *nodes, const
 __global__ void __launch_bounds__(T) mrd_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
                                                 int32_t k, int64_t n_nodes, int32_t budget, Work w,
                                                 int32_t *plan, int64_t plan_cap, int64_t *plan_off,
-                                                int64_t *stats, int32_t *status) {
+                                                int64_t *stats, int32_t *status, const int32_t *only_if) {
   __shared__ int s_l[NW], s_r[NW];
+  if (only_if != nullptr && *only_if == 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   const int64_t nb = (n_edges + bs - 1) / bs;
@@ -265,7 +270,8 @@ struct ClusterWork {
 
 __global__ void __launch_bounds__(T, 1) next_use_cluster_kernel(const int32_t *nodes, const int32_t *nbr,
                                                                 int64_t n_edges, int32_t bs, int32_t k,
-                                                                int64_t n_nodes, Work w) {
+                                                                int64_t n_nodes, Work w, const int32_t *only_if) {
+  if (only_if != nullptr && *only_if == 0) return;      // (the same in every block of the cluster)
   const int GT = T * (int)cluster_size();
   const int gt = (int)cluster_rank() * T + threadIdx.x;
   const int64_t nb = (n_edges + bs - 1) / bs;
@@ -394,8 +400,10 @@ __device__ __forceinline__ void sort_first_cluster(tie::Shared w, uint32_t *tot,
 __global__ void __launch_bounds__(T, 1) mrd_cluster_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges,
                                                            int32_t bs, int32_t k, int64_t n_nodes, int32_t budget,
                                                            ClusterWork cw, int32_t *plan, int64_t plan_cap,
-                                                           int64_t *plan_off, int64_t *stats, int32_t *status) {
+                                                           int64_t *plan_off, int64_t *stats, int32_t *status,
+                                                           const int32_t *only_if) {
   __shared__ uint32_t s_tot[NW];
+  if (only_if != nullptr && *only_if == 0) return;
   const Work &w = cw.w;
   const int GT = T * (int)cluster_size();
   const int gt = (int)cluster_rank() * T + threadIdx.x;
@@ -723,7 +731,9 @@ using namespace orca;
 extern "C" int64_t orca_plan_mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
                                                  int32_t budget) {
   if (n_edges < 0 || bs <= 0 || k < 1 || n_nodes <= 0 || budget <= 0) return -1;
-  return mrd::layout(n_edges, bs, k, n_nodes, budget).total;
+  // (one form after the other: they share the memory, but for the state in front)
+  const int64_t walk = 256 + mrd::layout(n_edges, bs, k, n_nodes, budget).total;
+  return lists::mrd_takes(n_edges, bs) ? std::max(walk, lists::mrd_workspace_bytes(n_edges, bs, k, n_nodes, budget)) : walk;
 }
 
 extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k, const int32_t *d_nbr,
@@ -735,11 +745,12 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
   ORCA_CHECK_ARG(n_nodes < (1ll << 31) && (n_edges + bs - 1) / bs < (1ll << 29));
   ORCA_CHECK_ARG(mrd::cand_cap(bs, k, budget) < (1ll << 31));
   const mrd::Layout L = mrd::layout(n_edges, bs, k, n_nodes, budget);
-  if (workspace_bytes < L.total)
+  const int64_t need = orca_plan_mrd_workspace_bytes(n_edges, bs, k, n_nodes, budget);
+  if (workspace_bytes < need)
     return set_error(ORCA_E_CAPACITY, "orca_plan_mrd: workspace of %lld bytes, %lld needed", (long long)workspace_bytes,
-                     (long long)L.total);
+                     (long long)need);
   ORCA_CHECK_ARG(((uintptr_t)d_workspace & 255) == 0);
-  char *base = (char *)d_workspace;
+  char *base = (char *)d_workspace + 256;
   mrd::Work w;
   w.nx_query = (int32_t *)(base + L.off[0]);
   w.nx_table = (int32_t *)(base + L.off[1]);
@@ -761,6 +772,14 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
   if (n_edges == 0) {
     ORCA_CUDA(cudaMemsetAsync(d_plan_off, 0, sizeof(int64_t), s));
     return ORCA_OK;
+  }
+  // From lists of distinct nodes (planner_lists.cu), unless a candidate list is too long for them, which shows on the way:
+  // the kernels below look at the word that says so.
+  const int32_t *only_if = nullptr;
+  if (lists::mrd_takes(n_edges, bs)) {
+    const int rc = lists::launch_mrd(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, d_plan_flat, plan_cap, d_plan_off,
+                                     d_stats, d_status, d_workspace, &only_if, s);
+    if (rc != ORCA_OK || std::min(mrd::cand_cap(bs, k, budget), n_nodes) <= lists::CAP) return rc;
   }
   // A cluster of 16 (else 8) CTAs shares every phase when the device can place such a cluster and the
   // candidate list fits its threads' registers (a phase costs a cluster barrier of ~600 cycles, an L2 round
@@ -818,19 +837,20 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    ORCA_CUDA(cudaLaunchKernelEx(&cfg, mrd::next_use_cluster_kernel, d_nodes, d_nbr, n_edges, bs, k, n_nodes, w));
+    ORCA_CUDA(cudaLaunchKernelEx(&cfg, mrd::next_use_cluster_kernel, d_nodes, d_nbr, n_edges, bs, k, n_nodes, w,
+                                 only_if));
     ORCA_COUNT_LAUNCH();
     cfg.dynamicSmemBytes = smem;
     ORCA_CUDA(cudaLaunchKernelEx(&cfg, mrd::mrd_cluster_kernel, d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, cw,
-                                 d_plan_flat, plan_cap, d_plan_off, d_stats, d_status));
+                                 d_plan_flat, plan_cap, d_plan_off, d_stats, d_status, only_if));
     ORCA_COUNT_LAUNCH();
     return ORCA_OK;
   }
-  mrd::next_use_kernel<<<1, mrd::T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, w);
+  mrd::next_use_kernel<<<1, mrd::T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, w, only_if);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   mrd::mrd_kernel<<<1, mrd::T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, w, d_plan_flat, plan_cap,
-                                       d_plan_off, d_stats, d_status);
+                                       d_plan_off, d_stats, d_status, only_if);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;
