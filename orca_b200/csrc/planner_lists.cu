@@ -132,11 +132,7 @@ int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_e
 }
 
 // ------------------------------------------------------------------------------ MRD
-// A node's state is a word: key << 16 | the batch its embedding was computed in.  An entry of the selection: key and place
-// in the candidate list.
-constexpr int KEY_BITS = 16, IDX_BITS = 14;
-constexpr uint32_t FAR = (1u << KEY_BITS) - 1, IDX = (1u << IDX_BITS) - 1;    // FAR: no next use as a neighbour
-static_assert(CAP <= 1 << IDX_BITS && KEY_BITS + IDX_BITS <= 32, "an entry is a word");
+// A node's state is a word: key << 16 | the batch its embedding was computed in.
 
 // The key of every listed node at its batch: the batch of its next use if that is as an out-of-batch neighbour, else
 // FAR.  (The reference sorts by the distance to it, or 1e8 + 1: the same order.)  One block, backwards: a batch waits for
@@ -190,230 +186,6 @@ struct MrdArgs {
   int64_t *plan_off;
   int32_t *status;
 };
-
-// Bitmaps over places of a list, with the number of bits before each word.
-struct Word {
-  uint32_t bits;
-  int32_t before;
-};
-// Fills `before` in; returns the number of bits.  All T threads, n <= T words, behind a barrier; ends with one.
-__device__ __forceinline__ int count_words(Word *w, int n, int32_t *s_w) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c = tid < n ? __popc(w[tid].bits) : 0;
-  int incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int up = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += up;
-  }
-  if (lane == 31) s_w[warp] = incl;
-  __syncthreads();
-  const int x = s_w[lane];
-  const int before = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0), all = __reduce_add_sync(0xffffffffu, x);
-  if (tid < n) w[tid].before = before + incl - c;
-  __syncthreads();
-  return all;
-}
-__device__ __forceinline__ bool bit_of(Word w, int i) { return (w.bits >> (i & 31)) & 1u; }
-__device__ __forceinline__ int bits_before(Word w, int i) { return w.before + __popc(w.bits & ((1u << (i & 31)) - 1u)); }
-// the place of bit number m (there are more than m)
-__device__ __forceinline__ int bit_number(const Word *w, int n, int m) {
-  int lo = 0, hi = n;      // the last word with no more than m bits before it
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (w[mid].before <= m) lo = mid;
-    else hi = mid;
-  }
-  uint32_t bits = w[lo].bits;
-  m -= w[lo].before;
-  int at = 0;
-#pragma unroll
-  for (int half = 16; half > 0; half >>= 1) {
-    const int c = __popc(bits & ((1u << half) - 1u));
-    if (m >= c) m -= c, at += half, bits >>= half;
-  }
-  return 32 * lo + at;
-}
-
-// Numba's quicksort on a range [lo, hi] of equal keys: the place of the entry that ends up at place y.  A step parks the
-// middle entry at the end, turns the others round and puts it back in the middle; ranges of fewer than 16 stay as they
-// are.  So: down to the range in which y stays, and back through the steps.
-__device__ __forceinline__ int source_of_equal(int y, int lo, int hi) {
-  constexpr int DEPTH = 11;      // (the range is halved: no longer than 2^DEPTH * 15)
-  static_assert(CAP <= 15 << DEPTH, "");
-  int l[DEPTH], h[DEPTH], d = 0;
-  bool there = false;
-#pragma unroll
-  for (int i = 0; i < DEPTH; ++i) {
-    l[i] = lo, h[i] = hi;
-    const int mid = (lo + hi) >> 1;
-    there |= hi - lo < 15 || y == mid;
-    if (!there) {
-      d = i + 1;
-      if (y < mid) hi = mid - 1;
-      else lo = mid + 1;
-    }
-  }
-  int q = y;
-#pragma unroll
-  for (int i = DEPTH - 1; i >= 0; --i)
-    if (i < d) {
-      const int mid = (l[i] + h[i]) >> 1;
-      if (q == h[i]) q = mid;
-      q = l[i] + h[i] - 1 - q;
-      if (q == mid) q = h[i];
-    }
-  return q;
-}
-
-// Calls drop(entry's index) for the entries of e[0 .. n) (key << IDX_BITS | index, in candidate order) that numba's
-// argsort leaves at `keep` or behind, 0 < keep < n: its steps on the range that contains the line, until that range is
-// short or its keys are equal.  left, right: [n]; words: [(n + 31) / 32].  All T threads; no barrier at the end.
-//
-// A step whose pivot is the largest key there is, FAR, is the usual one, and needs no swap: its left list is the FAR
-// entries, its right list everything, so that the m-th FAR entry from the left goes to place hi - 1 - m for as long as it
-// lies left of that, and these places are the right part.
-template <class F>
-__device__ __forceinline__ void select_first(uint32_t *e, int n, int keep, uint16_t *left, uint16_t *right, Word *words,
-                                             uint32_t *s_tot, int32_t *s_place, F drop) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  const auto key = [&](int i) { return e[i] >> IDX_BITS; };
-  const auto swap = [&](int i, int j) { const uint32_t x = e[i]; e[i] = e[j]; e[j] = x; };
-  const auto park = [&](int lo, int hi) {
-    const int mid = (lo + hi) >> 1;
-    uint32_t a = e[lo], c = e[mid], d = e[hi], t;
-    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
-    if (d >> IDX_BITS < c >> IDX_BITS) t = d, d = c, c = t;
-    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
-    e[lo] = a, e[mid] = d, e[hi] = c;
-  };
-  int lo = 0, hi = n - 1;
-  bool line = true, equal = false;      // the line falls into [lo, hi]; all its keys are equal
-  if (hi - lo >= 15) {
-    if (tid == 0) park(lo, hi);
-    __syncthreads();
-  }
-  while (line && !equal && hi - lo >= 15) {
-    const uint32_t p = key(hi);
-    if (p == FAR) {
-      // FAR entries of [lo, hi), a bit each; their number before every word
-      const int len = hi - lo, n_words = (len + 31) / 32;
-#pragma unroll 4
-      for (int i0 = warp * 32; i0 < len; i0 += T) {
-        const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < len && key(lo + i0 + lane) == FAR);
-        if (lane == 0) words[i0 >> 5].bits = w;
-      }
-      if (tid == 0) *s_place = 0;
-      __syncthreads();
-      count_words(words, n_words, (int32_t *)s_tot);
-      // swaps of the step: entry m at i swaps while i + m < len - 1, which grows from entry to entry
-      if (tid < n_words) {
-        uint32_t w = words[tid].bits;
-        const int first = 32 * tid + words[tid].before;
-        if (w != 0 && first + 31 - __clz(w) + __popc(w) - 1 >= len - 1) {     // (the word's last one does not)
-          int c = 0;
-          for (; w != 0 && first + __ffs(w) - 1 + c < len - 1; w &= w - 1) ++c;
-          w = (1u << c) - 1u;
-        }
-        if (w != 0) atomicAdd(s_place, __popc(w));
-      }
-      __syncthreads();
-      const int swaps = *s_place, mid = len - 1 - swaps;
-      // the pivot's place: the middle, if a FAR entry that need not swap lies there, else where the right part begins
-      bool stays = false;
-      if (mid >= 0 && mid < len) {
-        const Word w = words[mid >> 5];
-        stays = bit_of(w, mid) && bits_before(w, mid) == swaps;
-      }
-      const int m = lo + (stays ? mid : len - swaps);
-      if (keep > m + 1) {
-        // the right part: its places hi - 1, hi - 2, ... hold the first FAR entries, place hi the one after them
-        for (int y = keep + tid; y <= hi; y += T) {
-          const int q = source_of_equal(y, m + 1, hi);
-          drop((int)(e[lo + bit_number(words, n_words, q == hi ? hi - m - 1 : hi - 1 - q)] & IDX));
-        }
-        for (int pos = hi + 1 + tid; pos < n; pos += T) drop((int)(e[pos] & IDX));
-        return;      // (the parked entry is the pivot, at m: it stays)
-      }
-      __syncthreads();      // (s_place)
-    }
-    const int len = hi - lo, items = (len + T - 1) / T, first = lo + warp * 32 * items + lane;
-    uint32_t fl = 0, fr = 0, at = 0;
-    for (int i = 0; i < items; ++i) {
-      const int pos = first + 32 * i;
-      const uint32_t kv = pos < hi ? key(pos) : 0;
-      const bool l = pos < hi && kv >= p, r = pos < hi && kv <= p;
-      fl |= (l ? 1u : 0u) << i;
-      fr |= (r ? 1u : 0u) << i;
-      at += __popc(__ballot_sync(0xffffffffu, l)) | __popc(__ballot_sync(0xffffffffu, r)) << 16;
-    }
-    if (lane == 0) s_tot[warp] = at;
-    __syncthreads();
-    const uint32_t t = s_tot[lane], all = __reduce_add_sync(0xffffffffu, t);
-    at = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
-    const int nl = all & 0xffff, nr = all >> 16;
-    if (nl == len && nr == len) {       // (uniform over the block)
-      __syncthreads();
-      if (tid == 0) swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
-      equal = true;
-      break;
-    }
-    for (int i = 0; i < items; ++i) {
-      const int pos = first + 32 * i;
-      const bool l = (fl >> i) & 1u, r = (fr >> i) & 1u;
-      const uint32_t ml = __ballot_sync(0xffffffffu, l), mr = __ballot_sync(0xffffffffu, r);
-      if (l) left[(at & 0xffff) + __popc(ml & lt)] = (uint16_t)pos;
-      if (r) right[(at >> 16) + __popc(mr & lt)] = (uint16_t)pos;
-      at += __popc(ml) | __popc(mr) << 16;
-    }
-    __syncthreads();
-    // the m-th of the left list swaps with the m-th from the end of the right list while it lies left of it
-    const int pairs = min(nl, nr);
-    for (int m = tid; m < pairs; m += T) {
-      const int pl = left[m], pr = right[nr - 1 - m];
-      if (pl >= pr) {
-        if (m == 0) *s_place = pl;
-        break;                          // (behind a pair that does not swap, none does)
-      }
-      const int next_l = m + 1 < nl ? (int)left[m + 1] : hi;
-      if (m + 1 >= pairs || next_l >= (int)right[nr - 2 - m]) *s_place = min(next_l, pr);
-      swap(pl, pr);
-    }
-    if (tid == 0 && pairs == 0) *s_place = nl > 0 ? (int)left[0] : hi;
-    __syncthreads();
-    const int m = *s_place;             // the pivot's place
-    const int old_hi = hi;
-    if (keep <= m) {
-      line = keep > lo && keep < m;     // (keep == m: the left part stays, the rest goes)
-      hi = m - 1;
-      if (!line) lo = keep, hi = keep - 1;
-    } else {
-      line = keep > m + 1;
-      lo = m + 1;
-      if (!line) hi = lo - 1;
-    }
-    if (tid == 0) {
-      swap(m, old_hi);
-      if (line && !equal && hi - lo >= 15) park(lo, hi);
-    }
-    __syncthreads();
-  }
-  if (equal) __syncthreads();           // (the entries of the undone step)
-  if (equal) {
-    for (int y = keep + tid; y <= hi; y += T) drop((int)(e[source_of_equal(y, lo, hi)] & IDX));
-    lo = hi + 1;
-  }
-  for (int pos = lo + tid; pos < n; pos += T) {
-    if (pos <= hi) {
-      const uint32_t k = key(pos);
-      int place = lo;
-      for (int q = lo; q <= hi; ++q) place += key(q) < k || (key(q) == k && q < pos) ? 1 : 0;
-      if (place < keep) continue;
-    }
-    drop((int)(e[pos] & IDX));
-  }
-}
 
 // Forward sweep over batches b0 .. b1, one block.  Shared memory: [cached ids | later the lists of a step][entries of the
 // selection], `cap` words each, then bitmaps.  What a batch costs is the walk over all of its candidates, twice (into the
@@ -535,7 +307,7 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
     }
     __syncthreads();
     if (keep < n)
-      select_first(s_ent, n, keep, left, right, s_list, s_tot, &s_place,
+      select_by_order<false>(s_ent, n, keep, left, right, s_list, s_tot, &s_place,
                    [&](int i) { atomicAnd(&s_kept[i >> 5].bits, ~(1u << (i & 31))); });
     __syncthreads();
     count_words(s_kept, n_words, (int32_t *)s_tot);

@@ -7,6 +7,7 @@ namespace orca {
 namespace lists {
 
 constexpr int T = tie::T, NW = tie::NW;
+constexpr int CAP = tie::SHARED_MAX;      // entries of a list that is selected from
 
 // The distinct nodes of every batch in ascending order, batch b's from b * stride: its endpoints (TARGET set) and the
 // out-of-batch neighbours of its table.
@@ -37,8 +38,233 @@ inline int64_t scratch_bytes(int64_t n_batches, int64_t n_nodes) {
 int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
                        const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init, cudaStream_t s);
 
+// An entry of a selection: key and place in its list.
+constexpr int KEY_BITS = 16, IDX_BITS = 14;
+constexpr uint32_t FAR = (1u << KEY_BITS) - 1, IDX = (1u << IDX_BITS) - 1;    // FAR: the largest key
+static_assert(CAP <= 1 << IDX_BITS && KEY_BITS + IDX_BITS <= 32, "an entry is a word");
+
+// Bitmaps over places of a list, with the number of bits before each word.
+struct Word {
+  uint32_t bits;
+  int32_t before;
+};
+// Fills `before` in; returns the number of bits.  All T threads, n <= T words, behind a barrier; ends with one.
+__device__ __forceinline__ int count_words(Word *w, int n, int32_t *s_w) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = tid < n ? __popc(w[tid].bits) : 0;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) s_w[warp] = incl;
+  __syncthreads();
+  const int x = s_w[lane];
+  const int before = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0), all = __reduce_add_sync(0xffffffffu, x);
+  if (tid < n) w[tid].before = before + incl - c;
+  __syncthreads();
+  return all;
+}
+__device__ __forceinline__ bool bit_of(Word w, int i) { return (w.bits >> (i & 31)) & 1u; }
+__device__ __forceinline__ int bits_before(Word w, int i) { return w.before + __popc(w.bits & ((1u << (i & 31)) - 1u)); }
+// the place of bit number m (there are more than m)
+__device__ __forceinline__ int bit_number(const Word *w, int n, int m) {
+  int lo = 0, hi = n;      // the last word with no more than m bits before it
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (w[mid].before <= m) lo = mid;
+    else hi = mid;
+  }
+  uint32_t bits = w[lo].bits;
+  m -= w[lo].before;
+  int at = 0;
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+    const int c = __popc(bits & ((1u << half) - 1u));
+    if (m >= c) m -= c, at += half, bits >>= half;
+  }
+  return 32 * lo + at;
+}
+
+// Numba's quicksort on a range [lo, hi] of equal keys: the place of the entry that ends up at place y.  A step parks the
+// middle entry at the end, turns the others round and puts it back in the middle; ranges of fewer than 16 stay as they
+// are.  So: down to the range in which y stays, and back through the steps.
+__device__ __forceinline__ int source_of_equal(int y, int lo, int hi) {
+  constexpr int DEPTH = 11;      // (the range is halved: no longer than 2^DEPTH * 15)
+  static_assert(CAP <= 15 << DEPTH, "");
+  int l[DEPTH], h[DEPTH], d = 0;
+  bool there = false;
+#pragma unroll
+  for (int i = 0; i < DEPTH; ++i) {
+    l[i] = lo, h[i] = hi;
+    const int mid = (lo + hi) >> 1;
+    there |= hi - lo < 15 || y == mid;
+    if (!there) {
+      d = i + 1;
+      if (y < mid) hi = mid - 1;
+      else lo = mid + 1;
+    }
+  }
+  int q = y;
+#pragma unroll
+  for (int i = DEPTH - 1; i >= 0; --i)
+    if (i < d) {
+      const int mid = (l[i] + h[i]) >> 1;
+      if (q == h[i]) q = mid;
+      q = l[i] + h[i] - 1 - q;
+      if (q == mid) q = h[i];
+    }
+  return q;
+}
+
+// Calls f(index) for the entries of e[0 .. n) (key << IDX_BITS | index, in list order) that numba's argsort leaves at
+// `keep` or behind, 0 < keep < n (FIRST: for those before `keep`; no key is FAR then): its steps on the range that contains the line, until that range is
+// short or its keys are equal.  left, right: [n]; words: [(n + 31) / 32].  All T threads; no barrier at the end.
+//
+// A step whose pivot is the largest key there is, FAR, is the usual one, and needs no swap: its left list is the FAR
+// entries, its right list everything, so that the m-th FAR entry from the left goes to place hi - 1 - m for as long as it
+// lies left of that, and these places are the right part.
+template <bool FIRST, class F>
+__device__ __forceinline__ void select_by_order(uint32_t *e, int n, int keep, uint16_t *left, uint16_t *right, Word *words,
+                                             uint32_t *s_tot, int32_t *s_place, F f) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const auto key = [&](int i) { return e[i] >> IDX_BITS; };
+  const auto swap = [&](int i, int j) { const uint32_t x = e[i]; e[i] = e[j]; e[j] = x; };
+  const auto park = [&](int lo, int hi) {
+    const int mid = (lo + hi) >> 1;
+    uint32_t a = e[lo], c = e[mid], d = e[hi], t;
+    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
+    if (d >> IDX_BITS < c >> IDX_BITS) t = d, d = c, c = t;
+    if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
+    e[lo] = a, e[mid] = d, e[hi] = c;
+  };
+  int lo = 0, hi = n - 1;
+  bool line = true, equal = false;      // the line falls into [lo, hi]; all its keys are equal
+  if (hi - lo >= 15) {
+    if (tid == 0) park(lo, hi);
+    __syncthreads();
+  }
+  while (line && !equal && hi - lo >= 15) {
+    const uint32_t p = key(hi);
+    if (!FIRST && p == FAR) {
+      // FAR entries of [lo, hi), a bit each; their number before every word
+      const int len = hi - lo, n_words = (len + 31) / 32;
+#pragma unroll 4
+      for (int i0 = warp * 32; i0 < len; i0 += T) {
+        const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < len && key(lo + i0 + lane) == FAR);
+        if (lane == 0) words[i0 >> 5].bits = w;
+      }
+      if (tid == 0) *s_place = 0;
+      __syncthreads();
+      count_words(words, n_words, (int32_t *)s_tot);
+      // swaps of the step: entry m at i swaps while i + m < len - 1, which grows from entry to entry
+      if (tid < n_words) {
+        uint32_t w = words[tid].bits;
+        const int first = 32 * tid + words[tid].before;
+        if (w != 0 && first + 31 - __clz(w) + __popc(w) - 1 >= len - 1) {     // (the word's last one does not)
+          int c = 0;
+          for (; w != 0 && first + __ffs(w) - 1 + c < len - 1; w &= w - 1) ++c;
+          w = (1u << c) - 1u;
+        }
+        if (w != 0) atomicAdd(s_place, __popc(w));
+      }
+      __syncthreads();
+      const int swaps = *s_place, mid = len - 1 - swaps;
+      // the pivot's place: the middle, if a FAR entry that need not swap lies there, else where the right part begins
+      bool stays = false;
+      if (mid >= 0 && mid < len) {
+        const Word w = words[mid >> 5];
+        stays = bit_of(w, mid) && bits_before(w, mid) == swaps;
+      }
+      const int m = lo + (stays ? mid : len - swaps);
+      if (keep > m + 1) {
+        // the right part: its places hi - 1, hi - 2, ... hold the first FAR entries, place hi the one after them
+        for (int y = keep + tid; y <= hi; y += T) {
+          const int q = source_of_equal(y, m + 1, hi);
+          f((int)(e[lo + bit_number(words, n_words, q == hi ? hi - m - 1 : hi - 1 - q)] & IDX));
+        }
+        for (int pos = hi + 1 + tid; pos < n; pos += T) f((int)(e[pos] & IDX));
+        return;      // (the parked entry is the pivot, at m: it stays)
+      }
+      __syncthreads();      // (s_place)
+    }
+    const int len = hi - lo, items = (len + T - 1) / T, first = lo + warp * 32 * items + lane;
+    uint32_t fl = 0, fr = 0, at = 0;
+    for (int i = 0; i < items; ++i) {
+      const int pos = first + 32 * i;
+      const uint32_t kv = pos < hi ? key(pos) : 0;
+      const bool l = pos < hi && kv >= p, r = pos < hi && kv <= p;
+      fl |= (l ? 1u : 0u) << i;
+      fr |= (r ? 1u : 0u) << i;
+      at += __popc(__ballot_sync(0xffffffffu, l)) | __popc(__ballot_sync(0xffffffffu, r)) << 16;
+    }
+    if (lane == 0) s_tot[warp] = at;
+    __syncthreads();
+    const uint32_t t = s_tot[lane], all = __reduce_add_sync(0xffffffffu, t);
+    at = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
+    const int nl = all & 0xffff, nr = all >> 16;
+    if (nl == len && nr == len) {       // (uniform over the block)
+      __syncthreads();
+      if (tid == 0) swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
+      equal = true;
+      break;
+    }
+    for (int i = 0; i < items; ++i) {
+      const int pos = first + 32 * i;
+      const bool l = (fl >> i) & 1u, r = (fr >> i) & 1u;
+      const uint32_t ml = __ballot_sync(0xffffffffu, l), mr = __ballot_sync(0xffffffffu, r);
+      if (l) left[(at & 0xffff) + __popc(ml & lt)] = (uint16_t)pos;
+      if (r) right[(at >> 16) + __popc(mr & lt)] = (uint16_t)pos;
+      at += __popc(ml) | __popc(mr) << 16;
+    }
+    __syncthreads();
+    // the m-th of the left list swaps with the m-th from the end of the right list while it lies left of it
+    const int pairs = min(nl, nr);
+    for (int m = tid; m < pairs; m += T) {
+      const int pl = left[m], pr = right[nr - 1 - m];
+      if (pl >= pr) {
+        if (m == 0) *s_place = pl;
+        break;                          // (behind a pair that does not swap, none does)
+      }
+      const int next_l = m + 1 < nl ? (int)left[m + 1] : hi;
+      if (m + 1 >= pairs || next_l >= (int)right[nr - 2 - m]) *s_place = min(next_l, pr);
+      swap(pl, pr);
+    }
+    if (tid == 0 && pairs == 0) *s_place = nl > 0 ? (int)left[0] : hi;
+    __syncthreads();
+    const int m = *s_place;             // the pivot's place
+    const int old_hi = hi;
+    if (keep <= m) {
+      line = keep > lo && keep < m;     // (keep == m: the left part stays, the rest goes)
+      hi = m - 1;
+      if (!line) lo = keep, hi = keep - 1;
+    } else {
+      line = keep > m + 1;
+      lo = m + 1;
+      if (!line) hi = lo - 1;
+    }
+    if (tid == 0) {
+      swap(m, old_hi);
+      if (line && !equal && hi - lo >= 15) park(lo, hi);
+    }
+    __syncthreads();
+  }
+  if (equal) __syncthreads();           // (the entries of the undone step)
+  if (equal) {
+    for (int y = (FIRST ? lo : keep) + tid; y < (FIRST ? keep : hi + 1); y += T) f((int)(e[source_of_equal(y, lo, hi)] & IDX));
+  } else if (lo + tid <= hi) {          // (fewer than 16)
+    const int pos = lo + tid;
+    const uint32_t k = key(pos);
+    int place = lo;
+    for (int q = lo; q <= hi; ++q) place += key(q) < k || (key(q) == k && q < pos) ? 1 : 0;
+    if ((place < keep) == FIRST) f((int)(e[pos] & IDX));
+  }
+  for (int pos = (FIRST ? 0 : hi + 1) + tid; pos < (FIRST ? lo : n); pos += T) f((int)(e[pos] & IDX));
+}
+
 // MRD over lists.  Candidate lists longer than CAP set *State::failed: the kernels of planner_mrd.cu do the plan then.
-constexpr int CAP = tie::SHARED_MAX;
 bool mrd_takes(int64_t n_edges, int32_t bs);
 int64_t mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget);
 int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,

@@ -5,17 +5,19 @@
 // consumes depends on the numbers (rejection sampling), but not on what is shuffled: one warp takes the generator's
 // numbers 32 at a time and finds by votes which of them are accepted and for which swap.  The swaps themselves are one
 // serial chain, in shared memory, and are left out where the whole list is taken whatever its order.
-// The rest is data parallel over the block: the split of the batch's neighbour table into targets / out-of-batch
-// neighbours (stamps; eight entries a thread at a time, so that their loads overlap), the reuse statistics, sets as
-// bitmaps that list their members in ascending order by a popcount scan (np.unique / np.where of the reference), and
-// the LRU evictions, which are the first entries of numba's argsort of the last-use times (tie_shared.cuh, or
-// tie_order.cuh for lists that do not fit shared memory).
+// The out-of-batch neighbours of all batches, without duplicates, are listed before (planner_lists.cu).  The rest is data
+// parallel over the block: the reuse statistics, sets as bitmaps that list their members in ascending order by a popcount
+// scan (np.where of the reference), and the LRU evictions, which are the first entries of numba's argsort of the
+// last-use times: only which they are matters, so only the range that the line falls into is partitioned
+// (planner_lists.cuh; tie_order.cuh for lists that do not fit shared memory).
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
-// 250 batches of 600 edges with 20 neighbours, LRU: 19.2 ms a plan with draws, swaps, bitmaps and sort
-// in global memory, 12.1 to 12.4 here.
+// 250 batches of 600 edges with 20 neighbours, LRU, ms of the kernel: 19.2 with draws, swaps, bitmaps and sort in global
+// memory, 9.9 with those in shared memory, 3.8 with lists in place of the tables' 24,000 entries a batch and without the
+// levels of the sort that do not decide.
 #include <algorithm>
 
 #include "common.cuh"
+#include "planner_lists.cuh"
 #include "tie_shared.cuh"
 
 namespace orca {
@@ -86,14 +88,15 @@ struct Twister {
 };
 
 struct Work {
-  int32_t *stamp;                 // [n_nodes] last batch in which the node was a target
+  lists::Lists lists;
   int32_t *t0, *t1, *t2;          // [n_nodes] LRU: last use, arrival; 2Q: LRU last use, LRU arrival, FIFO arrival
-  uint32_t *bm[5];                // [words] LRU: cached, candidates; 2Q: fifo, lru, promote, fresh, touched
+  uint32_t *bm[2];                // [words] LRU: cached; 2Q: fifo, lru
   int32_t *list[4];               // [cap] member lists
   tie::Buf sort;
   int64_t cap;
   int cap_shared;                 // entries of a list in shared memory
-  bool bm_shared;                 // the bitmaps, and one of the targets in place of the stamps, lie behind them
+  bool bm_shared;                 // the bitmaps lie behind them
+  bool keys_fit;                  // a batch's number is a key of a selection (planner_lists.cuh)
 };
 
 // (bitmaps lie in shared memory where they fit, else in global memory, where their words are changed by atomics, which
@@ -175,18 +178,23 @@ __device__ void shuffle(const Work &w, Twister &rng, int32_t *x, int n, bool any
   __syncthreads();
 }
 
-// the first `count` entries of numba's argsort of key[ids[i]] (i < n): calls f(id) for each of them
+// the first `count` entries, fewer than n, of numba's argsort of key[ids[i]] (i < n): calls f(id) for each of them
 template <class F>
 __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int count, const int32_t *key, int *s_a,
                                  int *s_b, F f) {
-  if (n <= w.cap_shared) {
-    const tie::Shared sh{w.cap_shared};
-    for (int i = threadIdx.x; i < n; i += T) {
-      sh.key(i) = key[ids[i]];
-      sh.idx(i) = (uint16_t)i;
-    }
-    const auto use = [&](int, int i) { f(ids[i]); };
-    tie::sort_first_shared(sh, (uint32_t *)s_a, n, count, use);
+  if (count >= n) {
+    for (int i = threadIdx.x; i < n; i += T) f(ids[i]);
+    __syncthreads();
+    return true;
+  }
+  if (n <= w.cap_shared && w.keys_fit) {
+    uint32_t *e = (uint32_t *)tie::smem;
+    uint16_t *left = (uint16_t *)(e + w.cap_shared), *right = left + w.cap_shared;
+    for (int i = threadIdx.x; i < n; i += T) e[i] = (uint32_t)key[ids[i]] << lists::IDX_BITS | (uint32_t)i;
+    __syncthreads();
+    lists::select_by_order<true>(e, n, count, left, right, (lists::Word *)(right + w.cap_shared), (uint32_t *)s_a, s_b,
+                                 [&](int i) { f(ids[i]); });
+    __syncthreads();
     return true;
   }
   for (int i = threadIdx.x; i < n; i += T) w.sort.e[i] = ((uint64_t)(uint32_t)key[ids[i]] << 32) | (uint32_t)i;
@@ -198,49 +206,51 @@ __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int c
   return true;
 }
 
-// The bitmaps of a plan (SH: in shared memory, behind the lists); one more for the targets of a batch if so.
-constexpr int N_BM = 5;
+// The bitmaps of a plan (SH: in shared memory, behind the lists).
+constexpr int N_BM = 2;
 template <bool SH>
 __device__ __forceinline__ uint32_t *bitmap(const Work &w, int i, int64_t words) {
   return SH ? (uint32_t *)(tie::smem + tie::Shared::BYTES * w.cap_shared) + i * words : w.bm[i];
 }
 template <bool SH>
 __device__ void clear_bitmaps(const Work &w, int64_t words) {
-  for (int64_t i = threadIdx.x; i < (SH ? N_BM + 1 : N_BM) * words; i += T)
-    bitmap<SH>(w, SH ? 0 : (int)(i / words), words)[SH ? i : i % words] = 0;
+  for (int64_t i = threadIdx.x; i < N_BM * words; i += T) bitmap<SH>(w, (int)(i / words), words)[i % words] = 0;
 }
 
-// Calls use(v, load(v)) for the out-of-batch entries of a batch's neighbour table, eight entries a thread at a time.
-// Most entries are targets or padding: `load` is left to the others, since one block's scattered loads are what this
-// phase waits for.
-constexpr int STEP = 8;
-template <bool SH, class Load, class Use>
-__device__ __forceinline__ void for_neighbors(const Work &w, uint32_t *target, const int32_t *q, int m2, const int32_t *tab, int n,
-                              int32_t now, Load load, Use use) {
-  for (int i = threadIdx.x; i < m2; i += T) {
-    if (SH) set_bit(target, q[i]);
-    else w.stamp[q[i]] = now;
+// Deals the out-of-batch neighbours of a batch out to three lists: kind(v, entries of the table) says which (0 .. 2, else
+// none).  The lists stay in ascending order; n: their lengths, the same in every thread.  s_cnt: NW words.  All T threads;
+// ends behind a barrier.
+template <class Kind>
+__device__ __forceinline__ void deal_neighbors(const lists::Lists &l, int64_t b, int32_t *const (&out)[3], int (&n)[3],
+                                               uint32_t *s_cnt, Kind kind) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int n_list = l.count[b];
+  const int32_t *id = l.id + b * l.stride, *mult = l.mult + b * l.stride;
+  n[0] = n[1] = n[2] = 0;
+  for (int i0 = 0; i0 < n_list; i0 += T) {
+    const int i = i0 + tid;
+    const int32_t v = i < n_list ? id[i] : lists::TARGET;
+    const int k = v >= 0 ? kind(v, mult[i]) : 3;
+    uint32_t m[3], c = 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      m[j] = __ballot_sync(0xffffffffu, k == j);
+      c |= __popc(m[j]) << 10 * j;       // (32 at most)
+    }
+    __syncthreads();      // (s_cnt of the turn before)
+    if (lane == 0) s_cnt[warp] = c;
+    __syncthreads();
+    const uint32_t x = s_cnt[lane];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int mine = (x >> 10 * j) & 1023u;
+      const int before = __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
+      if (k == j) out[j][n[j] + before + __popc(m[j] & lt)] = v;
+      n[j] += __reduce_add_sync(0xffffffffu, mine);
+    }
   }
   __syncthreads();
-  for (int i0 = threadIdx.x; i0 < n; i0 += STEP * T) {
-    int32_t v[STEP];
-    bool out[STEP];
-    decltype(load(0)) x[STEP];
-#pragma unroll
-    for (int u = 0; u < STEP; ++u) v[u] = i0 + u * T < n ? tab[i0 + u * T] : 0;
-#pragma unroll
-    for (int u = 0; u < STEP; ++u) out[u] = v[u] != 0 && !(SH ? bit(target, v[u]) : w.stamp[v[u]] == now);
-#pragma unroll
-    for (int u = 0; u < STEP; ++u)
-      if (out[u]) x[u] = load(v[u]);
-#pragma unroll
-    for (int u = 0; u < STEP; ++u)
-      if (out[u]) use(v[u], x[u]);
-  }
-  if (SH) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < m2; i += T) target[q[i] >> 5] = 0;
-  }
 }
 
 struct Totals {
@@ -262,21 +272,18 @@ __device__ void write_totals(const Totals &t, int64_t *stats) {
 
 // ------------------------------------------------------------------------------ LRU (utils/cache.py:338-403)
 template <bool SH>
-__global__ void __launch_bounds__(T, 1) lru_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
-                                                int32_t k, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
+__global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
                                                 int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
                                                 int32_t *status) {
   __shared__ Twister rng;
   __shared__ int s_a[NW], s_b[NW];
   const int tid = threadIdx.x;
-  const int64_t nb = (n_edges + bs - 1) / bs, words = (n_nodes + 31) / 32;
+  const int64_t words = (n_nodes + 31) / 32;
   clear_bitmaps<SH>(w, words);
-  uint32_t *cached = bitmap<SH>(w, 0, words), *candbm = bitmap<SH>(w, 1, words);
-  uint32_t *target = SH ? bitmap<SH>(w, N_BM, words) : nullptr;
+  uint32_t *cached = bitmap<SH>(w, 0, words);
   int32_t *used_at = w.t0, *arrived = w.t1;
   int32_t *cand = w.list[0], *held = w.list[1];
   for (int64_t v = tid; v < n_nodes; v += T) {
-    w.stamp[v] = -1;
     used_at[v] = 0;
     arrived[v] = 0;
   }
@@ -284,24 +291,21 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(const int32_t *nodes, const i
   __syncthreads();
   Totals tot;
   int64_t used = 0;
+  int n_held = 0;      // members of `cached`, listed in `held`
   for (int64_t b = 0; b < nb; ++b) {
-    const int64_t s = b * bs;
-    const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
-    const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
-    for_neighbors<SH>(w, target, q, m2, tab, m2 * k, (int32_t)b,
-                  [&](int32_t v) { return make_int2((int)bit(cached, v), arrived[v]); },
-                  [&](int32_t v, int2 x) {
-                    if (x.x) {
-                      ++tot.reuse;
-                      tot.dist += b - x.y;
-                      used_at[v] = (int32_t)b;
-                    } else {
-                      ++tot.recompute;
-                      set_bit(candbm, v);
-                    }
-                  });
-    const int n_cand = list_members(candbm, words, cand, true, s_a);
-    const int n_held = list_members(cached, words, held, false, s_a);
+    int32_t *const out[3] = {cand, nullptr, nullptr};
+    int n[3];
+    deal_neighbors(w.lists, b, out, n, (uint32_t *)s_a, [&](int32_t v, int m) {
+      if (!bit(cached, v)) {
+        tot.recompute += m;
+        return 0;
+      }
+      tot.reuse += m;
+      tot.dist += (b - arrived[v]) * m;
+      used_at[v] = (int32_t)b;
+      return 3;
+    });
+    const int n_cand = n[0];
     const int room = budget - n_held;
     const int evict = room >= n_cand ? 0 : min(n_cand - room, n_held);
     const int take = (evict + room >= n_cand) ? n_cand : budget;
@@ -318,14 +322,14 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(const int32_t *nodes, const i
       set_bit(cached, v);
       used_at[v] = arrived[v] = (int32_t)b;
     }
-    const int n_plan = list_members(cached, words, held, false, s_a);
-    if (used + n_plan > plan_cap) {
+    n_held = list_members(cached, words, held, false, s_a);
+    if (used + n_held > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       break;
     }
-    for (int i = tid; i < n_plan; i += T) plan[used + i] = held[i];
+    for (int i = tid; i < n_held; i += T) plan[used + i] = held[i];
     if (tid == 0) plan_off[b] = used;
-    used += n_plan;
+    used += n_held;
     __syncthreads();
   }
   write_totals(tot, stats);
@@ -335,23 +339,19 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(const int32_t *nodes, const i
 // ------------------------------------------------------------------------------ 2Q (utils/cache.py:175-333)
 // a FIFO half and an LRU half of budget / 2 entries each
 template <bool SH>
-__global__ void __launch_bounds__(T, 1) twoq_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
-                                                 int32_t k, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
+__global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t nb, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
                                                  int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
                                                  int32_t *status) {
   __shared__ Twister rng;
   __shared__ int s_a[NW], s_b[NW];
   const int tid = threadIdx.x;
-  const int64_t nb = (n_edges + bs - 1) / bs, words = (n_nodes + 31) / 32;
+  const int64_t words = (n_nodes + 31) / 32;
   const int half = budget / 2;
   clear_bitmaps<SH>(w, words);
-  uint32_t *fifo = bitmap<SH>(w, 0, words), *lru = bitmap<SH>(w, 1, words), *promote_bm = bitmap<SH>(w, 2, words);
-  uint32_t *fresh_bm = bitmap<SH>(w, 3, words), *touched_bm = bitmap<SH>(w, 4, words);
-  uint32_t *target = SH ? bitmap<SH>(w, N_BM, words) : nullptr;
+  uint32_t *fifo = bitmap<SH>(w, 0, words), *lru = bitmap<SH>(w, 1, words);
   int32_t *lru_used = w.t0, *lru_arr = w.t1, *fifo_arr = w.t2;
   int32_t *promote = w.list[0], *fresh = w.list[1], *touched = w.list[2], *ids = w.list[3];
   for (int64_t v = tid; v < n_nodes; v += T) {
-    w.stamp[v] = -1;
     lru_used[v] = lru_arr[v] = fifo_arr[v] = 0;
   }
   if (tid == 0) rng.seed(seed);
@@ -362,28 +362,23 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(const int32_t *nodes, const 
   bool failed = false;
   for (int64_t b = 0; b < nb && !failed; ++b) {
     const int32_t now = (int32_t)b;
-    const int64_t s = b * bs;
-    const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
-    const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
-    for_neighbors<SH>(w, target, q, m2, tab, m2 * k, now,
-                  [&](int32_t v) { return make_int4((int)bit(fifo, v), (int)bit(lru, v), fifo_arr[v], lru_arr[v]); },
-                  [&](int32_t v, int4 x) {
-                    if (x.x) {
-                      ++tot.reuse;
-                      tot.dist += now - x.z;
-                      set_bit(promote_bm, v);
-                    } else if (x.y) {
-                      ++tot.reuse;
-                      tot.dist += now - x.w;
-                      set_bit(touched_bm, v);
-                    } else {
-                      ++tot.recompute;
-                      set_bit(fresh_bm, v);
-                    }
-                  });
-    const int n_promote = list_members(promote_bm, words, promote, true, s_a);
-    const int n_fresh = list_members(fresh_bm, words, fresh, true, s_a);
-    const int n_touched = list_members(touched_bm, words, touched, true, s_a);
+    int32_t *const out[3] = {promote, fresh, touched};
+    int n_out[3];
+    deal_neighbors(w.lists, b, out, n_out, (uint32_t *)s_a, [&](int32_t v, int m) {
+      if (bit(fifo, v)) {
+        tot.reuse += m;
+        tot.dist += (long long)(now - fifo_arr[v]) * m;
+        return 0;
+      }
+      if (bit(lru, v)) {
+        tot.reuse += m;
+        tot.dist += (long long)(now - lru_arr[v]) * m;
+        return 2;
+      }
+      tot.recompute += m;
+      return 1;
+    });
+    const int n_promote = n_out[0], n_fresh = n_out[1], n_touched = n_out[2];
     // ---- FIFO half
     const int fifo_kept = n_fifo - n_promote, fifo_room = half - fifo_kept;
     for (int i = tid; i < n_promote; i += T) clear_bit(fifo, promote[i]);
@@ -472,9 +467,9 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(const int32_t *nodes, const 
 }
 
 struct Layout {
-  int64_t stamp, t[3], bm[5], list[4], sort, total, cap;
+  int64_t id, mult, count, scratch, t[3], bm[N_BM], list[4], sort, total, cap;
 };
-static Layout layout(int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
+static Layout layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
   Layout L;
   const int64_t words = (n_nodes + 31) / 32;
   L.cap = std::max<int64_t>(2ll * bs * k, budget) + 64;
@@ -484,9 +479,13 @@ static Layout layout(int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
     at += (bytes + 255) & ~255ll;
     return o;
   };
-  L.stamp = take(n_nodes * 4);
+  const int64_t nb = (n_edges + bs - 1) / bs, stride = lists::stride_of(bs, k, n_nodes);
+  L.id = take(nb * stride * 4);
+  L.mult = take(nb * stride * 4);
+  L.count = take(nb * 4);
+  L.scratch = take(lists::scratch_bytes(nb, n_nodes));
   for (int i = 0; i < 3; ++i) L.t[i] = take(n_nodes * 4);
-  for (int i = 0; i < 5; ++i) L.bm[i] = take(words * 4);
+  for (int i = 0; i < N_BM; ++i) L.bm[i] = take(words * 4);
   for (int i = 0; i < 4; ++i) L.list[i] = take(L.cap * 4);
   L.sort = take(tie::buf_bytes(L.cap) + 7 * 256);
   L.total = at;
@@ -508,7 +507,7 @@ extern "C" int64_t orca_plan_device_workspace_bytes(int32_t strategy, int64_t n_
                                                     int64_t n_nodes, int32_t budget) {
   if (strategy == 0) return orca_plan_mrd_workspace_bytes(n_edges, bs, k, n_nodes, budget);
   if (strategy < 0 || strategy > 2 || n_edges < 0 || bs <= 0 || k < 1 || n_nodes <= 0 || budget <= 0) return -1;
-  return rnd::layout(bs, k, n_nodes, budget).total;
+  return rnd::layout(n_edges, bs, k, n_nodes, budget).total;
 }
 
 extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k,
@@ -523,17 +522,20 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
   ORCA_CHECK_ARG(n_edges >= 0 && bs > 0 && k >= 1 && k <= ORCA_MAX_K && n_nodes > 0 && budget > 0);
   ORCA_CHECK_ARG(n_nodes < (1ll << 31) && (n_edges + bs - 1) / bs < (1ll << 30) && 2ll * bs * k < (1ll << 30));
   ORCA_CHECK_ARG(((uintptr_t)d_workspace & 255) == 0);
-  const rnd::Layout L = rnd::layout(bs, k, n_nodes, budget);
+  const rnd::Layout L = rnd::layout(n_edges, bs, k, n_nodes, budget);
   if (workspace_bytes < L.total)
     return set_error(ORCA_E_CAPACITY, "orca_plan_device: workspace of %lld bytes, %lld needed",
                      (long long)workspace_bytes, (long long)L.total);
   char *base = (char *)d_workspace;
   rnd::Work w;
-  w.stamp = (int32_t *)(base + L.stamp);
+  const int64_t nb = (n_edges + bs - 1) / bs;
+  w.lists.id = (int32_t *)(base + L.id), w.lists.mult = (int32_t *)(base + L.mult);
+  w.lists.count = (int32_t *)(base + L.count), w.lists.stride = lists::stride_of(bs, k, n_nodes);
+  w.keys_fit = nb < (int64_t)lists::FAR;
   w.t0 = (int32_t *)(base + L.t[0]);
   w.t1 = (int32_t *)(base + L.t[1]);
   w.t2 = (int32_t *)(base + L.t[2]);
-  for (int i = 0; i < 5; ++i) w.bm[i] = (uint32_t *)(base + L.bm[i]);
+  for (int i = 0; i < rnd::N_BM; ++i) w.bm[i] = (uint32_t *)(base + L.bm[i]);
   for (int i = 0; i < 4; ++i) w.list[i] = (int32_t *)(base + L.list[i]);
   w.cap = L.cap;
   {
@@ -552,12 +554,11 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
     w.sort.swaps = (int32_t *)take(2 * L.cap * 4);
     w.sort.cap = L.cap;
   }
-  // Shared memory: lists first, then six bitmaps where they fit (up to some 200,000 nodes: each of their scattered reads
-  // costs a trip to L2 otherwise).  The lists that are sorted are no longer than the budget; more room than for those,
-  // or for the shuffles of 7000 entries, only takes L1 from the table entries' loads (the same time with room for
-  // every node here).
+  // Shared memory: lists first, then two bitmaps where they fit (up to some 600,000 nodes: each of their scattered reads
+  // costs a trip to L2 otherwise).  The lists that are selected from are no longer than the budget; there is room for
+  // those, and for the shuffles of 7000 entries.
   constexpr int64_t per = tie::Shared::BYTES, most = per * tie::SHARED_MAX;
-  const int64_t bitmaps = (rnd::N_BM + 1) * ((n_nodes + 31) / 32) * 4;
+  const int64_t bitmaps = rnd::N_BM * ((n_nodes + 31) / 32) * 4;
   w.cap_shared = (int)((std::min({L.cap, n_nodes, std::max<int64_t>(budget, 4096), (int64_t)tie::SHARED_MAX}) + 15) & ~15ll);
   if (per * w.cap_shared + bitmaps > most && per * (budget + 16ll) + bitmaps <= most)
     w.cap_shared = (int)(((most - bitmaps) / per) & ~15ll);
@@ -572,7 +573,9 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
   auto kernel = strategy == 1 ? (w.bm_shared ? rnd::lru_kernel<true> : rnd::lru_kernel<false>)
                               : (w.bm_shared ? rnd::twoq_kernel<true> : rnd::twoq_kernel<false>);
   ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kernel<<<1, rnd::T, smem, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, seed, w, d_plan_flat, plan_cap,
+  const int rc = lists::launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, w.lists, base + L.scratch, nullptr, 0, s);
+  if (rc != ORCA_OK) return rc;
+  kernel<<<1, rnd::T, smem, s>>>(nb, n_nodes, budget, seed, w, d_plan_flat, plan_cap,
                                  d_plan_off, d_stats, d_status);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
