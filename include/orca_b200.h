@@ -583,6 +583,9 @@ typedef struct {
   int32_t nb, bs, b_last;     /* batches of this group; edges of a batch and of the group's last one */
   int32_t nb_max, u_cap, plan_cap; /* most batches of a group, most uncached neighbours and plan entries of a batch */
   int32_t *h_status;          /* page-locked, may be NULL: four words, the status word as phase 2 leaves it */
+  /* optional: link-prediction metrics of the group's batches, orca_link_metric_parts(bs) records of four doubles each a
+   * batch; see orca_link_metrics_of_parts */
+  double *d_metrics, *h_metrics;
 } orca_group_t;
 /* batches worth putting into one group */
 int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode);
@@ -595,6 +598,10 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
  * batch i covers edges [i * bs, (i + 1) * bs), h_out[3 * i .. 3 * i + 2] = {AP, AUC, share of edges with
  * pos >= neg}.  Host memory only; a score that is not finite is ORCA_E_BADARG. */
 int orca_link_metrics(const float *h_pos, const float *h_neg, int64_t n_edges, int32_t bs, double *h_out);
+/* The same from the records that orca_tgn_eval_group leaves (h_metrics): sums over parts of a batch.
+ * orca_link_metric_parts: records a batch, 0 for batches that are too large to be evaluated on the device. */
+int32_t orca_link_metric_parts(int32_t bs);
+int orca_link_metrics_of_parts(const double *h_parts, int64_t n_edges, int32_t bs, double *h_out);
 
 /* Sharing the exchange buffer of the multi-GPU split between the processes of one node (no counterpart
  * in the reference).  orca_ipc_export: the 64-byte CUDA IPC handle of the allocation that holds d_ptr and

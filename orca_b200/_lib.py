@@ -91,7 +91,7 @@ class CallT(C.Structure):
 class GroupT(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("h_i32", "h_ts", "off_i32", "n_plan", "h_rows")] + [("seq", C.c_int64)] + \
         [(n, C.c_int32) for n in ("phase", "nb", "bs", "b_last", "nb_max", "u_cap", "plan_cap")] + \
-        [("h_status", C.c_void_p)]
+        [(n, C.c_void_p) for n in ("h_status", "d_metrics", "h_metrics")]
 
 
 # every symbol the header declares: name -> (restype, argtypes)
@@ -147,6 +147,8 @@ SYMBOLS = {
     "orca_group_workspace_bytes": (_I64, [_I32, _I32, _I32, _I32, _I32, _I64, _I32, _I32]),
     "orca_tgn_eval_group": (C.c_int, [C.POINTER(TgnT), C.POINTER(GroupT), _V, _I64, _V, _V, _V, _V]),
     "orca_link_metrics": (C.c_int, [_V, _V, _I64, _I32, _V]),
+    "orca_link_metric_parts": (_I32, [_I32]),
+    "orca_link_metrics_of_parts": (C.c_int, [_V, _I64, _I32, _V]),
     "orca_stage_h2d": (C.c_int, [_V, _V, C.c_int64, _V]),
     "orca_ipc_export": (C.c_int, [_V, _V, C.POINTER(C.c_int64)]),
     "orca_ipc_open": (C.c_int, [_V, C.c_int64, C.POINTER(C.c_void_p)]),

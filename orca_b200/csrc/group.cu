@@ -498,6 +498,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   ORCA_CHECK_ARG(m && g && d_workspace && d_prob && d_status && g->h_i32 && g->h_ts && g->off_i32 && g->n_plan);
   ORCA_CHECK_ARG(g->nb > 0 && g->nb <= g->nb_max && g->nb_max <= grp::MAX_BATCHES && g->bs > 0 && g->b_last > 0 &&
                  g->b_last <= g->bs && g->u_cap >= 0 && g->h_rows && g->seq >= 0);
+  ORCA_CHECK_ARG(g->d_metrics == nullptr || (g->h_metrics && orca_link_metric_parts(g->bs) > 0));
   ORCA_CHECK_ARG((m->n_layers == 1 || m->n_layers == 2) && m->k >= 1 && m->k <= ORCA_MAX_K && m->world <= 1);
   const int layers = m->n_layers, k = m->k, mode = layers == 2 ? m->mode : ORCA_MODE_BUDGET;
   ORCA_CHECK_ARG(mode == ORCA_MODE_BUDGET || mode == ORCA_MODE_REUSE_ALL || mode == ORCA_MODE_NO_REUSE);
@@ -630,6 +631,11 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     ORCA_CUDA(launch_dep(grp::write_back_kernel, c->sm_count * 8, 256, 0, s, a, log, (const float *)w.emb1, m->mem.memory,
                          m->hist_emb, g->h_status));
     ORCA_COUNT_LAUNCH();
+    if (g->d_metrics != nullptr) {
+      ORCA_TRY(launch_link_metrics(d_prob, g->nb, g->bs, g->b_last, g->d_metrics, s));
+      ORCA_CUDA(cudaMemcpyAsync(g->h_metrics, g->d_metrics, (size_t)g->nb * orca_link_metric_parts(g->bs) * 4 * sizeof(double),
+                                cudaMemcpyDeviceToHost, s));
+    }
     if (h_prob != nullptr) ORCA_CUDA(cudaMemcpyAsync(h_prob, d_prob, (size_t)2 * E * 4, cudaMemcpyDeviceToHost, s));
     ORCA_CUDA(cudaEventRecord(c->ev_gdone[p], s));
     c->gdone_recorded[p] = true;

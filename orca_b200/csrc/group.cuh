@@ -143,4 +143,7 @@ __device__ __forceinline__ int history_row(const Args &a, int v, int n) {
 }
 
 }  // namespace grp
+
+// metrics.cu: records of a group's scores ([pos | neg] of batch n from n * 2 * bs)
+int launch_link_metrics(const float *d_prob, int nb, int bs, int b_last, double *d_out, cudaStream_t s);
 }  // namespace orca

@@ -4,9 +4,8 @@ stream, one uniform negative destination per positive edge drawn batch by batch 
 
 The reference calls the model once per batch and brings the scores back per batch; here the
 negatives of all batches are drawn first (same draws, same order: the sampler is consumed exactly as
-the reference consumes it) and the whole stream goes through ``TGN.eval_epoch`` -- one library call.
-The metrics are those of scikit-learn, per batch as in the reference, computed by the library
-(``orca_link_metrics``).
+the reference consumes it) and the whole stream goes through ``TGN.eval_epoch_metrics`` -- one call.
+The metrics are those of scikit-learn, per batch as in the reference, computed by the library.
 """
 from __future__ import annotations
 
@@ -15,6 +14,7 @@ import math
 import numpy as np
 
 from . import _lib
+from .tgn import TGN
 
 
 class RandEdgeSampler:
@@ -55,14 +55,18 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
     for i in range(nb):
         lo, hi = i * batch_size, min(n, (i + 1) * batch_size)
         negatives[lo:hi] = draw(hi - lo)
-    pos, neg = model.eval_epoch(data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n],
-                                data.edge_idxs[:n], n_neighbors, batch_size, cache_plan, reuse=reuse)
     # per batch, as the reference does; the positive "wins" when its score is not below the negative's
     # (evaluation/evaluation.py:39-40)
-    m = np.empty((nb, 3))
-    rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, batch_size, m.ctypes.data)
-    if rc == _lib.E_BADARG:
-        raise ValueError(_lib.lib().orca_last_error().decode())
-    _lib.check(rc)
+    stream = (data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n], data.edge_idxs[:n], n_neighbors,
+              batch_size, cache_plan)
+    if getattr(model.eval_epoch, "__func__", None) is TGN.eval_epoch:
+        m = model.eval_epoch_metrics(*stream, reuse=reuse)
+    else:       # (a model with an eval_epoch of its own: its scores count)
+        pos, neg = model.eval_epoch(*stream, reuse=reuse)
+        m = np.empty((nb, 3))
+        rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, batch_size, m.ctypes.data)
+        if rc == _lib.E_BADARG:
+            raise ValueError(_lib.lib().orca_last_error().decode())
+        _lib.check(rc)
     val_ap, val_auc, val_acc = np.mean(m, axis=0)
     return val_ap, val_auc, val_acc

@@ -763,6 +763,29 @@ class TGN(nn.Module):
         cache_plan: list with one id array per batch (or None: the plan-less flag rule).
         Returns (pos, neg): float32 numpy arrays with one score per edge.  Raises what the kernels of these or of
         earlier batches reported (ids outside a table, a bounded wait that gave up)."""
+        return self._eval_stream(sources, destinations, negatives, timestamps, edge_idxs, n_neighbors, batch_size,
+                                 cache_plan, reuse, False)
+
+    def eval_epoch_metrics(self, sources, destinations, negatives, timestamps, edge_idxs, n_neighbors, batch_size,
+                           cache_plan=None, reuse=True):
+        """The stream of eval_epoch, of which only the metrics of every batch are wanted (evaluation/evaluation.py:30-44):
+        an array of one row {average precision, ROC area, share of edges whose positive score is not below the negative
+        one's} per batch.  They are computed beside the scores, on the GPU, where the stream goes through groups."""
+        E, bs = len(sources), int(batch_size)
+        m = np.empty(((E + bs - 1) // bs, 3))
+        r = self._eval_stream(sources, destinations, negatives, timestamps, edge_idxs, n_neighbors, batch_size,
+                              cache_plan, reuse, True)
+        L = _lib.lib()
+        rc = L.orca_link_metrics(r[0].ctypes.data, r[1].ctypes.data, E, bs, m.ctypes.data) if isinstance(r, tuple) else \
+            L.orca_link_metrics_of_parts(r.ctypes.data, E, bs, m.ctypes.data)
+        if rc == _lib.E_BADARG:
+            raise ValueError(L.orca_last_error().decode())
+        _lib.check(rc)
+        return m
+
+    def _eval_stream(self, sources, destinations, negatives, timestamps, edge_idxs, n_neighbors, batch_size, cache_plan,
+                     reuse, metrics):
+        """eval_epoch's scores, or (metrics, where the stream goes through groups) records of orca_link_metrics_of_parts."""
         E = len(sources)
         bs, k = int(batch_size), int(n_neighbors)
         nb = (E + bs - 1) // bs
@@ -781,7 +804,7 @@ class TGN(nn.Module):
             if world == 1 and (cache_plan is not None or self._mode != MODE_BUDGET or self.n_layers == 1) and \
                     not any(self._options.get(o) for o in (_lib.OPT_PROJECTION_MODE, _lib.OPT_TRACE)):
                 return self._eval_groups(sources, destinations, negatives, timestamps, edge_idxs, k, bs,
-                                         cache_plan if self.n_layers == 2 else None)
+                                         cache_plan if self.n_layers == 2 else None, metrics)
             return self._eval_chunks(sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan)
         except BaseException:
             # (an array that cannot be packed, an allocation that fails: batches before it may be in flight, on the
@@ -914,7 +937,7 @@ class TGN(nn.Module):
             raise failed
         return pos, neg
 
-    def _eval_groups(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan):
+    def _eval_groups(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, cache_plan, metrics):
         """eval_epoch in groups of consecutive batches (orca_tgn_eval_group)."""
         L = _lib.lib()
         E = len(sources)
@@ -962,6 +985,11 @@ class TGN(nn.Module):
         stream = torch.cuda.current_stream(self.device)
         h_rows, h_status = pinned("rows", 2, torch.int32), self._status_buffer().data_ptr()
         groups = []
+        parts = 4 * L.orca_link_metric_parts(bs) if metrics else 0      # doubles a batch; 0: from the scores
+        if parts:
+            h_parts = pinned("parts", parts * nb, torch.float64)
+            if keep.get("d_parts") is None or keep["d_parts"].numel() < parts * nb:
+                keep["d_parts"] = torch.empty(parts * nb, dtype=torch.float64, device=self.device)
 
         def prepare(i0):
             i1 = min(nb, i0 + nb_max)
@@ -977,7 +1005,9 @@ class TGN(nn.Module):
                 if n_plan[i]:
                     hi[o + 4 * n:off[i + 1]] = cache_plan[i]
             g = _lib.GroupT(h_i32.data_ptr(), h_ts.data_ptr() + 8 * lo, off.ctypes.data + 8 * i0, n_plan.ctypes.data + 4 * i0,
-                            h_rows.data_ptr(), len(groups), 1, i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap, h_status)
+                            h_rows.data_ptr(), len(groups), 1, i1 - i0, bs, up - (i1 - 1) * bs, nb_max, u_cap, plan_cap, h_status,
+                            keep["d_parts"].data_ptr() + 8 * parts * i0 if parts else None,
+                            h_parts.data_ptr() + 8 * parts * i0 if parts else None)
             groups.append((g, lo))
             enqueue(g, lo)
 
@@ -997,6 +1027,8 @@ class TGN(nn.Module):
         failed = self._finish_epoch(stream)
         if failed is not None:
             raise failed
+        if parts:
+            return h_parts.numpy()[:parts * nb]
         # per batch [pos | neg]; the last batch may be short
         scores, full = h_prob.numpy()[:2 * E], E // bs
         out = np.empty((2, E), dtype=np.float32)

@@ -98,3 +98,24 @@ def test_a_stream_that_fails_leaves_a_model_that_works(monkeypatch):
     for a, b in zip(run(m, plan, E), run(fresh, plan, E)):
         assert np.array_equal(a, b)
     assert torch.equal(m.memory.memory, fresh.memory.memory)
+
+
+@pytest.mark.parametrize("bs,E", [(1, 40), (255, 700), (256, 1024), (257, 1000), (4096, 9000), (5000, 9000)])
+def test_metrics_on_the_device_equal_the_hosts(bs, E):
+    """eval_epoch_metrics against orca_link_metrics over the scores of the same stream, on both sides of a part's 256
+    edges and of the largest batch that is evaluated on the device; with scores that are equal (nodes that a fresh model
+    knows nothing of)."""
+    import dataclasses
+    from orca_b200 import _lib
+    from test_gpu_model import make_model
+    g = graph("c1")
+    k = g.spec.n_degree
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs))
+    neg = synthetic.negative_destinations(g, seed=1)
+    args = (g.sources[:E], g.destinations[:E], neg[:E], g.timestamps[:E], g.edge_idxs[:E], k, bs)
+    pos, ngs = make_model(g).eval_epoch(*args)
+    assert len(np.unique(pos)) < E or bs == 1
+    want = np.empty((-(-E // bs), 3))
+    assert _lib.lib().orca_link_metrics(pos.ctypes.data, ngs.ctypes.data, E, bs, want.ctypes.data) == 0
+    # (sums of at most bs doubles of one sign in another order: bs * 2^-53)
+    np.testing.assert_allclose(make_model(g).eval_epoch_metrics(*args), want, rtol=1e-12)
