@@ -51,7 +51,7 @@ __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 lo2(const float4 &v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4 &v) { return make_float2(v.z, v.w); }
 
-// cos of two arguments below 2^15 at once: the Cody-Waite reduction of cos_small in packed arithmetic;
+// cos of two arguments below COS_SMALL at once: the Cody-Waite reduction of cos_small in packed arithmetic;
 // the nearest integer of x / 2pi comes from adding and subtracting 1.5 * 2^23
 __device__ __forceinline__ float2 cos_small2(float2 x) {
   const float2 t = mul2(x, dup2(0.15915494309189535f));
@@ -225,7 +225,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       int my_nl;
       {
         const float adt = fabsf(my_dt);
-        my_nl = (adt * wg0 >= 32768.f ? 1 : 0) + (adt * wg1 >= 32768.f ? 1 : 0) + (adt * wg2 >= 32768.f ? 1 : 0);
+        my_nl = (adt * wg0 >= COS_SMALL ? 1 : 0) + (adt * wg1 >= COS_SMALL ? 1 : 0) + (adt * wg2 >= COS_SMALL ? 1 : 0);
         if (!(adt * wg0 < 1073741824.f)) my_nl = -1;   // beyond the fixed-point range (or not finite)
       }
       const float *q_src = qt + (size_t)row * QT_LD;
