@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
     // ------------------------------------------------------------------ stages
     if (lane == 0) {
       const char *w1 = reinterpret_cast<const char *>(g.w.G_img), *w2 = reinterpret_cast<const char *>(g.w.W2_img);
+      const uint64_t once = policy_evict_first();      // (the rows are not read again: 1 % of a stream)
       int it = 0;
       for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x) {
         const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
@@ -105,8 +106,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
           mbar_wait(empty(s), (use_of(it) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
           if (st < K_STAGES) {
             mbar_expect_tx(full(s), STAGE);
-            bulk_g2s(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
-                     A_STAGE, full(s));
+            bulk_g2s_hint(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
+                          A_STAGE, full(s), once);
             bulk_g2s(at + A_STAGE, w1 + (size_t)st * W_STAGE, W_STAGE, full(s));
           } else {
             mbar_expect_tx(full(s), W_STAGE);
