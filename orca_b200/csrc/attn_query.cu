@@ -1,13 +1,14 @@
 // Query side of an attention layer on the tensor cores: qt[r] = feat[row of r] . Mq + cq, [rows, 1056] floats.
 //
-// A launch writes 4.2 KB per row and reads 0.7.  At many rows it is bound by the path of those stores through L1 (70 %
-// busy at 48 k rows: a warp's store touches 32 lines; tensor pipe 36 %, DRAM 31 %, L2 45 %) and by its one accumulator
-// buffer, which must be read before the next block's products start.  A CTA keeps its weight
+// A launch writes 4.2 KB per row and reads 0.7 six times over (once per weight tile).  A CTA keeps its weight
 // tile (heads and tails of 176 columns) for the whole launch and walks row blocks of 128, which come as an operand image
 // (attn_out.cuh): one thread streams 16 KB stages through a ring, one multiplies, eight warps carry the accumulators from
-// tensor memory to qt, a thread per row and 32 bytes a store (whole sectors, no staging).  51 k rows: 145 us for the
-// general projection kernel (weights streamed again for every row block, load, product and store one after the other),
-// 75 here.  orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
+// tensor memory to qt.  51 k rows: 145 us for the general projection kernel (weights streamed again for every row block,
+// load, product and store one after the other), 75 with a thread per row and 32 bytes a store, which kept the path of the
+// stores through L1 70 % busy (a warp's store touched 32 lines), 70 with whole lines out of shared memory.  Now it is
+// what reads and writes take between SMs and L2 (410 MB, 6 TB/s) and the one accumulator buffer, which must be read before
+// the next block's products start.
+// orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
 // for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
 #include <algorithm>
 
@@ -23,10 +24,11 @@ constexpr int BM = 128;
 constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;                // K = 172, padded to 176
 constexpr int BN = 176, TILES = QT_LD / BN;                   // 6
 constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
-constexpr int STAGES = 5, STAGE = img::STAGE_BYTES;
+constexpr int STAGES = 4, STAGE = img::STAGE_BYTES;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
+constexpr int BOX = 32 * 128;                                 // of a warp: 32 rows x 32 columns on their way out
 constexpr int RING = (2 * W_BYTES + 1023) / 1024 * 1024;      // (the swizzle wants aligned stages)
-constexpr int SMEM = RING + STAGES * STAGE + 1024;
+constexpr int SMEM = RING + STAGES * STAGE + EPI_WARPS * BOX + 1024;
 constexpr int TMEM_COLS = 512, SMALL = 256;                   // one buffer of main + cross-term accumulators
 
 struct Args {
@@ -40,19 +42,6 @@ struct Args {
   long long wait_limit;
 };
 
-template <bool WIDE>
-__device__ __forceinline__ void st_global_8(float *p, const float (&v)[8]) {
-  if (!WIDE) {     // (a result that is aligned to 16 bytes only)
-    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    return;
-  }
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-               : "memory");
-}
-
-template <bool WIDE>
 __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __grid_constant__ Args g) {
   using namespace tc;
   extern __shared__ unsigned char raw[];
@@ -142,13 +131,14 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
     // (six chunks of 16 columns for the first four warps, five for the others)
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int c0 = half * 6, nc = half ? 5 : 6;
+    const uint32_t box = ring + STAGES * STAGE + (warp - 2) * BOX;
     int t = 0;
     for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
-      const int m = blk * BM + quarter * 32 + lane;
+      const int m0 = blk * BM + quarter * 32;
       mbar_wait(accfull, t & 1, g.status, 560, alive, g.wait_limit);
       tc_fence_after();
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + c0 * 16;
-      float *out = g.qt + (size_t)m * QT_LD + nt * BN + c0 * 16;
+      float *out = g.qt + (size_t)m0 * QT_LD + nt * BN + c0 * 16;
       float v[6][16];
 #pragma unroll
       for (int ch = 0; ch < 6; ++ch)
@@ -156,17 +146,27 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(accfree);      // (the next block's products may start before this one is stored)
-      if (m < M) {
+      // 32 columns at a time through shared memory (16-byte pieces of a row exchanged by its number's low bits: no bank
+      // conflicts either way), out in whole lines of a row
 #pragma unroll
-        for (int ch = 0; ch < 6; ++ch)
+      for (int b = 0; b < 3; ++b) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (ch >= nc) continue;
-            float y[8];
+        for (int p = 0; p < 8; ++p) {
+          const int ch = 2 * b + (p >> 2), c = 4 * (p & 3);
+          if (ch >= nc) continue;
+          const float4 y = *reinterpret_cast<const float4 *>(s_bias + (c0 + ch) * 16 + c);
+          st_shared_f4(box + lane * 128 + ((p ^ (lane & 7)) << 4),
+                       make_float4(v[ch][c] + y.x, v[ch][c + 1] + y.y, v[ch][c + 2] + y.z, v[ch][c + 3] + y.w));
+        }
+        __syncwarp();
+        const bool whole = 2 * b + 1 < nc;      // (the last box of the others is half empty)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) y[i] = v[ch][8 * q + i] + s_bias[(c0 + ch) * 16 + 8 * q + i];
-            st_global_8<WIDE>(out + ch * 16 + 8 * q, y);
-          }
+        for (int i = 0; i < 8; ++i) {
+          const int r = whole ? 4 * i + (lane >> 3) : 8 * i + (lane >> 2), p = whole ? lane & 7 : lane & 3;
+          if ((whole || i < 4) && m0 + r < M)
+            *reinterpret_cast<float4 *>(out + (size_t)r * QT_LD + 32 * b + 4 * p) = ld_shared_f4(box + r * 128 + ((p ^ (r & 7)) << 4));
+        }
+        __syncwarp();
       }
     }
   }
@@ -223,14 +223,12 @@ int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_ca
   ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && ((uintptr_t)d_qt & 15) == 0);
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
-    for (auto kernel : {aqi::attn_query_image_kernel<true>, aqi::attn_query_image_kernel<false>})
-      ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
+    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
     configured_device = c->device;
   }
   const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, c->status_word, c->wait_limit};
   const dim3 grid(aqi::TILES, std::min(ceil_div(n_cap, aqi::BM), std::max(1, c->sm_count / aqi::TILES)));
-  auto kernel = ((uintptr_t)d_qt & 31) == 0 ? aqi::attn_query_image_kernel<true> : aqi::attn_query_image_kernel<false>;
-  ORCA_CUDA(launch_dep(kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
+  ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;
