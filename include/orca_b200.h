@@ -371,12 +371,19 @@ int orca_plan_host(int32_t strategy, const int64_t *h_src, const int64_t *h_dst,
                    uint32_t seed, int32_t *h_plan_flat, int64_t plan_cap, int64_t *h_plan_off,
                    double *h_stats);
 
+/* The query list of a stream of batches, from host arrays of n_edges: batch b contributes its sources, then its
+ * destinations, each with its edge's time (utils/cache.py:46-53).  Ids are narrowed and copied into page-locked memory
+ * on the way: h_pinned and d_buffer hold 16 bytes an edge, d_buffer 8-byte aligned.  d_nodes: [2*n_edges] int32, d_ts:
+ * [2*n_edges].  Enqueues on `stream`; h_pinned is in use until that is done. */
+int orca_plan_queries(const int64_t *h_src, const int64_t *h_dst, const double *h_ts, int64_t n_edges, int32_t bs,
+                      void *h_pinned, void *d_buffer, int32_t *d_nodes, double *d_ts, void *stream);
+
 /* The MRD plan computed on the device (utils/cache.py:19-89 and 92-166, one call for both).
  * d_nodes: the query list described above ([2*n_edges] int32, batch b = its sources, then its
- * destinations); d_nbr: the neighbour table sampled for it ([2*n_edges, k] int32).  Two kernels walk
- * the batches, one backwards (next use of every node at every batch) and one forwards (candidates from
- * bitmaps in ascending order, keys, the first `budget` places of numba's argsort with its order among
- * equal keys, statistics).  Outputs, all on the device: d_plan_flat / d_plan_off as in orca_plan_host
+ * destinations); d_nbr: the neighbour table sampled for it ([2*n_edges, k] int32).  Lists of the batches' distinct
+ * nodes, then two kernels that walk the batches, one backwards (next use of every node at every batch) and one forwards
+ * (candidates in ascending order, which of them lie in the first `budget` places of numba's argsort with its order
+ * among equal keys, statistics), then that order for all batches.  Outputs, all on the device: d_plan_flat / d_plan_off as in orca_plan_host
  * (plan_cap >= n_batches * budget always suffices), d_stats = int64 {n_reuse, n_recompute, sum of
  * reuse distances}, d_status (int32[4], ORCA_E_CAPACITY when d_plan_flat is too small).
  * Enqueues on `stream`; the workspace (256-byte aligned) is sized by orca_plan_mrd_workspace_bytes. */
@@ -387,9 +394,9 @@ int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k
                   int64_t workspace_bytes, void *stream);
 
 /* Any of the three plans on the device: strategy 0 = MRD (the call above), 1 = LRU (utils/cache.py:338-403),
- * 2 = 2Q (:175-333).  LRU and 2Q run as one thread block: their random evictions are a serial Fisher-Yates
- * shuffle per batch, driven by numba's Mersenne Twister (`seed` as in orca_plan_host) and walked by one
- * thread; the split of the tables, the statistics, the ascending member lists of the sets and the
+ * 2 = 2Q (:175-333).  LRU and 2Q run as one thread block over lists of the batches' distinct neighbours: their random
+ * evictions are a serial Fisher-Yates shuffle per batch, driven by numba's Mersenne Twister (`seed` as in
+ * orca_plan_host) and walked by one thread; the statistics, the ascending member lists of the sets and the
  * least-recently-used evictions (first entries of numba's argsort of the last-use times) are data parallel
  * around it.  Arguments, outputs and plan order as in orca_plan_mrd / orca_plan_host
  * (plan_cap >= n_batches * budget always suffices). */

@@ -133,6 +133,7 @@ SYMBOLS = {
     "orca_csr_build_from_host": (C.c_int, [_V, _V, _V, _V, _I64, _I64, _V, _I64, _V, _V, _V, _V, _V, _I64, _V]),
     "orca_plan_mrd_workspace_bytes": (_I64, [_I64, _I32, _I32, _I64, _I32]),
     "orca_plan_mrd": (C.c_int, [_V, _I64, _I32, _I32, _V, _I64, _I32, _V, _I64, _V, _V, _V, _V, _I64, _V]),
+    "orca_plan_queries": (C.c_int, [_V, _V, _V, _I64, _I32, _V, _V, _V, _V, _V]),
     "orca_plan_device_workspace_bytes": (_I64, [_I32, _I64, _I32, _I32, _I64, _I32]),
     "orca_plan_device": (C.c_int, [_I32, _V, _I64, _I32, _I32, _V, _I64, _I32, C.c_uint32, _V, _I64, _V, _V, _V, _V,
                                    _I64, _V]),

@@ -18,6 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from .neighbor_finder import NeighborFinder
 
 STRATEGIES = {"MRD": 0, "LRU": 1, "2Q": 2}
 
@@ -74,22 +75,63 @@ def plan_device(strategy, nodes, nbr_table, n_edges, bs, k, n_nodes, budget, see
     nb = math.ceil(n_edges / bs)
     code = STRATEGIES[strategy]
     L = _lib.lib()
+    # what the host waits for: [plan offsets | statistics | status word]
     with torch.cuda.device(dev):
         ws_bytes = L.orca_plan_device_workspace_bytes(code, n_edges, bs, k, n_nodes, budget)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         cap = max(nb * budget, 1)
         flat = torch.empty(cap, dtype=torch.int32, device=dev)
-        off = torch.zeros(nb + 1, dtype=torch.int64, device=dev)
-        stats = torch.zeros(3, dtype=torch.int64, device=dev)
-        status = torch.zeros(4, dtype=torch.int32, device=dev)
+        head = torch.zeros(nb + 1 + 3 + 2, dtype=torch.int64, device=dev)
+        off, stats, status = head[:nb + 1], head[nb + 1:nb + 4], head[nb + 4:]
         _lib.check(L.orca_plan_device(code, nodes.data_ptr(), n_edges, bs, k, nbr_table.data_ptr(), n_nodes, budget,
                                       seed, flat.data_ptr(), cap, off.data_ptr(), stats.data_ptr(),
                                       status.data_ptr(), ws.data_ptr(), ws_bytes, _lib.stream_ptr(dev)))
-        _lib.check(L.orca_read_status(None, status.data_ptr(), None, _lib.stream_ptr(dev)))
-    off_h = off.cpu().numpy()
-    flat_h = flat[:int(off_h[-1])].cpu().numpy().astype(np.int64)
-    plan = [flat_h[off_h[b]:off_h[b + 1]] for b in range(nb)]
-    return plan, stats.cpu().numpy().astype(np.float64)
+        head_h = head.cpu().numpy()
+        if head_h[nb + 4:].view(np.int32)[0] != 0:
+            _lib.check(L.orca_read_status(None, status.data_ptr(), None, _lib.stream_ptr(dev)))
+        flat_h = _ids_to_host(flat[:int(head_h[nb])])
+    at = head_h[:nb + 1].tolist()
+    plan = [flat_h[a:z] for a, z in zip(at, at[1:])]
+    return plan, head_h[nb + 1:nb + 4].astype(np.float64)
+
+
+def _ids_to_host(ids):
+    """int32 ids on the device as an int64 array.  They are widened there and stay in the page-locked memory that they are
+    copied to: two million ids take 0.4 ms so, 7 as a pageable copy and a conversion, nearly all of it page faults.  More
+    than one plan may hold, or callers may hold together, comes back in ordinary memory."""
+    nbytes = 8 * ids.numel()
+    share = None
+    if 0 < nbytes <= NeighborFinder.PINNED_TABLE:
+        share = NeighborFinder.LENT.take(1 << (nbytes - 1).bit_length())
+    if share is None:
+        return ids.cpu().numpy().astype(np.int64)
+    pin = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+    pin.view(torch.int64).copy_(ids.to(torch.int64), non_blocking=True)
+    torch.cuda.current_stream(ids.device).synchronize()
+    return share.array(pin).view(np.int64)
+
+
+def _queries_device(sources, destinations, timestamps, bs, device):
+    """batch_query_order's list on the device.  The edges cross the bus as they are (16 bytes each) and are put in order
+    there; streams of more edges than the page-locked buffer takes are put in order on the host."""
+    E = len(sources)
+    if not 0 < 16 * E <= NeighborFinder.PINNED_TABLE:
+        nodes, ts = batch_query_order(sources, destinations, timestamps, bs)
+        return torch.as_tensor(nodes).to(device), torch.as_tensor(ts).to(device)
+    src, dst = (np.ascontiguousarray(a, dtype=np.int64) for a in (sources, destinations))
+    t = np.ascontiguousarray(timestamps, dtype=np.float64)
+    if not (src.shape == dst.shape == t.shape == (E,)):
+        raise ValueError("sources, destinations and timestamps must have one length")
+    pin = torch.empty(16 * E, dtype=torch.uint8, pin_memory=True)
+    with torch.cuda.device(device):
+        buffer = torch.empty(16 * E, dtype=torch.uint8, device=device)
+        nodes = torch.empty(2 * E, dtype=torch.int32, device=device)
+        ts = torch.empty(2 * E, dtype=torch.float64, device=device)
+        rc = _lib.lib().orca_plan_queries(src.ctypes.data, dst.ctypes.data, t.ctypes.data, E, bs, pin.data_ptr(),
+                                          buffer.data_ptr(), nodes.data_ptr(), ts.data_ptr(), _lib.stream_ptr(device))
+        torch.cuda.current_stream(device).synchronize()      # (the page-locked buffer goes back to its pool)
+        _lib.check(rc)
+    return nodes, ts
 
 
 def plan_mrd_device(nodes, nbr_table, n_edges, bs, k, n_nodes, budget):
@@ -99,8 +141,8 @@ def plan_mrd_device(nodes, nbr_table, n_edges, bs, k, n_nodes, budget):
 def _plan_local(args, train_data, neighbor_finder, num_embeddings, strategy, seed):
     budget = args.budget
     t0 = time.time()
-    nodes, ts = batch_query_order(train_data.sources, train_data.destinations, train_data.timestamps, args.bs)
-    nodes_dev = torch.as_tensor(nodes).to(neighbor_finder.device)
+    nodes_dev, ts = _queries_device(train_data.sources, train_data.destinations, train_data.timestamps, args.bs,
+                                    neighbor_finder.device)
     nbr, _, _, _ = neighbor_finder.sample_device(nodes_dev, ts, args.n_degree)
     torch.cuda.synchronize(neighbor_finder.device)
     t_prepare = time.time() - t0

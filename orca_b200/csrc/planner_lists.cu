@@ -16,10 +16,23 @@
 
 #include "common.cuh"
 #include "context.cuh"
+#include "host_threads.cuh"
 #include "planner_lists.cuh"
 
 namespace orca {
 namespace lists {
+
+// ------------------------------------------------------------------------------ queries
+// [times][sources][destinations] of the edges -> the query list and its times
+__global__ void __launch_bounds__(256) queries_kernel(const double *ts, const int32_t *src, const int32_t *dst, int64_t n_edges,
+                                                      int32_t bs, int32_t *nodes, double *out_ts) {
+  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < n_edges; i += gridDim.x * 256ll) {
+    const int64_t b = i / bs, lo = b * bs, n = min((int64_t)bs, n_edges - lo), at = 2 * lo + (i - lo);
+    nodes[at] = src[i];
+    nodes[at + n] = dst[i];
+    out_ts[at] = out_ts[at + n] = ts[i];
+  }
+}
 
 // ------------------------------------------------------------------------------ lists
 // One block a batch, blocks walk the batches.  Two bitmaps over the nodes (the batch's nodes, its endpoints) and the
@@ -448,3 +461,34 @@ int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, in
 
 }  // namespace lists
 }  // namespace orca
+
+using namespace orca;
+
+extern "C" int orca_plan_queries(const int64_t *h_src, const int64_t *h_dst, const double *h_ts, int64_t n_edges, int32_t bs,
+                                 void *h_pinned, void *d_buffer, int32_t *d_nodes, double *d_ts, void *stream) {
+  ORCA_CHECK_ARG(n_edges >= 0 && bs > 0);
+  if (n_edges == 0) return ORCA_OK;
+  ORCA_CHECK_ARG(h_src && h_dst && h_ts && h_pinned && d_buffer && d_nodes && d_ts && ((uintptr_t)d_buffer & 7) == 0);
+  double *ts = (double *)h_pinned;
+  int32_t *src = (int32_t *)(ts + n_edges), *dst = src + n_edges;
+  // (a thread is worth starting for 50,000 edges: 400,000 take 0.9 ms on one, 0.2 on eight)
+  const int threads = (int)std::max<int64_t>(1, std::min<int64_t>({8, n_edges / 50000, (int64_t)std::thread::hardware_concurrency()}));
+  const int rc = on_threads(threads, [&](int t) {
+    const int64_t lo = n_edges * t / threads, hi = n_edges * (t + 1) / threads;
+    for (int64_t i = lo; i < hi; ++i) {
+      ts[i] = h_ts[i];
+      src[i] = (int32_t)h_src[i];
+      dst[i] = (int32_t)h_dst[i];
+    }
+  }, "orca_plan_queries");
+  if (rc != ORCA_OK) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  ORCA_CUDA(cudaMemcpyAsync(d_buffer, h_pinned, (size_t)n_edges * 16, cudaMemcpyHostToDevice, s));
+  const double *dt = (const double *)d_buffer;
+  const int32_t *ds = (const int32_t *)(dt + n_edges);
+  lists::queries_kernel<<<(int)std::min<int64_t>((n_edges + 255) / 256, 1184), 256, 0, s>>>(dt, ds, ds + n_edges, n_edges, bs,
+                                                                                             d_nodes, d_ts);
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
+}

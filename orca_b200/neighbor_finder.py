@@ -19,7 +19,7 @@ from . import _lib
 
 
 class _Lent:
-    """Bytes of page-locked memory that returned tables hold, over the process: at most `limit` of them."""
+    """Bytes of page-locked memory that returned tables and plans hold, over the process: at most `limit` of them."""
 
     def __init__(self, limit):
         self.limit, self.held = limit, 0

@@ -126,3 +126,13 @@ def test_plan_buffer_too_small_is_reported():
         _lib.check(L.orca_plan_mrd(nd.data_ptr(), g.n_edges, bs, k, nbr.data_ptr(), g.n_nodes, budget,
                                    flat.data_ptr(), 60, off.data_ptr(), stats.data_ptr(), status.data_ptr(),
                                    ws.data_ptr(), ws_bytes - 1, _lib.stream_ptr(torch.device("cuda"))))
+
+
+@pytest.mark.parametrize("E,bs", [(1, 1), (7, 7), (1000, 300), (101, 100), (250001, 2000), (3, 10)])
+def test_queries_on_the_device_are_in_batch_order(E, bs):
+    from orca_b200 import cache
+    rs = np.random.RandomState(E)
+    src, dst, ts = rs.randint(1, 1 << 30, E), rs.randint(1, 1 << 30, E), rs.rand(E)
+    want = cache.batch_query_order(src, dst, ts, bs)
+    got = cache._queries_device(src, dst, ts, bs, torch.device("cuda"))
+    assert all(np.array_equal(g.cpu().numpy(), w) for g, w in zip(got, want))
