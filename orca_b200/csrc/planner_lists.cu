@@ -10,8 +10,8 @@
 // the range that the budget line falls into are needed, one or two as a rule: two candidates in three share the largest
 // key, which is the first pivot then, and where the equal keys of a range end up follows from its length alone.
 // 200 batches of 2000 edges, 10,700 candidates each, ms of kernels: 24.4 with the kernels of planner_mrd.cu, which walk
-// tables and sort whole lists batch after batch on a cluster of 16 SMs, 4.4 here: lists 0.13, next uses 0.39, the serial
-// step 3.5 (17.7 us a batch: the block's instructions and barriers), orders 0.29.
+// tables and sort whole lists batch after batch on a cluster of 16 SMs, 3.8 here: lists 0.13, next uses 0.39, the serial
+// step 3.0 (15 us a batch: the block's instructions and barriers), orders 0.30.
 #include <algorithm>
 
 #include "common.cuh"
@@ -179,6 +179,13 @@ __global__ void __launch_bounds__(T) next_use_lists_kernel(Lists l, int64_t nb, 
   }
 }
 
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 struct State {           // of a plan, between the launches for its chunks of batches
   int32_t n_cached, failed;
   int64_t used;
@@ -191,33 +198,38 @@ struct MrdArgs {
   int32_t budget, cap;
   State *st;
   int32_t *cached;              // [cap] cached ids, ascending (between launches)
-  uint32_t *cached_state;       // [cap] their states
+  uint32_t *cached_state;       // [cap] their states (between launches)
   int32_t *place;               // [cap] of the listed nodes: cached ids before it
-  int2 *cand;                   // [batches of a launch][cap] candidates and their states
+  int32_t *cand;                // [batches of a launch][2][cap] candidates, and their states
   int32_t *cand_n;              // [batches of a launch]
   int64_t plan_cap;
   int64_t *plan_off;
   int32_t *status;
 };
 
-// Forward sweep over batches b0 .. b1, one block.  Shared memory: [cached ids | later the lists of a step][entries of the
-// selection], `cap` words each, then bitmaps.  What a batch costs is the walk over all of its candidates, twice (into the
-// list and back into the cached ids): a warp takes a word of the bitmaps at a time.
+// Forward sweep over batches b0 .. b1, one block.  Shared memory: cached ids and their states, later entries and lists of
+// a selection; candidates and their states; four words each, then bitmaps.  What a batch costs is the walk over all of
+// its candidates, twice (into the list and back into the cached ids), a warp for a word of the bitmaps at a time, and the
+// selection.  (With the states in global memory the two walks took 17,000 of a batch's 34,000 cycles: an SM's own loads
+// and stores get some 15 bytes a cycle out of L2.)  Candidates leave by bulk copies that nobody waits for.
 __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__ MrdArgs g) {
   extern __shared__ __align__(16) char raw[];
   __shared__ uint32_t s_tot[NW];
-  __shared__ int32_t s_place;
+  __shared__ Line s_line;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cap = g.cap, n_words = cap / 32;
   int32_t *s_cached = (int32_t *)raw;
-  uint32_t *s_ent = (uint32_t *)(s_cached + cap);
-  uint16_t *left = (uint16_t *)s_cached, *right = left + cap;
-  Word *s_list = (Word *)(s_ent + cap), *s_new = s_list + n_words, *s_kept = s_new + n_words;
+  uint32_t *s_state = (uint32_t *)(s_cached + cap);
+  int32_t *s_cand = (int32_t *)(s_state + cap);
+  uint32_t *s_cand_state = (uint32_t *)(s_cand + cap);
+  uint32_t *s_ent = (uint32_t *)s_cached;
+  uint16_t *left = (uint16_t *)s_state, *right = left + cap;
+  Word *s_list = (Word *)(s_cand_state + cap), *s_new = s_list + n_words, *s_kept = s_new + n_words;
   uint32_t *s_known = (uint32_t *)(s_kept + n_words);
   if (g.st->failed) return;
   int n_cached = g.st->n_cached;
   int64_t used = g.st->used;
   unsigned long long reuse = 0, recompute = 0, dist = 0;
-  for (int i = tid; i < n_cached; i += T) s_cached[i] = g.cached[i];
+  for (int i = tid; i < n_cached; i += T) s_cached[i] = g.cached[i], s_state[i] = g.cached_state[i];
   bool failed = false;
   // the first nodes of the next batch's list, loaded ahead
   constexpr int AHEAD = 2;
@@ -235,12 +247,13 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
   for (int64_t b = g.b0; b < g.b1; ++b) {
     const int64_t at = b * g.l.stride;
     const int n_list = n_next;
-    int2 *cand = g.cand + (b - g.b0) * cap;
+    int32_t *cand = g.cand + (b - g.b0) * 2 * cap;
     if (n_list > cap) {      // (uniform over the block)
       failed = true;
       break;
     }
     for (int i = tid; i < n_words; i += T) s_new[i].bits = s_known[i] = s_list[i].bits = 0;
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // (the candidates of the batch before)
     __syncthreads();         // (and the cached ids are there)
     // which of the batch's nodes are cached: a bit in s_list; statistics of the reuse
     const auto look_up = [&](int i, int32_t x, int m) {
@@ -258,7 +271,7 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
         if (x >= 0) {
           if (cached) {
             reuse += m;
-            dist += (unsigned long long)m * (unsigned long long)(b - (g.cached_state[lo] & 0xffffu));
+            dist += (unsigned long long)m * (unsigned long long)(b - (s_state[lo] & 0xffffu));
           } else {
             recompute += m;
           }
@@ -287,8 +300,8 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
       const Word w = s_list[i >> 5];
       const int c = g.place[i], pos = c + i - bits_before(w, i);
       const bool cached = bit_of(w, i);
-      s_ent[pos] = key << IDX_BITS | (uint32_t)pos;
-      cand[pos] = make_int2(x & ~TARGET, (int)(key << 16 | (x < 0 || !cached ? (uint32_t)b : g.cached_state[c] & 0xffffu)));
+      s_cand[pos] = x & ~TARGET;
+      s_cand_state[pos] = key << 16 | (x < 0 || !cached ? (uint32_t)b : s_state[c] & 0xffffu);
       atomicOr(cached ? &s_known[pos >> 5] : &s_new[pos >> 5].bits, 1u << (pos & 31));
     };
 #pragma unroll
@@ -306,9 +319,8 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
       const int pos = 32 * w + lane;
       if (pos < n && !(((add.bits | s_known[w]) >> lane) & 1u)) {
         const int c = pos - bits_before(add, lane);
-        const uint32_t st = g.cached_state[c];
-        s_ent[pos] = st >> 16 << IDX_BITS | (uint32_t)pos;
-        cand[pos] = make_int2(s_cached[c], (int)st);
+        s_cand[pos] = s_cached[c];
+        s_cand_state[pos] = s_state[c];
       }
       if (lane == 0) s_kept[w].bits = n >= 32 * w + 32 ? 0xffffffffu : n > 32 * w ? (1u << (n - 32 * w)) - 1u : 0u;
     }
@@ -318,10 +330,22 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
       failed = true;
       break;
     }
+    fence_async();           // (what the bulk copies read)
     __syncthreads();
-    if (keep < n)
-      select_by_order<false>(s_ent, n, keep, left, right, s_list, s_tot, &s_place,
-                   [&](int i) { atomicAnd(&s_kept[i >> 5].bits, ~(1u << (i & 31))); });
+    if (tid == 0) {
+      const uint32_t bytes = (uint32_t)(n + 3) / 4 * 16;
+      bulk_s2g(cand, s_cand, bytes);
+      bulk_s2g(cand + cap, s_cand_state, bytes);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    if (keep < n) {
+      const auto drop = [&](int i) { atomicAnd(&s_kept[i >> 5].bits, ~(1u << (i & 31))); };
+      if (!select_by_far_step([&](int i) { return s_cand_state[i] >> 16; }, n, keep, s_list, s_tot, drop)) {
+        for (int i = tid; i < n; i += T) s_ent[i] = s_cand_state[i] >> 16 << IDX_BITS | (uint32_t)i;
+        __syncthreads();
+        select_by_order<false>(s_ent, n, keep, left, right, s_tot, &s_line, drop);
+      }
+    }
     __syncthreads();
     count_words(s_kept, n_words, (int32_t *)s_tot);
 #pragma unroll 4
@@ -329,9 +353,8 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
       const Word kept = s_kept[w];
       if (!bit_of(kept, lane)) continue;
       const int c = bits_before(kept, lane);
-      const int2 x = __ldcg(&cand[32 * w + lane]);
-      s_cached[c] = x.x;
-      g.cached_state[c] = (uint32_t)x.y;
+      s_cached[c] = s_cand[32 * w + lane];
+      s_state[c] = s_cand_state[32 * w + lane];
     }
     if (tid == 0) {
       g.plan_off[b] = used;
@@ -341,7 +364,8 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
     used += keep;
   }
   __syncthreads();
-  for (int i = tid; i < n_cached && !failed; i += T) g.cached[i] = s_cached[i];
+  for (int i = tid; i < n_cached && !failed; i += T) g.cached[i] = s_cached[i], g.cached_state[i] = s_state[i];
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // (shared memory is read until then)
   for (int o = 16; o > 0; o >>= 1) {
     reuse += __shfl_xor_sync(0xffffffffu, reuse, o);
     recompute += __shfl_xor_sync(0xffffffffu, recompute, o);
@@ -369,13 +393,13 @@ __global__ void __launch_bounds__(T, 1) sort_plan_kernel(const __grid_constant__
   const tie::Shared w{g.cap};
   for (int64_t b = g.b0 + blockIdx.x; b < g.b1; b += gridDim.x) {
     const int n = g.cand_n[b - g.b0], keep = min(n, g.budget);
-    const int2 *cand = g.cand + (b - g.b0) * g.cap;
+    const int32_t *cand = g.cand + (b - g.b0) * 2 * g.cap;
     int32_t *out = plan + g.plan_off[b];
     for (int i = threadIdx.x; i < n; i += T) {
-      w.key(i) = (int32_t)((uint32_t)cand[i].y >> 16);
+      w.key(i) = (int32_t)((uint32_t)cand[g.cap + i] >> 16);
       w.idx(i) = (uint16_t)i;
     }
-    tie::sort_first_shared(w, s_tot, n, keep, [&](int place, int i) { out[place] = cand[i].x; });
+    tie::sort_first_shared(w, s_tot, n, keep, [&](int place, int i) { out[place] = cand[i]; });
   }
 }
 
@@ -433,7 +457,7 @@ int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, in
   g.st = (State *)(base + L.state);
   g.cached = (int32_t *)(base + L.cached), g.cached_state = (uint32_t *)(base + L.cached_state);
   g.place = (int32_t *)(base + L.place);
-  g.cand = (int2 *)(base + L.cand);
+  g.cand = (int32_t *)(base + L.cand);
   g.cand_n = (int32_t *)(base + L.cand_n);
   g.plan_cap = plan_cap, g.plan_off = d_plan_off, g.status = d_status;
   ORCA_CUDA(cudaMemsetAsync(g.st, 0, sizeof(State), s));
@@ -443,7 +467,7 @@ int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, in
   next_use_lists_kernel<<<1, T, 0, s>>>(g.l, g.nb, (int32_t *)(base + L.next), (int32_t *)(base + L.key));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
-  const int smem = 8 * L.cap + 7 * (L.cap / 32) * 4, smem_sort = tie::Shared::BYTES * L.cap;
+  const int smem = 16 * L.cap + 7 * (L.cap / 32) * 4, smem_sort = tie::Shared::BYTES * L.cap;
   ORCA_CUDA(cudaFuncSetAttribute(mrd_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   ORCA_CUDA(cudaFuncSetAttribute(sort_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_sort));
   for (g.b0 = 0; g.b0 < g.nb; g.b0 = g.b1) {

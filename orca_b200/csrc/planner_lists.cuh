@@ -7,7 +7,7 @@ namespace orca {
 namespace lists {
 
 constexpr int T = tie::T, NW = tie::NW;
-constexpr int CAP = tie::SHARED_MAX;      // entries of a list that is selected from
+constexpr int CAP = 13696;      // entries of a list that is selected from: 17 bytes of shared memory each, whole words of bits
 
 // The distinct nodes of every batch in ascending order, batch b's from b * stride: its endpoints (TARGET set) and the
 // out-of-batch neighbours of its table.
@@ -118,83 +118,120 @@ __device__ __forceinline__ int source_of_equal(int y, int lo, int hi) {
   return q;
 }
 
-// Calls f(index) for the entries of e[0 .. n) (key << IDX_BITS | index, in list order) that numba's argsort leaves at
-// `keep` or behind, 0 < keep < n (FIRST: for those before `keep`; no key is FAR then): its steps on the range that contains the line, until that range is
-// short or its keys are equal.  left, right: [n]; words: [(n + 31) / 32].  All T threads; no barrier at the end.
-//
-// A step whose pivot is the largest key there is, FAR, is the usual one, and needs no swap: its left list is the FAR
-// entries, its right list everything, so that the m-th FAR entry from the left goes to place hi - 1 - m for as long as it
-// lies left of that, and these places are the right part.
-template <bool FIRST, class F>
-__device__ __forceinline__ void select_by_order(uint32_t *e, int n, int keep, uint16_t *left, uint16_t *right, Word *words,
-                                             uint32_t *s_tot, int32_t *s_place, F f) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  const auto key = [&](int i) { return e[i] >> IDX_BITS; };
-  const auto swap = [&](int i, int j) { const uint32_t x = e[i]; e[i] = e[j]; e[j] = x; };
-  const auto park = [&](int lo, int hi) {
+// A range of at most WARP_RANGE entries is partitioned by one warp, without the block's barriers: a level takes it 300 to
+// 700 cycles, the block 1400 whatever the length.  Moves [lo, hi] (the pivot parked at hi) to the range that the line
+// falls into, until it is short, its keys are equal, or the line lies between ranges.
+constexpr int WARP_RANGE = 512;
+struct Line {
+  int lo, hi;
+  bool in, equal;     // the line falls into [lo, hi]; all its keys are equal
+};
+struct Entries {      // of a selection: key << IDX_BITS | index
+  uint32_t *e;
+  __device__ uint32_t key(int i) const { return e[i] >> IDX_BITS; }
+  __device__ void swap(int i, int j) const { const uint32_t x = e[i]; e[i] = e[j]; e[j] = x; }
+  // median of three, the pivot at the end (the head of numba's partition step)
+  __device__ void park(int lo, int hi) const {
     const int mid = (lo + hi) >> 1;
     uint32_t a = e[lo], c = e[mid], d = e[hi], t;
     if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
     if (d >> IDX_BITS < c >> IDX_BITS) t = d, d = c, c = t;
     if (c >> IDX_BITS < a >> IDX_BITS) t = a, a = c, c = t;
     e[lo] = a, e[mid] = d, e[hi] = c;
-  };
-  int lo = 0, hi = n - 1;
-  bool line = true, equal = false;      // the line falls into [lo, hi]; all its keys are equal
-  if (hi - lo >= 15) {
-    if (tid == 0) park(lo, hi);
-    __syncthreads();
   }
-  while (line && !equal && hi - lo >= 15) {
-    const uint32_t p = key(hi);
-    if (!FIRST && p == FAR) {
-      // FAR entries of [lo, hi), a bit each; their number before every word
-      const int len = hi - lo, n_words = (len + 31) / 32;
+};
+// the part of the line's range behind a step whose pivot came to place m
+__device__ __forceinline__ Line next_range(Line r, int m, int keep) {
+  if (keep <= m) {
+    r.in = keep < m;        // (keep == m: the left part stays, the rest goes; keep > lo, for the line is in the range)
+    r.hi = m - 1;
+    if (!r.in) r.lo = keep, r.hi = keep - 1;
+  } else {
+    r.in = keep > m + 1;
+    r.lo = m + 1;
+    if (!r.in) r.hi = r.lo - 1;
+  }
+  return r;
+}
+__device__ __forceinline__ Line partition_warp(Entries e, Line r, int keep, uint16_t *left, uint16_t *right) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  while (r.in && !r.equal && r.hi - r.lo >= 15) {
+    const int lo = r.lo, hi = r.hi, len = hi - lo;
+    const uint32_t p = e.key(hi);
+    int nl = 0, nr = 0;
 #pragma unroll 4
-      for (int i0 = warp * 32; i0 < len; i0 += T) {
-        const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < len && key(lo + i0 + lane) == FAR);
-        if (lane == 0) words[i0 >> 5].bits = w;
-      }
-      if (tid == 0) *s_place = 0;
-      __syncthreads();
-      count_words(words, n_words, (int32_t *)s_tot);
-      // swaps of the step: entry m at i swaps while i + m < len - 1, which grows from entry to entry
-      if (tid < n_words) {
-        uint32_t w = words[tid].bits;
-        const int first = 32 * tid + words[tid].before;
-        if (w != 0 && first + 31 - __clz(w) + __popc(w) - 1 >= len - 1) {     // (the word's last one does not)
-          int c = 0;
-          for (; w != 0 && first + __ffs(w) - 1 + c < len - 1; w &= w - 1) ++c;
-          w = (1u << c) - 1u;
-        }
-        if (w != 0) atomicAdd(s_place, __popc(w));
-      }
-      __syncthreads();
-      const int swaps = *s_place, mid = len - 1 - swaps;
-      // the pivot's place: the middle, if a FAR entry that need not swap lies there, else where the right part begins
-      bool stays = false;
-      if (mid >= 0 && mid < len) {
-        const Word w = words[mid >> 5];
-        stays = bit_of(w, mid) && bits_before(w, mid) == swaps;
-      }
-      const int m = lo + (stays ? mid : len - swaps);
-      if (keep > m + 1) {
-        // the right part: its places hi - 1, hi - 2, ... hold the first FAR entries, place hi the one after them
-        for (int y = keep + tid; y <= hi; y += T) {
-          const int q = source_of_equal(y, m + 1, hi);
-          f((int)(e[lo + bit_number(words, n_words, q == hi ? hi - m - 1 : hi - 1 - q)] & IDX));
-        }
-        for (int pos = hi + 1 + tid; pos < n; pos += T) f((int)(e[pos] & IDX));
-        return;      // (the parked entry is the pivot, at m: it stays)
-      }
-      __syncthreads();      // (s_place)
+    for (int i0 = lo; i0 < hi; i0 += 32) {
+      const int pos = i0 + lane;
+      const uint32_t k = pos < hi ? e.key(pos) : 0;
+      const uint32_t ml = __ballot_sync(0xffffffffu, pos < hi && k >= p), mr = __ballot_sync(0xffffffffu, pos < hi && k <= p);
+      if (ml >> lane & 1u) left[nl + __popc(ml & lt)] = (uint16_t)pos;
+      if (mr >> lane & 1u) right[nr + __popc(mr & lt)] = (uint16_t)pos;
+      nl += __popc(ml);
+      nr += __popc(mr);
     }
-    const int len = hi - lo, items = (len + T - 1) / T, first = lo + warp * 32 * items + lane;
+    __syncwarp();
+    if (nl == len && nr == len) {
+      if (lane == 0) e.swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
+      r.equal = true;
+      break;
+    }
+    const int pairs = min(nl, nr);
+    int swaps = 0;
+    for (int m0 = 0; m0 < pairs; m0 += 32) {
+      const int m = m0 + lane, pl = m < pairs ? (int)left[m] : 0, pr = m < pairs ? (int)right[nr - 1 - m] : 0;
+      if (pl < pr) e.swap(pl, pr);
+      const int c = __popc(__ballot_sync(0xffffffffu, pl < pr));
+      swaps += c;
+      if (c < 32) break;                             // (behind a pair that does not swap, none does)
+    }
+    const int next_l = swaps < nl ? (int)left[swaps] : hi;
+    const int m = swaps > 0 ? min(next_l, (int)right[nr - swaps]) : next_l;     // the pivot's place
+    r = next_range(r, m, keep);
+    __syncwarp();
+    if (lane == 0) {
+      e.swap(m, hi);
+      if (r.in && r.hi - r.lo >= 15) e.park(r.lo, r.hi);
+    }
+    __syncwarp();
+  }
+  return r;
+}
+
+// Calls f(index) for the entries of e[0 .. n) (key << IDX_BITS | index, in list order) that numba's argsort leaves at
+// `keep` or behind, 0 < keep < n (FIRST: for those before `keep`): its steps on the range that contains the line, until
+// that range is short or its keys are equal.  left, right: [n].  All T threads, behind a barrier; no barrier at the end.
+template <bool FIRST, class F>
+__device__ __forceinline__ void select_by_order(uint32_t *ents, int n, int keep, uint16_t *left, uint16_t *right,
+                                                uint32_t *s_tot, Line *s_line, F f) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const Entries e{ents};
+  if (tid == 0) {
+    *s_line = Line{0, n - 1, true, false};
+    if (n - 1 >= 15) e.park(0, n - 1);
+  }
+  __syncthreads();
+  while (true) {
+    const Line r = *s_line;
+    const int lo = r.lo, hi = r.hi, len = hi - lo;
+    if (!r.in || r.equal || len < 15) break;
+    if (len < WARP_RANGE) {
+      __syncthreads();      // (everybody has read the range)
+      if (warp == 0) {
+        const Line z = partition_warp(e, r, keep, left, right);
+        if (lane == 0) *s_line = z;
+      }
+      __syncthreads();
+      break;
+    }
+    const uint32_t p = e.key(hi);
+    const int items = (len + T - 1) / T, first = lo + warp * 32 * items + lane;
     uint32_t fl = 0, fr = 0, at = 0;
+#pragma unroll 4
     for (int i = 0; i < items; ++i) {
       const int pos = first + 32 * i;
-      const uint32_t kv = pos < hi ? key(pos) : 0;
+      const uint32_t kv = pos < hi ? e.key(pos) : 0;
       const bool l = pos < hi && kv >= p, r = pos < hi && kv <= p;
       fl |= (l ? 1u : 0u) << i;
       fr |= (r ? 1u : 0u) << i;
@@ -206,11 +243,14 @@ __device__ __forceinline__ void select_by_order(uint32_t *e, int n, int keep, ui
     at = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
     const int nl = all & 0xffff, nr = all >> 16;
     if (nl == len && nr == len) {       // (uniform over the block)
+      if (tid == 0) {
+        e.swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
+        s_line->equal = true;
+      }
       __syncthreads();
-      if (tid == 0) swap((lo + hi) >> 1, hi);     // as before the step: source_of_equal counts from there
-      equal = true;
       break;
     }
+#pragma unroll 4
     for (int i = 0; i < items; ++i) {
       const int pos = first + 32 * i;
       const bool l = (fl >> i) & 1u, r = (fr >> i) & 1u;
@@ -220,48 +260,98 @@ __device__ __forceinline__ void select_by_order(uint32_t *e, int n, int keep, ui
       at += __popc(ml) | __popc(mr) << 16;
     }
     __syncthreads();
-    // the m-th of the left list swaps with the m-th from the end of the right list while it lies left of it
+    // the m-th of the left list swaps with the m-th from the end of the right list while it lies left of it; s_tot[0]:
+    // the pivot's place
     const int pairs = min(nl, nr);
     for (int m = tid; m < pairs; m += T) {
       const int pl = left[m], pr = right[nr - 1 - m];
       if (pl >= pr) {
-        if (m == 0) *s_place = pl;
+        if (m == 0) s_tot[0] = (uint32_t)pl;
         break;                          // (behind a pair that does not swap, none does)
       }
       const int next_l = m + 1 < nl ? (int)left[m + 1] : hi;
-      if (m + 1 >= pairs || next_l >= (int)right[nr - 2 - m]) *s_place = min(next_l, pr);
-      swap(pl, pr);
+      if (m + 1 >= pairs || next_l >= (int)right[nr - 2 - m]) s_tot[0] = (uint32_t)min(next_l, pr);
+      e.swap(pl, pr);
     }
-    if (tid == 0 && pairs == 0) *s_place = nl > 0 ? (int)left[0] : hi;
+    if (tid == 0 && pairs == 0) s_tot[0] = (uint32_t)(nl > 0 ? (int)left[0] : hi);
     __syncthreads();
-    const int m = *s_place;             // the pivot's place
-    const int old_hi = hi;
-    if (keep <= m) {
-      line = keep > lo && keep < m;     // (keep == m: the left part stays, the rest goes)
-      hi = m - 1;
-      if (!line) lo = keep, hi = keep - 1;
-    } else {
-      line = keep > m + 1;
-      lo = m + 1;
-      if (!line) hi = lo - 1;
-    }
     if (tid == 0) {
-      swap(m, old_hi);
-      if (line && !equal && hi - lo >= 15) park(lo, hi);
+      const int m = (int)s_tot[0];
+      const Line z = next_range(r, m, keep);
+      e.swap(m, hi);
+      if (z.in && z.hi - z.lo >= 15) e.park(z.lo, z.hi);
+      *s_line = z;
     }
     __syncthreads();
   }
-  if (equal) __syncthreads();           // (the entries of the undone step)
-  if (equal) {
-    for (int y = (FIRST ? lo : keep) + tid; y < (FIRST ? keep : hi + 1); y += T) f((int)(e[source_of_equal(y, lo, hi)] & IDX));
+  const Line r = *s_line;
+  const int lo = r.lo, hi = r.hi;
+  if (r.equal) {
+    for (int y = (FIRST ? lo : keep) + tid; y < (FIRST ? keep : hi + 1); y += T) f((int)(ents[source_of_equal(y, lo, hi)] & IDX));
   } else if (lo + tid <= hi) {          // (fewer than 16)
     const int pos = lo + tid;
-    const uint32_t k = key(pos);
+    const uint32_t k = e.key(pos);
     int place = lo;
-    for (int q = lo; q <= hi; ++q) place += key(q) < k || (key(q) == k && q < pos) ? 1 : 0;
-    if ((place < keep) == FIRST) f((int)(e[pos] & IDX));
+    for (int q = lo; q <= hi; ++q) place += e.key(q) < k || (e.key(q) == k && q < pos) ? 1 : 0;
+    if ((place < keep) == FIRST) f((int)(ents[pos] & IDX));
   }
-  for (int pos = (FIRST ? 0 : hi + 1) + tid; pos < (FIRST ? lo : n); pos += T) f((int)(e[pos] & IDX));
+  for (int pos = (FIRST ? 0 : hi + 1) + tid; pos < (FIRST ? lo : n); pos += T) f((int)(ents[pos] & IDX));
+}
+
+// The usual first step of a selection over a list whose keys are given by key(i): its pivot is the largest key there is,
+// FAR, the right part contains the line, and nothing needs to be moved.  The step's left list is the FAR entries, its right list
+// everything, so that the m-th FAR entry from the left goes to place n - 2 - m for as long as it lies left of that, and
+// these places are the right part, all of one key.  Calls f(i) for the entries left at `keep` or behind and returns
+// true, or returns false if the step is another one.  words: [(n + 31) / 32].  All T threads, behind a barrier.
+template <class Key, class F>
+__device__ __forceinline__ bool select_by_far_step(Key key, int n, int keep, Word *words, uint32_t *s_tot, F f) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int hi = n - 1, mid = hi >> 1;
+  if (hi < 15) return false;
+  // the parked three: a at place 0, d in the middle, the pivot c at the end
+  int a = 0, c = mid, d = hi, t;
+  if (key(c) < key(a)) t = a, a = c, c = t;
+  if (key(d) < key(c)) t = d, d = c, c = t;
+  if (key(c) < key(a)) t = a, a = c, c = t;
+  if (key(c) != FAR) return false;
+  const auto entry = [&](int i) { return i == 0 ? a : i == mid ? d : i; };      // i < hi
+  const int n_words = (hi + 31) / 32;
+#pragma unroll 4
+  for (int i0 = warp * 32; i0 < hi; i0 += T) {
+    const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < hi && key(entry(min(i0 + lane, hi - 1))) == FAR);
+    if (lane == 0) words[i0 >> 5].bits = w;
+  }
+  __syncthreads();
+  count_words(words, n_words, (int32_t *)s_tot);
+  if (tid == 0) s_tot[0] = 0;
+  __syncthreads();
+  // swaps of the step: entry m at i swaps while i + m < hi - 1, which grows from entry to entry
+  if (tid < n_words) {
+    uint32_t w = words[tid].bits;
+    const int first = 32 * tid + words[tid].before;
+    int count = __popc(w);
+    if (w != 0 && first + 31 - __clz(w) + count - 1 >= hi - 1) {     // (the word's last one does not)
+      count = 0;
+      for (; w != 0 && first + __ffs(w) - 1 + count < hi - 1; w &= w - 1) ++count;
+    }
+    if (count != 0) atomicAdd(&s_tot[0], (uint32_t)count);
+  }
+  __syncthreads();
+  const int swaps = (int)s_tot[0], at = hi - 1 - swaps;
+  // the pivot's place: a FAR entry that need not swap, if it lies in the middle, else where the right part begins
+  bool stays = false;
+  if (at >= 0 && at < hi) {
+    const Word w = words[at >> 5];
+    stays = bit_of(w, at) && bits_before(w, at) == swaps;
+  }
+  const int m = stays ? at : hi - swaps;
+  if (keep <= m + 1) return false;
+  // the right part: its places hi - 1, hi - 2, ... hold the first FAR entries, place hi the one after them
+  for (int y = keep + tid; y <= hi; y += T) {
+    const int q = source_of_equal(y, m + 1, hi);
+    f(entry(bit_number(words, n_words, q == hi ? hi - m - 1 : hi - 1 - q)));
+  }
+  return true;
 }
 
 // MRD over lists.  Candidate lists longer than CAP set *State::failed: the kernels of planner_mrd.cu do the plan then.

@@ -12,7 +12,7 @@
 // (planner_lists.cuh; tie_order.cuh for lists that do not fit shared memory).
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
 // 250 batches of 600 edges with 20 neighbours, LRU, ms of the kernel: 19.2 with draws, swaps, bitmaps and sort in global
-// memory, 9.9 with those in shared memory, 3.8 with lists in place of the tables' 24,000 entries a batch and without the
+// memory, 9.9 with those in shared memory, 3.5 with lists in place of the tables' 24,000 entries a batch and without the
 // levels of the sort that do not decide.
 #include <algorithm>
 
@@ -192,8 +192,8 @@ __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int c
     uint16_t *left = (uint16_t *)(e + w.cap_shared), *right = left + w.cap_shared;
     for (int i = threadIdx.x; i < n; i += T) e[i] = (uint32_t)key[ids[i]] << lists::IDX_BITS | (uint32_t)i;
     __syncthreads();
-    lists::select_by_order<true>(e, n, count, left, right, (lists::Word *)(right + w.cap_shared), (uint32_t *)s_a, s_b,
-                                 [&](int i) { f(ids[i]); });
+    __shared__ lists::Line s_line;
+    lists::select_by_order<true>(e, n, count, left, right, (uint32_t *)s_a, &s_line, [&](int i) { f(ids[i]); });
     __syncthreads();
     return true;
   }
@@ -322,12 +322,15 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, 
       set_bit(cached, v);
       used_at[v] = arrived[v] = (int32_t)b;
     }
+    // (no more than the budget; a plan that would not fit is listed elsewhere)
+    held = used + min((int64_t)budget, n_nodes) <= plan_cap ? plan + used : w.list[1];
     n_held = list_members(cached, words, held, false, s_a);
     if (used + n_held > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       break;
     }
-    for (int i = tid; i < n_held; i += T) plan[used + i] = held[i];
+    if (held != plan + used)
+      for (int i = tid; i < n_held; i += T) plan[used + i] = held[i];
     if (tid == 0) plan_off[b] = used;
     used += n_held;
     __syncthreads();
