@@ -304,28 +304,43 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
 
 // Message table, times and flags of every node that the group updated, as its last update leaves them (the rows of
 // batches in between are never looked at).  Runs behind the chain and before the memory table is written.
+// An update: 172 pieces of 16 bytes (own memory, other memory, edge features, time encoding).  A group has thousands of them
+// and gives each a warp (a block each waited for one chain of loads after the other: 24 -> 9 us for 6000), a single batch has
+// few and gives each a block of four (5.0 us for 60, 5.4 with a warp each).
+template <int WARPS>
 __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constant__ ChainArgs g) {
   const Args &a = g.a;
   dep_trigger();
   dep_wait();
-  const int part = threadIdx.x / 64, lane = threadIdx.x % 64;
+  constexpr int PIECES = MSG / 4, ROW_PIECES = D / 4;
+  constexpr int LANES = 32 * WARPS;      // of an update
+  const int lane = threadIdx.x % LANES, step = gridDim.x * (blockDim.x / LANES);
   const int n = a.last_at != nullptr ? a.cnt->n_last : a.cnt->n_win[0];
-  for (int l = blockIdx.x; l < n; l += gridDim.x) {
+  for (int l = (blockIdx.x * blockDim.x + threadIdx.x) / LANES; l < n; l += step) {
     const int i = a.last_at != nullptr ? a.last_at[l] : l;
-    const int node = a.win_node[i];
-    const float gap = a.win_gap != nullptr ? a.win_gap[i] : a.win_t[i] - g.mem.last_update[node];
-    float *dst = g.mem.messages + (size_t)node * MSG + part * D;
-    auto row = [&](int r) { return (r >= a.n_nodes ? g.log : g.mem.memory) + (size_t)r * D; };
-    if (part < 3) {
-      const float *src = part == 0 ? row(a.win_mem[i]) : part == 1 ? row(a.win_other[i])
-                                                                  : g.edge_table + (size_t)a.win_eid[i] * D;
-      if (lane < D / 4) reinterpret_cast<float4 *>(dst)[lane] = reinterpret_cast<const float4 *>(src)[lane];
-    } else {
-      for (int d = lane; d < D; d += 64) dst[d] = cos_any(gap * __ldg(g.time_w + d));
+    const int node = a.win_node[i], self = a.win_mem[i], other = a.win_other[i];
+    const float t = a.win_t[i], gap = a.win_gap != nullptr ? a.win_gap[i] : t - g.mem.last_update[node];
+    const float4 *src[3] = {reinterpret_cast<const float4 *>((self >= a.n_nodes ? g.log : g.mem.memory) + (size_t)self * D),
+                            reinterpret_cast<const float4 *>((other >= a.n_nodes ? g.log : g.mem.memory) + (size_t)other * D),
+                            reinterpret_cast<const float4 *>(g.edge_table + (size_t)a.win_eid[i] * D)};
+    constexpr int TURNS = (PIECES + LANES - 1) / LANES;
+    float4 x[TURNS];
+#pragma unroll
+    for (int q = 0; q < TURNS; ++q) {
+      const int at = lane + LANES * q, part = at / ROW_PIECES, c = at - part * ROW_PIECES;
+      if (part < 3) x[q] = src[part][c];
+      else if (at < PIECES) {
+        const float4 w = __ldg(reinterpret_cast<const float4 *>(g.time_w) + c);
+        x[q] = make_float4(cos_any(gap * w.x), cos_any(gap * w.y), cos_any(gap * w.z), cos_any(gap * w.w));
+      }
     }
-    __syncthreads();     // (the last update has been read)
-    if (threadIdx.x == 0) {
-      const float t = a.win_t[i];
+    float4 *dst = reinterpret_cast<float4 *>(g.mem.messages + (size_t)node * MSG);
+#pragma unroll
+    for (int q = 0; q < TURNS; ++q)
+      if (lane + LANES * q < PIECES) dst[lane + LANES * q] = x[q];
+    if (WARPS > 1) __syncthreads();     // (the last update has been read)
+    else __syncwarp();
+    if (lane == 0) {
       g.mem.msg_ts[node] = t;
       g.mem.last_update[node] = t;
       g.mem.msg_flag[node] = 0;
@@ -362,7 +377,8 @@ static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
   cfg.numAttrs = g.a.nb > 1 ? 1 : 0;
   ORCA_CUDA(cudaLaunchKernelEx(&cfg, gru_chain_kernel, g));
   ORCA_COUNT_LAUNCH();
-  ORCA_CUDA(launch_dep(last_messages_kernel, std::min(most, c->sm_count * 4), 256, 0, s, g));
+  if (g.a.nb > 1) ORCA_CUDA(launch_dep(last_messages_kernel<1>, std::min(ceil_div(most, 8), c->sm_count * 6), 256, 0, s, g));
+  else ORCA_CUDA(launch_dep(last_messages_kernel<4>, std::min(most, c->sm_count * 8), 128, 0, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;
