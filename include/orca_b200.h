@@ -594,8 +594,10 @@ typedef struct {
    * batch; see orca_link_metrics_of_parts */
   double *d_metrics, *h_metrics;
 } orca_group_t;
-/* batches worth putting into one group */
+/* batches worth putting into one group, at most */
 int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode);
+/* how to cut a stream of n_batches into groups: their sizes (h_sizes has room for n_batches), returns their number */
+int32_t orca_group_sizes(int32_t n_batches, int32_t bs, int32_t k, int32_t n_layers, int32_t mode, int32_t *h_sizes);
 int64_t orca_group_workspace_bytes(int32_t bs, int32_t nb_max, int32_t k, int32_t u_cap, int32_t plan_cap,
                                    int64_t n_nodes, int32_t n_layers, int32_t mode);
 int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_workspace, int64_t workspace_bytes,

@@ -145,6 +145,7 @@ SYMBOLS = {
     "orca_tgn_eval_epoch": (C.c_int, [C.POINTER(TgnT), C.POINTER(EpochT), _I32, _V, _I64, _V, _I64, _V, _V, _V, _V]),
     "orca_tgn_call": (C.c_int, [C.POINTER(TgnT), C.POINTER(CallT), _I32, _V, _I64, _V, _V, _V, _V, _V]),
     "orca_group_size": (_I32, [_I32, _I32, _I32, _I32]),
+    "orca_group_sizes": (_I32, [_I32, _I32, _I32, _I32, _I32, _V]),
     "orca_group_workspace_bytes": (_I64, [_I32, _I32, _I32, _I32, _I32, _I64, _I32, _I32]),
     "orca_tgn_eval_group": (C.c_int, [C.POINTER(TgnT), C.POINTER(GroupT), _V, _I64, _V, _V, _V, _V]),
     "orca_link_metrics": (C.c_int, [_V, _V, _I64, _I32, _V]),

@@ -21,6 +21,7 @@ from . import _lib
 from .neighbor_finder import NeighborFinder
 
 STRATEGIES = {"MRD": 0, "LRU": 1, "2Q": 2}
+PINNED_FROM = 2 << 20     # bytes of a plan from which it is left in page-locked memory
 
 
 def batch_query_order(sources, destinations, timestamps, bs):
@@ -98,13 +99,14 @@ def plan_device(strategy, nodes, nbr_table, n_edges, bs, k, n_nodes, budget, see
 def _ids_to_host(ids):
     """int32 ids on the device as an int64 array.  They are widened there and stay in the page-locked memory that they are
     copied to: two million ids take 0.4 ms so, 7 as a pageable copy and a conversion, nearly all of it page faults.  More
-    than one plan may hold, or callers may hold together, comes back in ordinary memory."""
+    than one plan may hold, or callers may hold together, comes back in ordinary memory; so does what is not worth a
+    page-locked block of its own (a fresh one takes a few ms, and a plan is kept for as long as its stream is scored)."""
     nbytes = 8 * ids.numel()
     share = None
-    if 0 < nbytes <= NeighborFinder.PINNED_TABLE:
+    if PINNED_FROM <= nbytes <= NeighborFinder.PINNED_TABLE:
         share = NeighborFinder.LENT.take(1 << (nbytes - 1).bit_length())
     if share is None:
-        return ids.cpu().numpy().astype(np.int64)
+        return ids.to(torch.int64).cpu().numpy()
     pin = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
     pin.view(torch.int64).copy_(ids.to(torch.int64), non_blocking=True)
     torch.cuda.current_stream(ids.device).synchronize()

@@ -375,14 +375,35 @@ static inline uint32_t pow2_at_least(uint64_t x) {
   return p;
 }
 
-// Batches per group: enough rows for several tiles of every projection kernel on every SM (48 k rows = 2.6 row
-// blocks of 128 per SM), at most a bit each.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without reuse,
-// by rows of a group: 12 k 3.67 / 3.76 / 8.03 / 5.29, 24 k 3.19 / 3.34 / 7.00 / 3.07, 36 k 3.12 / 3.11 / 6.53 / 2.59, 48 k
-// 3.05 / 3.08 / 6.47 / 2.36, 64 k 3.11 / 3.13 / 6.43 / 2.25, 96 k 3.11 / 3.12 / 6.38 / 2.08: up to 48 k every stream
-// gains, beyond it some lose 2 % (a short stream has too few groups to overlap) and the workspace keeps growing.
+// Batches per group: at most four row blocks of 128 per SM, at most a bit each.  A larger group has fewer partly empty last
+// rounds of row blocks.  What the first group costs before its layers start, index kernels and the memory chain (8 us a
+// batch), is not hidden by anything, so that group is half as large (two blocks per SM; where the chain matters, that is not
+// without reuse), and the rest is dealt out evenly.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
+// reuse / 40 x 200, by rows of a group and of the first: 48 k, one after the other 2.84 / 2.85 / 5.42 / 2.25 / 1.77; 76 k so
+// 2.93 / 2.82 / 5.26 / 2.00 / 1.77; evenly, 49 k and 19 k 2.89 / 2.92 / 5.42 / - / 1.65, 76 k and 19 k 2.87 / 2.84 / 5.22 / - /
+// 1.65, 76 k and 38 k 2.80 / 2.81 / 5.25 / 2.02 / 1.65, 76 k and 57 k 2.85 / 2.91 / 5.33 / - / 1.66, 95 k and 38 k 2.82 / 2.82 /
+// 5.26 / 2.03 / 1.66.
+constexpr int GROUP_ROWS = 4 * 128 * 148, FIRST_ROWS = GROUP_ROWS / 2;
+static int64_t batch_rows(int bs, int k, int layers, int mode) {
+  return 3ll * bs * (layers == 2 && mode == ORCA_MODE_NO_REUSE ? 1 + k : 1);
+}
 static int group_size(int bs, int k, int layers, int mode) {
-  const int64_t rows = 3ll * bs * (layers == 2 && mode == ORCA_MODE_NO_REUSE ? 1 + k : 1);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, 49152 / rows));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, GROUP_ROWS / batch_rows(bs, k, layers, mode)));
+}
+// sizes of the groups of a stream of n batches -> sizes (n entries); their number
+static int group_sizes(int n, int bs, int k, int layers, int mode, int32_t *sizes) {
+  const int most = group_size(bs, k, layers, mode);
+  const int64_t rows = batch_rows(bs, k, layers, mode);
+  int groups = 0, left = n;
+  if (!(layers == 2 && mode == ORCA_MODE_NO_REUSE) && n * rows > 2ll * FIRST_ROWS) {
+    sizes[groups++] = (int)std::max<int64_t>(1, std::min<int64_t>(most, FIRST_ROWS / rows));
+    left -= sizes[0];
+  }
+  for (int rest = ceil_div(left, most); rest > 0; --rest) {
+    sizes[groups] = left / rest;
+    left -= sizes[groups++];
+  }
+  return groups;
 }
 
 // The memory chain is serial, so only what a later batch of the group reads belongs there: in a group of 2000-edge
@@ -515,6 +536,11 @@ extern "C" {
 int32_t orca_group_size(int32_t bs, int32_t k, int32_t n_layers, int32_t mode) {
   if (bs <= 0 || k < 1 || k > ORCA_MAX_K) return -1;
   return grp::group_size(bs, k, n_layers, mode);
+}
+
+int32_t orca_group_sizes(int32_t n_batches, int32_t bs, int32_t k, int32_t n_layers, int32_t mode, int32_t *h_sizes) {
+  if (n_batches <= 0 || bs <= 0 || k < 1 || k > ORCA_MAX_K || h_sizes == nullptr) return -1;
+  return grp::group_sizes(n_batches, bs, k, n_layers, mode, h_sizes);
 }
 
 int64_t orca_group_workspace_bytes(int32_t bs, int32_t nb, int32_t k, int32_t u_cap, int32_t plan_cap, int64_t n_nodes,

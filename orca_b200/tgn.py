@@ -955,7 +955,12 @@ class TGN(nn.Module):
                 h.n_prev[0] = -1
         keep = self.__dict__.setdefault("_group_buffers", {})
         u_cap = min(3 * bs * k, self.n_nodes) if budget else 0
-        nb_max = min(L.orca_group_size(bs, k, self.n_layers, mode), nb)
+        sizes = np.zeros(nb, dtype=np.int32)
+        n_groups = L.orca_group_sizes(nb, bs, k, self.n_layers, mode, sizes.ctypes.data)
+        if n_groups < 0:
+            raise ValueError(f"no groups of batches of {bs} edges with {k} neighbours")
+        ends = np.cumsum(sizes[:n_groups]).tolist()
+        nb_max = int(sizes.max())
         shape = (bs, k, u_cap, self.n_layers, mode, self.n_nodes)
         if keep.get("shape") != shape or keep["nb_max"] < nb_max or keep["plan_cap"] < most:
             if keep.get("shape") == shape:
@@ -991,8 +996,7 @@ class TGN(nn.Module):
             if keep.get("d_parts") is None or keep["d_parts"].numel() < parts * nb:
                 keep["d_parts"] = torch.empty(parts * nb, dtype=torch.float64, device=self.device)
 
-        def prepare(i0):
-            i1 = min(nb, i0 + nb_max)
+        def prepare(i0, i1):
             lo, up = i0 * bs, min(E, i1 * bs)
             hts[lo:up] = timestamps[lo:up]
             for i in range(i0, i1):
@@ -1016,11 +1020,10 @@ class TGN(nn.Module):
                                              h_prob.data_ptr() + 8 * lo, self._status.data_ptr(), stream.cuda_stream))
 
         # a group's index work and memory updates are enqueued ahead of the layers of the group before it
-        starts = range(0, nb, nb_max)
-        prepare(0)
-        for j in range(len(starts)):
-            if j + 1 < len(starts):
-                prepare(starts[j + 1])
+        prepare(0, ends[0])
+        for j in range(n_groups):
+            if j + 1 < n_groups:
+                prepare(ends[j], ends[j + 1])
             g, lo = groups[j]
             g.phase = 2
             enqueue(g, lo)

@@ -22,7 +22,7 @@ def _plan(g, bs, k, budget, strategy, E):
 
 
 # (graph, batch size, k, edges, recursion, layers)
-CASES = [("t_nb2", 37, 10, 5011, "budget", 2),       # 136 batches: five groups, the last one short
+CASES = [("t_nb2", 37, 10, 5011, "budget", 2),       # 136 batches: five groups, the last batch short
          ("t_bip2", 64, 5, 64 * 64, "budget", 2),    # two full groups
          ("t_2q", 1, 10, 70, "budget", 2),           # one edge a batch
          ("t_lru", 300, 20, 5999, "budget", 2),      # k above 16; more rows than a tile of either kernel
@@ -31,7 +31,8 @@ CASES = [("t_nb2", 37, 10, 5011, "budget", 2),       # 136 batches: five groups,
          ("t_nb2", 50, 10, 2030, "none", 2),         # no reuse: a layer-1 row per sampled neighbour
          ("t_lru", 33, 20, 700, "none", 2),
          ("c1", 129, 10, 6000, "budget", 1),
-         ("c1", 600, 10, 20000, "budget", 2)]        # a group whose last updates leave the memory chain, then one without
+         ("c1", 600, 10, 20000, "budget", 2),        # groups whose last updates leave the memory chain
+         ("c1", 512, 10, 16400, "budget", 2)]        # a group without, then one with
 
 
 @pytest.mark.parametrize("name,bs,k,E,recursion,layers", CASES)
