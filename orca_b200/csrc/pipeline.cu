@@ -415,8 +415,12 @@ static Ctx *ctx_of(const orca_tgn_t *m) {
   return m->ctx != nullptr ? reinterpret_cast<Ctx *>(m->ctx) : default_ctx();
 }
 
-// The one-layer model and the recursions without a cache budget: one stream, except for the raw-message /
-// GRU chain, which may run on the side stream once layer 1 no longer reads the memory table.
+// The one-layer model and the recursions without a cache budget: one stream, except for the raw messages and the memory
+// update on the side stream.  They read the same memory rows as layer 1; only the write of the memory table waits for
+// layer 1 to have read it.  In a one-layer model they run beside the layer from the start (us a call, behind the scores /
+// beside the layer: 37 edges 97 / 70, 200 101 / 76, 700 118 / 86, 1024 128 / 93, 2000 154 / 106, 4000 207 / 177).  With two
+// layers they run beside layer 2, which leaves more of the chip (beside layer 1, without reuse: 1000 edges 332 -> 338, 2000
+// 537 -> 569; unlimited reuse: 153 -> 158, 192 -> 192).
 static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, const double *d_batch_ts, int b,
                        int u_cap, Workspace &w, float *d_prob, float *d_emb_out, int32_t *d_status, cudaStream_t s) {
   const int k = m->k;
@@ -436,9 +440,37 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   ORCA_TRY(tr.mark(PH_PREP, s));
+  const bool beside = c->overlap && !tr.on;
+  cudaStream_t ms = beside ? c->aux : s;
+  if (beside && m->n_layers == 1) ORCA_CUDA(cudaEventRecord(c->fork, s));
+  // raw messages of the batch (last occurrence per node in [src|dst]) and the new memory rows
+  const bool single = one_launch_updates(b);
+  auto update = [&]() -> int {
+    if (beside) ORCA_CUDA(cudaStreamWaitEvent(ms, c->fork, 0));
+    ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, *m->epoch_base, x.win_pos, x.n_win,
+                                     d_status, ms, updates_of(x, d_batch_ts)));
+    *m->epoch_base += 2 * b;
+    ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
+    if (single) {
+      ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid,
+                                      x.upd_t, x.cnt, w.upd_image, w.gru_h, ms));
+    } else {
+      ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
+                                  d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, ms));
+      ORCA_TRY(gru_project(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, w.gru_h, ms));
+    }
+    ORCA_TRY(tr.mark(PH_MESSAGE, s));
+    return ORCA_OK;
+  };
+  // the memory table is written (layer 1 has read it)
+  auto write_memory = [&]() -> int {
+    if (single) ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, ms));
+    else ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, ms));
+    ORCA_TRY(tr.mark(PH_GRU, s));
+    return ORCA_OK;
+  };
 
   float *emb_top = d_emb_out ? d_emb_out : w.emb2;
-  bool forked = false;
   if (m->n_layers == 1) {
     ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1, x.ts1, N,
                               nullptr, k, x.nbr1, x.eid1, nullptr, x.dt1, d_status, s));
@@ -447,8 +479,14 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     ORCA_TRY(tr.mark(PH_QUERY_L2, s));
     ORCA_TRY(layer_gather(m, m->mem.memory, x.nbr1, x.eid1, x.dt1, N, nullptr, 0, nullptr, l, tk, s));
     ORCA_TRY(tr.mark(PH_GATHER_L2, s));
+    // (given to the GPU now: the layer's first kernels come before it, its longest one beside it)
+    if (beside) ORCA_TRY(update());
     ORCA_TRY(layer_output(&m->attn[0], l, m->mem.memory, x.nodes1, N, nullptr, emb_top, Push{}, s));
     ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
+    if (beside) {
+      ORCA_TRY(link(s, ms, c->ev_o1));
+      ORCA_TRY(write_memory());
+    }
   } else {
     // top-level neighbour table; then the row list of layer 1 by recursion mode
     const int32_t *nbr1 = x.nbr1, *eid1 = x.eid1, *gather2 = x.nbr2;
@@ -491,10 +529,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     ORCA_TRY(layer_output(&m->attn[0], l, m->mem.memory, x.nodes1, R1, d_n1, w.emb1[0],
                           push1 ? Push{m->hist_emb, x.nodes1, w.win1} : Push{}, s, nullptr, w.feat2[0], N));
     ORCA_TRY(tr.mark(PH_OUTPUT_L1, s));
-    if (c->overlap && !tr.on) {
-      ORCA_TRY(link(s, c->aux, c->fork));
-      forked = true;
-    }
+    if (beside) ORCA_CUDA(cudaEventRecord(c->fork, s));
     ORCA_TRY(tr.mark(PH_FLAGS, s));
     LaneBuf l2 = l;
     l2.feat = w.feat2[0];
@@ -509,26 +544,11 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
   ORCA_TRY(orca_score(&m->score, emb_top, b, d_prob, s));
   ORCA_TRY(tr.mark(PH_SCORE, s));
 
-  // raw messages of the batch (last occurrence per node in [src|dst]) and the memory update
-  cudaStream_t ms = forked ? c->aux : s;
-  const bool single = one_launch_updates(b);
-  ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, *m->epoch_base, x.win_pos, x.n_win,
-                                   d_status, ms, updates_of(x, d_batch_ts)));
-  *m->epoch_base += 2 * b;
-  ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
-  if (single) {
-    ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid, x.upd_t,
-                                    x.cnt, w.upd_image, w.gru_h, ms));
-    ORCA_TRY(tr.mark(PH_MESSAGE, s));
-    ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, ms));
-  } else {
-  ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
-                              d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, ms));
-  ORCA_TRY(tr.mark(PH_MESSAGE, s));
-  ORCA_TRY(orca_gru_update(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, ms));
+  if (!beside || m->n_layers == 2) {
+    ORCA_TRY(update());
+    ORCA_TRY(write_memory());
   }
-  ORCA_TRY(tr.mark(PH_GRU, s));
-  if (forked) ORCA_TRY(link(c->aux, s, c->join));
+  if (beside) ORCA_TRY(link(ms, s, c->join));
   publish_counts_kernel<<<1, 1, 0, s>>>(x.n1, x.n_win, d_status);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
