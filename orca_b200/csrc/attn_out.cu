@@ -3,15 +3,14 @@
 //
 // The rows come as an operand image (attn_out.cuh): bf16 heads and tails, split once by the kernels that computed them,
 // in the form the tensor core reads.  So the main loop is nothing but bulk copies and MMAs: one thread streams stages
-// of 32 K columns through a ring, one multiplies, eight warps do the two epilogues -- of one row block while the stages of
-// the next are already landing.  A block of 128 rows takes 39 stages of 6 MMAs (10.5 us of tensor time).
-// What bounds it is what L2 gives all SMs together, 7.5 TB/s: more stages in flight (five slots of 38 KB instead of three)
-// gained nothing.  So CTAs work in pairs (cta_group::2): 256 rows, each CTA with its own 128 and half of the weights' columns,
-// 27 KB a stage instead of 38.  Copies are each CTA's own; a thread of rank 1 passes on what has landed there, rank 0 issues
-// for both.  (Those arrivals must not be release.cluster: a fence a stage, 129 us.)  48 k rows: 82 us with a CTA a block, 72
-// here; the general projection kernel, whose producer warps load fp32 rows, convert and store them stage by stage, takes
-// 49 us per block whatever the number of blocks.  The ring has four slots; seven for the first product of the first
-// blocks, while the room of the hidden tile is still unused: a launch of few blocks waits for these loads.
+// of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three (of five for the first product of a CTA's
+// first block, while the room of the hidden tile is still unused: a launch of few blocks waits for these loads), one
+// thread multiplies, eight warps do the two epilogues -- of one row block while the stages of the next are already
+// landing.  A block of 128 rows takes 39
+// stages of 6 MMAs (10.5 us of tensor time) and 1.5 MB from L2.  The general projection kernel, whose producer warps
+// load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; 51 k
+// rows: 145 us with it, 82 to 86 here, where the bound is what three slots keep in flight: 114 KB an SM at 7.3 TB/s from L2
+// (58 % of it weights) is a round trip of 2.3 us; tensor pipe 42 %, DRAM 41 %, L2 27 % busy.
 // Between the two products the hidden tile stays on the SM (bias + ReLU, split, A image of the second product), and
 // the second product's accumulators reuse the first one's columns.
 // Warp 0: copies.  Warp 1: tensor memory, MMA issue.  Warps 2-9: epilogues (thread = row, then warp = row).
@@ -25,17 +24,16 @@ namespace orca {
 namespace ao {
 
 constexpr int BM = img::ROWS, BN = 176;
-constexpr int STAGES = 4;
-constexpr int HALF = BN / 2;                       // weight columns in each CTA of a pair
-constexpr int A_STAGE = img::STAGE_BYTES, W_LBO = HALF * 16, W_STAGE = 2 * 4 * W_LBO, STAGE = A_STAGE + W_STAGE;
+constexpr int STAGES = 3;
+constexpr int A_STAGE = img::STAGE_BYTES, W_LBO = BN * 16, W_STAGE = 2 * 4 * W_LBO, STAGE = A_STAGE + W_STAGE;
 constexpr int K_STAGES = img::CTX_STAGES + img::FEAT_STAGES;                     // 39
 constexpr int K2_CHUNKS = BN / 8, K2_STAGES = (K2_CHUNKS + 3) / 4;               // 22, 6
 constexpr int A2_LBO = BM * 16 + 16, A2_BYTES = K2_CHUNKS * A2_LBO;
 constexpr int TILE_LD = 180;                       // floats per row of the output tile (conflict-free 16-byte stores)
 constexpr int FRONT = 90 * 1024;                   // hidden image, then output tile
 static_assert(2 * A2_BYTES <= FRONT && BM * TILE_LD * 4 <= FRONT && STAGE % 1024 == 0, "");
-constexpr int FIRST = 7;                           // stages of the first product of a CTA's first block
-static_assert((FIRST - STAGES) * STAGE <= FRONT && K_STAGES % FIRST == STAGES, "");
+constexpr int FIRST = 5;                           // stages of the first product of a CTA's first block
+static_assert((FIRST - STAGES) * STAGE <= FRONT && K_STAGES % FIRST == FIRST - 1, "");
 constexpr int FIRST_USES = K_STAGES / FIRST + 1;   // of each of the first STAGES slots
 constexpr int SMEM = FRONT + STAGES * STAGE + 1024;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
@@ -43,23 +41,18 @@ constexpr int TMEM_COLS = 512, SMALL = 256;
 
 using img::desc_sw64;
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-attn_output_image_kernel(const __grid_constant__ OutArgs g) {
+__global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __grid_constant__ OutArgs g) {
   using namespace tc;
   extern __shared__ unsigned char raw[];
   __shared__ __align__(16) float s_b1[BN], s_g[BN], s_b2[BN], s_lw[BN], s_lb[BN];
-  __shared__ __align__(8) unsigned long long s_bar[3 * FIRST + 4];
+  __shared__ __align__(8) unsigned long long s_bar[2 * FIRST + 4];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u, ring = base + FRONT;
   auto full = [&](int s) { return smem_addr(&s_bar[s]); };
   auto empty = [&](int s) { return smem_addr(&s_bar[FIRST + s]); };
-  auto full2 = [&](int s) { return smem_addr(&s_bar[2 * FIRST + s]); };      // (rank 0: the other CTA's stage has landed)
-  const uint32_t acc1 = smem_addr(&s_bar[3 * FIRST]), a2bar = smem_addr(&s_bar[3 * FIRST + 1]),
-                 acc2 = smem_addr(&s_bar[3 * FIRST + 2]), tfree = smem_addr(&s_bar[3 * FIRST + 3]);
-  const uint32_t rank = cta_rank();
-  // row blocks: 2 * pair + rank, and on by the number of CTAs.  Both CTAs take as many turns as there are blocks of rank 0
-  const int blk0 = blockIdx.x - (int)rank;
+  const uint32_t acc1 = smem_addr(&s_bar[2 * FIRST]), a2bar = smem_addr(&s_bar[2 * FIRST + 1]),
+                 acc2 = smem_addr(&s_bar[2 * FIRST + 2]), tfree = smem_addr(&s_bar[2 * FIRST + 3]);
   // stage number `it` of this CTA: its slot, how often the slot was used before, and where it lies
   auto slot_of = [&](int it) { return it < K_STAGES ? it % FIRST : (it - K_STAGES) % STAGES; };
   auto use_of = [&](int it) { return it < K_STAGES ? it / FIRST : FIRST_USES + (it - K_STAGES) / STAGES; };
@@ -69,19 +62,18 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
     for (int s = 0; s < FIRST; ++s) {
       mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
-      mbar_init(full2(s), 1);
     }
     mbar_init(acc1, 1);
-    mbar_init(a2bar, 2 * EPI_WARPS);
+    mbar_init(a2bar, EPI_WARPS);
     mbar_init(acc2, 1);
-    mbar_init(tfree, 2 * EPI_WARPS);
+    mbar_init(tfree, EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
                  "r"(TMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   for (int i = tid; i < BN; i += THREADS) {
     const bool in = i < D;
@@ -94,8 +86,7 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
   dep_wait();
   const int M = rows_of(g.n_cap, g.d_n);
   tc_fence_before();
-  __syncwarp();
-  cluster_barrier();       // (barriers and tensor memory of both are ready)
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_tmem, 0);
   bool alive = true;
@@ -106,9 +97,7 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
       const char *w1 = reinterpret_cast<const char *>(g.w.G_img), *w2 = reinterpret_cast<const char *>(g.w.W2_img);
       const uint64_t once = policy_evict_first();      // (the rows are not read again: 1 % of a stream)
       int it = 0;
-      for (int b0 = blk0; b0 * BM < M; b0 += gridDim.x) {
-        const int blk = b0 + (int)rank;
-        const bool rows = blk * BM < M;      // (a pair's second block may not exist: its half of the weights is wanted all the same)
+      for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x) {
         const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
         const char *feat = g.feat + (size_t)blk * img::FEAT_STAGES * A_STAGE;
         for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
@@ -116,44 +105,30 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
           const uint32_t at = place(s);
           mbar_wait(empty(s), (use_of(it) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
           if (st < K_STAGES) {
-            mbar_expect_tx(full(s), rows ? STAGE : W_STAGE);
-            if (rows)
-              bulk_g2s_hint(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
-                            A_STAGE, full(s), once);
-            bulk_g2s(at + A_STAGE, w1 + (size_t)(2 * st + (int)rank) * W_STAGE, W_STAGE, full(s));
+            mbar_expect_tx(full(s), STAGE);
+            bulk_g2s_hint(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
+                          A_STAGE, full(s), once);
+            bulk_g2s(at + A_STAGE, w1 + (size_t)st * W_STAGE, W_STAGE, full(s));
           } else {
             mbar_expect_tx(full(s), W_STAGE);
-            bulk_g2s(at + A_STAGE, w2 + (size_t)(2 * (st - K_STAGES) + (int)rank) * W_STAGE, W_STAGE, full(s));
+            bulk_g2s(at + A_STAGE, w2 + (size_t)(st - K_STAGES) * W_STAGE, W_STAGE, full(s));
           }
         }
       }
     }
     __syncwarp();
-  } else if (warp == 1 && rank != 0) {
-    // ------------------------------------------------------------------ tells rank 0 what has landed here
-    if (lane == 0) {
-      int it = 0;
-      for (int b0 = blk0; b0 * BM < M; b0 += gridDim.x)
-        for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
-          const int s = slot_of(it);
-          mbar_wait(full(s), use_of(it) & 1, g.status, 730, alive, g.wait_limit);
-          mbar_arrive_at(full2(s), 0);
-        }
-    }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issue
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     int it = 0, t = 0;
-    for (int b0 = blk0; b0 * BM < M; b0 += gridDim.x, ++t) {
-      if (t > 0) mbar_wait_cluster(tfree, (t - 1) & 1, g.status, 710, alive, g.wait_limit);
+    for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x, ++t) {
+      if (t > 0) mbar_wait(tfree, (t - 1) & 1, g.status, 710, alive, g.wait_limit);
       tc_fence_after();
       for (int st = 0; st < K_STAGES; ++st, ++it) {
         const int s = slot_of(it);
         const uint32_t a = place(s), w = a + A_STAGE;
         const bool half = st == img::CTX_STAGES - 1 || st == K_STAGES - 1;     // (the second step is nothing but padding)
         mbar_wait(full(s), use_of(it) & 1, g.status, 711, alive, g.wait_limit);
-        mbar_wait_cluster(full2(s), use_of(it) & 1, g.status, 714, alive, g.wait_limit);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -162,22 +137,21 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
             const uint64_t ah = desc_sw64(a + ks * 32), al = desc_sw64(a + A_STAGE / 2 + ks * 32);
             const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
             const uint32_t more = (st > 0 || ks > 0) ? 1u : 0u;
-            mma_bf16_pair(tmem, ah, bh, idesc, more);
-            mma_bf16_pair(tmem + SMALL, al, bh, idesc, more);
-            mma_bf16_pair(tmem + SMALL, ah, bl, idesc, 1u);
+            mma_bf16(tmem, ah, bh, idesc, more);
+            mma_bf16(tmem + SMALL, al, bh, idesc, more);
+            mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit_pair(empty(s));
-          if (st == K_STAGES - 1) mma_commit_pair(acc1);
+          mma_commit(empty(s));
+          if (st == K_STAGES - 1) mma_commit(acc1);
         }
         __syncwarp();
       }
-      mbar_wait_cluster(a2bar, t & 1, g.status, 712, alive, g.wait_limit);
+      mbar_wait(a2bar, t & 1, g.status, 712, alive, g.wait_limit);
       tc_fence_after();
       for (int st = 0; st < K2_STAGES; ++st, ++it) {
         const int s = slot_of(it);
         const uint32_t w = place(s) + A_STAGE, a = base + st * 4 * A2_LBO;
         mbar_wait(full(s), use_of(it) & 1, g.status, 713, alive, g.wait_limit);
-        mbar_wait_cluster(full2(s), use_of(it) & 1, g.status, 715, alive, g.wait_limit);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -187,12 +161,12 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
             const uint64_t al = make_desc(a + A2_BYTES + ks * 2 * A2_LBO, A2_LBO, 128);
             const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
             const uint32_t more = (st > 0 || ks > 0) ? 1u : 0u;
-            mma_bf16_pair(tmem, ah, bh, idesc, more);
-            mma_bf16_pair(tmem + SMALL, al, bh, idesc, more);
-            mma_bf16_pair(tmem + SMALL, ah, bl, idesc, 1u);
+            mma_bf16(tmem, ah, bh, idesc, more);
+            mma_bf16(tmem + SMALL, al, bh, idesc, more);
+            mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit_pair(empty(s));
-          if (st == K2_STAGES - 1) mma_commit_pair(acc2);
+          mma_commit(empty(s));
+          if (st == K2_STAGES - 1) mma_commit(acc2);
         }
         __syncwarp();
       }
@@ -207,8 +181,8 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
     const float4 f4z = make_float4(0.f, 0.f, 0.f, 0.f);
     auto vec = [&](const float *s, int j, bool on) { return on ? *reinterpret_cast<const float4 *>(s + 4 * j) : f4z; };
     int t = 0;
-    for (int b0 = blk0; b0 * BM < M; b0 += gridDim.x, ++t) {
-      const int m0 = (b0 + (int)rank) * BM, m_rows = min(BM, M - m0);      // (none or less: no rows here)
+    for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x, ++t) {
+      const int m0 = blk * BM, m_rows = min(BM, M - m0);
       const float on = (row < m_rows && (g.valid == nullptr || g.valid[m0 + row] != 0)) ? 1.f : 0.f;
       // history push: lane i holds what row ew + 8 * i of the output pass needs
       int push_id = 0, push = 0;
@@ -238,7 +212,7 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
       fence_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(a2bar, 0);
+      if (lane == 0) mbar_arrive(a2bar);
       // second: accumulators -> row-major tile (over the hidden image, which has been read), then whole rows
       mbar_wait(acc2, t & 1, g.status, 721, alive, g.wait_limit);
       tc_fence_after();
@@ -252,7 +226,7 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(tfree, 0);
+      if (lane == 0) mbar_arrive(tfree);
       asm volatile("bar.sync 1, 256;" ::: "memory");
       constexpr int RB = 4;     // rows in flight per warp
       for (int i0 = 0; i0 < BM / EPI_WARPS; i0 += RB) {
@@ -310,11 +284,10 @@ attn_output_image_kernel(const __grid_constant__ OutArgs g) {
     }
   }
   tc_fence_before();
-  __syncwarp();
-  cluster_barrier();       // (neither CTA leaves while the other may still arrive on its barriers or read its shared memory)
+  __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
   if (g.peer.world > 0) {
     // every CTA (with or without rows) checks out; the last one posts the batch's sequence number to all ranks, after
@@ -346,8 +319,7 @@ int attn_output_rows(const OutArgs &args, cudaStream_t s) {
   OutArgs g = args;
   g.status = c->status_word;
   g.wait_limit = c->wait_limit;
-  // pairs of CTAs; one wave
-  const int grid = 2 * std::min(ceil_div(g.n_cap, 2 * ao::BM), c->sm_count / 2);
+  const int grid = std::min(ceil_div(g.n_cap, ao::BM), c->sm_count);
   ORCA_CUDA(launch_dep(ao::attn_output_image_kernel, grid, ao::THREADS, ao::SMEM, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();

@@ -97,63 +97,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-
-// ---- a pair of CTAs (cluster of two) as one tensor-core unit: 256 rows, of which each CTA holds 128 in its own shared and
-// tensor memory; each holds half of the columns of B.  The CTA of rank 0 issues.
-__device__ __forceinline__ uint32_t cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// arrives on the barrier at the same place in CTA `rank` of the cluster
-__device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t rank) {
-  asm volatile(
-      "{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\n"
-      "mbarrier.arrive.shared::cluster.b64 _, [a];\n}\n" ::"r"(bar),
-      "r"(rank)
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// mbar_wait for a barrier that the other CTA arrives on, too
-__device__ __forceinline__ void mbar_wait_cluster(uint32_t bar, uint32_t parity, int32_t *status, int where, bool &alive,
-                                                  long long limit) {
-  if (!alive) return;
-  if (mbar_try_cluster(bar, parity)) return;
-  const long long t0 = clock64();
-  while (!mbar_try_cluster(bar, parity)) {
-    if (clock64() - t0 > limit) {
-      report(status, ORCA_E_TIMEOUT, where);
-      alive = false;
-      return;
-    }
-  }
-}
-__device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// on the barrier at this place in both CTAs
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
-      : "memory");
-}
 // 16 consecutive accumulator columns of this thread's lane (= tile row); complete after tcgen05.wait::ld
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(

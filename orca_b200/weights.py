@@ -68,11 +68,10 @@ def pack_query(W):
 
 def pack_stages(*parts):
     """Weights with 172 columns for csrc/attn_out.cu: the parts one below the other, each padded to a multiple of 32
-    rows; one stage per 32 rows, each [columns 0 .. 87 | 88 .. 175][head | tail][4 chunks][88 columns][8] (a half for each
-    CTA of a pair)."""
+    rows; one stage per 32 rows, each [head | tail][4 chunks][176 columns][8]."""
     at = np.cumsum([0] + [-(-len(p) // 32) * 32 for p in parts])
     return _packed(list(zip(parts, at[:-1])), (int(at[-1]), TC_BN),
-                   lambda X: X.reshape(2, -1, 4, 8, 2, TC_BN // 2).permute(1, 4, 0, 2, 5, 3))
+                   lambda X: X.reshape(2, -1, 4, 8, TC_BN).permute(1, 0, 2, 4, 3))
 
 
 def pack_gru(Wg, dim=D):
