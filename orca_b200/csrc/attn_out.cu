@@ -9,8 +9,10 @@
 // landing.  A block of 128 rows takes 39
 // stages of 6 MMAs (10.5 us of tensor time) and 1.5 MB from L2.  The general projection kernel, whose producer warps
 // load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; 51 k
-// rows: 145 us with it, 82 to 86 here, where the bound is what three slots keep in flight: 114 KB an SM at 7.3 TB/s from L2
-// (58 % of it weights) is a round trip of 2.3 us; tensor pipe 42 %, DRAM 41 %, L2 27 % busy.
+// rows: 145 us with it, 82 to 86 here, where the bound is what L2 gives all SMs together, 7.3 TB/s, 58 % of it weights
+// (tensor pipe 42 %, DRAM 41 %): five slots instead of three gain nothing.  Pairs of CTAs with half of the weights each
+// (cta_group::2) take 72 us, but wait for two free SMs side by side: 50 batches of 2000 1.2 % faster, single calls of 3000
+// and 4000 edges with 20 neighbours 13 and 8 % slower.
 // Between the two products the hidden tile stays on the SM (bias + ReLU, split, A image of the second product), and
 // the second product's accumulators reuse the first one's columns.
 // Warp 0: copies.  Warp 1: tensor memory, MMA issue.  Warps 2-9: epilogues (thread = row, then warp = row).

@@ -381,7 +381,7 @@ static inline uint32_t pow2_at_least(uint64_t x) {
 // without reuse), and the rest is dealt out evenly.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
 // reuse / 40 x 200, by rows of a group and of the first: 48 k, one after the other 2.84 / 2.85 / 5.42 / 2.25 / 1.77; 76 k so
 // 2.93 / 2.82 / 5.26 / 2.00 / 1.77; evenly, 49 k and 19 k 2.89 / 2.92 / 5.42 / - / 1.65, 76 k and 19 k 2.87 / 2.84 / 5.22 / - /
-// 1.65, 76 k and 38 k 2.80 / 2.81 / 5.25 / 2.02 / 1.65, 76 k and 57 k 2.85 / 2.91 / 5.33 / - / 1.66, 95 k and 38 k 2.82 / 2.82 /
+// 1.65, 76 k and 38 k 2.80 / 2.81 / 5.25 / 2.02 / 1.65 (2.86 / 2.85 / 5.44 / 2.04 / 1.67 with the output kernel as it is), 76 k and 57 k 2.85 / 2.91 / 5.33 / - / 1.66, 95 k and 38 k 2.82 / 2.82 /
 // 5.26 / 2.03 / 1.66.
 constexpr int GROUP_ROWS = 4 * 128 * 148, FIRST_ROWS = GROUP_ROWS / 2;
 static int64_t batch_rows(int bs, int k, int layers, int mode) {
