@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
 // Message table, times and flags of every node that the group updated, as its last update leaves them (the rows of
 // batches in between are never looked at).  Runs behind the chain and before the memory table is written.
 // An update: 172 pieces of 16 bytes (own memory, other memory, edge features, time encoding).  A group has thousands of them
-// and gives each a warp (a block each waited for one chain of loads after the other: 24 -> 9 us for 6000), a single batch has
-// few and gives each a block of four (5.0 us for 60, 5.4 with a warp each).
+// and gives each a warp (a block each waited for one chain of loads after the other: 24 -> 9 us for 6000); where all can have
+// a block of four side by side, they do (5.0 us for 60, 5.4 with a warp each).
 template <int WARPS>
 __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constant__ ChainArgs g) {
   const Args &a = g.a;
@@ -377,7 +377,7 @@ static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
   cfg.numAttrs = g.a.nb > 1 ? 1 : 0;
   ORCA_CUDA(cudaLaunchKernelEx(&cfg, gru_chain_kernel, g));
   ORCA_COUNT_LAUNCH();
-  if (g.a.nb > 1) ORCA_CUDA(launch_dep(last_messages_kernel<1>, std::min(ceil_div(most, 8), c->sm_count * 6), 256, 0, s, g));
+  if (g.a.nb > 1 && most > c->sm_count * 8) ORCA_CUDA(launch_dep(last_messages_kernel<1>, std::min(ceil_div(most, 8), c->sm_count * 6), 256, 0, s, g));
   else ORCA_CUDA(launch_dep(last_messages_kernel<4>, std::min(most, c->sm_count * 8), 128, 0, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();

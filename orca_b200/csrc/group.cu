@@ -301,8 +301,9 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
 }
 
 // ------------------------------------------------------------------------------------------------ last versions
-// A warp takes eight items, memory rows first and then layer-1 rows: its lanes look them up side by side, and what is to be
-// copied goes four rows at a time.  (64 threads an item, one chain of lookups after the other: 20 us for 50 k rows, 10 so.)
+// A warp takes up to eight items, memory rows first and then layer-1 rows: its lanes look them up side by side, and what is
+// to be copied goes four rows at a time.  (64 threads an item, one chain of lookups after the other: 20 us for 50 k rows,
+// 10 so.)  Where there are fewer items than eight a warp, they are spread over all warps.
 __global__ void __launch_bounds__(256)
 write_back_kernel(const __grid_constant__ Args a, const float *log, const float *emb1, float *memory, float *history,
                   int32_t *h_status) {
@@ -310,14 +311,15 @@ write_back_kernel(const __grid_constant__ Args a, const float *log, const float 
   dep_wait();
   // the last kernel of the group: what the others have reported goes straight to the host
   if (h_status != nullptr && blockIdx.x == 0 && threadIdx.x < 4) h_status[threadIdx.x] = __ldcg(a.status + threadIdx.x);
-  constexpr int ITEMS = 8, ROWS = 4, PIECES = D / 4;
+  constexpr int MOST = 8, ROWS = 4, PIECES = D / 4;
   const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
   const int n_upd = a.cnt->n_last, batch_rows = 3 * a.edges();
   const int n_items = n_upd + (a.keeps_history() ? a.cnt->n_rows : 0);
-  for (int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ITEMS; i0 < n_items; i0 += warps * ITEMS) {
+  const int items = min(MOST, (n_items + warps - 1) / warps);
+  for (int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * items; i0 < n_items; i0 += warps * items) {
     const int i = i0 + lane;
     int to = -1, from = 0;      // this lane's row: where it goes (history: behind the memory rows), where it lies
-    if (lane < ITEMS && i < n_items) {
+    if (lane < items && i < n_items) {
       if (i < n_upd) {
         to = a.last_node[i];
         from = a.log_base + a.last_at[i];
@@ -379,10 +381,12 @@ static inline uint32_t pow2_at_least(uint64_t x) {
 // rounds of row blocks.  What the first group costs before its layers start, index kernels and the memory chain (8 us a
 // batch), is not hidden by anything, so that group is half as large (two blocks per SM; where the chain matters, that is not
 // without reuse), and the rest is dealt out evenly.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
-// reuse / 40 x 200, by rows of a group and of the first: 48 k, one after the other 2.84 / 2.85 / 5.42 / 2.25 / 1.77; 76 k so
-// 2.93 / 2.82 / 5.26 / 2.00 / 1.77; evenly, 49 k and 19 k 2.89 / 2.92 / 5.42 / - / 1.65, 76 k and 19 k 2.87 / 2.84 / 5.22 / - /
-// 1.65, 76 k and 38 k 2.80 / 2.81 / 5.25 / 2.02 / 1.65 (2.86 / 2.85 / 5.44 / 2.04 / 1.67 with the output kernel as it is), 76 k and 57 k 2.85 / 2.91 / 5.33 / - / 1.66, 95 k and 38 k 2.82 / 2.82 /
-// 5.26 / 2.03 / 1.66.
+// reuse / 40 x 200, by rows of a group and of the first (all with an output kernel on pairs of CTAs):
+//   48 k, one after the other  2.84 / 2.85 / 5.42 / 2.25 / 1.77      76 k so           2.93 / 2.82 / 5.26 / 2.00 / 1.77
+//   evenly, 49 k and 19 k      2.89 / 2.92 / 5.42 /  -   / 1.65      76 k and 19 k     2.87 / 2.84 / 5.22 /  -   / 1.65
+//   76 k and 38 k              2.80 / 2.81 / 5.25 / 2.02 / 1.65      76 k and 57 k     2.85 / 2.91 / 5.33 /  -   / 1.66
+//   95 k and 38 k              2.82 / 2.82 / 5.26 / 2.03 / 1.66
+// With the output kernel as it is, 76 k and 38 k: 2.86 / 2.85 / 5.44 / 2.04 / 1.67.
 constexpr int GROUP_ROWS = 4 * 128 * 148, FIRST_ROWS = GROUP_ROWS / 2;
 static int64_t batch_rows(int bs, int k, int layers, int mode) {
   return 3ll * bs * (layers == 2 && mode == ORCA_MODE_NO_REUSE ? 1 + k : 1);
