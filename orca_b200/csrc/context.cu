@@ -95,6 +95,14 @@ Ctx *default_ctx() {
   return of_device[dev];
 }
 
+int settled(int rc, Ctx *c, cudaStream_t s) {
+  if (rc == ORCA_OK) return rc;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) return rc;
+  for (cudaStream_t x : {c->copy, c->idx, c->lane1, c->aux, s}) cudaStreamSynchronize(x);
+  return rc;
+}
+
 Ctx *cur() { return g_cur != nullptr ? g_cur : default_ctx(); }
 
 CtxScope::CtxScope(Ctx *c) : prev(g_cur) { g_cur = c; }

@@ -84,6 +84,10 @@ Ctx *default_ctx();
 // device memory in the order of stream s for entry points whose callers bring no scratch, given back with cudaFreeAsync;
 // the context keeps up to 64 MB of it between calls.  nullptr: there is none to be had.
 void *scratch_alloc(Ctx *c, size_t bytes, cudaStream_t s);
+// How the entry points that spread work over the context's streams end: a call that fails half-way has enqueued kernels on
+// streams that it never joined, which the next call would not wait for although it lays its rows into the same buffers.  So
+// they are waited for here, before the error is returned.  (Not under capture: nothing runs, and the capture cannot end well.)
+int settled(int rc, Ctx *c, cudaStream_t s);
 struct CtxScope {
   Ctx *prev;
   explicit CtxScope(Ctx *c);

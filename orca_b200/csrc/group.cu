@@ -709,7 +709,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   const int rc = body();
   c->status_word = saved_status;
   c->last_batch_launches = launch_counter();
-  return rc;
+  return settled(rc, c, s);
 }
 
 }  // extern "C"

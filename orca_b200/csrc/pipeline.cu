@@ -935,7 +935,7 @@ int orca_tgn_eval_batch(const orca_tgn_t *m, const int32_t *d_batch_i32, const d
   }
   c->status_word = saved_status;
   c->last_batch_launches = launch_counter();
-  return rc;
+  return settled(rc, c, (cudaStream_t)stream);
 }
 
 int orca_tgn_eval_batch_sharded(const orca_tgn_t *m, int32_t phase, const int32_t *d_batch_i32,
@@ -967,7 +967,7 @@ int orca_tgn_eval_batch_sharded(const orca_tgn_t *m, int32_t phase, const int32_
                              d_emb1_local, d_emb1_all, d_prob_local, d_emb2_local, d_status, (cudaStream_t)stream);
   c->status_word = saved_status;
   if (phase != 1) c->last_batch_launches = launch_counter();
-  return rc;
+  return settled(rc, c, (cudaStream_t)stream);
 }
 
 int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_cap, void *d_workspace,
@@ -986,7 +986,7 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
   const int64_t slot_bytes = (stage_bytes / kSlots) & ~(int64_t)255;
   orca_tgn_t mm = *m;
   mm.input_stream = c->copy;
-  for (int64_t i = 0; i < e->n_batches; ++i) {
+  auto batch = [&](int64_t i) -> int {
     const int b = e->b[i], n_plan = e->n_plan[i];
     ORCA_CHECK_ARG(b > 0);
     const int64_t bytes_i32 = ((int64_t)4 * b + (n_plan > 0 ? n_plan : 0)) * 4;
@@ -1023,8 +1023,11 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
       ORCA_CUDA(cudaMemcpyAsync(h_prob + e->off_prob[i], prob, (size_t)n_scores * 4, cudaMemcpyDeviceToHost, s));
     ORCA_CUDA(cudaEventRecord(c->ev_slot[slot], s));
     c->slot_used[slot] = true;
-  }
-  return ORCA_OK;
+    return ORCA_OK;
+  };
+  int rc = ORCA_OK;
+  for (int64_t i = 0; rc == ORCA_OK && i < e->n_batches; ++i) rc = batch(i);
+  return settled(rc, c, s);
 }
 
 // The whole of one call with host arrays: narrowed into the call's pinned slot, copied on the copy stream, computed, the
@@ -1055,14 +1058,18 @@ int orca_tgn_call(const orca_tgn_t *m, const orca_call_t *a, int32_t u_cap, void
   ORCA_TRY(check_batch_ids(m, (const int32_t *)h, b, 0, "orca_tgn_call"));
   if (n_plan > 0) narrow(a->plan, n_plan);
   memcpy(h + off_ts, a->ts, (size_t)b * 8);
-  ORCA_CUDA(cudaMemcpyAsync(d, h, (size_t)bytes, cudaMemcpyHostToDevice, c->copy));
-  orca_tgn_t mm = *m;
-  mm.input_stream = c->copy;
-  ORCA_TRY(orca_tgn_eval_batch(&mm, (const int32_t *)d, (const double *)(d + off_ts), b,
-                               a->n_plan >= 0 ? (const int32_t *)d + 4 * (size_t)b : nullptr, n_plan, u_cap, d_workspace,
-                               workspace_bytes, d_prob, d_emb_out, d_status, stream));
-  ORCA_CUDA(cudaMemcpyAsync(h_status, d_status, 16, cudaMemcpyDeviceToHost, s));
-  ORCA_CUDA(cudaEventRecord(c->ev_call[slot], s));
+  auto enqueue = [&]() -> int {
+    ORCA_CUDA(cudaMemcpyAsync(d, h, (size_t)bytes, cudaMemcpyHostToDevice, c->copy));
+    orca_tgn_t mm = *m;
+    mm.input_stream = c->copy;
+    ORCA_TRY(orca_tgn_eval_batch(&mm, (const int32_t *)d, (const double *)(d + off_ts), b,
+                                 a->n_plan >= 0 ? (const int32_t *)d + 4 * (size_t)b : nullptr, n_plan, u_cap, d_workspace,
+                                 workspace_bytes, d_prob, d_emb_out, d_status, stream));
+    ORCA_CUDA(cudaMemcpyAsync(h_status, d_status, 16, cudaMemcpyDeviceToHost, s));
+    ORCA_CUDA(cudaEventRecord(c->ev_call[slot], s));
+    return ORCA_OK;
+  };
+  ORCA_TRY(settled(enqueue(), c, s));
   c->call_used[slot] = true;
   return ORCA_OK;
 }

@@ -713,3 +713,35 @@ def test_a_call_takes_the_forms_of_arrays_it_took_before():
               (src, dst, np.stack([neg, neg], 1), ts, eidx), (src, dst, neg, ts[:, None], eidx)):
         with pytest.raises(ValueError):
             run(*a)
+
+
+@pytest.mark.parametrize("name,reuse,budget,updates", [("c1", True, None, True), ("t_nb2", True, None, True),
+                                                       ("t_nb2", True, 0, False), ("t_nb2", False, None, False)])
+def test_a_call_that_fails_half_way_leaves_nothing_in_flight(name, reuse, budget, updates):
+    """A batch whose scorer is refused (no weights) has enqueued its layers and, in the first two recursions, on a stream of
+    the library's own, its memory update by then.  All of it has finished when the error is raised, although it stood behind
+    0.1 s of other work, and the model goes on."""
+    from orca_b200 import _lib
+    g = graph(name)
+    k = g.spec.n_degree
+    m = make_model(g, reuse=reuse, budget=budget)
+    run = lambda i: m.compute_edge_probabilities(*[a[200 * i:200 * (i + 1)] for a in (
+        g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)], k, reuse, False, None)
+    run(0)
+    m.check_status()
+    before = m.memory.memory.clone()
+    torch.cuda.synchronize()
+    weights, m._desc.score.W1t = m._desc.score.W1t, None
+    torch.cuda._sleep(200_000_000)
+    with pytest.raises(_lib.OrcaError):
+        run(1)
+    assert torch.cuda.current_stream().query()
+    beside = torch.cuda.Stream()
+    with torch.cuda.stream(beside):
+        now = m.memory.memory.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(now, m.memory.memory) and torch.equal(now, before) != updates
+    m._desc.score.W1t = weights
+    pos, neg = run(2)
+    m.check_status()
+    assert torch.isfinite(pos).all() and torch.isfinite(neg).all()
