@@ -115,15 +115,15 @@ def _ids_to_host(ids):
 
 def _queries_device(sources, destinations, timestamps, bs, device):
     """batch_query_order's list on the device.  The edges cross the bus as they are (16 bytes each) and are put in order
-    there; streams of more edges than the page-locked buffer takes are put in order on the host."""
+    there; streams of more edges than the page-locked buffer takes, and columns that are not one entry an edge (longer ones
+    count up to the number of sources), go through batch_query_order, which says what of them it takes."""
     E = len(sources)
-    if not 0 < 16 * E <= NeighborFinder.PINNED_TABLE:
+    edges = [np.asarray(a[:E]) for a in (sources, destinations, timestamps)]
+    if not 0 < 16 * E <= NeighborFinder.PINNED_TABLE or any(a.shape != (E,) for a in edges):
         nodes, ts = batch_query_order(sources, destinations, timestamps, bs)
         return torch.as_tensor(nodes).to(device), torch.as_tensor(ts).to(device)
-    src, dst = (np.ascontiguousarray(a, dtype=np.int64) for a in (sources, destinations))
-    t = np.ascontiguousarray(timestamps, dtype=np.float64)
-    if not (src.shape == dst.shape == t.shape == (E,)):
-        raise ValueError("sources, destinations and timestamps must have one length")
+    src, dst = (np.ascontiguousarray(a, dtype=np.int64) for a in edges[:2])
+    t = np.ascontiguousarray(edges[2], dtype=np.float64)
     pin = torch.empty(16 * E, dtype=torch.uint8, pin_memory=True)
     with torch.cuda.device(device):
         buffer = torch.empty(16 * E, dtype=torch.uint8, device=device)

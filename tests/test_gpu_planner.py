@@ -136,3 +136,29 @@ def test_queries_on_the_device_are_in_batch_order(E, bs):
     want = cache.batch_query_order(src, dst, ts, bs)
     got = cache._queries_device(src, dst, ts, bs, torch.device("cuda"))
     assert all(np.array_equal(g.cpu().numpy(), w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("on_host", [False, True])
+def test_columns_of_a_plan_may_be_longer_than_the_sources_but_not_shorter(on_host, monkeypatch):
+    """`sources` says how many edges there are, whichever way the queries take to the device."""
+    import argparse
+    import types
+    from orca_b200 import cache
+    from orca_b200.neighbor_finder import NeighborFinder, get_neighbor_finder
+    g = graph("t_nb2")
+    if on_host:
+        monkeypatch.setattr(NeighborFinder, "PINNED_TABLE", 16)
+    nf, args = get_neighbor_finder(g), argparse.Namespace(bs=100, n_degree=10, budget=50)
+    plan = lambda n, m, t: cache.get_cache_plan(args, types.SimpleNamespace(
+        sources=g.sources[:n], destinations=g.destinations[:m], timestamps=g.timestamps[:t]), nf, g.n_nodes, "LRU")
+    want = plan(950, 950, 950)
+    for more in ((950, 1000, 950), (950, 950, 951), (950, 1200, 1000)):
+        got = plan(*more)
+        assert len(got) == len(want) and all(np.array_equal(a, w) for a, w in zip(got, want)), more
+    for fewer in ((950, 940, 950), (950, 950, 300)):
+        with pytest.raises(ValueError):
+            plan(*fewer)
+    as_lists = cache._queries_device(list(g.sources[:950]), g.destinations[:950].astype(np.int32),
+                                     g.timestamps[:950].astype(np.float32), 100, torch.device("cuda"))
+    host = cache.batch_query_order(g.sources[:950], g.destinations[:950], g.timestamps[:950].astype(np.float32), 100)
+    assert all(np.array_equal(a.cpu().numpy(), w) for a, w in zip(as_lists, host))
