@@ -149,8 +149,10 @@ def _plan_local(args, train_data, neighbor_finder, num_embeddings, strategy, see
     torch.cuda.synchronize(neighbor_finder.device)
     t_prepare = time.time() - t0
     t0 = time.time()
+    # (the planners keep tables and bitmaps over the nodes, as many as there are: the ids come from the graph, which the
+    # sampling has held them against, so it says how many at least)
     plan, stats = plan_device(strategy, nodes_dev, nbr, len(train_data.sources), args.bs, args.n_degree,
-                              num_embeddings, budget, seed)
+                              max(num_embeddings, neighbor_finder.n_nodes), budget, seed)
     t_cache = time.time() - t0
     n_reuse, n_recompute = int(stats[0]), int(stats[1])
     avg = stats[2] / stats[0] if stats[0] else float("nan")

@@ -162,3 +162,26 @@ def test_columns_of_a_plan_may_be_longer_than_the_sources_but_not_shorter(on_hos
                                      g.timestamps[:950].astype(np.float32), 100, torch.device("cuda"))
     host = cache.batch_query_order(g.sources[:950], g.destinations[:950], g.timestamps[:950].astype(np.float32), 100)
     assert all(np.array_equal(a.cpu().numpy(), w) for a, w in zip(as_lists, host))
+
+
+@pytest.mark.parametrize("strategy", ["MRD", "LRU", "2Q"])
+def test_a_plan_covers_the_nodes_of_its_graph_whatever_number_is_given(strategy):
+    """A number of nodes below the graph's (one short, as without the padding node, or far off) must not make the planners
+    reach outside their tables."""
+    import argparse
+    from orca_b200 import cache
+    from orca_b200.neighbor_finder import get_neighbor_finder
+    g = graph("t_nb2")
+    nf, args = get_neighbor_finder(g), argparse.Namespace(bs=100, n_degree=10, budget=50)
+    seen = []
+    plan_device = cache.plan_device
+    cache_plan = lambda n: cache.get_cache_plan(args, g, nf, n, strategy)
+    try:
+        cache.plan_device = lambda *a: (seen.append(a[6]), plan_device(*a))[1]
+        want = cache_plan(g.n_nodes)
+        for n in (g.n_nodes - 1, 10, g.n_nodes + 70000):
+            got = cache_plan(n)
+            assert len(got) == len(want) and all(np.array_equal(a, w) for a, w in zip(got, want)), n
+    finally:
+        cache.plan_device = plan_device
+    assert seen == [g.n_nodes] * 3 + [g.n_nodes + 70000]
