@@ -386,7 +386,8 @@ int orca_plan_queries(const int64_t *h_src, const int64_t *h_dst, const double *
  * among equal keys, statistics), then that order for all batches.  Outputs, all on the device: d_plan_flat / d_plan_off as in orca_plan_host
  * (plan_cap >= n_batches * budget always suffices), d_stats = int64 {n_reuse, n_recompute, sum of
  * reuse distances}, d_status (int32[4], ORCA_E_CAPACITY when d_plan_flat is too small).
- * Enqueues on `stream`; the workspace (256-byte aligned) is sized by orca_plan_mrd_workspace_bytes. */
+ * Enqueues on `stream`; the workspace (256-byte aligned) is sized by orca_plan_mrd_workspace_bytes: some 8 (k + 1) bytes
+ * an edge (7.8 M edges with 10 neighbours: 0.77 GB), 200 MB or the worst case for streams shorter than that. */
 int64_t orca_plan_mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget);
 int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k, const int32_t *d_nbr,
                   int64_t n_nodes, int32_t budget, int32_t *d_plan_flat, int64_t plan_cap,
@@ -399,7 +400,8 @@ int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k
  * orca_plan_host) and walked by one thread; the statistics, the ascending member lists of the sets and the
  * least-recently-used evictions (first entries of numba's argsort of the last-use times) are data parallel
  * around it.  Arguments, outputs and plan order as in orca_plan_mrd / orca_plan_host
- * (plan_cap >= n_batches * budget always suffices). */
+ * (plan_cap >= n_batches * budget always suffices).  LRU and 2Q walk a stream in parts, so that their workspace does not
+ * grow with it (150 MB at most for a million nodes and batches of 2000 edges). */
 int64_t orca_plan_device_workspace_bytes(int32_t strategy, int64_t n_edges, int32_t bs, int32_t k,
                                          int64_t n_nodes, int32_t budget);
 int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k,

@@ -38,11 +38,12 @@ __global__ void __launch_bounds__(256) queries_kernel(const double *ts, const in
 // One block a batch, blocks walk the batches.  Two bitmaps over the nodes (the batch's nodes, its endpoints) and the
 // prefix counts of the first, in global memory, left empty.  Bound by the latency of the table entries' lookups.
 __global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, const int32_t *nbr, int64_t n_edges, int32_t bs,
-                                                        int32_t k, int64_t n_nodes, Lists l, uint32_t *bitmaps, int32_t *code,
-                                                        int32_t code_init) {
+                                                        int32_t k, int64_t n_nodes, int64_t b0, int64_t b1, Lists l,
+                                                        uint32_t *bitmaps, int32_t *code, int32_t code_init) {
   __shared__ int s_cnt[NW];
+  __shared__ int64_t s_at;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t words = (n_nodes + 31) / 32, nb = (n_edges + bs - 1) / bs;
+  const int64_t words = (n_nodes + 31) / 32;
   uint32_t *all = bitmaps + blockIdx.x * 3 * words, *target = all + words;
   int32_t *before = (int32_t *)(target + words);
   for (int64_t i = tid; i < 2 * words; i += T) all[i] = 0;
@@ -51,11 +52,10 @@ __global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, co
   __syncthreads();
   const int64_t chunk = ((words + NW - 1) / NW + 31) & ~31ll;     // words of a warp
   constexpr int STEP = 8;
-  for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+  for (int64_t b = b0 + blockIdx.x; b < b1; b += gridDim.x) {
     const int64_t s = b * bs;
     const int m2 = 2 * (int)(min(n_edges, s + bs) - s);
     const int32_t *q = nodes + 2 * s, *tab = nbr + 2 * s * k;
-    int32_t *id = l.id + b * l.stride, *mult = l.mult + b * l.stride;
     for (int i = tid; i < m2; i += T) {
       const int32_t v = q[i];
       const uint32_t bit = 1u << (v & 31);
@@ -95,6 +95,25 @@ __global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, co
     const int c_lane = s_cnt[lane];
     int base = __reduce_add_sync(0xffffffffu, lane < warp ? c_lane : 0);
     const int n = __reduce_add_sync(0xffffffffu, c_lane);
+    if (tid == 0) {
+      int64_t at = (b - b0) * l.stride;
+      if (l.stride == 0) {
+        at = n <= CAP ? (int64_t)atomicAdd(l.used, (unsigned long long)n) : l.room;
+        if (at + n > l.room) {
+          at = -1;
+          *l.failed = 1;
+        }
+      }
+      s_at = at;
+      l.span[b - b0] = Span{max(at, (int64_t)0), at < 0 ? 0 : n};
+    }
+    __syncthreads();
+    if (s_at < 0) {      // (nobody looks at these lists)
+      for (int64_t i = tid; i < 2 * words; i += T) all[i] = 0;
+      __syncthreads();
+      continue;
+    }
+    int32_t *id = l.id + s_at, *mult = l.mult + s_at;
     for (int64_t j = 0; j < chunk; j += 32) {
       const int64_t wi = warp * chunk + j + lane;
       uint32_t bits = wi < words ? __ldcg(&all[wi]) : 0;
@@ -118,7 +137,6 @@ __global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, co
         }
       }
     }
-    if (tid == 0) l.count[b] = n;
     __syncthreads();
     neighbors([&](int32_t v) {
       atomicAdd(&mult[__ldcg(&before[v >> 5]) + __popc(__ldcg(&all[v >> 5]) & ((1u << (v & 31)) - 1u))], 1);
@@ -134,11 +152,13 @@ __global__ void __launch_bounds__(T) batch_lists_kernel(const int32_t *nodes, co
 }
 
 int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
-                       const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init, cudaStream_t s) {
+                       int64_t b0, int64_t b1, const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init,
+                       cudaStream_t s) {
   const Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "launch_batch_lists: no context for the current device");
-  const int grid = blocks_for((n_edges + bs - 1) / bs, n_nodes, std::min(c->sm_count, MOST_BLOCKS));
-  batch_lists_kernel<<<grid, T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, l, (uint32_t *)d_scratch, d_code, code_init);
+  const int grid = blocks_for(b1 - b0, n_nodes, std::min(c->sm_count, MOST_BLOCKS));
+  batch_lists_kernel<<<grid, T, 0, s>>>(d_nodes, d_nbr, n_edges, bs, k, n_nodes, b0, b1, l, (uint32_t *)d_scratch, d_code,
+                                        code_init);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;
@@ -153,27 +173,28 @@ int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_e
 __global__ void __launch_bounds__(T) next_use_lists_kernel(Lists l, int64_t nb, int32_t *next, int32_t *key) {
   const int tid = threadIdx.x;
   constexpr int AHEAD = 2;
-  const auto load = [&](int64_t b, int n, int i) { return i < n ? l.id[b * l.stride + i] : 0; };
-  int n = l.count[nb - 1], n_next = nb > 1 ? l.count[nb - 2] : 0;
+  if (*l.failed) return;
+  const auto load = [&](Span a, int i) { return i < a.n ? l.id[a.at + i] : 0; };
+  Span a = l.span[nb - 1], a_next = nb > 1 ? l.span[nb - 2] : Span{0, 0};
   int32_t x[AHEAD], y[AHEAD];
 #pragma unroll
-  for (int u = 0; u < AHEAD; ++u) x[u] = load(nb - 1, n, tid + u * T);
+  for (int u = 0; u < AHEAD; ++u) x[u] = load(a, tid + u * T);
   for (int64_t b = nb - 1; b >= 0; --b) {
     const auto node = [&](int i, int32_t e) {
       const int32_t v = e & ~TARGET;
-      key[b * l.stride + i] = __ldcg(&next[v]);
+      key[a.at + i] = __ldcg(&next[v]);
       next[v] = e < 0 ? (int32_t)FAR : (int32_t)b;     // (distinct nodes: nobody else reads or writes it in this batch)
     };
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u)
-      if (tid + u * T < n) node(tid + u * T, x[u]);
-    for (int i = tid + AHEAD * T; i < n; i += T) node(i, l.id[b * l.stride + i]);
-    const int n_after = b > 1 ? l.count[b - 2] : 0;
+      if (tid + u * T < a.n) node(tid + u * T, x[u]);
+    for (int i = tid + AHEAD * T; i < a.n; i += T) node(i, l.id[a.at + i]);
+    const Span a_after = b > 1 ? l.span[b - 2] : Span{0, 0};
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) y[u] = b > 0 ? load(b - 1, n_next, tid + u * T) : 0;
+    for (int u = 0; u < AHEAD; ++u) y[u] = load(a_next, tid + u * T);
     __syncthreads();
-    n = n_next;
-    n_next = n_after;
+    a = a_next;
+    a_next = a_after;
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) x[u] = y[u];
   }
@@ -189,7 +210,7 @@ __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.
 struct State {           // of a plan, between the launches for its chunks of batches
   int32_t n_cached, failed;
   int64_t used;
-  unsigned long long reuse, recompute, dist;
+  unsigned long long reuse, recompute, dist, listed;
 };
 struct MrdArgs {
   Lists l;
@@ -234,24 +255,20 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
   // the first nodes of the next batch's list, loaded ahead
   constexpr int AHEAD = 2;
   int32_t x_next[AHEAD], mult_next[AHEAD];
-  int n_next = g.l.count[g.b0];
-  const auto load_ahead = [&](int64_t b) {
+  Span next = g.l.span[g.b0];
+  const auto load_ahead = [&]() {
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
       const int64_t i = tid + u * T;
-      x_next[u] = i < n_next ? g.l.id[b * g.l.stride + i] : 0;
-      mult_next[u] = i < n_next ? g.l.mult[b * g.l.stride + i] : 0;
+      x_next[u] = i < next.n ? g.l.id[next.at + i] : 0;
+      mult_next[u] = i < next.n ? g.l.mult[next.at + i] : 0;
     }
   };
-  load_ahead(g.b0);
+  load_ahead();
   for (int64_t b = g.b0; b < g.b1; ++b) {
-    const int64_t at = b * g.l.stride;
-    const int n_list = n_next;
+    const int64_t at = next.at;
+    const int n_list = next.n;      // (no more than cap)
     int32_t *cand = g.cand + (b - g.b0) * 2 * cap;
-    if (n_list > cap) {      // (uniform over the block)
-      failed = true;
-      break;
-    }
     for (int i = tid; i < n_words; i += T) s_new[i].bits = s_known[i] = s_list[i].bits = 0;
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // (the candidates of the batch before)
     __syncthreads();         // (and the cached ids are there)
@@ -308,8 +325,8 @@ __global__ void __launch_bounds__(T, 1) mrd_lists_kernel(const __grid_constant__
     for (int u = 0; u < AHEAD; ++u) place(tid + u * T, x_next[u]);
     for (int i = tid + AHEAD * T; i < n_list; i += T) place(i, g.l.id[at + i]);
     if (b + 1 < g.b1) {
-      n_next = g.l.count[b + 1];
-      load_ahead(b + 1);
+      next = g.l.span[b + 1];
+      load_ahead();
     }
     __syncthreads();
     count_words(s_new, n_words, (int32_t *)s_tot);
@@ -405,13 +422,24 @@ __global__ void __launch_bounds__(T, 1) sort_plan_kernel(const __grid_constant__
 
 constexpr int64_t CHUNK = 512;      // batches of a launch: bounds the candidates that wait for their order (2 x 4 * CAP bytes each)
 
+// Entries that the lists of a plan have room for: all that there can be, up to 16 M (12 bytes each; 400,000 edges with 20
+// neighbours), and beyond that a third, which is what the tables of the kernels of planner_mrd.cu take, in whose workspace
+// these lists lie.  (Lists of the largest graph's stream fill a thirtieth, those of streams with few repetitions a third.)
+constexpr int64_t ROOM = 16 << 20;
+static int64_t room_for(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes) {
+  const int64_t most = (n_edges + bs - 1) / bs * std::min<int64_t>(stride_of(bs, k, n_nodes), CAP);
+  return std::min(most, std::max(ROOM, 2 * n_edges * (k + 1) / 3));
+}
+
 struct MrdLayout {
-  int64_t state, id, mult, count, key, next, scratch, cached, cached_state, place, cand, cand_n, total;
+  int64_t state, id, mult, span, key, next, scratch, cached, cached_state, place, cand, cand_n, total;
+  int64_t room;
   int32_t cap;
 };
 static MrdLayout mrd_layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
   MrdLayout L;
-  const int64_t nb = (n_edges + bs - 1) / bs, stride = stride_of(bs, k, n_nodes), chunk = std::min(nb, CHUNK);
+  const int64_t nb = (n_edges + bs - 1) / bs, chunk = std::min(nb, CHUNK);
+  L.room = room_for(n_edges, bs, k, n_nodes);
   L.cap = (int32_t)((std::min<int64_t>({(int64_t)budget + 2ll * bs * (k + 1), n_nodes, (int64_t)CAP}) + 31) & ~31ll);
   int64_t at = 0;
   auto take = [&](int64_t bytes) {
@@ -420,10 +448,10 @@ static MrdLayout mrd_layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_no
     return o;
   };
   L.state = take(sizeof(State));
-  L.id = take(nb * stride * 4);
-  L.mult = take(nb * stride * 4);
-  L.count = take(nb * 4);
-  L.key = take(nb * stride * 4);
+  L.id = take(L.room * 4);
+  L.mult = take(L.room * 4);
+  L.span = take(nb * sizeof(Span));
+  L.key = take(L.room * 4);
   L.next = take(n_nodes * 4);
   L.scratch = take(scratch_bytes(nb, n_nodes));
   L.cached = take(L.cap * 4);
@@ -437,6 +465,10 @@ static MrdLayout mrd_layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_no
 
 // (a key has to name every batch)
 bool mrd_takes(int64_t n_edges, int32_t bs) { return (n_edges + bs - 1) / bs < (int64_t)FAR; }
+bool mrd_always(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
+  const int64_t list = stride_of(bs, k, n_nodes);
+  return std::min(budget + list, n_nodes) <= CAP && room_for(n_edges, bs, k, n_nodes) == (n_edges + bs - 1) / bs * list;
+}
 int64_t mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
   return mrd_layout(n_edges, bs, k, n_nodes, budget).total;
 }
@@ -449,20 +481,20 @@ int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, in
   const MrdLayout L = mrd_layout(n_edges, bs, k, n_nodes, budget);
   char *base = (char *)d_workspace;
   MrdArgs g{};
-  g.l.id = (int32_t *)(base + L.id), g.l.mult = (int32_t *)(base + L.mult), g.l.count = (int32_t *)(base + L.count);
-  g.l.stride = stride_of(bs, k, n_nodes);
+  g.l.id = (int32_t *)(base + L.id), g.l.mult = (int32_t *)(base + L.mult), g.l.span = (Span *)(base + L.span);
   g.key = (int32_t *)(base + L.key);
   g.nb = (n_edges + bs - 1) / bs;
   g.budget = budget, g.cap = L.cap;
   g.st = (State *)(base + L.state);
+  g.l.stride = 0, g.l.used = &g.st->listed, g.l.room = L.room, g.l.failed = &g.st->failed;
   g.cached = (int32_t *)(base + L.cached), g.cached_state = (uint32_t *)(base + L.cached_state);
   g.place = (int32_t *)(base + L.place);
   g.cand = (int32_t *)(base + L.cand);
   g.cand_n = (int32_t *)(base + L.cand_n);
   g.plan_cap = plan_cap, g.plan_off = d_plan_off, g.status = d_status;
   ORCA_CUDA(cudaMemsetAsync(g.st, 0, sizeof(State), s));
-  int rc = launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, g.l, base + L.scratch, (int32_t *)(base + L.next),
-                              (int32_t)FAR, s);
+  int rc = launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, 0, g.nb, g.l, base + L.scratch,
+                              (int32_t *)(base + L.next), (int32_t)FAR, s);
   if (rc != ORCA_OK) return rc;
   next_use_lists_kernel<<<1, T, 0, s>>>(g.l, g.nb, (int32_t *)(base + L.next), (int32_t *)(base + L.key));
   ORCA_COUNT_LAUNCH();

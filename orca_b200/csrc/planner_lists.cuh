@@ -9,14 +9,24 @@ namespace lists {
 constexpr int T = tie::T, NW = tie::NW;
 constexpr int CAP = 13696;      // entries of a list that is selected from: 17 bytes of shared memory each, whole words of bits
 
-// The distinct nodes of every batch in ascending order, batch b's from b * stride: its endpoints (TARGET set) and the
-// out-of-batch neighbours of its table.
+// The distinct nodes of a batch in ascending order: its endpoints (TARGET set) and the out-of-batch neighbours of its table.
+// A batch can have as many as its table has entries and has a tenth of them or less as a rule (1,450 of 44,000 on the largest
+// graph), so the lists of a whole plan lie one behind the other as they get ready, in as much memory as the caller gives
+// (with a stride of the most there can be, the lists of 7.8 M edges took 2.1 GB, 0.07 of it in use); those of a part of a
+// plan have a stride.
 constexpr int32_t TARGET = (int32_t)0x80000000u;
+struct __align__(16) Span {
+  int64_t at;        // of the batch's first entry
+  int32_t n;
+};
 struct Lists {
   int32_t *id;       // node | TARGET
   int32_t *mult;     // out-of-batch neighbours: entries of the table that hold the node
-  int32_t *count;    // [batches]
-  int64_t stride;
+  Span *span;        // [batches]
+  int64_t stride;    // 0: one behind the other, and
+  unsigned long long *used;     // entries taken,
+  int64_t room;      // entries there are,
+  int32_t *failed;   // set when a list has more than CAP of them, or there is no room
 };
 inline int64_t stride_of(int32_t bs, int32_t k, int64_t n_nodes) {
   const int64_t most = 2ll * bs * (k + 1);
@@ -34,9 +44,10 @@ constexpr int MOST_BLOCKS = 256;     // what a workspace has room for (devices h
 inline int64_t scratch_bytes(int64_t n_batches, int64_t n_nodes) {
   return blocks_for(n_batches, n_nodes, MOST_BLOCKS) * block_bytes(n_nodes);
 }
-// code (optional): set to `code_init` for every node on the way
+// The lists of batches [b0, b1) (l.span[0] is b0's).  code (optional): set to `code_init` for every node on the way
 int launch_batch_lists(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
-                       const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init, cudaStream_t s);
+                       int64_t b0, int64_t b1, const Lists &l, void *d_scratch, int32_t *d_code, int32_t code_init,
+                       cudaStream_t s);
 
 // An entry of a selection: key and place in its list.
 constexpr int KEY_BITS = 16, IDX_BITS = 14;
@@ -354,8 +365,10 @@ __device__ __forceinline__ bool select_by_far_step(Key key, int n, int keep, Wor
   return true;
 }
 
-// MRD over lists.  Candidate lists longer than CAP set *State::failed: the kernels of planner_mrd.cu do the plan then.
+// MRD over lists.  Lists or candidates of more than CAP entries, or more lists than there is room for, set
+// *State::failed: the kernels of planner_mrd.cu do the plan then.
 bool mrd_takes(int64_t n_edges, int32_t bs);
+bool mrd_always(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget);      // (it cannot fail)
 int64_t mrd_workspace_bytes(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget);
 int launch_mrd(const int32_t *d_nodes, const int32_t *d_nbr, int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes,
                int32_t budget, int32_t *d_plan, int64_t plan_cap, int64_t *d_plan_off, int64_t *d_stats, int32_t *d_status,

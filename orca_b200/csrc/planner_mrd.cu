@@ -773,13 +773,13 @@ extern "C" int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs
     ORCA_CUDA(cudaMemsetAsync(d_plan_off, 0, sizeof(int64_t), s));
     return ORCA_OK;
   }
-  // From lists of distinct nodes (planner_lists.cu), unless a candidate list is too long for them, which shows on the way:
+  // From lists of distinct nodes (planner_lists.cu), unless these or a candidate list are too long, which shows on the way:
   // the kernels below look at the word that says so.
   const int32_t *only_if = nullptr;
   if (lists::mrd_takes(n_edges, bs)) {
     const int rc = lists::launch_mrd(d_nodes, d_nbr, n_edges, bs, k, n_nodes, budget, d_plan_flat, plan_cap, d_plan_off,
                                      d_stats, d_status, d_workspace, &only_if, s);
-    if (rc != ORCA_OK || std::min(mrd::cand_cap(bs, k, budget), n_nodes) <= lists::CAP) return rc;
+    if (rc != ORCA_OK || lists::mrd_always(n_edges, bs, k, n_nodes, budget)) return rc;
   }
   // A cluster of 16 (else 8) CTAs shares every phase when the device can place such a cluster and the
   // candidate list fits its threads' registers (a phase costs a cluster barrier of ~600 cycles, an L2 round

@@ -87,8 +87,16 @@ struct Twister {
   }
 };
 
+// Of a plan, between the launches for its chunks of batches.
+struct State {
+  uint32_t rng[Twister::N];
+  int32_t rng_pos, failed, n[2];      // n: LRU: cached; 2Q: fifo, lru
+  int64_t used;
+};
+
 struct Work {
-  lists::Lists lists;
+  State *st;
+  lists::Lists lists;             // of the launch's batches
   int32_t *t0, *t1, *t2;          // [n_nodes] LRU: last use, arrival; 2Q: LRU last use, LRU arrival, FIFO arrival
   uint32_t *bm[2];                // [words] LRU: cached; 2Q: fifo, lru
   int32_t *list[4];               // [cap] member lists
@@ -212,21 +220,28 @@ template <bool SH>
 __device__ __forceinline__ uint32_t *bitmap(const Work &w, int i, int64_t words) {
   return SH ? (uint32_t *)(tie::smem + tie::Shared::BYTES * w.cap_shared) + i * words : w.bm[i];
 }
-template <bool SH>
-__device__ void clear_bitmaps(const Work &w, int64_t words) {
-  for (int64_t i = threadIdx.x; i < N_BM * words; i += T) bitmap<SH>(w, (int)(i / words), words)[i % words] = 0;
+// at the start of a launch: the first one's are empty, the others' as the one before left them (LOAD: false: that)
+template <bool SH, bool LOAD>
+__device__ void move_bitmaps(const Work &w, int64_t words, bool first) {
+  for (int64_t i = threadIdx.x; i < N_BM * words; i += T) {
+    const int m = (int)(i / words);
+    const int64_t j = i % words;
+    if (LOAD && first) bitmap<SH>(w, m, words)[j] = 0;
+    else if (SH && LOAD) bitmap<SH>(w, m, words)[j] = w.bm[m][j];
+    else if (SH) w.bm[m][j] = bitmap<SH>(w, m, words)[j];
+  }
 }
 
-// Deals the out-of-batch neighbours of a batch out to three lists: kind(v, entries of the table) says which (0 .. 2, else
+// Deals the out-of-batch neighbours of list a out to three lists: kind(v, entries of the table) says which (0 .. 2, else
 // none).  The lists stay in ascending order; n: their lengths, the same in every thread.  s_cnt: NW words.  All T threads;
 // ends behind a barrier.
 template <class Kind>
-__device__ __forceinline__ void deal_neighbors(const lists::Lists &l, int64_t b, int32_t *const (&out)[3], int (&n)[3],
+__device__ __forceinline__ void deal_neighbors(const lists::Lists &l, lists::Span a, int32_t *const (&out)[3], int (&n)[3],
                                                uint32_t *s_cnt, Kind kind) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
-  const int n_list = l.count[b];
-  const int32_t *id = l.id + b * l.stride, *mult = l.mult + b * l.stride;
+  const int n_list = a.n;
+  const int32_t *id = l.id + a.at, *mult = l.mult + a.at;
   n[0] = n[1] = n[2] = 0;
   for (int i0 = 0; i0 < n_list; i0 += T) {
     const int i = i0 + tid;
@@ -270,32 +285,58 @@ __device__ void write_totals(const Totals &t, int64_t *stats) {
   }
 }
 
+// The state of a plan at the start and at the end of a launch; false: an earlier launch has failed.
+__device__ __forceinline__ bool resume(const Work &w, Twister &rng, uint32_t seed, bool first) {
+  if (first) {
+    if (threadIdx.x == 0) rng.seed(seed);
+    return true;
+  }
+  if (w.st->failed) return false;
+  for (int i = threadIdx.x; i < Twister::N; i += T) rng.s[i] = w.st->rng[i];
+  if (threadIdx.x == 0) rng.pos = w.st->rng_pos;
+  return true;
+}
+__device__ __forceinline__ void suspend(const Work &w, const Twister &rng, bool failed, int n0, int n1, int64_t used) {
+  for (int i = threadIdx.x; i < Twister::N; i += T) w.st->rng[i] = rng.s[i];
+  if (threadIdx.x == 0) {
+    w.st->rng_pos = rng.pos, w.st->failed = failed;
+    w.st->n[0] = n0, w.st->n[1] = n1, w.st->used = used;
+  }
+}
+
 // ------------------------------------------------------------------------------ LRU (utils/cache.py:338-403)
 template <bool SH>
-__global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
-                                                int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
-                                                int32_t *status) {
+__global__ void __launch_bounds__(T, 1) lru_kernel(int64_t b0, int64_t b1, int64_t nb, int64_t n_nodes, int32_t budget,
+                                                uint32_t seed, Work w, int32_t *plan, int64_t plan_cap, int64_t *plan_off,
+                                                int64_t *stats, int32_t *status) {
   __shared__ Twister rng;
   __shared__ int s_a[NW], s_b[NW];
   const int tid = threadIdx.x;
   const int64_t words = (n_nodes + 31) / 32;
-  clear_bitmaps<SH>(w, words);
+  if (!resume(w, rng, seed, b0 == 0)) return;
+  move_bitmaps<SH, true>(w, words, b0 == 0);
   uint32_t *cached = bitmap<SH>(w, 0, words);
   int32_t *used_at = w.t0, *arrived = w.t1;
-  int32_t *cand = w.list[0], *held = w.list[1];
-  for (int64_t v = tid; v < n_nodes; v += T) {
+  int32_t *cand = w.list[0];
+  for (int64_t v = tid; b0 == 0 && v < n_nodes; v += T) {
     used_at[v] = 0;
     arrived[v] = 0;
   }
-  if (tid == 0) rng.seed(seed);
   __syncthreads();
   Totals tot;
-  int64_t used = 0;
-  int n_held = 0;      // members of `cached`, listed in `held`
-  for (int64_t b = 0; b < nb; ++b) {
+  int64_t used = b0 == 0 ? 0 : w.st->used;
+  int n_held = b0 == 0 ? 0 : w.st->n[0];      // members of `cached`, listed in `held`
+  // (no more than the budget; a plan that would not fit is listed elsewhere)
+  const auto listed_at = [&](int64_t at) { return at + min((int64_t)budget, n_nodes) <= plan_cap ? plan + at : w.list[1]; };
+  int32_t *held = listed_at(used - n_held);
+  bool failed = false;
+  lists::Span span_next = w.lists.span[0];
+  for (int64_t b = b0; b < b1; ++b) {
+    const lists::Span span = span_next;
+    if (b + 1 < b1) span_next = w.lists.span[b + 1 - b0];
     int32_t *const out[3] = {cand, nullptr, nullptr};
     int n[3];
-    deal_neighbors(w.lists, b, out, n, (uint32_t *)s_a, [&](int32_t v, int m) {
+    deal_neighbors(w.lists, span, out, n, (uint32_t *)s_a, [&](int32_t v, int m) {
       if (!bit(cached, v)) {
         tot.recompute += m;
         return 0;
@@ -313,6 +354,7 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, 
       if (!for_first_by_key(w, held, n_held, evict, used_at, s_a, s_b,
                             [&](int32_t v) { clear_bit(cached, v); })) {
         if (tid == 0) report(status, ORCA_E_TIMEOUT, (int)b);
+        failed = true;
         break;
       }
     }
@@ -322,11 +364,11 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, 
       set_bit(cached, v);
       used_at[v] = arrived[v] = (int32_t)b;
     }
-    // (no more than the budget; a plan that would not fit is listed elsewhere)
-    held = used + min((int64_t)budget, n_nodes) <= plan_cap ? plan + used : w.list[1];
+    held = listed_at(used);
     n_held = list_members(cached, words, held, false, s_a);
     if (used + n_held > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
+      failed = true;
       break;
     }
     if (held != plan + used)
@@ -336,38 +378,45 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t nb, int64_t n_nodes, 
     __syncthreads();
   }
   write_totals(tot, stats);
-  if (tid == 0) plan_off[nb] = used;
+  if (b1 < nb) {
+    suspend(w, rng, failed, n_held, 0, used);
+    move_bitmaps<SH, false>(w, words, false);
+  }
+  if (tid == 0 && (failed || b1 == nb)) plan_off[nb] = used;
 }
 
 // ------------------------------------------------------------------------------ 2Q (utils/cache.py:175-333)
 // a FIFO half and an LRU half of budget / 2 entries each
 template <bool SH>
-__global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t nb, int64_t n_nodes, int32_t budget, uint32_t seed, Work w,
-                                                 int32_t *plan, int64_t plan_cap, int64_t *plan_off, int64_t *stats,
-                                                 int32_t *status) {
+__global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int64_t nb, int64_t n_nodes, int32_t budget,
+                                                 uint32_t seed, Work w, int32_t *plan, int64_t plan_cap, int64_t *plan_off,
+                                                 int64_t *stats, int32_t *status) {
   __shared__ Twister rng;
   __shared__ int s_a[NW], s_b[NW];
   const int tid = threadIdx.x;
   const int64_t words = (n_nodes + 31) / 32;
   const int half = budget / 2;
-  clear_bitmaps<SH>(w, words);
+  if (!resume(w, rng, seed, b0 == 0)) return;
+  move_bitmaps<SH, true>(w, words, b0 == 0);
   uint32_t *fifo = bitmap<SH>(w, 0, words), *lru = bitmap<SH>(w, 1, words);
   int32_t *lru_used = w.t0, *lru_arr = w.t1, *fifo_arr = w.t2;
   int32_t *promote = w.list[0], *fresh = w.list[1], *touched = w.list[2], *ids = w.list[3];
-  for (int64_t v = tid; v < n_nodes; v += T) {
+  for (int64_t v = tid; b0 == 0 && v < n_nodes; v += T) {
     lru_used[v] = lru_arr[v] = fifo_arr[v] = 0;
   }
-  if (tid == 0) rng.seed(seed);
   __syncthreads();
   Totals tot;
-  int64_t used = 0;
-  int n_fifo = 0, n_lru = 0;
+  int64_t used = b0 == 0 ? 0 : w.st->used;
+  int n_fifo = b0 == 0 ? 0 : w.st->n[0], n_lru = b0 == 0 ? 0 : w.st->n[1];
   bool failed = false;
-  for (int64_t b = 0; b < nb && !failed; ++b) {
+  lists::Span span_next = w.lists.span[0];
+  for (int64_t b = b0; b < b1 && !failed; ++b) {
+    const lists::Span span = span_next;
+    if (b + 1 < b1) span_next = w.lists.span[b + 1 - b0];
     const int32_t now = (int32_t)b;
     int32_t *const out[3] = {promote, fresh, touched};
     int n_out[3];
-    deal_neighbors(w.lists, b, out, n_out, (uint32_t *)s_a, [&](int32_t v, int m) {
+    deal_neighbors(w.lists, span, out, n_out, (uint32_t *)s_a, [&](int32_t v, int m) {
       if (bit(fifo, v)) {
         tot.reuse += m;
         tot.dist += (long long)(now - fifo_arr[v]) * m;
@@ -452,13 +501,15 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t nb, int64_t n_nodes,
     n_fifo = list_members(fifo, words, ids, false, s_a);
     if (used + n_fifo > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
-      break;
+      failed = true;
+      continue;
     }
     for (int i = tid; i < n_fifo; i += T) plan[used + i] = ids[i];
     n_lru = list_members(lru, words, ids, false, s_a);
     if (used + n_fifo + n_lru > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
-      break;
+      failed = true;
+      continue;
     }
     for (int i = tid; i < n_lru; i += T) plan[used + n_fifo + i] = ids[i];
     if (tid == 0) plan_off[b] = used;
@@ -466,11 +517,22 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t nb, int64_t n_nodes,
     __syncthreads();
   }
   write_totals(tot, stats);
-  if (tid == 0) plan_off[nb] = used;
+  if (b1 < nb) {
+    suspend(w, rng, failed, n_fifo, n_lru, used);
+    move_bitmaps<SH, false>(w, words, false);
+  }
+  if (tid == 0 && (failed || b1 == nb)) plan_off[nb] = used;
+}
+
+// Batches whose lists lie in memory at a time: as many as fit 64 MB (250 of 600 edges with 20 neighbours are one launch).
+// A launch more costs some 10 us of state and bitmaps, the 330 batches of it 4.6 ms.
+constexpr int64_t LISTS = 64 << 20;
+static int64_t chunk_of(int64_t nb, int32_t bs, int32_t k, int64_t n_nodes) {
+  return std::min(nb, std::max<int64_t>(1, LISTS / (8 * lists::stride_of(bs, k, n_nodes))));
 }
 
 struct Layout {
-  int64_t id, mult, count, scratch, t[3], bm[N_BM], list[4], sort, total, cap;
+  int64_t st, id, mult, span, scratch, t[3], bm[N_BM], list[4], sort, total, cap;
 };
 static Layout layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, int32_t budget) {
   Layout L;
@@ -482,11 +544,12 @@ static Layout layout(int64_t n_edges, int32_t bs, int32_t k, int64_t n_nodes, in
     at += (bytes + 255) & ~255ll;
     return o;
   };
-  const int64_t nb = (n_edges + bs - 1) / bs, stride = lists::stride_of(bs, k, n_nodes);
-  L.id = take(nb * stride * 4);
-  L.mult = take(nb * stride * 4);
-  L.count = take(nb * 4);
-  L.scratch = take(lists::scratch_bytes(nb, n_nodes));
+  const int64_t stride = lists::stride_of(bs, k, n_nodes), chunk = chunk_of((n_edges + bs - 1) / bs, bs, k, n_nodes);
+  L.st = take(sizeof(State));
+  L.id = take(chunk * stride * 4);
+  L.mult = take(chunk * stride * 4);
+  L.span = take(chunk * sizeof(lists::Span));
+  L.scratch = take(lists::scratch_bytes(chunk, n_nodes));
   for (int i = 0; i < 3; ++i) L.t[i] = take(n_nodes * 4);
   for (int i = 0; i < N_BM; ++i) L.bm[i] = take(words * 4);
   for (int i = 0; i < 4; ++i) L.list[i] = take(L.cap * 4);
@@ -532,8 +595,9 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
   char *base = (char *)d_workspace;
   rnd::Work w;
   const int64_t nb = (n_edges + bs - 1) / bs;
-  w.lists.id = (int32_t *)(base + L.id), w.lists.mult = (int32_t *)(base + L.mult);
-  w.lists.count = (int32_t *)(base + L.count), w.lists.stride = lists::stride_of(bs, k, n_nodes);
+  w.st = (rnd::State *)(base + L.st);
+  w.lists = lists::Lists{(int32_t *)(base + L.id), (int32_t *)(base + L.mult), (lists::Span *)(base + L.span),
+                         lists::stride_of(bs, k, n_nodes), nullptr, 0, nullptr};
   w.keys_fit = nb < (int64_t)lists::FAR;
   w.t0 = (int32_t *)(base + L.t[0]);
   w.t1 = (int32_t *)(base + L.t[1]);
@@ -576,11 +640,15 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
   auto kernel = strategy == 1 ? (w.bm_shared ? rnd::lru_kernel<true> : rnd::lru_kernel<false>)
                               : (w.bm_shared ? rnd::twoq_kernel<true> : rnd::twoq_kernel<false>);
   ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const int rc = lists::launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, w.lists, base + L.scratch, nullptr, 0, s);
-  if (rc != ORCA_OK) return rc;
-  kernel<<<1, rnd::T, smem, s>>>(nb, n_nodes, budget, seed, w, d_plan_flat, plan_cap,
-                                 d_plan_off, d_stats, d_status);
-  ORCA_COUNT_LAUNCH();
-  ORCA_LAUNCH_CHECK();
+  const int64_t chunk = rnd::chunk_of(nb, bs, k, n_nodes);
+  for (int64_t b0 = 0; b0 < nb; b0 += chunk) {
+    const int64_t b1 = std::min(nb, b0 + chunk);
+    const int rc = lists::launch_batch_lists(d_nodes, d_nbr, n_edges, bs, k, n_nodes, b0, b1, w.lists, base + L.scratch,
+                                             nullptr, 0, s);
+    if (rc != ORCA_OK) return rc;
+    kernel<<<1, rnd::T, smem, s>>>(b0, b1, nb, n_nodes, budget, seed, w, d_plan_flat, plan_cap, d_plan_off, d_stats, d_status);
+    ORCA_COUNT_LAUNCH();
+    ORCA_LAUNCH_CHECK();
+  }
   return ORCA_OK;
 }

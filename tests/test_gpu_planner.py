@@ -185,3 +185,44 @@ def test_a_plan_covers_the_nodes_of_its_graph_whatever_number_is_given(strategy)
     finally:
         cache.plan_device = plan_device
     assert seen == [g.n_nodes] * 3 + [g.n_nodes + 70000]
+
+
+@pytest.mark.parametrize("strategy", ["MRD", "LRU", "2Q"])
+@pytest.mark.parametrize("n_src", [130000, 700000])      # sets in shared memory and in global memory
+def test_plans_of_several_launches(n_src, strategy):
+    """The lists of 67 batches of 2000 edges with 30 neighbours lie in memory at a time (LRU, 2Q): two full launches and one
+    of two batches, the last of them short.  Against the host's policies over the same tables."""
+    from orca_b200 import cache, synthetic
+    spec = dataclasses.replace(synthetic.SPECS["t_nb2"], n_src=n_src, n_edges=271001, bs=2000, budget=3000)
+    g = synthetic.make_graph(spec, seed=13)
+    nodes, ts = cache.batch_query_order(g.sources, g.destinations, g.timestamps, 2000)
+    from orca_b200.neighbor_finder import get_neighbor_finder
+    nbr = get_neighbor_finder(g, g.n_nodes - 1).sample_device(nodes, ts, 30)[0]
+    got, stats = cache.plan_device(strategy, torch.as_tensor(nodes).cuda(), nbr, g.n_edges, 2000, 30, g.n_nodes, 3000, seed=4)
+    want, wstats = cache.plan_from_tables(strategy, g.sources, g.destinations, 2000, 30, nbr.cpu().numpy(), g.n_nodes, 3000,
+                                          seed=4)
+    assert len(got) == len(want) == 136 and max(map(len, want)) > 2000
+    for b, (a, w) in enumerate(zip(got, want)):
+        assert np.array_equal(a, w), f"batch {b}"
+    assert np.array_equal(stats, wstats)
+
+
+def test_mrd_plan_with_more_lists_than_there_is_room_for():
+    """15,000 nodes met evenly: nearly every entry of a batch's table is another node, 17 M and more in all.  The kernels that
+    need no lists make the plan."""
+    from orca_b200 import cache
+    from orca_b200.neighbor_finder import NeighborFinder
+    rs = np.random.RandomState(3)
+    E, n, bs, k, budget = 500000, 15000, 50, 32, 400
+    src, dst, ts = rs.randint(1, n, E), rs.randint(1, n, E), np.arange(E, dtype=np.float64)
+    nf = NeighborFinder.build_on_device(src, dst, np.arange(1, E + 1), ts, n)
+    nodes, t = cache.batch_query_order(src, dst, ts, bs)
+    nbr = nf.sample_device(nodes, t, k)[0]
+    table = nbr.cpu().numpy().reshape(E // bs, -1)
+    assert sum(len(np.unique(r)) for r in table) > 16 << 20
+    got, stats = cache.plan_device("MRD", torch.as_tensor(nodes).cuda(), nbr, E, bs, k, n, budget)
+    want, wstats = cache.plan_from_tables("MRD", src, dst, bs, k, nbr.cpu().numpy(), n, budget)
+    assert len(got) == len(want)
+    for b, (a, w) in enumerate(zip(got, want)):
+        assert np.array_equal(a, w), f"batch {b}"
+    assert np.array_equal(stats, wstats)

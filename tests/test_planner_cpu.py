@@ -56,3 +56,16 @@ def test_unknown_strategy_exits():
     with pytest.raises(SystemExit):
         cache.plan_from_tables("FIFO", g.sources, g.destinations, 200, 10, np.zeros((2 * g.n_edges, 10), np.int32),
                                g.n_nodes, 10)
+
+
+def test_workspaces_of_plans_stay_small():
+    """The planners' device memory: for LRU and 2Q no more for a long stream than for a short one, for MRD within 150 MB of
+    the 8 (k + 1) bytes an edge that the tables of next uses take, at any batch size."""
+    from orca_b200 import _lib, build
+    build.build()
+    need = _lib.lib().orca_plan_device_workspace_bytes
+    n, E, k = 1140150, 7833140, 10
+    for bs in (100, 200, 2000, 4000):
+        for strategy in (1, 2):
+            assert need(strategy, 8 * E, bs, k, n, 10000) == need(strategy, E, bs, k, n, 10000) < 160e6
+        assert need(0, E, bs, k, n, 10000) < 8 * (k + 1) * E + 150e6
