@@ -98,14 +98,18 @@ __device__ __forceinline__ float warp_sum(float v) {
 // hundred instructions; double-precision reduction is no way out either (the fp64 and conversion
 // pipes of this GPU made a warp-wide cosine cost ~160 cycles).  fp32 and integer pipes only:
 //   |x| < 2^24   Cody-Waite: k = rint(x / 2pi) (< 2^22), r = x - k*C1 - k*C2 - k*C3 with 2pi split so that the first
-//                two differences are exact (C1 8 bits, C2 11 bits); error against 64 bits, the hardware cosine left
-//                out: 2.4e-7 at most, 3.2e-8 rms;
+//                two differences are exact (C1 8 bits, C2 11 bits); reduction error 2.4e-7 at most, 3.2e-8 rms.  x / 2pi
+//                is rounded before it is rounded to k, by up to a quarter at 2^24, so that k can be one off and |r| exceeds
+//                pi: 3.15 / 3.33 / 3.87 / 4.60 below 2^17 / 2^21 / 2^23 / 2^24;
 //   |x| < 2^30   fixed point: x = m * 2^e with a 24-bit m; the fraction of x / 2pi is the low part of
 //                m * F (F = 2^64 / 2pi) shifted by e, of which the top 32 bits are kept (96-bit product
 //                from two 32 x 32 multiplies); cos is even, so |fraction| (24 bits) goes back to a
 //                float through the 2^23 exponent trick; reduction error 3.8e-7 at most, 1.3e-7 rms;
 //   else         cosf().
-// The hardware cosine approximation is applied to the reduced argument in [-pi, pi] (2^-21 absolute).
+// The hardware cosine approximation is applied to the remainder.  CUDA states its error for [-pi, pi] only (2^-21.19);
+// measured against 64 bits over every float: 4.0e-7 at most up to pi, 2.2e-7 up to 3.5, 4.0e-7 up to 4, 5.3e-7 up to 4.7.
+// So what decides is the error of the whole, over every float of a binade: Cody-Waite 4.9e-7 at most below 2^23, 6.9e-7 up
+// to 2^24, 1.3e-7 rms; fixed point 7.1e-7 at most, 2.1e-7 rms, in each of these binades.
 constexpr float COS_SMALL = 16777216.f;    // 2^24
 // |x| < COS_SMALL, branch free
 __device__ __forceinline__ float cos_small(float x) {

@@ -396,6 +396,35 @@ def test_message_store_and_gru(dev):
     assert mem.nodes.sum() == 0
 
 
+@pytest.mark.parametrize("e", [0, 8, 14, 15, 17, 18, 20, 21, 22, 23, 24, 27, 29])
+def test_time_encoding_of_large_arguments(dev, e):
+    """cos(gap * w) for arguments in [2^(e-1), 2^(e+1)), on both sides of the lines between the reductions.  Bounds: the
+    reduction's error (2.4e-7 at most below 2^24, 3.8e-7 beyond) and the hardware cosine's (5.3e-7 over remainders up to 4.7,
+    4.0e-7 up to pi) added up; for the root mean square what all floats of a binade give (1.29e-7, 2.06e-7) and 7 % for the
+    sample's 100,000 values, whose own deviation is a quarter of a per cent."""
+    from orca_b200 import _lib
+    from orca_b200.memory import Memory
+    rs = np.random.RandomState(e)
+    b = 640
+    mem = Memory(b + 1, D, 4 * D, 4 * D, device=dev)
+    ts = (2.0 ** e * (1 + rs.rand(b))).astype(np.float32)
+    w = (0.5 + 0.5 * rs.rand(D)).astype(np.float32)
+    node = np.arange(1, b + 1)
+    src, other, eidx, pos = (_i32(a, dev) for a in (node, node, np.zeros(b), np.arange(b)))
+    n_win, win = torch.full((1,), b, dtype=torch.int32, device=dev), torch.zeros(b, dtype=torch.int32, device=dev)
+    edges, d_w = torch.zeros(1, D, device=dev), torch.from_numpy(w).to(dev)
+    d_ts = torch.from_numpy(ts.astype(np.float64)).to(dev)
+    _lib.check(_lib.lib().orca_message_store(mem.c_struct(), edges.data_ptr(), d_w.data_ptr(), src.data_ptr(), other.data_ptr(),
+                                             d_ts.data_ptr(), eidx.data_ptr(), b, pos.data_ptr(), b, n_win.data_ptr(),
+                                             win.data_ptr(), _lib.stream_ptr(dev)))
+    x = ts[:, None] * w
+    err = np.abs(mem.messages[1:, 3 * D:].cpu().numpy().astype(np.float64) - np.cos(x.astype(np.float64)))
+    small = x < 2 ** 24
+    for part, most, rms in ((small, 7.7e-7, 1.38e-7), (~small, 7.8e-7, 2.2e-7)):
+        if part.any():
+            assert err[part].max() < most and np.sqrt(np.mean(err[part] ** 2)) < rms
+
+
 @pytest.mark.parametrize("n_nodes", [1501, 70000, 1700000])
 def test_find_uncached_marked_by_sampler(dev, n_nodes):
     """The two-kernel form: the sampling launch marks the candidates, a light single block finishes."""
