@@ -39,7 +39,7 @@ constexpr int A_CHUNKS = 2 * PART_CHUNKS, A_LBO = ROWS * 16 + 16, A_BYTES = A_CH
 constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 1024;
 constexpr int EPI_WARPS = 4, PRODUCERS = 256, THREADS = 32 * EPI_WARPS + PRODUCERS + 32;
 constexpr int TMEM_COLS = 128, BUF_COLS = 64, SMALL = 32;   // two accumulator buffers of main + cross terms
-constexpr int GROUP_ROWS = 32;                 // updates a row block takes before there is another one (16 to 64: the same)
+constexpr int BLOCK_ROWS = 32;                 // updates a row block takes before there is another one (16 to 64: the same)
 constexpr int META = 4;                        // steps whose memory rows are kept
 constexpr int PER = 6;                         // chunks a producer thread has in flight: 34 rows at a time
 
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) gru_chain_kernel(const __grid_cons
   // others have nothing to do
   int most = 0;
   for (int n = 0; n < a.nb; ++n) most = max(most, s_win[n]);
-  const int n_rb = a.split ? max(1, min((int)gridDim.y, (most + GROUP_ROWS - 1) / GROUP_ROWS)) : (int)gridDim.y;
+  const int n_rb = a.split ? max(1, min((int)gridDim.y, (most + BLOCK_ROWS - 1) / BLOCK_ROWS)) : (int)gridDim.y;
   const int n_cta = gridDim.x * n_rb, nb = rb < n_rb ? a.nb : 0;
   // rows of a row block in a batch: the updates spread over the blocks, in steps of eight, at most a tile's
   auto rows_per = [&](int win) { return min(ROWS, ((win + n_rb - 1) / n_rb + 7) & ~7); };

@@ -380,27 +380,35 @@ static inline uint32_t pow2_at_least(uint64_t x) {
 // Batches per group: at most four row blocks of 128 per SM, at most a bit each.  A larger group has fewer partly empty last
 // rounds of row blocks.  What the first group costs before its layers start, index kernels and the memory chain (8 us a
 // batch), is not hidden by anything, so that group is half as large (two blocks per SM; where the chain matters, that is not
-// without reuse), and the rest is dealt out evenly.  ms for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
-// reuse / 40 x 200, by rows of a group and of the first (all with an output kernel on pairs of CTAs):
-//   48 k, one after the other  2.84 / 2.85 / 5.42 / 2.25 / 1.77      76 k so           2.93 / 2.82 / 5.26 / 2.00 / 1.77
-//   evenly, 49 k and 19 k      2.89 / 2.92 / 5.42 /  -   / 1.65      76 k and 19 k     2.87 / 2.84 / 5.22 /  -   / 1.65
-//   76 k and 38 k              2.80 / 2.81 / 5.25 / 2.02 / 1.65      76 k and 57 k     2.85 / 2.91 / 5.33 /  -   / 1.66
-//   95 k and 38 k              2.82 / 2.82 / 5.26 / 2.03 / 1.66
-// With the output kernel as it is, 76 k and 38 k: 2.86 / 2.85 / 5.44 / 2.04 / 1.67.
-constexpr int GROUP_ROWS = 4 * 128 * 148, FIRST_ROWS = GROUP_ROWS / 2;
+// without reuse), and the rest is dealt out evenly.  us for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
+// reuse / 40 x 200, by rows of a group and of the first, 148 SMs:
+//   48 k, one after the other  2862 / 2859 / 5492 / 2247 / 1742      76 k so           2972 / 2808 / 5312 / 1987 / 1743
+//   57 k and 38 k              2819 / 2828 / 5311 / 2103 / 1620      76 k and 19 k     2856 / 2833 / 5309 / 2008 / 1621
+//   76 k and 38 k              2814 / 2837 / 5351 / 2011 / 1621      76 k and 57 k     2853 / 2895 / 5441 / 2013 / 1620
+//   95 k and 38 k              2811 / 2831 / 5274 / 2015 / 1622
+// (Device memory of a group's buffers at 2000 edges a batch, K 10: 2.4 GB, half of it queries and attention sums.)
+static int group_rows() {
+  int device = 0, sms = 0;      // (asked of the device itself: no context is made for it)
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    sms = 148;
+  }
+  return 4 * 128 * sms;
+}
 static int64_t batch_rows(int bs, int k, int layers, int mode) {
   return 3ll * bs * (layers == 2 && mode == ORCA_MODE_NO_REUSE ? 1 + k : 1);
 }
 static int group_size(int bs, int k, int layers, int mode) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, GROUP_ROWS / batch_rows(bs, k, layers, mode)));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(MAX_BATCHES, group_rows() / batch_rows(bs, k, layers, mode)));
 }
 // sizes of the groups of a stream of n batches -> sizes (n entries); their number
 static int group_sizes(int n, int bs, int k, int layers, int mode, int32_t *sizes) {
-  const int most = group_size(bs, k, layers, mode);
+  const int most = group_size(bs, k, layers, mode), first_rows = group_rows() / 2;
   const int64_t rows = batch_rows(bs, k, layers, mode);
   int groups = 0, left = n;
-  if (!(layers == 2 && mode == ORCA_MODE_NO_REUSE) && n * rows > 2ll * FIRST_ROWS) {
-    sizes[groups++] = (int)std::max<int64_t>(1, std::min<int64_t>(most, FIRST_ROWS / rows));
+  if (!(layers == 2 && mode == ORCA_MODE_NO_REUSE) && n * rows > 2ll * first_rows) {
+    sizes[groups++] = (int)std::max<int64_t>(1, std::min<int64_t>(most, first_rows / rows));
     left -= sizes[0];
   }
   for (int rest = ceil_div(left, most); rest > 0; --rest) {
@@ -413,9 +421,13 @@ static int group_sizes(int n, int bs, int k, int layers, int mode, int32_t *size
 // The memory chain is serial, so only what a later batch of the group reads belongs there: in a group of 2000-edge
 // batches on the largest graph 125 of a batch's 890 updates.  The others, every node's last update in the group, wait for
 // nobody, and one launch of the general projection does them behind the chain (chain 208 -> 74 us a group on half of the
-// SMs).  That launch and the message rows it reads are 25 us of latency, which a group with few updates does not win
-// back: streams of 27 x 600 / 16 x 1000 / 8 x 2000 edges a group 3.08 / 3.08 / 6.46 ms without, 3.04 / 3.03 / 5.79 with;
-// 7 x 200 (no reuse) / 32 x 200 2.36 / 2.14 without, 2.38 / 2.13 with.
+// SMs).  That launch and the message rows it reads are 25 us of latency, of which a group with few updates wins back
+// nothing, while the largest graph's wins at every size.  us for a stream of one group, without / with, by its positions:
+//            8 k      12 k     16 k     20 k     24 k     32 k        40 k
+//   2000     457/439  568/530  719/661  840/754  953/847  1224/1107   1498/1342      edges a batch, largest graph
+//   1000     448/462  545/554  690/695  793/802  896/902  1148/1150   1416/1409
+//   600      611/625  840/852  936/944  1149/1154  1367/1372  1701/1705              (K 20)
+//   200      621/630  884/887
 constexpr int SPLIT_FROM = 16384;      // positions [src | dst] of a group
 
 // Index buffers (two of each) and main-stream buffers.  The layer-1 rows that exist at all are few more than the
