@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
         float v[16];
         tmem_ld16_sum(trow + ch * 16, SMALL, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + s_b1[ch * 16 + i] + on * s_g[ch * 16 + i], 0.f);
+        for (int i = 0; i < 16; ++i) v[i] = relu(v[i] + s_b1[ch * 16 + i] + on * s_g[ch * 16 + i]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint4 hi, lo;

@@ -86,6 +86,13 @@ __device__ __forceinline__ void report(int32_t *status, int code, int detail) {
   if (status != nullptr && atomicCAS(status, 0, code) == 0) status[3] = detail;
 }
 
+// torch's relu: a value that is not a number stays one (fmaxf would make it 0, and what follows plausible)
+__device__ __forceinline__ float relu(float x) {
+  float y;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

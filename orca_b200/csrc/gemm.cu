@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(F2_THREADS) attn_output_kernel(SimtOutArgs g) 
     for (int j = 0; j < F2_J; ++j) {
       const int c = tx + 16 * j;
       float h = 0.f;
-      if (c < D) h = fmaxf(acc[i][j] + __ldg(g.w.b1 + c) + v * __ldg(g.w.g + c), 0.f);
+      if (c < D) h = relu(acc[i][j] + __ldg(g.w.b1 + c) + v * __ldg(g.w.g + c));
       s.Hs[r][c] = h;
       acc[i][j] = 0.f;
     }
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(F2_THREADS) score_kernel(ScoreArgs g) {
 #pragma unroll
     for (int j = 0; j < F2_J; ++j) {
       const int c = tx + 16 * j;
-      if (c < D) part += fmaxf(acc[i][j] + __ldg(g.w.b1 + c), 0.f) * __ldg(g.w.w2 + c);
+      if (c < D) part += relu(acc[i][j] + __ldg(g.w.b1 + c)) * __ldg(g.w.w2 + c);
     }
     const float z = half_warp_sum(part) + g.w.b2;
     if (tx == 0 && m < M) g.prob[m] = 1.f / (1.f + expf(-z));

@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
           float v[16];
           tmem_ld16_sum(trow + ch * 16, TMEM_SMALL, v);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + s_bias[ch * 16 + i] + row_on * s_v1[ch * 16 + i], 0.f);
+          for (int i = 0; i < 16; ++i) v[i] = relu(v[i] + s_bias[ch * 16 + i] + row_on * s_v1[ch * 16 + i]);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint4 hi, lo;
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const int c = ch * 16 + i;
-            if (c < D) dot += fmaxf(v[i] + s_bias[c], 0.f) * s_v1[c];
+            if (c < D) dot += relu(v[i] + s_bias[c]) * s_v1[c];
           }
         } else {
 #pragma unroll

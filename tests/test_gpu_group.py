@@ -120,3 +120,33 @@ def test_metrics_on_the_device_equal_the_hosts(bs, E):
     assert _lib.lib().orca_link_metrics(pos.ctypes.data, ngs.ctypes.data, E, bs, want.ctypes.data) == 0
     # (sums of at most bs doubles of one sign in another order: bs * 2^-53)
     np.testing.assert_allclose(make_model(g).eval_epoch_metrics(*args), want, rtol=1e-12)
+
+
+@pytest.mark.parametrize("bs", [256, 300, 4096, 4200])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_metrics_of_scores_that_are_not_finite_are_refused(bs, bad):
+    """A memory row that is not finite makes the scores of its node's edges NaN.  The metrics are refused with the batch's
+    number, as the host's are, whether they are made on the device (up to 4096 edges a batch) or not."""
+    import dataclasses
+    from orca_b200 import _lib
+    from test_gpu_model import make_model
+    g = graph("c1")
+    E = 2 * bs
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs))
+    args = (g.sources[:E], g.destinations[:E], synthetic.negative_destinations(g, seed=1)[:E], g.timestamps[:E],
+            g.edge_idxs[:E], g.spec.n_degree, bs)
+    node = int(np.setdiff1d(g.sources[bs:E], np.r_[g.sources[:bs], g.destinations[:bs], args[2][:bs]])[0])
+    said = []
+    for metrics in (False, True):
+        m = make_model(g)
+        m.memory.memory[node] = bad
+        if metrics:
+            with pytest.raises(ValueError) as e:
+                m.eval_epoch_metrics(*args)
+            said.append(str(e.value))
+        else:
+            pos, neg = m.eval_epoch(*args)
+            assert np.isnan(pos).any() and np.isfinite(pos).any()
+            assert _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, E, bs, np.empty((2, 3)).ctypes.data) == 1
+            said.append(_lib.lib().orca_last_error().decode())
+    assert said[0] == said[1]

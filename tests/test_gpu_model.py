@@ -745,3 +745,28 @@ def test_a_call_that_fails_half_way_leaves_nothing_in_flight(name, reuse, budget
     pos, neg = run(2)
     m.check_status()
     assert torch.isfinite(pos).all() and torch.isfinite(neg).all()
+
+
+@pytest.mark.parametrize("projection", [0, 1])
+@pytest.mark.parametrize("name", ["c1", "t_nb2"])
+def test_values_that_are_not_numbers_reach_the_scores(name, projection):
+    """A node whose memory is not a number: in the first batch the scores of its own edges and of those that see it as a
+    neighbour are NaN, as the reference's are, and the others are what they were."""
+    from orca_b200 import _lib
+    g = graph(name)
+    k = g.spec.n_degree
+    lo = g.n_edges // 2
+    a = [x[lo:lo + 200] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
+    out = []
+    for bad in (0.0, float("nan")):
+        m = make_model(g)
+        m.set_option(_lib.OPT_PROJECTION_MODE, projection)
+        node = int(a[0][17])
+        m.memory.memory[node] = bad
+        out.append([t.cpu().numpy().ravel() for t in m.compute_edge_probabilities(*a, k, False, False, None)])
+        m.check_status()
+    own = a[0] == node
+    for score, was, ends in zip(out[1], out[0], (own | (a[1] == node), own | (a[2] == node))):
+        assert np.isnan(score[ends]).all()
+        assert np.isfinite(was).all() and np.isfinite(score).any()
+        assert np.array_equal(score[~np.isnan(score)], was[~np.isnan(score)])
