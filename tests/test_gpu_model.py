@@ -747,6 +747,33 @@ def test_a_call_that_fails_half_way_leaves_nothing_in_flight(name, reuse, budget
     assert torch.isfinite(pos).all() and torch.isfinite(neg).all()
 
 
+@pytest.mark.parametrize("option", ["dependent_launch", "overlap"])
+@pytest.mark.parametrize("name,reuse,budget", [("c1", True, None), ("t_nb2", True, 0), ("t_nb2", False, None)])
+def test_switches_change_nothing_in_the_recursions_on_two_streams(name, reuse, budget, option):
+    """One layer, unlimited reuse and no reuse: the memory update runs on a stream of its own beside a layer.  Calls of
+    changing size, back to back without a synchronisation, give the same bits with it off."""
+    from orca_b200 import _lib
+    g = graph(name)
+    k = g.spec.n_degree
+    opt = {"dependent_launch": _lib.OPT_DEPENDENT_LAUNCH, "overlap": _lib.OPT_OVERLAP}[option]
+    sizes = [37, 200, 5, 130, 1100, 64, 37, 1] * 2      # (more than 1024 edges: the update as a pair of launches)
+    out = []
+    for enable in (0, 1):
+        m = make_model(g, reuse=reuse, budget=budget)
+        m.set_option(opt, enable)
+        scores, lo = [], 0
+        for n in sizes:
+            a = [x[lo:lo + n] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
+            scores += m.compute_edge_probabilities(*a, k, reuse, False, None)
+            lo += n
+        m.check_status()
+        out.append([torch.cat(scores)] + [getattr(m.memory, t).clone() for t in ("memory", "last_update", "messages",
+                                                                                 "timestamps", "nodes_dev")])
+    assert lo <= g.n_edges
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("projection", [0, 1])
 @pytest.mark.parametrize("name", ["c1", "t_nb2"])
 def test_values_that_are_not_numbers_reach_the_scores(name, projection):

@@ -226,3 +226,25 @@ def test_mrd_plan_with_more_lists_than_there_is_room_for():
     for b, (a, w) in enumerate(zip(got, want)):
         assert np.array_equal(a, w), f"batch {b}"
     assert np.array_equal(stats, wstats)
+
+
+def test_plans_that_callers_keep_hold_a_bounded_amount_of_page_locked_memory(monkeypatch):
+    """A plan of 2 MB or more stays in the page-locked memory that it was copied to, for as long as one of its batches is
+    held; beyond the limit on what callers hold, and below 2 MB, plans are ordinary arrays with the same contents."""
+    import gc
+    from orca_b200 import cache
+    from orca_b200.neighbor_finder import NeighborFinder, _Lent
+    monkeypatch.setattr(NeighborFinder, "LENT", _Lent(16 << 20))
+    rs = np.random.RandomState(2)
+    locked = lambda a: torch.from_numpy(a).is_pinned()
+    for n, share in (((2 << 20) // 8 - 1, 0), ((2 << 20) // 8, 2 << 20), (400000, 4 << 20), (3 << 20, None)):
+        ids = rs.randint(0, 1 << 31, n).astype(np.int32)
+        d_ids = torch.from_numpy(ids).cuda()
+        held = [cache._ids_to_host(d_ids)[n // 2:] for _ in range(10)]      # (a batch of each keeps all of it)
+        gc.collect()
+        want = 0 if not share else min(10, (16 << 20) // share)
+        assert [locked(a) for a in held] == [True] * want + [False] * (10 - want), n
+        for a in held:
+            assert a.dtype == np.int64 and np.array_equal(a, ids[n // 2:])
+        del held, a
+        gc.collect()
