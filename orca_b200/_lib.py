@@ -18,6 +18,7 @@ QT_DIM = 1032
 QT_LD = 1056
 MSG_DIM = 688
 E_BADARG = 1      # ORCA_E_BADARG
+E_BOUNDS = 5      # ORCA_E_BOUNDS
 CAND_CAP = 2048   # ORCA_CAND_CAP
 EXCHANGE_SLOTS = 4  # ORCA_EXCHANGE_SLOTS
 FLAG_WORDS = 48     # ORCA_FLAG_WORDS

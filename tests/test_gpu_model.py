@@ -797,3 +797,66 @@ def test_values_that_are_not_numbers_reach_the_scores(name, projection):
         assert np.isnan(score[ends]).all()
         assert np.isfinite(was).all() and np.isfinite(score).any()
         assert np.array_equal(score[~np.isnan(score)], was[~np.isnan(score)])
+
+
+@pytest.mark.parametrize("layers", [1, 2])
+def test_a_graph_that_knows_fewer_nodes_than_the_model(layers):
+    """get_neighbor_finder(data) knows nodes up to the largest id of its edges.  Edges of nodes beyond that are scored as
+    those of nodes without interactions: the same bits as with a graph that has empty lists for them."""
+    import dataclasses
+    import types
+    from orca_b200.neighbor_finder import get_neighbor_finder
+    g = graph("t_nb2")
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, n_layers=layers))
+    k, low = g.spec.n_degree, g.n_nodes // 2
+    pick = np.nonzero((g.sources < low) & (g.destinations < low))[0]
+    part = types.SimpleNamespace(sources=g.sources[pick], destinations=g.destinations[pick], edge_idxs=g.edge_idxs[pick],
+                                 timestamps=g.timestamps[pick])
+    small, padded = get_neighbor_finder(part), get_neighbor_finder(part, max_node_idx=g.n_nodes - 1)
+    assert small.n_nodes <= low < padded.n_nodes == g.n_nodes and (g.sources[-400:] >= low).any()
+    a = [x[-400:] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
+    out = []
+    for nf in (small, padded):
+        m = make_model(g)
+        m.set_neighbor_finder(nf)
+        got = [np.r_[tuple(t.cpu().numpy().ravel() for t in m.compute_edge_probabilities(*[x[:200] for x in a], k, True, False,
+                                                                                          None))]]
+        got += m.eval_epoch(*a, k, 200, [np.zeros(0, np.int64)] * 2)
+        m.check_status()
+        out.append(got)
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
+def test_a_graph_with_ids_that_the_model_has_no_rows_for_is_refused():
+    """Kernels read the rows of the neighbours and edges that a graph names: it is held against the model's tables when
+    it is first used, and against edge features that replace others."""
+    from orca_b200 import _lib
+    from orca_b200.neighbor_finder import NeighborFinder
+    g = graph("t_nb2")
+    k = g.spec.n_degree
+    a = [x[:100] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
+    m = make_model(g)
+    score = lambda: m.compute_edge_probabilities(*a, k, True, False, None)
+    def lists(node, edge):
+        own = [np.zeros(0)] * g.n_nodes
+        own[3] = np.array([node])
+        return NeighborFinder(own, [np.full(len(x), edge) for x in own], [np.zeros(len(x)) for x in own])
+    score()
+    for node, edge in ((g.n_nodes, 1), (-1, 1), (2, g.n_edges + 1), (2, -5)):
+        m.set_neighbor_finder(lists(node, edge))
+        for run in (score, score, lambda: m.eval_epoch(*a, k, 50, None)):
+            with pytest.raises(_lib.OrcaError) as e:
+                run()
+            assert e.value.code == _lib.E_BOUNDS
+    m.set_neighbor_finder(lists(g.n_nodes - 1, g.n_edges))
+    score()
+    whole = m.edge_raw_features
+    m.edge_raw_features = whole[:-1].clone()
+    for _ in range(2):
+        with pytest.raises(_lib.OrcaError) as e:
+            score()
+        assert e.value.code == _lib.E_BOUNDS
+    m.edge_raw_features = whole
+    score()
+    m.check_status()
