@@ -401,7 +401,7 @@ int orca_plan_mrd(const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k
  * least-recently-used evictions (first entries of numba's argsort of the last-use times) are data parallel
  * around it.  Arguments, outputs and plan order as in orca_plan_mrd / orca_plan_host
  * (plan_cap >= n_batches * budget always suffices).  LRU and 2Q walk a stream in parts, so that their workspace does not
- * grow with it (150 MB at most for a million nodes and batches of 2000 edges). */
+ * grow with it (215 MB for a million nodes and batches of 2000 edges). */
 int64_t orca_plan_device_workspace_bytes(int32_t strategy, int64_t n_edges, int32_t bs, int32_t k,
                                          int64_t n_nodes, int32_t budget);
 int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_t n_edges, int32_t bs, int32_t k,

@@ -10,8 +10,8 @@
 // the range that the budget line falls into are needed, one or two as a rule: two candidates in three share the largest
 // key, which is the first pivot then, and where the equal keys of a range end up follows from its length alone.
 // 200 batches of 2000 edges, 10,700 candidates each, ms of kernels: 24.4 with the kernels of planner_mrd.cu, which walk
-// tables and sort whole lists batch after batch on a cluster of 16 SMs, 3.8 here: lists 0.13, next uses 0.39, the serial
-// step 3.0 (15 us a batch: the block's instructions and barriers), orders 0.30.
+// tables and sort whole lists batch after batch on a cluster of 16 SMs, 3.64 here: lists 0.14, next uses 0.34, the serial
+// step 2.88 (14 us a batch: the block's instructions and barriers), orders 0.29.
 #include <algorithm>
 
 #include "common.cuh"

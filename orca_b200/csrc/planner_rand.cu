@@ -12,7 +12,7 @@
 // (planner_lists.cuh; tie_order.cuh for lists that do not fit shared memory).
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
 // 250 batches of 600 edges with 20 neighbours, LRU, ms of the kernel: 19.2 with draws, swaps, bitmaps and sort in global
-// memory, 9.9 with those in shared memory, 3.5 with lists in place of the tables' 24,000 entries a batch and without the
+// memory, 9.9 with those in shared memory, 3.4 with lists in place of the tables' 24,000 entries a batch and without the
 // levels of the sort that do not decide.
 #include <algorithm>
 
@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
   if (tid == 0 && (failed || b1 == nb)) plan_off[nb] = used;
 }
 
-// Batches whose lists lie in memory at a time: as many as fit 64 MB (250 of 600 edges with 20 neighbours are one launch).
-// A launch more costs some 10 us of state and bitmaps, the 330 batches of it 4.6 ms.
-constexpr int64_t LISTS = 64 << 20;
+// Batches whose lists lie in memory at a time: as many as fit 128 MB (670,000 edges with 20 neighbours, 600 a batch, are one
+// launch of 16.1 ms; with 64 MB they are two, which take 16.3: lists that nothing runs beside, and state and bitmaps).
+constexpr int64_t LISTS = 128 << 20;
 static int64_t chunk_of(int64_t nb, int32_t bs, int32_t k, int64_t n_nodes) {
   return std::min(nb, std::max<int64_t>(1, LISTS / (8 * lists::stride_of(bs, k, n_nodes))));
 }

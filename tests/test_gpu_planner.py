@@ -190,10 +190,10 @@ def test_a_plan_covers_the_nodes_of_its_graph_whatever_number_is_given(strategy)
 @pytest.mark.parametrize("strategy", ["MRD", "LRU", "2Q"])
 @pytest.mark.parametrize("n_src", [130000, 700000])      # sets in shared memory and in global memory
 def test_plans_of_several_launches(n_src, strategy):
-    """The lists of 67 batches of 2000 edges with 30 neighbours lie in memory at a time (LRU, 2Q): two full launches and one
-    of two batches, the last of them short.  Against the host's policies over the same tables."""
+    """The lists of 135 batches of 2000 edges with 30 neighbours lie in memory at a time (LRU, 2Q): two full launches and one
+    of a short batch.  Against the host's policies over the same tables."""
     from orca_b200 import cache, synthetic
-    spec = dataclasses.replace(synthetic.SPECS["t_nb2"], n_src=n_src, n_edges=271001, bs=2000, budget=3000)
+    spec = dataclasses.replace(synthetic.SPECS["t_nb2"], n_src=n_src, n_edges=541001, bs=2000, budget=3000)
     g = synthetic.make_graph(spec, seed=13)
     nodes, ts = cache.batch_query_order(g.sources, g.destinations, g.timestamps, 2000)
     from orca_b200.neighbor_finder import get_neighbor_finder
@@ -201,7 +201,7 @@ def test_plans_of_several_launches(n_src, strategy):
     got, stats = cache.plan_device(strategy, torch.as_tensor(nodes).cuda(), nbr, g.n_edges, 2000, 30, g.n_nodes, 3000, seed=4)
     want, wstats = cache.plan_from_tables(strategy, g.sources, g.destinations, 2000, 30, nbr.cpu().numpy(), g.n_nodes, 3000,
                                           seed=4)
-    assert len(got) == len(want) == 136 and max(map(len, want)) > 2000
+    assert len(got) == len(want) == 271 and max(map(len, want)) > 2000
     for b, (a, w) in enumerate(zip(got, want)):
         assert np.array_equal(a, w), f"batch {b}"
     assert np.array_equal(stats, wstats)

@@ -67,5 +67,5 @@ def test_workspaces_of_plans_stay_small():
     n, E, k = 1140150, 7833140, 10
     for bs in (100, 200, 2000, 4000):
         for strategy in (1, 2):
-            assert need(strategy, 8 * E, bs, k, n, 10000) == need(strategy, E, bs, k, n, 10000) < 160e6
+            assert need(strategy, 8 * E, bs, k, n, 10000) == need(strategy, E, bs, k, n, 10000) < 230e6
         assert need(0, E, bs, k, n, 10000) < 8 * (k + 1) * E + 150e6
