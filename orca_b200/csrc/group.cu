@@ -39,6 +39,10 @@ __device__ __forceinline__ void set_bit(uint32_t *word, uint32_t bit) {
   if ((__ldcg(word) & bit) == 0) atomicOr(word, bit);    // (hub nodes: the bit is set nearly always)
 }
 
+__device__ __forceinline__ KnownIds known_ids(const Args &a) {
+  return {(uint32_t)(a.n_nodes - 1), (uint32_t)a.n_edge_rows - 1};
+}
+
 // neighbour tables of the batch rows; membership bits; last positions; cache bits of the plans inside the group
 template <int G>
 __global__ void __launch_bounds__(256) head_kernel(const __grid_constant__ Args a) {
@@ -53,8 +57,8 @@ __global__ void __launch_bounds__(256) head_kernel(const __grid_constant__ Args 
     const int n = q / (3 * a.bs), r = q - n * 3 * a.bs, b = a.b_of(n);
     const int node = a.img[a.off[n] + r];
     const double t = a.ts[n * a.bs + r % b];
-    sample_query<G>(a.indptr, a.adj_nbr, a.adj_eid, a.adj_ts, a.n_nodes, node, t, q, a.k, lane, gmask, gshift, a.nbr1,
-                    a.eid1, nullptr, a.dt1, a.status, nullptr, nullptr, nullptr, nullptr);
+    sample_query<G>(a.indptr, a.adj_nbr, a.adj_eid, a.adj_ts, a.n_nodes, known_ids(a), node, t, q, a.k, lane, gmask, gshift,
+                    a.nbr1, a.eid1, nullptr, a.dt1, a.status, nullptr, nullptr, nullptr, nullptr);
   }
   // Membership, a thread per row.  A batch holds its hub nodes hundreds of times over: rows of one node that meet in a
   // warp make one entry (the last of them), else every one of them queues at the same words.
@@ -251,8 +255,8 @@ __global__ void __launch_bounds__(256) append_kernel(const __grid_constant__ Arg
       }
     }
     if (lane == 0) a.app_node[p] = v;
-    sample_query<G>(a.indptr, a.adj_nbr, a.adj_eid, a.adj_ts, a.n_nodes, v, t, batch_rows + p, a.k, lane, gmask, gshift,
-                    a.nbr1, a.eid1, nullptr, a.dt1, a.status, nullptr, nullptr, nullptr, nullptr);
+    sample_query<G>(a.indptr, a.adj_nbr, a.adj_eid, a.adj_ts, a.n_nodes, known_ids(a), v, t, batch_rows + p, a.k, lane, gmask,
+                    gshift, a.nbr1, a.eid1, nullptr, a.dt1, a.status, nullptr, nullptr, nullptr, nullptr);
   }
 }
 

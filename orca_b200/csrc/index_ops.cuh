@@ -17,6 +17,10 @@ int launch_batch_head(const orca_tgn_t *m, const int32_t *d_batch, const double 
                       double *ts1, int32_t *cat_dst, int32_t *o_nbr, int32_t *o_eid, float *o_dt, int32_t *status,
                       int64_t *d_last_pos, long long base, cudaStream_t s);
 
+// the neighbour tables of n_cap (d_n: a count on the device) rows of a batch
+int launch_sample_rows(const orca_tgn_t *m, const int32_t *d_nodes, const double *d_ts, int n_cap, const int32_t *d_n,
+                       int32_t *d_nbr, int32_t *d_eid, float *d_delta, int32_t *d_status, cudaStream_t s);
+
 // appends the uncached set to the row list: *d_n_total = n_query + |U|, *d_n_unc = |U|; d_last_pos / base:
 // the records launch_batch_head made for the batch rows
 int launch_uncached_finish(const orca_tgn_t *m, int n_query, int32_t *nodes_io, double *ts_io, int u_cap,

@@ -472,8 +472,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
 
   float *emb_top = d_emb_out ? d_emb_out : w.emb2;
   if (m->n_layers == 1) {
-    ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1, x.ts1, N,
-                              nullptr, k, x.nbr1, x.eid1, nullptr, x.dt1, d_status, s));
+    ORCA_TRY(launch_sample_rows(m, x.nodes1, x.ts1, N, nullptr, x.nbr1, x.eid1, x.dt1, d_status, s));
     ORCA_TRY(tr.mark(PH_SAMPLE_TOP, s));
     ORCA_TRY(layer_query(&m->attn[0], m->mem.memory, x.nodes1, N, nullptr, l, s));
     ORCA_TRY(tr.mark(PH_QUERY_L2, s));
@@ -493,8 +492,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     const float *dt1 = x.dt1;
     const float *table2 = m->hist_emb;
     const int32_t *d_n1 = x.n1;
-    ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1, x.ts1, N,
-                              nullptr, k, x.nbr2, x.eid2, nullptr, x.dt2, d_status, s));
+    ORCA_TRY(launch_sample_rows(m, x.nodes1, x.ts1, N, nullptr, x.nbr2, x.eid2, x.dt2, d_status, s));
     ORCA_TRY(tr.mark(PH_SAMPLE_TOP, s));
     if (mode == ORCA_MODE_NO_REUSE) {
       expand_rows_kernel<<<ceil_div(N * k, 256), 256, 0, s>>>(x.nbr2, N, k, x.nodes1, x.ts1, x.nbr2_loc, x.n1);
@@ -509,8 +507,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
       nbr1 = x.nbr2, eid1 = x.eid2, dt1 = x.dt2;
       d_n1 = nullptr;
     } else {
-      ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1, x.ts1, R1,
-                                x.n1, k, x.nbr1, x.eid1, nullptr, x.dt1, d_status, s));
+      ORCA_TRY(launch_sample_rows(m, x.nodes1, x.ts1, R1, x.n1, x.nbr1, x.eid1, x.dt1, d_status, s));
     }
     ORCA_TRY(tr.mark(PH_SAMPLE_L1, s));
     const bool push1 = mode == ORCA_MODE_REUSE_ALL;
@@ -639,8 +636,7 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
                                                             x.loc_ts, x.n1_loc);
         ORCA_COUNT_LAUNCH();
         ORCA_LAUNCH_CHECK();
-        ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.loc_nodes, x.loc_ts,
-                                  rpr, x.n1_loc, k, x.nbr1, x.eid1, nullptr, x.dt1, d_status, si));
+        ORCA_TRY(launch_sample_rows(m, x.loc_nodes, x.loc_ts, rpr, x.n1_loc, x.nbr1, x.eid1, x.dt1, d_status, si));
       }
       if (b_loc > 0) {
         shard_l2_kernel<<<ceil_div(3 * b_loc, 8), 256, 0, si>>>(x.nbr2, x.eid2, x.dt2, b, k, rb, wb, wa, rpr, b_loc,
@@ -649,9 +645,8 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
         ORCA_LAUNCH_CHECK();
       }
     } else if (u_cap > 0) {
-      ORCA_TRY(orca_sample_topk(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, x.nodes1 + N, x.ts1 + N,
-                                u_cap, x.n_unc, k, x.nbr1 + (size_t)N * k, x.eid1 + (size_t)N * k, nullptr,
-                                x.dt1 + (size_t)N * k, d_status, si));
+      ORCA_TRY(launch_sample_rows(m, x.nodes1 + N, x.ts1 + N, u_cap, x.n_unc, x.nbr1 + (size_t)N * k,
+                                  x.eid1 + (size_t)N * k, x.dt1 + (size_t)N * k, d_status, si));
     }
     // the order in which the two gather launches hand out their rows (heaviest first)
     if (sharded)

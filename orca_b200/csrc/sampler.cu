@@ -31,7 +31,7 @@ template <int G>
 __global__ void __launch_bounds__(256)
 sample_topk_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict__ adj_nbr,
                    const int32_t *__restrict__ adj_eid, const double *__restrict__ adj_ts,
-                   int64_t n_nodes, const int32_t *__restrict__ nodes, const double *__restrict__ qts,
+                   int64_t n_nodes, KnownIds known, const int32_t *__restrict__ nodes, const double *__restrict__ qts,
                    int n_cap, const int32_t *__restrict__ d_n, int k, int32_t *__restrict__ o_nbr,
                    int32_t *__restrict__ o_eid, float *__restrict__ o_et, float *__restrict__ o_dt,
                    int32_t *status, const uint8_t *__restrict__ cache_flag, uint32_t *__restrict__ cand_bitmap) {
@@ -43,7 +43,7 @@ sample_topk_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict
   const int gshift = (threadIdx.x % 32) / G * G;
   const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << gshift);
   for (int q = blockIdx.x * groups_per_block + threadIdx.x / G; q < n; q += gridDim.x * groups_per_block)
-    sample_query<G>(indptr, adj_nbr, adj_eid, adj_ts, n_nodes, nodes[q], qts[q], q, k, lane, gmask, gshift, o_nbr,
+    sample_query<G>(indptr, adj_nbr, adj_eid, adj_ts, n_nodes, known, nodes[q], qts[q], q, k, lane, gmask, gshift, o_nbr,
                     o_eid, o_et, o_dt, status, cache_flag, cand_bitmap, nullptr, nullptr);
 }
 
@@ -54,7 +54,7 @@ sample_topk_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict
 template <int G>
 __global__ void __launch_bounds__(256)
 batch_head_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict__ adj_nbr,
-                  const int32_t *__restrict__ adj_eid, const double *__restrict__ adj_ts, int64_t n_nodes,
+                  const int32_t *__restrict__ adj_eid, const double *__restrict__ adj_ts, int64_t n_nodes, KnownIds known,
                   const int32_t *__restrict__ batch, const double *__restrict__ bts, int b, int k,
                   int32_t *__restrict__ nodes1, double *__restrict__ ts1, int32_t *__restrict__ cat_dst,
                   int32_t *__restrict__ o_nbr, int32_t *__restrict__ o_eid, float *__restrict__ o_dt, int32_t *status,
@@ -77,7 +77,7 @@ batch_head_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
       if (q < 2 * b) cat_dst[q] = q < b ? batch[b + q] : batch[q - b];
       if (node >= 0 && node < n_nodes) atomicMax(&last_pos[node], (unsigned long long)(base + q));
     }
-    sample_query<G>(indptr, adj_nbr, adj_eid, adj_ts, n_nodes, node, t, q, k, lane, gmask, gshift, o_nbr, o_eid,
+    sample_query<G>(indptr, adj_nbr, adj_eid, adj_ts, n_nodes, known, node, t, q, k, lane, gmask, gshift, o_nbr, o_eid,
                     nullptr, o_dt, status, cache_flag, cand_bitmap, cand_count, cand_list, last_pos,
                     (unsigned long long)base);
   }
@@ -558,6 +558,13 @@ static int sm_count() {
   return c != nullptr ? c->sm_count : 148;
 }
 
+static KnownIds known_ids(const orca_tgn_t *m) {
+  KnownIds x;
+  x.nbr = (uint32_t)(m->n_nodes - 1);
+  if (m->n_edge_rows > 0) x.edge = (uint32_t)std::min<int64_t>(m->n_edge_rows - 1, 0x7fffffff);
+  return x;
+}
+
 int launch_batch_head(const orca_tgn_t *m, const int32_t *d_batch, const double *d_bts, int b, int32_t *nodes1,
                       double *ts1, int32_t *cat_dst, int32_t *o_nbr, int32_t *o_eid, float *o_dt, int32_t *status,
                       int64_t *d_last_pos, long long base, cudaStream_t s) {
@@ -568,12 +575,12 @@ int launch_batch_head(const orca_tgn_t *m, const int32_t *d_batch, const double 
   if (k <= 16) {
     const int grid = std::min(ceil_div(n, threads / 16), sm_count() * 16);
     ORCA_CUDA(launch_dep(batch_head_kernel<16>, grid, threads, 0, s, m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts,
-                         m->n_nodes, d_batch, d_bts, b, k, nodes1, ts1, cat_dst, o_nbr, o_eid, o_dt, status,
+                         m->n_nodes, known_ids(m), d_batch, d_bts, b, k, nodes1, ts1, cat_dst, o_nbr, o_eid, o_dt, status,
                          m->cache_flag, m->cand_bitmap, cand_count, cand_list, lp, base));
   } else {
     const int grid = std::min(ceil_div(n, threads / 32), sm_count() * 16);
     ORCA_CUDA(launch_dep(batch_head_kernel<32>, grid, threads, 0, s, m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts,
-                         m->n_nodes, d_batch, d_bts, b, k, nodes1, ts1, cat_dst, o_nbr, o_eid, o_dt, status,
+                         m->n_nodes, known_ids(m), d_batch, d_bts, b, k, nodes1, ts1, cat_dst, o_nbr, o_eid, o_dt, status,
                          m->cache_flag, m->cand_bitmap, cand_count, cand_list, lp, base));
   }
   ORCA_COUNT_LAUNCH();
@@ -668,7 +675,7 @@ int orca_csr_build_host(const int64_t *h_src, const int64_t *h_dst, const int64_
 }
 
 static int orca_sample_topk_impl(const int64_t *d_indptr, const int32_t *d_adj_nbr, const int32_t *d_adj_eid,
-                            const double *d_adj_ts, int64_t n_nodes, const int32_t *d_nodes,
+                            const double *d_adj_ts, int64_t n_nodes, KnownIds known, const int32_t *d_nodes,
                             const double *d_ts, int32_t n_query_cap, const int32_t *d_n_query, int32_t k,
                             int32_t *d_nbr, int32_t *d_eid, float *d_edge_times, float *d_delta,
                             int32_t *d_status, const uint8_t *d_cache_flag, uint32_t *d_cand_bitmap, void *stream) {
@@ -683,13 +690,13 @@ static int orca_sample_topk_impl(const int64_t *d_indptr, const int32_t *d_adj_n
     // (a launch whose row count lives on the device usually covers far fewer rows than its capacity)
     const int grid = std::min(ceil_div(n_query_cap, per), d_n_query ? sm_count() * 2 : sm_count() * 16);
     ORCA_CUDA(launch_dep(sample_topk_kernel<16>, grid, threads, 0, s, d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes,
-                         d_nodes, d_ts, n_query_cap, d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status,
+                         known, d_nodes, d_ts, n_query_cap, d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status,
                          d_cache_flag, d_cand_bitmap));
   } else {
     const int per = threads / 32;
     const int grid = std::min(ceil_div(n_query_cap, per), sm_count() * 16);
     ORCA_CUDA(launch_dep(sample_topk_kernel<32>, grid, threads, 0, s, d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes,
-                         d_nodes, d_ts, n_query_cap, d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status,
+                         known, d_nodes, d_ts, n_query_cap, d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status,
                          d_cache_flag, d_cand_bitmap));
   }
   ORCA_COUNT_LAUNCH();
@@ -702,7 +709,7 @@ int orca_sample_topk(const int64_t *d_indptr, const int32_t *d_adj_nbr, const in
                      const double *d_ts, int32_t n_query_cap, const int32_t *d_n_query, int32_t k,
                      int32_t *d_nbr, int32_t *d_eid, float *d_edge_times, float *d_delta,
                      int32_t *d_status, void *stream) {
-  return orca_sample_topk_impl(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, d_nodes, d_ts, n_query_cap,
+  return orca_sample_topk_impl(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, KnownIds(), d_nodes, d_ts, n_query_cap,
                           d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status, nullptr, nullptr, stream);
 }
 
@@ -713,7 +720,7 @@ int orca_sample_topk_mark(const int64_t *d_indptr, const int32_t *d_adj_nbr, con
                           int32_t *d_status, const uint8_t *d_cache_flag, uint32_t *d_cand_bitmap,
                           void *stream) {
   ORCA_CHECK_ARG(d_cache_flag && d_cand_bitmap);
-  return orca_sample_topk_impl(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, d_nodes, d_ts, n_query_cap,
+  return orca_sample_topk_impl(d_indptr, d_adj_nbr, d_adj_eid, d_adj_ts, n_nodes, KnownIds(), d_nodes, d_ts, n_query_cap,
                           d_n_query, k, d_nbr, d_eid, d_edge_times, d_delta, d_status, d_cache_flag,
                           d_cand_bitmap, stream);
 }
@@ -850,3 +857,13 @@ int orca_last_occurrence(const int32_t *d_ids, int32_t n_cap, const int32_t *d_n
 }
 
 }  // extern "C"
+
+namespace orca {
+
+int launch_sample_rows(const orca_tgn_t *m, const int32_t *d_nodes, const double *d_ts, int n_cap, const int32_t *d_n,
+                       int32_t *d_nbr, int32_t *d_eid, float *d_delta, int32_t *d_status, cudaStream_t s) {
+  return orca_sample_topk_impl(m->indptr, m->adj_nbr, m->adj_eid, m->adj_ts, m->n_nodes, known_ids(m), d_nodes, d_ts, n_cap,
+                               d_n, m->k, d_nbr, d_eid, nullptr, d_delta, d_status, nullptr, nullptr, s);
+}
+
+}  // namespace orca

@@ -34,7 +34,13 @@ __device__ __forceinline__ long long lower_bound_group(const double *__restrict_
   return lo + __popc(b);
 }
 
-// One query: lower bound, copy of the k entries in front of it (right-aligned, zero padded), and --
+// The largest neighbour and edge id that the caller's tables have rows for (left alone: it reads none).
+struct KnownIds {
+  uint32_t nbr = 0xffffffffu, edge = 0xffffffffu;
+};
+
+// One query: lower bound, copy of the k entries in front of it (right-aligned, zero padded; an id that is not `known` is
+// reported and its slot left empty), and --
 // optionally -- marking of the sampled neighbours as candidates of the uncached set: the neighbour
 // (the padding node 0 for an empty slot) gets its bit in `cand_bitmap` when its cache flag is clear.
 // Hub nodes are sampled thousands of times per batch, so the bit is tested first and only the first
@@ -43,7 +49,7 @@ __device__ __forceinline__ long long lower_bound_group(const double *__restrict_
 template <int G>
 __device__ __forceinline__ void sample_query(const int64_t *__restrict__ indptr, const int32_t *__restrict__ adj_nbr,
                                              const int32_t *__restrict__ adj_eid, const double *__restrict__ adj_ts,
-                                             int64_t n_nodes, int node, double t, int q, int k, int lane,
+                                             int64_t n_nodes, KnownIds known, int node, double t, int q, int k, int lane,
                                              unsigned gmask, int gshift, int32_t *__restrict__ o_nbr,
                                              int32_t *__restrict__ o_eid, float *__restrict__ o_et,
                                              float *__restrict__ o_dt, int32_t *status,
@@ -67,6 +73,11 @@ __device__ __forceinline__ void sample_query(const int64_t *__restrict__ indptr,
       nb = adj_nbr[src];
       ei = adj_eid[src];
       et = (float)adj_ts[src];
+      if ((uint32_t)nb > known.nbr || (uint32_t)ei > known.edge) {
+        report(status, ORCA_E_BOUNDS, q);
+        nb = ei = 0;
+        et = 0.f;
+      }
     }
     const size_t o = (size_t)q * k + lane;
     o_nbr[o] = nb;

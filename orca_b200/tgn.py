@@ -441,7 +441,6 @@ class TGN(nn.Module):
             seen = ([x.data_ptr() for x in tables], _versions(tables), d["_mode"], d["_rank"], d["_world"],
                     d["_layer1_ranks"], d["_input_stream"])
             if seen != d["_desc_seen"] or edges is not d["_desc_edges"] or seen[1] is None:
-                self._check_edges(d["_desc_last_edge"], edges)
                 d["_desc_seen"], d["_desc_edges"] = seen, edges
                 tm = d["_desc_mem"]
                 tm.memory, tm.last_update, tm.messages, tm.msg_ts, tm.msg_flag, t.edge_table = seen[0][:6]
@@ -452,11 +451,12 @@ class TGN(nn.Module):
                 t.mode, t.rank, t.world, t.layer1_ranks, t.input_stream = seen[2:]
                 _lib.settle(self.device)
             return t
-        indptr, last_edge = self._adjacency(nf)
-        self._check_edges(last_edge, self.edge_raw_features)
         t = _lib.TgnT()
         d["_desc_seen"] = d["_desc_edges"] = None
-        d["_desc_indptr"], d["_desc_last_edge"] = indptr, last_edge
+        # (the kernels look up every node of the model's tables: one that the graph does not know, as one of the training
+        # edges alone knows ids up to their largest, has no interactions)
+        more = self.n_nodes - nf.n_nodes
+        indptr = d["_desc_indptr"] = torch.cat([nf.indptr, nf.indptr[-1:].expand(more)]) if more > 0 else nf.indptr
         if getattr(self, "_exchange", None) is not None:
             rows, flags, cap, _, grus, gcap = self._exchange
             for r in range(len(rows)):
@@ -500,24 +500,6 @@ class TGN(nn.Module):
         t.input_stream = self._input_stream
         _lib.settle(self.device)
         return t
-
-    def _adjacency(self, nf):
-        """(indptr, largest edge id) of a graph for this model: the kernels look up every node of the model's tables in the
-        graph, and read the rows of every neighbour and edge that it names.  A node that the graph does not know (a graph of
-        the training edges alone knows ids up to their largest) has no interactions."""
-        first, last, first_edge, last_edge = torch.stack([x for a in (nf.adj_nbr, nf.adj_eid) for x in a.aminmax()]).tolist()
-        if first < 0 or last >= self.n_nodes:
-            raise _lib.OrcaError(_lib.E_BOUNDS, f"the graph has neighbours {first} to {last}, the model {self.n_nodes} nodes")
-        if first_edge < 0:
-            raise _lib.OrcaError(_lib.E_BOUNDS, f"the graph has an edge {first_edge}")
-        more = self.n_nodes - nf.n_nodes
-        return (torch.cat([nf.indptr, nf.indptr[-1:].expand(more)]) if more > 0 else nf.indptr), last_edge
-
-    @staticmethod
-    def _check_edges(last_edge, features):
-        if last_edge >= features.shape[0]:
-            raise _lib.OrcaError(_lib.E_BOUNDS, f"the graph has edges up to {last_edge}, the edge features {features.shape[0]} "
-                                                "rows")
 
     def _workspace(self, b, k):
         u_cap = min(3 * b * k, self.n_nodes) if self.n_layers == 2 else 0

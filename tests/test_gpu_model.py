@@ -828,35 +828,41 @@ def test_a_graph_that_knows_fewer_nodes_than_the_model(layers):
         assert np.array_equal(x, y)
 
 
-def test_a_graph_with_ids_that_the_model_has_no_rows_for_is_refused():
-    """Kernels read the rows of the neighbours and edges that a graph names: it is held against the model's tables when
-    it is first used, and against edge features that replace others."""
+@pytest.mark.parametrize("k", [10, 20])
+@pytest.mark.parametrize("name,reuse,budget", [("c1", True, None), ("t_nb2", True, None), ("t_nb2", True, 0), ("t_nb2", False, None)])
+def test_sampled_ids_without_rows_are_reported(name, reuse, budget, k):
+    """A graph can name nodes or edges that the model's tables have no rows for.  A slot that one of them is sampled into is
+    left empty and reported -- by a single call to a later one, by a stream when it ends -- and one that no query reaches
+    does no harm."""
+    import dataclasses
     from orca_b200 import _lib
     from orca_b200.neighbor_finder import NeighborFinder
-    g = graph("t_nb2")
-    k = g.spec.n_degree
-    a = [x[:100] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
-    m = make_model(g)
-    score = lambda: m.compute_edge_probabilities(*a, k, True, False, None)
-    def lists(node, edge):
+    g = graph(name)
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, n_degree=k))
+    hub = int(np.bincount(g.sources[:200]).argmax())
+    a = [x[:200] for x in (g.sources, g.destinations, np.roll(g.destinations, 1), g.timestamps, g.edge_idxs)]
+    a[3] = a[3] + 10.0
+
+    def lists(node, edge, time):
         own = [np.zeros(0)] * g.n_nodes
-        own[3] = np.array([node])
-        return NeighborFinder(own, [np.full(len(x), edge) for x in own], [np.zeros(len(x)) for x in own])
-    score()
-    for node, edge in ((g.n_nodes, 1), (-1, 1), (2, g.n_edges + 1), (2, -5)):
-        m.set_neighbor_finder(lists(node, edge))
-        for run in (score, score, lambda: m.eval_epoch(*a, k, 50, None)):
+        own[hub] = np.array([1, node, 2])
+        return NeighborFinder(own, [np.array([3, edge, 4])[:len(x)] for x in own], [np.array([1.0, time, time])[:len(x)] for x in own])
+
+    def run(nf, stream):
+        m = make_model(g, reuse=reuse, budget=budget)
+        m.set_neighbor_finder(nf)
+        plan = [np.zeros(0, np.int64)] * 4 if reuse and budget is None else None
+        if stream:
+            return m.eval_epoch(*a, k, 50, plan, reuse=reuse)
+        s = m.compute_edge_probabilities(*a, k, reuse, False, plan[0] if plan else None)
+        m.check_status()
+        return [x.cpu().numpy() for x in s]
+    for stream in (False, True):
+        for node, edge in ((g.n_nodes, 1), (-1, 1), (2, g.n_edges + 1), (2, -5), (2 ** 31 - 1, 2 ** 31 - 1)):
             with pytest.raises(_lib.OrcaError) as e:
-                run()
+                run(lists(node, edge, 2.0), stream)
             assert e.value.code == _lib.E_BOUNDS
-    m.set_neighbor_finder(lists(g.n_nodes - 1, g.n_edges))
-    score()
-    whole = m.edge_raw_features
-    m.edge_raw_features = whole[:-1].clone()
-    for _ in range(2):
-        with pytest.raises(_lib.OrcaError) as e:
-            score()
-        assert e.value.code == _lib.E_BOUNDS
-    m.edge_raw_features = whole
-    score()
-    m.check_status()
+        late = run(lists(g.n_nodes, -5, 1e30), stream)      # (behind every query)
+        for x, y in zip(run(lists(g.n_nodes - 1, g.n_edges, 1e30), stream), late):
+            assert np.array_equal(x, y) and np.isfinite(x).all()
+        run(lists(g.n_nodes - 1, g.n_edges, 2.0), stream)
