@@ -430,7 +430,8 @@ int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_t n_edges, 
 #define ORCA_MODE_NO_REUSE 2
 
 typedef struct {
-  /* graph */
+  /* graph: indptr has n_nodes + 1 entries; a sampled neighbour that is no node of the model, or edge beyond n_edge_rows
+   * (where that is given), leaves its slot empty and ORCA_E_BOUNDS in the status word */
   const int64_t *indptr; const int32_t *adj_nbr; const int32_t *adj_eid; const double *adj_ts;
   const float *edge_table; int64_t n_nodes; int64_t n_edge_rows;
   /* weights */
@@ -555,6 +556,7 @@ int orca_tgn_eval_epoch(const orca_tgn_t *m, const orca_epoch_t *e, int32_t u_ca
  * One batch from host arrays (one GPU): orca_tgn_eval_batch with its inputs narrowed into a ring of ORCA_CALL_SLOTS
  * page-locked slots and copied from there on the context's copy stream.  Waits only when the ring is full.  The status
  * word follows the batch to h_status (page-locked) in `stream` order.
+ * An entry that runs batches and fails half-way waits for what it has enqueued before it returns (not under capture).
  * An id outside its table: this entry and orca_tgn_eval_epoch return ORCA_E_BOUNDS with nothing of the batch enqueued;
  * the kernels of orca_tgn_eval_group read it as node or edge 0 and leave ORCA_E_BOUNDS in the status word.
  */
