@@ -16,20 +16,30 @@
 
 namespace orca {
 
-// One warp per query row.  A row's slots are taken two at a time: their pieces are loaded into registers -- every lane
-// owns 16-byte pieces l, l + 32, l + 64 of the gathered [neighbour | edge feature] part and column PAIRS l, l + 32,
+// One warp per query row.  A row's slots are taken two or four at a time: their pieces are loaded into registers -- every
+// lane owns 16-byte pieces l, l + 32, l + 64 of the gathered [neighbour | edge feature] part and column PAIRS l, l + 32,
 // l + 64 of the time-encoding part, which is computed (cos of delta * w) two columns at a time with the packed
 // two-wide fp32 instructions of this architecture while the loads are in flight -- then come the partial dot products
-// with the two query heads, one cross-lane sum of all four logits at once, a running softmax and the weighted sums, all
-// from the same registers.
-// What bounds it (48 k rows of ten slots, 165 us; under the profiler 169): the instructions of a row (1800 a warp, a
-// third of them the time encodings) against 16 resident warps per SM: issue slots 49 % busy, a warp issues every 8
-// cycles (3 of them for loads), DRAM 29 %, L2 25 %, L1 50 %.  Measured against it: two passes over the rows with parked
-// logits and time encodings (the form before) 178 us; four slots a step at 12 warps 186; slots copied ahead with
-// cp.async, two or four at a time, 167 to 201; the long cosine inlined with a variant of the loop per range, 360
-// (instruction cache).  A launch of a single batch is no faster than the two passes were (6000 rows 29.2 us, before
-// 28.9): there the two or three rows of each warp, one after the other, are what it takes.  The 688-byte rows are not moved by cp.async.bulk: an SM retires only
-// about one small bulk copy per ~130 cycles.
+// with the two query heads, one cross-lane sum of all logits of the step at once, a running softmax and the weighted sums,
+// all from the same registers.
+// What bounds it: the instructions of a row against the 16 or 12 warps an SM that the registers allow (a warp issues every
+// 7 cycles, issue slots half busy), and with ten slots a row DRAM, which carries the queries in and the images out
+// (66 k rows of the largest graph: 0.85 GB, 5 TB/s).  Loads of the slots' rows cost next to nothing: with all of them in L1
+// a launch took 2 % less.  So what helps is fewer instructions a slot (193 -> 160, and 143 four at a time, of 75 that the sums,
+// products and cosines cannot do without) and queries that do not pass through L1 once a step:
+//   - what all lanes need of a slot (addresses, time difference) is worked out once a row, a slot a lane, and read back from
+//     shared memory; so are the weights, twice each, as the packed instructions take them;
+//   - one exponential a step gives weights and scales, in lanes of their own; sums are rescaled where a maximum rose;
+//   - a row's query is brought to shared memory by one bulk copy while the row before it is written.
+// us a launch (queries written by the kernel before; 66 k rows of the largest graph, K 10 / 60 k of c4, K 10 / 54 k, K 20):
+// before 197 / 197 / 340; so 166 / 162 / 254.  Four slots a step at 168 registers against two at 128, 27 k rows, K 8 / 10 / 12 /
+// 14 / 16 / 20 / 32: 79 / 97 / 97 / 116 / 117 / 136 / 187 against 83 / 93 / 106 / 118 / 130 / 152 / 214; 30 k of c4, where rows are
+// shorter: 81 / 95 / 97 / 112 / 112 / 128 / 175 against 80 / 89 / 97 / 108 / 116 / 136 / 192: four from K 11 on.
+// Measured against it: queries in registers at 12 warps (181 / 175 / 288); a row's first slots loaded before the row in front
+// of it is written (177 / 173 / 307); four slots and a tail of two (176 / 172 / 260).  Of the form before: two passes over the
+// rows with parked logits 8 % slower, slots copied ahead with cp.async up to 20 %, the long cosine inlined with a variant of
+// the loop per range twice the time (instruction cache).  The 688-byte rows are not moved by cp.async.bulk: an SM retires
+// only about one small bulk copy per ~130 cycles.
 //
 // Work distribution.  Rows differ tenfold in cost (0 to k valid slots) and a launch of a single batch holds only two
 // to three rows per resident warp, so WHO gets WHICH row decides the length of the launch:
@@ -37,9 +47,10 @@ namespace orca {
 //   - tickets walk the rows in the order of `order` (rows sorted by falling number of valid slots,
 //     made by row_order_kernel beside the sampling), so that the launch ends on its lightest rows.
 // A warp draws its next ticket when it starts a row and reads it after the row's first slots; the indices of the next
-// row are loaded while the rest of the row is worked on.  No block-level synchronisation, no shared memory.
-constexpr int GA_THREADS = 64, GA_BLOCKS = 8;    // 16 warps per SM at 128 registers
-constexpr int GS = 2;                           // slots per step
+// row are loaded while the rest of the row is worked on.  No block-level synchronisation.
+constexpr int GA_THREADS = 64, GA_WARPS = GA_THREADS / 32;
+constexpr int ga_blocks(int slots) { return slots == 2 ? 8 : 6; }   // an SM: 16 warps at 128 registers, 12 at 168
+constexpr int GA_WIDE_FROM = 11;                // slots a row from which they are taken four at a time
 constexpr int GA_MEM_F4 = 2 * D / 4;            // 86 sixteen-byte pieces of [neighbour | edge feature]
 constexpr int GA_ROW_F4 = D / 4;                // 43 pieces per table row
 constexpr int GA_P_ITERS = 3;                   // pieces / time-column pairs per lane (the third for lanes 0..21)
@@ -51,14 +62,14 @@ __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 lo2(const float4 &v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4 &v) { return make_float2(v.z, v.w); }
 
-// cos of two arguments below COS_SMALL at once: the Cody-Waite reduction of cos_small in packed arithmetic;
-// the nearest integer of x / 2pi comes from adding and subtracting 1.5 * 2^23
+// cos of two arguments below COS_SMALL at once: the reduction of cos_small in packed arithmetic with fewer steps.  The
+// nearest integer k of x / 2pi comes from adding and subtracting 1.5 * 2^23, in one fused step, and 2pi is split in two:
+// x - k * C1 is a multiple of 2^-22 below 4 (C1 has 24 bits, the last of them 2^-21), so the first difference is exact.
 __device__ __forceinline__ float2 cos_small2(float2 x) {
-  const float2 t = mul2(x, dup2(0.15915494309189535f));
-  const float2 kk = add2(add2(t, dup2(12582912.f)), dup2(-12582912.f));
-  float2 r = fma2(kk, dup2(-6.28125f), x);
-  r = fma2(kk, dup2(-0.0019350051879882812f), r);
-  r = fma2(kk, dup2(-3.019916050561733e-07f), r);
+  const float2 t = fma2(x, dup2(0.15915494309189535f), dup2(12582912.f));
+  const float2 kk = add2(t, dup2(-12582912.f));
+  float2 r = fma2(kk, dup2(-6.2831855f), x);
+  r = fma2(kk, dup2(1.7484556e-07f), r);
   return make_float2(__cosf(r.x), __cosf(r.y));
 }
 
@@ -115,22 +126,16 @@ row_order_kernel(const int32_t *__restrict__ nbr_a, int n_cap_a, const int32_t *
   for (int r = tid; r < n; r += 1024) order[atomicAdd(&s_bin[count(r)], 1)] = r;
 }
 
-// Loads one slot's pieces of this lane: piece l of the neighbour row; piece l + 32 of the concatenation (neighbour row
-// for l < 11, else edge row piece l - 11); piece l + 64 (edge row piece l + 21, l < 22; the other lanes re-read piece 0
-// of the edge row, which is never used).
-struct SlotRows {
-  const float4 *n0, *n1;
-  int at1, at2, split;
-  bool from_edge;
-  const float4 *e_tab;
-  __device__ __forceinline__ void load(int nb, int ei, int lane, float4 (&x)[3]) const {
-    const float4 *nrow = (nb >= split ? n1 : n0) + (size_t)nb * GA_ROW_F4;
-    const float4 *erow = e_tab + (size_t)ei * GA_ROW_F4;
-    x[0] = __ldg(nrow + lane);
-    x[1] = __ldg((from_edge ? erow : nrow) + at1);
-    x[2] = __ldg(erow + at2);
-  }
+// What a step needs of a slot, by all lanes at once: where its two rows start, its time difference (twice: an operand of
+// the packed instructions) and how many pair groups of its time encoding hold large arguments (time_terms).  The edge row's
+// address is a row early, so that a lane's pieces l, l + 32, l + 64 of [neighbour | edge feature] lie 0, 512 and 1024 bytes
+// behind 16 l of the one or the other.
+struct __align__(16) SlotRec {
+  const char *nbr, *edge;
+  float dt[2];
+  int large, unused;
 };
+__device__ __forceinline__ float4 ldg4(const char *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
 
 // Sums V values (V a power of two up to 32) over the warp: lane l returns the total of value l / (32 / V).
 template <int V>
@@ -151,35 +156,38 @@ __device__ __forceinline__ float warp_sum_many(float (&v)[V], int lane) {
   return s;
 }
 
-template <bool IMAGE>
-__global__ void __launch_bounds__(GA_THREADS, GA_BLOCKS)
+template <bool IMAGE, int GS>
+__global__ void __launch_bounds__(GA_THREADS, ga_blocks(GS))
 attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_table,
                    const float *__restrict__ nbr_table2, int nbr_split,
                    const float *__restrict__ edge_table, const float *__restrict__ time_w,
                    const int32_t *__restrict__ nbr, const int32_t *__restrict__ eid,
                    const float *__restrict__ delta, int k, int n_cap, const int32_t *__restrict__ d_n,
                    const int32_t *__restrict__ order, void *__restrict__ ctx, uint8_t *__restrict__ valid_out,
-                   int32_t *__restrict__ ticket, unsigned long long *__restrict__ prof) {
+                   int32_t *__restrict__ ticket, unsigned long long *__restrict__ prof, int32_t *status, long long wait_limit) {
   constexpr unsigned FULL = 0xffffffffu;
+  __shared__ __align__(128) float s_q[GA_WARPS][QT_LD];
+  __shared__ SlotRec s_rec[GA_WARPS][ORCA_MAX_K + GS - 1];
+  __shared__ __align__(16) float s_p[GA_WARPS][4 * GS + 4];
+  __shared__ __align__(8) unsigned long long s_bar[GA_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t qbar = tc::smem_addr(&s_bar[warp]);
+  if (lane == 0) {
+    tc::mbar_init(qbar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
   dep_trigger();
   dep_wait();
   const int n = rows_of(n_cap, d_n);
-  const int lane = threadIdx.x & 31;
   const bool third = lane + 64 < GA_MEM_F4;       // lanes 0..21 own a third piece / pair
-  // this lane's time-encoding frequencies, as column pairs, and the largest frequency of each pair group
+  const bool from_edge = lane >= GA_ROW_F4 - 32;  // whose piece l + 32 is one of the edge row
   float2 wt[GA_P_ITERS];
 #pragma unroll
   for (int i = 0; i < GA_P_ITERS; ++i)
     wt[i] = (i < 2 || third) ? __ldg(reinterpret_cast<const float2 *>(time_w) + lane + 32 * i) : make_float2(0.f, 0.f);
   const float wg0 = __ldg(time_w), wg1 = __ldg(time_w + 64), wg2 = __ldg(time_w + 128);
   unsigned long long prof_rows = 0, prof_slots = 0;
-  SlotRows rows;
-  rows.n0 = reinterpret_cast<const float4 *>(nbr_table), rows.n1 = reinterpret_cast<const float4 *>(nbr_table2);
-  rows.e_tab = reinterpret_cast<const float4 *>(edge_table);
-  rows.from_edge = lane >= GA_ROW_F4 - 32;
-  rows.at1 = rows.from_edge ? lane - (GA_ROW_F4 - 32) : lane + 32;
-  rows.at2 = third ? lane + 64 - GA_ROW_F4 : 0;
-  rows.split = nbr_split;
 
   // (A group's rows from the last one back: the queries written last are still in L2, and so are the images of the rows
   // that the output kernel starts with.  200 MB of queries a launch do not fit it: 50 batches of 2000 5.80 -> 5.68 ms, 51 of
@@ -194,19 +202,33 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       o_dt = delta[o];
     }
   };
+  bool alive = true;
+  uint32_t phase = 0;
+  auto fetch_query = [&](int r) {
+    if (lane == 0 && alive) {
+      tc::mbar_expect_tx(qbar, QT_LD * 4);
+      tc::bulk_g2s(tc::smem_addr(s_q[warp]), qt + (size_t)r * QT_LD, QT_LD * 4, qbar);
+    }
+  };
   int tkt = 0;
   if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
   tkt = __shfl_sync(FULL, tkt, 0);
   int row = tkt < n ? row_of_ticket(tkt) : -1;
   int my_nbr = 0, my_eid = 0;
   float my_dt = 0.f;
-  if (row >= 0) load_indices(row, my_nbr, my_eid, my_dt);
+  if (row >= 0) {
+    fetch_query(row);
+    load_indices(row, my_nbr, my_eid, my_dt);
+  }
+  float4 x[GS][3];                                 // (the third piece of the lanes that have none stays zero)
+#pragma unroll
+  for (int s = 0; s < GS; ++s) x[s][2] = make_float4(0.f, 0.f, 0.f, 0.f);
+  float *const pbuf = s_p[warp];
   while (row >= 0) {
     // the next ticket is drawn now and its row's indices are requested after the first slots (see above)
     if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
     int next = -1, nx_nbr = 0, nx_eid = 0;
     float nx_dt = 0.f;
-    bool drawn = false;
     auto draw_next = [&]() {
       const int t = __shfl_sync(FULL, tkt, 0);
       if (t < n) {
@@ -215,46 +237,65 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       }
     };
     const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
-    const int n_valid = __popc(vmask);
     float4 am0[3], am1[3];                         // weighted sums of the gathered part, heads 0 / 1
     float2 at0[GA_P_ITERS], at1[GA_P_ITERS];       // and of the time part
 #pragma unroll
     for (int i = 0; i < 3; ++i) am0[i] = am1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
-    float inv0 = 0.f, inv1 = 0.f;
-    if (n_valid > 0) {
-      // which pair groups of this lane's slot need the fixed-point cosine (see time_terms)
-      int my_nl;
+    float sum0 = 0.f, sum1 = 0.f;
+    tc::mbar_wait(qbar, phase, status, 800, alive, wait_limit);
+    if (vmask != 0) {
+      const int first = __ffs(vmask) - 1, range = 32 - __clz(vmask) - first;
+      const unsigned valid = vmask >> first;
       {
+        // empty places among the slots, and behind them up to a whole step, repeat the first slot with weight zero
+        const int f_nbr = __shfl_sync(FULL, my_nbr, first), f_eid = __shfl_sync(FULL, my_eid, first);
+        const float f_dt = __shfl_sync(FULL, my_dt, first);
+        if (my_nbr == 0) my_nbr = f_nbr, my_eid = f_eid, my_dt = f_dt;
+        // which pair groups of the slot need the fixed-point cosine (see time_terms)
         const float adt = fabsf(my_dt);
-        my_nl = (adt * wg0 >= COS_SMALL ? 1 : 0) + (adt * wg1 >= COS_SMALL ? 1 : 0) + (adt * wg2 >= COS_SMALL ? 1 : 0);
-        if (!(adt * wg0 < 1073741824.f)) my_nl = -1;   // beyond the fixed-point range (or not finite)
+        int large = (adt * wg0 >= COS_SMALL ? 1 : 0) + (adt * wg1 >= COS_SMALL ? 1 : 0) + (adt * wg2 >= COS_SMALL ? 1 : 0);
+        if (!(adt * wg0 < 1073741824.f)) large = -1;   // beyond the fixed-point range (or not finite)
+        SlotRec rec;
+        rec.nbr = reinterpret_cast<const char *>(my_nbr >= nbr_split ? nbr_table2 : nbr_table) + (size_t)my_nbr * ROW_BYTES;
+        rec.edge = reinterpret_cast<const char *>(edge_table) + (size_t)my_eid * ROW_BYTES - ROW_BYTES;
+        rec.dt[0] = rec.dt[1] = my_dt;
+        rec.large = large;
+        rec.unused = 0;
+        if (lane >= first) s_rec[warp][lane - first] = rec;
+        if (lane == first)
+          for (int u = 0; u < GS - 1; ++u) s_rec[warp][range + u] = rec;
+        __syncwarp();
       }
-      const float *q_src = qt + (size_t)row * QT_LD;
-      float m = -INFINITY, sum = 0.f;     // running maximum / sum of this lane's head
-      unsigned todo = vmask;
+      const float *q_src = s_q[warp];
+      float m = -INFINITY;     // running maximum of this lane's head
       // GS slots at a time, each row of them in registers from its dot products to its weighted sum: nothing is
       // loaded twice, and the cross-lane sums of 2 * GS logits cost little more than those of one
       constexpr int V = 2 * GS, LPV = 32 / V;
-      for (int left = n_valid; left > 0; left -= GS) {
-        float4 x[GS][3];
+      for (int at = 0; at < range; at += GS) {
         float2 te[GS][GA_P_ITERS];
-        int js[GS];
+        float4 dts[GS];
 #pragma unroll
         for (int s = 0; s < GS; ++s) {
-          const int j = todo ? __ffs(todo) - 1 : -1;
-          js[s] = j;
-          todo &= todo - 1;
-          const int jj = j >= 0 ? j : js[0];      // (an empty place repeats the first slot with weight zero)
-          rows.load(__shfl_sync(FULL, my_nbr, jj), __shfl_sync(FULL, my_eid, jj), lane, x[s]);
+          const ulonglong2 p = *reinterpret_cast<const ulonglong2 *>(&s_rec[warp][at + s].nbr);
+          const char *nrow = reinterpret_cast<const char *>(p.x) + 16 * lane, *erow = reinterpret_cast<const char *>(p.y) + 16 * lane;
+          x[s][0] = ldg4(nrow);
+          x[s][1] = ldg4((from_edge ? erow : nrow) + 512);
+          if (third) x[s][2] = ldg4(erow + 1024);
+          dts[s] = *reinterpret_cast<const float4 *>(&s_rec[warp][at + s].dt);
         }
+        int any = 0;        // (of all slots of the step: one branch, and the usual case is straight code)
 #pragma unroll
-        for (int s = 0; s < GS; ++s) {
-          const int jj = js[s] >= 0 ? js[s] : js[0];
-          const float dt = __shfl_sync(FULL, my_dt, jj);
-          const int nl = __shfl_sync(FULL, my_nl, jj);
-          time_terms(dt, nl, wt, te[s]);
+        for (int s = 0; s < GS; ++s) any |= __float_as_int(dts[s].z);
+        if (any == 0) {
+#pragma unroll
+          for (int s = 0; s < GS; ++s)
+#pragma unroll
+            for (int i = 0; i < GA_P_ITERS; ++i) te[s][i] = cos_small2(mul2(make_float2(dts[s].x, dts[s].y), wt[i]));
+        } else {
+#pragma unroll
+          for (int s = 0; s < GS; ++s) time_terms(dts[s].x, __float_as_int(dts[s].z), wt, te[s]);
         }
         // partial logits: value 2 * s + head
         float2 a0[GS], a1[GS];
@@ -262,20 +303,22 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         for (int s = 0; s < GS; ++s) a0[s] = a1[s] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < GA_P_ITERS; ++i) {
+          // (a lane without a third piece multiplies zeros by what lies there; its third time pair is cos(0))
+          const float4 qa = *(reinterpret_cast<const float4 *>(q_src) + lane + 32 * i);
+          const float4 qb = *(reinterpret_cast<const float4 *>(q_src + QT_HEAD) + lane + 32 * i);
+          float2 qta = make_float2(0.f, 0.f), qtb = qta;
           if (i < 2 || third) {
-            const float4 qa = __ldg(reinterpret_cast<const float4 *>(q_src) + lane + 32 * i);
-            const float4 qb = __ldg(reinterpret_cast<const float4 *>(q_src + QT_HEAD) + lane + 32 * i);
-            const float2 qta = __ldg(reinterpret_cast<const float2 *>(q_src + 2 * D) + lane + 32 * i);
-            const float2 qtb = __ldg(reinterpret_cast<const float2 *>(q_src + QT_HEAD + 2 * D) + lane + 32 * i);
+            qta = *(reinterpret_cast<const float2 *>(q_src + 2 * D) + lane + 32 * i);
+            qtb = *(reinterpret_cast<const float2 *>(q_src + QT_HEAD + 2 * D) + lane + 32 * i);
+          }
 #pragma unroll
-            for (int s = 0; s < GS; ++s) {
-              a0[s] = fma2(te[s][i], qta, a0[s]);
-              a1[s] = fma2(te[s][i], qtb, a1[s]);
-              a0[s] = fma2(lo2(x[s][i]), lo2(qa), a0[s]);
-              a0[s] = fma2(hi2(x[s][i]), hi2(qa), a0[s]);
-              a1[s] = fma2(lo2(x[s][i]), lo2(qb), a1[s]);
-              a1[s] = fma2(hi2(x[s][i]), hi2(qb), a1[s]);
-            }
+          for (int s = 0; s < GS; ++s) {
+            a0[s] = fma2(te[s][i], qta, a0[s]);
+            a1[s] = fma2(te[s][i], qtb, a1[s]);
+            a0[s] = fma2(lo2(x[s][i]), lo2(qa), a0[s]);
+            a0[s] = fma2(hi2(x[s][i]), hi2(qa), a0[s]);
+            a1[s] = fma2(lo2(x[s][i]), lo2(qb), a1[s]);
+            a1[s] = fma2(hi2(x[s][i]), hi2(qb), a1[s]);
           }
         }
         float v[V];
@@ -283,35 +326,40 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         for (int s = 0; s < GS; ++s) v[2 * s] = a0[s].x + a0[s].y, v[2 * s + 1] = a1[s].x + a1[s].y;
         // lane l holds value l / LPV = 2 * slot + head; head = one lane bit
         float lg = warp_sum_many<V>(v, lane);
-        const int slot = lane / (2 * LPV);
-#pragma unroll
-        for (int s = 1; s < GS; ++s)
-          if (slot == s && js[s] < 0) lg = -INFINITY;
+        // the next row of this warp: its indices land while this one is finished
+        if (at == 0) draw_next();
+        if (!(valid >> (at + lane / (2 * LPV)) & 1u)) lg = -INFINITY;
         float top = lg;
 #pragma unroll
         for (int o = 2 * LPV; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
         const float m_new = fmaxf(m, top);
-        const float scale = expf(m - m_new);       // (0 the first time)
-        const float p = expf(lg - m_new);
-        float ps = p;
-#pragma unroll
-        for (int o = 2 * LPV; o < 32; o <<= 1) ps += __shfl_xor_sync(FULL, ps, o);
-        sum = sum * scale + ps;
+        // even lanes: the slot's weight; odd lanes: what the sums so far are scaled by (0 the first time)
+        const float p = expf((lane & 1 ? m : lg) - m_new);
         m = m_new;
-        const float2 S0 = dup2(__shfl_sync(FULL, scale, 0)), S1 = dup2(__shfl_sync(FULL, scale, LPV));
+        // [slot][head] weights, [head] scales, each twice (operands of the packed instructions)
+        const int where = lane & 1 ? 2 * GS + (lane / LPV & 1) : lane / LPV;
+        reinterpret_cast<float2 *>(pbuf)[where] = dup2(p);
+        __syncwarp();
+        const float4 S = *reinterpret_cast<const float4 *>(pbuf + 4 * GS);
+        sum0 *= S.x, sum1 *= S.z;
+        if (at > 0 && (S.x != 1.f || S.z != 1.f)) {
+          const float2 S0 = lo2(S), S1 = hi2(S);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          float2 r;
-          r = mul2(S0, lo2(am0[i])); am0[i].x = r.x; am0[i].y = r.y;
-          r = mul2(S0, hi2(am0[i])); am0[i].z = r.x; am0[i].w = r.y;
-          r = mul2(S1, lo2(am1[i])); am1[i].x = r.x; am1[i].y = r.y;
-          r = mul2(S1, hi2(am1[i])); am1[i].z = r.x; am1[i].w = r.y;
-          at0[i] = mul2(S0, at0[i]);
-          at1[i] = mul2(S1, at1[i]);
+          for (int i = 0; i < 3; ++i) {
+            float2 r;
+            r = mul2(S0, lo2(am0[i])); am0[i].x = r.x; am0[i].y = r.y;
+            r = mul2(S0, hi2(am0[i])); am0[i].z = r.x; am0[i].w = r.y;
+            r = mul2(S1, lo2(am1[i])); am1[i].x = r.x; am1[i].y = r.y;
+            r = mul2(S1, hi2(am1[i])); am1[i].z = r.x; am1[i].w = r.y;
+            at0[i] = mul2(S0, at0[i]);
+            at1[i] = mul2(S1, at1[i]);
+          }
         }
 #pragma unroll
         for (int s = 0; s < GS; ++s) {
-          const float2 P0 = dup2(__shfl_sync(FULL, p, 2 * s * LPV)), P1 = dup2(__shfl_sync(FULL, p, (2 * s + 1) * LPV));
+          const float4 P = *reinterpret_cast<const float4 *>(pbuf + 4 * s);
+          const float2 P0 = lo2(P), P1 = hi2(P);
+          sum0 += P.x, sum1 += P.z;
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             float2 r;
@@ -323,47 +371,67 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
             at1[i] = fma2(P1, te[s][i], at1[i]);
           }
         }
-        if (!drawn) {
-          // the next row of this warp: its indices land while this one is finished
-          drawn = true;
-          draw_next();
-        }
+        __syncwarp();
       }
-      inv0 = 1.f / __shfl_sync(FULL, sum, 0), inv1 = 1.f / __shfl_sync(FULL, sum, LPV);
       prof_rows += 1;
-      prof_slots += (unsigned long long)n_valid;
+      prof_slots += (unsigned long long)__popc(vmask);
+    } else {
+      draw_next();
     }
-    if (!drawn) draw_next();
+    __syncwarp();        // (the query has been read by all lanes: the next one may land)
+    if (next >= 0) fetch_query(next);
+    phase ^= 1;
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
-    if (IMAGE || n_valid > 0) {
+    const float inv0 = vmask ? 1.f / sum0 : 0.f, inv1 = vmask ? 1.f / sum1 : 0.f;
+    if (IMAGE) {
+      char *im = (char *)ctx + (size_t)(row / img::ROWS) * (img::CTX_STAGES * img::STAGE_BYTES) + (row % img::ROWS) * 64;
+      const int sw = (row << 3) & 0x30;
+      // (img::at, with the row's part taken out: the four pieces of a lane advance by whole stages)
+      auto place = [&](int c) { return im + (((c >> 5) * img::STAGE_BYTES + (c >> 3 & 3) * 16 + 2 * (c & 7)) ^ sw); };
+      char *o0 = place(4 * lane), *o1 = place(KEY + 4 * lane), *o2 = place(2 * D + 2 * lane), *o3 = place(KEY + 2 * D + 2 * lane);
+      auto put4 = [&](char *p, float4 v, float inv) {
+        const float2 a = mul2(dup2(inv), lo2(v)), b = mul2(dup2(inv), hi2(v));
+        uint2 hi, lo;
+        hi.x = tc::pack_split(a.x, a.y, lo.x);
+        hi.y = tc::pack_split(b.x, b.y, lo.y);
+        *reinterpret_cast<uint2 *>(p) = hi;
+        *reinterpret_cast<uint2 *>(p + img::STAGE_BYTES / 2) = lo;
+      };
+      auto put2 = [&](char *p, float2 v, float inv) {
+        const float2 a = mul2(dup2(inv), v);
+        uint32_t lo;
+        const uint32_t hi = tc::pack_split(a.x, a.y, lo);
+        *reinterpret_cast<uint32_t *>(p) = hi;
+        *reinterpret_cast<uint32_t *>(p + img::STAGE_BYTES / 2) = lo;
+      };
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (i < 2 || third) {
+          put4(o0 + i * 4 * img::STAGE_BYTES, am0[i], inv0);
+          put4(o1 + i * 4 * img::STAGE_BYTES, am1[i], inv1);
+          put2(o2 + i * 2 * img::STAGE_BYTES, at0[i], inv0);
+          put2(o3 + i * 2 * img::STAGE_BYTES, at1[i], inv1);
+        }
+      if (lane < (img::CTX_STAGES * img::STAGE_K - QT) / 4) {    // padding
+        char *p = place(QT + 4 * lane);
+        *reinterpret_cast<uint2 *>(p) = make_uint2(0, 0);
+        *reinterpret_cast<uint2 *>(p + img::STAGE_BYTES / 2) = make_uint2(0, 0);
+      }
+    } else if (vmask != 0) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const int f = lane + 32 * i;
         if (i < 2 || third) {
-          const float4 m0 = make_float4(am0[i].x * inv0, am0[i].y * inv0, am0[i].z * inv0, am0[i].w * inv0);
-          const float4 m1 = make_float4(am1[i].x * inv1, am1[i].y * inv1, am1[i].z * inv1, am1[i].w * inv1);
-          const float2 t0 = make_float2(at0[i].x * inv0, at0[i].y * inv0);
-          const float2 t1 = make_float2(at1[i].x * inv1, at1[i].y * inv1);
-          if (IMAGE) {
-            char *im = (char *)ctx;
-            img::put4<img::CTX_STAGES>(im, row, 4 * f, m0);
-            img::put4<img::CTX_STAGES>(im, row, KEY + 4 * f, m1);
-            img::put2<img::CTX_STAGES>(im, row, 2 * D + 2 * f, t0);
-            img::put2<img::CTX_STAGES>(im, row, KEY + 2 * D + 2 * f, t1);
-          } else {
-            float *out = (float *)ctx + (size_t)row * QT;
-            reinterpret_cast<float4 *>(out)[f] = m0;
-            reinterpret_cast<float4 *>(out + KEY)[f] = m1;
-            reinterpret_cast<float2 *>(out + 2 * D)[f] = t0;
-            reinterpret_cast<float2 *>(out + KEY + 2 * D)[f] = t1;
-          }
+          float *out = (float *)ctx + (size_t)row * QT;
+          reinterpret_cast<float4 *>(out)[f] = make_float4(am0[i].x * inv0, am0[i].y * inv0, am0[i].z * inv0, am0[i].w * inv0);
+          reinterpret_cast<float4 *>(out + KEY)[f] = make_float4(am1[i].x * inv1, am1[i].y * inv1, am1[i].z * inv1, am1[i].w * inv1);
+          reinterpret_cast<float2 *>(out + 2 * D)[f] = make_float2(at0[i].x * inv0, at0[i].y * inv0);
+          reinterpret_cast<float2 *>(out + KEY + 2 * D)[f] = make_float2(at1[i].x * inv1, at1[i].y * inv1);
         }
       }
     }
-    if (IMAGE && lane < (img::CTX_STAGES * img::STAGE_K - QT) / 4)    // padding
-      img::put4<img::CTX_STAGES>((char *)ctx, row, QT + 4 * lane, make_float4(0.f, 0.f, 0.f, 0.f));
-    if (lane == 0) valid_out[row] = n_valid > 0 ? 1 : 0;
+    if (lane == 0) valid_out[row] = vmask != 0 ? 1 : 0;
     row = next;
     my_nbr = nx_nbr;
     my_eid = nx_eid;
@@ -414,17 +482,19 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
   }
   // one resident wave at most; fewer blocks when the caller expects fewer rows than the capacity
   const int rows = rows_hint > 0 ? std::min(rows_hint, n_rows_cap) : n_rows_cap;
-  const int grid = std::min(ceil_div(rows, GA_THREADS / 32), c->sm_count * GA_BLOCKS);
-  auto kernel = image ? attn_gather_kernel<true> : attn_gather_kernel<false>;
+  const bool wide = k >= GA_WIDE_FROM;
+  const int grid = std::min(ceil_div(rows, GA_WARPS), c->sm_count * ga_blocks(wide ? 4 : 2));
+  auto kernel = image ? (wide ? attn_gather_kernel<true, 4> : attn_gather_kernel<true, 2>)
+                      : (wide ? attn_gather_kernel<false, 4> : attn_gather_kernel<false, 2>);
   // (the profiling events would sit between this kernel and its neighbours: plain launch then)
   if (pf.on)
     kernel<<<grid, GA_THREADS, 0, stream>>>(d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table, d_time_w, d_nbr, d_eid,
                                             d_delta, k, n_rows_cap, d_n_rows, d_order, d_ctx, d_valid, d_ticket,
-                                            pf.d_counters);
+                                            pf.d_counters, c->status_word, c->wait_limit);
   else
     ORCA_CUDA(launch_dep(kernel, grid, GA_THREADS, 0, stream, d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table,
                          d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_ctx, d_valid,
-                         d_ticket, (unsigned long long *)nullptr));
+                         d_ticket, (unsigned long long *)nullptr, c->status_word, c->wait_limit));
   if (pf.on) {
     ORCA_CUDA(cudaEventRecord(pf.ev[pf.used + 1], stream));
     pf.used += 2;

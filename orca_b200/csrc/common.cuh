@@ -104,27 +104,26 @@ __device__ __forceinline__ float warp_sum(float v) {
 // far outside the range where cosf() stays on its fast path, and its slow path (Payne-Hanek) costs a
 // hundred instructions; double-precision reduction is no way out either (the fp64 and conversion
 // pipes of this GPU made a warp-wide cosine cost ~160 cycles).  fp32 and integer pipes only:
-//   |x| < 2^24   Cody-Waite: k = rint(x / 2pi) (< 2^22), r = x - k*C1 - k*C2 - k*C3 with 2pi split so that the first
-//                two differences are exact (C1 8 bits, C2 11 bits); reduction error 2.4e-7 at most, 3.2e-8 rms.  x / 2pi
-//                is rounded before it is rounded to k, by up to a quarter at 2^24, so that k can be one off and |r| exceeds
-//                pi: 3.15 / 3.33 / 3.87 / 4.60 below 2^17 / 2^21 / 2^23 / 2^24;
+//   |x| < 2^24   Cody-Waite: k = rint(x / 2pi) (< 2^22) by adding and subtracting 1.5 * 2^23, r = x - k*C1 - k*C2 with C1 the
+//                nearest float to 2pi: its last bit is 2^-21, so x - k*C1 has at most 24 bits and is exact; reduction error
+//                1.3e-7 at most.  1/2pi is a float, too: k can be one off, and |r| reaches 3.15 / 3.23 / 3.48 / 3.82 below
+//                2^17 / 2^21 / 2^23 / 2^24;
 //   |x| < 2^30   fixed point: x = m * 2^e with a 24-bit m; the fraction of x / 2pi is the low part of
 //                m * F (F = 2^64 / 2pi) shifted by e, of which the top 32 bits are kept (96-bit product
 //                from two 32 x 32 multiplies); cos is even, so |fraction| (24 bits) goes back to a
 //                float through the 2^23 exponent trick; reduction error 3.8e-7 at most, 1.3e-7 rms;
 //   else         cosf().
 // The hardware cosine approximation is applied to the remainder.  CUDA states its error for [-pi, pi] only (2^-21.19);
-// measured against 64 bits over every float: 4.0e-7 at most up to pi, 2.2e-7 up to 3.5, 4.0e-7 up to 4, 5.3e-7 up to 4.7.
-// So what decides is the error of the whole, over every float of a binade: Cody-Waite 4.9e-7 at most below 2^23, 6.9e-7 up
-// to 2^24, 1.3e-7 rms; fixed point 7.1e-7 at most, 2.1e-7 rms, in each of these binades.
+// measured against 64 bits over every float: 4.0e-7 at most up to pi, 2.2e-7 up to 3.5, 4.0e-7 up to 4.
+// So what decides is the error of the whole, over every float of a binade: Cody-Waite 4.9e-7 at most and 1.3e-7 rms below
+// 2^24; fixed point 7.1e-7 at most, 2.1e-7 rms, up to 2^24.
 constexpr float COS_SMALL = 16777216.f;    // 2^24
 // |x| < COS_SMALL, branch free
 __device__ __forceinline__ float cos_small(float x) {
   const float ax = fabsf(x);
-  const float k = rintf(ax * 0.15915494309189535f);
-  float r = fmaf(-k, 6.28125f, ax);
-  r = fmaf(-k, 0.0019350051879882812f, r);
-  r = fmaf(-k, 3.019916050561733e-07f, r);
+  const float k = fmaf(ax, 0.15915494309189535f, 12582912.f) - 12582912.f;
+  float r = fmaf(-k, 6.2831855f, ax);
+  r = fmaf(k, 1.7484556e-07f, r);
   return __cosf(r);
 }
 // 2^-8 <= |x| < 2^30, branch free

@@ -265,6 +265,49 @@ def test_attention_layer(dev, k, n, layer):
             assert np.array_equal(pt[src_ids[r]], got[r])
 
 
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 9, 10, 11, 12, 13, 14, 31, 32])
+def test_attention_gather_slots(dev, k):
+    """The gather kernel against 64 bits where its steps of two (K to 10) and four slots end: rows of 0 to K slots at either
+    end of the table and with holes between them, time differences on all sides of the cosine's ranges.  Bounds: a logit is
+    a sum of 1.5 K products in chains of 18 and five levels (23 roundings of 2^-24) of cosines good to 7.8e-7; what it is off by
+    goes into a weight twice (exponential and normalisation), with 1e-6 for the exponential, the sums and the division."""
+    from orca_b200 import _lib
+    rs = np.random.RandomState(k)
+    n, n_tab = 37 * (k + 1), 300
+    tab, etab = (rs.randn(n_tab, D).astype(np.float32) for _ in range(2))
+    nbr, eid = rs.randint(1, n_tab, (2, n, k))
+    for r in range(n):
+        m = r % (k + 1)                      # slots of the row
+        keep = np.arange(k) >= k - m if r % 3 == 0 else np.arange(k) < m if r % 3 == 1 else rs.permutation(k) < m
+        nbr[r, ~keep] = 0
+    dt = (10.0 ** rs.uniform(0, 9.6, (n, k))).astype(np.float32)
+    dt[::5] = rs.rand(len(dt[::5]), k) * 1000
+    w = (1 / 10 ** np.linspace(0, 9, D)).astype(np.float32)
+    q = (rs.randn(n, 1056) * 0.1).astype(np.float32)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    d_q, d_tab, d_etab, d_w, d_nbr, d_eid, d_dt = up(q), up(tab), up(etab), up(w), _i32(nbr, dev), _i32(eid, dev), up(dt)
+    ctx = torch.full((n, 1032), 3.0, device=dev)
+    valid = torch.full((n,), 7, dtype=torch.uint8, device=dev)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    _lib.check(_lib.lib().orca_attn_gather(d_q.data_ptr(), d_tab.data_ptr(), d_etab.data_ptr(), d_w.data_ptr(), d_nbr.data_ptr(),
+                                           d_eid.data_ptr(), d_dt.data_ptr(), k, n, None, ctx.data_ptr(), valid.data_ptr(),
+                                           status.data_ptr(), _lib.stream_ptr(dev)))
+    got, on = ctx.cpu().numpy(), nbr != 0
+    assert np.array_equal(valid.cpu().numpy(), on.any(1)) and np.all(got[~on.any(1)] == 3.0)
+    te = np.cos((dt[:, :, None] * w).astype(np.float64))
+    x = np.concatenate([tab[nbr], etab[eid], te], 2).astype(np.float64)
+    for h in range(2):
+        qh = q[:, h * 528:h * 528 + 516].astype(np.float64)
+        logit = np.where(on, np.einsum("nkc,nc->nk", x, qh), -np.inf)
+        delta = np.where(on, 23 * 2.0 ** -24 * np.einsum("nkc,nc->nk", np.abs(x), np.abs(qh)), 0).max(1)
+        delta += 7.8e-7 * np.abs(qh[:, 2 * D:]).sum(1)
+        rows = on.any(1)
+        p = np.exp(logit[rows] - logit[rows].max(1, keepdims=True))
+        want = np.einsum("nk,nkc->nc", p / p.sum(1, keepdims=True), x[rows])
+        most = np.abs(np.where(on[rows][:, :, None], x[rows], 0)).max(1)
+        assert np.all(np.abs(got[rows, h * 516:(h + 1) * 516] - want) < (4 * delta[rows] + 1e-6)[:, None] * most + 7.8e-7)
+
+
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 // 6 + 1, 9000])
 def test_attention_query(dev, n):
     """The stand-alone query projection against 64 bits, rows past the device-side count untouched, an output that is
