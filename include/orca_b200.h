@@ -228,7 +228,8 @@ typedef struct {
   const float *ln_w; /* [172]        */
   const float *ln_b; /* [172]        */
   const float *G_tc, *W2t_tc;
-  const float *Mq_img, *G_img, *W2_img;   /* operands of the kernels that take their rows as images */
+  /* operands of the kernels that take their rows as images: [Mq | last 172 rows of G], the other rows of G, W2t */
+  const float *Mq_img, *G_img, *W2_img;
 } orca_attn_weights_t;
 
 /* Step 1 of TemporalAttentionLayer.forward (model/temporal_attention.py:41-48, the query side of

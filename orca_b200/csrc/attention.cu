@@ -163,8 +163,9 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
                    const float *__restrict__ edge_table, const float *__restrict__ time_w,
                    const int32_t *__restrict__ nbr, const int32_t *__restrict__ eid,
                    const float *__restrict__ delta, int k, int n_cap, const int32_t *__restrict__ d_n,
-                   const int32_t *__restrict__ order, void *__restrict__ ctx, uint8_t *__restrict__ valid_out,
-                   int32_t *__restrict__ ticket, unsigned long long *__restrict__ prof, int32_t *status, long long wait_limit) {
+                   const int32_t *__restrict__ order, const int32_t *__restrict__ q_row, void *__restrict__ ctx,
+                   uint8_t *__restrict__ valid_out, int32_t *__restrict__ ticket, unsigned long long *__restrict__ prof,
+                   int32_t *status, long long wait_limit) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ __align__(128) float s_q[GA_WARPS][QT_LD];
   __shared__ SlotRec s_rec[GA_WARPS][ORCA_MAX_K + GS - 1];
@@ -193,7 +194,8 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   // that the output kernel starts with.  200 MB of queries a launch do not fit it: 50 batches of 2000 5.80 -> 5.68 ms, 51 of
   // 600 3.00 -> 2.96, without reuse 2.36 -> 2.30.)
   auto row_of_ticket = [&](int t) -> int { return order != nullptr ? order[t] : n - 1 - t; };
-  auto load_indices = [&](int r, int &o_nbr, int &o_eid, float &o_dt) {
+  auto load_indices = [&](int r, int &o_nbr, int &o_eid, float &o_dt, int &o_q) {
+    o_q = q_row != nullptr ? q_row[r] : r;
     o_nbr = 0, o_eid = 0, o_dt = 0.f;
     if (lane < k) {
       const size_t o = (size_t)r * k + lane;
@@ -217,8 +219,9 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   int my_nbr = 0, my_eid = 0;
   float my_dt = 0.f;
   if (row >= 0) {
-    fetch_query(row);
-    load_indices(row, my_nbr, my_eid, my_dt);
+    int q;
+    load_indices(row, my_nbr, my_eid, my_dt, q);
+    fetch_query(q);
   }
   float4 x[GS][3];                                 // (the third piece of the lanes that have none stays zero)
 #pragma unroll
@@ -227,13 +230,13 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   while (row >= 0) {
     // the next ticket is drawn now and its row's indices are requested after the first slots (see above)
     if (lane == 0) tkt = atomicAdd(&ticket[0], 1);
-    int next = -1, nx_nbr = 0, nx_eid = 0;
+    int next = -1, nx_nbr = 0, nx_eid = 0, nx_q = 0;
     float nx_dt = 0.f;
     auto draw_next = [&]() {
       const int t = __shfl_sync(FULL, tkt, 0);
       if (t < n) {
         next = row_of_ticket(t);
-        load_indices(next, nx_nbr, nx_eid, nx_dt);
+        load_indices(next, nx_nbr, nx_eid, nx_dt, nx_q);
       }
     };
     const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
@@ -379,7 +382,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       draw_next();
     }
     __syncwarp();        // (the query has been read by all lanes: the next one may land)
-    if (next >= 0) fetch_query(next);
+    if (next >= 0) fetch_query(nx_q);
     phase ^= 1;
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
@@ -453,13 +456,14 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
 
 // d_nbr_table2 (optional): neighbour rows >= nbr_split are read from it; its address is already moved back by
 // nbr_split rows
+// d_q_row (optional): row r's query is row d_q_row[r] of d_qt
 // `ticket`: two zeroed device words that the launch leaves at zero; launches that may overlap on the GPU
 // need words of their own
 int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float *d_edge_table,
                        const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid, const float *d_delta,
                        int k, int n_rows_cap, const int32_t *d_n_rows, int rows_hint, const int32_t *d_order,
                        void *d_ctx, bool image, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream,
-                       const float *d_nbr_table2, int nbr_split) {
+                       const float *d_nbr_table2, int nbr_split, const int32_t *d_q_row) {
   if (d_nbr_table2 == nullptr) nbr_split = 0x7fffffff;
   ORCA_CHECK_ARG(d_qt && d_nbr_table && d_edge_table && d_time_w && d_nbr && d_eid && d_delta && d_ctx &&
                  d_valid && d_ticket);
@@ -489,11 +493,11 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
   // (the profiling events would sit between this kernel and its neighbours: plain launch then)
   if (pf.on)
     kernel<<<grid, GA_THREADS, 0, stream>>>(d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table, d_time_w, d_nbr, d_eid,
-                                            d_delta, k, n_rows_cap, d_n_rows, d_order, d_ctx, d_valid, d_ticket,
+                                            d_delta, k, n_rows_cap, d_n_rows, d_order, d_q_row, d_ctx, d_valid, d_ticket,
                                             pf.d_counters, c->status_word, c->wait_limit);
   else
     ORCA_CUDA(launch_dep(kernel, grid, GA_THREADS, 0, stream, d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table,
-                         d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_ctx, d_valid,
+                         d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_q_row, d_ctx, d_valid,
                          d_ticket, (unsigned long long *)nullptr, c->status_word, c->wait_limit));
   if (pf.on) {
     ORCA_CUDA(cudaEventRecord(pf.ev[pf.used + 1], stream));

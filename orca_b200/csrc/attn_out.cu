@@ -1,13 +1,14 @@
 // Output side of an attention layer on the tensor cores:
-//   out[r] = LayerNorm(relu([ctx | feat] . G + b1 + valid * g) . W2t + b2), optional history push and peer delivery
-//
+//   out[r] = LayerNorm(relu(ctx . G[:1032] + own + b1 + valid * g) . W2t + b2), optional history push and peer delivery
+// where own = feat . G[1032:] comes from the kernel that computes the queries from the same features (attn_query.cu): of rows
+// that share their features (a group's layer 1) it is computed once, and a block's chain here is six stages shorter.
 // The rows come as an operand image (attn_out.cuh): bf16 heads and tails, split once by the kernels that computed them,
 // in the form the tensor core reads.  So the main loop is nothing but bulk copies and MMAs: one thread streams stages
 // of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three (of five for the first product of a CTA's
 // first block, while the room of the hidden tile is still unused: a launch of few blocks waits for these loads), one
 // thread multiplies, eight warps do the two epilogues -- of one row block while the stages of the next are already
-// landing.  A block of 128 rows takes 39
-// stages of 6 MMAs (10.5 us of tensor time) and 1.5 MB from L2.  The general projection kernel, whose producer warps
+// landing.  A block of 128 rows takes 33 + 6
+// stages of 6 MMAs and 1.4 MB from L2.  The general projection kernel, whose producer warps
 // load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; 51 k
 // rows: 145 us with it, 82 to 86 here, where the bound is what L2 gives all SMs together, 7.3 TB/s, 58 % of it weights
 // (tensor pipe 42 %, DRAM 41 %): five slots instead of three gain nothing.  Pairs of CTAs with half of the weights each
@@ -28,14 +29,14 @@ namespace ao {
 constexpr int BM = img::ROWS, BN = 176;
 constexpr int STAGES = 3;
 constexpr int A_STAGE = img::STAGE_BYTES, W_LBO = BN * 16, W_STAGE = 2 * 4 * W_LBO, STAGE = A_STAGE + W_STAGE;
-constexpr int K_STAGES = img::CTX_STAGES + img::FEAT_STAGES;                     // 39
+constexpr int K_STAGES = img::CTX_STAGES;                                        // 33
 constexpr int K2_CHUNKS = BN / 8, K2_STAGES = (K2_CHUNKS + 3) / 4;               // 22, 6
 constexpr int A2_LBO = BM * 16 + 16, A2_BYTES = K2_CHUNKS * A2_LBO;
 constexpr int TILE_LD = 180;                       // floats per row of the output tile (conflict-free 16-byte stores)
 constexpr int FRONT = 90 * 1024;                   // hidden image, then output tile
 static_assert(2 * A2_BYTES <= FRONT && BM * TILE_LD * 4 <= FRONT && STAGE % 1024 == 0, "");
 constexpr int FIRST = 5;                           // stages of the first product of a CTA's first block
-static_assert((FIRST - STAGES) * STAGE <= FRONT && K_STAGES % FIRST == FIRST - 1, "");
+static_assert((FIRST - STAGES) * STAGE <= FRONT && K_STAGES % FIRST >= STAGES, "");
 constexpr int FIRST_USES = K_STAGES / FIRST + 1;   // of each of the first STAGES slots
 constexpr int SMEM = FRONT + STAGES * STAGE + 1024;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
@@ -101,15 +102,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       int it = 0;
       for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x) {
         const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
-        const char *feat = g.feat + (size_t)blk * img::FEAT_STAGES * A_STAGE;
         for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
           const int s = slot_of(it);
           const uint32_t at = place(s);
           mbar_wait(empty(s), (use_of(it) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
           if (st < K_STAGES) {
             mbar_expect_tx(full(s), STAGE);
-            bulk_g2s_hint(at, st < img::CTX_STAGES ? ctx + (size_t)st * A_STAGE : feat + (size_t)(st - img::CTX_STAGES) * A_STAGE,
-                          A_STAGE, full(s), once);
+            bulk_g2s_hint(at, ctx + (size_t)st * A_STAGE, A_STAGE, full(s), once);
             bulk_g2s(at + A_STAGE, w1 + (size_t)st * W_STAGE, W_STAGE, full(s));
           } else {
             mbar_expect_tx(full(s), W_STAGE);
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       for (int st = 0; st < K_STAGES; ++st, ++it) {
         const int s = slot_of(it);
         const uint32_t a = place(s), w = a + A_STAGE;
-        const bool half = st == img::CTX_STAGES - 1 || st == K_STAGES - 1;     // (the second step is nothing but padding)
+        const bool half = st == K_STAGES - 1;     // (the second step is nothing but padding)
         mbar_wait(full(s), use_of(it) & 1, g.status, 711, alive, g.wait_limit);
         tc_fence_after();
         if (elect_one()) {
@@ -194,12 +193,30 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
         push = g.push_win != nullptr ? g.push_win[m]
                : (m >= g.push_all_from || g.push_last_pos[push_id] == (unsigned long long)(g.push_base + m)) ? 1 : 0;
       }
-      // first: hidden = relu(acc + b1 + valid * g), split, A image of the second product
+      // what the row's own features add: asked for while the product is still running
+      float4 own[6][4];
+      {
+        const int m = m0 + min(row, m_rows - 1);
+        const float4 *src = reinterpret_cast<const float4 *>(g.own + (size_t)(g.own_row != nullptr ? g.own_row[m] : m) * OWN_LD) + 4 * ch0;
+#pragma unroll
+        for (int ch = 0; ch < 6; ++ch)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) own[ch][q] = ch < ch1 - ch0 ? __ldg(src + 4 * ch + q) : f4z;
+      }
+      // first: hidden = relu(acc + own + b1 + valid * g), split, A image of the second product
       mbar_wait(acc1, t & 1, g.status, 720, alive, g.wait_limit);
       tc_fence_after();
-      for (int ch = ch0; ch < ch1; ++ch) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        const int ch = ch0 + c;
+        if (ch >= ch1) break;
         float v[16];
         tmem_ld16_sum(trow + ch * 16, SMALL, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          v[4 * q] += own[c][q].x, v[4 * q + 1] += own[c][q].y;
+          v[4 * q + 2] += own[c][q].z, v[4 * q + 3] += own[c][q].w;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = relu(v[i] + s_b1[ch * 16 + i] + on * s_g[ch * 16 + i]);
 #pragma unroll
@@ -312,7 +329,7 @@ int attn_output_rows(const OutArgs &args, cudaStream_t s) {
   if (args.n_cap <= 0) return ORCA_OK;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_output_rows: no context for the current device");
-  ORCA_CHECK_ARG(args.w.G_img && args.w.W2_img && args.ctx && args.feat && args.out);
+  ORCA_CHECK_ARG(args.w.G_img && args.w.W2_img && args.ctx && args.own && args.out);
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
     ORCA_CUDA(cudaFuncSetAttribute(ao::attn_output_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ao::SMEM));

@@ -12,8 +12,8 @@ namespace img {
 // by the kernels that compute them, in the form the tensor core reads from shared memory: blocks of 128 rows, K in
 // stages of 32 columns, a stage = [128 rows x 64 bytes of heads | the same of tails] with the 16-byte chunks of a row
 // swizzled by bits 1 and 2 of the row (64-byte swizzle), so that a stage is one contiguous copy and a row's piece of
-// it one 64-byte write.  Two images per layer: the rows' own features (172 columns, padded to 192; also the operand of
-// the query product) and the attention sums (1032 columns, padded to 1056).  Padding is zero.
+// it one 64-byte write.  Two images per layer: the rows' own features (172 columns, padded to 192; attn_query.cu) and the
+// attention sums (1032 columns, padded to 1056; attn_out.cu).  Padding is zero.
 constexpr int ROWS = 128;
 constexpr int STAGE_K = 32;
 constexpr int STAGE_BYTES = 2 * ROWS * STAGE_K * 2;
@@ -52,7 +52,9 @@ __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {   // K-major, 64-
 
 struct OutArgs {
   orca_attn_weights_t w;
-  const char *ctx, *feat;     // operand images of the rows
+  const char *ctx;            // operand image of the rows' attention sums
+  const float *own;           // [., OWN_LD] what the rows' own features add to the hidden layer (attn_query.cu)
+  const int32_t *own_row;     // row m's place in it (nullptr: m)
   const uint8_t *valid;       // rows whose slots are all padding have no attention term
   int n_cap;
   const int32_t *d_n;
@@ -73,9 +75,9 @@ struct OutArgs {
 };
 // operand image of rows of a (two-part) table
 int feat_image(const tc::RowSrc &feat, int n_cap, const int32_t *d_n, char *d_image, cudaStream_t s);
-// qt = feat . Mq + cq, from the rows' image
+// qt = feat . Mq + cq and (optional) own = feat . G[1032:], [., OWN_LD], from the rows' image
 int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_cap, const int32_t *d_n, float *d_qt,
-                     cudaStream_t s);
+                     float *d_own, cudaStream_t s);
 int attn_output_rows(const OutArgs &g, cudaStream_t s);
 
 }  // namespace orca

@@ -1,13 +1,15 @@
-// Query side of an attention layer on the tensor cores: qt[r] = feat[row of r] . Mq + cq, [rows, 1056] floats.
+// What an attention layer makes of its rows' own features, on the tensor cores: qt[r] = feat[row of r] . Mq + cq, [rows, 1056]
+// floats, and own[r] = feat[row of r] . G[1032:], [rows, 192], the features' part of the merger's hidden layer (attn_out.cu
+// adds it).
 //
-// A launch writes 4.2 KB per row and reads 0.7 six times over (once per weight tile).  A CTA keeps its weight
-// tile (heads and tails of 176 columns) for the whole launch and walks row blocks of 128, which come as an operand image
+// A launch writes 5 KB per row and reads 0.7 six times over (once per weight tile).  A CTA keeps its weight
+// tile (heads and tails of 208 columns) for the whole launch and walks row blocks of 128, which come as an operand image
 // (attn_out.cuh): one thread streams 16 KB stages through a ring, one multiplies, eight warps carry the accumulators from
-// tensor memory to qt.  51 k rows: 145 us for the general projection kernel (weights streamed again for every row block,
-// load, product and store one after the other), 75 with a thread per row and 32 bytes a store, which kept the path of the
-// stores through L1 70 % busy (a warp's store touched 32 lines), 70 with whole lines out of shared memory.  Now it is
-// what reads and writes take between SMs and L2 (410 MB, 6 TB/s) and the one accumulator buffer, which must be read before
-// the next block's products start.
+// tensor memory to the outputs, in whole lines through shared memory.  6 / 31 / 66 k rows: 16 / 55 / 106 us (qt alone,
+// tiles of 176 columns: 14 / 50 / 92).  A group's layer 1, where 0.18 to 0.48 of the rows are distinct, asks for those
+// only (66 k rows of the largest graph: 92 -> 51 us, 57 k of 600-edge batches 75 -> 20), and the output kernel leaves six of
+// its 39 stages out.  What bounds it: 4.8 us a block and CTA against 1.8 of products; without the stores 92 us, without the
+// reading of the accumulators 102, with rows from L2 100.
 // orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
 // for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
 #include <algorithm>
@@ -22,9 +24,10 @@ namespace aqi {
 
 constexpr int BM = 128;
 constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;                // K = 172, padded to 176
-constexpr int BN = 176, TILES = QT_LD / BN;                   // 6
+constexpr int BN = 208, TILES = (QT_LD + D + BN - 1) / BN;   // 6
+static_assert(TILES * BN >= QT_LD + D && QT_LD % 32 == 0 && OWN_LD % 32 == 0, "whole lines belong to one of the two outputs");
 constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
-constexpr int STAGES = 4, STAGE = img::STAGE_BYTES;
+constexpr int STAGES = 3, STAGE = img::STAGE_BYTES;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
 constexpr int BOX = 32 * 128;                                 // of a warp: 32 rows x 32 columns on their way out
 constexpr int RING = (2 * W_BYTES + 1023) / 1024 * 1024;      // (the swizzle wants aligned stages)
@@ -37,7 +40,7 @@ struct Args {
   const int32_t *d_n;
   const void *w;
   const float *bias;
-  float *qt;
+  float *qt, *own;
   int32_t *status;
   long long wait_limit;
 };
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (tid >= 64 && tid < 64 + BN) s_bias[tid - 64] = g.bias[nt * BN + tid - 64];
+  if (tid >= 64 && tid < 64 + BN) s_bias[tid - 64] = nt * BN + tid - 64 < QT_LD ? g.bias[nt * BN + tid - 64] : 0.f;
   dep_wait();
   const int M = rows_of(g.n_cap, g.d_n);
   tc_fence_before();
@@ -128,43 +131,51 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
       }
     }
   } else {
-    // (six chunks of 16 columns for the first four warps, five for the others)
-    const int quarter = warp & 3, half = (warp - 2) >> 2;
-    const int c0 = half * 6, nc = half ? 5 : 6;
+    // A tile has 13 chunks of 16 columns, so every other one starts in the middle of a 128-byte line.  The warps' parts are six
+    // chunks from a line's start (even tiles: 0 and 6, odd ones: 1 and 7) and, for the first (odd) or last (even) four warps,
+    // the half line that is left.
+    const int quarter = warp & 3, half = (warp - 2) >> 2, odd = nt & 1;
+    const int c0 = half * 6 + odd, single = odd ? 0 : 12;
+    const bool seven = half != odd;
     const uint32_t box = ring + STAGES * STAGE + (warp - 2) * BOX;
     int t = 0;
     for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
       const int m0 = blk * BM + quarter * 32;
       mbar_wait(accfull, t & 1, g.status, 560, alive, g.wait_limit);
       tc_fence_after();
-      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + c0 * 16;
-      float *out = g.qt + (size_t)m0 * QT_LD + nt * BN + c0 * 16;
-      float v[6][16];
+      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
+      float v[7][16];
 #pragma unroll
-      for (int ch = 0; ch < 6; ++ch)
-        if (ch < nc) tmem_ld16_sum(acc + ch * 16, SMALL, v[ch]);
+      for (int ch = 0; ch < 7; ++ch)
+        if (ch < 6 || seven) tmem_ld16_sum(acc + (ch < 6 ? c0 + ch : single) * 16, SMALL, v[ch]);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(accfree);      // (the next block's products may start before this one is stored)
       // 32 columns at a time through shared memory (16-byte pieces of a row exchanged by its number's low bits: no bank
       // conflicts either way), out in whole lines of a row
 #pragma unroll
-      for (int b = 0; b < 3; ++b) {
+      for (int b = 0; b < 4; ++b) {
+        if (b == 3 && !seven) break;
+        const int at = b < 3 ? (c0 + 2 * b) * 16 : single * 16;      // first column of the box in the tile
 #pragma unroll
         for (int p = 0; p < 8; ++p) {
           const int ch = 2 * b + (p >> 2), c = 4 * (p & 3);
-          if (ch >= nc) continue;
-          const float4 y = *reinterpret_cast<const float4 *>(s_bias + (c0 + ch) * 16 + c);
+          if (ch >= 7) continue;
+          const float4 y = *reinterpret_cast<const float4 *>(s_bias + at + 16 * (p >> 2) + c);
           st_shared_f4(box + lane * 128 + ((p ^ (lane & 7)) << 4),
                        make_float4(v[ch][c] + y.x, v[ch][c + 1] + y.y, v[ch][c + 2] + y.z, v[ch][c + 3] + y.w));
         }
         __syncwarp();
-        const bool whole = 2 * b + 1 < nc;      // (the last box of the others is half empty)
+        const int p = b < 3 ? lane & 7 : lane & 3, col = nt * BN + at + 4 * p;
+        const bool query = col < QT_LD;
+        float *out = query ? g.qt + col : g.own + (col - QT_LD);
+        const int ld = query ? QT_LD : OWN_LD;
+        const bool on = query || (g.own != nullptr && col < QT_LD + OWN_LD);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = whole ? 4 * i + (lane >> 3) : 8 * i + (lane >> 2), p = whole ? lane & 7 : lane & 3;
-          if ((whole || i < 4) && m0 + r < M)
-            *reinterpret_cast<float4 *>(out + (size_t)r * QT_LD + 32 * b + 4 * p) = ld_shared_f4(box + r * 128 + ((p ^ (r & 7)) << 4));
+        for (int i = 0; i < (b < 3 ? 8 : 4); ++i) {
+          const int r = b < 3 ? 4 * i + (lane >> 3) : 8 * i + (lane >> 2);
+          if (on && m0 + r < M)
+            *reinterpret_cast<float4 *>(out + (size_t)(m0 + r) * ld) = ld_shared_f4(box + r * 128 + ((p ^ (r & 7)) << 4));
         }
         __syncwarp();
       }
@@ -216,17 +227,17 @@ int feat_image(const tc::RowSrc &feat, int n_cap, const int32_t *d_n, char *d_im
 }
 
 int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_cap, const int32_t *d_n, float *d_qt,
-                     cudaStream_t s) {
+                     float *d_own, cudaStream_t s) {
   if (n_cap <= 0) return ORCA_OK;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_query_image: no context for the current device");
-  ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && ((uintptr_t)d_qt & 15) == 0);
+  ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && (((uintptr_t)d_qt | (uintptr_t)d_own) & 15) == 0);
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
     ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
     configured_device = c->device;
   }
-  const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, c->status_word, c->wait_limit};
+  const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, d_own, c->status_word, c->wait_limit};
   const dim3 grid(aqi::TILES, std::min(ceil_div(n_cap, aqi::BM), std::max(1, c->sm_count / aqi::TILES)));
   ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
   ORCA_COUNT_LAUNCH();

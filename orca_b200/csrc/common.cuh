@@ -15,6 +15,7 @@ constexpr int KEY = ORCA_KEY_DIM;    // 516
 constexpr int QT = ORCA_QT_DIM;      // 1032
 constexpr int QT_LD = ORCA_QT_LD;    // 1056: head h of a projected query starts at h * 528
 constexpr int QT_HEAD = QT_LD / H;   // 528
+constexpr int OWN_LD = 192;          // floats a row of the own features' part of the merger's hidden layer (172 used; whole lines)
 constexpr int MSG = ORCA_MSG_DIM;    // 688
 constexpr int ROW_BYTES = D * 4;     // 688
 

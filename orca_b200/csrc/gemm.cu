@@ -507,7 +507,7 @@ int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int
     void *image = scratch_alloc(c, img::bytes(n_rows_cap, img::FEAT_STAGES), s);
     if (image != nullptr) {
       int rc = feat_image(tc::RowSrc{d_feat, d_idx, D, 0, 0}, n_rows_cap, d_n_rows, (char *)image, s);
-      if (rc == ORCA_OK) rc = attn_query_image(w, (const char *)image, n_rows_cap, d_n_rows, d_qt, s);
+      if (rc == ORCA_OK) rc = attn_query_image(w, (const char *)image, n_rows_cap, d_n_rows, d_qt, nullptr, s);
       ORCA_CUDA(cudaFreeAsync(image, s));
       return rc;
     }

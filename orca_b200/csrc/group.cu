@@ -267,21 +267,39 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   const int batch_rows = 3 * a.edges(), n_slots = a.cnt->n_rows * a.k;
   for (int i = tid; i < n_slots; i += step) {
-    const int row = i / a.k, j = i - row * a.k;
-    int n, node;
+    const int row = i / a.k;
+    int n;
     if (row < batch_rows) {
       n = row / (3 * a.bs);
-      node = j == 0 ? a.img[a.off[n] + row - n * 3 * a.bs] : 0;
     } else {
       const int p = row - batch_rows;
       n = a.mode == ORCA_MODE_NO_REUSE ? p / a.k / (3 * a.bs) : batch_of_app(a, p);
-      node = j == 0 ? a.app_node[p] : 0;
     }
     const int v = a.nbr1[i];
     if (row < batch_rows && a.layers == 2)
       a.nbr2[i] = v == 0 ? 0 : a.mode == ORCA_MODE_NO_REUSE ? (int)a.n_nodes + batch_rows + i : history_row(a, v, n);
     if (v != 0) a.nbr1[i] = memory_row(a, v, n);
-    if (j == 0) a.own1[row] = node > 0 && node < a.n_nodes ? memory_row(a, node, n) : 0;
+  }
+  // The rows' own nodes.  Rows that share their own features share what layer 1 makes of them (the query, the merger's
+  // part): 0.18 to 0.48 of a group's rows are distinct (hub nodes fill a batch, and most nodes have not changed since the
+  // batch before).  A thread a row: one atomic a warp on the list's counter.
+  for (int row = tid; row < a.cnt->n_rows; row += step) {
+    int n, node;
+    if (row < batch_rows) {
+      n = row / (3 * a.bs);
+      node = a.img[a.off[n] + row - n * 3 * a.bs];
+    } else {
+      const int p = row - batch_rows;
+      n = a.mode == ORCA_MODE_NO_REUSE ? p / a.k / (3 * a.bs) : batch_of_app(a, p);
+      node = a.app_node[p];
+    }
+    const int own = node > 0 && node < a.n_nodes ? memory_row(a, node, n) : 0;
+    a.own1[row] = own;
+    if (__ldcg(&a.own_seen[own]) == 0 && atomicCAS(&a.own_seen[own], 0, -1) == 0) {
+      const int l = place(&a.cnt->n_own, 0);
+      a.own_list[l] = own;
+      a.own_seen[own] = l + 1;
+    }
   }
   const int per = 2 * a.bs;
   for (int i = tid; i < a.nb * per; i += step) {
@@ -302,6 +320,14 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
       a.score1[i] = 3 * n * a.bs + b + r;
     }
   }
+}
+
+// the layer-1 rows' places in own_list
+__global__ void __launch_bounds__(256) own_kernel(const __grid_constant__ Args a) {
+  dep_trigger();
+  dep_wait();
+  const int n = a.cnt->n_rows;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a.own_at[i] = a.own_seen[a.own1[i]] - 1;
 }
 
 // ------------------------------------------------------------------------------------------------ last versions
@@ -444,7 +470,7 @@ struct Parity {
   unsigned long long *app_table;
   Counters *cnt;
   size_t zero_bytes;       // bits, tables and counters are zeroed together, from `bits`
-  int32_t *cand, *app_node, *nbr1, *eid1, *nbr2, *own1, *score0, *score1;
+  int32_t *cand, *app_node, *nbr1, *eid1, *nbr2, *own1, *own_seen, *own_list, *own_at, *score0, *score1;
   float *dt1;
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;
@@ -455,7 +481,7 @@ struct Parity {
 struct Buffers {
   Parity par[2];
   float *log;              // two parities, one after the other
-  float *qt, *emb1, *emb2;
+  float *qt, *own, *emb1, *emb2;
   char *ctx, *feat, *feat2;   // operand images (attn_out.cuh): attention sums, own features, layer 2's own features
   uint8_t *valid;
   uint32_t table_size, app_size;
@@ -482,6 +508,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.bits = (NodeBits *)take((size_t)n_nodes * sizeof(NodeBits));
     x.table = (Entry *)take((size_t)w.table_size * sizeof(Entry));
     x.app_table = (unsigned long long *)take((size_t)w.app_size * 8);
+    x.own_seen = (int32_t *)take((size_t)(n_nodes + 4 * E) * 4);
     x.cnt = (Counters *)take(sizeof(Counters));
     x.zero_bytes = off - first;
     x.cand = (int32_t *)take(budget ? (size_t)apps * 4 : 4);
@@ -491,6 +518,8 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.dt1 = (float *)take((size_t)w.rows_max * k * 4);
     x.nbr2 = (int32_t *)take((size_t)batch_rows * k * 4);
     x.own1 = (int32_t *)take((size_t)w.rows_max * 4);
+    x.own_list = (int32_t *)take((size_t)w.rows_max * 4);
+    x.own_at = (int32_t *)take((size_t)w.rows_max * 4);
     x.score0 = (int32_t *)take((size_t)2 * E * 4);
     x.score1 = (int32_t *)take((size_t)2 * E * 4);
     x.win_node = (int32_t *)take((size_t)2 * E * 4);
@@ -506,6 +535,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
   }
   w.log = (float *)take((size_t)2 * 2 * E * D * 4);
   w.qt = (float *)take((size_t)w.chunk * QT_LD * 4);
+  w.own = (float *)take((size_t)w.chunk * OWN_LD * 4);
   w.ctx = (char *)take(img::bytes(w.chunk, img::CTX_STAGES));
   w.feat = (char *)take(img::bytes(w.chunk, img::FEAT_STAGES));
   w.feat2 = (char *)take(layers == 2 ? img::bytes(batch_rows, img::FEAT_STAGES) : 4);
@@ -536,7 +566,8 @@ static int launch_index(const Args &a, const float *last_update, size_t zero_byt
     ORCA_COUNT_LAUNCH();
   }
   ORCA_CUDA(launch_dep(resolve_kernel, grid_slots, 256, 0, s, a, last_update));
-  for (int i = 0; i < 4; ++i) ORCA_COUNT_LAUNCH();
+  ORCA_CUDA(launch_dep(own_kernel, std::min(ceil_div(rows, 256), sms * 8), 256, 0, s, a));
+  for (int i = 0; i < 5; ++i) ORCA_COUNT_LAUNCH();
   return ORCA_OK;
 }
 
@@ -619,7 +650,8 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   a.table_mask = w.table_size - 1, a.app_mask = w.app_size - 1;
   if (g->seq > 0) a.prev_bits = prev.bits, a.prev_table = prev.table, a.prev_mask = w.table_size - 1;
   a.cand = x.cand, a.app_node = x.app_node, a.nbr1 = x.nbr1, a.eid1 = x.eid1, a.dt1 = x.dt1, a.nbr2 = x.nbr2;
-  a.own1 = x.own1, a.score0 = x.score0, a.score1 = x.score1;
+  a.own1 = x.own1, a.own_seen = x.own_seen, a.own_list = x.own_list, a.own_at = x.own_at;
+  a.score0 = x.score0, a.score1 = x.score1;
   a.win_node = x.win_node, a.win_eid = x.win_eid, a.win_mem = x.win_mem, a.win_other = x.win_other, a.win_t = x.win_t, a.win_gap = x.win_gap;
   a.last_at = x.last_at, a.last_node = x.last_node;
   a.split = 2 * E > grp::SPLIT_FROM;
@@ -675,32 +707,34 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
       ORCA_CUDA(cudaStreamWaitEvent(s, c->ev_gidx[p], 0));
     }
     int32_t *tk = c->d_words + CTX_TICKET_MAIN;
-    auto output = [&](int layer, int rows, float *out) {
+    auto output = [&](int layer, int rows, const int32_t *own_row, float *out) {
       OutArgs o{};
-      o.w = m->attn[layer], o.ctx = w.ctx, o.feat = layer == 0 ? w.feat : w.feat2, o.valid = w.valid, o.n_cap = rows;
-      o.out = out;
+      o.w = m->attn[layer], o.ctx = w.ctx, o.own = w.own, o.own_row = own_row, o.valid = w.valid, o.n_cap = rows, o.out = out;
       return o;
     };
+    // (a group with a cold cache, whose rows take several chunks, goes without sharing)
+    const bool shared = n_rows <= w.chunk;
     for (int r0 = 0; r0 < n_rows; r0 += w.chunk) {
       const int rows = std::min(w.chunk, n_rows - r0);
       const size_t slot = (size_t)r0 * k;
-      const tc::RowSrc own{m->mem.memory, x.own1 + r0, D, 0, 0, log, (int)m->n_nodes};
-      ORCA_TRY(feat_image(own, rows, nullptr, w.feat, s));
-      ORCA_TRY(attn_query_image(&m->attn[0], w.feat, rows, nullptr, w.qt, s));
+      const tc::RowSrc own{m->mem.memory, shared ? x.own_list : x.own1 + r0, D, 0, 0, log, (int)m->n_nodes};
+      const int32_t *d_own = shared ? &x.cnt->n_own : nullptr, *own_at = shared ? x.own_at : nullptr;
+      ORCA_TRY(feat_image(own, rows, d_own, w.feat, s));
+      ORCA_TRY(attn_query_image(&m->attn[0], w.feat, rows, d_own, w.qt, w.own, s));
       ORCA_TRY(launch_attn_gather(w.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1 + slot, x.eid1 + slot, x.dt1 + slot, k,
-                                  rows, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, log, (int)m->n_nodes));
-      OutArgs o = output(0, rows, w.emb1 + (size_t)r0 * D);
+                                  rows, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, log, (int)m->n_nodes, own_at));
+      OutArgs o = output(0, rows, own_at, w.emb1 + (size_t)r0 * D);
       // (the batch rows are layer 2's rows; they all lie in the first chunk)
       if (layers == 2 && r0 == 0) o.out_image = w.feat2, o.out_image_rows = 3 * E;
       ORCA_TRY(attn_output_rows(o, s));
     }
     const float *top = w.emb1;
     if (layers == 2) {
-      ORCA_TRY(attn_query_image(&m->attn[1], w.feat2, 3 * E, nullptr, w.qt, s));
+      ORCA_TRY(attn_query_image(&m->attn[1], w.feat2, 3 * E, nullptr, w.qt, w.own, s));
       // (without reuse every row lies in the layer-1 output: the first part is never read)
       ORCA_TRY(launch_attn_gather(w.qt, history ? m->hist_emb : m->mem.memory, m->edge_table, m->time_w, x.nbr2, x.eid1,
                                   x.dt1, k, 3 * E, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, emb, (int)m->n_nodes));
-      ORCA_TRY(attn_output_rows(output(1, 3 * E, w.emb2), s));
+      ORCA_TRY(attn_output_rows(output(1, 3 * E, nullptr, w.emb2), s));
       top = w.emb2;
     }
     // (positions of a short last batch's scores: the arrays are indexed by 2 * bs per batch, only the last is short)

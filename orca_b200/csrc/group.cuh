@@ -30,6 +30,7 @@ struct Counters {
   // launch behind the chain (Args::split) at the back.
   int32_t n_win[MAX_BATCHES], n_back[MAX_BATCHES];
   int32_t n_last;                          // entries of last_at
+  int32_t n_own;                           // entries of own_list
   int32_t dropped[MAX_BATCHES];            // smallest candidate of the batch (-1: none): it is not recomputed
   int32_t app_off[MAX_BATCHES + 1];        // first recomputed row of the batch, counted from the group's first
   int32_t n_rows;                          // layer-1 rows of the group
@@ -67,6 +68,8 @@ struct Args {
   float *dt1;
   int32_t *nbr2;                    // batch rows: rows of (history table | layer-1 output)
   int32_t *own1;                    // row of (memory table | log) of the row's own node
+  int32_t *own_seen;                // by row of (memory table | log): 1 + its place in own_list, 0: not there
+  int32_t *own_list, *own_at;       // the distinct rows of own1, and own1's places in the list
   int32_t *score0, *score1;         // the two embeddings of every score
   // memory updates: batch n's at n * 2 * bs (Counters says which of these places are taken)
   int32_t *win_node, *win_eid, *win_mem, *win_other;

@@ -54,6 +54,7 @@ struct IdxBuf {
 struct LaneBuf {
   float *qt, *hidden;
   char *ctx, *feat;    // operand images of the attention sums and of the rows' own features (attn_out.cuh)
+  float *own;          // what the own features add to the merger's hidden layer
   uint8_t *valid;
 };
 struct Workspace {
@@ -111,6 +112,7 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
     w.lane[q].qt = (float *)take(rows * QT_LD * 4);
     w.lane[q].ctx = (char *)take(img::bytes(rows, img::CTX_STAGES));   // (no smaller than [rows, 1032] floats)
     w.lane[q].feat = (char *)take(img::bytes(rows, img::FEAT_STAGES));
+    w.lane[q].own = (float *)take(rows * OWN_LD * 4);
     w.lane[q].hidden = (float *)take(rows * D * 4);
     w.lane[q].valid = (uint8_t *)take(rows);
   }
@@ -365,7 +367,7 @@ static int layer_query(const orca_attn_weights_t *w, const float *d_feat, const 
       const int rc = feat_image(tc::RowSrc{d_feat, d_idx, D, 0, 0}, cap, d_n, l.feat, s);
       if (rc) return rc;
     }
-    return attn_query_image(w, l.feat, cap, d_n, l.qt, s);
+    return attn_query_image(w, l.feat, cap, d_n, l.qt, l.own, s);
   }
   return orca_attn_query(w, d_feat, d_idx, cap, d_n, l.qt, s);
 }
@@ -390,7 +392,7 @@ static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d
     return attn_output_impl(w, (const float *)l.ctx, l.valid, d_feat, d_idx, cap, d_n, d_out, push.table, push.ids,
                             push.win, push.last_pos, push.base, push.all_from, l.hidden, s);
   OutArgs a{};
-  a.w = *w, a.ctx = l.ctx, a.feat = l.feat, a.valid = l.valid, a.n_cap = cap, a.d_n = d_n, a.out = d_out;
+  a.w = *w, a.ctx = l.ctx, a.own = l.own, a.valid = l.valid, a.n_cap = cap, a.d_n = d_n, a.out = d_out;
   a.push_table = push.table, a.push_ids = push.ids, a.push_win = push.last_pos != nullptr ? nullptr : push.win;
   a.push_last_pos = reinterpret_cast<const unsigned long long *>(push.last_pos);
   a.push_base = push.base, a.push_all_from = push.all_from;

@@ -25,6 +25,7 @@ HEADS = 2
 QT_HEAD = 528     # column stride of one head of the projected query (516 used)
 TC_BN, TC_BK = 176, 64
 GRU_PART, CHAIN_N = 176, 32
+QUERY_BN = 208    # columns of a weight tile of csrc/attn_query.cu
 
 
 def _packed(W, shape, image):
@@ -60,18 +61,16 @@ def pack_tc(W, bn=None):
 
 
 def pack_query(W):
-    """Query weights [172, 1056] for csrc/attn_query.cu: K padded to 176, one image per 176 columns, each
-    [head | tail][K / 8][176 columns][8]: uint16 [6, 2, 22, 176, 8]."""
-    return _packed(W, (GRU_PART, W.shape[1]),
-                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, TC_BN).permute(3, 0, 1, 4, 2))
+    """Weights [172, n] of the rows' own features for csrc/attn_query.cu: K padded to 176, one image per 208 columns, each
+    [head | tail][K / 8][208 columns][8]: uint16 [tiles, 2, 22, 208, 8]."""
+    return _packed(W, (GRU_PART, -(-W.shape[1] // QUERY_BN) * QUERY_BN),
+                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, QUERY_BN).permute(3, 0, 1, 4, 2))
 
 
-def pack_stages(*parts):
-    """Weights with 172 columns for csrc/attn_out.cu: the parts one below the other, each padded to a multiple of 32
-    rows; one stage per 32 rows, each [head | tail][4 chunks][176 columns][8]."""
-    at = np.cumsum([0] + [-(-len(p) // 32) * 32 for p in parts])
-    return _packed(list(zip(parts, at[:-1])), (int(at[-1]), TC_BN),
-                   lambda X: X.reshape(2, -1, 4, 8, TC_BN).permute(1, 0, 2, 4, 3))
+def pack_stages(W):
+    """Weights with 172 columns for csrc/attn_out.cu, padded to a multiple of 32 rows; one stage per 32 rows, each
+    [head | tail][4 chunks][176 columns][8]."""
+    return _packed(W, (-(-len(W) // 32) * 32, TC_BN), lambda X: X.reshape(2, -1, 4, 8, TC_BN).permute(1, 0, 2, 4, 3))
 
 
 def pack_gru(Wg, dim=D):
@@ -90,8 +89,10 @@ def pack_gru(Wg, dim=D):
 def packed_attention(w):
     """The operand images that go with prepare_attention's matrices (numpy arrays or tensors)."""
     kd2 = w["G"].shape[0] - w["Mq"].shape[0]
-    return {"G_tc": pack_tc(w["G"]), "W2t_tc": pack_tc(w["W2t"]), "Mq_img": pack_query(w["Mq"]),
-            "G_img": pack_stages(w["G"][:kd2], w["G"][kd2:]), "W2_img": pack_stages(w["W2t"])}
+    # (everything that is multiplied by the rows' own features in one operand: the query's columns, then the merger's)
+    own = (torch.cat if isinstance(w["G"], torch.Tensor) else np.concatenate)([w["Mq"], w["G"][kd2:]], 1)
+    return {"G_tc": pack_tc(w["G"]), "W2t_tc": pack_tc(w["W2t"]), "Mq_img": pack_query(own),
+            "G_img": pack_stages(w["G"][:kd2]), "W2_img": pack_stages(w["W2t"])}
 
 
 def _f64(x):

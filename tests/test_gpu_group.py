@@ -68,6 +68,42 @@ def test_group_equals_batches(name, bs, k, E, recursion, layers):
             assert torch.equal(ha.emb, hb.emb) and torch.equal(ha.cache_flag_dev, hb.cache_flag_dev)
 
 
+@pytest.mark.parametrize("budget,chunks", [(1, "several"), (1500, "one")])
+def test_rows_that_share_features_equal_batches(budget, chunks):
+    """Layer 1 of a group computes what depends on a row's own features once per distinct memory row if the group's rows fit
+    one chunk, and per row otherwise (next to nothing is cached: the recomputed rows outnumber the batches' own).  Either
+    way the scores and tables are those of the single batches, whose rows share nothing."""
+    import argparse
+    import dataclasses
+    import types
+    from orca_b200.cache import get_cache_plan
+    from test_gpu_model import make_model
+    g = graph("c1")
+    bs, k, E = 100, 20, 3000
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs, n_degree=k, n_layers=2, budget=budget))
+    neg = synthetic.negative_destinations(g, seed=1)
+    lo = len(g.sources) - E
+    part = lambda x, a, b: x[lo + a:lo + b]
+    data = types.SimpleNamespace(sources=part(g.sources, 0, E), destinations=part(g.destinations, 0, E),
+                                 timestamps=part(g.timestamps, 0, E))
+    m = make_model(g)
+    nf = m.embedding_module.neighbor_finder
+    plan = get_cache_plan(argparse.Namespace(bs=bs, n_degree=k, budget=budget), data, nf, g.n_nodes, "MRD")
+    one, rows = [], 0
+    for i in range(E // bs):
+        a = [part(x, i * bs, (i + 1) * bs) for x in (g.sources, g.destinations, neg, g.timestamps, g.edge_idxs)]
+        one.append(torch.cat(m.compute_edge_probabilities(*a, k, True, False, plan[i])).cpu().numpy().ravel())
+        rows += m.check_status()[0]
+    assert (rows > 3 * E + 3 * E // 4) == (chunks == "several")
+    b = make_model(g)
+    p, q = b.eval_epoch(*[part(x, 0, E) for x in (g.sources, g.destinations, neg, g.timestamps, g.edge_idxs)], k, bs, plan)
+    one = np.stack(one).reshape(-1, 2, bs)
+    assert np.array_equal(one[:, 0].ravel(), p) and np.array_equal(one[:, 1].ravel(), q)
+    for t in ("memory", "last_update", "messages"):
+        assert torch.equal(getattr(m.memory, t), getattr(b.memory, t)), t
+    assert torch.equal(m.embedding_module.histories[0].emb, b.embedding_module.histories[0].emb)
+
+
 def test_a_stream_that_fails_leaves_a_model_that_works(monkeypatch):
     """A stream can fail in the middle -- here an id that cannot be packed, in the third group, and a workspace that
     cannot be allocated.  What was enqueued has finished when the error is raised, and the next stream runs as on a
