@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
   extern __shared__ unsigned char raw[];
   __shared__ __align__(16) float s_b1[BN], s_g[BN], s_b2[BN], s_lw[BN], s_lb[BN];
   __shared__ __align__(8) unsigned long long s_bar[2 * FIRST + 4];
+  __shared__ float2 s_sum[2][BM];                  // of a row's two halves: sum and sum of squares
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t base = (smem_addr(raw) + 1023u) & ~1023u, ring = base + FRONT;
@@ -232,59 +233,62 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(a2bar);
-      // second: accumulators -> row-major tile (over the hidden image, which has been read), then whole rows
+      // second: accumulators -> row-major tile (over the hidden image, which has been read) with the bias added; this thread's
+      // half of its row gives both moments in one sweep (the row is O(1) after the merger, so E[y^2] - mean^2 loses nothing
+      // that matters at the 1e-5 epsilon; columns from 172 on are zero, bias included)
       mbar_wait(acc2, t & 1, g.status, 721, alive, g.wait_limit);
       tc_fence_after();
+      float sum = 0.f, sq = 0.f;
+#pragma unroll 1
       for (int ch = ch0; ch < ch1; ++ch) {
         float v[16];
         tmem_ld16_sum(trow + ch * 16, SMALL, v);
+        float4 a = f4z, b = f4z;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          st_shared_f4(base + (uint32_t)(row * TILE_LD + ch * 16 + q * 4) * 4u,
-                       make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]));
+        for (int q = 0; q < 4; ++q) {
+          const float4 y = *reinterpret_cast<const float4 *>(s_b2 + ch * 16 + q * 4);
+          const float4 z = make_float4(v[q * 4] + y.x, v[q * 4 + 1] + y.y, v[q * 4 + 2] + y.z, v[q * 4 + 3] + y.w);
+          a.x += z.x, a.y += z.y, a.z += z.z, a.w += z.w;
+          b.x += z.x * z.x, b.y += z.y * z.y, b.z += z.z * z.z, b.w += z.w * z.w;
+          st_shared_f4(base + (uint32_t)(row * TILE_LD + ch * 16 + q * 4) * 4u, z);
+        }
+        sum += (a.x + a.y) + (a.z + a.w);
+        sq += (b.x + b.y) + (b.z + b.w);
       }
       tc_fence_before();
+      s_sum[half][row] = make_float2(sum, sq);
       __syncwarp();
       if (lane == 0) mbar_arrive(tfree);
       asm volatile("bar.sync 1, 256;" ::: "memory");
+      // then whole rows, a warp each
+      const float4 wA = vec(s_lw, lane, true), wB = vec(s_lw, lane + 32, has1);
+      const float4 lA = vec(s_lb, lane, true), lB = vec(s_lb, lane + 32, has1);
       constexpr int RB = 4;     // rows in flight per warp
+#pragma unroll 1
       for (int i0 = 0; i0 < BM / EPI_WARPS; i0 += RB) {
         if (ew + EPI_WARPS * i0 >= m_rows) break;
         float4 a[RB], b[RB];
-        float sum[RB], sq[RB];
-        const float4 bA = vec(s_b2, lane, true), bB = vec(s_b2, lane + 32, has1);
+        float mean[RB], inv[RB];
 #pragma unroll
         for (int k = 0; k < RB; ++k) {
-          const uint32_t ra = base + (uint32_t)((ew + EPI_WARPS * (i0 + k)) * TILE_LD + 4 * lane) * 4u;
-          const float4 x = ld_shared_f4(ra), y = has1 ? ld_shared_f4(ra + 512u) : f4z;
-          a[k] = make_float4(x.x + bA.x, x.y + bA.y, x.z + bA.z, x.w + bA.w);
-          b[k] = make_float4(y.x + bB.x, y.y + bB.y, y.z + bB.z, y.w + bB.w);
-          // both moments in one sweep (the row is O(1) after the merger, so E[y^2] - mean^2 loses nothing that matters
-          // at the 1e-5 epsilon)
-          sum[k] = (a[k].x + a[k].y) + (a[k].z + a[k].w) + (b[k].x + b[k].y) + (b[k].z + b[k].w);
-          sq[k] = a[k].x * a[k].x + a[k].y * a[k].y + a[k].z * a[k].z + a[k].w * a[k].w + b[k].x * b[k].x + b[k].y * b[k].y +
-                  b[k].z * b[k].z + b[k].w * b[k].w;
+          const int r = ew + EPI_WARPS * (i0 + k);
+          const uint32_t ra = base + (uint32_t)(r * TILE_LD + 4 * lane) * 4u;
+          a[k] = ld_shared_f4(ra);
+          b[k] = has1 ? ld_shared_f4(ra + 512u) : f4z;
+          const float2 x = s_sum[0][r], y = s_sum[1][r];
+          const float total = x.x + y.x;
+          mean[k] = total * (1.f / D);
+          inv[k] = 1.f / sqrtf(fmaxf(x.y + y.y - total * mean[k], 0.f) * (1.f / D) + 1e-5f);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int k = 0; k < RB; ++k) {
-            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
-            sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], o);
-          }
-        const float4 wA = vec(s_lw, lane, true), wB = vec(s_lw, lane + 32, has1);
-        const float4 lA = vec(s_lb, lane, true), lB = vec(s_lb, lane + 32, has1);
 #pragma unroll
         for (int k = 0; k < RB; ++k) {
           const int r = ew + EPI_WARPS * (i0 + k);
           const int to = __shfl_sync(0xffffffffu, push_id, i0 + k), win = __shfl_sync(0xffffffffu, push, i0 + k);
           if (r >= m_rows) continue;
-          const float mean = sum[k] * (1.f / D);
-          const float inv = 1.f / sqrtf(fmaxf(sq[k] - sum[k] * mean, 0.f) * (1.f / D) + 1e-5f);
-          const float4 ya = make_float4((a[k].x - mean) * inv * wA.x + lA.x, (a[k].y - mean) * inv * wA.y + lA.y,
-                                        (a[k].z - mean) * inv * wA.z + lA.z, (a[k].w - mean) * inv * wA.w + lA.w);
-          const float4 yb = make_float4((b[k].x - mean) * inv * wB.x + lB.x, (b[k].y - mean) * inv * wB.y + lB.y,
-                                        (b[k].z - mean) * inv * wB.z + lB.z, (b[k].w - mean) * inv * wB.w + lB.w);
+          const float4 ya = make_float4((a[k].x - mean[k]) * inv[k] * wA.x + lA.x, (a[k].y - mean[k]) * inv[k] * wA.y + lA.y,
+                                        (a[k].z - mean[k]) * inv[k] * wA.z + lA.z, (a[k].w - mean[k]) * inv[k] * wA.w + lA.w);
+          const float4 yb = make_float4((b[k].x - mean[k]) * inv[k] * wB.x + lB.x, (b[k].y - mean[k]) * inv[k] * wB.y + lB.y,
+                                        (b[k].z - mean[k]) * inv[k] * wB.z + lB.z, (b[k].w - mean[k]) * inv[k] * wB.w + lB.w);
           auto store = [&](float *o) {
             *reinterpret_cast<float4 *>(o + 4 * lane) = ya;
             if (has1) *reinterpret_cast<float4 *>(o + 4 * lane + 128) = yb;
