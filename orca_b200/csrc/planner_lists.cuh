@@ -212,9 +212,15 @@ __device__ __forceinline__ Line partition_warp(Entries e, Line r, int keep, uint
 // Calls f(index) for the entries of e[0 .. n) (key << IDX_BITS | index, in list order) that numba's argsort leaves at
 // `keep` or behind, 0 < keep < n (FIRST: for those before `keep`): its steps on the range that contains the line, until
 // that range is short or its keys are equal.  left, right: [n].  All T threads, behind a barrier; no barrier at the end.
-template <bool FIRST, class F>
-__device__ __forceinline__ void select_by_order(uint32_t *ents, int n, int keep, uint16_t *left, uint16_t *right,
-                                                uint32_t *s_tot, Line *s_line, F f) {
+// aside(): work of one warp that may be done beside the first one's partition steps; returns whether it was (the same in
+// every thread).
+struct Nothing {
+  __device__ void operator()() const {}
+};
+template <bool FIRST, class F, class Aside = Nothing>
+__device__ __forceinline__ bool select_by_order(uint32_t *ents, int n, int keep, uint16_t *left, uint16_t *right,
+                                                uint32_t *s_tot, Line *s_line, F f, Aside aside = Aside()) {
+  bool done = false;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   const Entries e{ents};
@@ -232,7 +238,10 @@ __device__ __forceinline__ void select_by_order(uint32_t *ents, int n, int keep,
       if (warp == 0) {
         const Line z = partition_warp(e, r, keep, left, right);
         if (lane == 0) *s_line = z;
+      } else if (warp == 1) {
+        aside();
       }
+      done = true;
       __syncthreads();
       break;
     }
@@ -307,6 +316,7 @@ __device__ __forceinline__ void select_by_order(uint32_t *ents, int n, int keep,
     if ((place < keep) == FIRST) f((int)(ents[pos] & IDX));
   }
   for (int pos = (FIRST ? 0 : hi + 1) + tid; pos < (FIRST ? lo : n); pos += T) f((int)(ents[pos] & IDX));
+  return done;
 }
 
 // The usual first step of a selection over a list whose keys are given by key(i): its pivot is the largest key there is,

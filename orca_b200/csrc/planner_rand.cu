@@ -13,7 +13,7 @@
 // One CTA of 1024 threads per plan; its bound is latency, of the barriers and of the scattered loads in between.
 // 250 batches of 600 edges with 20 neighbours, LRU, ms of the kernel: 19.2 with draws, swaps, bitmaps and sort in global
 // memory, 9.9 with those in shared memory, 3.4 with lists in place of the tables' 24,000 entries a batch and without the
-// levels of the sort that do not decide.
+// levels of the sort that do not decide, 3.0 with the generator beside the selection and members listed by half words.
 #include <algorithm>
 
 #include "common.cuh"
@@ -54,7 +54,7 @@ struct Twister {
   // The draws of a shuffle of n entries, from the back: entry i swaps with draw[i] (draw may be null: the generator
   // moves on all the same).  Number l of a group of 32 is accepted iff it lies below its bound, which falls by one for
   // every number accepted before it: the votes settle from the left, in two or three rounds as a rule, 33 at most.
-  __device__ void draws(int n, int32_t *draw) {
+  __device__ __noinline__ void draws(int n, int32_t *draw) {
     const int lane = threadIdx.x & 31;
     int at = pos;
     while (n > 1) {
@@ -115,9 +115,41 @@ __device__ __forceinline__ void set_bit(uint32_t *bm, int32_t v) { atomicOr(&bm[
 __device__ __forceinline__ void clear_bit(uint32_t *bm, int32_t v) { atomicAnd(&bm[v >> 5], ~(1u << (v & 31))); }
 
 // Members of a bitmap in ascending order -> out; returns their number (the same in every thread).  All T
-// threads call it; `clear` empties the bitmap on the way.  s_cnt: NW ints of shared memory.
-__device__ __forceinline__ int list_members(uint32_t *bm, int64_t words, int32_t *out, bool clear, int *s_cnt) {
+// threads call it.  s_cnt: NW ints of shared memory.
+// Bitmaps of a few words a thread are dealt out by half words, neighbouring ones to a thread: a thread then lists a handful
+// of members (343 words, a word a lane of eleven warps: 5,600 cycles a batch with the copy out; half words over all of them: 3,400).
+constexpr int FEW_WORDS = 2 * T;
+__device__ __forceinline__ int list_members(uint32_t *bm, int64_t words, int32_t *out, int *s_cnt) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (words <= FEW_WORDS) {
+    constexpr int MOST = 2 * FEW_WORDS / T;
+    const int halves = 2 * (int)words, per = (halves + T - 1) / T;
+    __syncthreads();   // (earlier writes to the bitmap; earlier readers of s_cnt)
+    uint32_t bits[MOST];
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) {
+      const int at = tid * per + i;
+      bits[i] = i < per && at < halves ? word(bm, at >> 1) >> 16 * (at & 1) & 0xffffu : 0u;
+      cnt += __popc(bits[i]);
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) s_cnt[warp] = incl;
+    __syncthreads();
+    const int x = s_cnt[lane];
+    int pos = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0) + incl - cnt;
+    const int n = __reduce_add_sync(0xffffffffu, x);
+#pragma unroll
+    for (int i = 0; i < MOST; ++i)
+      for (uint32_t b = bits[i]; b != 0; b &= b - 1) out[pos++] = 16 * (tid * per + i) + __ffs(b) - 1;
+    __syncthreads();
+    return n;
+  }
   const int wchunk = (int)(((words + NW - 1) / NW + 31) & ~31ll);
   __syncthreads();   // (earlier writes to the bitmap; earlier readers of s_cnt)
   int cnt = 0;
@@ -137,10 +169,7 @@ __device__ __forceinline__ int list_members(uint32_t *bm, int64_t words, int32_t
   for (int j = 0; j < wchunk; j += 32) {
     const int64_t wi = (int64_t)warp * wchunk + j + lane;
     uint32_t bits = 0;
-    if (wi < words) {
-      bits = word(bm, wi);
-      if (clear && bits) bm[wi] = 0;
-    }
+    if (wi < words) bits = word(bm, wi);
     const int c = __popc(bits);
     int incl = c;
     for (int o = 1; o < 32; o <<= 1) {
@@ -186,10 +215,11 @@ __device__ void shuffle(const Work &w, Twister &rng, int32_t *x, int n, bool any
   __syncthreads();
 }
 
-// the first `count` entries, fewer than n, of numba's argsort of key[ids[i]] (i < n): calls f(id) for each of them
-template <class F>
+// the first `count` entries, fewer than n, of numba's argsort of key[ids[i]] (i < n): calls f(id) for each of them.
+// aside: select_by_order's; `beside` is set if it was done
+template <class F, class Aside>
 __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int count, const int32_t *key, int *s_a,
-                                 int *s_b, F f) {
+                                 int *s_b, F f, Aside aside, bool &beside) {
   if (count >= n) {
     for (int i = threadIdx.x; i < n; i += T) f(ids[i]);
     __syncthreads();
@@ -201,7 +231,7 @@ __device__ bool for_first_by_key(const Work &w, const int32_t *ids, int n, int c
     for (int i = threadIdx.x; i < n; i += T) e[i] = (uint32_t)key[ids[i]] << lists::IDX_BITS | (uint32_t)i;
     __syncthreads();
     __shared__ lists::Line s_line;
-    lists::select_by_order<true>(e, n, count, left, right, (uint32_t *)s_a, &s_line, [&](int i) { f(ids[i]); });
+    beside = lists::select_by_order<true>(e, n, count, left, right, (uint32_t *)s_a, &s_line, [&](int i) { f(ids[i]); }, aside);
     __syncthreads();
     return true;
   }
@@ -350,22 +380,24 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t b0, int64_t b1, int64
     const int room = budget - n_held;
     const int evict = room >= n_cand ? 0 : min(n_cand - room, n_held);
     const int take = (evict + room >= n_cand) ? n_cand : budget;
+    // (where all candidates are taken only the generator moves: beside the selection, 3,600 of 27,500 cycles a batch)
+    bool drawn = false;
     if (evict != 0) {
-      if (!for_first_by_key(w, held, n_held, evict, used_at, s_a, s_b,
-                            [&](int32_t v) { clear_bit(cached, v); })) {
+      if (!for_first_by_key(w, held, n_held, evict, used_at, s_a, s_b, [&](int32_t v) { clear_bit(cached, v); },
+                            [&]() { if (take == n_cand) rng.draws(n_cand, nullptr); }, drawn)) {
         if (tid == 0) report(status, ORCA_E_TIMEOUT, (int)b);
         failed = true;
         break;
       }
     }
-    shuffle(w, rng, cand, n_cand, take == n_cand);
+    if (!drawn || take != n_cand) shuffle(w, rng, cand, n_cand, take == n_cand);
     for (int i = tid; i < take; i += T) {
       const int32_t v = cand[i];
       set_bit(cached, v);
       used_at[v] = arrived[v] = (int32_t)b;
     }
     held = listed_at(used);
-    n_held = list_members(cached, words, held, false, s_a);
+    n_held = list_members(cached, words, held, s_a);
     if (used + n_held > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
@@ -453,7 +485,7 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       }
       n_fifo = half;
     } else {
-      const int n_ids = list_members(fifo, words, ids, false, s_a);
+      const int n_ids = list_members(fifo, words, ids, s_a);
       shuffle(w, rng, ids, n_ids, false);
       for (int i = tid; i < n_fresh - fifo_room; i += T) clear_bit(fifo, ids[i]);
       __syncthreads();
@@ -477,9 +509,10 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       for (int i = tid; i < n_promote; i += T) admit(promote[i]);
       n_lru += n_promote;
     } else if (n_promote <= lru_room + lru_evictable) {
-      const int n_ids = list_members(lru, words, ids, false, s_a);
+      const int n_ids = list_members(lru, words, ids, s_a);
+      bool beside = false;
       if (!for_first_by_key(w, ids, n_ids, n_promote - lru_room, lru_used, s_a, s_b,
-                            [&](int32_t v) { clear_bit(lru, v); })) {
+                            [&](int32_t v) { clear_bit(lru, v); }, lists::Nothing(), beside)) {
         if (tid == 0) report(status, ORCA_E_TIMEOUT, (int)b);
         failed = true;
         continue;
@@ -487,7 +520,7 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       for (int i = tid; i < n_promote; i += T) admit(promote[i]);
       n_lru = half;
     } else {
-      const int n_ids = list_members(lru, words, ids, false, s_a);
+      const int n_ids = list_members(lru, words, ids, s_a);
       for (int i = tid; i < n_ids; i += T)
         if (lru_used[ids[i]] < now) clear_bit(lru, ids[i]);
       __syncthreads();
@@ -498,14 +531,14 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       n_lru = half;
     }
     // ---- plan = FIFO ids ascending, then LRU ids ascending
-    n_fifo = list_members(fifo, words, ids, false, s_a);
+    n_fifo = list_members(fifo, words, ids, s_a);
     if (used + n_fifo > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
       continue;
     }
     for (int i = tid; i < n_fifo; i += T) plan[used + i] = ids[i];
-    n_lru = list_members(lru, words, ids, false, s_a);
+    n_lru = list_members(lru, words, ids, s_a);
     if (used + n_fifo + n_lru > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
