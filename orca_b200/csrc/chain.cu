@@ -39,7 +39,7 @@ constexpr int A_CHUNKS = 2 * PART_CHUNKS, A_LBO = ROWS * 16 + 16, A_BYTES = A_CH
 constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 1024;
 constexpr int EPI_WARPS = 4, PRODUCERS = 256, THREADS = 32 * EPI_WARPS + PRODUCERS + 32;
 constexpr int TMEM_COLS = 128, BUF_COLS = 64, SMALL = 32;   // two accumulator buffers of main + cross terms
-constexpr int BLOCK_ROWS = 32;                 // updates a row block takes before there is another one (16 to 64: the same)
+constexpr int BLOCK_ROWS = 64;                 // updates a row block takes before there is another one
 constexpr int META = 4;                        // steps whose memory rows are kept
 constexpr int PER = 6;                         // chunks a producer thread has in flight: 34 rows at a time
 
