@@ -42,6 +42,26 @@ class RandEdgeSampler:
         self.random_state = np.random.RandomState(self.seed)
 
 
+class _Drawn:
+    """The negatives of a stream, one draw a batch in the stream's order, made when a batch is first asked for (TGN.eval_epoch
+    packs a group of batches while the GPU works on the one before)."""
+
+    def __init__(self, n, batch_size, draw):
+        self.ids, self.batch_size, self.draw, self.drawn = np.empty(n, dtype=np.int64), batch_size, draw, 0
+        self[:1]      # (a sampler that cannot draw says so before anything is scored)
+
+    def __len__(self):
+        return len(self.ids)
+
+    def __getitem__(self, part):
+        upto = len(self.ids) if part.stop is None else min(part.stop, len(self.ids))
+        while self.drawn < upto:
+            n = min(self.batch_size, len(self.ids) - self.drawn)
+            self.ids[self.drawn:self.drawn + n] = self.draw(n)
+            self.drawn += n
+        return self.ids[part]
+
+
 def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_size, reuse=True, cache_plan=None):
     assert negative_edge_sampler.seed is not None
     negative_edge_sampler.reset_random_state()
@@ -51,10 +71,10 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
         lambda size: negative_edge_sampler.sample(size)[1]
     n = data.n_interactions
     nb = math.ceil(n / batch_size)
-    negatives = np.empty(n, dtype=np.int64)
-    for i in range(nb):
-        lo, hi = i * batch_size, min(n, (i + 1) * batch_size)
-        negatives[lo:hi] = draw(hi - lo)
+    negatives = _Drawn(n, batch_size, draw)
+    own = all(getattr(getattr(model, f, None), "__func__", None) is getattr(TGN, f) for f in ("eval_epoch", "eval_epoch_metrics"))
+    if not own or type(negative_edge_sampler) is not RandEdgeSampler:
+        negatives = negatives[:]      # (somebody else's: all draws before the first batch, as the reference's caller sees it)
     # per batch, as the reference does; the positive "wins" when its score is not below the negative's
     # (evaluation/evaluation.py:39-40)
     stream = (data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n], data.edge_idxs[:n], n_neighbors,

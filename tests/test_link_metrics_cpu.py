@@ -34,3 +34,16 @@ def test_scores_that_are_not_finite_are_refused():
         neg[3] = bad
         rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, 10, 10, out.ctypes.data)
         assert rc == _lib.E_BADARG
+
+
+@pytest.mark.parametrize("n,bs", [(1, 5), (7, 7), (20, 6), (23, 1)])
+def test_negatives_drawn_when_asked_for_are_those_drawn_at_once(n, bs):
+    from orca_b200.evaluation import RandEdgeSampler, _Drawn
+    at_once, lazily = (RandEdgeSampler(np.arange(5), np.arange(100), seed=3) for _ in range(2))
+    want = np.concatenate([at_once.sample(min(bs, n - lo))[1] for lo in range(0, n, bs)])
+    drawn = _Drawn(n, bs, lazily.sample_destinations)
+    assert drawn.drawn == min(bs, n) and len(drawn) == n
+    for lo in range(0, n, 3):
+        assert np.array_equal(drawn[lo:lo + 3], want[lo:lo + 3]) and drawn.drawn < lo + 3 + bs
+    assert np.array_equal(drawn[:], want)
+    assert at_once.random_state.randint(1 << 30) == lazily.random_state.randint(1 << 30)
