@@ -22,6 +22,7 @@
 // Every wait is bounded; one that gives up reports ORCA_E_TIMEOUT and the kernel runs to its end.
 #include "chain.cuh"
 #include "context.cuh"
+#include "gru_rows.cuh"
 #include "tc_gemm.cuh"
 #include "tc_ptx.cuh"
 
@@ -336,8 +337,11 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
     }
     float4 *dst = reinterpret_cast<float4 *>(g.mem.messages + (size_t)node * MSG);
 #pragma unroll
-    for (int q = 0; q < TURNS; ++q)
-      if (lane + LANES * q < PIECES) dst[lane + LANES * q] = x[q];
+    for (int q = 0; q < TURNS; ++q) {
+      const int at = lane + LANES * q;
+      if (at < PIECES) dst[at] = x[q];
+      if (WARPS == 1 && g.msg_image != nullptr && at < PIECES) put_message(g.msg_image, l, at / ROW_PIECES, at % ROW_PIECES, x[q]);
+    }
     if (WARPS > 1) __syncthreads();     // (the last update has been read)
     else __syncwarp();
     if (lane == 0) {

@@ -17,6 +17,7 @@ struct ChainArgs {
   const void *w;            // weights.prepare_gru: one image per column tile
   const float *bias;
   void *image;              // update_image_bytes(nb * 2 * bs)
+  char *msg_image;          // optional: operand image of the messages of every node's last update (gru_rows.cuh)
   int32_t *status;          // set by launch_gru_chain
   long long wait_limit;
 };

@@ -478,17 +478,6 @@ static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, 
   a.nodes = d_nodes;
   return a;
 }
-int gru_rows(const orca_gru_weights_t *w, const orca_memory_t &mem, const int32_t *d_node, const int32_t *d_out_row, int cap,
-             const int32_t *d_n, float *d_out, cudaStream_t s) {
-  ORCA_CHECK_ARG(w->Wg_tc != nullptr && w->bg != nullptr);
-  tc::Args a = gru_args(w, &mem, d_node, cap, d_n, d_out);
-  a.a1 = tc::RowSrc{};
-  a.Kd = MSG;
-  a.memory = mem.messages;
-  a.memory_ld = MSG;
-  a.out_rows = d_out_row;
-  return tc::launch(tc::EPI_GRU, a, 4, s);
-}
 
 }  // namespace orca
 

@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "context.cuh"
 #include "group.cuh"
+#include "gru_rows.cuh"
 #include "index_ops.cuh"
 #include "sampling.cuh"
 #include "tc_gemm.cuh"
@@ -481,6 +482,7 @@ struct Parity {
 struct Buffers {
   Parity par[2];
   float *log;              // two parities, one after the other
+  char *msg_image;         // of the messages of every node's last update (groups whose last updates leave the chain)
   float *qt, *own, *emb1, *emb2;
   char *ctx, *feat, *feat2;   // operand images (attn_out.cuh): attention sums, own features, layer 2's own features
   uint8_t *valid;
@@ -534,6 +536,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.upd_image = take(update_image_bytes(2 * E));
   }
   w.log = (float *)take((size_t)2 * 2 * E * D * 4);
+  w.msg_image = (char *)take(2 * E > SPLIT_FROM ? gru_image_bytes(std::min(2 * E, n_nodes)) : 4);
   w.qt = (float *)take((size_t)w.chunk * QT_LD * 4);
   w.own = (float *)take((size_t)w.chunk * OWN_LD * 4);
   w.ctx = (char *)take(img::bytes(w.chunk, img::CTX_STAGES));
@@ -692,9 +695,11 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     if (si != s) ORCA_CUDA(cudaEventRecord(c->ev_gidx[p], si));     // (from here on: index work and flags)
     // ---- memory chain
     grp::ChainArgs ch{a, m->mem, log, w.log + (size_t)p * 2 * E_max * D, m->edge_table, m->time_w, m->gru.Wg_chain, m->gru.bg,
-                      x.upd_image, nullptr, 0};
+                      x.upd_image, a.split ? w.msg_image : nullptr, nullptr, 0};
     ORCA_TRY(grp::launch_gru_chain(ch, sx));
-    if (a.split) ORCA_TRY(gru_rows(&m->gru, m->mem, x.last_node, x.last_at, 2 * g->nb * g->bs, &x.cnt->n_last, ch.log_out, sx));
+    if (a.split)
+      ORCA_TRY(gru_rows(&m->gru, m->mem, w.msg_image, x.last_node, x.last_at, (int)std::min<int64_t>(2 * E, m->n_nodes), &x.cnt->n_last,
+                        ch.log_out, sx));
     if (sx != s) ORCA_CUDA(cudaEventRecord(c->ev_gchain[p], sx));
     return ORCA_OK;
   };

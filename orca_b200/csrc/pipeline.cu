@@ -31,6 +31,7 @@
 #include "chain.cuh"
 #include "common.cuh"
 #include "context.cuh"
+#include "gru_rows.cuh"
 #include "index_ops.cuh"
 #include "tc_gemm.cuh"
 
@@ -66,6 +67,7 @@ struct Workspace {
   uint8_t *win1;
   float *gru_h;
   void *upd_image;           // split inputs of the memory updates (chain.cu)
+  char *msg_image;           // operand image of the batch's messages (gru_rows.cu)
   void *bitmap;
   size_t bytes;
 };
@@ -122,6 +124,7 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
   w.win1 = (uint8_t *)take(R1);
   w.gru_h = (float *)take(2 * (size_t)b_cap * D * 4);
   w.upd_image = take(grp::update_image_bytes(2 * (int64_t)b_cap));
+  w.msg_image = (char *)take(gru_image_bytes(2 * (int64_t)b_cap));
   w.bitmap = take((size_t)orca_find_uncached_scratch_bytes(n_nodes));
   w.bytes = off;
   return w;
@@ -401,6 +404,17 @@ static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d
   return attn_output_rows(a, s);
 }
 
+// raw messages of a batch and its new memory rows, to w.gru_h, as a pair of launches
+static int store_and_update(const orca_tgn_t *m, Workspace &w, IdxBuf &x, const int32_t *d_batch_i32, const double *d_batch_ts,
+                            int b, cudaStream_t s) {
+  const bool from_image = projections_on_tensor_cores();
+  const int rc = message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts, d_batch_i32 + 3 * b, b,
+                               x.win_pos, 2 * b, x.n_win, x.win_nodes, from_image ? w.msg_image : nullptr, s);
+  if (rc != ORCA_OK) return rc;
+  return from_image ? gru_rows(&m->gru, m->mem, w.msg_image, x.win_nodes, nullptr, 2 * b, x.n_win, w.gru_h, s)
+                    : gru_project(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, w.gru_h, s);
+}
+
 // Raw messages and GRU of a batch by the memory chain's kernel (chain.cu), or as a pair of launches.  The chain's kernel
 // is the faster one where a batch's launches stand in one line (eval_serial; one layer, us a call, pair / chain: 37 edges
 // 100.5 / 97.5, 200 115 / 102.6, 500 128 / 117, 800 125 / 123, 1024 129 / 130), not in the lanes of a budgeted batch,
@@ -457,9 +471,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
       ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid,
                                       x.upd_t, x.cnt, w.upd_image, w.gru_h, ms));
     } else {
-      ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
-                                  d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, ms));
-      ORCA_TRY(gru_project(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, w.gru_h, ms));
+      ORCA_TRY(store_and_update(m, w, x, d_batch_i32, d_batch_ts, b, ms));
     }
     ORCA_TRY(tr.mark(PH_MESSAGE, s));
     return ORCA_OK;
@@ -683,10 +695,13 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
       if (si != s) ORCA_CUDA(cudaStreamWaitEvent(sx, c->ev_idx[p], 0));
       else ORCA_TRY(link(s, sx, c->fork));
     }
-    ORCA_TRY(orca_message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts,
-                                d_batch_i32 + 3 * b, b, x.win_pos, 2 * b, x.n_win, x.win_nodes, sx));
+    const bool from_image = !gru_split && projections_on_tensor_cores();
+    ORCA_TRY(message_store(&m->mem, m->edge_table, m->time_w, d_batch_i32, x.cat_dst, d_batch_ts, d_batch_i32 + 3 * b, b,
+                           x.win_pos, 2 * b, x.n_win, x.win_nodes, from_image ? w.msg_image : nullptr, sx));
     ORCA_TRY(tr.mark(PH_MESSAGE, s));
-    if (gru_split && !in_a) {
+    if (from_image) {
+      ORCA_TRY(gru_rows(&m->gru, m->mem, w.msg_image, x.win_nodes, nullptr, 2 * b, x.n_win, w.gru_h, sx));
+    } else if (gru_split && !in_a) {
       // (split by layer: the layer-1 ranks compute the memory update; this rank only receives the rows)
     } else if (gru_split) {
       // the memory update is split by node: this rank computes every wa-th unique positive and stores the

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "gru_rows.cuh"
 
 namespace orca {
 
@@ -45,7 +46,7 @@ message_store_kernel(orca_memory_t mem, const float *__restrict__ edge_table, co
                      const int32_t *__restrict__ cat_src, const int32_t *__restrict__ cat_dst,
                      const double *__restrict__ ts, const int32_t *__restrict__ eidx, int b,
                      const int32_t *__restrict__ win_pos, int n_cap, const int32_t *d_n,
-                     int32_t *__restrict__ win_nodes) {
+                     int32_t *__restrict__ win_nodes, char *__restrict__ image) {
   dep_trigger();
   dep_wait();
   const int n = rows_of(n_cap, d_n);
@@ -62,16 +63,37 @@ message_store_kernel(orca_memory_t mem, const float *__restrict__ edge_table, co
     const float *src = part == 0 ? mem.memory + (size_t)node * D
                      : part == 1 ? mem.memory + (size_t)other * D
                                  : edge_table + (size_t)e * D;
-    if (lane < ROW_F4) reinterpret_cast<float4 *>(dst)[lane] = reinterpret_cast<const float4 *>(src)[lane];
-  } else {
+    if (lane < ROW_F4) {
+      const float4 x = reinterpret_cast<const float4 *>(src)[lane];
+      reinterpret_cast<float4 *>(dst)[lane] = x;
+      if (image != nullptr) put_message(image, w, part, lane, x);
+    }
+  } else if (lane < ROW_F4) {
     const float gap = t - mem.last_update[node];
-    for (int d = lane; d < D; d += 64) dst[d] = cos_any(gap * __ldg(time_w + d));
+    const float *f = time_w + 4 * lane;
+    const float4 x = make_float4(cos_any(gap * __ldg(f)), cos_any(gap * __ldg(f + 1)), cos_any(gap * __ldg(f + 2)), cos_any(gap * __ldg(f + 3)));
+    reinterpret_cast<float4 *>(dst)[lane] = x;
+    if (image != nullptr) put_message(image, w, part, lane, x);
   }
   if (threadIdx.x == 0) {
     mem.msg_ts[node] = t;
     mem.msg_flag[node] = 1;
     if (win_nodes) win_nodes[w] = node;
   }
+}
+
+int message_store(const orca_memory_t *mem, const float *d_edge_table, const float *d_time_w, const int32_t *d_cat_src,
+                  const int32_t *d_cat_dst, const double *d_ts, const int32_t *d_eidx, int32_t b, const int32_t *d_win_pos,
+                  int32_t n_win_cap, const int32_t *d_n_win, int32_t *d_win_nodes, char *d_image, cudaStream_t s) {
+  ORCA_CHECK_ARG(mem && mem->memory && mem->last_update && mem->messages && mem->msg_ts && mem->msg_flag);
+  ORCA_CHECK_ARG(d_edge_table && d_time_w && d_cat_src && d_cat_dst && d_ts && d_eidx && d_win_pos);
+  ORCA_CHECK_ARG(b >= 0 && n_win_cap >= 0);
+  if (n_win_cap == 0 || b == 0) return ORCA_OK;
+  ORCA_CUDA(launch_dep(message_store_kernel, n_win_cap, 256, 0, s, *mem, d_edge_table, d_time_w, d_cat_src, d_cat_dst, d_ts,
+                       d_eidx, b, d_win_pos, n_win_cap, d_n_win, d_win_nodes, d_image));
+  ORCA_COUNT_LAUNCH();
+  ORCA_LAUNCH_CHECK();
+  return ORCA_OK;
 }
 
 }  // namespace orca
@@ -123,15 +145,8 @@ int orca_message_store(const orca_memory_t *mem, const float *d_edge_table, cons
                        const int32_t *d_cat_src, const int32_t *d_cat_dst, const double *d_ts,
                        const int32_t *d_eidx, int32_t b, const int32_t *d_win_pos, int32_t n_win_cap,
                        const int32_t *d_n_win, int32_t *d_win_nodes, void *stream) {
-  ORCA_CHECK_ARG(mem && mem->memory && mem->last_update && mem->messages && mem->msg_ts && mem->msg_flag);
-  ORCA_CHECK_ARG(d_edge_table && d_time_w && d_cat_src && d_cat_dst && d_ts && d_eidx && d_win_pos);
-  ORCA_CHECK_ARG(b >= 0 && n_win_cap >= 0);
-  if (n_win_cap == 0 || b == 0) return ORCA_OK;
-  ORCA_CUDA(launch_dep(message_store_kernel, n_win_cap, 256, 0, (cudaStream_t)stream, *mem, d_edge_table, d_time_w,
-                       d_cat_src, d_cat_dst, d_ts, d_eidx, b, d_win_pos, n_win_cap, d_n_win, d_win_nodes));
-  ORCA_COUNT_LAUNCH();
-  ORCA_LAUNCH_CHECK();
-  return ORCA_OK;
+  return message_store(mem, d_edge_table, d_time_w, d_cat_src, d_cat_dst, d_ts, d_eidx, b, d_win_pos, n_win_cap, d_n_win,
+                       d_win_nodes, nullptr, (cudaStream_t)stream);
 }
 
 }  // extern "C"

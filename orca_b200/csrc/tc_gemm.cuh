@@ -122,10 +122,6 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
 // scorer over the rows of a group of batches (gemm.cu); tensor cores only
 int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
                float *d_prob, cudaStream_t s);
-// GRU of rows whose messages are in the message table and whose memory row is the own part of it: row m is the message
-// of node d_node[m], its new memory goes to row d_out_row[m] (gemm.cu); tensor cores only
-int gru_rows(const orca_gru_weights_t *w, const orca_memory_t &mem, const int32_t *d_node, const int32_t *d_out_row, int cap,
-             const int32_t *d_n, float *d_out, cudaStream_t s);
 // whether the projections run on the tensor cores (orca_set_projection_mode(0)); the fp32 debug path has
 // no peer fan-out
 bool projections_on_tensor_cores();

@@ -866,3 +866,40 @@ def test_sampled_ids_without_rows_are_reported(name, reuse, budget, k):
         for x, y in zip(run(lists(g.n_nodes - 1, g.n_edges, 1e30), stream), late):
             assert np.array_equal(x, y) and np.isfinite(x).all()
         run(lists(g.n_nodes - 1, g.n_edges, 2.0), stream)
+
+
+@pytest.mark.parametrize("b", [1, 63, 64, 65, 128, 200, 1100])
+def test_updates_of_a_batch_against_64_bits(b):
+    """Memory rows of a budgeted batch, whose messages come to the GRU as an operand image, against the GRU in 64 bits from the
+    message table: fewer rows than a block, a block and a bit, several.  Operands carry 16 significant bits (relative error
+    2^-17 each, both sides of a product): a gate's sum is off by 2^-16 of the sum of the products' sizes, the gates' slopes are
+    at most 1/4 (twice) and 1, and the candidate is scaled by the reset gate's sum once more."""
+    g = graph("c1")
+    tgn = _two_layer_model(g, b)
+    rs = np.random.RandomState(b)
+    old = torch.from_numpy((rs.randn(g.n_nodes, 172) * 0.4).astype(np.float32)).cuda()
+    tgn.memory.memory.copy_(old)
+    lo = len(g.sources) // 2
+    part = [x[lo:lo + b] for x in (g.sources, g.destinations, g.destinations[::-1], g.timestamps, g.edge_idxs)]
+    tgn.compute_edge_probabilities(*part, 10, True, False, np.unique(part[0])[:20])
+    tgn.check_status()
+    nodes = np.unique(np.concatenate(part[:2]))
+    p = "memory_updater.memory_updater."
+    wi, wh, bi, bh = (torch.from_numpy(state_dict(2)[p + n]).double() for n in ("weight_ih", "weight_hh", "bias_ih", "bias_hh"))
+    x, h = tgn.memory.messages.cpu()[nodes].double(), old.cpu()[nodes].double()
+    assert torch.equal(x[:, :172].float(), old.cpu()[nodes])
+    i, j = (x @ wi.T + bi).chunk(3, 1), (h @ wh.T + bh).chunk(3, 1)
+    r, z = torch.sigmoid(i[0] + j[0]), torch.sigmoid(i[1] + j[1])
+    want = (1 - z) * torch.tanh(i[2] + r * j[2]) + z * h
+    size = (x.abs() @ wi.abs().T).chunk(3, 1), (h.abs() @ wh.abs().T).chunk(3, 1)
+    off = [2.0 ** -16 * (a + c) for a, c in zip(*size)]
+    bound = off[2] + off[0] / 4 * (1 + j[2].abs()) + off[1] / 4 * (1 + h.abs()) + 2e-6
+    got = tgn.memory.memory.cpu().double()
+    assert bool(((got[nodes] - want).abs() < bound).all())
+    rest = np.setdiff1d(np.arange(g.n_nodes), nodes)
+    assert torch.equal(got[rest].float(), old.cpu()[rest])
+
+
+def _two_layer_model(g, bs):
+    import dataclasses
+    return make_model(dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs, n_layers=2, n_degree=10, budget=20)))
