@@ -5,9 +5,8 @@
 // a pipeline filled and drained, two launches) whatever the batch size, and it is the only part of a group that is
 // serial: with small batches it is what a stream waits for.  What a batch really waits for is its memory rows.  So
 // one cooperative grid walks the batches:
-//   - 22 column tiles of 32 gate columns (eight units) times row blocks of 64 updates, one CTA each: up to six for a
-//     single batch, five for a group, whose layers run beside it (launch).  A CTA
-//     keeps its weight columns (880 x 32, bf16 head and tail, 113 KB) in shared memory for the whole launch.
+//   - 22 column tiles of 32 gate columns (eight units) times row blocks of 64 updates, one CTA each, up to five (launch).
+//     A CTA keeps its weight columns (880 x 32, bf16 head and tail, 113 KB) in shared memory for the whole launch.
 //   - K is laid out so that what does not depend on the batch before comes first: edge features and time encoding
 //     (352 columns).  A launch of its own splits them for all updates of the group (computed in the chain, the cosines
 //     alone were half of a turn), and they are multiplied for batch n + 1 while batch n is still being finished.
@@ -54,7 +53,7 @@ __global__ void __launch_bounds__(256) update_image_kernel(const __grid_constant
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.nb * 2 * a.bs; i += (gridDim.x * blockDim.x) >> 5) {
     const int n = i / (2 * a.bs), w = i - n * 2 * a.bs;
     if (w >= a.cnt->n_win[n]) continue;
-    const float gap = a.win_gap != nullptr ? a.win_gap[i] : a.win_t[i] - g.mem.last_update[a.win_node[i]];
+    const float gap = a.win_gap[i];
     if (lane < 12) {
       const int r = lane < 6 ? a.win_mem[i] : a.win_other[i];
       if (r < a.n_nodes)
@@ -316,11 +315,11 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
   constexpr int PIECES = MSG / 4, ROW_PIECES = D / 4;
   constexpr int LANES = 32 * WARPS;      // of an update
   const int lane = threadIdx.x % LANES, step = gridDim.x * (blockDim.x / LANES);
-  const int n = a.last_at != nullptr ? a.cnt->n_last : a.cnt->n_win[0];
+  const int n = a.cnt->n_last;
   for (int l = (blockIdx.x * blockDim.x + threadIdx.x) / LANES; l < n; l += step) {
-    const int i = a.last_at != nullptr ? a.last_at[l] : l;
+    const int i = a.last_at[l];
     const int node = a.win_node[i], self = a.win_mem[i], other = a.win_other[i];
-    const float t = a.win_t[i], gap = a.win_gap != nullptr ? a.win_gap[i] : t - g.mem.last_update[node];
+    const float t = a.win_t[i], gap = a.win_gap[i];
     const float4 *src[3] = {reinterpret_cast<const float4 *>((self >= a.n_nodes ? g.log : g.mem.memory) + (size_t)self * D),
                             reinterpret_cast<const float4 *>((other >= a.n_nodes ? g.log : g.mem.memory) + (size_t)other * D),
                             reinterpret_cast<const float4 *>(g.edge_table + (size_t)a.win_eid[i] * D)};
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(256) last_messages_kernel(const __grid_constan
   }
 }
 
-static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
+int launch_gru_chain(const ChainArgs &args, cudaStream_t s) {
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "launch_gru_chain: no context for the current device");
   static thread_local int configured_device = -1;
@@ -367,10 +366,10 @@ static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
   ORCA_CUDA(launch_dep(update_image_kernel, std::min(ceil_div(most, 8), c->sm_count * 8), 256, 0, s, g));
   ORCA_COUNT_LAUNCH();
   cudaLaunchConfig_t cfg = {};
-  // A group's chain leaves one row block's SMs to the layers that run beside it: 48 batches of 1000 3.12 -> 3.08 ms, 50 of
-  // 2000 6.56 -> 6.49, others unchanged; two row blocks fewer cost batches of 600 3 %.
-  const int fit = c->sm_count / COL_TILES - (g.a.nb > 1 ? 1 : 0);
-  cfg.gridDim = dim3(COL_TILES, std::max(1, std::min(blocks, fit)));
+  // As many row blocks as fit (a batch with more updates than rows takes another turn), less one, whose SMs are left to the
+  // layers that run beside the chain: 48 batches of 1000 3.12 -> 3.08 ms, 50 of 2000 6.56 -> 6.49, others unchanged; two row
+  // blocks fewer cost batches of 600 3 %.
+  cfg.gridDim = dim3(COL_TILES, std::max(1, std::min(ceil_div(2 * g.a.bs, 8), c->sm_count / COL_TILES - 1)));
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = s;
@@ -378,53 +377,11 @@ static int launch(const ChainArgs &args, int blocks, cudaStream_t s) {
   attr[0].id = cudaLaunchAttributeCooperative;     // the CTAs wait for one another
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = g.a.nb > 1 ? 1 : 0;
+  cfg.numAttrs = 1;
   ORCA_CUDA(cudaLaunchKernelEx(&cfg, gru_chain_kernel, g));
   ORCA_COUNT_LAUNCH();
-  if (g.a.nb > 1 && most > c->sm_count * 8) ORCA_CUDA(launch_dep(last_messages_kernel<1>, std::min(ceil_div(most, 8), c->sm_count * 6), 256, 0, s, g));
+  if (most > c->sm_count * 8) ORCA_CUDA(launch_dep(last_messages_kernel<1>, std::min(ceil_div(most, 8), c->sm_count * 6), 256, 0, s, g));
   else ORCA_CUDA(launch_dep(last_messages_kernel<4>, std::min(most, c->sm_count * 8), 128, 0, s, g));
-  ORCA_COUNT_LAUNCH();
-  ORCA_LAUNCH_CHECK();
-  return ORCA_OK;
-}
-
-int launch_gru_chain(const ChainArgs &g, cudaStream_t s) {
-  // as many row blocks as `launch` allows: a batch with more updates than rows takes another turn
-  return launch(g, ceil_div(2 * g.a.bs, 8), s);
-}
-
-__global__ void __launch_bounds__(256) scatter_updates_kernel(float *__restrict__ memory, const int32_t *__restrict__ node,
-                                                              const Counters *__restrict__ cnt, int cap,
-                                                              const float *__restrict__ rows) {
-  dep_trigger();
-  dep_wait();
-  const int t = threadIdx.x & 63, n = min(cap, cnt->n_win[0]);
-  for (int w = blockIdx.x * 4 + threadIdx.x / 64; w < n; w += gridDim.x * 4)
-    if (t < D / 4)
-      reinterpret_cast<float4 *>(memory + (size_t)node[w] * D)[t] = reinterpret_cast<const float4 *>(rows + (size_t)w * D)[t];
-}
-
-int launch_gru_single(const orca_memory_t &mem, const orca_gru_weights_t &w, const float *edge_table, const float *time_w,
-                      int b, const int32_t *d_node, const int32_t *d_other, const int32_t *d_eid, const float *d_t,
-                      Counters *d_cnt, void *d_image, float *d_rows, cudaStream_t s) {
-  ORCA_CHECK_ARG(w.Wg_chain != nullptr && w.bg != nullptr);
-  ChainArgs g{};
-  g.a.nb = 1, g.a.bs = g.a.b_last = b, g.a.n_nodes = mem.n_nodes, g.a.cnt = d_cnt;
-  // (every row is read from the memory table: its ids are its rows)
-  g.a.win_node = const_cast<int32_t *>(d_node), g.a.win_mem = const_cast<int32_t *>(d_node);
-  g.a.win_other = const_cast<int32_t *>(d_other), g.a.win_eid = const_cast<int32_t *>(d_eid);
-  g.a.win_t = const_cast<float *>(d_t);
-  g.mem = mem, g.log = mem.memory, g.log_out = d_rows, g.edge_table = edge_table, g.time_w = time_w;
-  g.w = w.Wg_chain, g.bias = w.bg, g.image = d_image;
-  // two fifths of the positions of a batch are winners, or fewer: as few row blocks as take those in one turn, since the
-  // launch runs beside the layers
-  return launch(g, ceil_div(2 * b * 2 / 5, ROWS), s);
-}
-
-int scatter_updates(const orca_memory_t &mem, const int32_t *d_node, const Counters *d_cnt, int cap, const float *d_rows,
-                    cudaStream_t s) {
-  ORCA_CUDA(launch_dep(scatter_updates_kernel, std::min(ceil_div(cap, 4), 592), 256, 0, s, mem.memory, d_node, d_cnt, cap,
-                       d_rows));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

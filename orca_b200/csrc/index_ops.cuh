@@ -29,16 +29,8 @@ int launch_uncached_finish(const orca_tgn_t *m, int n_query, int32_t *nodes_io, 
 
 // positions of the last occurrence of every id, in position order (single block; n up to a few
 // thousand); d_status (optional): the count is also written to status word 2
-// (u, optional: d_ids is a batch [src | dst | neg | edge ids], n = 2 * b, with times u.ts: the winners are also written
-// out as memory updates -- node, other endpoint, edge, time)
-struct UpdateList {
-  const double *ts = nullptr;
-  int32_t *node = nullptr, *other = nullptr, *eid = nullptr;
-  float *t = nullptr;
-};
 int launch_last_occ_compact(const int32_t *d_ids, int n, int64_t n_nodes, int64_t *d_last_pos, long long base,
-                            int32_t *d_compact, int32_t *d_n_compact, int32_t *d_status, cudaStream_t s,
-                            const UpdateList &u = UpdateList());
+                            int32_t *d_compact, int32_t *d_n_compact, int32_t *d_status, cudaStream_t s);
 
 // cache flags after a batch with a plan (History.update_flag): those of m->prev_plan cleared, those of d_plan set
 int launch_plan_flags(const orca_tgn_t *m, const int32_t *d_plan, int n_plan, cudaStream_t s);

@@ -28,7 +28,6 @@
 #include <vector>
 
 #include "attn_out.cuh"
-#include "chain.cuh"
 #include "common.cuh"
 #include "context.cuh"
 #include "gru_rows.cuh"
@@ -47,8 +46,6 @@ struct IdxBuf {
   int32_t *cat_dst; int32_t *win_pos; int32_t *n_win; int32_t *win_nodes;
   int32_t *loc_nodes; double *loc_ts; int32_t *n1_loc;               // sharded layer 1
   int32_t *feat_idx; int32_t *nbr2_loc, *eid2_loc; float *dt2_loc;  // sharded layer 2 / no-reuse index
-  int32_t *upd_node, *upd_other, *upd_eid; float *upd_t;   // memory updates of the batch (chain.cu)
-  grp::Counters *cnt;                                       // of which n_win[0] is their number
   int32_t *order1, *order2;                    // rows of the two gather launches, heaviest first
 };
 // projection / gather buffers of one attention layer in flight (one set per compute lane)
@@ -66,7 +63,6 @@ struct Workspace {
   float *emb2;
   uint8_t *win1;
   float *gru_h;
-  void *upd_image;           // split inputs of the memory updates (chain.cu)
   char *msg_image;           // operand image of the batch's messages (gru_rows.cu)
   void *bitmap;
   size_t bytes;
@@ -92,12 +88,7 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
     x.dt2 = (float *)take(N * k * 4);
     x.cat_dst = (int32_t *)take(2 * (size_t)b_cap * 4);
     x.win_pos = (int32_t *)take(2 * (size_t)b_cap * 4);
-    x.cnt = (grp::Counters *)take(sizeof(grp::Counters));
-    x.n_win = x.cnt != nullptr ? &x.cnt->n_win[0] : nullptr;
-    x.upd_node = (int32_t *)take(2 * (size_t)b_cap * 4);
-    x.upd_other = (int32_t *)take(2 * (size_t)b_cap * 4);
-    x.upd_eid = (int32_t *)take(2 * (size_t)b_cap * 4);
-    x.upd_t = (float *)take(2 * (size_t)b_cap * 4);
+    x.n_win = (int32_t *)take(4);
     x.win_nodes = (int32_t *)take(2 * (size_t)b_cap * 4);
     x.loc_nodes = (int32_t *)take(R1 * 4);
     x.loc_ts = (double *)take(R1 * 8);
@@ -123,15 +114,14 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
   w.emb2 = (float *)take(N * D * 4);
   w.win1 = (uint8_t *)take(R1);
   w.gru_h = (float *)take(2 * (size_t)b_cap * D * 4);
-  w.upd_image = take(grp::update_image_bytes(2 * (int64_t)b_cap));
   w.msg_image = (char *)take(gru_image_bytes(2 * (int64_t)b_cap));
   w.bitmap = take((size_t)orca_find_uncached_scratch_bytes(n_nodes));
   w.bytes = off;
   return w;
 }
 
-// nodes1[0..3b) = [src|dst|neg], ts1[r] = ts[r % b], cat_dst = [dst|src]
-__global__ void batch_prep_kernel(const int32_t *__restrict__ batch, const double *__restrict__ ts, int b,
+// nodes1[0..3b) = [src|dst|neg], ts1[r] = ts[r % b], cat_dst = [dst|src] (ids that the tables have no row for: 0)
+__global__ void batch_prep_kernel(const int32_t *__restrict__ batch, const double *__restrict__ ts, int b, int64_t n_nodes,
                                   int32_t *__restrict__ nodes1, double *__restrict__ ts1,
                                   int32_t *__restrict__ cat_dst, int32_t *__restrict__ n1) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,7 +129,10 @@ __global__ void batch_prep_kernel(const int32_t *__restrict__ batch, const doubl
     nodes1[i] = batch[i];
     ts1[i] = ts[i % b];
   }
-  if (i < 2 * b) cat_dst[i] = i < b ? batch[b + i] : batch[i - b];
+  if (i < 2 * b) {
+    const int other = i < b ? batch[b + i] : batch[i - b];
+    cat_dst[i] = other >= 0 && other < n_nodes ? other : 0;
+  }
   if (i == 0) *n1 = 3 * b;
 }
 
@@ -415,18 +408,6 @@ static int store_and_update(const orca_tgn_t *m, Workspace &w, IdxBuf &x, const 
                     : gru_project(&m->gru, &m->mem, x.win_nodes, 2 * b, x.n_win, w.gru_h, s);
 }
 
-// Raw messages and GRU of a batch by the memory chain's kernel (chain.cu), or as a pair of launches.  The chain's kernel
-// is the faster one where a batch's launches stand in one line (eval_serial; one layer, us a call, pair / chain: 37 edges
-// 100.5 / 97.5, 200 115 / 102.6, 500 128 / 117, 800 125 / 123, 1024 129 / 130), not in the lanes of a budgeted batch,
-// where it takes most of the chip while the layers beside it want it (200 edges 84.3 / 85.0, 500 84.7 / 86.5, 800 94.8 /
-// 100.5, 1024 104.7 / 111.2, 2000 147 / 154).  The fp32 projections take the pair.
-static bool one_launch_updates(int b) { return projections_on_tensor_cores() && b <= 1024; }
-static UpdateList updates_of(const IdxBuf &x, const double *d_ts) {
-  UpdateList u;
-  u.ts = d_ts, u.node = x.upd_node, u.other = x.upd_other, u.eid = x.upd_eid, u.t = x.upd_t;
-  return u;
-}
-
 static Ctx *ctx_of(const orca_tgn_t *m) {
   return m->ctx != nullptr ? reinterpret_cast<Ctx *>(m->ctx) : default_ctx();
 }
@@ -452,7 +433,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
   if (m->input_stream != nullptr) ORCA_TRY(link((cudaStream_t)m->input_stream, s, c->ev_in));
 
   ORCA_TRY(tr.mark(-1, s));
-  batch_prep_kernel<<<ceil_div(N, 256), 256, 0, s>>>(d_batch_i32, d_batch_ts, b, x.nodes1, x.ts1, x.cat_dst, x.n1);
+  batch_prep_kernel<<<ceil_div(N, 256), 256, 0, s>>>(d_batch_i32, d_batch_ts, b, m->n_nodes, x.nodes1, x.ts1, x.cat_dst, x.n1);
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   ORCA_TRY(tr.mark(PH_PREP, s));
@@ -460,26 +441,19 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
   cudaStream_t ms = beside ? c->aux : s;
   if (beside && m->n_layers == 1) ORCA_CUDA(cudaEventRecord(c->fork, s));
   // raw messages of the batch (last occurrence per node in [src|dst]) and the new memory rows
-  const bool single = one_launch_updates(b);
   auto update = [&]() -> int {
     if (beside) ORCA_CUDA(cudaStreamWaitEvent(ms, c->fork, 0));
     ORCA_TRY(launch_last_occ_compact(d_batch_i32, 2 * b, m->n_nodes, lp_msg, *m->epoch_base, x.win_pos, x.n_win,
-                                     d_status, ms, updates_of(x, d_batch_ts)));
+                                     d_status, ms));
     *m->epoch_base += 2 * b;
     ORCA_TRY(tr.mark(PH_LAST_OCC_MSG, s));
-    if (single) {
-      ORCA_TRY(grp::launch_gru_single(m->mem, m->gru, m->edge_table, m->time_w, b, x.upd_node, x.upd_other, x.upd_eid,
-                                      x.upd_t, x.cnt, w.upd_image, w.gru_h, ms));
-    } else {
-      ORCA_TRY(store_and_update(m, w, x, d_batch_i32, d_batch_ts, b, ms));
-    }
+    ORCA_TRY(store_and_update(m, w, x, d_batch_i32, d_batch_ts, b, ms));
     ORCA_TRY(tr.mark(PH_MESSAGE, s));
     return ORCA_OK;
   };
   // the memory table is written (layer 1 has read it)
   auto write_memory = [&]() -> int {
-    if (single) ORCA_TRY(grp::scatter_updates(m->mem, x.upd_node, x.cnt, 2 * b, w.gru_h, ms));
-    else ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, ms));
+    ORCA_TRY(gru_scatter(&m->mem, x.win_nodes, 2 * b, x.n_win, 1, w.gru_h, ms));
     ORCA_TRY(tr.mark(PH_GRU, s));
     return ORCA_OK;
   };

@@ -470,7 +470,7 @@ compact_flags_kernel(const uint8_t *__restrict__ is_last, int n_cap, const int32
 __global__ void __launch_bounds__(1024)
 last_occ_compact_kernel(const int32_t *__restrict__ ids, int n, int64_t n_nodes,
                         unsigned long long *__restrict__ last_pos, long long base,
-                        int32_t *__restrict__ compact, int32_t *__restrict__ n_compact, int32_t *status, UpdateList up) {
+                        int32_t *__restrict__ compact, int32_t *__restrict__ n_compact, int32_t *status) {
   __shared__ int s_scan[32];
   __shared__ int s_base;
   const int tid = threadIdx.x;
@@ -530,17 +530,7 @@ last_occ_compact_kernel(const int32_t *__restrict__ ids, int n, int64_t n_nodes,
       }
       __syncthreads();
       const int pos = s_base + s_scan[tid >> 5] + incl - f[u];
-      if (f[u]) {
-        const int i = i0 + u * 1024 + tid;
-        compact[pos] = i;
-        if (up.node != nullptr) {
-          const int b = n / 2, other = ids[i < b ? i + b : i - b];
-          up.node[pos] = ids[i];
-          up.other[pos] = other >= 0 && other < n_nodes ? other : 0;
-          up.eid[pos] = ids[3 * b + i % b];
-          up.t[pos] = (float)up.ts[i % b];
-        }
-      }
+      if (f[u]) compact[pos] = i0 + u * 1024 + tid;
       __syncthreads();
       if (tid == 1023) s_base = pos + f[u];
       __syncthreads();
@@ -612,10 +602,9 @@ int launch_uncached_finish(const orca_tgn_t *m, int n_query, int32_t *nodes_io, 
 }
 
 int launch_last_occ_compact(const int32_t *d_ids, int n, int64_t n_nodes, int64_t *d_last_pos, long long base,
-                            int32_t *d_compact, int32_t *d_n_compact, int32_t *d_status, cudaStream_t s,
-                            const UpdateList &u) {
+                            int32_t *d_compact, int32_t *d_n_compact, int32_t *d_status, cudaStream_t s) {
   ORCA_CUDA(launch_dep(last_occ_compact_kernel, 1, 1024, 0, s, d_ids, n, n_nodes,
-                       reinterpret_cast<unsigned long long *>(d_last_pos), base, d_compact, d_n_compact, d_status, u));
+                       reinterpret_cast<unsigned long long *>(d_last_pos), base, d_compact, d_n_compact, d_status));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

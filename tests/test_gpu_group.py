@@ -104,6 +104,11 @@ def test_rows_that_share_features_equal_batches(budget, chunks):
     assert torch.equal(m.embedding_module.histories[0].emb, b.embedding_module.histories[0].emb)
 
 
+def test_groups_of_one_large_batch_equal_batches():
+    """A batch that fills a group alone, with enough updates that the last of every node leave the memory chain."""
+    test_group_equals_batches("c1", 9000, 10, 18500, "budget", 2)
+
+
 def test_a_stream_that_fails_leaves_a_model_that_works(monkeypatch):
     """A stream can fail in the middle -- here an id that cannot be packed, in the third group, and a workspace that
     cannot be allocated.  What was enqueued has finished when the error is raised, and the next stream runs as on a
