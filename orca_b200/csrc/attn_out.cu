@@ -44,6 +44,8 @@ constexpr int TMEM_COLS = 512, SMALL = 256;
 
 using img::desc_sw64;
 
+// PAIRS: the top layer, whose rows go where the pairs that are scored want them (and to g.out, if given)
+template <bool PAIRS>
 __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __grid_constant__ OutArgs g) {
   using namespace tc;
   extern __shared__ unsigned char raw[];
@@ -186,9 +188,14 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
     for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x, ++t) {
       const int m0 = blk * BM, m_rows = min(BM, M - m0);
       const float on = (row < m_rows && (g.valid == nullptr || g.valid[m0 + row] != 0)) ? 1.f : 0.f;
-      // history push: lane i holds what row ew + 8 * i of the output pass needs
+      // lane i holds what row ew + 8 * i of the output pass needs: history push; or the row's (first) pair, and how much
+      // further its second one is (0: it is a destination or negative, the second of one pair)
       int push_id = 0, push = 0;
-      if (g.push_table != nullptr && lane < BM / EPI_WARPS && ew + EPI_WARPS * lane < m_rows) {
+      if (PAIRS) {
+        const int m = m0 + ew + EPI_WARPS * (lane & 15), n = m / (3 * g.pair_bs), i = m - n * 3 * g.pair_bs;
+        const int b = n == g.pair_nb - 1 ? g.pair_last : g.pair_bs;
+        push_id = n * 2 * g.pair_bs + (i < b ? i : i - b), push = i < b ? b : 0;
+      } else if (g.push_table != nullptr && lane < BM / EPI_WARPS && ew + EPI_WARPS * lane < m_rows) {
         const int m = m0 + ew + EPI_WARPS * lane;
         push_id = g.push_ids[m];
         push = g.push_win != nullptr ? g.push_win[m]
@@ -293,12 +300,39 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
             *reinterpret_cast<float4 *>(o + 4 * lane) = ya;
             if (has1) *reinterpret_cast<float4 *>(o + 4 * lane + 128) = yb;
           };
+          // heads and tails of the lane's columns; behind the row, the padding
+          uint2 hiA, loA, hiB, loB;
+          auto pack = [](float4 x, uint2 &hi, uint2 &lo) {
+            hi.x = pack_split(x.x, x.y, lo.x);
+            hi.y = pack_split(x.z, x.w, lo.y);
+          };
+          // (img::at, with the row's part taken out)
+          auto put = [&](char *row, int sw, int c, bool second) {
+            auto at = [&](int x) { return row + (((x >> 5) * A_STAGE + (x >> 3 & 3) * 16 + 2 * (x & 7)) ^ sw); };
+            char *p = at(c), *q = at(c + 128);
+            *reinterpret_cast<uint2 *>(p) = hiA;
+            *reinterpret_cast<uint2 *>(p + A_STAGE / 2) = loA;
+            if (second) {
+              *reinterpret_cast<uint2 *>(q) = hiB;
+              *reinterpret_cast<uint2 *>(q + A_STAGE / 2) = loB;
+            }
+          };
+          if (PAIRS || m0 + r < g.out_image_rows) pack(ya, hiA, loA), pack(has1 ? yb : f4z, hiB, loB);
+          if (PAIRS) {
+            if (g.out != nullptr) store(g.out + (size_t)(m0 + r) * D);
+            const int second = win == 0;
+            auto to_pair = [&](int pair) {
+              put(g.pair_image + (size_t)(pair / img::ROWS) * (img::PAIR_STAGES * A_STAGE) + (pair % img::ROWS) * 64, (pair << 3) & 0x30,
+                  4 * lane + second * D, lane < D / 4 - 32 + 2 * second);
+            };
+            to_pair(to);
+            if (!second) to_pair(to + win);
+            continue;
+          }
           store(g.out + (size_t)(m0 + r) * D);
           if (g.push_table != nullptr && win != 0) store(g.push_table + (size_t)to * D);
-          if (m0 + r < g.out_image_rows) {     // (columns 172 .. 191 are padding)
-            img::put4<img::FEAT_STAGES>(g.out_image, m0 + r, 4 * lane, ya);
-            if (lane < 16) img::put4<img::FEAT_STAGES>(g.out_image, m0 + r, 128 + 4 * lane, has1 ? yb : f4z);
-          }
+          if (m0 + r < g.out_image_rows)     // (columns 172 .. 191 are padding)
+            put(g.out_image + (size_t)blk * (img::FEAT_STAGES * A_STAGE) + r * 64, (r << 3) & 0x30, 4 * lane, lane < 16);
           // multi-GPU exchange: the row also goes to every rank's exchange buffer (peer stores)
           for (int q = 0; q < g.peer.world; ++q) store(g.peer.rows[q] + g.peer.off + (size_t)(m0 + r) * D);
         }
@@ -312,7 +346,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
-  if (g.peer.world > 0) {
+  if (!PAIRS && g.peer.world > 0) {
     // every CTA (with or without rows) checks out; the last one posts the batch's sequence number to all ranks, after
     // every CTA's peer stores have been fenced system-wide
     __threadfence_system();
@@ -333,17 +367,22 @@ int attn_output_rows(const OutArgs &args, cudaStream_t s) {
   if (args.n_cap <= 0) return ORCA_OK;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "attn_output_rows: no context for the current device");
-  ORCA_CHECK_ARG(args.w.G_img && args.w.W2_img && args.ctx && args.own && args.out);
+  ORCA_CHECK_ARG(args.w.G_img && args.w.W2_img && args.ctx && args.own && (args.out || args.pair_image));
+  // (the top layer of one GPU: no push, no image of its own, no delivery)
+  ORCA_CHECK_ARG(args.pair_image == nullptr || (args.push_table == nullptr && args.out_image_rows == 0 && args.peer.world == 0));
+  ORCA_CHECK_ARG(args.pair_image == nullptr || (args.pair_bs > 0 && args.pair_nb > 0 && args.pair_last > 0 && args.pair_last <= args.pair_bs));
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(ao::attn_output_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ao::SMEM));
+    ORCA_CUDA(cudaFuncSetAttribute(ao::attn_output_image_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ao::SMEM));
+    ORCA_CUDA(cudaFuncSetAttribute(ao::attn_output_image_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ao::SMEM));
     configured_device = c->device;
   }
   OutArgs g = args;
   g.status = c->status_word;
   g.wait_limit = c->wait_limit;
   const int grid = std::min(ceil_div(g.n_cap, ao::BM), c->sm_count);
-  ORCA_CUDA(launch_dep(ao::attn_output_image_kernel, grid, ao::THREADS, ao::SMEM, s, g));
+  ORCA_CUDA(launch_dep(g.pair_image != nullptr ? ao::attn_output_image_kernel<true> : ao::attn_output_image_kernel<false>, grid,
+                       ao::THREADS, ao::SMEM, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

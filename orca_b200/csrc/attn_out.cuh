@@ -18,6 +18,7 @@ constexpr int ROWS = 128;
 constexpr int STAGE_K = 32;
 constexpr int STAGE_BYTES = 2 * ROWS * STAGE_K * 2;
 constexpr int FEAT_STAGES = 6, CTX_STAGES = 33;
+constexpr int PAIR_STAGES = 11;     // two embeddings one after the other, 344 columns, padded to 352 (score_rows.cu)
 inline size_t bytes(int64_t rows, int stages) { return (size_t)((rows + ROWS - 1) / ROWS) * stages * STAGE_BYTES; }
 
 // columns c .. c + 3 / c, c + 1 of row r: heads, and tails half a stage further
@@ -58,9 +59,13 @@ struct OutArgs {
   const uint8_t *valid;       // rows whose slots are all padding have no attention term
   int n_cap;
   const int32_t *d_n;
-  float *out;                 // [rows, 172]
+  float *out;                 // [rows, 172]; may be nullptr where pair_image is not
   char *out_image;            // optional: operand image of the first out_image_rows rows (the next layer's features)
   int out_image_rows;
+  // optional: operand image of the pairs that are scored.  The rows are [src | dst | neg] of pair_nb batches of pair_bs edges
+  // (the last one: pair_last), the pairs [positive | negative] of batch n from n * 2 * pair_bs on.
+  char *pair_image;
+  int pair_bs, pair_nb, pair_last;
   // optional history push: winners by flag, or (push_win == nullptr) by record: row m wins if m >= push_all_from or
   // push_last_pos[push_ids[m]] == push_base + m
   float *push_table;
@@ -79,5 +84,7 @@ int feat_image(const tc::RowSrc &feat, int n_cap, const int32_t *d_n, char *d_im
 int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_cap, const int32_t *d_n, float *d_qt,
                      float *d_own, cudaStream_t s);
 int attn_output_rows(const OutArgs &g, cudaStream_t s);
+// scores of pairs that lie in an operand image
+int score_rows(const orca_score_weights_t *w, const char *d_pairs, int pairs, float *d_prob, cudaStream_t s);
 
 }  // namespace orca

@@ -418,7 +418,7 @@ static inline int kblocks(int k) { return (k + tc::BK - 1) / tc::BK; }
 
 namespace orca {
 
-// Arguments of the tensor-core projections (score_rows serves a group of batches, group.cu).
+// Arguments of the tensor-core projections.
 static tc::Args output_args(const orca_attn_weights_t *w, const float *d_ctx, const uint8_t *d_valid,
                             const tc::RowSrc &feat, int n_cap, const int32_t *d_n, float *d_out) {
   tc::Args a{};
@@ -453,13 +453,6 @@ static tc::Args score_args(const orca_score_weights_t *w, const float *d_emb, in
   a.b2 = w->b2;
   a.out = d_prob;
   return a;
-}
-int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
-               float *d_prob, cudaStream_t s) {
-  tc::Args a = score_args(w, d_emb, rows, d_prob);
-  a.a0.idx = d_a;
-  a.a1.idx = d_b;
-  return tc::launch(tc::EPI_SCORE, a, 1, s);
 }
 static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, const int32_t *d_nodes, int n_cap,
                          const int32_t *d_n, float *d_out) {

@@ -304,22 +304,17 @@ __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ Ar
   }
   const int per = 2 * a.bs;
   for (int i = tid; i < a.nb * per; i += step) {
-    const int n = i / per, r = i - n * per, b = a.b_of(n);
-    if (a.is_update(n, r)) {
-      const int v = a.win_node[i], row = memory_row_early(a, v, n);
-      if (!a.again(v, n)) {
-        const int l = place(&a.cnt->n_last, 0);
-        a.last_at[l] = i;
-        a.last_node[l] = v;
-      }
-      a.win_mem[i] = row;
-      a.win_gap[i] = a.win_t[i] - last_update_of(a, last_update, v, row);
-      a.win_other[i] = memory_row_early(a, a.win_other[i], n);
+    const int n = i / per;
+    if (!a.is_update(n, i - n * per)) continue;
+    const int v = a.win_node[i], row = memory_row_early(a, v, n);
+    if (!a.again(v, n)) {
+      const int l = place(&a.cnt->n_last, 0);
+      a.last_at[l] = i;
+      a.last_node[l] = v;
     }
-    if (r < 2 * b) {     // score r of batch n pairs source r % b with destination r or negative r - b
-      a.score0[i] = 3 * n * a.bs + r % b;
-      a.score1[i] = 3 * n * a.bs + b + r;
-    }
+    a.win_mem[i] = row;
+    a.win_gap[i] = a.win_t[i] - last_update_of(a, last_update, v, row);
+    a.win_other[i] = memory_row_early(a, a.win_other[i], n);
   }
 }
 
@@ -471,7 +466,7 @@ struct Parity {
   unsigned long long *app_table;
   Counters *cnt;
   size_t zero_bytes;       // bits, tables and counters are zeroed together, from `bits`
-  int32_t *cand, *app_node, *nbr1, *eid1, *nbr2, *own1, *own_seen, *own_list, *own_at, *score0, *score1;
+  int32_t *cand, *app_node, *nbr1, *eid1, *nbr2, *own1, *own_seen, *own_list, *own_at;
   float *dt1;
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;
@@ -483,8 +478,9 @@ struct Buffers {
   Parity par[2];
   float *log;              // two parities, one after the other
   char *msg_image;         // of the messages of every node's last update (groups whose last updates leave the chain)
-  float *qt, *own, *emb1, *emb2;
-  char *ctx, *feat, *feat2;   // operand images (attn_out.cuh): attention sums, own features, layer 2's own features
+  float *qt, *own, *emb1;
+  // operand images (attn_out.cuh): attention sums, own features, layer 2's own features, pairs that are scored
+  char *ctx, *feat, *feat2, *pairs;
   uint8_t *valid;
   uint32_t table_size, app_size;
   int64_t rows_max;        // layer-1 rows a group can have
@@ -522,8 +518,6 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
     x.own1 = (int32_t *)take((size_t)w.rows_max * 4);
     x.own_list = (int32_t *)take((size_t)w.rows_max * 4);
     x.own_at = (int32_t *)take((size_t)w.rows_max * 4);
-    x.score0 = (int32_t *)take((size_t)2 * E * 4);
-    x.score1 = (int32_t *)take((size_t)2 * E * 4);
     x.win_node = (int32_t *)take((size_t)2 * E * 4);
     x.win_eid = (int32_t *)take((size_t)2 * E * 4);
     x.win_mem = (int32_t *)take((size_t)2 * E * 4);
@@ -544,7 +538,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
   w.feat2 = (char *)take(layers == 2 ? img::bytes(batch_rows, img::FEAT_STAGES) : 4);
   w.valid = (uint8_t *)take((size_t)w.chunk);
   w.emb1 = (float *)take((size_t)w.rows_max * D * 4);
-  w.emb2 = (float *)take(layers == 2 ? (size_t)batch_rows * D * 4 : 4);
+  w.pairs = (char *)take(img::bytes(2 * E, img::PAIR_STAGES));
   w.total = off;
   return w;
 }
@@ -654,7 +648,6 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
   if (g->seq > 0) a.prev_bits = prev.bits, a.prev_table = prev.table, a.prev_mask = w.table_size - 1;
   a.cand = x.cand, a.app_node = x.app_node, a.nbr1 = x.nbr1, a.eid1 = x.eid1, a.dt1 = x.dt1, a.nbr2 = x.nbr2;
   a.own1 = x.own1, a.own_seen = x.own_seen, a.own_list = x.own_list, a.own_at = x.own_at;
-  a.score0 = x.score0, a.score1 = x.score1;
   a.win_node = x.win_node, a.win_eid = x.win_eid, a.win_mem = x.win_mem, a.win_other = x.win_other, a.win_t = x.win_t, a.win_gap = x.win_gap;
   a.last_at = x.last_at, a.last_node = x.last_node;
   a.split = 2 * E > grp::SPLIT_FROM;
@@ -715,6 +708,7 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
     auto output = [&](int layer, int rows, const int32_t *own_row, float *out) {
       OutArgs o{};
       o.w = m->attn[layer], o.ctx = w.ctx, o.own = w.own, o.own_row = own_row, o.valid = w.valid, o.n_cap = rows, o.out = out;
+      if (layer == layers - 1) o.pair_image = w.pairs, o.pair_bs = g->bs, o.pair_nb = g->nb, o.pair_last = g->b_last;
       return o;
     };
     // (a group with a cold cache, whose rows take several chunks, goes without sharing)
@@ -728,22 +722,19 @@ int orca_tgn_eval_group(const orca_tgn_t *m, const orca_group_t *g, void *d_work
       ORCA_TRY(attn_query_image(&m->attn[0], w.feat, rows, d_own, w.qt, w.own, s));
       ORCA_TRY(launch_attn_gather(w.qt, m->mem.memory, m->edge_table, m->time_w, x.nbr1 + slot, x.eid1 + slot, x.dt1 + slot, k,
                                   rows, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, log, (int)m->n_nodes, own_at));
-      OutArgs o = output(0, rows, own_at, w.emb1 + (size_t)r0 * D);
+      OutArgs o = output(0, rows, own_at, layers == 2 ? w.emb1 + (size_t)r0 * D : nullptr);
       // (the batch rows are layer 2's rows; they all lie in the first chunk)
       if (layers == 2 && r0 == 0) o.out_image = w.feat2, o.out_image_rows = 3 * E;
       ORCA_TRY(attn_output_rows(o, s));
     }
-    const float *top = w.emb1;
     if (layers == 2) {
       ORCA_TRY(attn_query_image(&m->attn[1], w.feat2, 3 * E, nullptr, w.qt, w.own, s));
       // (without reuse every row lies in the layer-1 output: the first part is never read)
       ORCA_TRY(launch_attn_gather(w.qt, history ? m->hist_emb : m->mem.memory, m->edge_table, m->time_w, x.nbr2, x.eid1,
                                   x.dt1, k, 3 * E, nullptr, 0, nullptr, w.ctx, true, w.valid, tk, s, emb, (int)m->n_nodes));
-      ORCA_TRY(attn_output_rows(output(1, 3 * E, nullptr, w.emb2), s));
-      top = w.emb2;
+      ORCA_TRY(attn_output_rows(output(1, 3 * E, nullptr, nullptr), s));
     }
-    // (positions of a short last batch's scores: the arrays are indexed by 2 * bs per batch, only the last is short)
-    ORCA_TRY(score_rows(&m->score, top, x.score0, x.score1, 2 * E, d_prob, s));
+    ORCA_TRY(score_rows(&m->score, w.pairs, 2 * E, d_prob, s));
     ORCA_CUDA(launch_dep(grp::write_back_kernel, c->sm_count * 8, 256, 0, s, a, log, (const float *)w.emb1, m->mem.memory,
                          m->hist_emb, g->h_status));
     ORCA_COUNT_LAUNCH();

@@ -70,7 +70,6 @@ struct Args {
   int32_t *own1;                    // row of (memory table | log) of the row's own node
   int32_t *own_seen;                // by row of (memory table | log): 1 + its place in own_list, 0: not there
   int32_t *own_list, *own_at;       // the distinct rows of own1, and own1's places in the list
-  int32_t *score0, *score1;         // the two embeddings of every score
   // memory updates: batch n's at n * 2 * bs (Counters says which of these places are taken)
   int32_t *win_node, *win_eid, *win_mem, *win_other;
   float *win_t, *win_gap;           // time of the update, and since the node's update before it

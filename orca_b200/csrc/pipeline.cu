@@ -61,6 +61,7 @@ struct Workspace {
   float *emb1[2];
   char *feat2[2];            // operand image of layer 2's own features, written by layer 1 (one GPU)
   float *emb2;
+  char *pairs;               // operand image of the pairs that are scored
   uint8_t *win1;
   float *gru_h;
   char *msg_image;           // operand image of the batch's messages (gru_rows.cu)
@@ -112,6 +113,7 @@ static Workspace carve(void *base, int b_cap, int u_cap, int k, int64_t n_nodes)
   for (int q = 0; q < 2; ++q) w.emb1[q] = (float *)take(R1 * D * 4);
   for (int q = 0; q < 2; ++q) w.feat2[q] = (char *)take(img::bytes(N, img::FEAT_STAGES));
   w.emb2 = (float *)take(N * D * 4);
+  w.pairs = (char *)take(img::bytes(2 * (int64_t)b_cap, img::PAIR_STAGES));
   w.win1 = (uint8_t *)take(R1);
   w.gru_h = (float *)take(2 * (size_t)b_cap * D * 4);
   w.msg_image = (char *)take(gru_image_bytes(2 * (int64_t)b_cap));
@@ -383,7 +385,8 @@ struct Push {      // optional history push (OutArgs); win: flags, or scratch of
 };
 static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d_feat, const int32_t *d_idx, int cap,
                         const int32_t *d_n, float *d_out, const Push &push, cudaStream_t s,
-                        const tc::PeerOut *peer = nullptr, char *d_image = nullptr, int image_rows = 0) {
+                        const tc::PeerOut *peer = nullptr, char *d_image = nullptr, int image_rows = 0,
+                        char *d_pairs = nullptr) {
   if (!projections_on_tensor_cores())
     return attn_output_impl(w, (const float *)l.ctx, l.valid, d_feat, d_idx, cap, d_n, d_out, push.table, push.ids,
                             push.win, push.last_pos, push.base, push.all_from, l.hidden, s);
@@ -394,7 +397,23 @@ static int layer_output(const orca_attn_weights_t *w, LaneBuf &l, const float *d
   a.push_base = push.base, a.push_all_from = push.all_from;
   if (peer != nullptr) a.peer = *peer;
   a.out_image = d_image, a.out_image_rows = d_image != nullptr ? image_rows : 0;
+  a.pair_image = d_pairs, a.pair_bs = a.pair_last = cap / 3, a.pair_nb = 1;
   return attn_output_rows(a, s);
+}
+// The top layer's output and the scores of its b edges (cap = 3 b rows): with the fp32 projections from the embeddings, which
+// lie in scratch memory where the caller has no use for them.
+static int top_output(const orca_tgn_t *m, int layer, LaneBuf &l, const float *d_feat, const int32_t *d_idx, int b, Workspace &w,
+                      float *d_emb_out, cudaStream_t s) {
+  const bool image = projections_on_tensor_cores();
+  return layer_output(&m->attn[layer], l, d_feat, d_idx, 3 * b, nullptr, d_emb_out != nullptr || image ? d_emb_out : w.emb2, Push{}, s,
+                      nullptr, nullptr, 0, image ? w.pairs : nullptr);
+}
+static int top_scores(const orca_tgn_t *m, Workspace &w, const float *d_emb_out, int b, float *d_prob, cudaStream_t s) {
+  if (projections_on_tensor_cores()) {
+    ORCA_CHECK_ARG(m->score.W1t != nullptr);      // (as orca_score asks)
+    return score_rows(&m->score, w.pairs, 2 * b, d_prob, s);
+  }
+  return orca_score(&m->score, d_emb_out != nullptr ? d_emb_out : w.emb2, b, d_prob, s);
 }
 
 // raw messages of a batch and its new memory rows, to w.gru_h, as a pair of launches
@@ -458,7 +477,6 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     return ORCA_OK;
   };
 
-  float *emb_top = d_emb_out ? d_emb_out : w.emb2;
   if (m->n_layers == 1) {
     ORCA_TRY(launch_sample_rows(m, x.nodes1, x.ts1, N, nullptr, x.nbr1, x.eid1, x.dt1, d_status, s));
     ORCA_TRY(tr.mark(PH_SAMPLE_TOP, s));
@@ -468,7 +486,7 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     ORCA_TRY(tr.mark(PH_GATHER_L2, s));
     // (given to the GPU now: the layer's first kernels come before it, its longest one beside it)
     if (beside) ORCA_TRY(update());
-    ORCA_TRY(layer_output(&m->attn[0], l, m->mem.memory, x.nodes1, N, nullptr, emb_top, Push{}, s));
+    ORCA_TRY(top_output(m, 0, l, m->mem.memory, x.nodes1, b, w, d_emb_out, s));
     ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
     if (beside) {
       ORCA_TRY(link(s, ms, c->ev_o1));
@@ -523,10 +541,10 @@ static int eval_serial(const orca_tgn_t *m, Ctx *c, const int32_t *d_batch_i32, 
     ORCA_TRY(tr.mark(PH_QUERY_L2, s));
     ORCA_TRY(layer_gather(m, table2, gather2, x.eid2, x.dt2, N, nullptr, 0, nullptr, l2, tk, s));
     ORCA_TRY(tr.mark(PH_GATHER_L2, s));
-    ORCA_TRY(layer_output(&m->attn[1], l2, w.emb1[0], nullptr, N, nullptr, emb_top, Push{}, s));
+    ORCA_TRY(top_output(m, 1, l2, w.emb1[0], nullptr, b, w, d_emb_out, s));
     ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
   }
-  ORCA_TRY(orca_score(&m->score, emb_top, b, d_prob, s));
+  ORCA_TRY(top_scores(m, w, d_emb_out, b, d_prob, s));
   ORCA_TRY(tr.mark(PH_SCORE, s));
 
   if (!beside || m->n_layers == 2) {
@@ -817,7 +835,6 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
     }
     if (rows2 > 0) {
       ORCA_CHECK_ARG(d_prob != nullptr);
-      float *emb_top = d_emb_out ? d_emb_out : w.emb2;
       ORCA_TRY(layer_query(&m->attn[1], feat2, feat2_idx, rows2, nullptr, l2, s, !sharded));
       ORCA_TRY(tr.mark(PH_QUERY_L2, s));
       ORCA_TRY(layer_gather(m, m->hist_emb, nbr2, eid2, dt2, rows2, nullptr, 0, x.order2, l2,
@@ -827,9 +844,9 @@ static int eval_budget(const orca_tgn_t *m, Ctx *c, int phases, const int32_t *d
         ORCA_CUDA(cudaEventRecord(c->ev_g2, s));
         c->g2_recorded = true;
       }
-      ORCA_TRY(layer_output(&m->attn[1], l2, feat2, feat2_idx, rows2, nullptr, emb_top, Push{}, s));
+      ORCA_TRY(top_output(m, 1, l2, feat2, feat2_idx, b2, w, d_emb_out, s));
       ORCA_TRY(tr.mark(PH_OUTPUT_L2, s));
-      ORCA_TRY(orca_score(&m->score, emb_top, b2, d_prob, s));
+      ORCA_TRY(top_scores(m, w, d_emb_out, b2, d_prob, s));
       ORCA_TRY(tr.mark(PH_SCORE, s));
     }
     // the batch is complete on the caller's stream once the other lanes' parts of it are

@@ -119,9 +119,6 @@ int attn_output_impl(const orca_attn_weights_t *w, const float *d_ctx, const uin
                      float *d_push_table, const int32_t *d_push_ids, const uint8_t *d_push_win,
                      const int64_t *d_last_pos, long long base, int all_from, float *d_scratch_hidden,
                      cudaStream_t stream);
-// scorer over the rows of a group of batches (gemm.cu); tensor cores only
-int score_rows(const orca_score_weights_t *w, const float *d_emb, const int32_t *d_a, const int32_t *d_b, int rows,
-               float *d_prob, cudaStream_t s);
 // whether the projections run on the tensor cores (orca_set_projection_mode(0)); the fp32 debug path has
 // no peer fan-out
 bool projections_on_tensor_cores();

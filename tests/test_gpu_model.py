@@ -903,3 +903,24 @@ def test_updates_of_a_batch_against_64_bits(b):
 def _two_layer_model(g, bs):
     import dataclasses
     return make_model(dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=bs, n_layers=2, n_degree=10, budget=20)))
+
+
+@pytest.mark.parametrize("layers", [1, 2])
+@pytest.mark.parametrize("b", [1, 63, 64, 65, 128, 129, 300])
+def test_scores_of_a_batch_are_those_of_its_embeddings(layers, b):
+    """The pairs' operand image that the top layer leaves for the scorer, at its blocks' edges: the scores of a batch are bit
+    for bit orca_score's of the embeddings that the same batch returns on a second model."""
+    import dataclasses
+    from orca_b200 import _lib
+    g = graph("c1")
+    g = dataclasses.replace(g, spec=dataclasses.replace(g.spec, bs=b, n_layers=layers, n_degree=10, budget=20))
+    a, e = make_model(g), make_model(g)
+    lo = len(g.sources) // 2
+    part = [x[lo:lo + b] for x in (g.sources, g.destinations, np.roll(g.destinations, 7), g.timestamps, g.edge_idxs)]
+    plan = np.unique(part[0])[:20] if layers == 2 else None
+    pos, neg = a.compute_edge_probabilities(*part, 10, True, False, plan)
+    emb = torch.cat(e.compute_temporal_embeddings(*part, 10, True, False, plan)).contiguous()
+    want = torch.empty(2 * b, device=emb.device)
+    _lib.check(_lib.lib().orca_score(e.score_struct(), emb.data_ptr(), b, want.data_ptr(), _lib.stream_ptr(emb.device)))
+    a.check_status(), e.check_status()
+    assert torch.equal(torch.cat([pos, neg]).ravel(), want)
