@@ -7,13 +7,17 @@
 // of 32 K columns (16 KB of rows + 22 KB of weights) through a ring of three (of five for the first product of a CTA's
 // first block, while the room of the hidden tile is still unused: a launch of few blocks waits for these loads), one
 // thread multiplies, eight warps do the two epilogues -- of one row block while the stages of the next are already
-// landing.  A block of 128 rows takes 33 + 6
-// stages of 6 MMAs and 1.4 MB from L2.  The general projection kernel, whose producer warps
-// load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks; 51 k
-// rows: 145 us with it, 82 to 86 here, where the bound is what L2 gives all SMs together, 7.3 TB/s, 58 % of it weights
-// (tensor pipe 42 %, DRAM 41 %): five slots instead of three gain nothing.  Pairs of CTAs with half of the weights each
-// (cta_group::2) take 72 us, but wait for two free SMs side by side: 50 batches of 2000 1.2 % faster, single calls of 3000
-// and 4000 edges with 20 neighbours 13 and 8 % slower.
+// landing.  A block of 128 rows takes 33 + 6 stages of 6 MMAs and 1.4 MB.  The general projection kernel, whose producer
+// warps load fp32 rows, convert and store them stage by stage, takes 49 us per block whatever the number of blocks.
+// 66 k rows, 104 us: the first block's stages come at the pace of their MMAs (0.32 us), which read their operands from
+// shared memory, later ones at 0.6 us, since all SMs read their rows from DRAM at once (rows from L2: 12 % less; without
+// the weights' copies: the same).  A block is 20 us of that, 1 for the hidden tile, 2 for the second product, 0.5 for the
+// accumulators' way out; LayerNorm and stores run beside the next block's stages.
+// Measured instead: five slots with a LayerNorm in registers, 98 us alone, but streams 3 to 4 % slower and a single call's
+// launch 5 us longer (an unrolled epilogue runs once, from a cold instruction cache); pairs of CTAs with half of the weights
+// each (cta_group::2), which wait for two free SMs side by side: 50 batches of 2000 1.2 % faster, single calls of 3000 and
+// 4000 edges with 20 neighbours 13 and 8 % slower; a row block on a cluster of two or four CTAs that share the columns:
+// one block 27 -> 33 us, 36 blocks 29 -> 34 and 58 (a block waits for its chain of dependent stages, not for their width).
 // Between the two products the hidden tile stays on the SM (bias + ReLU, split, A image of the second product), and
 // the second product's accumulators reuse the first one's columns.
 // Warp 0: copies.  Warp 1: tensor memory, MMA issue.  Warps 2-9: epilogues (thread = row, then warp = row).

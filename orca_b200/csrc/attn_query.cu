@@ -8,8 +8,9 @@
 // tensor memory to the outputs, in whole lines through shared memory.  6 / 31 / 66 k rows: 16 / 55 / 106 us (qt alone,
 // tiles of 176 columns: 14 / 50 / 92).  A group's layer 1, where 0.18 to 0.48 of the rows are distinct, asks for those
 // only (66 k rows of the largest graph: 92 -> 51 us, 57 k of 600-edge batches 75 -> 20), and the output kernel leaves six of
-// its 39 stages out.  What bounds it: 4.8 us a block and CTA against 1.8 of products; without the stores 92 us, without the
-// reading of the accumulators 102, with rows from L2 100.
+// its 39 stages out.  What bounds it: 4.8 us a block and CTA against 2 of products; without the stores 66 us, stores alone 48.
+// Measured instead, 6 / 31 / 66 k rows: pairs of CTAs with half of a tile of 224 columns each and six stages 22 / 71 / 141;
+// stores of fragments without the boxes, five stages, 18 / 53 / 95; stores of the boxes by tensor map 16 / 53 / 104.
 // orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
 // for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
 #include <algorithm>

@@ -467,7 +467,6 @@ static tc::Args gru_args(const orca_gru_weights_t *w, const orca_memory_t *mem, 
   a.bias = w->bg;
   a.out = d_out;
   a.memory = mem->memory;
-  a.memory_ld = D;
   a.nodes = d_nodes;
   return a;
 }

@@ -408,11 +408,12 @@ static inline uint32_t pow2_at_least(uint64_t x) {
 // batch), is not hidden by anything, so that group is half as large (two blocks per SM; where the chain matters, that is not
 // without reuse), and the rest is dealt out evenly.  us for a stream of 600 x K 20 / 1000 / 2000 edges a batch / without
 // reuse / 40 x 200, by rows of a group and of the first, 148 SMs:
-//   48 k, one after the other  2862 / 2859 / 5492 / 2247 / 1742      76 k so           2972 / 2808 / 5312 / 1987 / 1743
-//   57 k and 38 k              2819 / 2828 / 5311 / 2103 / 1620      76 k and 19 k     2856 / 2833 / 5309 / 2008 / 1621
-//   76 k and 38 k              2814 / 2837 / 5351 / 2011 / 1621      76 k and 57 k     2853 / 2895 / 5441 / 2013 / 1620
-//   95 k and 38 k              2811 / 2831 / 5274 / 2015 / 1622
-// (Device memory of a group's buffers at 2000 edges a batch, K 10: 2.4 GB, half of it queries and attention sums.)
+//   57 k, one after the other  2280 / 2403 / 4587 / 1634 / 1566      76 k so           2274 / 2295 / 4538 / 1584 / 1552
+//   57 k and 38 k              2260 / 2341 / 4491 / 1634 / 1560      76 k and 19 k     2255 / 2368 / 4522 / 1589 / 1550
+//   76 k and 38 k              2260 / 2338 / 4517 / 1591 / 1547      76 k and 57 k     2277 / 2417 / 4540 / 1595 / 1553
+//   95 k and 38 k              2267 / 2347 / 4472 / 1594 / 1554
+// (the forms lie within 3 % of one another; before the layers' kernels were faster the first row was 6 to 14 % slower than the third)
+// (Device memory of a group's buffers at 2000 edges a batch, K 10: 2.5 GB, half of it queries and attention sums.)
 static int group_rows() {
   int device = 0, sms = 0;      // (asked of the device itself: no context is made for it)
   if (cudaGetDevice(&device) != cudaSuccess ||
@@ -446,14 +447,14 @@ static int group_sizes(int n, int bs, int k, int layers, int mode, int32_t *size
 
 // The memory chain is serial, so only what a later batch of the group reads belongs there: in a group of 2000-edge
 // batches on the largest graph 125 of a batch's 890 updates.  The others, every node's last update in the group, wait for
-// nobody, and one launch of the general projection does them behind the chain (chain 208 -> 74 us a group on half of the
-// SMs).  That launch and the message rows it reads are 25 us of latency, of which a group with few updates wins back
+// nobody, and one launch (gru_rows.cu) does them behind the chain (chain 208 -> 74 us a group on half of the
+// SMs).  That launch and the message rows it reads are some 20 us of latency, of which a group with few updates wins back
 // nothing, while the largest graph's wins at every size.  us for a stream of one group, without / with, by its positions:
 //            8 k      12 k     16 k     20 k     24 k     32 k        40 k
-//   2000     457/439  568/530  719/661  840/754  953/847  1224/1107   1498/1342      edges a batch, largest graph
-//   1000     448/462  545/554  690/695  793/802  896/902  1148/1150   1416/1409
-//   600      611/625  840/852  936/944  1149/1154  1367/1372  1701/1705              (K 20)
-//   200      621/630  884/887
+//   2000     441/414  539/491  700/632  806/716  883/775  1124/985    1352/1183      edges a batch, largest graph
+//   1000     448/450  508/507  631/629  719/721  828/815  1027/1028   1279/1265
+//   600      528/537  693/696  838/837  975/967  1102/1101  1419/1412                 (K 20)
+//   200      607/606  779/798
 constexpr int SPLIT_FROM = 16384;      // positions [src | dst] of a group
 
 // Index buffers (two of each) and main-stream buffers.  The layer-1 rows that exist at all are few more than the

@@ -1,7 +1,7 @@
 // Memory updates whose inputs are all there: gates = [message | memory] . Wg + bg and the new memory row, for rows that come
 // as an operand image (attn_out.cuh) of the message's four parts.
 //
-// The update of a single batch of more than 1024 edges and the last updates of a group.  A tile of the general projection
+// The update of a single call and the last updates of a group.  A tile of the general projection
 // kernel, whose producer warps fetch fp32 rows, convert and store them k-block by k-block, four times over (once per tile of
 // 44 units), takes 30 us; here the kernels that store the messages (state.cu, chain.cu) write the parts' heads and tails as
 // well, and the main loop is bulk copies and MMAs: 28 stages of 32 columns (16 KB of rows, 22 KB of weights) through a ring of

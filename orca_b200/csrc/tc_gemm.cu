@@ -112,7 +112,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       b[k] = has1 ? add4(ld_shared_f4(ra + 512u), bB) : f4z;
       hA[k] = hB[k] = 0.f;
       if (EPI == EPI_GRU && ok[k]) {
-        const float *hrow = g.memory + (size_t)mb[k] * g.memory_ld;
+        const float *hrow = g.memory + (size_t)mb[k] * D;
         if (uA < D) hA[k] = hrow[uA];
         if (has1 && uB < D) hB[k] = hrow[uB];
       }
@@ -159,7 +159,7 @@ __device__ __forceinline__ void tile_output(const Args &g, const float *tile, co
       for (int k = 0; k < RB; ++k)
         if (ok[k]) {
           // (row of the whole list; with the multi-GPU split the row also goes to every rank's buffer)
-          const size_t orow = (size_t)(g.out_rows != nullptr ? ma[k] : g.row_stride > 1 ? m[k] * g.row_stride + g.row_off : m[k]) * D;
+          const size_t orow = (size_t)(g.row_stride > 1 ? m[k] * g.row_stride + g.row_off : m[k]) * D;
           if (uA < D) {
             const float h = gru_gates(a[k], hA[k]);
             if (g.peer.world == 0) g.out[orow + uA] = h;
@@ -226,7 +226,6 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(Args g) {
         meta_b = g.push_ids[m];
         meta_a = g.push_win[m];
       }
-      if (EPI == EPI_GRU && g.out_rows != nullptr) meta_a = g.out_rows[m];
       if (EPI == EPI_GRU) meta_b = g.nodes[rstride > 1 ? min(m * rstride + g.row_off, g.idx_limit - 1) : m];
     }
   };

@@ -96,10 +96,8 @@ struct Args {
   const int32_t *push_ids;
   const uint8_t *push_win;
   // GRU
-  const float *memory;       // old memory values: row nodes[m], memory_ld floats each
-  int memory_ld;
+  const float *memory;       // old memory values: row nodes[m]
   const int32_t *nodes;
-  const int32_t *out_rows;   // optional: result row of m (else m)
   // SCORE
   const float *w2;
   float b2;
