@@ -2,10 +2,11 @@
 (evaluation/evaluation.py:6-47): mean average precision, AUC and accuracy over the batches of the
 stream, one uniform negative destination per positive edge drawn batch by batch from the sampler.
 
-The reference calls the model once per batch and brings the scores back per batch; here the
-negatives of all batches are drawn first (same draws, same order: the sampler is consumed exactly as
-the reference consumes it) and the whole stream goes through ``TGN.eval_epoch_metrics`` -- one call.
-The metrics are those of scikit-learn, per batch as in the reference, computed by the library.
+The reference calls the model once per batch and brings the scores back per batch; here the whole
+stream goes through ``TGN.eval_epoch_metrics`` -- one call.  The sampler is consumed exactly as the
+reference consumes it (same draws, same order): before the first batch, or, where it is this module's
+own and nothing of it has been replaced, while the GPU works on the batches before.  The metrics are
+those of scikit-learn, per batch as in the reference, computed by the library.
 """
 from __future__ import annotations
 
@@ -62,6 +63,14 @@ class _Drawn:
         return self.ids[part]
 
 
+def _plain(sampler):
+    """Whether the sampler's draws are this module's own all through, on its own lists and generator: such a draw does not
+    fail once the first one has succeeded, and nobody sees when it is made."""
+    return type(sampler) is RandEdgeSampler and not {"sample", "sample_destinations"} & vars(sampler).keys() and \
+        type(sampler.random_state) is np.random.RandomState and \
+        all(type(ids) is np.ndarray and ids.dtype.kind in "iu" for ids in (sampler.src_list, sampler.dst_list))
+
+
 def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_size, reuse=True, cache_plan=None):
     assert negative_edge_sampler.seed is not None
     negative_edge_sampler.reset_random_state()
@@ -73,7 +82,7 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
     nb = math.ceil(n / batch_size)
     negatives = _Drawn(n, batch_size, draw)
     own = all(getattr(getattr(model, f, None), "__func__", None) is getattr(TGN, f) for f in ("eval_epoch", "eval_epoch_metrics"))
-    if not own or type(negative_edge_sampler) is not RandEdgeSampler:
+    if not own or not _plain(negative_edge_sampler):
         negatives = negatives[:]      # (somebody else's: all draws before the first batch, as the reference's caller sees it)
     # per batch, as the reference does; the positive "wins" when its score is not below the negative's
     # (evaluation/evaluation.py:39-40)

@@ -47,3 +47,68 @@ def test_negatives_drawn_when_asked_for_are_those_drawn_at_once(n, bs):
         assert np.array_equal(drawn[lo:lo + 3], want[lo:lo + 3]) and drawn.drawn < lo + 3 + bs
     assert np.array_equal(drawn[:], want)
     assert at_once.random_state.randint(1 << 30) == lazily.random_state.randint(1 << 30)
+
+
+class _Streams:
+    """A model whose streams are TGN's as far as the evaluation can see: hands the negatives of two batches on and then
+    fails, or scores all of them."""
+
+    def __init__(self, fails):
+        from orca_b200.tgn import TGN
+        self.fails, self.taken = fails, 0
+        self.eval = lambda: self
+        self.eval_epoch, self.eval_epoch_metrics = (f.__get__(self) for f in (TGN.eval_epoch, TGN.eval_epoch_metrics))
+
+    def _eval_stream(self, sources, destinations, negatives, timestamps, edge_idxs, k, bs, *rest):
+        for lo in range(0, len(sources), bs):
+            if self.fails and lo == 2 * bs:
+                raise RuntimeError("in the middle")
+            self.taken += len(negatives[lo:lo + bs])
+        return np.linspace(0.6, 0.9, len(sources), dtype=np.float32), np.full(len(sources), 0.5, np.float32)
+
+
+def _evaluate(model, sampler, n=50, bs=10):
+    import types
+    from orca_b200.evaluation import eval_edge_prediction
+    a = np.arange(n)
+    data = types.SimpleNamespace(sources=a, destinations=a, timestamps=a, edge_idxs=a, n_interactions=n)
+    return eval_edge_prediction(model, sampler, data, 10, bs)
+
+
+@pytest.mark.parametrize("replace", ["sample_destinations", "random_state", "dst_list"])
+def test_draws_that_can_fail_are_made_before_anything_is_scored(replace):
+    """A RandEdgeSampler of which something was replaced is somebody else's: its third draw fails, and no batch has been
+    handed to the model by then."""
+    from orca_b200.evaluation import RandEdgeSampler
+
+    class Third:
+        calls = 0
+
+        def count(self):
+            self.calls += 1
+            if self.calls == 3:
+                raise KeyError("third draw")
+
+        def randint(self, lo, hi, size):
+            if hi == 100:
+                self.count()
+            return np.zeros(size, np.int64)
+
+        def __len__(self):
+            return 100
+
+        def __getitem__(self, at):
+            self.count()
+            return at
+
+    sampler, third = RandEdgeSampler(np.arange(5), np.arange(100), seed=3), Third()
+    if replace == "sample_destinations":
+        sampler.sample_destinations = lambda size: third[np.arange(size)]
+    elif replace == "random_state":
+        sampler.reset_random_state = lambda: setattr(sampler, "random_state", third)
+    else:
+        sampler.dst_list = third
+    model = _Streams(fails=False)
+    with pytest.raises(KeyError):
+        _evaluate(model, sampler)
+    assert model.taken == 0
