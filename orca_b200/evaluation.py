@@ -84,18 +84,21 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
     own = all(getattr(getattr(model, f, None), "__func__", None) is getattr(TGN, f) for f in ("eval_epoch", "eval_epoch_metrics"))
     if not own or not _plain(negative_edge_sampler):
         negatives = negatives[:]      # (somebody else's: all draws before the first batch, as the reference's caller sees it)
-    # per batch, as the reference does; the positive "wins" when its score is not below the negative's
-    # (evaluation/evaluation.py:39-40)
-    stream = (data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n], data.edge_idxs[:n], n_neighbors,
-              batch_size, cache_plan)
-    if getattr(model.eval_epoch, "__func__", None) is TGN.eval_epoch:
-        m = model.eval_epoch_metrics(*stream, reuse=reuse)
-    else:       # (a model with an eval_epoch of its own: its scores count)
-        pos, neg = model.eval_epoch(*stream, reuse=reuse)
-        m = np.empty((nb, 3))
-        rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, batch_size, m.ctypes.data)
-        if rc == _lib.E_BADARG:
-            raise ValueError(_lib.lib().orca_last_error().decode())
-        _lib.check(rc)
+    try:
+        # per batch, as the reference does; the positive "wins" when its score is not below the negative's
+        # (evaluation/evaluation.py:39-40)
+        stream = (data.sources[:n], data.destinations[:n], negatives, data.timestamps[:n], data.edge_idxs[:n], n_neighbors,
+                  batch_size, cache_plan)
+        if getattr(model.eval_epoch, "__func__", None) is TGN.eval_epoch:
+            m = model.eval_epoch_metrics(*stream, reuse=reuse)
+        else:       # (a model with an eval_epoch of its own: its scores count)
+            pos, neg = model.eval_epoch(*stream, reuse=reuse)
+            m = np.empty((nb, 3))
+            rc = _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, n, batch_size, m.ctypes.data)
+            if rc == _lib.E_BADARG:
+                raise ValueError(_lib.lib().orca_last_error().decode())
+            _lib.check(rc)
+    finally:
+        negatives[:]      # (the sampler is left behind all draws of the stream, also where that fails half-way)
     val_ap, val_auc, val_acc = np.mean(m, axis=0)
     return val_ap, val_auc, val_acc

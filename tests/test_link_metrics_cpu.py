@@ -112,3 +112,20 @@ def test_draws_that_can_fail_are_made_before_anything_is_scored(replace):
     with pytest.raises(KeyError):
         _evaluate(model, sampler)
     assert model.taken == 0
+
+
+@pytest.mark.parametrize("fails", [False, True])
+def test_the_sampler_is_left_behind_all_draws_of_the_stream(fails):
+    from orca_b200.evaluation import RandEdgeSampler
+    want, sampler = (RandEdgeSampler(np.arange(5), np.arange(100), seed=3) for _ in range(2))
+    for _ in range(5):
+        want.sample(10)
+    model = _Streams(fails)
+    if fails:
+        with pytest.raises(RuntimeError, match="in the middle"):
+            _evaluate(model, sampler)
+        assert model.taken == 20
+    else:
+        _evaluate(model, sampler)
+        assert model.taken == 50
+    assert np.array_equal(want.sample(20)[1], sampler.sample(20)[1])
