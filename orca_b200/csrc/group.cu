@@ -538,7 +538,7 @@ static Buffers carve(void *base, int bs, int nb, int k, int u_cap, int plan_cap,
   w.feat = (char *)take(img::bytes(w.chunk, img::FEAT_STAGES));
   w.feat2 = (char *)take(layers == 2 ? img::bytes(batch_rows, img::FEAT_STAGES) : 4);
   w.valid = (uint8_t *)take((size_t)w.chunk);
-  w.emb1 = (float *)take((size_t)w.rows_max * D * 4);
+  w.emb1 = (float *)take(layers == 2 ? (size_t)w.rows_max * D * 4 : 4);     // (one layer leaves pairs)
   w.pairs = (char *)take(img::bytes(2 * E, img::PAIR_STAGES));
   w.total = off;
   return w;

@@ -132,3 +132,11 @@ def test_no_exception_leaves_an_entry_point(entry, said):
     env = dict(os.environ, OMP_NUM_THREADS="1", OPENBLAS_NUM_THREADS="1", MALLOC_ARENA_MAX="1")
     r = subprocess.run([sys.executable, "-c", LIMITED, entry], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and said in r.stdout, (r.returncode, r.stdout, r.stderr[-2000:])
+
+
+@pytest.mark.parametrize("bs,nb,k", [(1, 1, 1), (37, 32, 5), (200, 20, 10), (2000, 11, 32)])
+def test_one_layer_has_no_room_for_embeddings_that_nobody_reads(L, bs, nb, k):
+    """A group of a one-layer model leaves its rows to the scores as pairs; with two layers (here the recursion that recomputes
+    no neighbours) every row has its embedding (688 bytes) and an operand image of it (192 columns of four bytes) beside that."""
+    one, two = (L.orca_group_workspace_bytes(bs, nb, k, 0, 0, 5000, layers, 1) for layers in (1, 2))
+    assert two - one >= 3 * bs * nb * (688 + 768) - 2 * 256
