@@ -383,7 +383,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     }
     __syncwarp();        // (the query has been read by all lanes: the next one may land)
     if (next >= 0) fetch_query(nx_q);
-    phase ^= 1;
+    phase ^= alive;      // (stays at the query that did not come)
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
     const float inv0 = vmask ? 1.f / sum0 : 0.f, inv1 = vmask ? 1.f / sum1 : 0.f;
@@ -441,6 +441,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     my_dt = nx_dt;
   }
   if (lane == 0) {
+    if (!alive) tc::mbar_settle(qbar, phase);
     // the last warp to run out of tickets leaves the counters at zero for the next launch
     const int total = (int)(gridDim.x * (blockDim.x >> 5));
     if (atomicAdd(&ticket[1], 1) == total - 1) {

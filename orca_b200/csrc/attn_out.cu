@@ -107,12 +107,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
       const char *w1 = reinterpret_cast<const char *>(g.w.G_img), *w2 = reinterpret_cast<const char *>(g.w.W2_img);
       const uint64_t once = policy_evict_first();      // (the rows are not read again: 1 % of a stream)
       int it = 0;
-      for (int blk = blockIdx.x; blk * BM < M; blk += gridDim.x) {
+      for (int blk = blockIdx.x; alive && blk * BM < M; blk += gridDim.x) {
         const char *ctx = g.ctx + (size_t)blk * img::CTX_STAGES * A_STAGE;
         for (int st = 0; st < K_STAGES + K2_STAGES; ++st, ++it) {
           const int s = slot_of(it);
           const uint32_t at = place(s);
           mbar_wait(empty(s), (use_of(it) & 1) ^ 1, g.status, 700, alive, g.wait_limit);
+          if (!alive) break;
           if (st < K_STAGES) {
             mbar_expect_tx(full(s), STAGE);
             bulk_g2s_hint(at, ctx + (size_t)st * A_STAGE, A_STAGE, full(s), once);
@@ -122,6 +123,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
             bulk_g2s(at + A_STAGE, w2 + (size_t)(st - K_STAGES) * W_STAGE, W_STAGE, full(s));
           }
         }
+      }
+      for (int q = it - 1, seen = 0; q >= max(0, it - FIRST); --q) {      // (the last use of every slot)
+        const int s = slot_of(q);
+        if (!(seen >> s & 1)) mbar_settle(full(s), use_of(q) & 1);
+        seen |= 1 << s;
       }
     }
     __syncwarp();
@@ -141,7 +147,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
-            if (ks == 1 && half) break;
+            if (!alive || (ks == 1 && half)) break;
             const uint64_t ah = desc_sw64(a + ks * 32), al = desc_sw64(a + A_STAGE / 2 + ks * 32);
             const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
             const uint32_t more = (st > 0 || ks > 0) ? 1u : 0u;
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
             mma_bf16(tmem + SMALL, al, bh, idesc, more);
             mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit(empty(s));
+          if (alive) mma_commit(empty(s));
           if (st == K_STAGES - 1) mma_commit(acc1);
         }
         __syncwarp();
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
-            if (2 * st + ks >= K2_CHUNKS / 2) break;
+            if (!alive || 2 * st + ks >= K2_CHUNKS / 2) break;
             const uint64_t ah = make_desc(a + ks * 2 * A2_LBO, A2_LBO, 128);
             const uint64_t al = make_desc(a + A2_BYTES + ks * 2 * A2_LBO, A2_LBO, 128);
             const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_STAGE / 2 + ks * 2 * W_LBO, W_LBO, 128);
@@ -173,12 +179,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_output_image_kernel(const __g
             mma_bf16(tmem + SMALL, al, bh, idesc, more);
             mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit(empty(s));
+          if (alive) mma_commit(empty(s));
           if (st == K2_STAGES - 1) mma_commit(acc2);
         }
         __syncwarp();
       }
     }
+    if (t > 0) mbar_settle(acc2, (t - 1) & 1);
   } else {
     // ------------------------------------------------------------------ epilogues
     const int ew = warp - 2, quarter = warp & 3, half = ew >> 2;

@@ -90,15 +90,18 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
   if (warp == 0) {
     if (lane == 0) {
       int it = 0;
-      for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y) {
+      for (int blk = blockIdx.y; alive && blk * BM < M; blk += gridDim.y) {
         const char *rows = g.image + (size_t)blk * img::FEAT_STAGES * STAGE;
         for (int st = 0; st < img::FEAT_STAGES; ++st, ++it) {
           const int s = it % STAGES;
           mbar_wait(empty(s), ((it / STAGES) & 1) ^ 1, g.status, 540, alive, g.wait_limit);
+          if (!alive) break;
           mbar_expect_tx(full(s), STAGE);
           bulk_g2s(ring + s * STAGE, rows + (size_t)st * STAGE, STAGE, full(s));
         }
       }
+      mbar_settle(wbar, 0);
+      for (int q = max(0, it - STAGES); q < it; ++q) mbar_settle(full(q % STAGES), (q / STAGES) & 1);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
-            if (2 * st + ks >= STEPS) continue;
+            if (2 * st + ks >= STEPS || !alive) continue;
             const uint32_t w = base + (2 * st + ks) * 2 * W_LBO;
             const uint64_t ah = img::desc_sw64(a + ks * 32), al = img::desc_sw64(a + STAGE / 2 + ks * 32);
             const uint64_t bh = make_desc(w, W_LBO, 128), bl = make_desc(w + W_BYTES, W_LBO, 128);
@@ -125,12 +128,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
             mma_bf16(tmem + SMALL, al, bh, idesc, more);
             mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit(empty(s));
+          if (alive) mma_commit(empty(s));
           if (st == img::FEAT_STAGES - 1) mma_commit(accfull);
         }
         __syncwarp();
       }
     }
+    if (t > 0) mbar_settle(accfull, (t - 1) & 1);
   } else {
     // A tile has 13 chunks of 16 columns, so every other one starts in the middle of a 128-byte line.  The warps' parts are six
     // chunks from a line's start (even tiles: 0 and 6, odd ones: 1 and 7) and, for the first (odd) or last (even) four warps,

@@ -81,12 +81,13 @@ __global__ void __launch_bounds__(THREADS, 1) score_rows_kernel(const __grid_con
     if (lane == 0) {
       const uint64_t once = policy_evict_first();
       int it = 0;
-      for (int blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
+      for (int blk = blockIdx.x; alive && blk < blocks; blk += gridDim.x) {
         const char *rows = g.image + (size_t)blk * K_STAGES * A_STAGE;
         for (int st = 0; st < K_STAGES; ++st, ++it) {
           const int s = it % SLOTS;
           const uint32_t at = base + s * STAGE;
           mbar_wait(empty(s), ((it / SLOTS) & 1) ^ 1, g.status, 1000, alive, g.wait_limit);
+          if (!alive) break;
           mbar_expect_tx(full(s), STAGE);
           bulk_g2s_hint(at, rows + (size_t)st * A_STAGE, A_STAGE, full(s), once);
           const char *kb = reinterpret_cast<const char *>(g.w) + (size_t)(st / 2) * KB_BYTES + (st & 1) * W_HALF;
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(THREADS, 1) score_rows_kernel(const __grid_con
           bulk_g2s(at + A_STAGE + W_HALF, kb + 2 * W_HALF, W_HALF, full(s));
         }
       }
+      for (int q = max(0, it - SLOTS); q < it; ++q) mbar_settle(full(q % SLOTS), (q / SLOTS) & 1);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(THREADS, 1) score_rows_kernel(const __grid_con
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
+            if (!alive) break;
             const uint64_t ah = img::desc_sw64(a + ks * 32), al = img::desc_sw64(a + A_STAGE / 2 + ks * 32);
             const uint64_t bh = make_desc(w + ks * 2 * W_LBO, W_LBO, 128), bl = make_desc(w + W_HALF + ks * 2 * W_LBO, W_LBO, 128);
             const uint32_t more = st > 0 || ks > 0 ? 1u : 0u;
@@ -117,12 +120,13 @@ __global__ void __launch_bounds__(THREADS, 1) score_rows_kernel(const __grid_con
             mma_bf16(tmem + SMALL, al, bh, idesc, more);
             mma_bf16(tmem + SMALL, ah, bl, idesc, 1u);
           }
-          mma_commit(empty(s));
+          if (alive) mma_commit(empty(s));
           if (st == K_STAGES - 1) mma_commit(accfull);
         }
         __syncwarp();
       }
     }
+    if (t > 0) mbar_settle(accfull, (t - 1) & 1);
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int row = quarter * 32 + lane, ch0 = half ? 6 : 0, ch1 = half ? BN / 16 : 6;     // chunks of 16 columns

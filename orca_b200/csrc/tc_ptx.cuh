@@ -44,6 +44,15 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int32_t
     }
   }
 }
+// The last wait for what a thread has in flight itself, before its CTA ends: a thread that gave up on another wait
+// (mbar_wait) must not leave a copy behind that would land in the next CTA's shared memory.  Bounded like the others; a
+// barrier that has flipped, which is the usual case, costs one look at it.
+__device__ __forceinline__ void mbar_settle(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity) && clock64() - t0 < 2000000000ll) {
+  }
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
