@@ -246,6 +246,7 @@ int orca_attn_query(const orca_attn_weights_t *w, const float *d_feat, const int
  *   d_ctx   [n_rows_cap, 1032]   sum_j a_hj * [nbr_j | efeat_j | tenc_j] per head
  *   d_valid [n_rows_cap]         0 where every slot is padding (the layer output of such a row
  *                                ignores the attention term, model/temporal_attention.py:46,52)
+ *   d_status [4] (may be NULL: the context's status word)  ORCA_E_TIMEOUT if a wait gave up: the rows are not valid then
  */
 int orca_attn_gather(const float *d_qt, const float *d_nbr_table, const float *d_edge_table,
                      const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid,

@@ -458,13 +458,14 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
 // d_nbr_table2 (optional): neighbour rows >= nbr_split are read from it; its address is already moved back by
 // nbr_split rows
 // d_q_row (optional): row r's query is row d_q_row[r] of d_qt
+// d_status (optional): where a wait that gave up is reported instead of the context's status word
 // `ticket`: two zeroed device words that the launch leaves at zero; launches that may overlap on the GPU
 // need words of their own
 int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float *d_edge_table,
                        const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid, const float *d_delta,
                        int k, int n_rows_cap, const int32_t *d_n_rows, int rows_hint, const int32_t *d_order,
                        void *d_ctx, bool image, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream,
-                       const float *d_nbr_table2, int nbr_split, const int32_t *d_q_row) {
+                       const float *d_nbr_table2, int nbr_split, const int32_t *d_q_row, int32_t *d_status) {
   if (d_nbr_table2 == nullptr) nbr_split = 0x7fffffff;
   ORCA_CHECK_ARG(d_qt && d_nbr_table && d_edge_table && d_time_w && d_nbr && d_eid && d_delta && d_ctx &&
                  d_valid && d_ticket);
@@ -485,6 +486,7 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
     }
     ORCA_CUDA(cudaEventRecord(pf.ev[pf.used], stream));
   }
+  if (d_status == nullptr) d_status = c->status_word;
   // one resident wave at most; fewer blocks when the caller expects fewer rows than the capacity
   const int rows = rows_hint > 0 ? std::min(rows_hint, n_rows_cap) : n_rows_cap;
   const bool wide = k >= GA_WIDE_FROM;
@@ -495,11 +497,11 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
   if (pf.on)
     kernel<<<grid, GA_THREADS, 0, stream>>>(d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table, d_time_w, d_nbr, d_eid,
                                             d_delta, k, n_rows_cap, d_n_rows, d_order, d_q_row, d_ctx, d_valid, d_ticket,
-                                            pf.d_counters, c->status_word, c->wait_limit);
+                                            pf.d_counters, d_status, c->wait_limit);
   else
     ORCA_CUDA(launch_dep(kernel, grid, GA_THREADS, 0, stream, d_qt, d_nbr_table, d_nbr_table2, nbr_split, d_edge_table,
                          d_time_w, d_nbr, d_eid, d_delta, (int)k, (int)n_rows_cap, d_n_rows, d_order, d_q_row, d_ctx, d_valid,
-                         d_ticket, (unsigned long long *)nullptr, c->status_word, c->wait_limit));
+                         d_ticket, (unsigned long long *)nullptr, d_status, c->wait_limit));
   if (pf.on) {
     ORCA_CUDA(cudaEventRecord(pf.ev[pf.used + 1], stream));
     pf.used += 2;
@@ -532,9 +534,9 @@ extern "C" int orca_attn_gather(const float *d_qt, const float *d_nbr_table, con
                                 const float *d_delta, int32_t k, int32_t n_rows_cap,
                                 const int32_t *d_n_rows, float *d_ctx, uint8_t *d_valid,
                                 int32_t *d_status, void *stream) {
-  (void)d_status;
   Ctx *c = cur();
   if (c == nullptr) return set_error(ORCA_E_CUDA, "orca_attn_gather: no context for the current device");
   return launch_attn_gather(d_qt, d_nbr_table, d_edge_table, d_time_w, d_nbr, d_eid, d_delta, k, n_rows_cap,
-                            d_n_rows, 0, nullptr, d_ctx, false, d_valid, c->d_words + CTX_TICKET_MAIN, (cudaStream_t)stream);
+                            d_n_rows, 0, nullptr, d_ctx, false, d_valid, c->d_words + CTX_TICKET_MAIN, (cudaStream_t)stream, nullptr, 0,
+                            nullptr, d_status);
 }

@@ -45,7 +45,8 @@ int launch_attn_gather(const float *d_qt, const float *d_nbr_table, const float 
                        const float *d_time_w, const int32_t *d_nbr, const int32_t *d_eid, const float *d_delta,
                        int k, int n_rows_cap, const int32_t *d_n_rows, int rows_hint, const int32_t *d_order,
                        void *d_ctx, bool image, uint8_t *d_valid, int32_t *d_ticket, cudaStream_t stream,
-                       const float *d_nbr_table2 = nullptr, int nbr_split = 0, const int32_t *d_q_row = nullptr);
+                       const float *d_nbr_table2 = nullptr, int nbr_split = 0, const int32_t *d_q_row = nullptr,
+                       int32_t *d_status = nullptr);
 // rows of two neighbour tables sorted by falling number of valid slots (one launch, one block per table)
 int launch_row_order(const int32_t *d_nbr_a, int n_cap_a, const int32_t *d_n_a, int32_t *d_order_a,
                      const int32_t *d_nbr_b, int n_cap_b, const int32_t *d_n_b, int32_t *d_order_b, int k,

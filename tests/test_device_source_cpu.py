@@ -33,3 +33,9 @@ def test_a_query_that_did_not_come_is_waited_for():
     text = _source("attention.cu")
     at = [text.index(x) for x in ("mbar_wait(qbar, phase", "phase ^= alive;", "if (!alive) tc::mbar_settle(qbar, phase);")]
     assert at == sorted(at)
+
+
+def test_no_entry_point_drops_the_status_word_it_is_given():
+    """Every entry point that takes one hands it to what it launches: its kernels have nothing else to say that rows are wrong."""
+    for name in os.listdir(CSRC):
+        assert name.endswith((".cu", ".cuh")) is False or "(void)d_status" not in _source(name), name

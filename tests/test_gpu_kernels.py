@@ -308,6 +308,28 @@ def test_attention_gather_slots(dev, k):
         assert np.all(np.abs(got[rows, h * 516:(h + 1) * 516] - want) < (4 * delta[rows] + 1e-6)[:, None] * most + 7.8e-7)
 
 
+@pytest.mark.parametrize("own", [True, False])
+@pytest.mark.parametrize("k", [10, 20])
+def test_attention_gather_reports_where_it_is_told(dev, own, k):
+    """The status words, the caller's and the context's, are zero after a launch of either form, with or without either."""
+    from orca_b200 import _lib
+    L, n = _lib.lib(), 3000
+    q, tab = torch.randn(n, 1056, device=dev), torch.randn(300, D, device=dev)
+    ids = torch.randint(1, 300, (n, k), device=dev, dtype=torch.int32)
+    dt, w = torch.rand(n, k, device=dev), torch.rand(D, device=dev)
+    ctx, valid = torch.zeros(n, 1032, device=dev), torch.zeros(n, dtype=torch.uint8, device=dev)
+    theirs, ours = torch.zeros(4, dtype=torch.int32, device=dev), torch.zeros(4, dtype=torch.int32, device=dev)
+    _lib.check(L.orca_ctx_set_status_word(None, ours.data_ptr()))
+    try:
+        _lib.check(L.orca_attn_gather(q.data_ptr(), tab.data_ptr(), tab.data_ptr(), w.data_ptr(), ids.data_ptr(), ids.data_ptr(),
+                                      dt.data_ptr(), k, n, None, ctx.data_ptr(), valid.data_ptr(), theirs.data_ptr() if own else None,
+                                      _lib.stream_ptr(dev)))
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(L.orca_ctx_set_status_word(None, None))
+    assert bool((valid == 1).all()) and not theirs.any() and not ours.any()
+
+
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 // 6 + 1, 9000])
 def test_attention_query(dev, n):
     """The stand-alone query projection against 64 bits, rows past the device-side count untouched, an output that is
