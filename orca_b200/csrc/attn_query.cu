@@ -11,8 +11,8 @@
 // its 39 stages out.  What bounds it: 4.8 us a block and CTA against 2 of products; without the stores 66 us, stores alone 48.
 // Measured instead, 6 / 31 / 66 k rows: pairs of CTAs with half of a tile of 224 columns each and six stages 22 / 71 / 141;
 // stores of fragments without the boxes, five stages, 18 / 53 / 95; stores of the boxes by tensor map 16 / 53 / 104.
-// orca_attn_query, whose rows come as floats, writes the image to scratch memory first: 14.7 / 20.8 / 90.5 us
-// for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
+// orca_attn_query, whose rows come as floats and which wants qt alone (tiles of 176 columns), writes the image to scratch memory
+// first: 14.7 / 20.8 / 84.4 us for 600 / 6000 / 51,000 rows, against 12.3 / 24.6 / 129 for a kernel of its own that split the rows eleven times over.
 #include <algorithm>
 
 #include "attn_out.cuh"
@@ -25,14 +25,24 @@ namespace aqi {
 
 constexpr int BM = 128;
 constexpr int CHUNKS = 22, STEPS = CHUNKS / 2;                // K = 172, padded to 176
-constexpr int BN = 208, TILES = (QT_LD + D + BN - 1) / BN;   // 6
-static_assert(TILES * BN >= QT_LD + D && QT_LD % 32 == 0 && OWN_LD % 32 == 0, "whole lines belong to one of the two outputs");
-constexpr int W_LBO = BN * 16, W_BYTES = CHUNKS * W_LBO;
-constexpr int STAGES = 3, STAGE = img::STAGE_BYTES;
+constexpr int TILES = 6;
+// weights: per eight columns [head | tail][K / 8][8 columns][8], so that any whole number of them is one piece
+constexpr int W_HALF = CHUNKS * 128, W_GROUP = 2 * W_HALF;
+constexpr int STAGE = img::STAGE_BYTES;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
 constexpr int BOX = 32 * 128;                                 // of a warp: 32 rows x 32 columns on their way out
-constexpr int RING = (2 * W_BYTES + 1023) / 1024 * 1024;      // (the swizzle wants aligned stages)
-constexpr int SMEM = RING + STAGES * STAGE + EPI_WARPS * BOX + 1024;
+// OWN: the features' part of the hidden layer as well, in tiles of 208 columns; without it tiles of 176 and a stage more
+// (orca_attn_query, 6 / 18 / 36 / 51 / 66 k rows, caches flushed: 20.8 / 37.2 / 63.8 / 84.4 / 106.8 us; with tiles of 208, whose
+// last columns nobody asked for, 20.8 / 39.3 / 67.9 / 92.4 / 115.1)
+template <bool OWN>
+struct Tile {
+  static constexpr int BN = OWN ? 208 : 176, CHUNKS_16 = BN / 16, MOST = (CHUNKS_16 + 1) / 2;   // MOST: 16-column chunks of a warp
+  static constexpr int W_BYTES = BN / 8 * W_GROUP;
+  static constexpr int STAGES = OWN ? 3 : 4;
+  static constexpr int RING = (W_BYTES + 1023) / 1024 * 1024;      // (the swizzle wants aligned stages)
+  static constexpr int SMEM = RING + STAGES * STAGE + EPI_WARPS * BOX + 1024;
+  static_assert(TILES * BN >= QT_LD + (OWN ? D : 0) && QT_LD % 32 == 0 && OWN_LD % 32 == 0, "whole lines belong to one of the two outputs");
+};
 constexpr int TMEM_COLS = 512, SMALL = 256;                   // one buffer of main + cross-term accumulators
 
 struct Args {
@@ -46,8 +56,10 @@ struct Args {
   long long wait_limit;
 };
 
+template <bool OWN>
 __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __grid_constant__ Args g) {
   using namespace tc;
+  constexpr int BN = Tile<OWN>::BN, STAGES = Tile<OWN>::STAGES, W_BYTES = Tile<OWN>::W_BYTES, RING = Tile<OWN>::RING;
   extern __shared__ unsigned char raw[];
   __shared__ __align__(16) float s_bias[BN];
   __shared__ __align__(8) unsigned long long s_bar[2 * STAGES + 3];
@@ -69,8 +81,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
     mbar_init(accfull, 1);
     mbar_init(accfree, EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(wbar, 2 * W_BYTES);       // (weights: written by nobody but the host, long ago)
-    bulk_g2s(base, reinterpret_cast<const char *>(g.w) + (size_t)nt * 2 * W_BYTES, 2 * W_BYTES, wbar);
+    mbar_expect_tx(wbar, W_BYTES);       // (weights: written by nobody but the host, long ago)
+    bulk_g2s(base, reinterpret_cast<const char *>(g.w) + (size_t)nt * W_BYTES, W_BYTES, wbar);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
@@ -120,9 +132,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
             if (2 * st + ks >= STEPS || !alive) continue;
-            const uint32_t w = base + (2 * st + ks) * 2 * W_LBO;
+            const uint32_t w = base + (2 * st + ks) * 2 * 128;
             const uint64_t ah = img::desc_sw64(a + ks * 32), al = img::desc_sw64(a + STAGE / 2 + ks * 32);
-            const uint64_t bh = make_desc(w, W_LBO, 128), bl = make_desc(w + W_BYTES, W_LBO, 128);
+            const uint64_t bh = make_desc(w, 128, W_GROUP), bl = make_desc(w + W_HALF, 128, W_GROUP);
             const uint32_t more = st > 0 || ks > 0 ? 1u : 0u;
             mma_bf16(tmem, ah, bh, idesc, more);
             mma_bf16(tmem + SMALL, al, bh, idesc, more);
@@ -136,12 +148,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
     }
     if (t > 0) mbar_settle(accfull, (t - 1) & 1);
   } else {
-    // A tile has 13 chunks of 16 columns, so every other one starts in the middle of a 128-byte line.  The warps' parts are six
+    // A tile of 13 chunks of 16 columns: every other one starts in the middle of a 128-byte line.  The warps' parts are six
     // chunks from a line's start (even tiles: 0 and 6, odd ones: 1 and 7) and, for the first (odd) or last (even) four warps,
-    // the half line that is left.
-    const int quarter = warp & 3, half = (warp - 2) >> 2, odd = nt & 1;
+    // the half line that is left.  A tile of 11: six chunks and five, from its start.
+    constexpr int MOST = Tile<OWN>::MOST;
+    const int quarter = warp & 3, half = (warp - 2) >> 2, odd = OWN ? nt & 1 : 0;
     const int c0 = half * 6 + odd, single = odd ? 0 : 12;
-    const bool seven = half != odd;
+    const bool last = OWN ? half != odd : half == 0;      // whether these warps have a last, the MOST-th, chunk
     const uint32_t box = ring + STAGES * STAGE + (warp - 2) * BOX;
     int t = 0;
     for (int blk = blockIdx.y; blk * BM < M; blk += gridDim.y, ++t) {
@@ -149,37 +162,38 @@ __global__ void __launch_bounds__(THREADS, 1) attn_query_image_kernel(const __gr
       mbar_wait(accfull, t & 1, g.status, 560, alive, g.wait_limit);
       tc_fence_after();
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
-      float v[7][16];
+      float v[MOST][16];
 #pragma unroll
-      for (int ch = 0; ch < 7; ++ch)
-        if (ch < 6 || seven) tmem_ld16_sum(acc + (ch < 6 ? c0 + ch : single) * 16, SMALL, v[ch]);
+      for (int ch = 0; ch < MOST; ++ch)
+        if (ch < MOST - 1 || last) tmem_ld16_sum(acc + (ch < 6 ? c0 + ch : single) * 16, SMALL, v[ch]);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(accfree);      // (the next block's products may start before this one is stored)
       // 32 columns at a time through shared memory (16-byte pieces of a row exchanged by its number's low bits: no bank
       // conflicts either way), out in whole lines of a row
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        if (b == 3 && !seven) break;
+      for (int b = 0; b < (MOST + 1) / 2; ++b) {
+        if (b == 3 && !last) break;
         const int at = b < 3 ? (c0 + 2 * b) * 16 : single * 16;      // first column of the box in the tile
+        const bool whole = OWN || b < 2 ? b < 3 : last;
 #pragma unroll
         for (int p = 0; p < 8; ++p) {
           const int ch = 2 * b + (p >> 2), c = 4 * (p & 3);
-          if (ch >= 7) continue;
+          if (ch >= MOST || (!OWN && ch == MOST - 1 && !last)) continue;
           const float4 y = *reinterpret_cast<const float4 *>(s_bias + at + 16 * (p >> 2) + c);
           st_shared_f4(box + lane * 128 + ((p ^ (lane & 7)) << 4),
                        make_float4(v[ch][c] + y.x, v[ch][c + 1] + y.y, v[ch][c + 2] + y.z, v[ch][c + 3] + y.w));
         }
         __syncwarp();
-        const int p = b < 3 ? lane & 7 : lane & 3, col = nt * BN + at + 4 * p;
-        const bool query = col < QT_LD;
+        const int p = whole ? lane & 7 : lane & 3, col = nt * BN + at + 4 * p;
+        const bool query = !OWN || col < QT_LD;
         float *out = query ? g.qt + col : g.own + (col - QT_LD);
         const int ld = query ? QT_LD : OWN_LD;
         const bool on = query || (g.own != nullptr && col < QT_LD + OWN_LD);
 #pragma unroll
         for (int i = 0; i < (b < 3 ? 8 : 4); ++i) {
-          const int r = b < 3 ? 4 * i + (lane >> 3) : 8 * i + (lane >> 2);
-          if (on && m0 + r < M)
+          const int r = whole ? 4 * i + (lane >> 3) : 8 * i + (lane >> 2);
+          if (on && (OWN || whole || i < 4) && m0 + r < M)
             *reinterpret_cast<float4 *>(out + (size_t)(m0 + r) * ld) = ld_shared_f4(box + r * 128 + ((p ^ (r & 7)) << 4));
         }
         __syncwarp();
@@ -239,12 +253,14 @@ int attn_query_image(const orca_attn_weights_t *w, const char *d_image, int n_ca
   ORCA_CHECK_ARG(w && w->Mq_img && w->cq && d_image && d_qt && (((uintptr_t)d_qt | (uintptr_t)d_own) & 15) == 0);
   static thread_local int configured_device = -1;
   if (configured_device != c->device) {
-    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::SMEM));
+    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::Tile<false>::SMEM));
+    ORCA_CUDA(cudaFuncSetAttribute(aqi::attn_query_image_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, aqi::Tile<true>::SMEM));
     configured_device = c->device;
   }
   const aqi::Args g{d_image, n_cap, d_n, w->Mq_img, w->cq, d_qt, d_own, c->status_word, c->wait_limit};
   const dim3 grid(aqi::TILES, std::min(ceil_div(n_cap, aqi::BM), std::max(1, c->sm_count / aqi::TILES)));
-  ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel, grid, aqi::THREADS, aqi::SMEM, s, g));
+  if (d_own != nullptr) ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel<true>, grid, aqi::THREADS, aqi::Tile<true>::SMEM, s, g));
+  else ORCA_CUDA(launch_dep(aqi::attn_query_image_kernel<false>, grid, aqi::THREADS, aqi::Tile<false>::SMEM, s, g));
   ORCA_COUNT_LAUNCH();
   ORCA_LAUNCH_CHECK();
   return ORCA_OK;

@@ -25,7 +25,7 @@ HEADS = 2
 QT_HEAD = 528     # column stride of one head of the projected query (516 used)
 TC_BN, TC_BK = 176, 64
 GRU_PART, CHAIN_N = 176, 32
-QUERY_BN = 208    # columns of a weight tile of csrc/attn_query.cu
+QUERY_COLS = 6 * 208    # columns of csrc/attn_query.cu's weight tiles
 
 
 def _packed(W, shape, image):
@@ -61,10 +61,10 @@ def pack_tc(W, bn=None):
 
 
 def pack_query(W):
-    """Weights [172, n] of the rows' own features for csrc/attn_query.cu: K padded to 176, one image per 208 columns, each
-    [head | tail][K / 8][208 columns][8]: uint16 [tiles, 2, 22, 208, 8]."""
-    return _packed(W, (GRU_PART, -(-W.shape[1] // QUERY_BN) * QUERY_BN),
-                   lambda X: X.reshape(2, GRU_PART // 8, 8, -1, QUERY_BN).permute(3, 0, 1, 4, 2))
+    """Weights [172, n] of the rows' own features for csrc/attn_query.cu: K padded to 176, columns to six tiles of 208; one
+    image per eight columns, each [head | tail][K / 8][8 columns][8], so that a tile of any width is one piece of it:
+    uint16 [156, 2, 22, 8, 8]."""
+    return _packed(W, (GRU_PART, QUERY_COLS), lambda X: X.reshape(2, GRU_PART // 8, 8, -1, 8).permute(3, 0, 1, 4, 2))
 
 
 def pack_stages(W):

@@ -88,3 +88,20 @@ def test_tensor_core_weight_packing():
     got = as_f32(P[0, k // 64, 0, (k % 64) // 8, n, k % 8]) + as_f32(P[0, k // 64, 1, (k % 64) // 8, n, k % 8])
     assert got == rec[k, n]
     assert weights.pack_tc(rs.randn(172, 1056).astype(np.float32)).shape == (6, 3, 2, 8, 176, 8)
+
+
+def test_query_weight_packing():
+    """Element (k, n) of the own features' weights lies at [n // 8][part][k // 8][n % 8][k % 8], so that the columns of a tile of
+    any width are one piece of the image; columns past the last, up to six tiles of 208, are zero."""
+    rs = np.random.RandomState(0)
+    W = rs.randn(172, 1056 + 172).astype(np.float32)
+    P = weights.pack_query(W)
+    assert P.shape == (156, 2, 22, 8, 8) and P.dtype == np.uint16
+    as_f32 = lambda bits: (bits.astype(np.uint32) << 16).view(np.float32)
+    rec = (as_f32(P[:, 0]) + as_f32(P[:, 1])).transpose(1, 3, 0, 2).reshape(176, 6 * 208)
+    assert np.max(np.abs(rec[:172, :1228] - W) / np.abs(W)) < 2 ** -15
+    assert not rec[172:].any() and not rec[:, 1228:].any()
+    for bn in (176, 208):
+        tile = P.reshape(-1)[5 * bn * 352:6 * bn * 352].reshape(-1, 2, 22, 8, 8)
+        got = (as_f32(tile[:, 0]) + as_f32(tile[:, 1])).transpose(1, 3, 0, 2).reshape(176, bn)
+        assert np.array_equal(got, rec[:, 5 * bn:6 * bn])
