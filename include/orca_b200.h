@@ -52,6 +52,12 @@ extern "C" {
 #define ORCA_QT_DIM (ORCA_HEADS * ORCA_KEY_DIM)
 #define ORCA_QT_LD 1056                      /* row stride of the projected query: 2 heads x 528 */
 
+/* Version of this interface, of the descriptors below and of the operands that a caller prepares (the *_tc, *_img and *_chain
+ * members; their sizes cannot be looked at here, and a kernel reads past the end of an operand of an earlier layout).  A caller
+ * that packs them itself compares orca_version() with the ORCA_VERSION it was written for.
+ * 1: Mq_img = Mq in tiles of 176 columns, G_img = all rows of G.
+ * 2: Mq_img = [Mq | last 172 rows of G] in pieces of eight columns (weights.pack_query), G_img = the other rows of G. */
+#define ORCA_VERSION 2
 const char *orca_last_error(void);
 int orca_version(void);
 

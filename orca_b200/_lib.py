@@ -22,6 +22,7 @@ E_BOUNDS = 5      # ORCA_E_BOUNDS
 CAND_CAP = 2048   # ORCA_CAND_CAP
 EXCHANGE_SLOTS = 4  # ORCA_EXCHANGE_SLOTS
 FLAG_WORDS = 48     # ORCA_FLAG_WORDS
+VERSION = 2      # ORCA_VERSION of the header that this file, tgn.py and weights.py were written for
 # options of orca_ctx_set
 OPT_PROJECTION_MODE, OPT_OVERLAP, OPT_DEPENDENT_LAUNCH, OPT_LOOKAHEAD, OPT_WAIT_LIMIT, OPT_TRACE = range(6)
 
@@ -173,6 +174,9 @@ def lib():
             raise ImportError(f"{LIB_PATH} is missing: build it with `python -m orca_b200.build` "
                               "(nvcc, sm_100a). There is no CPU fallback.")
         L = C.CDLL(LIB_PATH)
+        if L.orca_version() != VERSION:
+            raise ImportError(f"{LIB_PATH} has interface version {L.orca_version()}, this package needs {VERSION}: build it again "
+                              "with `python -m orca_b200.build` (it would read weights of another layout)")
         for name, (res, args) in SYMBOLS.items():
             fn = getattr(L, name)
             fn.restype = res

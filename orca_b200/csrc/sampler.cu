@@ -617,7 +617,7 @@ using namespace orca;
 extern "C" {
 
 const char *orca_last_error(void) { return orca::g_err; }
-int orca_version(void) { return 1; }
+int orca_version(void) { return ORCA_VERSION; }
 
 int orca_csr_build_host(const int64_t *h_src, const int64_t *h_dst, const int64_t *h_eidx,
                         const double *h_ts, int64_t n_edges, int64_t n_nodes, int64_t *h_indptr,

@@ -140,3 +140,13 @@ def test_one_layer_has_no_room_for_embeddings_that_nobody_reads(L, bs, nb, k):
     no neighbours) every row has its embedding (688 bytes) and an operand image of it (192 columns of four bytes) beside that."""
     one, two = (L.orca_group_workspace_bytes(bs, nb, k, 0, 0, 5000, layers, 1) for layers in (1, 2))
     assert two - one >= 3 * bs * nb * (688 + 768) - 2 * 256
+
+
+def test_version_of_the_prepared_operands(L, monkeypatch):
+    """Weights are packed for one layout: header, library and package name the same one, a library of another is refused."""
+    text = open(os.path.join(ROOT, "include", "orca_b200.h")).read()
+    assert int(re.search(r"#define ORCA_VERSION (\d+)", text).group(1)) == L.orca_version() == _lib.VERSION
+    monkeypatch.setattr(_lib, "VERSION", _lib.VERSION + 1)
+    monkeypatch.setattr(_lib, "_lib", None)
+    with pytest.raises(ImportError, match="interface version"):
+        _lib.lib()
