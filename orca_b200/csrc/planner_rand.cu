@@ -118,10 +118,16 @@ __device__ __forceinline__ void clear_bit(uint32_t *bm, int32_t v) { atomicAnd(&
 // threads call it.  s_cnt: NW ints of shared memory.
 // Bitmaps of a few words a thread are dealt out by half words, neighbouring ones to a thread: a thread then lists a handful
 // of members (343 words, a word a lane of eleven warps: 5,600 cycles a batch with the copy out; half words over all of them: 3,400).
+// Up to two words a thread, that is 65,536 nodes.  100 batches, words / half words, ms a plan: LRU 600 edges, budget 10,000,
+// 11 k nodes 1.64 / 1.47, 33 k 1.79 / 1.64, 65 k 1.80 / 1.72; 2Q 200 edges, budget 500, 3.51 / 2.99, 3.69 / 3.26, 3.74 / 3.39; LRU
+// 200 edges, budget 500, 1.57 / 1.60, 1.58 / 1.64, 1.62 / 1.72.  The kernels are made for either (FEW): with both forms in one
+// kernel plans of larger graphs took 1 to 12 % longer (LRU, 200 k nodes, 600 edges, budget 10,000 2.22 for 2.18 ms, 200 edges, budget 500
+// 2.05 for 1.83).
 constexpr int FEW_WORDS = 2 * T;
+template <bool FEW>
 __device__ __forceinline__ int list_members(uint32_t *bm, int64_t words, int32_t *out, int *s_cnt) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (words <= FEW_WORDS) {
+  if (FEW) {
     constexpr int MOST = 2 * FEW_WORDS / T;
     const int halves = 2 * (int)words, per = (halves + T - 1) / T;
     __syncthreads();   // (earlier writes to the bitmap; earlier readers of s_cnt)
@@ -335,7 +341,7 @@ __device__ __forceinline__ void suspend(const Work &w, const Twister &rng, bool 
 }
 
 // ------------------------------------------------------------------------------ LRU (utils/cache.py:338-403)
-template <bool SH>
+template <bool SH, bool FEW>
 __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t b0, int64_t b1, int64_t nb, int64_t n_nodes, int32_t budget,
                                                 uint32_t seed, Work w, int32_t *plan, int64_t plan_cap, int64_t *plan_off,
                                                 int64_t *stats, int32_t *status) {
@@ -397,7 +403,7 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t b0, int64_t b1, int64
       used_at[v] = arrived[v] = (int32_t)b;
     }
     held = listed_at(used);
-    n_held = list_members(cached, words, held, s_a);
+    n_held = list_members<FEW>(cached, words, held, s_a);
     if (used + n_held > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
@@ -419,7 +425,7 @@ __global__ void __launch_bounds__(T, 1) lru_kernel(int64_t b0, int64_t b1, int64
 
 // ------------------------------------------------------------------------------ 2Q (utils/cache.py:175-333)
 // a FIFO half and an LRU half of budget / 2 entries each
-template <bool SH>
+template <bool SH, bool FEW>
 __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int64_t nb, int64_t n_nodes, int32_t budget,
                                                  uint32_t seed, Work w, int32_t *plan, int64_t plan_cap, int64_t *plan_off,
                                                  int64_t *stats, int32_t *status) {
@@ -485,7 +491,7 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       }
       n_fifo = half;
     } else {
-      const int n_ids = list_members(fifo, words, ids, s_a);
+      const int n_ids = list_members<FEW>(fifo, words, ids, s_a);
       shuffle(w, rng, ids, n_ids, false);
       for (int i = tid; i < n_fresh - fifo_room; i += T) clear_bit(fifo, ids[i]);
       __syncthreads();
@@ -509,7 +515,7 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       for (int i = tid; i < n_promote; i += T) admit(promote[i]);
       n_lru += n_promote;
     } else if (n_promote <= lru_room + lru_evictable) {
-      const int n_ids = list_members(lru, words, ids, s_a);
+      const int n_ids = list_members<FEW>(lru, words, ids, s_a);
       bool beside = false;
       if (!for_first_by_key(w, ids, n_ids, n_promote - lru_room, lru_used, s_a, s_b,
                             [&](int32_t v) { clear_bit(lru, v); }, lists::Nothing(), beside)) {
@@ -520,7 +526,7 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       for (int i = tid; i < n_promote; i += T) admit(promote[i]);
       n_lru = half;
     } else {
-      const int n_ids = list_members(lru, words, ids, s_a);
+      const int n_ids = list_members<FEW>(lru, words, ids, s_a);
       for (int i = tid; i < n_ids; i += T)
         if (lru_used[ids[i]] < now) clear_bit(lru, ids[i]);
       __syncthreads();
@@ -531,14 +537,14 @@ __global__ void __launch_bounds__(T, 1) twoq_kernel(int64_t b0, int64_t b1, int6
       n_lru = half;
     }
     // ---- plan = FIFO ids ascending, then LRU ids ascending
-    n_fifo = list_members(fifo, words, ids, s_a);
+    n_fifo = list_members<FEW>(fifo, words, ids, s_a);
     if (used + n_fifo > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
       continue;
     }
     for (int i = tid; i < n_fifo; i += T) plan[used + i] = ids[i];
-    n_lru = list_members(lru, words, ids, s_a);
+    n_lru = list_members<FEW>(lru, words, ids, s_a);
     if (used + n_fifo + n_lru > plan_cap) {
       if (tid == 0) report(status, ORCA_E_CAPACITY, (int)b);
       failed = true;
@@ -670,8 +676,11 @@ extern "C" int orca_plan_device(int32_t strategy, const int32_t *d_nodes, int64_
     ORCA_CUDA(cudaMemsetAsync(d_plan_off, 0, sizeof(int64_t), s));
     return ORCA_OK;
   }
-  auto kernel = strategy == 1 ? (w.bm_shared ? rnd::lru_kernel<true> : rnd::lru_kernel<false>)
-                              : (w.bm_shared ? rnd::twoq_kernel<true> : rnd::twoq_kernel<false>);
+  const bool few = (n_nodes + 31) / 32 <= rnd::FEW_WORDS;
+  auto kernel = strategy == 1 ? (w.bm_shared ? (few ? rnd::lru_kernel<true, true> : rnd::lru_kernel<true, false>)
+                                             : (few ? rnd::lru_kernel<false, true> : rnd::lru_kernel<false, false>))
+                              : (w.bm_shared ? (few ? rnd::twoq_kernel<true, true> : rnd::twoq_kernel<true, false>)
+                                             : (few ? rnd::twoq_kernel<false, true> : rnd::twoq_kernel<false, false>));
   ORCA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int64_t chunk = rnd::chunk_of(nb, bs, k, n_nodes);
   for (int64_t b0 = 0; b0 < nb; b0 += chunk) {

@@ -101,6 +101,25 @@ def test_plans_at_the_limits_of_shared_memory(strategy, n_src, n_edges, bs, budg
     assert (int(stats[0]), int(stats[1])) == wstats[:2]
 
 
+@pytest.mark.parametrize("strategy", ["LRU", "2Q"])
+@pytest.mark.parametrize("n_nodes", [65536, 65537])
+@pytest.mark.parametrize("budget", [900, 30000])
+def test_plans_where_the_listing_of_sets_changes(strategy, n_nodes, budget):
+    """Sets of up to 65,536 nodes are listed by half words, larger ones by words; with the larger budget nothing is evicted."""
+    from oracle import planner
+    from orca_b200 import synthetic
+    spec = dataclasses.replace(synthetic.SPECS["t_nb2"], n_src=n_nodes - 1, n_edges=12000, bs=600, budget=budget)
+    g = synthetic.make_graph(spec, seed=13)
+    assert g.n_nodes == n_nodes
+    adj, got, stats = _device_plan(g, 600, 10, budget, strategy=strategy, seed=9)
+    rb = planner.read_batches(g.sources, g.destinations, g.timestamps, 600, 10, adj, g.n_nodes)
+    want, wstats = planner.solve(strategy, rb, g.n_nodes, budget, seed=9)
+    assert len(got) == len(want)
+    for b, (a, w) in enumerate(zip(got, want)):
+        assert np.array_equal(a, w), f"batch {b}"
+    assert (int(stats[0]), int(stats[1])) == wstats[:2]
+
+
 def test_plan_buffer_too_small_is_reported():
     from orca_b200 import _lib, cache
     g = graph("t_nb2")
