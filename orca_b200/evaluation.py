@@ -5,7 +5,7 @@ stream, one uniform negative destination per positive edge drawn batch by batch 
 The reference calls the model once per batch and brings the scores back per batch; here the whole
 stream goes through ``TGN.eval_epoch_metrics`` -- one call.  The sampler is consumed exactly as the
 reference consumes it (same draws, same order): before the first batch, or, where it is this module's
-own and nothing of it has been replaced, while the GPU works on the batches before.  The metrics are
+own and nothing of it has been replaced, for a longer stream while the GPU works on the batches before.  The metrics are
 those of scikit-learn, per batch as in the reference, computed by the library.
 """
 from __future__ import annotations
@@ -55,12 +55,14 @@ class _Drawn:
         return len(self.ids)
 
     def __getitem__(self, part):
-        upto = len(self.ids) if part.stop is None else min(part.stop, len(self.ids))
-        while self.drawn < upto:
-            n = min(self.batch_size, len(self.ids) - self.drawn)
-            self.ids[self.drawn:self.drawn + n] = self.draw(n)
-            self.drawn += n
-        return self.ids[part]
+        ids, bs, draw, at, upto, end = self.ids, self.batch_size, self.draw, self.drawn, part.stop, len(self.ids)
+        if upto is None or upto > end:
+            upto = end
+        while at < upto:
+            to = min(end, at + bs)
+            ids[at:to] = draw(to - at)
+            self.drawn = at = to
+        return ids[part]
 
 
 def _plain(sampler):
@@ -81,7 +83,11 @@ def eval_edge_prediction(model, negative_edge_sampler, data, n_neighbors, batch_
     n = data.n_interactions
     nb = math.ceil(n / batch_size)
     negatives = _Drawn(n, batch_size, draw)
-    own = all(getattr(getattr(model, f, None), "__func__", None) is getattr(TGN, f) for f in ("eval_epoch", "eval_epoch_metrics"))
+    # A stream that goes through the model as one group (orca_group_sizes: at most 32 batches, 76 k rows on 148 SMs, three an edge)
+    # has nothing to draw beside.  20 batches of 37 edges: 831 us, drawn beside it 850; 40 of 200, two groups: 1630, drawn beside it 1530.
+    one_group = nb <= 32 and n <= 25000 and reuse and (cache_plan is not None or getattr(model, "n_layers", 2) == 1)
+    own = not one_group and \
+        all(getattr(getattr(model, f, None), "__func__", None) is getattr(TGN, f) for f in ("eval_epoch", "eval_epoch_metrics"))
     if not own or not _plain(negative_edge_sampler):
         negatives = negatives[:]      # (somebody else's: all draws before the first batch, as the reference's caller sees it)
     try:

@@ -1008,12 +1008,13 @@ class TGN(nn.Module):
         def prepare(i0, i1):
             lo, up = i0 * bs, min(E, i1 * bs)
             hts[lo:up] = timestamps[lo:up]
+            neg = negatives[lo:up]      # (asked for once: they may be drawn only now, batch by batch)
             for i in range(i0, i1):
                 a, b = i * bs, min(E, (i + 1) * bs)
                 n, o = b - a, int(off[i])
                 hi[o:o + n] = sources[a:b]
                 hi[o + n:o + 2 * n] = destinations[a:b]
-                hi[o + 2 * n:o + 3 * n] = negatives[a:b]
+                hi[o + 2 * n:o + 3 * n] = neg[a - lo:b - lo]
                 hi[o + 3 * n:o + 4 * n] = edge_idxs[a:b]
                 if n_plan[i]:
                     hi[o + 4 * n:off[i + 1]] = cache_plan[i]

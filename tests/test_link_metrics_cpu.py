@@ -129,3 +129,40 @@ def test_the_sampler_is_left_behind_all_draws_of_the_stream(fails):
         _evaluate(model, sampler)
         assert model.taken == 50
     assert np.array_equal(want.sample(20)[1], sampler.sample(20)[1])
+
+
+def _model_taking(taken):
+    from orca_b200.tgn import TGN
+
+    class Model(TGN):
+        def __init__(self):
+            pass
+
+        n_layers = 2
+
+        def eval(self):
+            return self
+
+        def _eval_stream(self, sources, destinations, negatives, *rest):
+            taken.append((type(negatives), np.array(negatives[:])))
+            e = len(sources)
+            return np.full(e, .75, np.float32), np.full(e, .25, np.float32)
+
+    return Model()
+
+
+@pytest.mark.parametrize("n,bs,plan,reuse,beside", [(740, 37, True, True, False), (25000, 1000, True, True, False),
+                                                    (25001, 1000, True, True, True), (330, 10, True, True, True),
+                                                    (740, 37, False, True, True), (740, 37, True, False, True)])
+def test_negatives_of_one_group_are_drawn_before_it(n, bs, plan, reuse, beside):
+    """Negatives are drawn beside the GPU's work only where there is some: the ids are the same either way."""
+    import types
+    from orca_b200.evaluation import RandEdgeSampler, _Drawn, eval_edge_prediction
+    a, taken = np.arange(n), []
+    data = types.SimpleNamespace(sources=a, destinations=a, timestamps=a, edge_idxs=a, n_interactions=n)
+    eval_edge_prediction(_model_taking(taken), RandEdgeSampler(np.arange(5), np.arange(100), seed=3), data, 10, bs, reuse=reuse,
+                         cache_plan=[a[:1]] * (-(-n // bs)) if plan else None)
+    want = RandEdgeSampler(np.arange(5), np.arange(100), seed=3)
+    (kind, ids), = taken
+    assert (kind is _Drawn) == beside
+    assert np.array_equal(ids, np.concatenate([want.sample(min(bs, n - i))[1] for i in range(0, n, bs)]))
