@@ -218,9 +218,11 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   int row = tkt < n ? row_of_ticket(tkt) : -1;
   int my_nbr = 0, my_eid = 0;
   float my_dt = 0.f;
+  unsigned vmask = 0;                              // the row's valid slots
   if (row >= 0) {
     int q;
     load_indices(row, my_nbr, my_eid, my_dt, q);
+    vmask = __ballot_sync(FULL, my_nbr != 0);
     fetch_query(q);
   }
   float4 x[GS][3];                                 // (the third piece of the lanes that have none stays zero)
@@ -239,7 +241,6 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         load_indices(next, nx_nbr, nx_eid, nx_dt, nx_q);
       }
     };
-    const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
     float4 am0[3], am1[3];                         // weighted sums of the gathered part, heads 0 / 1
     float2 at0[GA_P_ITERS], at1[GA_P_ITERS];       // and of the time part
 #pragma unroll
@@ -247,15 +248,11 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
 #pragma unroll
     for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
     float sum0 = 0.f, sum1 = 0.f;
+    const int n_valid = __popc(vmask);
     tc::mbar_wait(qbar, phase, status, 800, alive, wait_limit);
-    if (vmask != 0) {
-      const int first = __ffs(vmask) - 1, range = 32 - __clz(vmask) - first;
-      const unsigned valid = vmask >> first;
+    phase ^= alive;      // (stays at a query that did not come)
+    if (n_valid > 0) {
       {
-        // empty places among the slots, and behind them up to a whole step, repeat the first slot with weight zero
-        const int f_nbr = __shfl_sync(FULL, my_nbr, first), f_eid = __shfl_sync(FULL, my_eid, first);
-        const float f_dt = __shfl_sync(FULL, my_dt, first);
-        if (my_nbr == 0) my_nbr = f_nbr, my_eid = f_eid, my_dt = f_dt;
         // which pair groups of the slot need the fixed-point cosine (see time_terms)
         const float adt = fabsf(my_dt);
         int large = (adt * wg0 >= COS_SMALL ? 1 : 0) + (adt * wg1 >= COS_SMALL ? 1 : 0) + (adt * wg2 >= COS_SMALL ? 1 : 0);
@@ -266,9 +263,11 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         rec.dt[0] = rec.dt[1] = my_dt;
         rec.large = large;
         rec.unused = 0;
-        if (lane >= first) s_rec[warp][lane - first] = rec;
-        if (lane == first)
-          for (int u = 0; u < GS - 1; ++u) s_rec[warp][range + u] = rec;
+        // the valid slots one behind the other; behind them, up to a whole step, the first one again with weight zero
+        const int at = __popc(vmask & ((1u << lane) - 1u));
+        if (my_nbr != 0) s_rec[warp][at] = rec;
+        if (my_nbr != 0 && at == 0)
+          for (int u = 0; u < GS - 1; ++u) s_rec[warp][n_valid + u] = rec;
         __syncwarp();
       }
       const float *q_src = s_q[warp];
@@ -276,7 +275,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       // GS slots at a time, each row of them in registers from its dot products to its weighted sum: nothing is
       // loaded twice, and the cross-lane sums of 2 * GS logits cost little more than those of one
       constexpr int V = 2 * GS, LPV = 32 / V;
-      for (int at = 0; at < range; at += GS) {
+      for (int at = 0; at < n_valid; at += GS) {
         float2 te[GS][GA_P_ITERS];
         float4 dts[GS];
 #pragma unroll
@@ -331,7 +330,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         float lg = warp_sum_many<V>(v, lane);
         // the next row of this warp: its indices land while this one is finished
         if (at == 0) draw_next();
-        if (!(valid >> (at + lane / (2 * LPV)) & 1u)) lg = -INFINITY;
+        if (at + lane / (2 * LPV) >= n_valid) lg = -INFINITY;
         float top = lg;
 #pragma unroll
         for (int o = 2 * LPV; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
@@ -377,13 +376,13 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         __syncwarp();
       }
       prof_rows += 1;
-      prof_slots += (unsigned long long)__popc(vmask);
+      prof_slots += (unsigned long long)n_valid;
     } else {
       draw_next();
     }
     __syncwarp();        // (the query has been read by all lanes: the next one may land)
+    const unsigned nx_mask = __ballot_sync(FULL, nx_nbr != 0);
     if (next >= 0) fetch_query(nx_q);
-    phase ^= alive;      // (stays at the query that did not come)
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
     const float inv0 = vmask ? 1.f / sum0 : 0.f, inv1 = vmask ? 1.f / sum1 : 0.f;
@@ -439,6 +438,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     my_nbr = nx_nbr;
     my_eid = nx_eid;
     my_dt = nx_dt;
+    vmask = nx_mask;
   }
   if (lane == 0) {
     if (!alive) tc::mbar_settle(qbar, phase);

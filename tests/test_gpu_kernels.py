@@ -308,6 +308,38 @@ def test_attention_gather_slots(dev, k):
         assert np.all(np.abs(got[rows, h * 516:(h + 1) * 516] - want) < (4 * delta[rows] + 1e-6)[:, None] * most + 7.8e-7)
 
 
+@pytest.mark.parametrize("k", [2, 3, 9, 10, 11, 12, 31, 32])
+def test_attention_gather_of_slots_with_gaps(dev, k):
+    """Only a row's valid slots, in their order, decide its result and the steps to it: the same bits wherever the empty places
+    lie among them (the rows are those of one table, with every number of valid slots, spread out and side by side)."""
+    from orca_b200 import _lib
+    rs = np.random.RandomState(k)
+    n, n_tab = 29 * (k + 1), 300
+    tab = torch.from_numpy(rs.randn(n_tab, D).astype(np.float32)).to(dev)
+    q = torch.from_numpy((rs.randn(n, 1056) * 0.3).astype(np.float32)).to(dev)
+    w = torch.from_numpy((1 / 10 ** np.linspace(0, 9, D)).astype(np.float32)).to(dev)
+    ids, dt = rs.randint(1, n_tab, (n, k)), (10.0 ** rs.uniform(0, 8, (n, k))).astype(np.float32)
+
+    def run(places):
+        nbr, delta = np.zeros((n, k), np.int32), np.zeros((n, k), np.float32)
+        for r, at in enumerate(places):
+            nbr[r, at], delta[r, at] = ids[r, :len(at)], dt[r, :len(at)]
+        d_nbr, d_dt = _i32(nbr, dev), torch.from_numpy(delta).to(dev)
+        ctx, valid = torch.full((n, 1032), 3.0, device=dev), torch.full((n,), 7, dtype=torch.uint8, device=dev)
+        _lib.check(_lib.lib().orca_attn_gather(q.data_ptr(), tab.data_ptr(), tab.data_ptr(), w.data_ptr(), d_nbr.data_ptr(),
+                                               d_nbr.data_ptr(), d_dt.data_ptr(), k, n, None, ctx.data_ptr(), valid.data_ptr(), None,
+                                               _lib.stream_ptr(dev)))
+        return ctx.cpu().numpy(), valid.cpu().numpy()
+
+    count = [r % (k + 1) for r in range(n)]
+    spread = run([np.sort(rs.permutation(k)[:m]) for m in count])
+    right = run([np.arange(k - m, k) for m in count])
+    left = run([np.arange(m) for m in count])
+    assert np.array_equal(right[1], np.minimum(count, 1)) and np.all(right[0][::k + 1] == 3.0)
+    for got in (spread, left):
+        assert np.array_equal(got[0], right[0]) and np.array_equal(got[1], right[1])
+
+
 @pytest.mark.parametrize("own", [True, False])
 @pytest.mark.parametrize("k", [10, 20])
 def test_attention_gather_reports_where_it_is_told(dev, own, k):
