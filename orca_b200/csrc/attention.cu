@@ -223,7 +223,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     int q;
     load_indices(row, my_nbr, my_eid, my_dt, q);
     vmask = __ballot_sync(FULL, my_nbr != 0);
-    fetch_query(q);
+    if (vmask != 0) fetch_query(q);
   }
   float4 x[GS][3];                                 // (the third piece of the lanes that have none stays zero)
 #pragma unroll
@@ -249,9 +249,9 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
     float sum0 = 0.f, sum1 = 0.f;
     const int n_valid = __popc(vmask);
-    tc::mbar_wait(qbar, phase, status, 800, alive, wait_limit);
-    phase ^= alive;      // (stays at a query that did not come)
     if (n_valid > 0) {
+      tc::mbar_wait(qbar, phase, status, 800, alive, wait_limit);
+      phase ^= alive;      // (stays at a query that did not come)
       {
         // which pair groups of the slot need the fixed-point cosine (see time_terms)
         const float adt = fabsf(my_dt);
@@ -382,7 +382,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
     }
     __syncwarp();        // (the query has been read by all lanes: the next one may land)
     const unsigned nx_mask = __ballot_sync(FULL, nx_nbr != 0);
-    if (next >= 0) fetch_query(nx_q);
+    if (nx_mask != 0) fetch_query(nx_q);      // (a row without valid slots asks for nothing)
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
     const float inv0 = vmask ? 1.f / sum0 : 0.f, inv1 = vmask ? 1.f / sum1 : 0.f;

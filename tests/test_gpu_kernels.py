@@ -340,6 +340,37 @@ def test_attention_gather_of_slots_with_gaps(dev, k):
         assert np.array_equal(got[0], right[0]) and np.array_equal(got[1], right[1])
 
 
+@pytest.mark.parametrize("k", [10, 20])
+@pytest.mark.parametrize("empty", [0.0, 0.5, 0.97, 1.0])
+def test_attention_gather_between_rows_without_slots(dev, k, empty):
+    """A row without valid slots asks for no query: its neighbours in a warp's run get theirs all the same (each row's result, bit
+    by bit, is that of the rows with slots alone), whatever lies where its own query would."""
+    from orca_b200 import _lib
+    rs = np.random.RandomState(k)
+    n, n_tab = 20000, 300
+    tab = torch.from_numpy(rs.randn(n_tab, D).astype(np.float32)).to(dev)
+    q = torch.from_numpy((rs.randn(n, 1056) * 0.3).astype(np.float32)).to(dev)
+    w = torch.from_numpy((1 / 10 ** np.linspace(0, 9, D)).astype(np.float32)).to(dev)
+    nbr, dt = rs.randint(1, n_tab, (n, k)), torch.from_numpy(rs.rand(n, k).astype(np.float32)).to(dev)
+    on = rs.rand(n) >= empty
+    nbr[~on] = 0
+    full = torch.from_numpy(on).to(dev)
+
+    def run(q, nbr, dt):
+        m = len(q)
+        ctx, valid = torch.full((m, 1032), 3.0, device=dev), torch.full((m,), 7, dtype=torch.uint8, device=dev)
+        _lib.check(_lib.lib().orca_attn_gather(q.data_ptr(), tab.data_ptr(), tab.data_ptr(), w.data_ptr(), nbr.data_ptr(),
+                                               nbr.data_ptr(), dt.data_ptr(), k, m, None, ctx.data_ptr(), valid.data_ptr(), None,
+                                               _lib.stream_ptr(dev)))
+        return ctx, valid
+
+    d_nbr = _i32(nbr, dev)
+    alone = run(q[full].contiguous(), d_nbr[full].contiguous(), dt[full].contiguous())[0] if on.any() else torch.empty(0, 1032, device=dev)
+    q[~full] = float("nan")
+    got, valid = run(q, d_nbr, dt)
+    assert torch.equal(valid, full.to(torch.uint8)) and torch.equal(got[full], alone) and bool((got[~full] == 3.0).all())
+
+
 @pytest.mark.parametrize("own", [True, False])
 @pytest.mark.parametrize("k", [10, 20])
 def test_attention_gather_reports_where_it_is_told(dev, own, k):
