@@ -218,12 +218,10 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   int row = tkt < n ? row_of_ticket(tkt) : -1;
   int my_nbr = 0, my_eid = 0;
   float my_dt = 0.f;
-  unsigned vmask = 0;                              // the row's valid slots
   if (row >= 0) {
     int q;
     load_indices(row, my_nbr, my_eid, my_dt, q);
-    vmask = __ballot_sync(FULL, my_nbr != 0);
-    if (vmask != 0) fetch_query(q);
+    if (__any_sync(FULL, my_nbr != 0)) fetch_query(q);
   }
   float4 x[GS][3];                                 // (the third piece of the lanes that have none stays zero)
 #pragma unroll
@@ -248,6 +246,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
 #pragma unroll
     for (int i = 0; i < GA_P_ITERS; ++i) at0[i] = at1[i] = make_float2(0.f, 0.f);
     float sum0 = 0.f, sum1 = 0.f;
+    const unsigned vmask = __ballot_sync(FULL, my_nbr != 0);
     const int n_valid = __popc(vmask);
     if (n_valid > 0) {
       tc::mbar_wait(qbar, phase, status, 800, alive, wait_limit);
@@ -381,11 +380,10 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
       draw_next();
     }
     __syncwarp();        // (the query has been read by all lanes: the next one may land)
-    const unsigned nx_mask = __ballot_sync(FULL, nx_nbr != 0);
-    if (nx_mask != 0) fetch_query(nx_q);      // (a row without valid slots asks for nothing)
+    if (__any_sync(FULL, nx_nbr != 0)) fetch_query(nx_q);      // (a row without valid slots asks for nothing)
     // write the row: [head 0: gathered 344 | time 172][head 1: ...].  A row whose slots are all padding has no attention
     // term: the image gets zeros (the fp32 form leaves such a row alone, `valid` says so).
-    const float inv0 = vmask ? 1.f / sum0 : 0.f, inv1 = vmask ? 1.f / sum1 : 0.f;
+    const float inv0 = n_valid > 0 ? 1.f / sum0 : 0.f, inv1 = n_valid > 0 ? 1.f / sum1 : 0.f;
     if (IMAGE) {
       char *im = (char *)ctx + (size_t)(row / img::ROWS) * (img::CTX_STAGES * img::STAGE_BYTES) + (row % img::ROWS) * 64;
       const int sw = (row << 3) & 0x30;
@@ -420,7 +418,7 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         *reinterpret_cast<uint2 *>(p) = make_uint2(0, 0);
         *reinterpret_cast<uint2 *>(p + img::STAGE_BYTES / 2) = make_uint2(0, 0);
       }
-    } else if (vmask != 0) {
+    } else if (n_valid > 0) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const int f = lane + 32 * i;
@@ -433,12 +431,11 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
         }
       }
     }
-    if (lane == 0) valid_out[row] = vmask != 0 ? 1 : 0;
+    if (lane == 0) valid_out[row] = n_valid > 0 ? 1 : 0;
     row = next;
     my_nbr = nx_nbr;
     my_eid = nx_eid;
     my_dt = nx_dt;
-    vmask = nx_mask;
   }
   if (lane == 0) {
     if (!alive) tc::mbar_settle(qbar, phase);
