@@ -191,3 +191,9 @@ def test_metrics_of_scores_that_are_not_finite_are_refused(bs, bad):
             assert _lib.lib().orca_link_metrics(pos.ctypes.data, neg.ctypes.data, E, bs, np.empty((2, 3)).ctypes.data) == 1
             said.append(_lib.lib().orca_last_error().decode())
     assert said[0] == said[1]
+
+
+@pytest.mark.parametrize("bs,k", [(2730, 32), (2731, 32), (2731, 1), (5462, 17)])
+def test_calls_that_order_more_rows_than_are_kept(bs, k):
+    """A call's rows are handed out in the order of their valid slots, which is kept for 8192 rows and counted again beyond."""
+    test_group_equals_batches("c1", bs, k, 2 * bs + 100, "budget", 2)
