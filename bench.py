@@ -472,10 +472,10 @@ def parity_vs_single(a, g, neg, plan, tgn, first, device, rank, world, n_batches
 
 
 # DRAM traffic of attn_gather_kernel: (dram__bytes_read.sum + dram__bytes_write.sum) of two consecutive
-# launches captured with ncu on workload c4 (15.37 + 14.96 MB read, 1 KB written) over the algorithmic bytes of
+# launches captured with ncu on workload c4 (15.38 + 14.96 MB read, nothing written) over the algorithmic bytes of
 # those launches (2 x 30.68 MB), applied to the algorithmic bytes of this run's launches; the counter cannot
 # be read while timing
-GATHER_TRAFFIC_RATIO = (15.372800 + 0.001024 + 14.955264) / (2 * 30.683416)
+GATHER_TRAFFIC_RATIO = (15.383552 + 14.960128) / (2 * 30.683416)
 
 
 def oracle_sample(g, neg, plan, first, n_batches, sub_bs, threads, min_seconds=0.0):

@@ -22,17 +22,19 @@ namespace orca {
 // two-wide fp32 instructions of this architecture while the loads are in flight -- then come the partial dot products
 // with the two query heads, one cross-lane sum of all logits of the step at once, a running softmax and the weighted sums,
 // all from the same registers.
-// What bounds it: the instructions of a row against the 16 or 12 warps an SM that the registers allow (a warp issues every
-// 7 cycles, issue slots half busy), and with ten slots a row DRAM, which carries the queries in and the images out
-// (66 k rows of the largest graph: 0.85 GB, 5 TB/s).  Loads of the slots' rows cost next to nothing: with all of them in L1
-// a launch took 2 % less.  So what helps is fewer instructions a slot (193 -> 160, and 143 four at a time, of 75 that the sums,
+// What bounds it: the instructions of a row and the SM's load path, against the 16 or 12 warps an SM that the registers allow
+// (66 k rows of the largest graph, counters: 0.42 GB to and from DRAM in layer 1, 0.56 in layer 2, 2.5 and 3.4 TB/s or 39 and
+// 52 % of what a copy reaches; 36 and 54 k rows of 194 k nodes: issue slots 55 % busy, L1 66 %, L2 28 %, DRAM 22 to 35 %).
+// Loads of the slots' rows cost next to nothing: with all of them in L1 a launch took 2 % less.  So what helps is fewer instructions a slot (193 -> 160, and 143 four at a time, of 75 that the sums,
 // products and cosines cannot do without) and queries that do not pass through L1 once a step:
 //   - what all lanes need of a slot (addresses, time difference) is worked out once a row, a slot a lane, and read back from
 //     shared memory; so are the weights, twice each, as the packed instructions take them;
 //   - one exponential a step gives weights and scales, in lanes of their own; sums are rescaled where a maximum rose;
 //   - a row's query is brought to shared memory by one bulk copy while the row before it is written.
 // us a launch (queries written by the kernel before; 66 k rows of the largest graph, K 10 / 60 k of c4, K 10 / 54 k, K 20):
-// before 197 / 197 / 340; so 166 / 162 / 254.  Four slots a step at 168 registers against two at 128, 27 k rows, K 8 / 10 / 12 /
+// before 197 / 197 / 340; so 166 / 162 / 254.  Valid slots side by side wherever their places are, no query for a row without any:
+// 40 k rows of ten / twenty slots 149 / 217 (152 / 220 from the first valid place to the last), half of the places empty 107 / 150
+// (127 / 199), none valid 31 (45).  Four slots a step at 168 registers against two at 128, 27 k rows, K 8 / 10 / 12 /
 // 14 / 16 / 20 / 32: 79 / 97 / 97 / 116 / 117 / 136 / 187 against 83 / 93 / 106 / 118 / 130 / 152 / 214; 30 k of c4, where rows are
 // shorter: 81 / 95 / 97 / 112 / 112 / 128 / 175 against 80 / 89 / 97 / 108 / 116 / 136 / 192: four from K 11 on.
 // Measured against it: queries in registers at 12 warps (181 / 175 / 288); a row's first slots loaded before the row in front
@@ -220,9 +222,9 @@ attn_gather_kernel(const float *__restrict__ qt, const float *__restrict__ nbr_t
   const float wg0 = __ldg(time_w), wg1 = __ldg(time_w + 64), wg2 = __ldg(time_w + 128);
   unsigned long long prof_rows = 0, prof_slots = 0;
 
-  // (A group's rows from the last one back: the queries written last are still in L2, and so are the images of the rows
-  // that the output kernel starts with.  200 MB of queries a launch do not fit it: 50 batches of 2000 5.80 -> 5.68 ms, 51 of
-  // 600 3.00 -> 2.96, without reuse 2.36 -> 2.30.)
+  // (A group's rows from the last one back: the images of the rows that the output kernel starts with are still in L2, and so,
+  // where every row has a query of its own, are the queries written last.  Measured when both layers' rows had: 200 MB of
+  // queries a launch do not fit L2, 50 batches of 2000 5.80 -> 5.68 ms, 51 of 600 3.00 -> 2.96, without reuse 2.36 -> 2.30.)
   auto row_of_ticket = [&](int t) -> int { return order != nullptr ? order[t] : n - 1 - t; };
   auto load_indices = [&](int r, int &o_nbr, int &o_eid, float &o_dt, int &o_q) {
     o_q = q_row != nullptr ? q_row[r] : r;

@@ -21,7 +21,7 @@ constexpr int FEAT_STAGES = 6, CTX_STAGES = 33;
 constexpr int PAIR_STAGES = 11;     // two embeddings one after the other, 344 columns, padded to 352 (score_rows.cu)
 inline size_t bytes(int64_t rows, int stages) { return (size_t)((rows + ROWS - 1) / ROWS) * stages * STAGE_BYTES; }
 
-// columns c .. c + 3 / c, c + 1 of row r: heads, and tails half a stage further
+// columns c .. c + 3 of row r: heads, and tails half a stage further
 template <int STAGES>
 __device__ __forceinline__ char *at(char *image, int r, int c) {
   return image + ((size_t)(r / ROWS) * STAGES + (c >> 5)) * STAGE_BYTES + (r % ROWS) * 64 +
@@ -35,14 +35,6 @@ __device__ __forceinline__ void put4(char *image, int r, int c, float4 x) {
   char *p = at<STAGES>(image, r, c);
   *reinterpret_cast<uint2 *>(p) = hi;
   *reinterpret_cast<uint2 *>(p + STAGE_BYTES / 2) = lo;
-}
-template <int STAGES>
-__device__ __forceinline__ void put2(char *image, int r, int c, float2 x) {
-  uint32_t lo;
-  const uint32_t hi = tc::pack_split(x.x, x.y, lo);
-  char *p = at<STAGES>(image, r, c);
-  *reinterpret_cast<uint32_t *>(p) = hi;
-  *reinterpret_cast<uint32_t *>(p + STAGE_BYTES / 2) = lo;
 }
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {   // K-major, 64-byte swizzle: 8 rows = 512 bytes
   return (uint64_t)((addr >> 4) & 0x3fff) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |

@@ -39,7 +39,11 @@ constexpr int A_CHUNKS = 2 * PART_CHUNKS, A_LBO = ROWS * 16 + 16, A_BYTES = A_CH
 constexpr int SMEM = 2 * W_BYTES + 2 * A_BYTES + 1024;
 constexpr int EPI_WARPS = 4, PRODUCERS = 256, THREADS = 32 * EPI_WARPS + PRODUCERS + 32;
 constexpr int TMEM_COLS = 128, BUF_COLS = 64, SMALL = 32;   // two accumulator buffers of main + cross terms
-constexpr int BLOCK_ROWS = 64;                 // updates a row block takes before there is another one
+// Updates that a row block takes before there is another one, in groups whose last updates leave the chain.  A CTA holds an SM
+// beside layers that want every one, and 64 rows take hardly longer than 32.  32 / 64, us a stream: 48 batches of 1000
+// 2527 / 2473, 50 of 2000 and 51 of 600 within 1 %; 30 of 400 970 / 978, 30 of 600 1213 / 1233; 20 to 2000 edges a batch, one and two
+// layers, 10 and 20 neighbours otherwise within 1 %.  (96 and 128 cost batches of 600 and 2000 2 and 3 %.)
+constexpr int BLOCK_ROWS = 64;
 constexpr int META = 4;                        // steps whose memory rows are kept
 constexpr int PER = 6;                         // chunks a producer thread has in flight: 34 rows at a time
 

@@ -399,8 +399,9 @@ extern "C" int64_t orca_csr_build_workspace_bytes(int64_t n_edges, int64_t n_nod
 }
 
 // slots of the packing threads; a thread is worth starting for a chunk or more.  7.8 M edges, the whole call: 24.9 ms
-// with one thread, 13.2 / 8.6 / 5.9 / 6.1 with 2 / 4 / 8 / 16 on 16 cores: from eight on the threads keep ahead of the
-// bus (2.9 ms), and what is left is the bus, the sort behind it (0.6 ms) and the gathers of emit_kernel (0.36).
+// with one thread, 13.2 / 8.6 / 5.9 / 6.1 with 2 / 4 / 8 / 16 on 16 cores (another box: 6.6 with 16): from eight on the threads are not
+// what it waits for.  The copies are: 120 chunks of 1.3 MB, most of them at the bus's rate (28 us) and others three to six times
+// that, 5.9 ms in all where the bus alone would take 2.9; then the sort (0.5 ms) and the gathers of emit_kernel (0.35).
 constexpr int MOST_THREADS = 16;
 static int pack_threads(int64_t n_edges) {
   const int64_t chunks = (n_edges + csr::CHUNK - 1) >> csr::CHUNK_LOG;
